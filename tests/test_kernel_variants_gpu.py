@@ -1,0 +1,178 @@
+"""Branches of the kernel dispatch at the sizes where they begin, end or leave a remainder, against plain PyTorch in fp32 / fp64."""
+import math
+
+import pytest
+import torch
+
+from llmq_b200.ops import kernels as K
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+BF = torch.bfloat16
+
+
+@pytest.fixture(autouse=True)
+def _check_status():
+    yield
+    torch.cuda.synchronize()
+    K.check_status(torch.device(DEV, 0))
+
+
+def rel(a, b):
+    a, b = a.double().cpu(), b.double().cpu()
+    return ((a - b).norm() / b.norm().clamp_min(1e-30)).item()
+
+
+# one head per CTA and clusters of 2 .. 8 CTAs (small grids), whole groups per CTA (large grids), one query tile without a second
+@pytest.mark.parametrize("HS", [64, 128])
+@pytest.mark.parametrize("B,T,Hq,Hkv", [(1, 1, 2, 1), (1, 63, 3, 1), (2, 64, 4, 2), (1, 65, 14, 2), (1, 128, 7, 1), (3, 129, 5, 1), (1, 257, 8, 1),
+                                        (1, 300, 16, 1), (2, 384, 6, 3), (1, 1000, 4, 4), (24, 130, 14, 7), (8, 1200, 12, 6)])
+def test_attention_head_splits(HS, B, T, Hq, Hkv):
+    g = torch.Generator(device=DEV).manual_seed(T)
+    qkv = torch.randn(B, T, Hq + 2 * Hkv, HS, device=DEV, generator=g).to(BF)
+    dout = torch.randn(B, T, Hq, HS, device=DEV, generator=g).to(BF)
+    out, lse = torch.full((B, T, Hq, HS), 9.0, device=DEV, dtype=BF), torch.empty(B, Hq, T, device=DEV)
+    dqkv, scratch = torch.full_like(qkv, 9.0), torch.empty(B * Hq * T, device=DEV)
+    K.attention_forward(out, lse, qkv, Hq, Hkv)
+    K.attention_backward(dqkv, scratch, dout, out, lse, qkv, Hq, Hkv)
+    again = torch.empty_like(dqkv)
+    K.attention_backward(again, scratch, dout, out, lse, qkv, Hq, Hkv)
+    assert torch.equal(dqkv, again)                       # no order depends on the schedule
+    x = qkv.float().requires_grad_(True)
+    o, l = K._attention_ref(x, Hq, Hkv)
+    o.backward(dout.float())
+    # 16-bit probabilities and score gradients (2^-9 each, random signs) and the 16-bit outputs
+    assert rel(out, o.detach()) < 1e-2 and (lse - l.detach()).abs().max() < 2e-3
+    if T > 1:
+        assert rel(dqkv[:, :, :Hq], x.grad[:, :, :Hq]) < 1.2e-2
+        assert rel(dqkv[:, :, Hq:Hq + Hkv], x.grad[:, :, Hq:Hq + Hkv]) < 1.2e-2
+    assert rel(dqkv[:, :, Hq + Hkv:], x.grad[:, :, Hq + Hkv:]) < 1.2e-2
+
+
+# one thread vector, exactly full CTAs (512 x 5 vectors), one vector more (two CTAs), four and eight CTAs, the largest row that
+# eight hold, and one more (streaming kernel); tails behind the last whole vector
+@pytest.mark.parametrize("V", [8, 13, 4096, 20480, 20488, 40967, 81920, 128256, 163840, 163847, 163848, 200000])
+@pytest.mark.parametrize("z_reg", [0.0, 1e-3])
+def test_fused_classifier_row_splits(V, z_reg):
+    rows, ld = 5, (V + 7) // 8 * 8
+    g = torch.Generator().manual_seed(V)
+    buf = torch.randn(rows, ld, generator=g).mul_(3).to(BF)
+    buf[3, 1:V] = -math.inf                               # one finite logit
+    buf[2, : V // 2] = torch.finfo(BF).min                # masked by the type's lowest value
+    logits = buf.to(DEV)[:, :V]
+    tg = torch.tensor([V - 1, -100, V // 2, 0, (V - 1) // 8 * 8], dtype=torch.int32)
+    losses, lse = torch.full((rows,), 0.5, device=DEV), torch.empty(rows, device=DEV)
+    K.fused_classifier(logits, losses, lse, tg.to(DEV), 0.25, z_reg * 0.25, True)
+    x = buf[:, :V].double()
+    ok, safe = tg >= 0, tg.clamp_min(0).long()
+    l = torch.logsumexp(x, -1)
+    want_loss = 0.5 + torch.where(ok, l - x[torch.arange(rows), safe], torch.zeros_like(l))
+    p = torch.exp(x - l[:, None]) * (0.25 * (1 + z_reg * l))[:, None]
+    p[torch.arange(rows), safe] -= 0.25
+    p[~ok] = 0
+    assert (losses.cpu().double() - want_loss).abs().max() < 2e-5 * (1 + want_loss.abs().max())
+    assert (lse.cpu().double() - torch.where(ok, l, torch.zeros_like(l))).abs().max() < 2e-5 * (1 + l[ok].abs().max())
+    # one bf16 rounding (2^-9 of the value); the target's entry keeps the fp32 error of p next to its -0.25
+    assert ((logits.cpu().double() - p).abs() <= p.abs() * 2 ** -8 + 1e-6).all()
+    if ld > V:
+        assert torch.equal(buf.to(DEV)[:, V:].cpu(), buf[:, V:])
+
+
+def test_fused_classifier_rows_without_a_finite_maximum():
+    V = 30000
+    x = torch.full((3, V), -math.inf)
+    x[1, 7] = math.inf
+    x[2] = 0.0
+    x[2, 5] = math.nan
+    losses, lse = torch.zeros(3, device=DEV), torch.zeros(3, device=DEV)
+    K.fused_classifier(x.to(BF).to(DEV), losses, lse, torch.tensor([1, 2, 3], dtype=torch.int32, device=DEV), 1.0)
+    assert lse[0].item() == -math.inf and math.isnan(lse[1].item()) and math.isnan(lse[2].item())
+
+
+# several rows side by side in a CTA, exactly one 512-thread row, rows of up to 1024 vectors, the two-pass kernels beyond
+@pytest.mark.parametrize("dtype", [BF, torch.float32])
+@pytest.mark.parametrize("C", [8, 264, 512, 896, 3584, 4096, 4104, 8192, 8200, 16384])
+@pytest.mark.parametrize("rows", [1, 37, 700])
+def test_rmsnorm_row_splits(dtype, C, rows):
+    if dtype == torch.float32 and C > 8192:
+        pytest.skip("longer than the backward kernel takes")
+    g = torch.Generator().manual_seed(C + rows)
+    r = lambda *s: torch.randn(*s, generator=g).to(dtype)
+    x, y, w, dy, dres, dw0 = r(rows, C), r(rows, C), r(C), r(rows, C), r(rows, C), r(C)
+    res, out, rstd = torch.empty(rows, C, dtype=dtype, device=DEV), torch.empty(rows, C, dtype=dtype, device=DEV), torch.empty(rows, device=DEV)
+    am, amb = torch.zeros(1, device=DEV), torch.zeros(1, device=DEV)
+    K.rmsnorm_forward(out, rstd, x.to(DEV), w.to(DEV), 1e-6, residual_out=res, inp2=y.to(DEV), absmax=am)
+    s = (x.float() + y.float()).to(dtype)
+    assert torch.equal(res.cpu(), s)
+    rs = torch.rsqrt(s.double().square().mean(-1, keepdim=True) + 1e-6)
+    want = s.double() * rs * w.double()
+    eps = 2 ** -8 if dtype == BF else 2 ** -22            # half a unit of the last place of the storage type; fp32: a few ulp
+    assert ((out.cpu().double() - want).abs() <= 2.1 * eps * want.abs() + 1e-30).all()        # x * rstd and its product with w are rounded
+    assert am.item() == out.float().abs().max().item()
+    assert (rstd.cpu().double() / rs[:, 0] - 1).abs().max() < 1e-6
+    plain = torch.empty_like(out)
+    K.rmsnorm_forward(plain, None, res, w.to(DEV), 1e-6)
+    assert torch.equal(plain, out)
+    dinp, dw = dres.to(DEV), dw0.to(DEV)
+    scratch = torch.full((K.rmsnorm_backward_scratch_elems(C, DEV),), math.nan, device=DEV)
+    K.rmsnorm_backward(dinp, dw, scratch, dy.to(DEV), res, w.to(DEV), rstd, absmax=amb)
+    xh, wdy = s.double() * rs, w.double() * dy.double()
+    gx = dres.double() + (wdy - xh * (wdy * xh).mean(-1, keepdim=True)) * rs
+    gw = dw0.double() + (dy.double() * xh).sum(0)
+    assert rel(dinp, gx) < eps and rel(dw, gw) < eps
+    assert amb.item() == dinp.float().abs().max().item()
+
+
+@pytest.mark.parametrize("N", [300, 301, 896])            # whole vectors of four columns, and not
+@pytest.mark.parametrize("out_dt", [BF, torch.float32])
+def test_split_k_reduce(N, out_dt):
+    g = torch.Generator().manual_seed(N)
+    M, Kd = 200, 4096
+    a, b, bias = torch.randn(M, Kd, generator=g).to(BF), torch.randn(N, Kd, generator=g).to(BF), torch.randn(N, generator=g).to(BF)
+    prev = torch.randn(M, N, generator=g).to(out_dt)
+    out, am = prev.to(DEV), torch.zeros(1, device=DEV)
+    K.gemm(out, a.to(DEV), b.to(DEV), bias=bias.to(DEV), accumulate=True, alpha=0.5, absmax=am)
+    want = 0.5 * (a.double() @ b.double().t()) + bias.double() + prev.double()
+    assert rel(out, want) < (2 ** -8 if out_dt == BF else 1e-5)
+    assert abs(am.item() - want.abs().max().item()) < 1e-3 * want.abs().max().item()
+
+
+@pytest.mark.parametrize("n", [8, 8 * 512 * 512 - 8, 8 * 512 * 512 * 4 + 8, 12345679])
+@pytest.mark.parametrize("dtype", [BF, torch.float32])
+def test_norm_squared_sizes(n, dtype):
+    x = torch.randn(n, device=DEV).to(dtype)
+    part, out = torch.full((512,), 0.25, device=DEV), torch.empty(1, device=DEV)
+    K.norm_squared(part, x)
+    K.deterministic_sum(out, part)
+    want = 128.0 + x.double().square().sum().item()
+    assert abs(out.item() - want) < 1e-5 * want
+
+
+def test_adamw_stores_non_finite_values_as_they_are():
+    n = 256
+    p, m, v = (torch.zeros(n, device=DEV, dtype=BF) for _ in range(3))
+    g = torch.ones(n, device=DEV, dtype=BF)
+    g[3], g[10], g[17] = math.inf, -math.inf, math.nan
+    K.adamw(p, g, m, v, lr=0.1, beta1=0.9, beta2=0.95, step=1, eps=1e-8, weight_decay=0.0, seed=3)
+    assert m[3].item() == math.inf and m[10].item() == -math.inf and math.isnan(m[17].item()) and math.isnan(p[17].item())
+    assert v[3].item() == math.inf and v[10].item() == math.inf and math.isnan(v[17].item())
+    ok = torch.ones(n, dtype=torch.bool, device=DEV)
+    ok[[3, 10, 17]] = False
+    assert (p[ok].float() + 0.1).abs().max() < 1e-3 and torch.isfinite(m[ok]).all()
+
+
+# MN-major operands whose extent is whole 128-byte chunks (one 3-D load per stage), the last tile partly outside the matrix, and
+# extents with a ragged last chunk (2-D boxes); one-CTA kernel and CTA pairs (from 2^21 outputs)
+@pytest.mark.parametrize("M,N,Kd", [(320, 448, 200), (64, 192, 72), (128, 384, 65), (2112, 1088, 136), (2112, 1152, 264), (2080, 1040, 130)])
+@pytest.mark.parametrize("dt", [BF, torch.float8_e4m3fn])
+@pytest.mark.parametrize("a_mn,b_mn", [(1, 0), (0, 1), (1, 1)])
+def test_gemm_mn_major_chunks(M, N, Kd, dt, a_mn, b_mn):
+    if not (a_mn and b_mn):
+        Kd = (Kd + 15) // 16 * 16                          # rows of a K-major operand start at multiples of 16 bytes
+    g = torch.Generator().manual_seed(M + N)
+    a, b = torch.randn(M, Kd, generator=g).to(dt), torch.randn(N, Kd, generator=g).to(dt)
+    sa = a.float().t().contiguous().to(dt) if a_mn else a
+    sb = b.float().t().contiguous().to(dt) if b_mn else b
+    out = torch.full((M, N), 5.0, dtype=torch.float32, device=DEV)
+    K.gemm(out, sa.to(DEV), sb.to(DEV), a_mn=bool(a_mn), b_mn=bool(b_mn))
+    assert rel(out, a.double() @ b.double().t()) < 1e-5    # exact products, fp32 sums
