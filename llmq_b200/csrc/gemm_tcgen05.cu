@@ -234,6 +234,51 @@ __global__ void __launch_bounds__(256) splitk_reduce_kernel(const GemmParams p, 
     if (p.absmax_out) block_absmax_commit(p.absmax_out, tmax, scratch);
 }
 
+// The same, four columns per thread, for bf16 / fp32 outputs with rows of whole 16-byte partial vectors (N and ldc multiples of
+// 4, aligned C): 16-byte loads of the parts, and a multiply instead of a 64-bit division per element.  1152 x 896 from two parts:
+// 3.8 us against 14.
+__global__ void __launch_bounds__(256) splitk_reduce_vec_kernel(const GemmParams p, float alpha_host, const FastDiv fd) {
+    __shared__ float scratch[32];
+    float alpha = alpha_host;
+    if (p.scale_a) alpha *= *p.scale_a;
+    if (p.scale_b) alpha *= *p.scale_b;
+    const long long total = static_cast<long long>(p.M) * p.N;
+    const uint32_t nvec = static_cast<uint32_t>(total / 4);
+    float tmax = 0.f;
+    for (uint32_t i = blockIdx.x * 256u + threadIdx.x; i < nvec; i += gridDim.x * 256u) {
+        uint32_t row, cv;
+        fd.divmod(i, row, cv);
+        const int col = static_cast<int>(cv) * 4;
+        float v[4] = {0.f, 0.f, 0.f, 0.f};
+        for (int s = 0; s < p.k_splits; ++s) {
+            const float4 q = *reinterpret_cast<const float4*>(p.partial + static_cast<long long>(s) * total + static_cast<long long>(i) * 4);
+            v[0] += q.x; v[1] += q.y; v[2] += q.z; v[3] += q.w;
+        }
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            v[k] *= alpha;
+            if (p.bias) v[k] += p.bias_dtype == 0 ? __bfloat162float(static_cast<const __nv_bfloat16*>(p.bias)[col + k]) : static_cast<const float*>(p.bias)[col + k];
+        }
+        if (p.c_dtype == 0) {
+            uint2* c = reinterpret_cast<uint2*>(static_cast<__nv_bfloat16*>(p.C) + row * p.ldc + col);
+            if (p.accumulate) {
+                const uint2 old = *c;
+                v[0] += __uint_as_float(old.x << 16); v[1] += __uint_as_float(old.x & 0xffff0000u);
+                v[2] += __uint_as_float(old.y << 16); v[3] += __uint_as_float(old.y & 0xffff0000u);
+            }
+            const __nv_bfloat162 lo = __floats2bfloat162_rn(v[0], v[1]), hi = __floats2bfloat162_rn(v[2], v[3]);
+            *c = make_uint2(*reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi));
+        } else {
+            float4* c = reinterpret_cast<float4*>(static_cast<float*>(p.C) + row * p.ldc + col);
+            if (p.accumulate) { const float4 old = *c; v[0] += old.x; v[1] += old.y; v[2] += old.z; v[3] += old.w; }
+            *c = make_float4(v[0], v[1], v[2], v[3]);
+        }
+#pragma unroll
+        for (int k = 0; k < 4; ++k) tmax = fmaxf(tmax, fabsf(v[k]));
+    }
+    if (p.absmax_out) block_absmax_commit(p.absmax_out, tmax, scratch);
+}
+
 // ------------------------------------------------------------------------------------------------
 // Host side: tensor-map encoding through the driver entry point (no link-time libcuda dependency).
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
@@ -439,7 +484,15 @@ static int gemm_impl(const void* A, const void* B, void* C, const void* bias,
     else if (eb == 2) gemm_tcgen05_kernel<0><<<grid, NUM_THREADS, SMEM_BYTES, stream>>>(ta, tb, p);
     else              gemm_tcgen05_kernel<2><<<grid, NUM_THREADS, SMEM_BYTES, stream>>>(ta, tb, p);
     if (splits > 1) {
-        long long blocks = (static_cast<long long>(M) * N + 255) / 256;
+        const long long total = static_cast<long long>(M) * N;
+        const int out_bytes = c_dtype == 0 ? 8 : 16;                       // four columns
+        if (N % 4 == 0 && ldc % 4 == 0 && total < (1ll << 31) && reinterpret_cast<uintptr_t>(C) % out_bytes == 0) {
+            long long blocks = (total / 4 + 255) / 256;
+            if (blocks > 8LL * num_sms) blocks = 8LL * num_sms;
+            splitk_reduce_vec_kernel<<<static_cast<unsigned int>(blocks), 256, 0, stream>>>(p, p.alpha, FastDiv(static_cast<uint32_t>(N / 4)));
+            return static_cast<int>(cudaGetLastError());
+        }
+        long long blocks = (total + 255) / 256;
         if (blocks > 4LL * num_sms) blocks = 4LL * num_sms;
         splitk_reduce_kernel<<<static_cast<unsigned int>(blocks), 256, 0, stream>>>(p, p.alpha);
     }
