@@ -58,6 +58,9 @@ struct GemmParams {
     // CTA-pair kernel: 1 when the kernel's third tensor map describes C (bf16, plain store) and the epilogue may write
     // its staged 32 x 64 blocks with TMA stores instead of per-lane global stores
     int c_tma;
+    // MN-major operands whose M / N extent is a multiple of the 128-byte chunk: the tensor map is 3-D (chunk column, K row, chunk)
+    // and one load fetches all chunks of a stage
+    int a_box3, b_box3;
 };
 
 // Adds bias[col0 .. col0+31] to the 32 values of one accumulator chunk (every lane needs the same 32 bias values:

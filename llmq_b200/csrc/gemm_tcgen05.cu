@@ -14,9 +14,9 @@
 // (src/kernels/matmul.cpp:46-153, src/kernels/gemm_mma.cu:21-291).
 //
 // Structure (192 threads per CTA, one CTA per SM):
-//   warp 0     TMA producer: fills a 4-stage ring of 128x(128 B) A and 256x(128 B) B tiles
+//   warp 0     TMA producer: fills a 4-stage ring of 128x(128 B) A and 256x(128 B) B tiles (6 stages with 128-wide B tiles)
 //   warp 1     MMA issuer (one elected lane): 4 tcgen05.mma per stage into one of two
-//              128x256 fp32 accumulators in TMEM, tcgen05.commit to free the stage
+//              128x256 (or 128x128) fp32 accumulators in TMEM, tcgen05.commit to free the stage
 //   warps 2-5  epilogue: tcgen05.ld the finished accumulator (while the other one is being
 //              computed), scale, add bias, optionally add the previous C, track abs-max, store
 #include "ptx_sm100.cuh"
@@ -29,15 +29,17 @@ using namespace sm100;
 namespace {
 
 constexpr int BM = 128;
-constexpr int BN = 256;
 constexpr int ROW_BYTES = 128;            // one swizzle row
-constexpr int STAGES = 4;
 constexpr int A_STAGE_BYTES = BM * ROW_BYTES;   // 16 KiB
-constexpr int B_STAGE_BYTES = BN * ROW_BYTES;   // 32 KiB
-constexpr int STAGE_BYTES = A_STAGE_BYTES + B_STAGE_BYTES;
 constexpr int NUM_THREADS = 192;
-constexpr int TMEM_COLS = 512;            // two 256-column accumulators
-constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 1024 /*alignment slack*/ + 256 /*barriers*/;
+// Tile width BN is 256, or 128 for outputs with so few tiles that half the SMs would idle.  Two accumulators of BN columns.
+template <int BN> struct Tile {
+    static constexpr int STAGES = BN == 256 ? 4 : 6;
+    static constexpr int B_STAGE_BYTES = BN * ROW_BYTES;
+    static constexpr int STAGE_BYTES = A_STAGE_BYTES + B_STAGE_BYTES;
+    static constexpr int TMEM_COLS = 2 * BN;
+    static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 1024 /*alignment slack*/ + 256 /*barriers*/;
+};
 
 
 __device__ __forceinline__ void tile_coords(int t, int tiles_m, int tiles_n, int& tm, int& tn) {
@@ -53,10 +55,12 @@ __device__ __forceinline__ void tile_coords(int t, int tiles_m, int tiles_n, int
 }
 
 // Kind: MMA kind of ptx_sm100.cuh's mma_issue (0 bf16, 1 8-bit floats, 2 tf32 on fp32 operands).
-template <int Kind>
+template <int Kind, int BN>
 __global__ void __launch_bounds__(NUM_THREADS, 1)
 gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
                     const GemmParams p) {
+    constexpr int STAGES = Tile<BN>::STAGES, B_STAGE_BYTES = Tile<BN>::B_STAGE_BYTES, STAGE_BYTES = Tile<BN>::STAGE_BYTES;
+    constexpr int TMEM_COLS = Tile<BN>::TMEM_COLS;
     extern __shared__ uint8_t smem_raw[];
     // 128B-swizzled tiles must start on a 1024-byte boundary
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -65,7 +69,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * STAGES + 4);
     volatile uint32_t* abort_flag = tmem_slot + 1;
 
-    const int warp = threadIdx.x >> 5;
+    const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0);      // uniform, and known to be
     const int lane = threadIdx.x & 31;
     const uint32_t smem_base = smem_u32(smem);
     const uint32_t bar_base = smem_u32(bars);
@@ -99,9 +103,10 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
 
     if (warp == 0) {
         // ------------------------------------------------------------------ TMA producer
-        if (lane == 0) {
-            tma_prefetch_desc(&tmap_a);
-            tma_prefetch_desc(&tmap_b);
+        // the whole warp runs the loop, the elected lane issues (see gemm_tcgen05_2cta.cu)
+        {
+            const bool leader = elect_one();
+            if (leader) { tma_prefetch_desc(&tmap_a); tma_prefetch_desc(&tmap_b); }
             int stage = 0; uint32_t phase = 0;
             const int mn_chunk = ROW_BYTES / p.elem_bytes;     // M/N elements per 128-byte row (MN-major)
             bool ok = true;
@@ -109,32 +114,40 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
                 int tm, tn; tile_coords(t / splits, tiles_m, tiles_n, tm, tn);
                 const int k_begin = (t % splits) * k_per_split, k_end = min(k_iters, k_begin + k_per_split);
                 for (int k = k_begin; k < k_end; ++k) {
-                    if (!mbar_wait(empty_bar(stage), phase ^ 1u, abort_flag)) { atomicOr(p.status, kErrEmptyWait); ok = false; break; }
+                    if (!mbar_wait_warp(empty_bar(stage), phase ^ 1u, abort_flag)) { if (leader) atomicOr(p.status, kErrEmptyWait); ok = false; break; }
                     uint32_t sa = smem_base + stage * STAGE_BYTES;
                     uint32_t sb = sa + A_STAGE_BYTES;
-                    mbar_expect_tx(full_bar(stage), STAGE_BYTES);
-                    if (!p.a_mn_major) {
-                        tma_load_2d(sa, &tmap_a, full_bar(stage), k * bk, tm * BM);
-                    } else {
-                        // boxes of [bk K-rows][128 B of M]; BM*elem_bytes/128 boxes side by side
-                        int nbox = BM * p.elem_bytes / ROW_BYTES;
-                        for (int b = 0; b < nbox; ++b)
-                            tma_load_2d(sa + b * (A_STAGE_BYTES / nbox), &tmap_a, full_bar(stage), tm * BM + b * mn_chunk, k * bk);
+                    if (leader) {
+                        mbar_expect_tx(full_bar(stage), STAGE_BYTES);
+                        if (!p.a_mn_major) {
+                            tma_load_2d(sa, &tmap_a, full_bar(stage), k * bk, tm * BM);
+                        } else if (p.a_box3) {
+                            tma_load_3d(sa, &tmap_a, full_bar(stage), 0, k * bk, tm * (BM / mn_chunk));
+                        } else {
+                            // boxes of [bk K-rows][128 B of M]; BM*elem_bytes/128 boxes side by side
+                            int nbox = BM * p.elem_bytes / ROW_BYTES;
+                            for (int b = 0; b < nbox; ++b)
+                                tma_load_2d(sa + b * (A_STAGE_BYTES / nbox), &tmap_a, full_bar(stage), tm * BM + b * mn_chunk, k * bk);
+                        }
+                        if (!p.b_mn_major) {
+                            tma_load_2d(sb, &tmap_b, full_bar(stage), k * bk, tn * BN);
+                        } else if (p.b_box3) {
+                            tma_load_3d(sb, &tmap_b, full_bar(stage), 0, k * bk, tn * (BN / mn_chunk));
+                        } else {
+                            int nbox = BN * p.elem_bytes / ROW_BYTES;
+                            for (int b = 0; b < nbox; ++b)
+                                tma_load_2d(sb + b * (B_STAGE_BYTES / nbox), &tmap_b, full_bar(stage), tn * BN + b * mn_chunk, k * bk);
+                        }
                     }
-                    if (!p.b_mn_major) {
-                        tma_load_2d(sb, &tmap_b, full_bar(stage), k * bk, tn * BN);
-                    } else {
-                        int nbox = BN * p.elem_bytes / ROW_BYTES;
-                        for (int b = 0; b < nbox; ++b)
-                            tma_load_2d(sb + b * (B_STAGE_BYTES / nbox), &tmap_b, full_bar(stage), tn * BN + b * mn_chunk, k * bk);
-                    }
+                    __syncwarp();
                     if (++stage == STAGES) { stage = 0; phase ^= 1u; }
                 }
             }
         }
     } else if (warp == 1) {
         // ------------------------------------------------------------------ MMA issuer
-        if (lane == 0) {
+        {
+            const bool leader = elect_one();
             const uint32_t idesc = make_instr_desc(p.a_fmt, p.b_fmt, p.a_mn_major, p.b_mn_major, BM, BN);
             // K-major: 8-row groups are 1024 B apart, a K step of one MMA is 32 B inside the row.
             // MN-major: a K step of one MMA is (mma_k rows * 128 B); next 128 B chunk along M/N
@@ -152,24 +165,28 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
             int acc = 0; uint32_t acc_phase = 0;
             bool ok = true;
             for (int t = blockIdx.x; t < num_tiles && ok; t += gridDim.x) {
-                if (!mbar_wait(tempty_bar(acc), acc_phase ^ 1u, abort_flag)) { atomicOr(p.status, kErrTmemEmpty); ok = false; break; }
+                if (!mbar_wait_warp(tempty_bar(acc), acc_phase ^ 1u, abort_flag)) { if (leader) atomicOr(p.status, kErrTmemEmpty); ok = false; break; }
                 tc_fence_after_sync();
                 const uint32_t d_tmem = tmem_base + acc * BN;
                 const int k_begin = (t % splits) * k_per_split, k_end = min(k_iters, k_begin + k_per_split);
                 for (int k = k_begin; k < k_end; ++k) {
-                    if (!mbar_wait(full_bar(stage), phase, abort_flag)) { atomicOr(p.status, kErrFullWait); ok = false; break; }
+                    if (!mbar_wait_warp(full_bar(stage), phase, abort_flag)) { if (leader) atomicOr(p.status, kErrFullWait); ok = false; break; }
                     tc_fence_after_sync();
                     const uint32_t alo = a_lo0 + stage * (STAGE_BYTES >> 4);
                     const uint32_t blo = b_lo0 + stage * (STAGE_BYTES >> 4);
-                    mma_issue<Kind, false>(d_tmem, alo, a_hi, blo, b_hi, idesc, k > k_begin ? 1u : 0u);
-                    mma_issue<Kind, false>(d_tmem, alo + a_inc, a_hi, blo + b_inc, b_hi, idesc, 1u);
-                    mma_issue<Kind, false>(d_tmem, alo + 2 * a_inc, a_hi, blo + 2 * b_inc, b_hi, idesc, 1u);
-                    mma_issue<Kind, false>(d_tmem, alo + 3 * a_inc, a_hi, blo + 3 * b_inc, b_hi, idesc, 1u);
-                    mma_commit(empty_bar(stage));          // stage reusable once these MMAs have read it
+                    if (leader) {
+                        mma_issue<Kind, false>(d_tmem, alo, a_hi, blo, b_hi, idesc, k > k_begin ? 1u : 0u);
+                        mma_issue<Kind, false>(d_tmem, alo + a_inc, a_hi, blo + b_inc, b_hi, idesc, 1u);
+                        mma_issue<Kind, false>(d_tmem, alo + 2 * a_inc, a_hi, blo + 2 * b_inc, b_hi, idesc, 1u);
+                        mma_issue<Kind, false>(d_tmem, alo + 3 * a_inc, a_hi, blo + 3 * b_inc, b_hi, idesc, 1u);
+                        mma_commit(empty_bar(stage));          // stage reusable once these MMAs have read it
+                    }
+                    __syncwarp();
                     if (++stage == STAGES) { stage = 0; phase ^= 1u; }
                 }
                 if (!ok) break;
-                mma_commit(tfull_bar(acc));                // accumulator complete
+                if (leader) mma_commit(tfull_bar(acc));    // accumulator complete
+                __syncwarp();
                 if (++acc == 2) { acc = 0; acc_phase ^= 1u; }
             }
         }
@@ -316,6 +333,22 @@ int llmq_encode_tmap_2d(CUtensorMap* out, const void* base, int elem_bytes, long
     return r == CUDA_SUCCESS ? 0 : static_cast<int>(r);
 }
 
+// 3-D view of an MN-major operand [rows = K, cols = M or N], cols a multiple of the 128-byte chunk: (column inside the chunk,
+// K row, chunk).  The box is `chunks` chunks of [box_rows][128 bytes] one behind the other, the layout of that many 2-D boxes.
+static int encode_tmap_chunks(CUtensorMap* out, const void* base, int elem_bytes, long long rows, long long cols, long long ld, int box_rows, int chunks) {
+    EncodeTiledFn fn = get_encode_fn();
+    if (!fn) return -1;
+    const int chunk = 128 / elem_bytes;
+    cuuint64_t dims[3] = {static_cast<cuuint64_t>(chunk), static_cast<cuuint64_t>(rows), static_cast<cuuint64_t>(cols / chunk)};
+    cuuint64_t strides[2] = {static_cast<cuuint64_t>(ld) * elem_bytes, 128};
+    cuuint32_t box[3] = {static_cast<cuuint32_t>(chunk), static_cast<cuuint32_t>(box_rows), static_cast<cuuint32_t>(chunks)};
+    cuuint32_t estr[3] = {1, 1, 1};
+    CUresult r = fn(out, elem_bytes == 2 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, const_cast<void*>(base), dims, strides,
+                    box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                    CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    return r == CUDA_SUCCESS ? 0 : static_cast<int>(r);
+}
+
 int llmq_gemm_2cta_launch(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tc, const GemmParams& p, int num_sms, cudaStream_t stream);
 
 // Tile-shape selection: 0 = automatic, 1 = force the one-CTA kernel, 2 = force the CTA-pair kernel.
@@ -395,7 +428,7 @@ extern "C" int llmq_gemm_swiglu(const void* A, const void* B, void* C, void* aux
 }
 
 extern "C" unsigned int llmq_gemm_rs_arrivals(int M, int N, int world) {
-    return static_cast<unsigned int>(world) * static_cast<unsigned int>(M / world / 32) * static_cast<unsigned int>((N + BN - 1) / BN);
+    return static_cast<unsigned int>(world) * static_cast<unsigned int>(M / world / 32) * static_cast<unsigned int>((N + 255) / 256);
 }
 
 static int gemm_impl(const void* A, const void* B, void* C, const void* bias,
@@ -416,19 +449,35 @@ static int gemm_impl(const void* A, const void* B, void* C, const void* bias,
     CUtensorMap ta, tb;
     const int bk = 128 / eb;
     int rc;
-    if (!a_mn_major) rc = llmq_encode_tmap_2d(&ta, A, eb, M, K, lda, BM);
-    else             rc = llmq_encode_tmap_2d(&ta, A, eb, K, M, lda, bk);
-    if (rc) return rc;
     // The CTA-pair kernel stages 128 rows of B per CTA; the one-CTA kernel stages all 256.
     const bool pair_kernel = eb != 4 && (rs != nullptr || ready_flags != nullptr || g_gemm_mode == 2 ||
                                          (g_gemm_mode == 0 && M >= 256 && static_cast<long long>(M) * N >= 256LL * 256 * 32));
-    if (!b_mn_major) rc = llmq_encode_tmap_2d(&tb, B, eb, N, K, ldb, pair_kernel ? 128 : BN);
+    // An MN-major stage that is several 128-byte chunks wide (16-bit operands; the 256 rows of B of the one-CTA kernel) is fetched with
+    // one 3-D load instead of one 2-D load per chunk: the loads of a stage were issued one after the other for longer than its MMAs
+    // run.  bf16, CTA pairs, TFLOP/s with 2-D loads / 3-D loads / 3-D loads and a K loop per kind of load (gemm_tcgen05_2cta.cu), K-major
+    // 1540: 17920 x 1536 x 16384 both operands 968-1062 / 1327 / 1435-1523, 16384 x 3584 x 4096 both 1052 / 1328 / 1520, B only 1352 / 1520 /
+    // 1545, 4096^3 both 906 / 1184 / 1427.  With a ragged last chunk the 2-D boxes stay (its columns beyond the matrix would lie in the
+    // next row), and for one chunk a 3-D box gains nothing.
+    // One-CTA kernel: 128-column tiles where 256-column ones fill less than half of the SMs.  They run twice as many CTAs with more
+    // stages in flight, and where that fills the GPU no split-K pass follows: 1152 x 896 x 1001 (both operands MN-major) and
+    // 1001 x 896 x 1152, the QKV gradients of a short batch, took 15 us each in two K parts
+    // and 4 more for their sum; they take 13 in one.
+    const int tiles256 = ((M + BM - 1) / BM) * ((N + 255) / 256);
+    const int bn = (eb != 4 && 2 * tiles256 <= num_sms) ? 128 : 256;
+    const int b_rows = pair_kernel ? 128 : bn;
+    const bool a_box3 = a_mn_major && eb < 4 && BM > bk && M % bk == 0, b_box3 = b_mn_major && eb < 4 && b_rows > bk && N % bk == 0;
+    if (!a_mn_major) rc = llmq_encode_tmap_2d(&ta, A, eb, M, K, lda, BM);
+    else if (a_box3) rc = encode_tmap_chunks(&ta, A, eb, K, M, lda, bk, BM / bk);
+    else             rc = llmq_encode_tmap_2d(&ta, A, eb, K, M, lda, bk);
+    if (rc) return rc;
+    if (!b_mn_major) rc = llmq_encode_tmap_2d(&tb, B, eb, N, K, ldb, b_rows);
+    else if (b_box3) rc = encode_tmap_chunks(&tb, B, eb, K, N, ldb, bk, b_rows / bk);
     else             rc = llmq_encode_tmap_2d(&tb, B, eb, K, N, ldb, bk);
     if (rc) return rc;
 
     GemmParams p{};
     p.M = M; p.N = N; p.K = K; p.elem_bytes = eb;
-    p.a_mn_major = a_mn_major; p.b_mn_major = b_mn_major;
+    p.a_mn_major = a_mn_major; p.b_mn_major = b_mn_major; p.a_box3 = a_box3; p.b_box3 = b_box3;
     p.a_fmt = ab_dtype == 3 ? 2 : (ab_dtype == 0 ? 1 : (ab_dtype == 1 ? 0 : 1));
     p.b_fmt = b_dtype == 3 ? 2 : (b_dtype == 0 ? 1 : (b_dtype == 1 ? 0 : 1));
     p.C = C; p.ldc = ldc; p.c_dtype = c_dtype; p.accumulate = accumulate;
@@ -460,13 +509,16 @@ static int gemm_impl(const void* A, const void* B, void* C, const void* bias,
     int dev = 0;
     cudaGetDevice(&dev);
     if (!attr_set[dev & 63]) {
-        cudaError_t e = cudaFuncSetAttribute(gemm_tcgen05_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
-        if (e == cudaSuccess) e = cudaFuncSetAttribute(gemm_tcgen05_kernel<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
-        if (e == cudaSuccess) e = cudaFuncSetAttribute(gemm_tcgen05_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
+        const cudaFuncAttribute at = cudaFuncAttributeMaxDynamicSharedMemorySize;
+        cudaError_t e = cudaFuncSetAttribute(gemm_tcgen05_kernel<1, 256>, at, Tile<256>::SMEM_BYTES);
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(gemm_tcgen05_kernel<0, 256>, at, Tile<256>::SMEM_BYTES);
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(gemm_tcgen05_kernel<2, 256>, at, Tile<256>::SMEM_BYTES);
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(gemm_tcgen05_kernel<1, 128>, at, Tile<128>::SMEM_BYTES);
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(gemm_tcgen05_kernel<0, 128>, at, Tile<128>::SMEM_BYTES);
         if (e != cudaSuccess) return static_cast<int>(e);
         attr_set[dev & 63] = true;
     }
-    const int tiles = ((M + BM - 1) / BM) * ((N + BN - 1) / BN);
+    const int tiles = ((M + BM - 1) / BM) * ((N + bn - 1) / bn);
     const int k_iters = (K + bk - 1) / bk;
     int splits = 1;
     if (g_splitk_ws && tiles * 2 <= num_sms && k_iters >= 16) {
@@ -476,13 +528,20 @@ static int gemm_impl(const void* A, const void* B, void* C, const void* bias,
         while (splits > 1 && static_cast<long long>(splits) * M * N > g_splitk_floats) --splits;
         // every split must get at least one K step
         while (splits > 1 && (splits - 1) * ((k_iters + splits - 1) / splits) >= k_iters) --splits;
+        // the pass that adds the parts costs about as much as 32 K steps of a 128-column tile
+        if (bn == 128 && splits > 1 && k_iters - (k_iters + splits - 1) / splits < 32) splits = 1;
     }
     if (splits > 1) { p.k_splits = splits; p.partial = g_splitk_ws; }
     const int items = tiles * splits;
     int grid = items < num_sms ? items : num_sms;
-    if (eb == 1)      gemm_tcgen05_kernel<1><<<grid, NUM_THREADS, SMEM_BYTES, stream>>>(ta, tb, p);
-    else if (eb == 2) gemm_tcgen05_kernel<0><<<grid, NUM_THREADS, SMEM_BYTES, stream>>>(ta, tb, p);
-    else              gemm_tcgen05_kernel<2><<<grid, NUM_THREADS, SMEM_BYTES, stream>>>(ta, tb, p);
+    if (bn == 128) {
+        if (eb == 1) gemm_tcgen05_kernel<1, 128><<<grid, NUM_THREADS, Tile<128>::SMEM_BYTES, stream>>>(ta, tb, p);
+        else         gemm_tcgen05_kernel<0, 128><<<grid, NUM_THREADS, Tile<128>::SMEM_BYTES, stream>>>(ta, tb, p);
+    } else {
+        if (eb == 1)      gemm_tcgen05_kernel<1, 256><<<grid, NUM_THREADS, Tile<256>::SMEM_BYTES, stream>>>(ta, tb, p);
+        else if (eb == 2) gemm_tcgen05_kernel<0, 256><<<grid, NUM_THREADS, Tile<256>::SMEM_BYTES, stream>>>(ta, tb, p);
+        else              gemm_tcgen05_kernel<2, 256><<<grid, NUM_THREADS, Tile<256>::SMEM_BYTES, stream>>>(ta, tb, p);
+    }
     if (splits > 1) {
         const long long total = static_cast<long long>(M) * N;
         const int out_bytes = c_dtype == 0 ? 8 : 16;                       // four columns

@@ -18,6 +18,7 @@
 // Each epilogue warp bumps the owner's arrival counter per tile (release, system scope).  After its last tile a
 // CTA waits (bounded) for the local counter to show all sources, then the epilogue warps of all CTAs sum the
 // `world` slots of this rank's rows, scale, add into the shard with stochastic rounding and collect the norm.
+#include <type_traits>
 #include "ptx_sm100.cuh"
 #include "api.h"
 #include "common.cuh"
@@ -110,6 +111,7 @@ gemm_tcgen05_2cta_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gri
             tma_prefetch_desc(&tmap_b);
             int stage = 0; uint32_t phase = 0;
             const int mn_chunk = ROW_BYTES / p.elem_bytes;
+            const uint32_t fb0 = map_to_cta(full_bar(0), 0);           // the leader CTA's barriers
             bool ok = true;
             // Fused all-gather: B rows pushed by peer GPUs are consumed as soon as their source's flag shows the
             // current generation.  `seen` caches the sources already confirmed.
@@ -130,32 +132,47 @@ gemm_tcgen05_2cta_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gri
                     const int last = min(brow0 + BN_HALF, p.N) - 1;
                     for (int src = brow0 / p.ready_rows_per_src; src <= last / p.ready_rows_per_src && ok; ++src) ensure_src(src);
                 }
-                for (int k = 0; k < k_iters && ok; ++k) {
-                    if (p.ready_flags && p.b_mn_major) {
-                        const int last = min(k * bk + bk, p.K) - 1;
-                        for (int src = (k * bk) / p.ready_rows_per_src; src <= last / p.ready_rows_per_src && ok; ++src) ensure_src(src);
-                        if (!ok) break;
+                // The K loop, specialised on how the operands are loaded (0 K-major, 1 one 3-D box, 2 a 2-D box per 128-byte chunk): the one
+                // lane that issues a stage's loads has the time of the stage's MMAs for them and for everything it decides in between.
+                auto k_loop = [&](auto a_load, auto b_load) {
+                    for (int k = 0; k < k_iters; ++k) {
+                        if (b_load != 0 && p.ready_flags) {
+                            const int last = min(k * bk + bk, p.K) - 1;
+                            for (int src = (k * bk) / p.ready_rows_per_src; src <= last / p.ready_rows_per_src && ok; ++src) ensure_src(src);
+                            if (!ok) return;
+                        }
+                        if (!mbar_wait(empty_bar(stage), phase ^ 1u, abort_flag)) { atomicOr(p.status, kErrEmptyWait); ok = false; return; }
+                        const uint32_t sa = smem_base + stage * STAGE_BYTES;
+                        const uint32_t sb = sa + A_STAGE_BYTES;
+                        const uint32_t fb = fb0 + 8u * stage;                                // the leader's barrier
+                        if (rank == 0) mbar_expect_tx(full_bar(stage), 2 * STAGE_BYTES);     // bytes of both CTAs
+                        if constexpr (a_load == 0)      tma_load_2d_pair(sa, &tmap_a, fb, k * bk, row0);
+                        else if constexpr (a_load == 1) tma_load_3d_pair(sa, &tmap_a, fb, 0, k * bk, row0 / mn_chunk);
+                        else {
+                            const int nbox = BM * p.elem_bytes / ROW_BYTES;
+                            for (int b = 0; b < nbox; ++b)
+                                tma_load_2d_pair(sa + b * (A_STAGE_BYTES / nbox), &tmap_a, fb, row0 + b * mn_chunk, k * bk);
+                        }
+                        if constexpr (b_load == 0)      tma_load_2d_pair(sb, &tmap_b, fb, k * bk, brow0);
+                        else if constexpr (b_load == 1) tma_load_3d_pair(sb, &tmap_b, fb, 0, k * bk, brow0 / mn_chunk);
+                        else {
+                            const int nbox = BN_HALF * p.elem_bytes / ROW_BYTES;
+                            for (int b = 0; b < nbox; ++b)
+                                tma_load_2d_pair(sb + b * (B_STAGE_BYTES / nbox), &tmap_b, fb, brow0 + b * mn_chunk, k * bk);
+                        }
+                        if (++stage == STAGES) { stage = 0; phase ^= 1u; }
                     }
-                    if (!mbar_wait(empty_bar(stage), phase ^ 1u, abort_flag)) { atomicOr(p.status, kErrEmptyWait); ok = false; break; }
-                    const uint32_t sa = smem_base + stage * STAGE_BYTES;
-                    const uint32_t sb = sa + A_STAGE_BYTES;
-                    const uint32_t fb = map_to_cta(full_bar(stage), 0);                 // the leader's barrier
-                    if (rank == 0) mbar_expect_tx(full_bar(stage), 2 * STAGE_BYTES);     // bytes of both CTAs
-                    if (!p.a_mn_major) {
-                        tma_load_2d_pair(sa, &tmap_a, fb, k * bk, row0);
-                    } else {
-                        int nbox = BM * p.elem_bytes / ROW_BYTES;
-                        for (int b = 0; b < nbox; ++b)
-                            tma_load_2d_pair(sa + b * (A_STAGE_BYTES / nbox), &tmap_a, fb, row0 + b * mn_chunk, k * bk);
-                    }
-                    if (!p.b_mn_major) {
-                        tma_load_2d_pair(sb, &tmap_b, fb, k * bk, brow0);
-                    } else {
-                        int nbox = BN_HALF * p.elem_bytes / ROW_BYTES;
-                        for (int b = 0; b < nbox; ++b)
-                            tma_load_2d_pair(sb + b * (B_STAGE_BYTES / nbox), &tmap_b, fb, brow0 + b * mn_chunk, k * bk);
-                    }
-                    if (++stage == STAGES) { stage = 0; phase ^= 1u; }
+                };
+                const std::integral_constant<int, 0> kmajor{};
+                const std::integral_constant<int, 1> box3{};
+                const std::integral_constant<int, 2> boxes{};
+                if (!ok) break;
+                if (!p.a_mn_major) {
+                    if (!p.b_mn_major) k_loop(kmajor, kmajor); else if (p.b_box3) k_loop(kmajor, box3); else k_loop(kmajor, boxes);
+                } else if (p.a_box3) {
+                    if (!p.b_mn_major) k_loop(box3, kmajor); else if (p.b_box3) k_loop(box3, box3); else k_loop(box3, boxes);
+                } else {
+                    if (!p.b_mn_major) k_loop(boxes, kmajor); else if (p.b_box3) k_loop(boxes, box3); else k_loop(boxes, boxes);
                 }
             }
         }

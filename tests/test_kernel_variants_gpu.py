@@ -176,3 +176,19 @@ def test_gemm_mn_major_chunks(M, N, Kd, dt, a_mn, b_mn):
     out = torch.full((M, N), 5.0, dtype=torch.float32, device=DEV)
     K.gemm(out, sa.to(DEV), sb.to(DEV), a_mn=bool(a_mn), b_mn=bool(b_mn))
     assert rel(out, a.double() @ b.double().t()) < 1e-5    # exact products, fp32 sums
+
+
+# 128-column tiles (few output tiles), with and without a split of K, up to the first shape with 256-column tiles (75 of them)
+@pytest.mark.parametrize("M,N,Kd", [(1, 8, 16), (129, 136, 320), (1001, 896, 1152), (896, 896, 4096), (1000, 2304, 208), (1152, 2048, 96), (9600, 256, 64),
+                                    (9472, 256, 64)])
+@pytest.mark.parametrize("dt", [BF, torch.float8_e4m3fn])
+@pytest.mark.parametrize("accumulate", [False, True])
+def test_gemm_tile_widths(M, N, Kd, dt, accumulate):
+    g = torch.Generator().manual_seed(M + N + Kd)
+    a, b = torch.randn(M, Kd, generator=g).to(dt), torch.randn(N, Kd, generator=g).to(dt)
+    bias, prev = torch.randn(N, generator=g).to(BF), torch.randn(M, N, generator=g)
+    out, am = prev.to(DEV), torch.zeros(1, device=DEV)
+    K.gemm(out, a.to(DEV), b.to(DEV), bias=bias.to(DEV), accumulate=accumulate, absmax=am)
+    want = a.double() @ b.double().t() + bias.double() + (prev.double() if accumulate else 0)
+    assert rel(out, want) < 1e-5                           # exact products, fp32 sums
+    assert abs(am.item() - want.abs().max().item()) < 1e-4 * want.abs().max().item()
