@@ -1,4 +1,4 @@
-// Causal grouped-query flash attention forward for head size 128: two query tiles per CTA, processed alternately.
+// Causal grouped-query flash attention forward (head sizes 64 and 128): two query tiles per CTA, processed alternately.
 //
 // A CTA owns 256 consecutive queries of one (batch, query head) as two 128-row tiles A and B.  Each tile has its own
 // softmax warpgroup (thread r owns row r = TMEM lane r and sees the whole 128-key score row, so the row maximum and the
@@ -6,13 +6,14 @@
 //
 //     columns   0..127  S_A   (fp32 scores of the current key tile; the bf16 probabilities P_A overwrite columns 0..63)
 //     columns 128..255  S_B
-//     columns 256..383  O_A   (fp32 output accumulator)
-//     columns 384..511  O_B
+//     columns 256 ..    O_A   (fp32 output accumulator, head size columns)
+//     then              O_B
 //
 // Per 128-key tile j and query tile X the chain is  S_X = Q_X K_j^T  ->  softmax warpgroup X: max, exp2, bf16, P_X into
 // tensor memory (handed over in two halves of 64 keys)  ->  O_X += P_X V_j (P is the A operand straight from tensor memory).  The two chains are independent,
-// so while one tile's warpgroup computes exponentials the tensor core runs the other tile's MMAs; the single-tile
-// kernel (attention_tcgen05.cu, still used for head size 64) left the tensor pipe idle during that time.
+// so while one tile's warpgroup computes exponentials the tensor core runs the other tile's MMAs.  Measured: 8 x 2048 tokens,
+// 28 / 4 heads of 128, 278 us (304 us with the MMAs issued by a lane on its own, see elect_one); 8 x 1024 tokens, 14 / 2 heads of 64,
+// 43 us (100 us for one query tile per CTA walking all heads of a group, which left the tensor pipe idle during the exponentials).
 // K and V tiles stream through two shared-memory stages each (TMA, 128-byte swizzle); Q_A and Q_B stay in shared memory
 // for the whole walk.  O is rescaled only when a row maximum moved by more than 2^8 since the last rescale (the stale
 // maximum keeps P <= 256, which is exact after the final normalisation), and then by the row's own thread.
@@ -27,11 +28,9 @@ using namespace sm100;
 
 namespace {
 
-constexpr int HS = 128;
 constexpr int BQ = 128;                      // rows per query tile
 constexpr int BKV = 128;                     // keys per tile
-constexpr int TILE_BYTES = 128 * HS * 2;     // 32 KiB: Q, K and V tiles alike (two 64-column chunks of 128 rows x 128 bytes)
-constexpr int CHUNK_BYTES = 128 * 128;
+constexpr int CHUNK_BYTES = 128 * 128;       // 128 rows x 64 columns of a Q, K or V tile; a tile has HS / 64 of them
 constexpr int KV_STAGES = 2;
 constexpr int NUM_THREADS = 352;             // 4 + 4 softmax warps, TMA producer, MMA issuer A, MMA issuer B
 constexpr uint32_t TMEM_COLS = 512;
@@ -62,8 +61,6 @@ __device__ __forceinline__ void warp_arrive(uint32_t bar) {
     if ((threadIdx.x & 31) == 0) mbar_arrive(bar);
 }
 
-#define DLO(base, lbo, off) (desc_lo((base), (lbo)) + static_cast<uint32_t>((off) >> 4))
-
 // One work item = 256 consecutive queries of one (batch, query head).  Items are numbered with the longest key walks first
 // (query block descending); a CTA walks the items  c, 2G-1-c, 2G+c, 4G-1-c, ...  (G = grid size): in every round of G items the
 // order of the CTAs flips, which evens out the total walk length per CTA.
@@ -92,9 +89,11 @@ __device__ __forceinline__ Item decode_item(int item, const FwdParams& p, int nq
 // an issuer starts the next item's first score tile while the softmax warpgroup still normalises and stores the current
 // item's rows (it only has to wait for that before the first P V product overwrites O); tile A moves on to the next item
 // while tile B walks its extra key tile.  All barrier phases are counted over the whole kernel.
+template <int HS>
 __global__ void __launch_bounds__(NUM_THREADS, 1)
 attn_fwd_pingpong_kernel(const __grid_constant__ CUtensorMap tmap_qkv,     // qkv as (B, T, W), box 128 rows x 64 columns
                          const FwdParams p) {
+    constexpr int NCH = HS / 64, TILE_BYTES = NCH * CHUNK_BYTES;
     extern __shared__ __align__(1024) uint8_t smem[];
     uint8_t* sQ = smem;                                   // [2 tiles][TILE_BYTES]
     uint8_t* sK = sQ + 2 * TILE_BYTES;                    // [KV_STAGES][TILE_BYTES]
@@ -103,7 +102,7 @@ attn_fwd_pingpong_kernel(const __grid_constant__ CUtensorMap tmap_qkv,     // qk
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 24);
     volatile uint32_t* abort_flag = tmem_slot + 1;
 
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;       // warp: uniform, and known to be
     if (smem_u32(smem) & 1023u) { if (tid == 0) atomicOr(p.status, kErrOther); return; }
 
     const int nqb = (p.T + 2 * BQ - 1) / (2 * BQ);
@@ -162,18 +161,18 @@ attn_fwd_pingpong_kernel(const __grid_constant__ CUtensorMap tmap_qkv,     // qk
                 if (it > 0 && !mbar_wait(q_empty, (it - 1) & 1, abort_flag)) { ok = false; break; }
                 mbar_expect_tx(q_full, active * TILE_BYTES);
                 for (int x = 0; x < active; ++x)
-                    for (int c = 0; c < 2; ++c)
+                    for (int c = 0; c < NCH; ++c)
                         tma_load_3d(smem_u32(sQ) + x * TILE_BYTES + c * CHUNK_BYTES, &tmap_qkv, q_full, qcol + c * 64, w.q0 + x * BQ, w.b);
                 for (int j = 0; j < w.n_max; ++j, ++kv) {
                     const int st = kv % KV_STAGES;
                     const uint32_t par = ((kv / KV_STAGES) - 1) & 1;
                     if (kv >= KV_STAGES && !mbar_wait(k_empty(st), par, abort_flag)) { ok = false; break; }
                     mbar_expect_tx(k_full(st), TILE_BYTES);
-                    for (int c = 0; c < 2; ++c)
+                    for (int c = 0; c < NCH; ++c)
                         tma_load_3d(smem_u32(sK) + st * TILE_BYTES + c * CHUNK_BYTES, &tmap_qkv, k_full(st), kcol + c * 64, j * BKV, w.b);
                     if (kv >= KV_STAGES && !mbar_wait(v_empty(st), par, abort_flag)) { ok = false; break; }
                     mbar_expect_tx(v_full(st), TILE_BYTES);
-                    for (int c = 0; c < 2; ++c)
+                    for (int c = 0; c < NCH; ++c)
                         tma_load_3d(smem_u32(sV) + st * TILE_BYTES + c * CHUNK_BYTES, &tmap_qkv, v_full(st), vcol + c * 64, j * BKV, w.b);
                 }
             }
@@ -182,12 +181,13 @@ attn_fwd_pingpong_kernel(const __grid_constant__ CUtensorMap tmap_qkv,     // qk
     } else if (warp >= 9) {
         // ============================================================ MMA issuer of query tile x
         const int x = warp - 9;
-        if (lane == 0) {
+        {
+            const bool leader = elect_one();
             const uint32_t idesc_s = make_instr_desc(1, 1, false, false, BQ, BKV);       // S = Q K^T
             const uint32_t idesc_o = make_instr_desc(1, 1, false, true, BQ, HS);         // O += P V  (V read as MN-major B)
             const uint32_t hi = desc_hi(1024);
             const uint32_t tS = tmem + x * BKV, tO = tmem + 2 * BKV + x * HS;
-            const uint32_t q_base = smem_u32(sQ) + x * TILE_BYTES;
+            const uint32_t q_lo = desc_lo(smem_u32(sQ) + x * TILE_BYTES, 16);
             uint32_t kv = 0, tiles = 0, walks = 0;           // stage uses, key tiles of this query tile, items in which it had any
             bool ok = true;
             for (int it = 0; ok; ++it) {
@@ -195,38 +195,45 @@ attn_fwd_pingpong_kernel(const __grid_constant__ CUtensorMap tmap_qkv,     // qk
                 if (item >= total) break;
                 const Item w = decode_item(item, p, nqb, nt);
                 const int n = x == 0 ? w.nA : w.nB;
-                if (!mbar_wait(q_full, it & 1, abort_flag)) { ok = false; break; }
-                if (n == 0) mbar_arrive(q_empty);             // this tile does not exist in the item: its Q buffer was not loaded
+                if (!mbar_wait_warp(q_full, it & 1, abort_flag)) { ok = false; break; }
+                if (n == 0 && leader) mbar_arrive(q_empty);             // this tile does not exist in the item: its Q buffer was not loaded
                 for (int j = 0; j < n && ok; ++j, ++kv, ++tiles) {
                     const int st = kv % KV_STAGES;
                     const uint32_t par = (kv / KV_STAGES) & 1;
-                    if (!mbar_wait(k_full(st), par, abort_flag)) { ok = false; break; }
+                    if (!mbar_wait_warp(k_full(st), par, abort_flag)) { ok = false; break; }
                     tc_fence_after_sync();
-                    const uint32_t k_base = smem_u32(sK) + st * TILE_BYTES;
+                    const uint32_t k_lo = desc_lo(smem_u32(sK) + st * TILE_BYTES, 16), ke = k_empty(st);
+                    const bool last = j == n - 1;
+                    if (leader) {
 #pragma unroll
-                    for (int k = 0; k < HS / 16; ++k)
-                        mma_issue<0, false>(tS, DLO(q_base, 16, (k / 4) * CHUNK_BYTES + (k % 4) * 32), hi,
-                                            DLO(k_base, 16, (k / 4) * CHUNK_BYTES + (k % 4) * 32), hi, idesc_s, k > 0);
-                    mma_commit(s_full(x));
-                    mma_commit(k_empty(st));
-                    if (j == n - 1) mma_commit(q_empty);      // the item's last read of this Q tile
-                    if (!mbar_wait(v_full(st), par, abort_flag)) { ok = false; break; }
+                        for (int k = 0; k < HS / 16; ++k)
+                            mma_issue<0, false>(tS, q_lo + (((k / 4) * CHUNK_BYTES + (k % 4) * 32) >> 4), hi,
+                                                k_lo + (((k / 4) * CHUNK_BYTES + (k % 4) * 32) >> 4), hi, idesc_s, k > 0);
+                        mma_commit(s_full(x));
+                        mma_commit(ke);
+                        if (last) mma_commit(q_empty);        // the item's last read of this Q tile
+                    }
+                    __syncwarp();
+                    if (!mbar_wait_warp(v_full(st), par, abort_flag)) { ok = false; break; }
                     // the first product of an item overwrites O: the warpgroup must have stored the previous item's rows
-                    if (j == 0 && walks > 0 && !mbar_wait(o_free(x), (walks - 1) & 1, abort_flag)) { ok = false; break; }
-                    const uint32_t v_base = smem_u32(sV) + st * TILE_BYTES;
+                    if (j == 0 && walks > 0 && !mbar_wait_warp(o_free(x), (walks - 1) & 1, abort_flag)) { ok = false; break; }
+                    const uint32_t v_lo = desc_lo(smem_u32(sV) + st * TILE_BYTES, CHUNK_BYTES), ve = v_empty(st);
+                    const uint32_t acc0 = j > 0;
                     // P arrives in two halves of 64 keys (a barrier each): the first half's MMAs run while the warpgroup still
                     // exponentiates the second half
 #pragma unroll
                     for (int half = 0; half < 2; ++half) {
-                        if (!mbar_wait(half == 0 ? p_ready(x) : p_ready2(x), tiles & 1, abort_flag)) { ok = false; break; }
+                        if (!mbar_wait_warp(half == 0 ? p_ready(x) : p_ready2(x), tiles & 1, abort_flag)) { ok = false; break; }
                         tc_fence_after_sync();
+                        if (leader) {
 #pragma unroll
-                        for (int k = half * 4; k < half * 4 + 4; ++k)
-                            mma_issue_f16_tmem_a(tO, tS + k * 8, DLO(v_base, CHUNK_BYTES, k * (16 * 128)), hi, idesc_o, (j > 0 || k > 0));
+                            for (int k = half * 4; k < half * 4 + 4; ++k)
+                                mma_issue_f16_tmem_a(tO, tS + k * 8, v_lo + ((k * (16 * 128)) >> 4), hi, idesc_o, k > 0 ? 1u : acc0);
+                            if (half == 1) { mma_commit(o_done(x)); mma_commit(ve); }
+                        }
+                        __syncwarp();
                     }
                     if (!ok) break;
-                    mma_commit(o_done(x));
-                    mma_commit(v_empty(st));
                 }
                 // the other tile may walk further: its stages still need this tile's arrival (wait for the stage's load first:
                 // it is only issued once the stage's previous use was released by both tiles, so this arrival cannot be counted
@@ -234,14 +241,15 @@ attn_fwd_pingpong_kernel(const __grid_constant__ CUtensorMap tmap_qkv,     // qk
                 for (int j = n; j < w.n_max && ok; ++j, ++kv) {
                     const int st = kv % KV_STAGES;
                     const uint32_t par = (kv / KV_STAGES) & 1;
-                    if (!mbar_wait(k_full(st), par, abort_flag)) { ok = false; break; }
-                    mbar_arrive(k_empty(st));
-                    if (!mbar_wait(v_full(st), par, abort_flag)) { ok = false; break; }
-                    mbar_arrive(v_empty(st));
+                    if (!mbar_wait_warp(k_full(st), par, abort_flag)) { ok = false; break; }
+                    if (leader) mbar_arrive(k_empty(st));
+                    if (!mbar_wait_warp(v_full(st), par, abort_flag)) { ok = false; break; }
+                    if (leader) mbar_arrive(v_empty(st));
                 }
                 if (n > 0) ++walks;
             }
-            if (!ok) { *abort_flag = 1u; atomicOr(p.status, kErrOther); }
+            if (!ok && leader) { *abort_flag = 1u; atomicOr(p.status, kErrOther); }
+            __syncwarp();
         }
     } else {
         // ============================================================ softmax warpgroup of query tile x
@@ -281,24 +289,27 @@ attn_fwd_pingpong_kernel(const __grid_constant__ CUtensorMap tmap_qkv,     // qk
 #pragma unroll
                     for (int i = 0; i < 128; ++i) if (i > lim) rs[i] = __float_as_uint(-INFINITY);
                 }
-                float mx0 = -INFINITY, mx1 = -INFINITY, mx2 = -INFINITY, mx3 = -INFINITY;
+                float mx0 = -INFINITY, mx1 = -INFINITY, mx2 = -INFINITY, mx3 = -INFINITY;      // 0, 1: first 64 keys, 2, 3: the others
 #pragma unroll
-                for (int i = 0; i < 128; i += 4) {
-                    mx0 = fmaxf(mx0, __uint_as_float(rs[i]));     mx1 = fmaxf(mx1, __uint_as_float(rs[i + 1]));
-                    mx2 = fmaxf(mx2, __uint_as_float(rs[i + 2])); mx3 = fmaxf(mx3, __uint_as_float(rs[i + 3]));
+                for (int i = 0; i < 64; i += 2) {
+                    mx0 = fmaxf(mx0, __uint_as_float(rs[i]));      mx1 = fmaxf(mx1, __uint_as_float(rs[i + 1]));
+                    mx2 = fmaxf(mx2, __uint_as_float(rs[64 + i])); mx3 = fmaxf(mx3, __uint_as_float(rs[64 + i + 1]));
                 }
-                const float mx = fmaxf(fmaxf(mx0, mx1), fmaxf(mx2, mx3));
+                const float mx_first = fmaxf(mx0, mx1), mx = fmaxf(mx_first, fmaxf(mx2, mx3));
+                // The reference of the exponentials starts as the maximum of the first key tile; with head size 64 as that of its first
+                // 64 keys (which gives the bits of a walk in 64-key tiles) unless the others exceed it by the threshold.
+                const bool early = HS == 64 && j == 0 && (mx - mx_first) * sl2 <= kRescaleThreshold;
                 // ---- lazy rescale of O (warp-collective tensor-memory accesses: the warp decides together)
                 const bool need = j == 0 || (mx - m_ref) * sl2 > kRescaleThreshold;
                 if (__any_sync(0xffffffffu, need)) {
-                    const float m_new = need ? fmaxf(m_ref, mx) : m_ref;
+                    const float m_new = need ? (early ? mx_first : fmaxf(m_ref, mx)) : m_ref;
                     if (j > 0) {
                         const float alpha = need ? ex2((m_ref - m_new) * sl2) : 1.f;
                         l_sum *= alpha;
                         if (!mbar_wait(o_done(x), (tiles - 1) & 1, abort_flag)) { ok = false; break; }      // PV of tile j-1 has landed
                         tc_fence_after_sync();
 #pragma unroll 1
-                        for (int ch = 0; ch < 4; ++ch) {
+                        for (int ch = 0; ch < HS / 32; ++ch) {
                             uint32_t ro[32];
                             tmem_ld_32x32b_x32(tO + ch * 32, ro);
                             tmem_ld_wait();
@@ -349,11 +360,11 @@ attn_fwd_pingpong_kernel(const __grid_constant__ CUtensorMap tmap_qkv,     // qk
                 const float inv = 1.f / l_sum;
                 __nv_bfloat16* o = p.out + ((static_cast<long long>(b) * p.T + (row_ok ? row : 0)) * p.Hq + h) * HS;
 #pragma unroll 1
-                for (int ch = 0; ch < 4; ++ch) {
+                for (int ch = 0; ch < HS / 32; ++ch) {
                     uint32_t ro[32];
                     tmem_ld_32x32b_x32(tO + ch * 32, ro);
                     tmem_ld_wait();
-                    if (ch == 3) {                                  // the last of O is in registers
+                    if (ch == HS / 32 - 1) {                        // the last of O is in registers
                         tc_fence_before_sync();
                         warp_arrive(o_free(x));
                     }
@@ -391,11 +402,8 @@ typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t,
                                   const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
                                   CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
 
-}  // namespace
-
-// Head size 128 only; same contract as llmq_attention_forward (which dispatches here).
-int llmq_attention_forward_pingpong(void* out, float* lse, const void* qkv, int B, int T, int Hq, int Hkv, float* absmax,
-                                    unsigned int* status, cudaStream_t s) {
+template <int HS>
+int launch(void* out, float* lse, const void* qkv, int B, int T, int Hq, int Hkv, float* absmax, unsigned int* status, cudaStream_t s) {
     static EncodeTiledFn encode = nullptr;
     if (!encode) {
         void* ptr = nullptr;
@@ -413,12 +421,12 @@ int llmq_attention_forward_pingpong(void* out, float* lse, const void* qkv, int 
                         CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                         CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS) return 1000 + static_cast<int>(r);
-    constexpr int smem = (2 + 2 * KV_STAGES) * TILE_BYTES + 256;
+    constexpr int smem = (2 + 2 * KV_STAGES) * (HS / 64) * CHUNK_BYTES + 256;
     static bool attr_done[64] = {};
     int dev = 0;
     cudaGetDevice(&dev);
     if (!attr_done[dev & 63]) {
-        cudaError_t e = cudaFuncSetAttribute(attn_fwd_pingpong_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+        cudaError_t e = cudaFuncSetAttribute(attn_fwd_pingpong_kernel<HS>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
         if (e != cudaSuccess) return 2000 + static_cast<int>(e);
         attr_done[dev & 63] = true;
     }
@@ -435,7 +443,15 @@ int llmq_attention_forward_pingpong(void* out, float* lse, const void* qkv, int 
         sms[dev & 63] = n;
     }
     const long long total = static_cast<long long>(nqb) * Hq * B;
-    const int grid = static_cast<int>(total < sms[dev & 63] ? total : sms[dev & 63]);       // one CTA per SM (shared memory, tensor memory)
-    attn_fwd_pingpong_kernel<<<grid, NUM_THREADS, smem, s>>>(tmap, p);
+    const int grid = static_cast<int>(total < sms[dev & 63] ? total : sms[dev & 63]);       // one CTA per SM (tensor memory)
+    attn_fwd_pingpong_kernel<HS><<<grid, NUM_THREADS, smem, s>>>(tmap, p);
     return LLMQ_LAUNCH_CHECK();
+}
+
+}  // namespace
+
+// Same contract as llmq_attention_forward (which dispatches here); head size 64 or 128.
+int llmq_attention_forward_pingpong(void* out, float* lse, const void* qkv, int B, int T, int Hq, int Hkv, int HS, float* absmax,
+                                    unsigned int* status, cudaStream_t s) {
+    return HS == 64 ? launch<64>(out, lse, qkv, B, T, Hq, Hkv, absmax, status, s) : launch<128>(out, lse, qkv, B, T, Hq, Hkv, absmax, status, s);
 }

@@ -5,23 +5,28 @@
 // packed gradient dqkv with the same layout.  It takes the place of the cuDNN SDPA graphs and the
 // scalar fallback kernel of the reference (src/kernels/cudnn_att.cpp:46-263, src/kernels/attention.cu).
 //
-// All three main kernels share one organisation.  A CTA owns a 128-row tile (queries for forward and dQ, keys for
-// dK / dV) and has 19 warps: 16 compute warps (four warpgroups; thread (wg, r) owns row r = TMEM lane r and a quarter
-// of the columns of every score tile), one warp whose lane 0 issues the score MMAs, one whose lane 0 issues the TMA
-// loads and one whose lane 0 issues the accumulation MMAs.  MMA issue is synchronous with execution, so two issuing
-// threads are needed to keep the tensor pipe busy while the other one waits for the compute warps.  Everything is
-// handed over through mbarriers (one arrival per warp); score tiles are double buffered in tensor memory, the
-// streamed operand (K / V, or Q / dO for dK / dV) sits in a ring of four shared-memory buffers.  Operands that are
-// constant during a walk live in tensor memory as A operands where the 512 columns allow it (Q in forward, Q and dO
-// in dQ; the bf16 probabilities of the forward pass too), so they are not re-read from shared memory by every MMA.
-// The shared-memory tile of V / K / Q / dO doubles as an MN-major B operand, so no transposed copy is ever made.
+// The forward kernel is in attention_fwd_pingpong.cu.  The two gradient kernels share one organisation.  A CTA owns a 128-row tile
+// (keys for dK / dV, queries for dQ) and has 18 warps: 16 compute warps (four warpgroups; thread (wg, r) owns row r = TMEM lane r
+// and a quarter of the columns of every score tile), one warp that issues all MMAs and one that issues the TMA loads.  Everything is
+// handed over through mbarriers (one arrival per warp); score tiles are double buffered in tensor memory, the streamed operand
+// (Q / dO for dK / dV, K / V for dQ) sits in a ring of four shared-memory buffers.  P^T, dS^T and dS never leave tensor memory: the
+// bf16 values take the place of the scores they were computed from and are the A operands of the accumulating MMAs, which saves the
+// shared-memory writes, the proxy fence and the A reads of a staged tile, and the wait for the MMAs that read the previous one.  Q and
+// dO of the dQ kernel are A operands in tensor memory too.  The shared-memory tile of V / K / Q / dO doubles as an MN-major B operand,
+// so no transposed copy is ever made.
 //
 // Backward is split into two deterministic kernels (no atomics):
-//   * dK/dV: one CTA per (batch, kv head, 128 keys) walks over all query heads of the group and all
-//     query blocks at or below the diagonal; dK and dV accumulate in TMEM across the whole walk.
-//   * dQ   : one CTA per (batch, kv head, 128 queries) walks over the query heads of the group and their key
-//     blocks; dQ accumulates in TMEM and is drained once per head.
+//   * dK/dV: one CTA per (batch, kv head, 128 keys) walks over the query heads of the group and all query blocks at or below the
+//     diagonal; dK and dV accumulate in TMEM across the whole walk.  With few such items up to four CTAs of a cluster share the
+//     heads and add their sums through distributed shared memory in a fixed order.
+//   * dQ   : one CTA per (batch, kv head, 128 queries) and part of the group walks over its query heads and their key blocks; dQ
+//     accumulates in TMEM and is drained once per head.
 // A small pre-pass computes delta = rowsum(dO * O).  Blocks with the longest walks are scheduled first.
+//
+// Bound by the issue of the N = 64 MMAs (about 60 cycles each, 48 executing) and the waits between them: 1650 cycles per 64-row
+// tile of dK / dV where the MMAs alone take 1280, 1250 of dQ where they take 770.  8 x 2048 tokens, 28 / 4 heads of 128: dK / dV 543 ->
+// 431 us, dQ 515 -> 400 us; most of it from the warp-uniform issue (elect_one), which tensor-memory operands and one issuing warp
+// (MMAs execute in issue order, so the buffers need no barrier between them) made the remaining limit.
 #include <cstdlib>
 #include "ptx_sm100.cuh"
 #include "api.h"
@@ -37,20 +42,14 @@ constexpr float kLog2e = 1.4426950408889634f;
 constexpr int kBwdWarpgroups = 4;
 constexpr int kBwdComputeThreads = 128 * kBwdWarpgroups;
 constexpr int kBwdComputeWarps = kBwdComputeThreads / 32;
-// + three single-lane helper warps: score-MMA issuer, TMA producer, accumulation-MMA issuer.  MMA issue is synchronous
-// with execution (the queue is shallow), so two issuing threads keep the tensor pipe fed while the other one waits.
-constexpr int kBwdThreads = kBwdComputeThreads + 96;
-// barrier 1: the compute threads among themselves (barrier 0 is __syncthreads of the whole CTA)
+// + two helper warps: MMA issuer and TMA producer
+constexpr int kBwdThreads = kBwdComputeThreads + 64;
 // One arrival per warp (512 single arrivals on one shared-memory word would serialise): the lanes' earlier
 // writes and fences are ordered before lane 0's releasing arrive by the warp barrier.
 __device__ __forceinline__ void warp_arrive(uint32_t bar) {
     __syncwarp();
     if ((threadIdx.x & 31) == 0) mbar_arrive(bar);
 }
-// barriers 2-5: the four warps (one per warpgroup) that share 32 rows of the tile
-__device__ __forceinline__ void row_group_barrier(int group) { asm volatile("bar.sync %0, 128;" ::"r"(2 + group) : "memory"); }
-__device__ __forceinline__ void compute_barrier() { asm volatile("bar.sync 1, %0;" ::"n"(kBwdComputeThreads) : "memory"); }
-
 // 2^x with the hardware approximation (-inf -> 0)
 __device__ __forceinline__ float fast_exp2(float x) {
     float r;
@@ -58,8 +57,6 @@ __device__ __forceinline__ float fast_exp2(float x) {
     return r;
 }
 
-// low descriptor half of (base + byte offset); the base part is loop invariant, the offset a constant after unrolling
-#define DLO(base, lbo, off) (desc_lo((base), (lbo)) + static_cast<uint32_t>((off) >> 4))
 #define kDescHi desc_hi(1024)
 
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
@@ -139,16 +136,6 @@ attn_delta_kernel(float* __restrict__ delta, const bf16* __restrict__ o, const b
 // P^T and dS^T, the tensor core already computes S(it+1) / dP(it+1) (score tiles are double buffered in TMEM) and
 // finishes dV / dK of tile it-1.  Q / dO tiles sit in a ring of four shared-memory buffers, loaded three tiles
 // ahead; P^T / dS^T are kept in registers until the MMAs that read the previous pair have completed.
-// 16 consecutive bf16 values (8 packed words): columns c0 .. c0+15 of row `row`
-__device__ __forceinline__ void store_row_chunk16_swz_packed(uint8_t* tile, int row, int c0, const uint32_t (&v)[8]) {
-    uint8_t* rowp = tile + row * 128;
-#pragma unroll
-    for (int g = 0; g < 2; ++g) {
-        const uint4 o = make_uint4(v[g * 4], v[g * 4 + 1], v[g * 4 + 2], v[g * 4 + 3]);
-        const int u = (c0 >> 3) + g;
-        *reinterpret_cast<uint4*>(rowp + ((u ^ (row & 7)) << 4)) = o;
-    }
-}
 // 16 fp32 accumulator values of one row -> 16 bf16 in global memory (32 bytes)
 __device__ __forceinline__ void store16_bf16(bf16* dst, const uint32_t (&r)[16]) {
 #pragma unroll
@@ -165,63 +152,67 @@ __device__ __forceinline__ uint32_t pack_bf16x2(float lo, float hi) {
     return *reinterpret_cast<uint32_t*>(&h);
 }
 
+__device__ __forceinline__ float ld_cluster_f32(uint32_t cluster_addr) {
+    float v;
+    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(cluster_addr) : "memory");
+    return v;
+}
+
 template <int HS>
 __global__ void __launch_bounds__(kBwdThreads, 1)
 attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmap_kv128,   // qkv, box 128 rows (K and V tiles)
                      const __grid_constant__ CUtensorMap tmap_q64,     // qkv, box 64 rows (Q tiles)
                      const __grid_constant__ CUtensorMap tmap_do64,    // dO, box 64 rows
-                     const AttnParams p) {
+                     const AttnParams p, const int heads_per_cta) {
     constexpr int BKV = 128, BQ = 64, NCH = HS / 64, NBUF = 4;
-    constexpr int KV_BYTES = BKV * HS * 2, Q_BYTES = BQ * HS * 2, PT_BYTES = BKV * BQ * 2;
+    constexpr int KV_BYTES = BKV * HS * 2, Q_BYTES = BQ * HS * 2;
     constexpr uint32_t TMEM_COLS = 512;                       // S0 S1 | dP0 dP1 | dV | dK
     constexpr int CW = BQ / kBwdWarpgroups;                   // score columns per compute thread
-    static_assert(CW == 16, "the column split below is written for 16 columns per thread");
+    static_assert(CW == 16, "the column split below is written for 16 columns per thread (one K step of the dV / dK MMAs)");
     extern __shared__ __align__(1024) uint8_t smem[];
     uint8_t* sK = smem;
     uint8_t* sV = sK + KV_BYTES;
     uint8_t* sQ = sV + KV_BYTES;              // NBUF buffers
     uint8_t* sdO = sQ + NBUF * Q_BYTES;       // NBUF buffers
-    uint8_t* sPT = sdO + NBUF * Q_BYTES;
-    uint8_t* sdST = sPT + PT_BYTES;
-    float* sLse = reinterpret_cast<float*>(sdST + PT_BYTES);      // [2][64] pre-multiplied by log2(e)
-    float* sDelta = sLse + 2 * BQ;                                // [2][64]
-    uint64_t* bars = reinterpret_cast<uint64_t*>(sDelta + 2 * BQ);
+    float* sLse = reinterpret_cast<float*>(sdO + NBUF * Q_BYTES);  // [NBUF][64] pre-multiplied by log2(e)
+    float* sDelta = sLse + NBUF * BQ;                              // [NBUF][64] pre-multiplied by the softmax scale
+    uint64_t* bars = reinterpret_cast<uint64_t*>(sDelta + NBUF * BQ);
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 16);
     volatile uint32_t* abort_flag = tmem_slot + 1;
 
-    const int tid = threadIdx.x, warp = tid >> 5;
+    const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);       // uniform, and known to be
     const bool issuer = warp == kBwdComputeWarps;             // MMA issuer (lane 0); its only other work is waiting
-    const bool producer = warp == kBwdComputeWarps + 1;       // TMA producer (lane 0)
-    const bool issuer2 = warp == kBwdComputeWarps + 2;        // issuer of the dV / dK MMAs (lane 0)
+    const bool producer = warp == kBwdComputeWarps + 1;       // TMA loads (lane 0) and row statistics (all lanes)
     const int wg = tid >> 7, r = tid & 127;                   // compute threads: column slice, row of the tile (TMEM lane)
     if (smem_u32(smem) & 1023u) { if (tid == 0) atomicOr(p.status, kErrOther); return; }
-    // 1-D grid, key block slowest: the blocks with the longest walks (small kb) start first on every SM
-    const int kb = blockIdx.x / (p.Hkv * p.B);
-    const int kvh = (blockIdx.x % (p.Hkv * p.B)) % p.Hkv, b = (blockIdx.x % (p.Hkv * p.B)) / p.Hkv;
+    // 1-D grid, key block slowest: the blocks with the longest walks (small kb) start first on every SM; `parts` CTAs of a
+    // cluster share the query heads of one (key block, kv head, batch) item
     const int G = p.Hq / p.Hkv;
+    const int parts = (G + heads_per_cta - 1) / heads_per_cta;
+    const int item = blockIdx.x / parts, part = blockIdx.x % parts;
+    const int kb = item / (p.Hkv * p.B);
+    const int kvh = (item % (p.Hkv * p.B)) % p.Hkv, b = (item % (p.Hkv * p.B)) / p.Hkv;
+    const int h0 = kvh * G + part * heads_per_cta;              // query heads [h0, h0 + nh)
+    const int nh = min(heads_per_cta, G - part * heads_per_cta);
     const int kv0 = kb * BKV;
     const int nqb = (p.T + BQ - 1) / BQ;
     const int qb_first = kv0 / BQ;
-    const int per_head = nqb - qb_first;
-    const int n_it = per_head * G;
+    const int n_it = (nqb - qb_first) * nh;
     const int kcol = (p.Hq + kvh) * HS, vcol = (p.Hq + p.Hkv + kvh) * HS;
 
-    // barriers: 0 kv | 1-4 q/dO ring | 5 sp (scores ready) | 6 acc (dV/dK MMAs of a tile done) | 7 p_ready (P^T/dS^T stored)
-    //           8-9 s_free (score buffer read by all compute threads) | 10 second sp | 11-14 q/dO buffer free
+    // barriers: 0 kv | 1-4 q/dO ring (TMA bytes + row statistics) | 5-6 scores ready | 7-8 P^T/dS^T in tensor memory | 9 all done
+    //           10-13 q/dO buffer free.  Two-entry sets alternate with the tile parity: the commit of tile it+2 needs every
+    //           compute warp to have handed over tile it, so a waiter can never miss a phase.
     const uint32_t bar0 = smem_u32(bars);
-    // Two score barriers, used alternately: the commit of tile it+2 needs every compute warp to have read tile it, so a
-    // waiter can never miss a phase (with one barrier, tiles 0 and 1 can both complete before a slow warp looks).
-    const uint32_t kv_bar = bar0, acc_bar = bar0 + 48, p_ready = bar0 + 56;
-    auto sp_bar = [&](int it) { return (it & 1) ? bar0 + 80 : bar0 + 40; };
+    const uint32_t kv_bar = bar0, done_bar = bar0 + 72;
     auto qdo_bar = [&](int buf) { return bar0 + 8 + 8 * buf; };
-    auto s_free = [&](int buf) { return bar0 + 64 + 8 * buf; };
-    auto qdo_free = [&](int buf) { return bar0 + 88 + 8 * buf; };
+    auto sp_bar = [&](int it) { return bar0 + 40 + 8 * (it & 1); };
+    auto p_ready = [&](int it) { return bar0 + 56 + 8 * (it & 1); };
+    auto qdo_free = [&](int buf) { return bar0 + 80 + 8 * buf; };
     if (tid == 0) {
-        for (int i = 0; i < 7; ++i) mbar_init(bar0 + 8 * i, 1);
-        for (int i = 10; i < 15; ++i) mbar_init(bar0 + 8 * i, 1);
-        mbar_init(p_ready, kBwdComputeWarps);
-        mbar_init(s_free(0), kBwdComputeWarps);
-        mbar_init(s_free(1), kBwdComputeWarps);
+        mbar_init(kv_bar, 1); mbar_init(done_bar, 1);
+        for (int i = 0; i < NBUF; ++i) { mbar_init(qdo_bar(i), 2); mbar_init(qdo_free(i), 1); }
+        for (int i = 0; i < 2; ++i) { mbar_init(sp_bar(i), 1); mbar_init(p_ready(i), kBwdComputeWarps); }
         *abort_flag = 0;
         mbar_init_fence();
     }
@@ -232,153 +223,158 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmap_kv128,   // qkv, b
     const uint32_t tmem = *tmem_slot;
     const uint32_t tdV = tmem + 4 * BQ, tdK = tmem + 4 * BQ + HS;
     const uint32_t lane_off = static_cast<uint32_t>((warp & 3) * 32) << 16;
-    auto tile_of = [&](int it, int& hq, int& qb) { hq = kvh * G + it / per_head; qb = qb_first + it % per_head; };
+    auto tS = [&](int it) { return tmem + (it & 1) * BQ; };
+    auto tdP = [&](int it) { return tmem + 2 * BQ + (it & 1) * BQ; };
     bool ok = true;
 
     if (producer) {
         // ============================================================ TMA producer warp
-        if ((tid & 31) == 0 && n_it > 0) {
+        const int lane = tid & 31;
+        if (lane == 0) {
             tma_prefetch_desc(&tmap_kv128); tma_prefetch_desc(&tmap_q64); tma_prefetch_desc(&tmap_do64);
-            mbar_expect_tx(kv_bar, 2 * KV_BYTES);
-            for (int c = 0; c < NCH; ++c) {
-                tma_load_3d(smem_u32(sK) + c * (BKV * 128), &tmap_kv128, kv_bar, kcol + c * 64, kv0, b);
-                tma_load_3d(smem_u32(sV) + c * (BKV * 128), &tmap_kv128, kv_bar, vcol + c * 64, kv0, b);
+            if (n_it > 0) {
+                mbar_expect_tx(kv_bar, 2 * KV_BYTES);
+                for (int c = 0; c < NCH; ++c) {
+                    tma_load_3d(smem_u32(sK) + c * (BKV * 128), &tmap_kv128, kv_bar, kcol + c * 64, kv0, b);
+                    tma_load_3d(smem_u32(sV) + c * (BKV * 128), &tmap_kv128, kv_bar, vcol + c * 64, kv0, b);
+                }
             }
-            int hq = kvh * G, qb = qb_first;
-            for (int it = 0; it < n_it; ++it) {
-                const int buf = it % NBUF;
-                // the buffer's previous tile, it - NBUF, has been consumed by its dV / dK MMAs
-                if (it >= NBUF && !mbar_wait(qdo_free(buf), ((it / NBUF) - 1) & 1, abort_flag)) { atomicOr(p.status, kErrOther); break; }
+        }
+        int hq = h0, qb = qb_first;
+        for (int it = 0; it < n_it; ++it) {
+            const int buf = it % NBUF;
+            // lse and delta of the tile's 64 queries, two per lane; rows beyond the sequence get probability 0
+            float l2[2], dl[2];
+#pragma unroll
+            for (int i = 0; i < 2; ++i) {
+                const int q = qb * BQ + lane + 32 * i;
+                const long long si = (static_cast<long long>(b) * p.Hq + hq) * p.T + q;
+                l2[i] = q < p.T ? __ldg(p.lse + si) * kLog2e : INFINITY;
+                dl[i] = q < p.T ? __ldg(p.delta + si) * p.scale : 0.f;
+            }
+            // the buffer's previous tile, it - NBUF, has been consumed by its dV / dK MMAs
+            if (it >= NBUF) {
+                bool got = true;
+                if (lane == 0) got = mbar_wait(qdo_free(buf), ((it / NBUF) - 1) & 1, abort_flag);
+                if (!__shfl_sync(0xffffffffu, static_cast<int>(got), 0)) { if (lane == 0) atomicOr(p.status, kErrOther); break; }
+            }
+            if (lane == 0) {
                 mbar_expect_tx(qdo_bar(buf), 2 * Q_BYTES);
                 for (int c = 0; c < NCH; ++c) {
                     tma_load_3d(smem_u32(sQ) + buf * Q_BYTES + c * (BQ * 128), &tmap_q64, qdo_bar(buf), hq * HS + c * 64, qb * BQ, b);
                     tma_load_3d(smem_u32(sdO) + buf * Q_BYTES + c * (BQ * 128), &tmap_do64, qdo_bar(buf), hq * HS + c * 64, qb * BQ, b);
                 }
-                if (++qb == nqb) { qb = qb_first; ++hq; }
             }
+#pragma unroll
+            for (int i = 0; i < 2; ++i) { sLse[buf * BQ + lane + 32 * i] = l2[i]; sDelta[buf * BQ + lane + 32 * i] = dl[i]; }
+            warp_arrive(qdo_bar(buf));
+            if (++qb == nqb) { qb = qb_first; ++hq; }
         }
     } else if (issuer) {
         // ============================================================ MMA issuer warp
-        if ((tid & 31) == 0 && n_it > 0) {
+        // One thread issues everything in the order S/dP(0), S/dP(1), dV/dK(0), S/dP(2), dV/dK(1), ...: MMAs of one CTA
+        // execute in issue order, so the scores of tile it+2 cannot overwrite the P^T / dS^T of tile it that live in the
+        // same columns, and the chain score tile -> probabilities has the time of 1280 tensor cycles to complete.
+        if (n_it > 0) {
+            const bool leader = elect_one();
             const uint32_t idesc_st = make_instr_desc(1, 1, false, false, BKV, BQ);     // S^T = K Q^T, dP^T = V dO^T
-            // scores of tile it: needs its Q / dO and, from tile 2 on, the score buffer read by every compute warp
+            const uint32_t idesc_acc = make_instr_desc(1, 1, false, true, BKV, HS);     // dV += P^T dO, dK += dS^T Q
+            const uint32_t k_lo = desc_lo(smem_u32(sK), 16), v_lo = desc_lo(smem_u32(sV), 16);
             auto issue_sp = [&](int it) -> bool {
                 const int buf = it % NBUF;
-                if (!mbar_wait(qdo_bar(buf), (it / NBUF) & 1, abort_flag)) return false;
-                if (it >= 2 && !mbar_wait(s_free(it & 1), ((it - 2) >> 1) & 1, abort_flag)) return false;
+                if (!mbar_wait_warp(qdo_bar(buf), (it / NBUF) & 1, abort_flag)) return false;
                 tc_fence_after_sync();
-                const uint32_t tS = tmem + (it & 1) * BQ, tdP = tmem + 2 * BQ + (it & 1) * BQ;
+                const uint32_t q_lo = desc_lo(smem_u32(sQ) + buf * Q_BYTES, 16), do_lo = desc_lo(smem_u32(sdO) + buf * Q_BYTES, 16);
+                const uint32_t s_t = tS(it), dp_t = tdP(it), bar = sp_bar(it);
+                if (leader) {
 #pragma unroll
-                for (int k = 0; k < HS / 16; ++k) {
-                    mma_issue<false, false>(tS, DLO(smem_u32(sK), 16, (k / 4) * (BKV * 128) + (k % 4) * 32), kDescHi,
-                                            DLO(smem_u32(sQ) + buf * Q_BYTES, 16, (k / 4) * (BQ * 128) + (k % 4) * 32), kDescHi, idesc_st, k > 0);
-                }
+                    for (int k = 0; k < HS / 16; ++k)
+                        mma_issue<false, false>(s_t, k_lo + (((k / 4) * (BKV * 128) + (k % 4) * 32) >> 4), kDescHi,
+                                                q_lo + (((k / 4) * (BQ * 128) + (k % 4) * 32) >> 4), kDescHi, idesc_st, k > 0);
 #pragma unroll
-                for (int k = 0; k < HS / 16; ++k) {
-                    mma_issue<false, false>(tdP, DLO(smem_u32(sV), 16, (k / 4) * (BKV * 128) + (k % 4) * 32), kDescHi,
-                                            DLO(smem_u32(sdO) + buf * Q_BYTES, 16, (k / 4) * (BQ * 128) + (k % 4) * 32), kDescHi, idesc_st, k > 0);
+                    for (int k = 0; k < HS / 16; ++k)
+                        mma_issue<false, false>(dp_t, v_lo + (((k / 4) * (BKV * 128) + (k % 4) * 32) >> 4), kDescHi,
+                                                do_lo + (((k / 4) * (BQ * 128) + (k % 4) * 32) >> 4), kDescHi, idesc_st, k > 0);
+                    mma_commit(bar);
                 }
-                mma_commit(sp_bar(it));
+                __syncwarp();
                 return true;
             };
-            ok = mbar_wait(kv_bar, 0, abort_flag);
-            for (int it = 0; it < n_it && ok; ++it) ok = issue_sp(it);
-            if (!ok) { *abort_flag = 1u; atomicOr(p.status, kErrOther); }
-        }
-    } else if (issuer2) {
-        // ============================================================ dV / dK MMA issuer warp
-        if ((tid & 31) == 0 && n_it > 0) {
-            const uint32_t idesc_acc = make_instr_desc(1, 1, false, true, BKV, HS);      // dV += P^T dO, dK += dS^T Q
+            ok = mbar_wait_warp(kv_bar, 0, abort_flag) && issue_sp(0);
             for (int it = 0; it < n_it && ok; ++it) {
-                if (!mbar_wait(p_ready, it & 1, abort_flag)) { ok = false; break; }
+                if (it + 1 < n_it) ok = issue_sp(it + 1);
+                if (!ok || !mbar_wait_warp(p_ready(it), (it >> 1) & 1, abort_flag)) { ok = false; break; }
                 tc_fence_after_sync();
                 const int buf = it % NBUF;
+                const uint32_t q_lo = desc_lo(smem_u32(sQ) + buf * Q_BYTES, BQ * 128), do_lo = desc_lo(smem_u32(sdO) + buf * Q_BYTES, BQ * 128);
+                const uint32_t s_t = tS(it), dp_t = tdP(it), bar = qdo_free(buf);
+                const uint32_t acc0 = it > 0;
+                if (leader) {
 #pragma unroll
-                for (int k = 0; k < BQ / 16; ++k) {
-                    mma_issue<false, false>(tdV, DLO(smem_u32(sPT), 16, k * 32), kDescHi,
-                                            DLO(smem_u32(sdO) + buf * Q_BYTES, BQ * 128, k * (16 * 128)), kDescHi, idesc_acc, (it > 0 || k > 0));
-                }
+                    for (int k = 0; k < BQ / 16; ++k)
+                        mma_issue_f16_tmem_a(tdV, s_t + k * CW, do_lo + ((k * (16 * 128)) >> 4), kDescHi, idesc_acc, k > 0 ? 1u : acc0);
 #pragma unroll
-                for (int k = 0; k < BQ / 16; ++k) {
-                    mma_issue<false, false>(tdK, DLO(smem_u32(sdST), 16, k * 32), kDescHi,
-                                            DLO(smem_u32(sQ) + buf * Q_BYTES, BQ * 128, k * (16 * 128)), kDescHi, idesc_acc, (it > 0 || k > 0));
+                    for (int k = 0; k < BQ / 16; ++k)
+                        mma_issue_f16_tmem_a(tdK, dp_t + k * CW, q_lo + ((k * (16 * 128)) >> 4), kDescHi, idesc_acc, k > 0 ? 1u : acc0);
+                    mma_commit(bar);
                 }
-                mma_commit(acc_bar);
-                mma_commit(qdo_free(buf));
+                __syncwarp();
             }
-            if (!ok) { *abort_flag = 1u; atomicOr(p.status, kErrOther); }
+            if (leader) {
+                if (ok) mma_commit(done_bar);
+                else { *abort_flag = 1u; atomicOr(p.status, kErrOther); }
+            }
+            __syncwarp();
         }
     } else {
         // ============================================================ compute warps
-        auto load_stats = [&](int it) {                         // lse (threads 0-63) and delta (64-127) of tile it
-            if (tid >= 128) return;
-            int hq, qb; tile_of(it, hq, qb);
-            const int q = qb * BQ + (tid & 63);
-            const long long si = (static_cast<long long>(b) * p.Hq + hq) * p.T + q;
-            float* dst = (tid < 64 ? sLse : sDelta) + (it & 1) * BQ + (tid & 63);
-            if (tid < 64) *dst = q < p.T ? p.lse[si] * kLog2e : INFINITY;
-            else *dst = q < p.T ? p.delta[si] * p.scale : 0.f;       // delta pre-multiplied by the softmax scale
-        };
         const float sl2 = p.scale * kLog2e;
         const int kv_row = kv0 + r;
         const int c0 = wg * CW;
-        if (n_it > 0) load_stats(0);
-        compute_barrier();
-        // One tile; false when a wait ran out.  The caller still runs the barrier of every remaining tile, so that a
-        // failure can never leave part of the CTA behind at a barrier.
-        auto tile_body = [&](int it) -> bool {
-            int hq, qb; tile_of(it, hq, qb);
-            if (it + 1 < n_it) load_stats(it + 1);             // read after the barrier at the end of this tile
-            if (!mbar_wait(sp_bar(it), (it >> 1) & 1, abort_flag)) return false;
-            tc_fence_after_sync();
-            const bool diag = qb * BQ < kv0 + BKV;              // some (kv, q) pairs have q < kv
-            const float* lse_t = sLse + (it & 1) * BQ;
-            const float* delta_t = sDelta + (it & 1) * BQ;
-            const uint32_t tS = tmem + (it & 1) * BQ, tdP = tmem + 2 * BQ + (it & 1) * BQ;
-            uint32_t ptp[CW / 2], dsp[CW / 2];
-            {
-                uint32_t rs[CW], rp[CW];
-                tmem_ld_32x32b_x16(tS + lane_off + c0, rs);
-                tmem_ld_32x32b_x16(tdP + lane_off + c0, rp);
-                tmem_ld_wait();
-                tc_fence_before_sync();
-                warp_arrive(s_free(it & 1));                    // this score buffer may be overwritten
-                float lse_c[CW], del_c[CW];
-#pragma unroll
-                for (int i = 0; i < CW; i += 4) {
-                    *reinterpret_cast<float4*>(lse_c + i) = *reinterpret_cast<const float4*>(lse_t + c0 + i);
-                    *reinterpret_cast<float4*>(del_c + i) = *reinterpret_cast<const float4*>(delta_t + c0 + i);
-                }
-                float pv[CW], ds[CW];
-#pragma unroll
-                for (int i = 0; i < CW; ++i) {
-                    pv[i] = fast_exp2(fmaf(__uint_as_float(rs[i]), sl2, -lse_c[i]));
-                    ds[i] = fmaf(__uint_as_float(rp[i]), p.scale, -del_c[i]);
-                }
-                if (diag) {                                     // only tiles that touch the diagonal pay for the mask
-                    const int lim = kv_row - qb * BQ - c0;      // columns below lim are above the diagonal (q < kv)
-#pragma unroll
-                    for (int i = 0; i < CW; ++i) if (i < lim) pv[i] = 0.f;
-                }
-#pragma unroll
-                for (int i = 0; i < CW; i += 2) {
-                    ptp[i / 2] = pack_bf16x2(pv[i], pv[i + 1]);
-                    dsp[i / 2] = pack_bf16x2(pv[i] * ds[i], pv[i + 1] * ds[i + 1]);
-                }
-            }
-            // P^T / dS^T of tile it-1 are read by its dV / dK MMAs until acc_bar completes
-            if (it > 0 && !mbar_wait(acc_bar, (it - 1) & 1, abort_flag)) return false;
-            store_row_chunk16_swz_packed(sPT, r, c0, ptp);
-            store_row_chunk16_swz_packed(sdST, r, c0, dsp);
-            fence_proxy_async_smem();
-            warp_arrive(p_ready);
-            return true;
-        };
+        int qb = qb_first;
         for (int it = 0; it < n_it; ++it) {
-            if (ok) ok = tile_body(it);
-            compute_barrier();                                  // statistics of tile it+1 visible to all compute threads
+            const int buf = it % NBUF;
+            if (!mbar_wait(sp_bar(it), (it >> 1) & 1, abort_flag) || !mbar_wait(qdo_bar(buf), (it / NBUF) & 1, abort_flag)) { ok = false; break; }
+            tc_fence_after_sync();
+            uint32_t rs[CW], rp[CW];
+            __syncwarp();
+            tmem_ld_32x32b_x16(tS(it) + lane_off + c0, rs);
+            tmem_ld_32x32b_x16(tdP(it) + lane_off + c0, rp);
+            const float* lse_t = sLse + buf * BQ + c0;
+            const float* delta_t = sDelta + buf * BQ + c0;
+            float lse_c[CW], del_c[CW];
+#pragma unroll
+            for (int i = 0; i < CW; i += 4) {
+                *reinterpret_cast<float4*>(lse_c + i) = *reinterpret_cast<const float4*>(lse_t + i);
+                *reinterpret_cast<float4*>(del_c + i) = *reinterpret_cast<const float4*>(delta_t + i);
+            }
+            tmem_ld_wait();
+            float pv[CW], ds[CW];
+#pragma unroll
+            for (int i = 0; i < CW; ++i) {
+                pv[i] = fast_exp2(fmaf(__uint_as_float(rs[i]), sl2, -lse_c[i]));
+                ds[i] = fmaf(__uint_as_float(rp[i]), p.scale, -del_c[i]);
+            }
+            if (qb * BQ < kv0 + BKV) {                          // only tiles that touch the diagonal pay for the mask
+                const int lim = kv_row - qb * BQ - c0;          // columns below lim are above the diagonal (q < kv)
+#pragma unroll
+                for (int i = 0; i < CW; ++i) if (i < lim) pv[i] = 0.f;
+            }
+            uint32_t ptp[CW / 2], dsp[CW / 2];
+#pragma unroll
+            for (int i = 0; i < CW; i += 2) {
+                ptp[i / 2] = pack_bf16x2(pv[i], pv[i + 1]);
+                dsp[i / 2] = pack_bf16x2(pv[i] * ds[i], pv[i + 1] * ds[i + 1]);
+            }
+            // Into the first half of the very columns this thread has just read: one K step of 16 queries per warpgroup
+            tmem_st_32x32b_x8(tS(it) + lane_off + c0, ptp);
+            tmem_st_32x32b_x8(tdP(it) + lane_off + c0, dsp);
+            tmem_st_wait();
+            tc_fence_before_sync();
+            warp_arrive(p_ready(it));
+            if (++qb == nqb) qb = qb_first;
         }
-        if (ok && n_it > 0) ok = mbar_wait(acc_bar, (n_it - 1) & 1, abort_flag);
+        if (ok && n_it > 0) ok = mbar_wait(done_bar, 0, abort_flag);
         tc_fence_after_sync();
         if (!ok && r == 0) atomicOr(p.status, kErrOther);
         if (ok && n_it > 0) {
@@ -388,6 +384,7 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmap_kv128,   // qkv, b
             const long long rbase = (static_cast<long long>(b) * p.T + (row_ok ? kv_row : 0)) * H;
             bf16* dk = p.dqkv + (rbase + p.Hq + kvh) * HS;
             bf16* dv = p.dqkv + (rbase + p.Hq + p.Hkv + kvh) * HS;
+            float* part_sum = reinterpret_cast<float*>(sQ);     // [dK, dV][HS columns][128 rows], over the Q / dO rings
             __syncwarp();
             constexpr int ECW = HS / kBwdWarpgroups;           // output columns per thread
 #pragma unroll
@@ -397,12 +394,49 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmap_kv128,   // qkv, b
                 tmem_ld_32x32b_x16(tdK + lane_off + col, rk);
                 tmem_ld_32x32b_x16(tdV + lane_off + col, rv);
                 tmem_ld_wait();
-                if (row_ok) {
+                if (parts > 1) {
+#pragma unroll
+                    for (int i = 0; i < 16; ++i) {
+                        part_sum[(col + i) * BKV + r] = __uint_as_float(rk[i]);
+                        part_sum[(HS + col + i) * BKV + r] = __uint_as_float(rv[i]);
+                    }
+                } else if (row_ok) {
                     store16_bf16(dk + col, rk);
                     store16_bf16(dv + col, rv);
                 }
             }
         }
+    }
+    if (parts > 1) {
+        // The CTAs of the cluster hold fp32 sums over their own query heads; each adds up a slice of the rows over all of
+        // them, in the order of the heads, and stores it.
+        __syncwarp();
+        cluster_arrive();
+        cluster_wait();
+        if (warp < kBwdComputeWarps) {
+            const int slice = (BKV + parts - 1) / parts, row0 = part * slice, rows = min(slice, BKV - row0);
+            const int H = p.Hq + 2 * p.Hkv;
+            const uint32_t base = smem_u32(sQ);
+            for (int i = tid; i < 2 * (HS / 8) * rows; i += kBwdComputeThreads) {
+                const int row = row0 + i % rows, grp = i / rows, which = grp / (HS / 8), col = (grp % (HS / 8)) * 8;
+                float v[8];
+#pragma unroll
+                for (int k = 0; k < 8; ++k) v[k] = 0.f;
+                for (int q = 0; q < parts; ++q) {
+                    const uint32_t src = map_to_cta(base + static_cast<uint32_t>(((which * HS + col) * BKV + row) * 4), q);
+#pragma unroll
+                    for (int k = 0; k < 8; ++k) v[k] += ld_cluster_f32(src + static_cast<uint32_t>(k * BKV * 4));
+                }
+                if (kv0 + row < p.T) {
+                    uint4 o = make_uint4(pack_bf16x2(v[0], v[1]), pack_bf16x2(v[2], v[3]), pack_bf16x2(v[4], v[5]), pack_bf16x2(v[6], v[7]));
+                    bf16* dst = p.dqkv + ((static_cast<long long>(b) * p.T + kv0 + row) * H + p.Hq + which * p.Hkv + kvh) * HS + col;
+                    *reinterpret_cast<uint4*>(dst) = o;
+                }
+            }
+        }
+        __syncwarp();
+        cluster_arrive();                                       // nobody leaves while its sums may still be read
+        cluster_wait();
     }
     tc_fence_before_sync();
     __syncthreads();
@@ -411,56 +445,59 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmap_kv128,   // qkv, b
 }
 
 // ------------------------------------------------------------------------------------------------
-// dQ.  One CTA owns 128 query rows of one kv head and walks over the query heads of that group, and for every head
-// over the key tiles up to the diagonal, so the start-up and drain costs of a CTA are paid once per group instead
-// of once per head.  Q and dO of the current head live in tensor memory as the A operands of the score MMAs (they
-// are constant during a key walk), K / V tiles stream through a ring of four shared-memory buffers three tiles
-// ahead of the MMAs, S / dP are double buffered in TMEM, dQ accumulates in TMEM and is drained once per head.
+// dQ.  One CTA owns 128 query rows and walks over `heads_per_cta` query heads of one kv head, and for every head over
+// the key tiles up to the diagonal.  Q and dO of the current head live in tensor memory as the A operands of the score
+// MMAs (they are constant during a key walk), K / V tiles stream through a ring of four shared-memory buffers three
+// tiles ahead of the MMAs, S / dP are double buffered in TMEM, dS takes the place of the dP tile it was computed from
+// (A operand of dQ += dS K), dQ accumulates in TMEM and is drained once per head while the scores of the next head's
+// first tile are computed.
 template <int HS>
 __global__ void __launch_bounds__(kBwdThreads, 1)
 attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmap_kv64,    // qkv, box 64 rows
-                   const AttnParams p) {
+                   const AttnParams p, const int heads_per_cta) {
     constexpr int BQ = 128, BKV = 64, NCH = HS / 64, NBUF = 4;
-    constexpr int KV_BYTES = BKV * HS * 2, DS_BYTES = BQ * BKV * 2;
+    constexpr int KV_BYTES = BKV * HS * 2;
     constexpr uint32_t TMEM_COLS = 512;                       // Q | dO (bf16 pairs, A operands) | S0 S1 | dP0 dP1 | dQ
     constexpr int CW = BKV / kBwdWarpgroups;
-    static_assert(CW == 16, "the column split below is written for 16 columns per thread");
+    static_assert(CW == 16, "the column split below is written for 16 columns per thread (one K step of the dQ MMA)");
     extern __shared__ __align__(1024) uint8_t smem[];
     uint8_t* sK = smem;                       // NBUF buffers
     uint8_t* sV = sK + NBUF * KV_BYTES;       // NBUF buffers
-    uint8_t* sdS = sV + NBUF * KV_BYTES;
-    uint64_t* bars = reinterpret_cast<uint64_t*>(sdS + DS_BYTES);
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 16);
+    uint64_t* bars = reinterpret_cast<uint64_t*>(sV + NBUF * KV_BYTES);
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 18);
     volatile uint32_t* abort_flag = tmem_slot + 1;
 
-    const int tid = threadIdx.x, warp = tid >> 5;
-    const bool issuer = warp == kBwdComputeWarps, producer = warp == kBwdComputeWarps + 1, issuer2 = warp == kBwdComputeWarps + 2;
+    const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);       // uniform, and known to be
+    const bool issuer = warp == kBwdComputeWarps, producer = warp == kBwdComputeWarps + 1;
     const int wg = tid >> 7, r = tid & 127;
     if (smem_u32(smem) & 1023u) { if (tid == 0) atomicOr(p.status, kErrOther); return; }
     const int nqb = (p.T + BQ - 1) / BQ;
-    const int qb = nqb - 1 - blockIdx.x / (p.Hkv * p.B);        // 1-D grid, longest key walks first
-    const int kvh = (blockIdx.x % (p.Hkv * p.B)) % p.Hkv, b = (blockIdx.x % (p.Hkv * p.B)) / p.Hkv;
     const int G = p.Hq / p.Hkv;
+    const int parts = (G + heads_per_cta - 1) / heads_per_cta;
+    const int per_qb = p.Hkv * p.B * parts;
+    const int qb = nqb - 1 - blockIdx.x / per_qb;               // 1-D grid, longest key walks first
+    const int rest = blockIdx.x % per_qb;
+    const int kvh = rest % p.Hkv, b = (rest / p.Hkv) % p.B, part = rest / (p.Hkv * p.B);
+    const int h0 = kvh * G + part * heads_per_cta;              // query heads [h0, h0 + nh)
+    const int nh = min(heads_per_cta, G - part * heads_per_cta);
     const int q0 = qb * BQ;
     const int n_kv = min((p.T + BKV - 1) / BKV, (q0 + BQ) / BKV);
-    const int total = n_kv * G;                                 // tiles of the whole walk, t = g * n_kv + j
+    const int total = n_kv * nh;                                // tiles of the whole walk, t = g * n_kv + j
     const int kcol = (p.Hq + kvh) * HS, vcol = (p.Hq + p.Hkv + kvh) * HS;
 
-    // barriers: 0 head_ready | 1-4 k/v ring | 5, 10 sp (alternating) | 6 dq (dQ MMA of a tile done) | 7 p_ready | 8-9 s_free
-    //           11-14 k/v buffer free
+    // barriers: 0 head_ready | 1-4 k/v ring | 5-6 S ready | 7-8 dP ready | 9-10 dS in tensor memory | 11 dQ of a head done
+    //           12 dQ of a head drained | 13-16 k/v buffer free.  Two-entry sets alternate with the tile parity.
     const uint32_t bar0 = smem_u32(bars);
-    const uint32_t head_ready = bar0, dq_bar = bar0 + 48, p_ready = bar0 + 56;
-    auto sp_bar = [&](int t) { return (t & 1) ? bar0 + 80 : bar0 + 40; };        // alternating, see the dK / dV kernel
+    const uint32_t head_ready = bar0, dq_bar = bar0 + 88, dq_drained = bar0 + 96;
     auto kv_bar = [&](int buf) { return bar0 + 8 + 8 * buf; };
-    auto s_free = [&](int buf) { return bar0 + 64 + 8 * buf; };
-    auto kv_free = [&](int buf) { return bar0 + 88 + 8 * buf; };
+    auto s_bar = [&](int t) { return bar0 + 40 + 8 * (t & 1); };
+    auto dp_bar = [&](int t) { return bar0 + 56 + 8 * (t & 1); };
+    auto p_ready = [&](int t) { return bar0 + 72 + 8 * (t & 1); };
+    auto kv_free = [&](int buf) { return bar0 + 104 + 8 * buf; };
     if (tid == 0) {
-        for (int i = 1; i < 7; ++i) mbar_init(bar0 + 8 * i, 1);
-        for (int i = 10; i < 15; ++i) mbar_init(bar0 + 8 * i, 1);
-        mbar_init(head_ready, kBwdComputeWarps);
-        mbar_init(p_ready, kBwdComputeWarps);
-        mbar_init(s_free(0), kBwdComputeWarps);
-        mbar_init(s_free(1), kBwdComputeWarps);
+        mbar_init(head_ready, kBwdComputeWarps); mbar_init(dq_drained, kBwdComputeWarps); mbar_init(dq_bar, 1);
+        for (int i = 0; i < NBUF; ++i) { mbar_init(kv_bar(i), 1); mbar_init(kv_free(i), 1); }
+        for (int i = 0; i < 2; ++i) { mbar_init(s_bar(i), 1); mbar_init(dp_bar(i), 1); mbar_init(p_ready(i), kBwdComputeWarps); }
         *abort_flag = 0;
         mbar_init_fence();
     }
@@ -469,7 +506,9 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmap_kv64,    // qkv, box
     __syncthreads();
     tc_fence_after_sync();
     const uint32_t tmem = *tmem_slot;
-    const uint32_t tQ = tmem, tdO = tmem + HS / 2, tS0 = tmem + HS, tdP0 = tmem + HS + 2 * BKV, tdQ = tmem + HS + 4 * BKV;
+    const uint32_t tQ = tmem, tdO = tmem + HS / 2, tdQ = tmem + HS + 4 * BKV;
+    auto tS = [&](int t) { return tmem + HS + (t & 1) * BKV; };
+    auto tdP = [&](int t) { return tmem + HS + 2 * BKV + (t & 1) * BKV; };
     const uint32_t lane_off = static_cast<uint32_t>((warp & 3) * 32) << 16;
     bool ok = true;
 
@@ -492,56 +531,58 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmap_kv64,    // qkv, box
         }
     } else if (issuer) {
         // ============================================================ MMA issuer warp
-        if ((tid & 31) == 0 && total > 0) {
+        // As in the dK / dV kernel one thread issues everything: S/dP(t+1) before dQ(t), except that the first tile of a
+        // head (which needs that head's Q / dO in tensor memory) comes after the last dQ MMA of the previous head.
+        if (total > 0) {
+            const bool leader = elect_one();
             const uint32_t idesc_s = make_instr_desc(1, 1, false, false, BQ, BKV);
-            // scores of tile t; needs its K / V tile and, from t = 2 on, the score buffer read by every compute warp
+            const uint32_t idesc_dq = make_instr_desc(1, 1, false, true, BQ, HS);
             auto issue_sp = [&](int t) -> bool {
                 const int buf = t % NBUF;
-                if (!mbar_wait(kv_bar(buf), (t / NBUF) & 1, abort_flag)) return false;
-                if (t >= 2 && !mbar_wait(s_free(t & 1), ((t - 2) >> 1) & 1, abort_flag)) return false;
+                if (!mbar_wait_warp(kv_bar(buf), (t / NBUF) & 1, abort_flag)) return false;
                 tc_fence_after_sync();
-                const uint32_t tS = tS0 + (t & 1) * BKV, tdP = tdP0 + (t & 1) * BKV;
+                const uint32_t k_lo = desc_lo(smem_u32(sK) + buf * KV_BYTES, 16), v_lo = desc_lo(smem_u32(sV) + buf * KV_BYTES, 16);
+                const uint32_t s_t = tS(t), dp_t = tdP(t), sb = s_bar(t), db = dp_bar(t);
+                if (leader) {
 #pragma unroll
-                for (int k = 0; k < HS / 16; ++k) {
-                    mma_issue_f16_tmem_a(tS, tQ + k * 8, DLO(smem_u32(sK) + buf * KV_BYTES, 16, (k / 4) * (BKV * 128) + (k % 4) * 32), kDescHi,
-                                         idesc_s, k > 0);
-                }
+                    for (int k = 0; k < HS / 16; ++k)
+                        mma_issue_f16_tmem_a(s_t, tQ + k * 8, k_lo + (((k / 4) * (BKV * 128) + (k % 4) * 32) >> 4), kDescHi, idesc_s, k > 0);
+                    mma_commit(sb);                              // the exponentials start while dP is still being computed
 #pragma unroll
-                for (int k = 0; k < HS / 16; ++k) {
-                    mma_issue_f16_tmem_a(tdP, tdO + k * 8, DLO(smem_u32(sV) + buf * KV_BYTES, 16, (k / 4) * (BKV * 128) + (k % 4) * 32), kDescHi,
-                                         idesc_s, k > 0);
+                    for (int k = 0; k < HS / 16; ++k)
+                        mma_issue_f16_tmem_a(dp_t, tdO + k * 8, v_lo + (((k / 4) * (BKV * 128) + (k % 4) * 32) >> 4), kDescHi, idesc_s, k > 0);
+                    mma_commit(db);
                 }
-                mma_commit(sp_bar(t));
+                __syncwarp();
                 return true;
             };
-            int g = 0, j = 0;
-            for (int t = 0; t < total && ok; ++t) {
-                // the first tile of a head needs that head's Q / dO in tensor memory
-                if (j == 0 && !mbar_wait(head_ready, g & 1, abort_flag)) { ok = false; break; }
-                ok = issue_sp(t);
-                if (++j == n_kv) { j = 0; ++g; }
-            }
-            if (!ok) { *abort_flag = 1u; atomicOr(p.status, kErrOther); }
-        }
-    } else if (issuer2) {
-        // ============================================================ dQ MMA issuer warp
-        if ((tid & 31) == 0 && total > 0) {
-            const uint32_t idesc_dq = make_instr_desc(1, 1, false, true, BQ, HS);
-            int j = 0;
-            for (int t = 0; t < total && ok; ++t) {
-                if (!mbar_wait(p_ready, t & 1, abort_flag)) { ok = false; break; }
-                tc_fence_after_sync();
-                const int buf = t % NBUF;
+            ok = mbar_wait_warp(head_ready, 0, abort_flag) && issue_sp(0);
+            int t = 0;
+            for (int g = 0; g < nh && ok; ++g) {
+                for (int j = 0; j < n_kv && ok; ++j, ++t) {
+                    if (j + 1 < n_kv && !issue_sp(t + 1)) { ok = false; break; }
+                    if (!mbar_wait_warp(p_ready(t), (t >> 1) & 1, abort_flag)) { ok = false; break; }
+                    // the first dQ MMA of a head overwrites the accumulator: the previous head's must have been read
+                    if (j == 0 && g > 0 && !mbar_wait_warp(dq_drained, (g - 1) & 1, abort_flag)) { ok = false; break; }
+                    tc_fence_after_sync();
+                    const int buf = t % NBUF;
+                    const uint32_t k_lo = desc_lo(smem_u32(sK) + buf * KV_BYTES, BKV * 128), dp_t = tdP(t), bar = kv_free(buf);
+                    const uint32_t acc0 = j > 0;
+                    if (leader) {
 #pragma unroll
-                for (int k = 0; k < BKV / 16; ++k) {
-                    mma_issue<false, false>(tdQ, DLO(smem_u32(sdS), 16, k * 32), kDescHi,
-                                            DLO(smem_u32(sK) + buf * KV_BYTES, BKV * 128, k * (16 * 128)), kDescHi, idesc_dq, (j > 0 || k > 0));
+                        for (int k = 0; k < BKV / 16; ++k)
+                            mma_issue_f16_tmem_a(tdQ, dp_t + k * CW, k_lo + ((k * (16 * 128)) >> 4), kDescHi, idesc_dq, k > 0 ? 1u : acc0);
+                        mma_commit(bar);
+                    }
+                    __syncwarp();
                 }
-                mma_commit(dq_bar);
-                mma_commit(kv_free(buf));
-                if (++j == n_kv) j = 0;
+                if (!ok) break;
+                if (leader) mma_commit(dq_bar);
+                __syncwarp();
+                if (g + 1 < nh) ok = mbar_wait_warp(head_ready, (g + 1) & 1, abort_flag) && issue_sp(t);
             }
-            if (!ok) { *abort_flag = 1u; atomicOr(p.status, kErrOther); }
+            if (!ok && leader) { *abort_flag = 1u; atomicOr(p.status, kErrOther); }
+            __syncwarp();
         }
     } else {
         // ============================================================ compute warps
@@ -552,8 +593,11 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmap_kv64,    // qkv, box
         const int H = p.Hq + 2 * p.Hkv;
         const bool stores_qdo = wg < HS / 32;                   // uniform per warp: the TMEM stores are warp-collective
         constexpr int ECW = HS / kBwdWarpgroups;                // dQ columns per thread
-        // this thread's 32-element slices of the Q and dO rows of head hq (16 packed words each)
-        auto load_qdo = [&](int hq, uint32_t (&wq)[16], uint32_t (&wo)[16]) {
+        // this thread's 32-element slices of the Q and dO rows of head hq (16 packed words each) and its row statistics
+        auto load_qdo = [&](int hq, uint32_t (&wq)[16], uint32_t (&wo)[16], float& lse2, float& delta_s) {
+            const long long si = (static_cast<long long>(b) * p.Hq + hq) * p.T + row;
+            lse2 = row_ok ? p.lse[si] * kLog2e : INFINITY;
+            delta_s = row_ok ? p.delta[si] * p.scale : 0.f;
             if (stores_qdo && row_ok) {
                 const uint4* gq = reinterpret_cast<const uint4*>(p.qkv + ((static_cast<long long>(b) * p.T + row) * H + hq) * HS + wg * 32);
                 const uint4* go = reinterpret_cast<const uint4*>(p.d_out + ((static_cast<long long>(b) * p.T + row) * p.Hq + hq) * HS + wg * 32);
@@ -569,6 +613,7 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmap_kv64,    // qkv, box
             }
         };
         auto store_qdo = [&](const uint32_t (&wq)[16], const uint32_t (&wo)[16]) {
+            __syncwarp();
             if (stores_qdo) {
                 tmem_st_32x32b_x16(tQ + lane_off + wg * 16, wq);
                 tmem_st_32x32b_x16(tdO + lane_off + wg * 16, wo);
@@ -578,351 +623,63 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmap_kv64,    // qkv, box
             warp_arrive(head_ready);
         };
         uint32_t wq[16], wo[16];
-        load_qdo(kvh * G, wq, wo);
+        float lse2, delta_s, lse2_next = 0.f, delta_next = 0.f;
+        load_qdo(h0, wq, wo, lse2, delta_s);
         store_qdo(wq, wo);
-        for (int g = 0; g < G && ok; ++g) {
-            const int h = kvh * G + g;
-            if (g + 1 < G) load_qdo(h + 1, wq, wo);             // prefetch: consumed when this head's walk is over
-            const long long si = (static_cast<long long>(b) * p.Hq + h) * p.T + row;
-            const float lse2 = row_ok ? p.lse[si] * kLog2e : INFINITY;
-            const float delta_s = row_ok ? p.delta[si] * p.scale : 0.f;
-            for (int j = 0; j < n_kv && ok; ++j) {
-                const int t = g * n_kv + j;
-                if (!mbar_wait(sp_bar(t), (t >> 1) & 1, abort_flag)) { ok = false; break; }
+        int t = 0;
+        for (int g = 0; g < nh && ok; ++g) {
+            if (g + 1 < nh) load_qdo(h0 + g + 1, wq, wo, lse2_next, delta_next);     // prefetch: consumed when this head's walk is over
+            for (int j = 0; j < n_kv; ++j, ++t) {
+                if (!mbar_wait(s_bar(t), (t >> 1) & 1, abort_flag)) { ok = false; break; }
                 tc_fence_after_sync();
-                const bool diag = (j + 1) * BKV > q0;
-                const uint32_t tS = tS0 + (t & 1) * BKV, tdP = tdP0 + (t & 1) * BKV;
-                uint32_t dsp[CW / 2];
-                {
-                    uint32_t rs[CW], rp[CW];
-                    tmem_ld_32x32b_x16(tS + lane_off + c0, rs);
-                    tmem_ld_32x32b_x16(tdP + lane_off + c0, rp);
-                    tmem_ld_wait();
-                    tc_fence_before_sync();
-                    warp_arrive(s_free(t & 1));
-                    float pv[CW];
+                uint32_t rv[CW];
+                float pv[CW];
+                __syncwarp();
+                tmem_ld_32x32b_x16(tS(t) + lane_off + c0, rv);
+                tmem_ld_wait();
 #pragma unroll
-                    for (int i = 0; i < CW; ++i) pv[i] = fast_exp2(fmaf(__uint_as_float(rs[i]), sl2, -lse2));
-                    if (diag) {
-                        const int lim = row - j * BKV - c0;     // columns above lim are beyond the diagonal (kv > q)
+                for (int i = 0; i < CW; ++i) pv[i] = fast_exp2(fmaf(__uint_as_float(rv[i]), sl2, -lse2));
+                if ((j + 1) * BKV > q0) {
+                    const int lim = row - j * BKV - c0;         // columns above lim are beyond the diagonal (kv > q)
 #pragma unroll
-                        for (int i = 0; i < CW; ++i) if (i > lim) pv[i] = 0.f;
-                    }
-#pragma unroll
-                    for (int i = 0; i < CW; i += 2)
-                        dsp[i / 2] = pack_bf16x2(pv[i] * fmaf(__uint_as_float(rp[i]), p.scale, -delta_s),
-                                                 pv[i + 1] * fmaf(__uint_as_float(rp[i + 1]), p.scale, -delta_s));
+                    for (int i = 0; i < CW; ++i) if (i > lim) pv[i] = 0.f;
                 }
-                // dS of tile t-1 is read by its dQ MMA until dq_bar completes
-                if (t > 0 && !mbar_wait(dq_bar, (t - 1) & 1, abort_flag)) { ok = false; break; }
-                store_row_chunk16_swz_packed(sdS, r, c0, dsp);
-                fence_proxy_async_smem();
-                warp_arrive(p_ready);
+                if (!mbar_wait(dp_bar(t), (t >> 1) & 1, abort_flag)) { ok = false; break; }
+                tc_fence_after_sync();
+                __syncwarp();
+                tmem_ld_32x32b_x16(tdP(t) + lane_off + c0, rv);
+                tmem_ld_wait();
+                uint32_t dsp[CW / 2];
+#pragma unroll
+                for (int i = 0; i < CW; i += 2)
+                    dsp[i / 2] = pack_bf16x2(pv[i] * fmaf(__uint_as_float(rv[i]), p.scale, -delta_s),
+                                             pv[i + 1] * fmaf(__uint_as_float(rv[i + 1]), p.scale, -delta_s));
+                // into the first half of the columns this thread has just read: one K step of 16 keys per warpgroup
+                tmem_st_32x32b_x8(tdP(t) + lane_off + c0, dsp);
+                tmem_st_wait();
+                tc_fence_before_sync();
+                warp_arrive(p_ready(t));
             }
             if (!ok) break;
-            // ---- the head's walk is over: drain dQ, hand the next head's Q / dO to the tensor core, then store
-            if (!mbar_wait(dq_bar, (g * n_kv + n_kv - 1) & 1, abort_flag)) { ok = false; break; }
+            // ---- the head's walk is over.  Its last dP tile is complete, so every MMA that reads Q / dO is: hand over the
+            // next head's, then drain dQ while the tensor core works on the next head's first scores.
+            if (g + 1 < nh) { store_qdo(wq, wo); lse2 = lse2_next; delta_s = delta_next; }
+            if (!mbar_wait(dq_bar, g & 1, abort_flag)) { ok = false; break; }
             tc_fence_after_sync();
             uint32_t acc[ECW];
             __syncwarp();
 #pragma unroll
             for (int c = 0; c < ECW; c += 16) tmem_ld_32x32b_x16(tdQ + lane_off + wg * ECW + c, *reinterpret_cast<uint32_t(*)[16]>(acc + c));
             tmem_ld_wait();
-            if (g + 1 < G) store_qdo(wq, wo);
+            tc_fence_before_sync();
+            warp_arrive(dq_drained);
             if (row_ok) {
-                bf16* dq = p.dqkv + ((static_cast<long long>(b) * p.T + row) * H + h) * HS + wg * ECW;
+                bf16* dq = p.dqkv + ((static_cast<long long>(b) * p.T + row) * H + h0 + g) * HS + wg * ECW;
 #pragma unroll
                 for (int c = 0; c < ECW; c += 16) store16_bf16(dq + c, *reinterpret_cast<const uint32_t(*)[16]>(acc + c));
             }
         }
         if (!ok && r == 0) atomicOr(p.status, kErrOther);
-    }
-    tc_fence_before_sync();
-    __syncthreads();
-    tc_fence_after_sync();
-    if (issuer) tmem_dealloc(tmem, TMEM_COLS);
-}
-
-// ------------------------------------------------------------------------------------------------
-// Forward.  Same organisation as the dQ kernel: one CTA owns 128 query rows of one kv head and walks over the query
-// heads of the group and, per head, over the 64-key tiles up to the diagonal.  Q lives in tensor memory as the A
-// operand of S = Q K^T; the bf16 probabilities go back into tensor memory (two buffers) and are the A operand of
-// O += P V, so neither Q nor P is ever re-read from shared memory; K / V stream through a ring of four buffers.
-// Four threads share a row (16 score columns each): the row maximum is exchanged through shared memory once per
-// tile, the row sum only at the end of a head.  O is rescaled only when a row maximum moved by more than 2^8 since
-// the last rescale (the stale maximum keeps P <= 256, exact after the final normalisation).
-template <int N> __device__ __forceinline__ void tmem_ld_cols(uint32_t addr, uint32_t (&r)[N]) {
-    if constexpr (N == 32) tmem_ld_32x32b_x32(addr, r); else tmem_ld_32x32b_x16(addr, r);
-}
-template <int N> __device__ __forceinline__ void tmem_st_cols(uint32_t addr, const uint32_t (&r)[N]) {
-    if constexpr (N == 32) tmem_st_32x32b_x32(addr, r); else tmem_st_32x32b_x16(addr, r);
-}
-
-template <int HS>
-__global__ void __launch_bounds__(kBwdThreads, 1)
-attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_kv64,    // qkv, box 64 rows
-                const AttnParams p) {
-    constexpr int BQ = 128, BKV = 64, NCH = HS / 64, NBUF = 4;
-    constexpr int KV_BYTES = BKV * HS * 2;
-    constexpr uint32_t TMEM_COLS = 512;                       // Q | S0 S1 | P0 P1 (bf16 pairs) | O
-    constexpr int CW = BKV / kBwdWarpgroups;                  // score columns per thread
-    constexpr int ECW = HS / kBwdWarpgroups;                  // output columns per thread
-    constexpr float kRescaleThreshold = 8.f;                  // in log2 units
-    static_assert(CW == 16, "the column split below is written for 16 columns per thread");
-    extern __shared__ __align__(1024) uint8_t smem[];
-    uint8_t* sK = smem;                       // NBUF buffers
-    uint8_t* sV = sK + NBUF * KV_BYTES;       // NBUF buffers
-    float* sMax = reinterpret_cast<float*>(sV + NBUF * KV_BYTES);     // [2][4][128] slice maxima of a tile
-    float* sSum = sMax + 2 * kBwdWarpgroups * BQ;                      // [4][128] slice sums of a head
-    uint64_t* bars = reinterpret_cast<uint64_t*>(sSum + kBwdWarpgroups * BQ);
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 20);
-    volatile uint32_t* abort_flag = tmem_slot + 1;
-
-    const int tid = threadIdx.x, warp = tid >> 5;
-    const bool issuer = warp == kBwdComputeWarps, producer = warp == kBwdComputeWarps + 1, issuer2 = warp == kBwdComputeWarps + 2;
-    const int wg = tid >> 7, r = tid & 127;
-    if (smem_u32(smem) & 1023u) { if (tid == 0) atomicOr(p.status, kErrOther); return; }
-    const int nqb = (p.T + BQ - 1) / BQ;
-    const int qb = nqb - 1 - blockIdx.x / (p.Hkv * p.B);        // 1-D grid, longest key walks first
-    const int kvh = (blockIdx.x % (p.Hkv * p.B)) % p.Hkv, b = (blockIdx.x % (p.Hkv * p.B)) / p.Hkv;
-    const int G = p.Hq / p.Hkv;
-    const int q0 = qb * BQ;
-    const int n_kv = min((p.T + BKV - 1) / BKV, (q0 + BQ) / BKV);
-    const int total = n_kv * G;                                 // tiles of the whole walk, t = g * n_kv + j
-    const int kcol = (p.Hq + kvh) * HS, vcol = (p.Hq + p.Hkv + kvh) * HS;
-
-    // barriers: 0 head_ready | 1-4 k/v ring | 5-6 s (scores ready) | 7-8 s_free | 9-10 p_ready | 11-12 p_free (PV of the
-    //           tile done) | 13-16 k/v buffer free.  Two-entry sets alternate with the tile parity.
-    const uint32_t bar0 = smem_u32(bars);
-    const uint32_t head_ready = bar0;
-    auto kv_bar = [&](int buf) { return bar0 + 8 + 8 * buf; };
-    auto s_bar = [&](int t) { return bar0 + 40 + 8 * (t & 1); };
-    auto s_free = [&](int t) { return bar0 + 56 + 8 * (t & 1); };
-    auto p_ready = [&](int t) { return bar0 + 72 + 8 * (t & 1); };
-    auto p_free = [&](int t) { return bar0 + 88 + 8 * (t & 1); };
-    auto kv_free = [&](int buf) { return bar0 + 104 + 8 * buf; };
-    if (tid == 0) {
-        mbar_init(head_ready, kBwdComputeWarps);
-        for (int i = 0; i < 4; ++i) { mbar_init(kv_bar(i), 1); mbar_init(kv_free(i), 1); }
-        for (int i = 0; i < 2; ++i) {
-            mbar_init(s_bar(i), 1); mbar_init(p_free(i), 1);
-            mbar_init(s_free(i), kBwdComputeWarps); mbar_init(p_ready(i), kBwdComputeWarps);
-        }
-        *abort_flag = 0;
-        mbar_init_fence();
-    }
-    if (issuer) { tmem_alloc(smem_u32(tmem_slot), TMEM_COLS); tmem_relinquish(); }
-    tc_fence_before_sync();
-    __syncthreads();
-    tc_fence_after_sync();
-    const uint32_t tmem = *tmem_slot;
-    const uint32_t tQ = tmem, tS0 = tmem + HS / 2, tP0 = tS0 + 2 * BKV, tO = tP0 + BKV;
-    const uint32_t lane_off = static_cast<uint32_t>((warp & 3) * 32) << 16;
-    bool ok = true;
-
-    if (producer) {
-        // ============================================================ TMA producer warp
-        if ((tid & 31) == 0 && total > 0) {
-            tma_prefetch_desc(&tmap_kv64);
-            int j = 0;
-            for (int t = 0; t < total; ++t) {
-                const int buf = t % NBUF;
-                if (t >= NBUF && !mbar_wait(kv_free(buf), ((t / NBUF) - 1) & 1, abort_flag)) { atomicOr(p.status, kErrOther); break; }
-                mbar_expect_tx(kv_bar(buf), 2 * KV_BYTES);
-                for (int c = 0; c < NCH; ++c) {
-                    tma_load_3d(smem_u32(sK) + buf * KV_BYTES + c * (BKV * 128), &tmap_kv64, kv_bar(buf), kcol + c * 64, j * BKV, b);
-                    tma_load_3d(smem_u32(sV) + buf * KV_BYTES + c * (BKV * 128), &tmap_kv64, kv_bar(buf), vcol + c * 64, j * BKV, b);
-                }
-                if (++j == n_kv) j = 0;
-            }
-        }
-    } else if (issuer) {
-        // ============================================================ S = Q K^T issuer warp
-        if ((tid & 31) == 0 && total > 0) {
-            const uint32_t idesc_s = make_instr_desc(1, 1, false, false, BQ, BKV);
-            int g = 0, j = 0;
-            for (int t = 0; t < total && ok; ++t) {
-                const int buf = t % NBUF;
-                if (j == 0 && !mbar_wait(head_ready, g & 1, abort_flag)) { ok = false; break; }       // this head's Q is in tensor memory
-                if (!mbar_wait(kv_bar(buf), (t / NBUF) & 1, abort_flag)) { ok = false; break; }
-                if (t >= 2 && !mbar_wait(s_free(t), ((t - 2) >> 1) & 1, abort_flag)) { ok = false; break; }
-                tc_fence_after_sync();
-#pragma unroll
-                for (int k = 0; k < HS / 16; ++k) {
-                    mma_issue_f16_tmem_a(tS0 + (t & 1) * BKV, tQ + k * 8,
-                                         DLO(smem_u32(sK) + buf * KV_BYTES, 16, (k / 4) * (BKV * 128) + (k % 4) * 32), kDescHi, idesc_s, k > 0);
-                }
-                mma_commit(s_bar(t));
-                if (++j == n_kv) { j = 0; ++g; }
-            }
-            if (!ok) { *abort_flag = 1u; atomicOr(p.status, kErrOther); }
-        }
-    } else if (issuer2) {
-        // ============================================================ O += P V issuer warp
-        if ((tid & 31) == 0 && total > 0) {
-            const uint32_t idesc_o = make_instr_desc(1, 1, false, true, BQ, HS);
-            int j = 0;
-            for (int t = 0; t < total && ok; ++t) {
-                if (!mbar_wait(p_ready(t), (t >> 1) & 1, abort_flag)) { ok = false; break; }
-                tc_fence_after_sync();
-                const int buf = t % NBUF;
-#pragma unroll
-                for (int k = 0; k < BKV / 16; ++k) {
-                    mma_issue_f16_tmem_a(tO, tP0 + (t & 1) * (BKV / 2) + k * 8,
-                                         DLO(smem_u32(sV) + buf * KV_BYTES, BKV * 128, k * (16 * 128)), kDescHi, idesc_o, (j > 0 || k > 0));
-                }
-                mma_commit(p_free(t));
-                mma_commit(kv_free(buf));
-                if (++j == n_kv) j = 0;
-            }
-            if (!ok) { *abort_flag = 1u; atomicOr(p.status, kErrOther); }
-        }
-    } else {
-        // ============================================================ compute warps
-        const float sl2 = p.scale * kLog2e;
-        const int row = q0 + r;
-        const bool row_ok = row < p.T;
-        const int c0 = wg * CW;
-        const int H = p.Hq + 2 * p.Hkv;
-        const bool stores_q = wg < HS / 32;                     // uniform per warp: the TMEM stores are warp-collective
-        auto load_q = [&](int hq, uint32_t (&wq)[16]) {
-            if (stores_q && row_ok) {
-                const uint4* gq = reinterpret_cast<const uint4*>(p.qkv + ((static_cast<long long>(b) * p.T + row) * H + hq) * HS + wg * 32);
-#pragma unroll
-                for (int q4 = 0; q4 < 4; ++q4) {
-                    const uint4 x = __ldg(gq + q4);
-                    wq[4 * q4] = x.x; wq[4 * q4 + 1] = x.y; wq[4 * q4 + 2] = x.z; wq[4 * q4 + 3] = x.w;
-                }
-            } else {
-#pragma unroll
-                for (int q4 = 0; q4 < 16; ++q4) wq[q4] = 0u;
-            }
-        };
-        auto store_q = [&](const uint32_t (&wq)[16]) {
-            if (stores_q) { tmem_st_32x32b_x16(tQ + lane_off + wg * 16, wq); tmem_st_wait(); }
-            tc_fence_before_sync();
-            warp_arrive(head_ready);
-        };
-        uint32_t wq[16];
-        load_q(kvh * G, wq);
-        store_q(wq);
-        float m_ref = -INFINITY, l_part = 0.f, omax = 0.f;
-        for (int g = 0; g < G; ++g) {
-            const int h = kvh * G + g;
-            if (g + 1 < G) load_q(h + 1, wq);                   // prefetch: consumed when this head's walk is over
-            m_ref = -INFINITY; l_part = 0.f;
-            for (int j = 0; j < n_kv; ++j) {
-                const int t = g * n_kv + j;
-                float sv[CW];
-                // ---- scores of this thread's 16 columns, masked; slice maximum to shared memory
-                if (ok) {
-                    ok = mbar_wait(s_bar(t), (t >> 1) & 1, abort_flag);
-                    if (ok) {
-                        tc_fence_after_sync();
-                        uint32_t rs[CW];
-                        tmem_ld_32x32b_x16(tS0 + (t & 1) * BKV + lane_off + c0, rs);
-                        tmem_ld_wait();
-                        tc_fence_before_sync();
-                        warp_arrive(s_free(t));
-#pragma unroll
-                        for (int i = 0; i < CW; ++i) sv[i] = __uint_as_float(rs[i]);
-                        if ((j + 1) * BKV > q0) {               // tile touches the diagonal
-                            const int lim = row - j * BKV - c0; // columns above lim are beyond the diagonal (kv > q)
-#pragma unroll
-                            for (int i = 0; i < CW; ++i) if (i > lim) sv[i] = -INFINITY;
-                        }
-                        float mx = sv[0];
-#pragma unroll
-                        for (int i = 1; i < CW; ++i) mx = fmaxf(mx, sv[i]);
-                        sMax[((t & 1) * kBwdWarpgroups + wg) * BQ + r] = mx;
-                    }
-                }
-                row_group_barrier(warp & 3);                              // every thread takes part, also after a failed wait
-                if (!ok) continue;
-                float m_tile = -INFINITY;
-#pragma unroll
-                for (int w4 = 0; w4 < kBwdWarpgroups; ++w4) m_tile = fmaxf(m_tile, sMax[((t & 1) * kBwdWarpgroups + w4) * BQ + r]);
-                // ---- lazy rescale.  The TMEM loads / stores are warp-collective, so the decision is taken per warp; the
-                // four warps that share rows see the same numbers and therefore decide alike.
-                const bool need = j == 0 || (m_tile - m_ref) * sl2 > kRescaleThreshold;
-                if (__any_sync(0xffffffffu, need)) {
-                    const float m_new = fmaxf(m_ref, m_tile);
-                    if (j > 0) {
-                        const float alpha = fast_exp2((m_ref - m_new) * sl2);
-                        l_part *= alpha;
-                        // O is being accumulated by the PV MMAs of tile t-1: wait for them, then scale this thread's columns
-                        if (!mbar_wait(p_free(t - 1), ((t - 1) >> 1) & 1, abort_flag)) { ok = false; continue; }
-                        tc_fence_after_sync();
-                        uint32_t ro[ECW];
-                        tmem_ld_cols<ECW>(tO + lane_off + wg * ECW, ro);
-                        tmem_ld_wait();
-#pragma unroll
-                        for (int i = 0; i < ECW; ++i) ro[i] = __float_as_uint(__uint_as_float(ro[i]) * alpha);
-                        tmem_st_cols<ECW>(tO + lane_off + wg * ECW, ro);
-                        tmem_st_wait();
-                    }
-                    m_ref = m_new;
-                }
-                // ---- probabilities -> bf16 -> tensor memory (A operand of the PV MMA)
-                const float moff = m_ref * sl2;
-                uint32_t pw[CW / 2];
-                float sum = 0.f;
-#pragma unroll
-                for (int i = 0; i < CW; i += 2) {
-                    const float p0 = fast_exp2(fmaf(sv[i], sl2, -moff)), p1 = fast_exp2(fmaf(sv[i + 1], sl2, -moff));
-                    sum += p0 + p1;
-                    pw[i / 2] = pack_bf16x2(p0, p1);
-                }
-                l_part += sum;
-                // this P buffer was read by the PV MMAs of tile t-2
-                if (t >= 2 && !mbar_wait(p_free(t), ((t - 2) >> 1) & 1, abort_flag)) { ok = false; continue; }
-                tc_fence_after_sync();
-                __syncwarp();
-                tmem_st_32x32b_x8(tP0 + (t & 1) * (BKV / 2) + lane_off + wg * (CW / 2), pw);
-                tmem_st_wait();
-                tc_fence_before_sync();
-                warp_arrive(p_ready(t));
-            }
-            // ---- the head's walk is over: row sums, normalise, store; hand the next head's Q to the tensor core
-            const int t_last = g * n_kv + n_kv - 1;
-            if (ok) ok = mbar_wait(p_free(t_last), (t_last >> 1) & 1, abort_flag);
-            tc_fence_after_sync();
-            sSum[wg * BQ + r] = l_part;
-            row_group_barrier(warp & 3);
-            if (ok) {
-                float l = 0.f;
-#pragma unroll
-                for (int w4 = 0; w4 < kBwdWarpgroups; ++w4) l += sSum[w4 * BQ + r];
-                const float inv = 1.f / l;
-                uint32_t ro[ECW];
-                __syncwarp();
-                tmem_ld_cols<ECW>(tO + lane_off + wg * ECW, ro);
-                tmem_ld_wait();
-                if (g + 1 < G) store_q(wq);
-                if (row_ok) {
-                    bf16* o = p.out + ((static_cast<long long>(b) * p.T + row) * p.Hq + h) * HS + wg * ECW;
-#pragma unroll
-                    for (int c = 0; c < ECW; c += 8) {
-                        uint4 v;
-                        __nv_bfloat162* vb = reinterpret_cast<__nv_bfloat162*>(&v);
-#pragma unroll
-                        for (int jj = 0; jj < 4; ++jj) {
-                            vb[jj] = __floats2bfloat162_rn(__uint_as_float(ro[c + 2 * jj]) * inv, __uint_as_float(ro[c + 2 * jj + 1]) * inv);
-                            const float2 f = __bfloat1622float2(vb[jj]);
-                            omax = fmaxf(omax, fmaxf(fabsf(f.x), fabsf(f.y)));
-                        }
-                        *reinterpret_cast<uint4*>(o + c) = v;
-                    }
-                    if (wg == 0) p.lse[(static_cast<long long>(b) * p.Hq + h) * p.T + row] = m_ref * p.scale + logf(l);
-                }
-            }
-            row_group_barrier(warp & 3);                                  // sSum is reused by the next head
-        }
-        if (!ok && r == 0) atomicOr(p.status, kErrOther);
-        if (p.absmax) {
-            omax = warp_reduce_max(omax);
-            if ((tid & 31) == 0 && omax > 0.f) atomic_max_float(p.absmax, omax);
-        }
     }
     tc_fence_before_sync();
     __syncthreads();
@@ -944,21 +701,28 @@ int set_smem(K kernel, int bytes) {
     return 0;
 }
 
-template <int HS>
-int fwd_impl(void* out, float* lse, const void* qkv, int B, int T, int Hq, int Hkv, float* absmax, unsigned int* status, cudaStream_t s) {
-    const int H = Hq + 2 * Hkv;
-    CUtensorMap tkv;
-    int rc = encode_btw(&tkv, qkv, B, T, static_cast<long long>(H) * HS, 64);
-    if (rc) return rc;
-    constexpr int smem = 8 * 64 * HS * 2 + 3 * kBwdWarpgroups * 128 * 4 + 256;
-    rc = set_smem<HS>(attn_fwd_kernel<HS>, smem);
-    if (rc) return rc;
-    AttnParams p{};
-    p.B = B; p.T = T; p.Hq = Hq; p.Hkv = Hkv; p.scale = 1.f / sqrtf(static_cast<float>(HS));
-    p.out = static_cast<bf16*>(out); p.lse = lse; p.status = status; p.qkv = static_cast<const bf16*>(qkv); p.absmax = absmax;
-    dim3 grid(((T + 127) / 128) * Hkv * B, 1, 1);
-    attn_fwd_kernel<HS><<<grid, kBwdThreads, smem, s>>>(tkv, p);
-    return LLMQ_LAUNCH_CHECK();
+int device_sms() {
+    static int sms[64] = {};
+    int dev = 0;
+    cudaGetDevice(&dev);
+    if (!sms[dev & 63]) cudaDeviceGetAttribute(&sms[dev & 63], cudaDevAttrMultiProcessorCount, dev);
+    return sms[dev & 63] > 0 ? sms[dev & 63] : 148;
+}
+
+// Query heads of a group that one CTA walks over; `base` = (row block, kv head, batch) items.  A CTA that walks a whole group pays
+// its start-up once and loads K / V (or keeps them) for all heads, but few items leave SMs idle: the group is cut into the fewest
+// parts that give 1.5 CTAs per SM, where the longest-first order evens the walks out.  Measured, kernel times in us (parts 1 / 2 / 3 /
+// 4 / 7):  dQ, 8 x 1024 tokens, 14 / 2 heads of 64 (128 items) 81 / 56 / 57 / 59 / 70;  4 x 1024 (64 items) 81 / 48 / 37 / 31 / 38;
+// 4 x 512 (32 items) 50 / 30 / 23 / 17 / 16;  8 x 2048, 28 / 4 heads of 128 (512 items) 398 / 390 / 407 / 415 / 494.
+// dK / dV, the same four: 87 / 64 / 86 / 84 / 155,  85 / 56 / 46 / 43 / 84,  48 / 32 / 26 / 19 / 41,  427 / 516 / 697 / 687 / 1216: its
+// parts are the CTAs of a cluster that meet at the end, and clusters of more than four no longer pack into a GPC's SMs.
+int heads_per_cta(int G, int base, int max_parts) {
+    int heads = G;
+    for (int parts = 1; parts <= G && parts <= max_parts; ++parts) {
+        heads = (G + parts - 1) / parts;
+        if (2 * base * ((G + heads - 1) / heads) >= 3 * device_sms()) break;
+    }
+    return heads;
 }
 
 template <int HS>
@@ -972,31 +736,37 @@ int bwd_impl(void* dqkv, float* delta, const void* d_out, const void* out, const
         int rc = LLMQ_LAUNCH_CHECK();
         if (rc) return rc;
     }
-    CUtensorMap t128, t64, tdo128, tdo64;
+    CUtensorMap t128, t64, tdo64;
     int rc = encode_btw(&t128, qkv, B, T, static_cast<long long>(H) * HS, 128);
     if (!rc) rc = encode_btw(&t64, qkv, B, T, static_cast<long long>(H) * HS, 64);
-    if (!rc) rc = encode_btw(&tdo128, d_out, B, T, static_cast<long long>(Hq) * HS, 128);
     if (!rc) rc = encode_btw(&tdo64, d_out, B, T, static_cast<long long>(Hq) * HS, 64);
     if (rc) return rc;
     AttnParams p{};
     p.B = B; p.T = T; p.Hq = Hq; p.Hkv = Hkv; p.scale = 1.f / sqrtf(static_cast<float>(HS));
     p.lse = const_cast<float*>(lse); p.delta = delta; p.dqkv = static_cast<bf16*>(dqkv); p.status = status;
     p.qkv = static_cast<const bf16*>(qkv); p.d_out = static_cast<const bf16*>(d_out);
+    const int base = ((T + 127) / 128) * Hkv * B, G = Hq / Hkv;
     {
-        constexpr int smem = 2 * 128 * HS * 2 + 8 * 64 * HS * 2 + 2 * 128 * 64 * 2 + 4 * 64 * 4 + 256;
+        constexpr int smem = 2 * 128 * HS * 2 + 8 * 64 * HS * 2 + 8 * 64 * 4 + 256;
         rc = set_smem<1000 + HS>(attn_bwd_dkdv_kernel<HS>, smem);
         if (rc) return rc;
-        dim3 grid(((T + 127) / 128) * Hkv * B, 1, 1);
-        attn_bwd_dkdv_kernel<HS><<<grid, kBwdThreads, smem, s>>>(t128, t64, tdo64, p);
-        rc = LLMQ_LAUNCH_CHECK();
+        const int heads = heads_per_cta(G, base, 4), parts = (G + heads - 1) / heads;
+        cudaLaunchConfig_t cfg{};
+        cfg.gridDim = dim3(base * parts); cfg.blockDim = dim3(kBwdThreads); cfg.dynamicSmemBytes = smem; cfg.stream = s;
+        cudaLaunchAttribute attr{};
+        attr.id = cudaLaunchAttributeClusterDimension;
+        attr.val.clusterDim.x = parts; attr.val.clusterDim.y = 1; attr.val.clusterDim.z = 1;
+        cfg.attrs = &attr; cfg.numAttrs = parts > 1 ? 1 : 0;
+        const cudaError_t e = cudaLaunchKernelEx(&cfg, attn_bwd_dkdv_kernel<HS>, t128, t64, tdo64, p, heads);
+        rc = e == cudaSuccess ? LLMQ_LAUNCH_CHECK() : static_cast<int>(e);
         if (rc) return rc;
     }
     {
-        constexpr int smem = 8 * 64 * HS * 2 + 128 * 64 * 2 + 256;
+        constexpr int smem = 8 * 64 * HS * 2 + 256;
         rc = set_smem<2000 + HS>(attn_bwd_dq_kernel<HS>, smem);
         if (rc) return rc;
-        dim3 grid(((T + 127) / 128) * Hkv * B, 1, 1);
-        attn_bwd_dq_kernel<HS><<<grid, kBwdThreads, smem, s>>>(t64, p);
+        const int heads = heads_per_cta(G, base, G);
+        attn_bwd_dq_kernel<HS><<<base * ((G + heads - 1) / heads), kBwdThreads, smem, s>>>(t64, p, heads);
         rc = LLMQ_LAUNCH_CHECK();
     }
     return rc;
@@ -1004,7 +774,7 @@ int bwd_impl(void* dqkv, float* delta, const void* d_out, const void* out, const
 
 }  // namespace
 
-int llmq_attention_forward_pingpong(void* out, float* lse, const void* qkv, int B, int T, int Hq, int Hkv, float* absmax,
+int llmq_attention_forward_pingpong(void* out, float* lse, const void* qkv, int B, int T, int Hq, int Hkv, int HS, float* absmax,
                                     unsigned int* status, cudaStream_t s);
 
 // qkv (B,T,Hq+2Hkv,HS) bf16 -> out (B,T,Hq,HS) bf16, lse (B,Hq,T) fp32.  HS in {64, 128}.
@@ -1013,14 +783,7 @@ extern "C" int llmq_attention_forward(void* out, float* lse, const void* qkv, in
                                       float* absmax, unsigned int* status, cudaStream_t s) {
     if (B <= 0 || T <= 0) return 0;
     if (Hq % Hkv) return -1;
-    if (HS == 64) return fwd_impl<64>(out, lse, qkv, B, T, Hq, Hkv, absmax, status, s);
-    if (HS == 128) {
-        // two query tiles per CTA, processed alternately (attention_fwd_pingpong.cu); LLMQ_ATTN_FWD_SINGLE=1 keeps the
-        // one-tile kernel of this file for comparisons
-        static const bool single = [] { const char* e = getenv("LLMQ_ATTN_FWD_SINGLE"); return e && e[0] == '1'; }();
-        if (!single) return llmq_attention_forward_pingpong(out, lse, qkv, B, T, Hq, Hkv, absmax, status, s);
-        return fwd_impl<128>(out, lse, qkv, B, T, Hq, Hkv, absmax, status, s);
-    }
+    if (HS == 64 || HS == 128) return llmq_attention_forward_pingpong(out, lse, qkv, B, T, Hq, Hkv, HS, absmax, status, s);
     return -2;
 }
 
