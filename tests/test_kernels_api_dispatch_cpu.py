@@ -1,0 +1,104 @@
+"""The custom ops of ``llmq_b200.kernels_api`` called directly against the same calls through ``torch.ops``: a plain eager call
+skips the dispatcher, every call that somebody watches or that the schema would refuse does not."""
+import pytest
+import torch
+from torch.utils._python_dispatch import TorchDispatchMode
+
+import llmq_b200.kernels_api as ops
+
+BF = torch.bfloat16
+
+
+def _norm_args(dtype=BF):
+    g = torch.Generator().manual_seed(0)
+    x, w = torch.randn(4, 64, generator=g).to(dtype), torch.randn(64, generator=g).to(dtype)
+    return torch.zeros_like(x), torch.zeros(4), x, w, torch.zeros(1), 1e-6
+
+
+def test_plain_call_equals_the_registered_op_and_bumps_versions():
+    a, b = _norm_args(), _norm_args()
+    before = [t._version for t in a[:5]]
+    assert ops.rmsnorm_forward(*a) is None
+    torch.ops.llmq_b200.rmsnorm_forward(*b)
+    for x, y in zip(a[:5], b[:5]):
+        assert torch.equal(x, y)
+    bumped = [t._version - v > 0 for t, v in zip(a[:5], before)]
+    assert bumped == [True, True, False, False, True]
+    c = torch.zeros(3, 4)
+    ops.matmul(c, torch.ones(3, 2), torch.ones(4, 2), None, None, None, None)          # defaults: mode "TN", no accumulation
+    assert torch.equal(c, torch.full((3, 4), 2.0))
+
+
+def test_watched_calls_take_the_dispatcher():
+    seen = []
+
+    class Mode(TorchDispatchMode):
+        def __torch_dispatch__(self, func, types, args=(), kwargs=None):
+            seen.append(str(func))
+            return func(*args, **(kwargs or {}))
+
+    with Mode():
+        ops.rmsnorm_forward(*_norm_args())
+    assert any("llmq_b200.rmsnorm_forward" in s for s in seen)
+    with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CPU]) as prof:
+        ops.rmsnorm_forward(*_norm_args())
+    assert any("llmq_b200::rmsnorm_forward" in e.key for e in prof.key_averages())
+    a = _norm_args()
+    gm = torch.fx.experimental.proxy_tensor.make_fx(lambda x: ops.rmsnorm_forward(a[0], a[1], x, a[3], None, 1e-6))(a[2])
+    assert "llmq_b200.rmsnorm_forward" in gm.code
+
+
+@pytest.mark.parametrize("call", ["grad", "dual", "vmap", "meta", "type", "missing", "inference"])
+def test_calls_outside_the_plain_case_do_what_the_registered_op_does(call):
+    def outcome(op):
+        a = list(_norm_args(torch.float32))
+        try:
+            if call == "grad":
+                a[2].requires_grad_(True)
+                op(*a)
+                a[0].sum().backward()
+            elif call == "dual":
+                with torch.autograd.forward_ad.dual_level():
+                    a[2] = torch.autograd.forward_ad.make_dual(a[2], torch.ones_like(a[2]))
+                    op(*a)
+            elif call == "vmap":
+                torch.func.vmap(lambda x: op(a[0], a[1], x, a[3], None, 1e-6))(torch.stack([a[2], a[2]]))
+            elif call == "meta":
+                op(*[t.to("meta") if isinstance(t, torch.Tensor) else t for t in a])
+            elif call == "type":
+                op(*a[:5], "1e-6")
+            elif call == "missing":
+                op(*a[:4])
+            else:
+                with torch.inference_mode():
+                    a = list(_norm_args(torch.float32))
+                    op(*a)
+            return "ok", a[0].detach().clone() if a[0].device.type == "cpu" else None
+        except Exception as e:                           # noqa: BLE001 - the kind of refusal is what is compared
+            return type(e).__name__, None
+
+    got, want = outcome(ops.rmsnorm_forward), outcome(torch.ops.llmq_b200.rmsnorm_forward.default)
+    assert got[0] == want[0], (got, want)
+    if want[1] is not None:
+        assert torch.equal(got[1], want[1])
+
+
+def test_an_integer_for_a_float_and_keywords_are_still_accepted():
+    a, b = _norm_args(), _norm_args()
+    ops.rmsnorm_forward(*a[:5], 1)
+    ops.rmsnorm_forward(out=b[0], rms=b[1], inp=b[2], weight=b[3], absmax=b[4], epsilon=1.0)
+    assert torch.equal(a[0], b[0])
+
+
+def test_a_kernel_registered_later_is_used():
+    calls = []
+    op = ops.grouped_loss_sum
+    out, losses = torch.zeros(1), torch.ones(1, 8)
+    op(out, losses)
+    assert out.item() == 8 and isinstance(op, torch._library.custom_ops.CustomOpDef)
+    try:
+        op.register_kernel("cpu")(lambda out, per_token_loss: calls.append(1))
+        op(out, losses)
+        assert calls == [1]
+    finally:
+        op.register_kernel("cpu")(lambda out, per_token_loss: ops.K.grouped_loss_sum(out, per_token_loss))
