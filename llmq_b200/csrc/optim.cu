@@ -80,6 +80,75 @@ template <> __device__ __forceinline__ void store8_srw<float>(float* p, const fl
 // bf16 state (950 MB) from 193 to 166-182 us.  For e4m3 first moments 16 consecutive threads share one
 // fp32 scale (128 elements); the scale is recomputed from the new values every step.
 template <typename P, typename G, typename M, typename Vv>
+__device__ __forceinline__ void adamw_vec(long long i, bool active, P* __restrict__ param, const G* __restrict__ grad, M* __restrict__ m_state,
+                                          Vv* __restrict__ v_state, float* __restrict__ m_scales, float lr, float beta1, float beta2, float bc1,
+                                          float bc2, float eps, float wd, float gs, uint32_t seed, long long elem_offset, float& tmax) {
+    const long long e = i * 8;
+    float p[8], g[8], m[8], v[8];
+    if (active) {
+        load8<P>(p, param + e);
+        load8<G>(g, grad + e);
+        load8<Vv>(v, v_state + e);
+        load8<M>(m, m_state + e);
+        if constexpr (sizeof(M) == 1) {
+            float sc = m_scales[e / 128];
+#pragma unroll
+            for (int k = 0; k < 8; ++k) m[k] *= sc;
+        }
+    } else {
+#pragma unroll
+        for (int k = 0; k < 8; ++k) { p[k] = g[k] = m[k] = v[k] = 0.f; }
+    }
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+        float gk = g[k] * gs;
+        m[k] = beta1 * m[k] + (1.f - beta1) * gk;
+        v[k] = beta2 * v[k] + (1.f - beta2) * gk * gk;
+        float mh = m[k] * bc1, vh = v[k] * bc2;
+        p[k] -= lr * (__fdividef(mh, sqrt_approx(vh) + eps) + wd * p[k]);
+    }
+    const uint64_t ctr = static_cast<uint64_t>(e + elem_offset);
+    const SrWords words(ctr, seed);
+    if constexpr (sizeof(M) == 1) {
+        float am = 0.f;
+#pragma unroll
+        for (int k = 0; k < 8; ++k) am = fmaxf(am, fabsf(m[k]));
+#pragma unroll
+        for (int o = 8; o > 0; o >>= 1) am = fmaxf(am, __shfl_xor_sync(0xffffffffu, am, o));
+        float sc = fmaxf(am, 1e-30f) / 448.f;
+        if (active) {
+            alignas(8) e4m3 q[8];
+            float inv = 1.f / sc;
+#pragma unroll
+            for (int k = 0; k < 8; k += 2) {
+                q[k] = sr_e4m3(m[k] * inv, words.get(4 + k));
+                q[k + 1] = sr_e4m3(m[k + 1] * inv, words.get(5 + k));
+            }
+            *reinterpret_cast<uint2*>(m_state + e) = *reinterpret_cast<uint2*>(q);
+            if ((i & 15) == 0) m_scales[e / 128] = sc;
+        }
+    } else {
+        if (active) store8_srw<M>(m_state + e, m, words, 4);
+    }
+    if (active) {
+        store8_srw<Vv>(v_state + e, v, words, 12);
+        if constexpr (sizeof(P) == 2) {
+            uint32_t o[4];
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                o[k] = sr_bf16x2(p[2 * k], p[2 * k + 1], words.get(k));
+                tmax = fmaxf(tmax, fmaxf(fabsf(__uint_as_float(o[k] << 16)), fabsf(__uint_as_float(o[k] & 0xFFFF0000u))));
+            }
+            *reinterpret_cast<uint4*>(reinterpret_cast<bf16*>(param) + e) = make_uint4(o[0], o[1], o[2], o[3]);
+        } else {
+            store8_srw<float>(reinterpret_cast<float*>(param) + e, p, words, 0);
+#pragma unroll
+            for (int k = 0; k < 8; ++k) tmax = fmaxf(tmax, fabsf(p[k]));
+        }
+    }
+}
+
+template <typename P, typename G, typename M, typename Vv>
 __global__ void __launch_bounds__(256)
 adamw_kernel(P* __restrict__ param, const G* __restrict__ grad, M* __restrict__ m_state, Vv* __restrict__ v_state,
              float* __restrict__ m_scales, long long n, float lr, float beta1, float beta2, float bc1, float bc2, float eps,
@@ -100,82 +169,56 @@ adamw_kernel(P* __restrict__ param, const G* __restrict__ grad, M* __restrict__ 
     const long long stride = static_cast<long long>(gridDim.x) * blockDim.x;
     // all threads of a 16-lane group must iterate together for the e4m3 path: round the loop bound up
     const long long nvec_pad = (nvec + 31) / 32 * 32;       // whole warps take part in the shuffles
-    for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < nvec_pad; i += stride) {
-        const bool active = i < nvec;
-        const long long e = i * 8;
-        float p[8], g[8], m[8], v[8];
-        if (active) {
-            load8<P>(p, param + e);
-            load8<G>(g, grad + e);
-            load8<Vv>(v, v_state + e);
-            load8<M>(m, m_state + e);
-            if constexpr (sizeof(M) == 1) {
-                float sc = m_scales[e / 128];
-#pragma unroll
-                for (int k = 0; k < 8; ++k) m[k] *= sc;
-            }
-        } else {
-#pragma unroll
-            for (int k = 0; k < 8; ++k) { p[k] = g[k] = m[k] = v[k] = 0.f; }
-        }
-#pragma unroll
-        for (int k = 0; k < 8; ++k) {
-            float gk = g[k] * gs;
-            m[k] = beta1 * m[k] + (1.f - beta1) * gk;
-            v[k] = beta2 * v[k] + (1.f - beta2) * gk * gk;
-            float mh = m[k] * bc1, vh = v[k] * bc2;
-            p[k] -= lr * (__fdividef(mh, sqrt_approx(vh) + eps) + wd * p[k]);
-        }
-        const uint64_t ctr = static_cast<uint64_t>(e + elem_offset);
-        const SrWords words(ctr, seed);
-        if constexpr (sizeof(M) == 1) {
-            float am = 0.f;
-#pragma unroll
-            for (int k = 0; k < 8; ++k) am = fmaxf(am, fabsf(m[k]));
-#pragma unroll
-            for (int o = 8; o > 0; o >>= 1) am = fmaxf(am, __shfl_xor_sync(0xffffffffu, am, o));
-            float sc = fmaxf(am, 1e-30f) / 448.f;
-            if (active) {
-                alignas(8) e4m3 q[8];
-                float inv = 1.f / sc;
-#pragma unroll
-                for (int k = 0; k < 8; k += 2) {
-                    q[k] = sr_e4m3(m[k] * inv, words.get(4 + k));
-                    q[k + 1] = sr_e4m3(m[k + 1] * inv, words.get(5 + k));
-                }
-                *reinterpret_cast<uint2*>(m_state + e) = *reinterpret_cast<uint2*>(q);
-                if ((i & 15) == 0) m_scales[e / 128] = sc;
-            }
-        } else {
-            if (active) store8_srw<M>(m_state + e, m, words, 4);
-        }
-        if (active) {
-            store8_srw<Vv>(v_state + e, v, words, 12);
-            if constexpr (sizeof(P) == 2) {
-                uint32_t o[4];
-#pragma unroll
-                for (int k = 0; k < 4; ++k) {
-                    o[k] = sr_bf16x2(p[2 * k], p[2 * k + 1], words.get(k));
-                    tmax = fmaxf(tmax, fmaxf(fabsf(__uint_as_float(o[k] << 16)), fabsf(__uint_as_float(o[k] & 0xFFFF0000u))));
-                }
-                *reinterpret_cast<uint4*>(reinterpret_cast<bf16*>(param) + e) = make_uint4(o[0], o[1], o[2], o[3]);
-            } else {
-                store8_srw<float>(reinterpret_cast<float*>(param) + e, p, words, 0);
-#pragma unroll
-                for (int k = 0; k < 8; ++k) tmax = fmaxf(tmax, fabsf(p[k]));
-            }
-        }
-    }
+    for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < nvec_pad; i += stride)
+        adamw_vec(i, i < nvec, param, grad, m_state, v_state, m_scales, lr, beta1, beta2, bc1, bc2, eps, wd, gs, seed, elem_offset, tmax);
     block_absmax_commit(absmax_out, tmax, scratch);
+}
+
+// All tensors of an optimizer step in one launch.  A model has a handful of large tensors and hundreds of small ones; one launch per
+// tensor left the GPU waiting for the host (about 10 us a call) and for the last CTAs of every launch.  A CTA takes chunks of
+// kAdamChunk elements and finds the tensor of a chunk by bisection.  Same arithmetic and random words as adamw_kernel.
+struct AdamTensor {                              // 12 x 8 bytes, filled by the host
+    void* param; const void* grad; void* m; void* v;
+    float* m_scales; float* absmax;              // optional
+    long long n, elem_offset, first_chunk;
+    long long seed;                              // added to the step's seed
+    long long decay;                             // 1: weight decay applies
+    long long unused;
+};
+constexpr int kAdamChunk = 16384;
+
+template <typename P, typename G, typename M, typename Vv>
+__global__ void __launch_bounds__(256)
+adamw_multi_kernel(const AdamTensor* __restrict__ tensors, int n_tensors, long long n_chunks, float lr, float beta1, float beta2, float bc1,
+                   float bc2, float eps, float wd, const float* __restrict__ grad_scale, uint32_t seed, const float* __restrict__ hyper) {
+    __shared__ float scratch[32];
+    if (hyper) {
+        lr = hyper[0]; beta1 = hyper[1]; beta2 = hyper[2]; bc1 = hyper[3]; bc2 = hyper[4]; eps = hyper[5]; wd = hyper[6];
+        seed += __float_as_uint(hyper[7]);
+    }
+    const float gs = grad_scale ? *grad_scale : 1.f;
+    for (long long chunk = blockIdx.x; chunk < n_chunks; chunk += gridDim.x) {
+        int lo = 0, hi = n_tensors - 1;          // last tensor whose first chunk is not behind this one
+        while (lo < hi) {
+            const int mid = (lo + hi + 1) / 2;
+            if (tensors[mid].first_chunk <= chunk) lo = mid; else hi = mid - 1;
+        }
+        const AdamTensor t = tensors[lo];
+        const long long nvec = t.n / 8, v0 = (chunk - t.first_chunk) * (kAdamChunk / 8);
+        const long long v1 = min((nvec + 31) / 32 * 32, v0 + kAdamChunk / 8);
+        float tmax = 0.f;
+        for (long long i = v0 + threadIdx.x; i < v1; i += blockDim.x)
+            adamw_vec(i, i < nvec, static_cast<P*>(t.param), static_cast<const G*>(t.grad), static_cast<M*>(t.m), static_cast<Vv*>(t.v), t.m_scales,
+                      lr, beta1, beta2, bc1, bc2, eps, t.decay ? wd : 0.f, gs, seed + static_cast<uint32_t>(t.seed), t.elem_offset, tmax);
+        block_absmax_commit(t.absmax, tmax, scratch);
+    }
 }
 
 // Sum of squares; block b adds its partial to out[b], so several tensors accumulate into the same
 // partial vector in stream order and the result does not depend on atomics.
 template <typename T>
-__global__ void __launch_bounds__(512) norm_squared_kernel(float* __restrict__ out, const T* __restrict__ x, long long n) {
-    __shared__ float scratch[32];
+__device__ __forceinline__ float thread_sum_squares(const T* __restrict__ x, long long n) {
     using V = Vec16<T>;
-    float s = 0.f;
     const long long nvec = n / V::N, stride = static_cast<long long>(gridDim.x) * blockDim.x;
     long long i0 = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x;
     // four loads of a thread in flight, four independent sums
@@ -194,11 +237,42 @@ __global__ void __launch_bounds__(512) norm_squared_kernel(float* __restrict__ o
 #pragma unroll
         for (int k = 0; k < V::N; ++k) { const float f = to_float(v.v[k]); s4[0] += f * f; }
     }
-    s = (s4[0] + s4[1]) + (s4[2] + s4[3]);
+    float s = (s4[0] + s4[1]) + (s4[2] + s4[3]);
     if (blockIdx.x == 0)
         for (long long i = nvec * V::N + threadIdx.x; i < n; i += blockDim.x) { float f = to_float(x[i]); s += f * f; }
-    s = block_reduce_sum(s, scratch);
+    return s;
+}
+
+template <typename T>
+__global__ void __launch_bounds__(512) norm_squared_kernel(float* __restrict__ out, const T* __restrict__ x, long long n) {
+    __shared__ float scratch[32];
+    const float s = block_reduce_sum(thread_sum_squares(x, n), scratch);
     if (threadIdx.x == 0) out[blockIdx.x] += s;
+}
+
+// The gradients of all tensors in one launch.  Bit for bit what norm_squared_kernel adds up launch by launch: the same sums per thread
+// and per tensor, and the tensors' block sums added to out[b] in their order.  Tensors are reduced 16 at a time (one per warp), so
+// that a block waits at one pair of barriers per 16 tensors instead of two barriers per tensor.
+template <typename T>
+__global__ void __launch_bounds__(512) norm_squared_multi_kernel(float* __restrict__ out, const AdamTensor* __restrict__ tensors, int n_tensors) {
+    __shared__ float warp_sums[16][16], sums[16];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    float total = threadIdx.x == 0 ? out[blockIdx.x] : 0.f;
+    for (int t0 = 0; t0 < n_tensors; t0 += 16) {
+        const int n = min(16, n_tensors - t0);
+        for (int t = 0; t < n; ++t) {
+            const float s = warp_reduce_sum(thread_sum_squares(static_cast<const T*>(tensors[t0 + t].grad), tensors[t0 + t].n));
+            if (lane == 0) warp_sums[t][warp] = s;
+        }
+        __syncthreads();
+        if (warp < n) {
+            const float s = warp_reduce_sum(lane < 16 ? warp_sums[warp][lane] : 0.f);
+            if (lane == 0) sums[warp] = s;
+        }
+        __syncthreads();
+        if (threadIdx.x == 0) for (int t = 0; t < n; ++t) total += sums[t];
+    }
+    if (threadIdx.x == 0) out[blockIdx.x] = total;
 }
 
 __global__ void __launch_bounds__(512) deterministic_sum_kernel(float* __restrict__ out, const float* __restrict__ in, int n) {
@@ -315,6 +389,45 @@ extern "C" int llmq_adamw_hyper(void* param, const void* grad, void* m, void* v,
     A_CASE(float, 3, bf16, 0, bf16, 0, bf16, 0)
 #undef A_CASE
     return -10;
+}
+
+// All tensors of a step: `tensors` is a device array of AdamTensor, first_chunk counts chunks of llmq_adamw_chunk() elements.  Every
+// tensor has the given types; sizes are multiples of 8 (128 with e4m3 moments).
+extern "C" int llmq_adamw_chunk() { return kAdamChunk; }
+extern "C" int llmq_adamw_multi(const void* tensors, int n_tensors, long long n_chunks, float lr, float beta1, float beta2, int step, float eps, float wd,
+                                const float* grad_scale, unsigned int seed, int p_dtype, int g_dtype, int m_dtype, int v_dtype, int num_sms,
+                                const float* hyper, cudaStream_t s) {
+    if (n_tensors <= 0 || n_chunks <= 0) return 0;
+    const float bc1 = 1.f / (1.f - powf(beta1, static_cast<float>(step)));
+    const float bc2 = 1.f / (1.f - powf(beta2, static_cast<float>(step)));
+    const int g = static_cast<int>(n_chunks < 8LL * num_sms ? n_chunks : 8LL * num_sms);
+    const AdamTensor* t = static_cast<const AdamTensor*>(tensors);
+#define A_CASE(P, PC, G, GC, M, MC, V, VC)                                                                          \
+    if (p_dtype == PC && g_dtype == GC && m_dtype == MC && v_dtype == VC) {                                         \
+        adamw_multi_kernel<P, G, M, V><<<g, 256, 0, s>>>(t, n_tensors, n_chunks, lr, beta1, beta2, bc1, bc2, eps, wd, grad_scale, seed, hyper); \
+        return LLMQ_LAUNCH_CHECK();                                                                                 \
+    }
+    A_CASE(bf16, 0, bf16, 0, bf16, 0, bf16, 0)
+    A_CASE(bf16, 0, bf16, 0, float, 3, float, 3)
+    A_CASE(bf16, 0, bf16, 0, float, 3, bf16, 0)
+    A_CASE(bf16, 0, bf16, 0, bf16, 0, float, 3)
+    A_CASE(bf16, 0, bf16, 0, e4m3, 1, bf16, 0)
+    A_CASE(bf16, 0, bf16, 0, e4m3, 1, float, 3)
+    A_CASE(float, 3, float, 3, float, 3, float, 3)
+    A_CASE(float, 3, float, 3, bf16, 0, bf16, 0)
+    A_CASE(float, 3, bf16, 0, float, 3, float, 3)
+    A_CASE(float, 3, bf16, 0, bf16, 0, bf16, 0)
+#undef A_CASE
+    return -10;
+}
+
+extern "C" int llmq_norm_squared_multi(float* partials, const void* tensors, int n_tensors, int dtype, int num_partials, cudaStream_t s) {
+    if (n_tensors <= 0) return 0;
+    const AdamTensor* t = static_cast<const AdamTensor*>(tensors);
+    if (dtype == 0) norm_squared_multi_kernel<bf16><<<num_partials, 512, 0, s>>>(partials, t, n_tensors);
+    else if (dtype == 3) norm_squared_multi_kernel<float><<<num_partials, 512, 0, s>>>(partials, t, n_tensors);
+    else return -10;
+    return LLMQ_LAUNCH_CHECK();
 }
 
 extern "C" int llmq_norm_squared(float* partials, const void* x, long long n, int dtype, int num_partials, cudaStream_t s) {

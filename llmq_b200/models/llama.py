@@ -915,8 +915,12 @@ class LlamaModel:
         on_device = self.device.type == "cuda" and all(
             t.device.type == "cuda" for name, master, spec, l in items for t in (master, shard_of[name], o.m[name], o.v[name]))
         graph_opt = self.graphs is not None and on_device
+        table = self._optimizer_table(items, shard_of) if on_device else None
 
         def norms():
+            if table is not None:
+                K.norm_squared_multi(self.norm_partials, table)
+                return
             for name, master, spec, l in items:
                 gs = shard_of[name]
                 gd = gs if gs.device.type == self.device.type else gs.to(self.device, non_blocking=True)
@@ -942,6 +946,9 @@ class LlamaModel:
             self._opt_hyper.copy_(self._opt_hyper_host, non_blocking=True)
 
             def adam_all():
+                if table is not None:
+                    K.adamw_multi(table, lr=0.0, beta1=0.0, beta2=0.0, step=1, eps=0.0, weight_decay=1.0, grad_scale=scale, hyper=self._opt_hyper)
+                    return
                 for idx, (name, master, spec, l) in enumerate(items):
                     am = w._stat(l, spec.name)[0:1] if (l is not None and spec.name in MATRICES and w.quantized) else None
                     if master.numel() % 8:
@@ -951,6 +958,9 @@ class LlamaModel:
                             m_scales=o.m_scales.get(name), seed=idx * 7919, elem_offset=self.comm.rank * master.numel(), hyper=self._opt_hyper)
             self.graphs.run(("opt-adamw",), adam_all)
             items = []                                           # the staged loop below has nothing left to do
+        elif table is not None:
+            K.adamw_multi(table, lr=lr, beta1=beta1, beta2=beta2, step=step, eps=eps, weight_decay=weight_decay, grad_scale=scale, seed=seed_base)
+            items = []
         stager = self._stager
         staged = [None] * len(items)
 
@@ -1003,6 +1013,25 @@ class LlamaModel:
         if self.opts.trigger_timing_events:
             res["time_breakdown"] = self.time_breakdown()
         return res
+
+    def _optimizer_table(self, items, shard_of):
+        """The optimizer's tensors as one table (everything on the device and of the same types), or None."""
+        o, w, rows = self.opt_state, self.weights, []
+        for idx, (name, master, spec, l) in enumerate(items):
+            if master.numel() % 8:
+                raise ValueError(f"parameter shard {name} has {master.numel()} elements; shard sizes must be multiples of 8")
+            am = w._stat(l, spec.name)[0:1] if (l is not None and spec.name in MATRICES and w.quantized) else None
+            rows.append({"param": master, "grad": shard_of[name], "m": o.m[name], "v": o.v[name], "m_scales": o.m_scales.get(name), "absmax": am,
+                         "elem_offset": self.comm.rank * master.numel(), "seed": idx * 7919, "decay": spec.matrix})
+        if len({(r["param"].dtype, r["grad"].dtype, r["m"].dtype, r["v"].dtype) for r in rows}) != 1 or not all(
+                r[k].is_contiguous() for r in rows for k in ("param", "grad", "m", "v")):
+            return None
+        table = getattr(self, "_opt_table", None)
+        if table is None or not table.matches(rows):
+            if torch.cuda.is_current_stream_capturing():
+                return None
+            table = self._opt_table = K.AdamTable(rows, self.device)
+        return table
 
     # ================================================================================== introspection
     def get_gradients(self) -> Dict[str, torch.Tensor]:

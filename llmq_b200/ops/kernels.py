@@ -726,6 +726,59 @@ def adamw_hyper(out: torch.Tensor, *, lr: float, beta1: float, beta2: float, ste
                                       ctypes.c_uint(seed & 0xFFFFFFFF))
 
 
+class AdamTable:
+    """Device table of the tensors of an optimizer step, for :func:`adamw_multi` and :func:`norm_squared_multi` (CUDA only).
+
+    ``rows``: one dict per tensor with ``param``, ``grad``, ``m``, ``v`` (flat sizes equal, the same types in every row), optional
+    ``m_scales`` and ``absmax``, and ``elem_offset``, ``seed``, ``decay`` (whether weight decay applies).  The table holds addresses:
+    :meth:`matches` says whether it still describes the given rows."""
+
+    FIELDS = 12                                         # 8-byte words per tensor, see AdamTensor in csrc/optim.cu
+
+    def __init__(self, rows, device):
+        self.key = self._key(rows)
+        self.types = {(r["param"].dtype, r["grad"].dtype, r["m"].dtype, r["v"].dtype) for r in rows}
+        if len(self.types) != 1:
+            raise ValueError("the tensors of one table have the same types")
+        chunk, first, words = L.kernels().llmq_adamw_chunk(), 0, []
+        for r, key in zip(rows, self.key):
+            n = r["param"].numel()
+            if n % (128 if _is_f8(r["m"].dtype) else 8):
+                raise ValueError("parameter shard sizes must be multiples of 8 (128 with e4m3 moments)")
+            if any(r[k].numel() != n or not r[k].is_contiguous() for k in ("param", "grad", "m", "v")):
+                raise ValueError("parameter, gradient and moments are contiguous and of one size")
+            words += [*key[:6], n, r["elem_offset"], first, r["seed"], int(r["decay"]), 0]
+            first += -(-n // chunk)
+        self.n_tensors, self.n_chunks = len(rows), first
+        self.words = torch.tensor(words, dtype=torch.int64).to(device)
+
+    @staticmethod
+    def _key(rows):
+        p = lambda t: 0 if t is None else t.data_ptr()
+        return [(p(r["param"]), p(r["grad"]), p(r["m"]), p(r["v"]), p(r.get("m_scales")), p(r.get("absmax")), r["param"].numel(), r["elem_offset"],
+                 r["seed"], bool(r["decay"]), r["param"].dtype, r["grad"].dtype, r["m"].dtype, r["v"].dtype) for r in rows]
+
+    def matches(self, rows) -> bool:
+        return self.key == self._key(rows)
+
+
+def adamw_multi(table: AdamTable, *, lr: float, beta1: float, beta2: float, step: int, eps: float, weight_decay: float,
+                grad_scale: Optional[torch.Tensor] = None, seed: int = 0, hyper: Optional[torch.Tensor] = None) -> None:
+    """:func:`adamw` on every tensor of the table in one launch: same results as one call per row with that row's ``m_scales``,
+    ``absmax``, ``elem_offset``, ``seed + row seed`` and, where ``decay`` is set, ``weight_decay``."""
+    (pt, gt, mt, vt), = table.types
+    L.check(L.kernels().llmq_adamw_multi(L.ptr(table.words), table.n_tensors, _ll(table.n_chunks), _f(lr), _f(beta1), _f(beta2), int(step), _f(eps),
+                                         _f(weight_decay), L.ptr(grad_scale), ctypes.c_uint(seed & 0xFFFFFFFF), L.dtype_code(pt), L.dtype_code(gt),
+                                         L.dtype_code(mt), L.dtype_code(vt), num_sms(table.words.device), L.ptr(hyper), L.stream_ptr()), "adamw_multi")
+
+
+def norm_squared_multi(partials: torch.Tensor, table: AdamTable) -> None:
+    """:func:`norm_squared` of every gradient of the table in one launch, with the same bits."""
+    (_, gt, _, _), = table.types
+    L.check(L.kernels().llmq_norm_squared_multi(L.ptr(partials), L.ptr(table.words), table.n_tensors, L.dtype_code(gt), partials.numel(),
+                                                L.stream_ptr()), "norm_squared_multi")
+
+
 NORM_PARTIALS = 512
 
 

@@ -192,3 +192,36 @@ def test_gemm_tile_widths(M, N, Kd, dt, accumulate):
     want = a.double() @ b.double().t() + bias.double() + (prev.double() if accumulate else 0)
     assert rel(out, want) < 1e-5                           # exact products, fp32 sums
     assert abs(am.item() - want.abs().max().item()) < 1e-4 * want.abs().max().item()
+
+
+@pytest.mark.parametrize("types", [(BF, BF, BF, BF), (BF, BF, torch.float32, torch.float32), (BF, BF, torch.float8_e4m3fn, BF), (torch.float32,) * 4])
+@pytest.mark.parametrize("sizes", [[128], [16384, 128, 16384 + 128, 896, 3 * 16384, 16384 - 128], [128 * (i + 1) for i in range(50)]])
+def test_adamw_and_norm_of_all_tensors_in_one_launch(types, sizes):
+    """Bit for bit the launches per tensor: sizes around one chunk of the table, more tensors than one round of the norm."""
+    g = torch.Generator(device=DEV).manual_seed(len(sizes))
+    r = lambda n, dt, s=1.0: (torch.randn(n, device=DEV, generator=g) * s).to(dt)
+    f8 = types[2] == torch.float8_e4m3fn
+
+    def rows():
+        g.manual_seed(len(sizes))
+        return [{"param": r(n, types[0]), "grad": r(n, types[1], 0.1), "m": r(n, types[2], 0.1), "v": r(n, torch.float32, 0.1).square().to(types[3]),
+                 "m_scales": r(n // 128, torch.float32).abs() + 0.1 if f8 else None, "absmax": torch.zeros(1, device=DEV) if i % 2 else None,
+                 "elem_offset": 128 * i, "seed": 7919 * i, "decay": i % 3 == 0} for i, n in enumerate(sizes)]
+
+    one, each = rows(), rows()
+    table = K.AdamTable(one, DEV)
+    assert table.matches(one) and not table.matches(each)
+    a, b = torch.full((512,), 0.5, device=DEV), torch.full((512,), 0.5, device=DEV)
+    K.norm_squared_multi(a, table)
+    for t in each:
+        K.norm_squared(b, t["grad"])
+    assert torch.equal(a, b)
+    scale, hyper = torch.full((1,), 0.7, device=DEV), dict(lr=1e-2, beta1=0.9, beta2=0.95, step=3, eps=1e-8)
+    K.adamw_multi(table, weight_decay=0.1, grad_scale=scale, seed=11, **hyper)
+    for t in each:
+        K.adamw(t["param"], t["grad"], t["m"], t["v"], weight_decay=0.1 if t["decay"] else 0.0, grad_scale=scale, absmax=t["absmax"],
+                m_scales=t["m_scales"], seed=11 + t["seed"], elem_offset=t["elem_offset"], **hyper)
+    for x, y in zip(one, each):
+        for k in ("param", "m", "v", "m_scales", "absmax"):
+            if x[k] is not None:
+                assert torch.equal(x[k].view(torch.uint8), y[k].view(torch.uint8)), k
