@@ -74,6 +74,10 @@ rmsnorm_fwd_kernel(T* __restrict__ residual_out,      // may be null when not fu
     block_absmax_commit(absmax_out, tmax, scratch);
 }
 
+// The sum of 8 warp sums in the order of block_reduce_sum's shuffle tree: the kernels below give the bits of a 256-thread block
+// reduction whatever their own shape is.
+__device__ __forceinline__ float tree8(const float* w) { return ((w[0] + w[4]) + (w[2] + w[6])) + ((w[1] + w[5]) + (w[3] + w[7])); }
+
 // Same contract for rows of up to 8 column vectors per thread: the row is read once (all loads of a thread in flight at once),
 // stays in registers across the reduction and is neither stored first nor read again.  A CTA is one row and as small as the row
 // allows (64 threads up to 512 vectors), so that many rows share an SM and one row's reduction hides behind the others' loads.
@@ -83,7 +87,7 @@ __global__ void __launch_bounds__(THREADS)
 rmsnorm_fwd_reg_kernel(T* __restrict__ residual_out, T* __restrict__ y_out, e4m3* __restrict__ q_out, float* __restrict__ rstd_out,
                        const T* __restrict__ in_a, const T* __restrict__ in_b, const T* __restrict__ weight, float eps, int C,
                        float* __restrict__ absmax_out, const float* __restrict__ known_absmax, float* __restrict__ q_scale_out) {
-    __shared__ float scratch[THREADS / 32], scratch_max[THREADS / 32];
+    __shared__ float scratch[8], scratch_max[THREADS / 32];
     using V = Vec16<T>;
     const long long row = blockIdx.x;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -112,23 +116,29 @@ rmsnorm_fwd_reg_kernel(T* __restrict__ residual_out, T* __restrict__ y_out, e4m3
             }
         }
     }
-    float ss = 0.f;
+    // Vector v of the row belongs to virtual thread v mod 256, which adds its vectors up in ascending order; with 64 threads a thread
+    // stands for four virtual threads.
+    constexpr int CHAINS = 256 / THREADS;
+    float ss[CHAINS];
+#pragma unroll
+    for (int q = 0; q < CHAINS; ++q) ss[q] = 0.f;
 #pragma unroll
     for (int k = 0; k < VPT; ++k) {
         const int c = (k * THREADS + threadIdx.x) * V::N;
         if (c < C) {
             if (residual_out) x[k].store(residual_out + row * C + c);
 #pragma unroll
-            for (int i = 0; i < V::N; ++i) { const float f = to_float(x[k].v[i]); ss += f * f; }
+            for (int i = 0; i < V::N; ++i) { const float f = to_float(x[k].v[i]); ss[k % CHAINS] += f * f; }
         }
     }
-    ss = warp_reduce_sum(ss);
-    if (lane == 0) scratch[warp] = ss;
-    __syncthreads();
-    ss = 0.f;
 #pragma unroll
-    for (int w = 0; w < THREADS / 32; ++w) ss += scratch[w];
-    const float rstd = rsqrtf(ss / C + eps);
+    for (int q = 0; q < CHAINS; ++q) {
+        const float s = warp_reduce_sum(ss[q]);
+        if (lane == 0) scratch[q * (THREADS / 32) + warp] = s;
+    }
+    __syncthreads();
+    const float sum = tree8(scratch);
+    const float rstd = rsqrtf(sum / C + eps);
     if (threadIdx.x == 0 && rstd_out) rstd_out[row] = rstd;
     float qmul = 0.f;
     if (q_out) {
@@ -292,10 +302,7 @@ rmsnorm_bwd_reg_kernel(T* __restrict__ dinp, float* __restrict__ dw_partial, con
         dot = warp_reduce_sum(dot);
         if ((threadIdx.x & 31) == 0) dots[par][threadIdx.x >> 5] = dot;
         __syncthreads();
-        dot = 0.f;
-#pragma unroll
-        for (int w = 0; w < NORM_THREADS / 32; ++w) dot += dots[par][w];
-        dot *= inv_c;
+        dot = tree8(dots[par]) * inv_c;
 #pragma unroll
         for (int k = 0; k < VPT; ++k) {
             const int c = (k * NORM_THREADS + threadIdx.x) * V::N;
@@ -318,78 +325,6 @@ rmsnorm_bwd_reg_kernel(T* __restrict__ dinp, float* __restrict__ dw_partial, con
 #pragma unroll
             for (int i = 0; i < V::N; ++i) dw_partial[static_cast<long long>(blockIdx.x) * C + c + i] = dw[k][i];
         }
-    }
-    block_absmax_commit(absmax_out, tmax, scratch);
-}
-
-// Same contract for short rows (at most 224 column vectors, with which most of the 256 threads above would idle; 4096 x 896: 12.2 us
-// against 14.2): `group` threads
-// (the row's vectors rounded up to whole warps) own one row at a time, one vector each, and a CTA of up to 448 threads runs several
-// such groups side by side, each with its own barrier.  The groups' weight gradients meet in shared memory at the end: one partial
-// row per CTA.
-constexpr int SHORT_ROW_THREADS = 448;
-template <typename T>
-__global__ void __launch_bounds__(SHORT_ROW_THREADS, 2)
-rmsnorm_bwd_short_kernel(T* __restrict__ dinp, float* __restrict__ dw_partial, const T* __restrict__ dout, const T* __restrict__ inp,
-                       const T* __restrict__ weight, const float* __restrict__ rstd, int rows, int C, int group, float* __restrict__ absmax_out) {
-    using V = Vec16<T>;
-    __shared__ float scratch[32];
-    __shared__ float dots[2][16];                            // per warp, alternating: one barrier per row is enough
-    __shared__ float dw_sum[SHORT_ROW_THREADS * V::N];
-    const int groups = blockDim.x / group, grp = threadIdx.x / group, t = threadIdx.x - grp * group;
-    const int warp = threadIdx.x >> 5, warp0 = grp * (group >> 5), gwarps = group >> 5;
-    const int c = t * V::N;
-    const bool on = c < C;
-    float dw[V::N];
-    V vw;
-    if (on) vw = V::load(weight + c);
-#pragma unroll
-    for (int i = 0; i < V::N; ++i) dw[i] = 0.f;
-    float tmax = 0.f;
-    const float inv_c = 1.f / C;
-    const long long stride = static_cast<long long>(gridDim.x) * groups;
-    long long row = static_cast<long long>(blockIdx.x) * groups + grp;
-    for (int par = 0; row < rows; row += stride, par ^= 1) {
-        V dy, x, dx;
-        if (on) { dy = V::load_stream(dout + row * C + c); x = V::load_stream(inp + row * C + c); dx = V::load_stream(dinp + row * C + c); }
-        const float rs = rstd[row];
-        float dot = 0.f;
-        if (on) {
-#pragma unroll
-            for (int i = 0; i < V::N; ++i) {
-                const float xh = to_float(x.v[i]) * rs, g = to_float(dy.v[i]);
-                dot += to_float(vw.v[i]) * g * xh;
-                dw[i] += g * xh;
-            }
-        }
-        dot = warp_reduce_sum(dot);
-        if ((threadIdx.x & 31) == 0) dots[par][warp] = dot;
-        if (gwarps > 1) asm volatile("bar.sync %0, %1;" ::"r"(1 + grp), "r"(group) : "memory");     // at most 7 such groups
-        else __syncwarp();
-        dot = 0.f;
-        for (int w = 0; w < gwarps; ++w) dot += dots[par][warp0 + w];
-        dot *= inv_c;
-        if (on) {
-#pragma unroll
-            for (int i = 0; i < V::N; ++i) {
-                const float xh = to_float(x.v[i]) * rs;
-                const float g = (to_float(vw.v[i]) * to_float(dy.v[i]) - xh * dot) * rs;
-                dx.v[i] = from_float<T>(to_float(dx.v[i]) + g);
-                tmax = fmaxf(tmax, fabsf(to_float(dx.v[i])));
-            }
-            dx.store(dinp + row * C + c);
-        }
-    }
-    float* out = dw_partial + static_cast<long long>(blockIdx.x) * C;
-    if (on) {
-#pragma unroll
-        for (int i = 0; i < V::N; ++i) dw_sum[grp * C + c + i] = dw[i];
-    }
-    __syncthreads();
-    for (int i = threadIdx.x; i < C; i += blockDim.x) {
-        float s = 0.f;
-        for (int g = 0; g < groups; ++g) s += dw_sum[g * C + i];
-        out[i] = s;
     }
     block_absmax_commit(absmax_out, tmax, scratch);
 }
@@ -451,24 +386,17 @@ int launch_bwd(void* dinp, void* dweight, float* scratch, const void* dout, cons
                const float* rstd, int rows, int C, float* absmax, int accumulate_dw, int num_blocks, cudaStream_t s) {
     using V = Vec16<T>;
     if (C % V::N) return -1;
-    const int vecs = C / V::N, vpt = ceil_div_i(vecs, NORM_THREADS);
-#define ARGS static_cast<T*>(dinp), scratch, static_cast<const T*>(dout), static_cast<const T*>(inp), static_cast<const T*>(w), rstd, rows, C
-    if (2 * vecs <= SHORT_ROW_THREADS) {
-        const int group = ceil_div_i(vecs, 32) * 32, groups = SHORT_ROW_THREADS / group;
-        int sms = 0, dev = 0;
-        cudaGetDevice(&dev);
-        if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess && num_blocks > 2 * sms) num_blocks = 2 * sms;
-        if (num_blocks > ceil_div_i(rows, groups)) num_blocks = ceil_div_i(rows, groups);
-        rmsnorm_bwd_short_kernel<T><<<num_blocks, group * groups, 0, s>>>(ARGS, group, absmax);
-    } else {
-        if (num_blocks > rows) num_blocks = rows;
-        if (vpt <= 1) rmsnorm_bwd_reg_kernel<T, 1><<<num_blocks, NORM_THREADS, 0, s>>>(ARGS, absmax);
-        else if (vpt <= 2) rmsnorm_bwd_reg_kernel<T, 2><<<num_blocks, NORM_THREADS, 0, s>>>(ARGS, absmax);
-        else if (vpt <= 4) rmsnorm_bwd_reg_kernel<T, 4><<<num_blocks, NORM_THREADS, 0, s>>>(ARGS, absmax);
-        else if (vpt <= 8) rmsnorm_bwd_kernel<T, 8><<<num_blocks, NORM_THREADS, 0, s>>>(ARGS, absmax);
-        else return -2;
-    }
-#undef ARGS
+    const int vecs = ceil_div_i(C / V::N, NORM_THREADS);
+    if (num_blocks > rows) num_blocks = rows;
+#define LAUNCH(KERNEL)                                                                                                       \
+    KERNEL<<<num_blocks, NORM_THREADS, 0, s>>>(static_cast<T*>(dinp), scratch, static_cast<const T*>(dout), static_cast<const T*>(inp), \
+                                               static_cast<const T*>(w), rstd, rows, C, absmax)
+    if (vecs <= 1) LAUNCH((rmsnorm_bwd_reg_kernel<T, 1>));
+    else if (vecs <= 2) LAUNCH((rmsnorm_bwd_reg_kernel<T, 2>));
+    else if (vecs <= 4) LAUNCH((rmsnorm_bwd_reg_kernel<T, 4>));
+    else if (vecs <= 8) LAUNCH((rmsnorm_bwd_kernel<T, 8>));
+    else return -2;
+#undef LAUNCH
     int rc = LLMQ_LAUNCH_CHECK();
     if (rc) return rc;
     rmsnorm_bwd_reduce_kernel<T><<<ceil_div_i(C, RED_COLS), RED_COLS * RED_GROUPS, 0, s>>>(static_cast<T*>(dweight), scratch, num_blocks, C, accumulate_dw);
