@@ -102,10 +102,10 @@ fused_ce_kernel(T* logits, float* __restrict__ losses, float* __restrict__ lse_o
 
 // bf16 rows, two CTAs of a cluster per row and three CTAs on an SM: the passes over one row (a stream of loads, two reductions, a
 // stream of loads and stores) overlap with those of other rows, while the rows in flight (222 of up to 300 KB) still fit the L2
-// between their two passes.  The CTAs exchange one (maximum, sum) pair through distributed shared memory.  Exponentials are the
+// between their two passes.  The CTAs exchange their warps' (maximum, sum) pairs through distributed shared memory.  Exponentials are the
 // hardware's directly (with a range step around it, exp2f costs four instructions more and two of them are spent per logit).
 // Bound by the two exponentials per logit (280 us of MUFU time at 4096 x 152064) and by memory (375 us for one read and one write):
-// 456 us there, 622 us with one 1024-thread CTA per row and SM, whose loads, reductions and stores followed one another.  A row kept
+// 446-459 us there, 622 us with one 1024-thread CTA per row and SM, whose loads, reductions and stores followed one another.  A row kept
 // in registers (clusters of eight CTAs, one read) took 819 us: its CTAs live 4 us, most of it start-up and cluster barriers.
 __device__ __forceinline__ void cluster_arrive_relaxed() { asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory"); }
 __device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
@@ -127,80 +127,77 @@ __device__ __forceinline__ float2 ce_unpack(uint32_t w) {
 
 constexpr int CE_ROW_THREADS = 512;
 
+// Thread t of CTA `part` does what thread part * 512 + t of a 1024-thread block would: vectors part * 512 + t, + 1024, ..., one after
+// the other, and the CTAs' 32 warp results are combined in every warp in the order of that block, so the sums have its bits.
 __global__ void __launch_bounds__(CE_ROW_THREADS, 3)
 fused_ce_row_kernel(bf16* logits, float* __restrict__ losses, float* __restrict__ lse_out, const int* __restrict__ targets,
-                    float dloss, float z_reg, int rows, int V, long long ld, int write_dlogits, int parts) {
-    __shared__ float scratch[32];
-    __shared__ float2 s_part[2];                // (maximum, sum) of every CTA of the cluster
-    const int part = blockIdx.x % parts;
-    const long long row = rows - 1 - static_cast<long long>(blockIdx.x / parts);     // newest GEMM output first: L2 hits
+                    float dloss, float z_reg, int rows, int V, long long ld, int write_dlogits) {
+    constexpr int PARTS = 2, STRIDE = PARTS * CE_ROW_THREADS;
+    __shared__ float2 s_part[32];               // (maximum, sum) of every warp of the cluster
+    const int part = blockIdx.x % PARTS, tid = threadIdx.x;
+    const long long row = rows - 1 - static_cast<long long>(blockIdx.x / PARTS);     // newest GEMM output first: L2 hits
     bf16* x = logits + row * ld;
     const int tgt = targets[row];
-    const int nvec = V / 8, per_part = (nvec + parts - 1) / parts;
-    const int v0 = part * per_part, v1 = min(nvec, v0 + per_part);
-    const int tail = part == parts - 1 ? V - nvec * 8 : 0;         // elements behind the last whole vector
-    const int tid = threadIdx.x;
+    const int nvec = V / 8, first = part * CE_ROW_THREADS + tid;
+    const int tail = part == 0 ? V - nvec * 8 : 0;                 // elements behind the last whole vector
     if (tgt < 0 || tgt >= V) {                  // masked row: the same decision in every CTA of the cluster
         if (write_dlogits) {
-            for (int i = v0 + tid; i < v1; i += CE_ROW_THREADS) __stcs(reinterpret_cast<uint4*>(x) + i, make_uint4(0u, 0u, 0u, 0u));
+            for (int i = first; i < nvec; i += STRIDE) __stcs(reinterpret_cast<uint4*>(x) + i, make_uint4(0u, 0u, 0u, 0u));
             if (tid < tail) x[nvec * 8 + tid] = __float2bfloat16_rn(0.f);
         }
         if (part == 0 && tid == 0 && lse_out) lse_out[row] = 0.f;
         return;
     }
-    if (parts > 1) cluster_arrive_relaxed();
+    cluster_arrive_relaxed();
     constexpr float kLog2e = 1.4426950408889634f;
-    const float xt = tid < tail ? __bfloat162float(x[nvec * 8 + tid]) : -INFINITY;
     const float tgt_logit = (part == 0 && tid == 0) ? __bfloat162float(x[tgt]) : 0.f;    // read before anyone overwrites it
-    // pass 1: online maximum and sum of exponentials, four vectors at a time
-    float m = xt, s = xt == -INFINITY ? 0.f : ce_exp2((xt - m) * kLog2e);
-    auto add = [&](const uint4* w, int n) {
-        __nv_bfloat162 mx2 = *reinterpret_cast<const __nv_bfloat162*>(&w[0]);
-        for (int j = 0; j < n; ++j) {
-            const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&w[j]);
-            mx2 = __hmax2(mx2, __hmax2(__hmax2(h[0], h[1]), __hmax2(h[2], h[3])));
-        }
+    // pass 1: online maximum and sum of exponentials (base-2 domain), four vectors in flight
+    float m = -INFINITY, s = 0.f;
+    auto add = [&](const uint4& w) {
+        const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&w);
+        const __nv_bfloat162 mx2 = __hmax2(__hmax2(h[0], h[1]), __hmax2(h[2], h[3]));
         const float lm = fmaxf(__low2float(mx2), __high2float(mx2));
-        if (lm > m) { s = m == -INFINITY ? s : s * ce_exp2((m - lm) * kLog2e); m = lm; }
+        if (lm > m) { s *= ce_exp2((m - lm) * kLog2e); m = lm; }
         const float moff = m == -INFINITY ? 0.f : m;           // nothing but -inf so far: every exponential is 0
-        float s0 = 0.f, s1 = 0.f;
-        for (int j = 0; j < n; ++j) {
-            const uint32_t u[4] = {w[j].x, w[j].y, w[j].z, w[j].w};
+        const uint32_t u[4] = {w.x, w.y, w.z, w.w};
 #pragma unroll
-            for (int q = 0; q < 4; ++q) {
-                const float2 f = ce_unpack(u[q]);
-                s0 += ce_exp2((f.x - moff) * kLog2e);
-                s1 += ce_exp2((f.y - moff) * kLog2e);
-            }
+        for (int q = 0; q < 4; ++q) {
+            const float2 f = ce_unpack(u[q]);
+            s += ce_exp2((f.x - moff) * kLog2e);
+            s += ce_exp2((f.y - moff) * kLog2e);
         }
-        s += s0 + s1;
     };
-    int i = v0 + tid;
-    for (; i + 3 * CE_ROW_THREADS < v1; i += 4 * CE_ROW_THREADS) {
+    int i = first;
+    for (; i + 3 * STRIDE < nvec; i += 4 * STRIDE) {
         uint4 w[4];
 #pragma unroll
-        for (int j = 0; j < 4; ++j) w[j] = *(reinterpret_cast<const uint4*>(x) + i + j * CE_ROW_THREADS);
-        add(w, 4);
+        for (int j = 0; j < 4; ++j) w[j] = *(reinterpret_cast<const uint4*>(x) + i + j * STRIDE);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) add(w[j]);
     }
-    for (; i < v1; i += CE_ROW_THREADS) {
-        const uint4 w = *(reinterpret_cast<const uint4*>(x) + i);
-        add(&w, 1);
+    for (; i < nvec; i += STRIDE) add(*(reinterpret_cast<const uint4*>(x) + i));
+    const float xt = tid < tail ? __bfloat162float(x[nvec * 8 + tid]) : -INFINITY;
+    if (tid < tail) {
+        if (xt > m) { s *= ce_exp2((m - xt) * kLog2e); m = xt; }
+        if (m != -INFINITY) s += ce_exp2((xt - m) * kLog2e);
     }
-    const float mb = block_reduce_max(m, scratch);
-    s = block_reduce_sum(m == -INFINITY ? s : s * ce_exp2((m - mb) * kLog2e), scratch);
-    m = mb;
-    if (parts > 1) {
-        cluster_wait();                                        // every CTA of the cluster has started
-        if (tid < parts) st_cluster_f32x2(&s_part[part], tid, m, s);
-        cluster_arrive();
-        cluster_wait();
-        float mg = -INFINITY, sg = 0.f;
-        for (int q = 0; q < parts; ++q) mg = fmaxf(mg, s_part[q].x);
-        for (int q = 0; q < parts; ++q) sg += s_part[q].x == -INFINITY ? s_part[q].y : s_part[q].y * ce_exp2((s_part[q].x - mg) * kLog2e);
-        m = mg; s = sg;
-    } else {
-        __syncthreads();                                       // x[tgt] has been read
-    }
+    auto combine = [&]() {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            const float om = __shfl_xor_sync(0xffffffffu, m, o), os = __shfl_xor_sync(0xffffffffu, s, o);
+            const float nm = fmaxf(m, om);
+            s = (m == -INFINITY ? 0.f : s * ce_exp2((m - nm) * kLog2e)) + (om == -INFINITY ? 0.f : os * ce_exp2((om - nm) * kLog2e));
+            m = nm;
+        }
+    };
+    combine();
+    const int lane = tid & 31, warp = tid >> 5;
+    cluster_wait();                                            // every CTA of the cluster has started
+    if (lane < PARTS) st_cluster_f32x2(&s_part[part * (CE_ROW_THREADS / 32) + warp], lane, m, s);
+    cluster_arrive();
+    cluster_wait();
+    m = s_part[lane].x; s = s_part[lane].y;
+    combine();
     const float lse = logf(s) + m;
     if (part == 0 && tid == 0) {
         losses[row] += lse - tgt_logit;
@@ -231,14 +228,14 @@ fused_ce_row_kernel(bf16* logits, float* __restrict__ losses, float* __restrict_
         }
         __stcs(reinterpret_cast<uint4*>(x) + at, make_uint4(u[0], u[1], u[2], u[3]));
     };
-    for (i = v0 + tid; i + 3 * CE_ROW_THREADS < v1; i += 4 * CE_ROW_THREADS) {
+    for (i = first; i + 3 * STRIDE < nvec; i += 4 * STRIDE) {
         uint4 w[4];
 #pragma unroll
-        for (int j = 0; j < 4; ++j) w[j] = __ldcs(reinterpret_cast<const uint4*>(x) + i + j * CE_ROW_THREADS);
+        for (int j = 0; j < 4; ++j) w[j] = __ldcs(reinterpret_cast<const uint4*>(x) + i + j * STRIDE);
 #pragma unroll
-        for (int j = 0; j < 4; ++j) grad(w[j], i + j * CE_ROW_THREADS);
+        for (int j = 0; j < 4; ++j) grad(w[j], i + j * STRIDE);
     }
-    for (; i < v1; i += CE_ROW_THREADS) grad(__ldcs(reinterpret_cast<const uint4*>(x) + i), i);
+    for (; i < nvec; i += STRIDE) grad(__ldcs(reinterpret_cast<const uint4*>(x) + i), i);
     if (tid < tail) {
         float g = ce_exp2(fmaf(xt, kLog2e, shift));
         if (nvec * 8 + tid == tgt) g -= dloss;
@@ -278,16 +275,15 @@ extern "C" int llmq_fused_classifier(void* logits, float* losses, float* lse_out
     if (rows <= 0) return 0;
     if (dtype == 0) {
         if (ld % 8) return -1;
-        const int parts = V > 8 * 4 * CE_ROW_THREADS ? 2 : 1;               // two CTAs once one has more than four vectors a thread
         if (rows > (1 << 30) - 1) return -1;
         cudaLaunchConfig_t cfg{};
-        cfg.gridDim = dim3(static_cast<unsigned int>(rows) * parts); cfg.blockDim = dim3(CE_ROW_THREADS); cfg.stream = s;
+        cfg.gridDim = dim3(static_cast<unsigned int>(rows) * 2); cfg.blockDim = dim3(CE_ROW_THREADS); cfg.stream = s;
         cudaLaunchAttribute attr{};
         attr.id = cudaLaunchAttributeClusterDimension;
-        attr.val.clusterDim.x = parts; attr.val.clusterDim.y = 1; attr.val.clusterDim.z = 1;
-        cfg.attrs = &attr; cfg.numAttrs = parts > 1 ? 1 : 0;
+        attr.val.clusterDim.x = 2; attr.val.clusterDim.y = 1; attr.val.clusterDim.z = 1;
+        cfg.attrs = &attr; cfg.numAttrs = 1;
         const cudaError_t e = cudaLaunchKernelEx(&cfg, fused_ce_row_kernel, static_cast<bf16*>(logits), losses, lse_out, targets, dloss, z_reg, rows, V, ld,
-                                                 write_dlogits, parts);
+                                                 write_dlogits);
         if (e != cudaSuccess) return static_cast<int>(e);
     } else if (dtype == 3) {
         if (ld % 4) return -1;
