@@ -274,7 +274,7 @@ attn_fwd_pingpong_kernel(const __grid_constant__ CUtensorMap tmap_qkv,     // qk
             // rate and then wait for the tensor pipe together.  A goes first; a warpgroup hands the turn over when its
             // exponentials are issued.  A's k-th wait (k >= 1) consumes B's arrival k-1, B's k-th wait A's arrival k.
             const int n_pair = (w.nB > 0 && p.turns) ? min(w.nA, w.nB) : 0;
-            float m_ref = -INFINITY, l_sum = 0.f;
+            float m_ref = -INFINITY, l_sum = 0.f, l4[4] = {0.f, 0.f, 0.f, 0.f};       // l4: head size 64 only, see below
             for (int j = 0; j < n && ok; ++j, ++tiles) {
                 if (!mbar_wait(s_full(x), tiles & 1, abort_flag)) { ok = false; break; }
                 tc_fence_after_sync();
@@ -306,6 +306,10 @@ attn_fwd_pingpong_kernel(const __grid_constant__ CUtensorMap tmap_qkv,     // qk
                     if (j > 0) {
                         const float alpha = need ? ex2((m_ref - m_new) * sl2) : 1.f;
                         l_sum *= alpha;
+                        if constexpr (HS == 64) {
+#pragma unroll
+                            for (int q = 0; q < 4; ++q) l4[q] *= alpha;
+                        }
                         if (!mbar_wait(o_done(x), (tiles - 1) & 1, abort_flag)) { ok = false; break; }      // PV of tile j-1 has landed
                         tc_fence_after_sync();
 #pragma unroll 1
@@ -332,11 +336,18 @@ attn_fwd_pingpong_kernel(const __grid_constant__ CUtensorMap tmap_qkv,     // qk
 #pragma unroll
                 for (int ch = 0; ch < 4; ++ch) {
                     uint32_t pw[16];
+                    float part = 0.f;
 #pragma unroll
                     for (int i = 0; i < 32; i += 2) {
                         const float p0 = ex2(fmaf(__uint_as_float(rs[ch * 32 + i]), sl2, -moff));         // masked scores are -inf -> 0
                         const float p1 = ex2(fmaf(__uint_as_float(rs[ch * 32 + i + 1]), sl2, -moff));
-                        sum0 += p0; sum1 += p1;
+                        if constexpr (HS == 64) {
+                            // with the early reference above, the row sum too is that of 64-key tiles: one sum per 16 columns of a tile
+                            part += p0 + p1;
+                            if (i == 14 || i == 30) { l4[(2 * ch + i / 16) % 4] += part; part = 0.f; }
+                        } else {
+                            sum0 += p0; sum1 += p1;
+                        }
                         pw[i / 2] = pack2(p0, p1);
                     }
                     tmem_st_32x32b_x16(tS + ch * 16, pw);
@@ -357,6 +368,7 @@ attn_fwd_pingpong_kernel(const __grid_constant__ CUtensorMap tmap_qkv,     // qk
             if (ok && n > 0) ok = mbar_wait(o_done(x), (tiles - 1) & 1, abort_flag);
             tc_fence_after_sync();
             if (ok && n > 0) {
+                if constexpr (HS == 64) l_sum = ((l4[0] + l4[1]) + l4[2]) + l4[3];
                 const float inv = 1.f / l_sum;
                 __nv_bfloat16* o = p.out + ((static_cast<long long>(b) * p.T + (row_ok ? row : 0)) * p.Hq + h) * HS;
 #pragma unroll 1

@@ -16,9 +16,8 @@
 // so no transposed copy is ever made.
 //
 // Backward is split into two deterministic kernels (no atomics):
-//   * dK/dV: one CTA per (batch, kv head, 128 keys) walks over the query heads of the group and all query blocks at or below the
-//     diagonal; dK and dV accumulate in TMEM across the whole walk.  With few such items up to four CTAs of a cluster share the
-//     heads and add their sums through distributed shared memory in a fixed order.
+//   * dK/dV: one CTA per (batch, kv head, 128 keys) walks over all query heads of the group and all query blocks at or below the
+//     diagonal; dK and dV accumulate in TMEM across the whole walk.
 //   * dQ   : one CTA per (batch, kv head, 128 queries) and part of the group walks over its query heads and their key blocks; dQ
 //     accumulates in TMEM and is drained once per head.
 // A small pre-pass computes delta = rowsum(dO * O).  Blocks with the longest walks are scheduled first.
@@ -26,7 +25,8 @@
 // Bound by the issue of the N = 64 MMAs (about 60 cycles each, 48 executing) and the waits between them: 1650 cycles per 64-row
 // tile of dK / dV where the MMAs alone take 1280, 1250 of dQ where they take 770.  8 x 2048 tokens, 28 / 4 heads of 128: dK / dV 543 ->
 // 431 us, dQ 515 -> 400 us; most of it from the warp-uniform issue (elect_one), which tensor-memory operands and one issuing warp
-// (MMAs execute in issue order, so the buffers need no barrier between them) made the remaining limit.
+// (MMAs execute in issue order, so the buffers need no barrier between them) made the remaining limit.  Score tiles of 128
+// columns (half as many MMAs, but no second score buffer) measured the same for dK / dV (416 us) and slower for dQ (486 us).
 #include <cstdlib>
 #include "ptx_sm100.cuh"
 #include "api.h"
@@ -152,18 +152,12 @@ __device__ __forceinline__ uint32_t pack_bf16x2(float lo, float hi) {
     return *reinterpret_cast<uint32_t*>(&h);
 }
 
-__device__ __forceinline__ float ld_cluster_f32(uint32_t cluster_addr) {
-    float v;
-    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(cluster_addr) : "memory");
-    return v;
-}
-
 template <int HS>
 __global__ void __launch_bounds__(kBwdThreads, 1)
 attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmap_kv128,   // qkv, box 128 rows (K and V tiles)
                      const __grid_constant__ CUtensorMap tmap_q64,     // qkv, box 64 rows (Q tiles)
                      const __grid_constant__ CUtensorMap tmap_do64,    // dO, box 64 rows
-                     const AttnParams p, const int heads_per_cta) {
+                     const AttnParams p) {
     constexpr int BKV = 128, BQ = 64, NCH = HS / 64, NBUF = 4;
     constexpr int KV_BYTES = BKV * HS * 2, Q_BYTES = BQ * HS * 2;
     constexpr uint32_t TMEM_COLS = 512;                       // S0 S1 | dP0 dP1 | dV | dK
@@ -185,19 +179,14 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmap_kv128,   // qkv, b
     const bool producer = warp == kBwdComputeWarps + 1;       // TMA loads (lane 0) and row statistics (all lanes)
     const int wg = tid >> 7, r = tid & 127;                   // compute threads: column slice, row of the tile (TMEM lane)
     if (smem_u32(smem) & 1023u) { if (tid == 0) atomicOr(p.status, kErrOther); return; }
-    // 1-D grid, key block slowest: the blocks with the longest walks (small kb) start first on every SM; `parts` CTAs of a
-    // cluster share the query heads of one (key block, kv head, batch) item
+    // 1-D grid, key block slowest: the blocks with the longest walks (small kb) start first on every SM
+    const int kb = blockIdx.x / (p.Hkv * p.B);
+    const int kvh = (blockIdx.x % (p.Hkv * p.B)) % p.Hkv, b = (blockIdx.x % (p.Hkv * p.B)) / p.Hkv;
     const int G = p.Hq / p.Hkv;
-    const int parts = (G + heads_per_cta - 1) / heads_per_cta;
-    const int item = blockIdx.x / parts, part = blockIdx.x % parts;
-    const int kb = item / (p.Hkv * p.B);
-    const int kvh = (item % (p.Hkv * p.B)) % p.Hkv, b = (item % (p.Hkv * p.B)) / p.Hkv;
-    const int h0 = kvh * G + part * heads_per_cta;              // query heads [h0, h0 + nh)
-    const int nh = min(heads_per_cta, G - part * heads_per_cta);
     const int kv0 = kb * BKV;
     const int nqb = (p.T + BQ - 1) / BQ;
     const int qb_first = kv0 / BQ;
-    const int n_it = (nqb - qb_first) * nh;
+    const int n_it = (nqb - qb_first) * G;
     const int kcol = (p.Hq + kvh) * HS, vcol = (p.Hq + p.Hkv + kvh) * HS;
 
     // barriers: 0 kv | 1-4 q/dO ring (TMA bytes + row statistics) | 5-6 scores ready | 7-8 P^T/dS^T in tensor memory | 9 all done
@@ -240,7 +229,7 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmap_kv128,   // qkv, b
                 }
             }
         }
-        int hq = h0, qb = qb_first;
+        int hq = kvh * G, qb = qb_first;
         for (int it = 0; it < n_it; ++it) {
             const int buf = it % NBUF;
             // lse and delta of the tile's 64 queries, two per lane; rows beyond the sequence get probability 0
@@ -384,7 +373,6 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmap_kv128,   // qkv, b
             const long long rbase = (static_cast<long long>(b) * p.T + (row_ok ? kv_row : 0)) * H;
             bf16* dk = p.dqkv + (rbase + p.Hq + kvh) * HS;
             bf16* dv = p.dqkv + (rbase + p.Hq + p.Hkv + kvh) * HS;
-            float* part_sum = reinterpret_cast<float*>(sQ);     // [dK, dV][HS columns][128 rows], over the Q / dO rings
             __syncwarp();
             constexpr int ECW = HS / kBwdWarpgroups;           // output columns per thread
 #pragma unroll
@@ -394,49 +382,12 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmap_kv128,   // qkv, b
                 tmem_ld_32x32b_x16(tdK + lane_off + col, rk);
                 tmem_ld_32x32b_x16(tdV + lane_off + col, rv);
                 tmem_ld_wait();
-                if (parts > 1) {
-#pragma unroll
-                    for (int i = 0; i < 16; ++i) {
-                        part_sum[(col + i) * BKV + r] = __uint_as_float(rk[i]);
-                        part_sum[(HS + col + i) * BKV + r] = __uint_as_float(rv[i]);
-                    }
-                } else if (row_ok) {
+                if (row_ok) {
                     store16_bf16(dk + col, rk);
                     store16_bf16(dv + col, rv);
                 }
             }
         }
-    }
-    if (parts > 1) {
-        // The CTAs of the cluster hold fp32 sums over their own query heads; each adds up a slice of the rows over all of
-        // them, in the order of the heads, and stores it.
-        __syncwarp();
-        cluster_arrive();
-        cluster_wait();
-        if (warp < kBwdComputeWarps) {
-            const int slice = (BKV + parts - 1) / parts, row0 = part * slice, rows = min(slice, BKV - row0);
-            const int H = p.Hq + 2 * p.Hkv;
-            const uint32_t base = smem_u32(sQ);
-            for (int i = tid; i < 2 * (HS / 8) * rows; i += kBwdComputeThreads) {
-                const int row = row0 + i % rows, grp = i / rows, which = grp / (HS / 8), col = (grp % (HS / 8)) * 8;
-                float v[8];
-#pragma unroll
-                for (int k = 0; k < 8; ++k) v[k] = 0.f;
-                for (int q = 0; q < parts; ++q) {
-                    const uint32_t src = map_to_cta(base + static_cast<uint32_t>(((which * HS + col) * BKV + row) * 4), q);
-#pragma unroll
-                    for (int k = 0; k < 8; ++k) v[k] += ld_cluster_f32(src + static_cast<uint32_t>(k * BKV * 4));
-                }
-                if (kv0 + row < p.T) {
-                    uint4 o = make_uint4(pack_bf16x2(v[0], v[1]), pack_bf16x2(v[2], v[3]), pack_bf16x2(v[4], v[5]), pack_bf16x2(v[6], v[7]));
-                    bf16* dst = p.dqkv + ((static_cast<long long>(b) * p.T + kv0 + row) * H + p.Hq + which * p.Hkv + kvh) * HS + col;
-                    *reinterpret_cast<uint4*>(dst) = o;
-                }
-            }
-        }
-        __syncwarp();
-        cluster_arrive();                                       // nobody leaves while its sums may still be read
-        cluster_wait();
     }
     tc_fence_before_sync();
     __syncthreads();
@@ -709,16 +660,16 @@ int device_sms() {
     return sms[dev & 63] > 0 ? sms[dev & 63] : 148;
 }
 
-// Query heads of a group that one CTA walks over; `base` = (row block, kv head, batch) items.  A CTA that walks a whole group pays
-// its start-up once and loads K / V (or keeps them) for all heads, but few items leave SMs idle: the group is cut into the fewest
-// parts that give 1.5 CTAs per SM, where the longest-first order evens the walks out.  Measured, kernel times in us (parts 1 / 2 / 3 /
-// 4 / 7):  dQ, 8 x 1024 tokens, 14 / 2 heads of 64 (128 items) 81 / 56 / 57 / 59 / 70;  4 x 1024 (64 items) 81 / 48 / 37 / 31 / 38;
-// 4 x 512 (32 items) 50 / 30 / 23 / 17 / 16;  8 x 2048, 28 / 4 heads of 128 (512 items) 398 / 390 / 407 / 415 / 494.
-// dK / dV, the same four: 87 / 64 / 86 / 84 / 155,  85 / 56 / 46 / 43 / 84,  48 / 32 / 26 / 19 / 41,  427 / 516 / 697 / 687 / 1216: its
-// parts are the CTAs of a cluster that meet at the end, and clusters of more than four no longer pack into a GPC's SMs.
-int heads_per_cta(int G, int base, int max_parts) {
+// Query heads of a group that one CTA of the dQ kernel walks over; `base` = (query block, kv head, batch) items.  A CTA that walks a
+// whole group pays its start-up once, but few items leave SMs idle: the group is cut into the fewest parts that give 1.5 CTAs per SM,
+// where the longest-first order evens the walks out.  Heads do not share sums, so the results do not depend on the cut.  Measured,
+// kernel times in us (parts 1 / 2 / 3 / 4 / 7): 8 x 1024 tokens, 14 / 2 heads of 64 (128 items) 81 / 56 / 57 / 59 / 70;  4 x 1024 (64
+// items) 81 / 48 / 37 / 31 / 38;  4 x 512 (32 items) 50 / 30 / 23 / 17 / 16;  8 x 2048, 28 / 4 heads of 128 (512 items) 398 / 390 / 407 /
+// 415 / 494.  dK / dV sum over the heads: cutting theirs (CTAs of a cluster that add up through distributed shared memory) was 1.3 to
+// 2.4 times as fast below 222 items, but the sums then round in another order, which was not wanted.
+int heads_per_cta(int G, int base) {
     int heads = G;
-    for (int parts = 1; parts <= G && parts <= max_parts; ++parts) {
+    for (int parts = 1; parts <= G; ++parts) {
         heads = (G + parts - 1) / parts;
         if (2 * base * ((G + heads - 1) / heads) >= 3 * device_sms()) break;
     }
@@ -750,22 +701,15 @@ int bwd_impl(void* dqkv, float* delta, const void* d_out, const void* out, const
         constexpr int smem = 2 * 128 * HS * 2 + 8 * 64 * HS * 2 + 8 * 64 * 4 + 256;
         rc = set_smem<1000 + HS>(attn_bwd_dkdv_kernel<HS>, smem);
         if (rc) return rc;
-        const int heads = heads_per_cta(G, base, 4), parts = (G + heads - 1) / heads;
-        cudaLaunchConfig_t cfg{};
-        cfg.gridDim = dim3(base * parts); cfg.blockDim = dim3(kBwdThreads); cfg.dynamicSmemBytes = smem; cfg.stream = s;
-        cudaLaunchAttribute attr{};
-        attr.id = cudaLaunchAttributeClusterDimension;
-        attr.val.clusterDim.x = parts; attr.val.clusterDim.y = 1; attr.val.clusterDim.z = 1;
-        cfg.attrs = &attr; cfg.numAttrs = parts > 1 ? 1 : 0;
-        const cudaError_t e = cudaLaunchKernelEx(&cfg, attn_bwd_dkdv_kernel<HS>, t128, t64, tdo64, p, heads);
-        rc = e == cudaSuccess ? LLMQ_LAUNCH_CHECK() : static_cast<int>(e);
+        attn_bwd_dkdv_kernel<HS><<<base, kBwdThreads, smem, s>>>(t128, t64, tdo64, p);
+        rc = LLMQ_LAUNCH_CHECK();
         if (rc) return rc;
     }
     {
         constexpr int smem = 8 * 64 * HS * 2 + 256;
         rc = set_smem<2000 + HS>(attn_bwd_dq_kernel<HS>, smem);
         if (rc) return rc;
-        const int heads = heads_per_cta(G, base, G);
+        const int heads = heads_per_cta(G, base);
         attn_bwd_dq_kernel<HS><<<base * ((G + heads - 1) / heads), kBwdThreads, smem, s>>>(t64, p, heads);
         rc = LLMQ_LAUNCH_CHECK();
     }
