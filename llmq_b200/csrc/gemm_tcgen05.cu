@@ -458,12 +458,23 @@ static int gemm_impl(const void* A, const void* B, void* C, const void* bias,
     // 1540: 17920 x 1536 x 16384 both operands 968-1062 / 1327 / 1435-1523, 16384 x 3584 x 4096 both 1052 / 1328 / 1520, B only 1352 / 1520 /
     // 1545, 4096^3 both 906 / 1184 / 1427.  With a ragged last chunk the 2-D boxes stay (its columns beyond the matrix would lie in the
     // next row), and for one chunk a 3-D box gains nothing.
-    // One-CTA kernel: 128-column tiles where 256-column ones fill less than half of the SMs.  They run twice as many CTAs with more
-    // stages in flight, and where that fills the GPU no split-K pass follows: 1152 x 896 x 1001 (both operands MN-major) and
-    // 1001 x 896 x 1152, the QKV gradients of a short batch, took 15 us each in two K parts
-    // and 4 more for their sum; they take 13 in one.
+    // One-CTA kernel: the K loop is cut into parts for outputs with fewer 256-column tiles than half of the SMs and a long K; where the
+    // GPU then still has room for twice as many CTAs the tiles are 128 columns wide (half the MMA time per stage, more stages in
+    // flight).  The cut depends on the 256-column tiles alone, so the sums have the same bits with both widths.  1001 x 896 x 1152 and
+    // 1152 x 896 x 1001, the QKV gradients of a short batch, launch included: 46 -> 20-24 us with the vector form of the second pass.
     const int tiles256 = ((M + BM - 1) / BM) * ((N + 255) / 256);
-    const int bn = (eb != 4 && 2 * tiles256 <= num_sms) ? 128 : 256;
+    const int k_iters = (K + bk - 1) / bk;
+    int splits = 1;
+    if (g_splitk_ws && tiles256 * 2 <= num_sms && k_iters >= 16) {
+        splits = num_sms / tiles256;
+        if (splits > 8) splits = 8;
+        if (splits > k_iters / 8) splits = k_iters / 8;
+        while (splits > 1 && static_cast<long long>(splits) * M * N > g_splitk_floats) --splits;
+        // every split must get at least one K step
+        while (splits > 1 && (splits - 1) * ((k_iters + splits - 1) / splits) >= k_iters) --splits;
+    }
+    const int tiles128 = ((M + BM - 1) / BM) * ((N + 127) / 128);
+    const int bn = (eb != 4 && tiles128 * splits <= num_sms) ? 128 : 256;
     const int b_rows = pair_kernel ? 128 : bn;
     const bool a_box3 = a_mn_major && eb < 4 && BM > bk && M % bk == 0, b_box3 = b_mn_major && eb < 4 && b_rows > bk && N % bk == 0;
     if (!a_mn_major) rc = llmq_encode_tmap_2d(&ta, A, eb, M, K, lda, BM);
@@ -518,19 +529,7 @@ static int gemm_impl(const void* A, const void* B, void* C, const void* bias,
         if (e != cudaSuccess) return static_cast<int>(e);
         attr_set[dev & 63] = true;
     }
-    const int tiles = ((M + BM - 1) / BM) * ((N + bn - 1) / bn);
-    const int k_iters = (K + bk - 1) / bk;
-    int splits = 1;
-    if (g_splitk_ws && tiles * 2 <= num_sms && k_iters >= 16) {
-        splits = num_sms / tiles;
-        if (splits > 8) splits = 8;
-        if (splits > k_iters / 8) splits = k_iters / 8;
-        while (splits > 1 && static_cast<long long>(splits) * M * N > g_splitk_floats) --splits;
-        // every split must get at least one K step
-        while (splits > 1 && (splits - 1) * ((k_iters + splits - 1) / splits) >= k_iters) --splits;
-        // the pass that adds the parts costs about as much as 32 K steps of a 128-column tile
-        if (bn == 128 && splits > 1 && k_iters - (k_iters + splits - 1) / splits < 32) splits = 1;
-    }
+    const int tiles = bn == 128 ? tiles128 : tiles256;
     if (splits > 1) { p.k_splits = splits; p.partial = g_splitk_ws; }
     const int items = tiles * splits;
     int grid = items < num_sms ? items : num_sms;
