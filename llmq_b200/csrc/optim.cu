@@ -77,7 +77,7 @@ template <> __device__ __forceinline__ void store8_srw<float>(float* p, const fl
 
 // One thread updates 8 consecutive parameters.  Bound by memory and by instruction issue at once: the 12 random words, 24 roundings
 // and conversions of a thread took longer than its loads and stores.  Roundings in pairs (sr_bf16x2) bring 67.9 M parameters with
-// bf16 state (950 MB) from 193 to 166-182 us.  For e4m3 first moments 16 consecutive threads share one
+// bf16 state (950 MB) from 193 to 157-182 us.  For e4m3 first moments 16 consecutive threads share one
 // fp32 scale (128 elements); the scale is recomputed from the new values every step.
 template <typename P, typename G, typename M, typename Vv>
 __device__ __forceinline__ void adamw_vec(long long i, bool active, P* __restrict__ param, const G* __restrict__ grad, M* __restrict__ m_state,
@@ -221,8 +221,7 @@ __device__ __forceinline__ float thread_sum_squares(const T* __restrict__ x, lon
     using V = Vec16<T>;
     const long long nvec = n / V::N, stride = static_cast<long long>(gridDim.x) * blockDim.x;
     long long i0 = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x;
-    // four loads of a thread in flight, four independent sums
-    float s4[4] = {0.f, 0.f, 0.f, 0.f};
+    float s = 0.f;                              // four loads of a thread in flight, added up in order
     for (; i0 + 3 * stride < nvec; i0 += 4 * stride) {
         V v[4];
 #pragma unroll
@@ -230,14 +229,13 @@ __device__ __forceinline__ float thread_sum_squares(const T* __restrict__ x, lon
 #pragma unroll
         for (int j = 0; j < 4; ++j)
 #pragma unroll
-            for (int k = 0; k < V::N; ++k) { const float f = to_float(v[j].v[k]); s4[j] += f * f; }
+            for (int k = 0; k < V::N; ++k) { const float f = to_float(v[j].v[k]); s += f * f; }
     }
     for (; i0 < nvec; i0 += stride) {
         V v = V::load_stream(x + i0 * V::N);
 #pragma unroll
-        for (int k = 0; k < V::N; ++k) { const float f = to_float(v.v[k]); s4[0] += f * f; }
+        for (int k = 0; k < V::N; ++k) { const float f = to_float(v.v[k]); s += f * f; }
     }
-    float s = (s4[0] + s4[1]) + (s4[2] + s4[3]);
     if (blockIdx.x == 0)
         for (long long i = nvec * V::N + threadIdx.x; i < n; i += blockDim.x) { float f = to_float(x[i]); s += f * f; }
     return s;
