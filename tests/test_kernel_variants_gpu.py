@@ -23,7 +23,7 @@ def rel(a, b):
     return ((a - b).norm() / b.norm().clamp_min(1e-30)).item()
 
 
-# one head per CTA and clusters of 2 .. 8 CTAs (small grids), whole groups per CTA (large grids), one query tile without a second
+# dQ with one head per CTA (few items), parts of a group, whole groups (many items); one query tile without a second
 @pytest.mark.parametrize("HS", [64, 128])
 @pytest.mark.parametrize("B,T,Hq,Hkv", [(1, 1, 2, 1), (1, 63, 3, 1), (2, 64, 4, 2), (1, 65, 14, 2), (1, 128, 7, 1), (3, 129, 5, 1), (1, 257, 8, 1),
                                         (1, 300, 16, 1), (2, 384, 6, 3), (1, 1000, 4, 4), (24, 130, 14, 7), (8, 1200, 12, 6)])
@@ -49,9 +49,9 @@ def test_attention_head_splits(HS, B, T, Hq, Hkv):
     assert rel(dqkv[:, :, Hq + Hkv:], x.grad[:, :, Hq + Hkv:]) < 1.2e-2
 
 
-# one thread vector, exactly full CTAs (512 x 5 vectors), one vector more (two CTAs), four and eight CTAs, the largest row that
-# eight hold, and one more (streaming kernel); tails behind the last whole vector
-@pytest.mark.parametrize("V", [8, 13, 4096, 20480, 20488, 40967, 81920, 128256, 163840, 163847, 163848, 200000])
+# less than a vector per thread of the cluster's two CTAs, whole rounds of four vectors a thread (32768) and not, tails behind the
+# last whole vector
+@pytest.mark.parametrize("V", [8, 13, 4096, 8192, 8200, 32768, 32776, 40967, 128256, 151936, 163847, 200000])
 @pytest.mark.parametrize("z_reg", [0.0, 1e-3])
 def test_fused_classifier_row_splits(V, z_reg):
     rows, ld = 5, (V + 7) // 8 * 8
@@ -89,9 +89,9 @@ def test_fused_classifier_rows_without_a_finite_maximum():
     assert lse[0].item() == -math.inf and math.isnan(lse[1].item()) and math.isnan(lse[2].item())
 
 
-# several rows side by side in a CTA, exactly one 512-thread row, rows of up to 1024 vectors, the two-pass kernels beyond
+# forward: rows of 1 .. 8 vectors per thread with 64 and with 256 threads, the two-pass kernel beyond; backward: 1, 2, 4 and 8 vectors
 @pytest.mark.parametrize("dtype", [BF, torch.float32])
-@pytest.mark.parametrize("C", [8, 264, 512, 896, 3584, 4096, 4104, 8192, 8200, 16384])
+@pytest.mark.parametrize("C", [8, 264, 512, 896, 2056, 3584, 4096, 4104, 8192, 8200, 16384])
 @pytest.mark.parametrize("rows", [1, 37, 700])
 def test_rmsnorm_row_splits(dtype, C, rows):
     if dtype == torch.float32 and C > 8192:
@@ -178,9 +178,9 @@ def test_gemm_mn_major_chunks(M, N, Kd, dt, a_mn, b_mn):
     assert rel(out, a.double() @ b.double().t()) < 1e-5    # exact products, fp32 sums
 
 
-# 128-column tiles (few output tiles), with and without a split of K, up to the first shape with 256-column tiles (75 of them)
+# 128-column tiles with and without a split of K, shapes on both sides of the line to 256-column tiles (148 tiles of 128 columns)
 @pytest.mark.parametrize("M,N,Kd", [(1, 8, 16), (129, 136, 320), (1001, 896, 1152), (896, 896, 4096), (1000, 2304, 208), (1152, 2048, 96), (9600, 256, 64),
-                                    (9472, 256, 64)])
+                                    (9472, 256, 64), (640, 2048, 1024), (1152, 896, 4096)])
 @pytest.mark.parametrize("dt", [BF, torch.float8_e4m3fn])
 @pytest.mark.parametrize("accumulate", [False, True])
 def test_gemm_tile_widths(M, N, Kd, dt, accumulate):
