@@ -6,14 +6,12 @@
 // scalar fallback kernel of the reference (src/kernels/cudnn_att.cpp:46-263, src/kernels/attention.cu).
 //
 // The forward kernel is in attention_fwd_pingpong.cu.  The two gradient kernels share one organisation.  A CTA owns a 128-row tile
-// (keys for dK / dV, queries for dQ) and has 18 warps: 16 compute warps (four warpgroups; thread (wg, r) owns row r = TMEM lane r
-// and a quarter of the columns of every score tile), one warp that issues all MMAs and one that issues the TMA loads.  Everything is
-// handed over through mbarriers (one arrival per warp); score tiles are double buffered in tensor memory, the streamed operand
-// (Q / dO for dK / dV, K / V for dQ) sits in a ring of four shared-memory buffers.  P^T, dS^T and dS never leave tensor memory: the
-// bf16 values take the place of the scores they were computed from and are the A operands of the accumulating MMAs, which saves the
-// shared-memory writes, the proxy fence and the A reads of a staged tile, and the wait for the MMAs that read the previous one.  Q and
-// dO of the dQ kernel are A operands in tensor memory too.  The shared-memory tile of V / K / Q / dO doubles as an MN-major B operand,
-// so no transposed copy is ever made.
+// (keys for dK / dV, queries for dQ) and walks over 64-column score tiles.  16 compute warps form two groups that take the tiles in
+// turn, two warps issue MMAs, the others load by TMA.  Everything is handed over through mbarriers (one arrival per warp); score tiles
+// are double buffered in tensor memory, the streamed operand (Q / dO for dK / dV, K / V for dQ) sits in a ring of shared-memory buffers.
+// P^T, dS^T and dS never leave tensor memory: the bf16 values take the place of the scores they were computed from and are the A
+// operands of the accumulating MMAs.  Q and dO of the dQ kernel, and with head size 64 K and V of the other one, are A operands in tensor
+// memory too.  The shared-memory tile of V / K / Q / dO doubles as an MN-major B operand, so no transposed copy is ever made.
 //
 // Backward is split into two deterministic kernels (no atomics):
 //   * dK/dV: one CTA per (batch, kv head, 128 keys) walks over all query heads of the group and all query blocks at or below the
@@ -22,11 +20,21 @@
 //     accumulates in TMEM and is drained once per head.
 // A small pre-pass computes delta = rowsum(dO * O).  Blocks with the longest walks are scheduled first.
 //
-// Bound by the issue of the N = 64 MMAs (about 60 cycles each, 48 executing) and the waits between them: 1650 cycles per 64-row
-// tile of dK / dV where the MMAs alone take 1280, 1250 of dQ where they take 770.  8 x 2048 tokens, 28 / 4 heads of 128: dK / dV 543 ->
-// 431 us, dQ 515 -> 400 us; most of it from the warp-uniform issue (elect_one), which tensor-memory operands and one issuing warp
-// (MMAs execute in issue order, so the buffers need no barrier between them) made the remaining limit.  Score tiles of 128
-// columns (half as many MMAs, but no second score buffer) measured the same for dK / dV (416 us) and slower for dQ (486 us).
+// What bounds it: no unit is saturated except the tensor pipe of dK / dV with head size 128 (1300 cycles of MMAs in about 1400 per tile;
+// 48 cycles per N = 64 MMA with both operands in shared memory, 33 with A in tensor memory, 64 per N = 128), the rest is the chain of
+// hand-overs of a tile.  A wait on an mbarrier costs a warp about 150 cycles even when the phase is complete, and several times that
+// while MMAs with both operands in shared memory run: those take nearly all of its bandwidth.  Hence two groups of compute warps, two
+// issuing warps, row statistics in few wide loads, and everything that comes from global memory (Q / dO and the statistics of the next
+// head or tile) fetched a tile or a head ahead by a warp of its own; the statistics that the producer used to wait for tile by tile alone
+// cost 10 to 20 % of dK / dV.  Kernel times in us, one group and one issuing warp -> now:
+//                                          dK / dV         dQ
+//   8 x 2048 tokens, 28 / 4 heads of 128   425 -> 364   403 -> 331
+//   1 x 8192, 32 / 8 heads of 128          880 -> 752   708 -> 620
+//   8 x 1024, 14 / 2 heads of 64            87 -> 68     56 -> 42
+//   2 x 4096, 32 / 8 heads of 64           368 -> 285   300 -> 221
+//   1 x 333, 12 / 2 heads of 128            37 -> 30     10 -> 9
+// Not better: score tiles of 128 columns without a second buffer; with head size 64 P^T in columns of its own and S issued before the sums
+// of the tile two before (dK / dV 68 -> 77: the groups then meet at the exponentials).
 #include <cstdlib>
 #include "ptx_sm100.cuh"
 #include "api.h"
@@ -37,13 +45,14 @@ using namespace sm100;
 namespace {
 
 constexpr float kLog2e = 1.4426950408889634f;
-// Backward kernels: four warpgroups share the 128 rows of a tile, each thread owns 16 score columns of its row, so
-// every scheduler has four warps to hide the latency of the exp / TMEM / shared-memory chain.
+// Backward kernels: two groups of two warpgroups; in a tile a thread of a group handles 32 score columns of its row(s)
 constexpr int kBwdWarpgroups = 4;
 constexpr int kBwdComputeThreads = 128 * kBwdWarpgroups;
 constexpr int kBwdComputeWarps = kBwdComputeThreads / 32;
-// + two helper warps: MMA issuer and TMA producer
-constexpr int kBwdThreads = kBwdComputeThreads + 64;
+constexpr int kBwdGroupWarps = kBwdComputeWarps / 2;              // two groups, alternating score tiles
+// + three helper warps: two MMA issuers and the TMA producer
+constexpr int kBwdThreads = kBwdComputeThreads + 96;
+constexpr int kBwdDqThreads = kBwdComputeThreads + 128;           // the dQ kernel has a second producer
 // One arrival per warp (512 single arrivals on one shared-memory word would serialise): the lanes' earlier
 // writes and fences are ordered before lane 0's releasing arrive by the warp barrier.
 __device__ __forceinline__ void warp_arrive(uint32_t bar) {
@@ -147,36 +156,44 @@ __device__ __forceinline__ uint32_t pack_bf16x2(float lo, float hi) {
 }
 
 // ------------------------------------------------------------------------------------------------
-// dK / dV.  Software pipeline over the (query head, query block) walk: while the threads turn S(it) / dP(it) into
-// P^T and dS^T, the tensor core already computes S(it+1) / dP(it+1) (score tiles are double buffered in TMEM) and
-// finishes dV / dK of tile it-1.  Q / dO tiles sit in a ring of four shared-memory buffers, loaded three tiles
-// ahead; P^T / dS^T go straight into the columns of the scores that they were computed from.
+// dK / dV.  Walk over the (query head, query block) tiles.  Q / dO tiles sit in a ring of shared-memory buffers, P^T / dS^T go back to
+// tensor memory.  The thread layout of the score tiles (16 x 256 bit TMEM accesses) gives a thread two of every eight columns of four
+// rows, so that the statistics of its columns are four 16-byte shared-memory loads a tile instead of sixteen: loads from shared
+// memory all but stop while MMAs with both operands there run.
+// With HS = 64 K and V live in tensor memory as A operands; with HS = 128 scores and accumulators fill it.
+template <int HS>
+struct DkdvShape {
+    static constexpr bool kTmemKV = HS == 64;
+    static constexpr int NBUF = HS == 64 ? 6 : 4;
+    static constexpr int KV_BYTES = 128 * HS * 2, Q_BYTES = 64 * HS * 2;
+    static constexpr int STAT_OFFSET = (kTmemKV ? 0 : 2 * KV_BYTES) + 2 * NBUF * Q_BYTES;
+    static constexpr int SMEM_BYTES = STAT_OFFSET + NBUF * 64 * 8 + 256;
+};
+
 template <int HS>
 __global__ void __launch_bounds__(kBwdThreads, 1)
 attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmap_kv128,   // qkv, box 128 rows (K and V tiles)
                      const __grid_constant__ CUtensorMap tmap_q64,     // qkv, box 64 rows (Q tiles)
                      const __grid_constant__ CUtensorMap tmap_do64,    // dO, box 64 rows
                      const AttnParams p) {
-    constexpr int BKV = 128, BQ = 64, NCH = HS / 64, NBUF = 4;
-    constexpr int KV_BYTES = BKV * HS * 2, Q_BYTES = BQ * HS * 2;
-    constexpr uint32_t TMEM_COLS = 512;                       // S0 S1 | dP0 dP1 | dV | dK
-    constexpr int CW = BQ / kBwdWarpgroups;                   // score columns per compute thread
-    static_assert(CW == 16, "the column split below is written for 16 columns per thread (one K step of the dV / dK MMAs)");
+    using Shape = DkdvShape<HS>;
+    constexpr int BKV = 128, BQ = 64, NCH = HS / 64, NBUF = Shape::NBUF;
+    constexpr int KV_BYTES = Shape::KV_BYTES, Q_BYTES = Shape::Q_BYTES;
+    constexpr bool kTmemKV = Shape::kTmemKV;
+    constexpr uint32_t TMEM_COLS = 512;                       // S0 S1 | dP0 dP1 | dV | dK (| K | V)
     extern __shared__ __align__(1024) uint8_t smem[];
-    uint8_t* sK = smem;
+    uint8_t* sK = smem;                                       // HS = 128
     uint8_t* sV = sK + KV_BYTES;
-    uint8_t* sQ = sV + KV_BYTES;              // NBUF buffers
-    uint8_t* sdO = sQ + NBUF * Q_BYTES;       // NBUF buffers
-    float* sLse = reinterpret_cast<float*>(sdO + NBUF * Q_BYTES);  // [NBUF][64] pre-multiplied by log2(e)
-    float* sDelta = sLse + NBUF * BQ;                              // [NBUF][64] pre-multiplied by the softmax scale
-    uint64_t* bars = reinterpret_cast<uint64_t*>(sDelta + NBUF * BQ);
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 16);
+    uint8_t* sQ = smem + (kTmemKV ? 0 : 2 * KV_BYTES);        // NBUF buffers
+    uint8_t* sdO = sQ + NBUF * Q_BYTES;                       // NBUF buffers
+    float2* sStat = reinterpret_cast<float2*>(smem + Shape::STAT_OFFSET);  // [NBUF][64] (lse * log2(e), delta * softmax scale)
+    uint64_t* bars = reinterpret_cast<uint64_t*>(sStat + NBUF * BQ);
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 28);
     volatile uint32_t* abort_flag = tmem_slot + 1;
 
     const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);       // uniform, and known to be
-    const bool issuer = warp == kBwdComputeWarps;             // MMA issuer (one elected lane); its only other work is waiting
-    const bool producer = warp == kBwdComputeWarps + 1;       // TMA loads (lane 0) and row statistics (all lanes)
-    const int wg = tid >> 7, r = tid & 127;                   // compute threads: column slice, row of the tile (TMEM lane)
+    const int role = warp - kBwdComputeWarps;                 // 0, 1: MMA issuers (one elected lane); 2: TMA loads and row statistics
+    const int wg = tid >> 7, r = tid & 127;                   // compute threads: warpgroup, TMEM lane
     if (smem_u32(smem) & 1023u) { if (tid == 0) atomicOr(p.status, kErrOther); return; }
     // 1-D grid, key block slowest: the blocks with the longest walks (small kb) start first on every SM
     const int kb = blockIdx.x / (p.Hkv * p.B);
@@ -188,39 +205,42 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmap_kv128,   // qkv, b
     const int n_it = (nqb - qb_first) * G;
     const int kcol = (p.Hq + kvh) * HS, vcol = (p.Hq + p.Hkv + kvh) * HS;
 
-    // barriers: 0 kv | 1-4 q/dO ring (TMA bytes + row statistics) | 5-6 scores ready | 7-8 P^T/dS^T in tensor memory | 9 all done
-    //           10-13 q/dO buffer free.  Two-entry sets alternate with the tile parity: the commit of tile it+2 needs every
-    //           compute warp to have handed over tile it, so a waiter can never miss a phase.
+    // barriers: 0 K / V in place | 1-2 S ready | 3-4 dP ready | 5-6 P^T in tensor memory | 7-8 dS^T in tensor memory | 9 all done |
+    //           10.. q/dO ring (TMA bytes + row statistics) | 16.. q/dO buffer free.  Two-entry sets alternate with the tile parity: the
+    //           commit of tile it+2 needs the group of tile it to have handed it over, so a waiter can never miss a phase.
     const uint32_t bar0 = smem_u32(bars);
     const uint32_t kv_bar = bar0, done_bar = bar0 + 72;
-    auto qdo_bar = [&](int buf) { return bar0 + 8 + 8 * buf; };
-    auto sp_bar = [&](int it) { return bar0 + 40 + 8 * (it & 1); };
-    auto p_ready = [&](int it) { return bar0 + 56 + 8 * (it & 1); };
-    auto qdo_free = [&](int buf) { return bar0 + 80 + 8 * buf; };
+    auto score_bar = [&](int which, int it) { return bar0 + 8 + 16 * which + 8 * (it & 1); };      // 0: S, 1: dP
+    auto ready_bar = [&](int which, int it) { return bar0 + 40 + 16 * which + 8 * (it & 1); };     // 0: P^T, 1: dS^T
+    auto qdo_bar = [&](int buf) { return bar0 + 80 + 8 * buf; };
+    auto qdo_free = [&](int buf) { return bar0 + 128 + 8 * buf; };
     if (tid == 0) {
-        mbar_init(kv_bar, 1); mbar_init(done_bar, 1);
-        for (int i = 0; i < NBUF; ++i) { mbar_init(qdo_bar(i), 2); mbar_init(qdo_free(i), 1); }
-        for (int i = 0; i < 2; ++i) { mbar_init(sp_bar(i), 1); mbar_init(p_ready(i), kBwdComputeWarps); }
+        mbar_init(kv_bar, kTmemKV ? kBwdComputeWarps : 1); mbar_init(done_bar, 2);
+        for (int i = 0; i < NBUF; ++i) { mbar_init(qdo_bar(i), 2); mbar_init(qdo_free(i), 2); }
+        for (int w = 0; w < 2; ++w)
+            for (int i = 0; i < 2; ++i) { mbar_init(score_bar(w, i), 1); mbar_init(ready_bar(w, i), kBwdGroupWarps); }
         *abort_flag = 0;
         mbar_init_fence();
     }
-    if (issuer) { tmem_alloc(smem_u32(tmem_slot), TMEM_COLS); tmem_relinquish(); }
+    if (role == 0) { tmem_alloc(smem_u32(tmem_slot), TMEM_COLS); tmem_relinquish(); }
     tc_fence_before_sync();
     __syncthreads();
     tc_fence_after_sync();
     const uint32_t tmem = *tmem_slot;
-    const uint32_t tdV = tmem + 4 * BQ, tdK = tmem + 4 * BQ + HS;
+    const uint32_t tdV = tmem + 4 * BQ, tdK = tdV + HS;
+    const uint32_t tK = tdK + HS, tV = tK + HS / 2;           // HS = 64
     const uint32_t lane_off = static_cast<uint32_t>((warp & 3) * 32) << 16;
     auto tS = [&](int it) { return tmem + (it & 1) * BQ; };
     auto tdP = [&](int it) { return tmem + 2 * BQ + (it & 1) * BQ; };
     bool ok = true;
 
-    if (producer) {
+    if (role == 2) {
         // ============================================================ TMA producer warp
         const int lane = tid & 31;
         if (lane == 0) {
-            tma_prefetch_desc(&tmap_kv128); tma_prefetch_desc(&tmap_q64); tma_prefetch_desc(&tmap_do64);
-            if (n_it > 0) {
+            tma_prefetch_desc(&tmap_q64); tma_prefetch_desc(&tmap_do64);
+            if (!kTmemKV && n_it > 0) {
+                tma_prefetch_desc(&tmap_kv128);
                 mbar_expect_tx(kv_bar, 2 * KV_BYTES);
                 for (int c = 0; c < NCH; ++c) {
                     tma_load_3d(smem_u32(sK) + c * (BKV * 128), &tmap_kv128, kv_bar, kcol + c * 64, kv0, b);
@@ -229,17 +249,21 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmap_kv128,   // qkv, b
             }
         }
         int hq = kvh * G, qb = qb_first;
-        for (int it = 0; it < n_it; ++it) {
-            const int buf = it % NBUF;
-            // lse and delta of the tile's 64 queries, two per lane; rows beyond the sequence get probability 0
-            float l2[2], dl[2];
+        // lse and delta of a tile's 64 queries, two per lane, read one tile ahead; rows beyond the sequence get probability 0
+        float2 stat[2], stat_next[2];
+        auto load_stats = [&](float2 (&st)[2]) {
 #pragma unroll
             for (int i = 0; i < 2; ++i) {
                 const int q = qb * BQ + lane + 32 * i;
                 const long long si = (static_cast<long long>(b) * p.Hq + hq) * p.T + q;
-                l2[i] = q < p.T ? __ldg(p.lse + si) * kLog2e : INFINITY;
-                dl[i] = q < p.T ? __ldg(p.delta + si) * p.scale : 0.f;
+                st[i] = q < p.T ? make_float2(__ldg(p.lse + si), __ldg(p.delta + si)) : make_float2(INFINITY, 0.f);
             }
+        };
+        if (n_it > 0) load_stats(stat);
+        for (int it = 0; it < n_it; ++it) {
+            const int buf = it % NBUF, hq_now = hq, qb_now = qb;
+            if (++qb == nqb) { qb = qb_first; ++hq; }
+            if (it + 1 < n_it) load_stats(stat_next);
             // the buffer's previous tile, it - NBUF, has been consumed by its dV / dK MMAs
             if (it >= NBUF) {
                 bool got = true;
@@ -249,64 +273,67 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmap_kv128,   // qkv, b
             if (lane == 0) {
                 mbar_expect_tx(qdo_bar(buf), 2 * Q_BYTES);
                 for (int c = 0; c < NCH; ++c) {
-                    tma_load_3d(smem_u32(sQ) + buf * Q_BYTES + c * (BQ * 128), &tmap_q64, qdo_bar(buf), hq * HS + c * 64, qb * BQ, b);
-                    tma_load_3d(smem_u32(sdO) + buf * Q_BYTES + c * (BQ * 128), &tmap_do64, qdo_bar(buf), hq * HS + c * 64, qb * BQ, b);
+                    tma_load_3d(smem_u32(sQ) + buf * Q_BYTES + c * (BQ * 128), &tmap_q64, qdo_bar(buf), hq_now * HS + c * 64, qb_now * BQ, b);
+                    tma_load_3d(smem_u32(sdO) + buf * Q_BYTES + c * (BQ * 128), &tmap_do64, qdo_bar(buf), hq_now * HS + c * 64, qb_now * BQ, b);
                 }
             }
 #pragma unroll
-            for (int i = 0; i < 2; ++i) { sLse[buf * BQ + lane + 32 * i] = l2[i]; sDelta[buf * BQ + lane + 32 * i] = dl[i]; }
+            for (int i = 0; i < 2; ++i) {
+                sStat[buf * BQ + lane + 32 * i] = make_float2(stat[i].x * kLog2e, stat[i].y * p.scale);
+                stat[i] = stat_next[i];
+            }
             warp_arrive(qdo_bar(buf));
-            if (++qb == nqb) { qb = qb_first; ++hq; }
         }
-    } else if (issuer) {
-        // ============================================================ MMA issuer warp
-        // One thread issues everything in the order S/dP(0), S/dP(1), dV/dK(0), S/dP(2), dV/dK(1), ...: MMAs of one CTA
-        // execute in issue order, so the scores of tile it+2 cannot overwrite the P^T / dS^T of tile it that live in the
-        // same columns, and the chain score tile -> probabilities has the time of 1280 tensor cycles to complete.
+    } else if (role >= 0) {
+        // ============================================================ MMA issuer warps
+        // Warp 0 issues S^T = K Q^T and dV += P^T dO, warp 1 dP^T = V dO^T and dK += dS^T Q: the same sequence, on other operands.  P^T (dS^T)
+        // of tile it lies in the buffer of S (dP) of tile it + 2; MMAs of one thread execute in issue order, so a buffer that a later MMA
+        // overwrites needs no barrier for the MMAs that read it.  One warp for both needs up to 1400 cycles a tile for its waits and the issue.
         if (n_it > 0) {
             const bool leader = elect_one();
-            const uint32_t idesc_st = make_instr_desc(1, 1, false, false, BKV, BQ);     // S^T = K Q^T, dP^T = V dO^T
-            const uint32_t idesc_acc = make_instr_desc(1, 1, false, true, BKV, HS);     // dV += P^T dO, dK += dS^T Q
-            const uint32_t k_lo = desc_lo(smem_u32(sK), 16), v_lo = desc_lo(smem_u32(sV), 16);
-            auto issue_sp = [&](int it) -> bool {
-                const int buf = it % NBUF;
-                if (!mbar_wait_warp(qdo_bar(buf), (it / NBUF) & 1, abort_flag)) return false;
-                tc_fence_after_sync();
-                const uint32_t q_lo = desc_lo(smem_u32(sQ) + buf * Q_BYTES, 16), do_lo = desc_lo(smem_u32(sdO) + buf * Q_BYTES, 16);
-                const uint32_t s_t = tS(it), dp_t = tdP(it), bar = sp_bar(it);
+            const uint32_t idesc_st = make_instr_desc(1, 1, false, false, BKV, BQ);
+            const uint32_t idesc_acc = make_instr_desc(1, 1, false, true, BKV, HS);
+            const uint32_t a_lo = desc_lo(smem_u32(role == 0 ? sK : sV), 16), a_tmem = role == 0 ? tK : tV;
+            const uint32_t b_score = desc_lo(smem_u32(role == 0 ? sQ : sdO), 16), b_acc = desc_lo(smem_u32(role == 0 ? sdO : sQ), BQ * 128);
+            const uint32_t t_score = role == 0 ? tS(0) : tdP(0), t_acc = role == 0 ? tdV : tdK;
+            auto issue_scores = [&](int it, int buf) {
+                const uint32_t d = t_score + (it & 1) * BQ, b_lo = b_score + buf * (Q_BYTES >> 4), bar = score_bar(role, it);
                 if (leader) {
 #pragma unroll
-                    for (int k = 0; k < HS / 16; ++k)
-                        mma_issue<false, false>(s_t, k_lo + (((k / 4) * (BKV * 128) + (k % 4) * 32) >> 4), kDescHi,
-                                                q_lo + (((k / 4) * (BQ * 128) + (k % 4) * 32) >> 4), kDescHi, idesc_st, k > 0);
-#pragma unroll
-                    for (int k = 0; k < HS / 16; ++k)
-                        mma_issue<false, false>(dp_t, v_lo + (((k / 4) * (BKV * 128) + (k % 4) * 32) >> 4), kDescHi,
-                                                do_lo + (((k / 4) * (BQ * 128) + (k % 4) * 32) >> 4), kDescHi, idesc_st, k > 0);
+                    for (int k = 0; k < HS / 16; ++k) {
+                        const uint32_t bk = b_lo + (((k / 4) * (BQ * 128) + (k % 4) * 32) >> 4);
+                        if constexpr (kTmemKV) mma_issue_f16_tmem_a(d, a_tmem + k * 8, bk, kDescHi, idesc_st, k > 0);
+                        else mma_issue<false, false>(d, a_lo + (((k / 4) * (BKV * 128) + (k % 4) * 32) >> 4), kDescHi, bk, kDescHi, idesc_st, k > 0);
+                    }
                     mma_commit(bar);
                 }
                 __syncwarp();
-                return true;
             };
-            ok = mbar_wait_warp(kv_bar, 0, abort_flag) && issue_sp(0);
-            for (int it = 0; it < n_it && ok; ++it) {
-                if (it + 1 < n_it) ok = issue_sp(it + 1);
-                if (!ok || !mbar_wait_warp(p_ready(it), (it >> 1) & 1, abort_flag)) { ok = false; break; }
+            ok = mbar_wait_warp(kv_bar, 0, abort_flag);
+            for (int it = 0; it < 2 && it < n_it && ok; ++it) {
+                ok = mbar_wait_warp(qdo_bar(it), 0, abort_flag);
                 tc_fence_after_sync();
-                const int buf = it % NBUF;
-                const uint32_t q_lo = desc_lo(smem_u32(sQ) + buf * Q_BYTES, BQ * 128), do_lo = desc_lo(smem_u32(sdO) + buf * Q_BYTES, BQ * 128);
-                const uint32_t s_t = tS(it), dp_t = tdP(it), bar = qdo_free(buf);
+                if (ok) issue_scores(it, it);
+            }
+            for (int it = 0; it < n_it && ok; ++it) {
+                const int buf = it % NBUF, buf2 = (it + 2) % NBUF;
+                const uint32_t phase2 = ((it + 2) / NBUF) & 1;
+                const bool loaded = it + 2 < n_it && mbar_test_wait(qdo_bar(buf2), phase2);          // asked early, answered by the time it is needed
+                if (!mbar_wait_warp(ready_bar(role, it), (it >> 1) & 1, abort_flag)) { ok = false; break; }
+                tc_fence_after_sync();
+                const uint32_t b_lo = b_acc + buf * (Q_BYTES >> 4), a_t = t_score + (it & 1) * BQ, bar = qdo_free(buf);
                 const uint32_t acc0 = it > 0;
                 if (leader) {
 #pragma unroll
                     for (int k = 0; k < BQ / 16; ++k)
-                        mma_issue_f16_tmem_a(tdV, s_t + k * CW, do_lo + ((k * (16 * 128)) >> 4), kDescHi, idesc_acc, k > 0 ? 1u : acc0);
-#pragma unroll
-                    for (int k = 0; k < BQ / 16; ++k)
-                        mma_issue_f16_tmem_a(tdK, dp_t + k * CW, q_lo + ((k * (16 * 128)) >> 4), kDescHi, idesc_acc, k > 0 ? 1u : acc0);
+                        mma_issue_f16_tmem_a(t_acc, a_t + k * 16, b_lo + ((k * (16 * 128)) >> 4), kDescHi, idesc_acc, k > 0 ? 1u : acc0);
                     mma_commit(bar);
                 }
                 __syncwarp();
+                if (it + 2 < n_it) {
+                    if (!__all_sync(0xffffffffu, loaded)) ok = mbar_wait_warp(qdo_bar(buf2), phase2, abort_flag);
+                    if (ok) issue_scores(it + 2, buf2);
+                }
             }
             if (leader) {
                 if (ok) mma_commit(done_bar);
@@ -316,51 +343,95 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmap_kv128,   // qkv, b
         }
     } else {
         // ============================================================ compute warps
+        // Two groups of two warpgroups take turns: group g works on the tiles of parity g, warpgroup `half` of it on 32 of their columns.
         const float sl2 = p.scale * kLog2e;
+        const int lane = tid & 31, grp = wg >> 1, half = wg & 1;
         const int kv_row = kv0 + r;
-        const int c0 = wg * CW;
-        int qb = qb_first;
-        for (int it = 0; it < n_it; ++it) {
+        if constexpr (kTmemKV) {
+            // rows of K (group 0) and V (group 1) into tensor memory, 16 packed words per thread; zeros beyond the sequence
+            if (n_it > 0) {
+                uint32_t w[16];
+#pragma unroll
+                for (int i = 0; i < 16; ++i) w[i] = 0u;
+                if (kv_row < p.T) {
+                    const uint4* src = reinterpret_cast<const uint4*>(p.qkv + (static_cast<long long>(b) * p.T + kv_row) * (p.Hq + 2 * p.Hkv) * HS +
+                                                                      (grp == 0 ? kcol : vcol) + half * 32);
+#pragma unroll
+                    for (int q4 = 0; q4 < 4; ++q4) {
+                        const uint4 x = __ldg(src + q4);
+                        w[4 * q4] = x.x; w[4 * q4 + 1] = x.y; w[4 * q4 + 2] = x.z; w[4 * q4 + 3] = x.w;
+                    }
+                }
+                __syncwarp();
+                tmem_st_32x32b_x16((grp == 0 ? tK : tV) + lane_off + half * 16, w);
+                tmem_st_wait();
+                tc_fence_before_sync();
+                warp_arrive(kv_bar);
+            }
+        }
+        int qb = qb_first + grp;
+        while (qb >= nqb) qb -= nqb - qb_first;
+        const int row_l = (warp & 3) * 32 + (lane >> 2), col_l = half * 32 + 2 * (lane & 3);  // tile row / column of this thread's first value
+        for (int it = grp; it < n_it; it += 2) {
             const int buf = it % NBUF;
-            if (!mbar_wait(sp_bar(it), (it >> 1) & 1, abort_flag) || !mbar_wait(qdo_bar(buf), (it / NBUF) & 1, abort_flag)) { ok = false; break; }
+            if (!mbar_wait(qdo_bar(buf), (it / NBUF) & 1, abort_flag)) { ok = false; break; }
+            float4 st[4];                                       // (lse, delta) of columns col_l + 8 i and + 1
+#pragma unroll
+            for (int i = 0; i < 4; ++i) st[i] = *reinterpret_cast<const float4*>(sStat + buf * BQ + col_l + 8 * i);
+            if (!mbar_wait(score_bar(0, it), (it >> 1) & 1, abort_flag)) { ok = false; break; }
             tc_fence_after_sync();
-            uint32_t rs[CW], rp[CW];
+            float pv[2][16];                                    // 16-row halves: [4 i + 2 r8 + c] = row + 8 r8, column 8 i + c
             __syncwarp();
-            tmem_ld_32x32b_x16(tS(it) + lane_off + c0, rs);
-            tmem_ld_32x32b_x16(tdP(it) + lane_off + c0, rp);
-            const float* lse_t = sLse + buf * BQ + c0;
-            const float* delta_t = sDelta + buf * BQ + c0;
-            float lse_c[CW], del_c[CW];
 #pragma unroll
-            for (int i = 0; i < CW; i += 4) {
-                *reinterpret_cast<float4*>(lse_c + i) = *reinterpret_cast<const float4*>(lse_t + i);
-                *reinterpret_cast<float4*>(del_c + i) = *reinterpret_cast<const float4*>(delta_t + i);
-            }
+            for (int h = 0; h < 2; ++h) tmem_ld_16x256b_x4(tS(it) + lane_off + (h << 20) + half * 32, *reinterpret_cast<uint32_t(*)[16]>(pv[h]));
             tmem_ld_wait();
-            float pv[CW], ds[CW];
 #pragma unroll
-            for (int i = 0; i < CW; ++i) {
-                pv[i] = fast_exp2(fmaf(__uint_as_float(rs[i]), sl2, -lse_c[i]));
-                ds[i] = fmaf(__uint_as_float(rp[i]), p.scale, -del_c[i]);
-            }
+            for (int h = 0; h < 2; ++h)
+#pragma unroll
+                for (int i = 0; i < 16; ++i) pv[h][i] = fast_exp2(fmaf(pv[h][i], sl2, -((i & 1) ? st[i / 4].z : st[i / 4].x)));
             if (qb * BQ < kv0 + BKV) {                          // only tiles that touch the diagonal pay for the mask
-                const int lim = kv_row - qb * BQ - c0;          // columns below lim are above the diagonal (q < kv)
+                const int lim = kv0 + row_l - qb * BQ - col_l;  // columns below lim (+ the row's offset) are above the diagonal (q < kv)
 #pragma unroll
-                for (int i = 0; i < CW; ++i) if (i < lim) pv[i] = 0.f;
-            }
-            uint32_t ptp[CW / 2], dsp[CW / 2];
+                for (int h = 0; h < 2; ++h)
 #pragma unroll
-            for (int i = 0; i < CW; i += 2) {
-                ptp[i / 2] = pack_bf16x2(pv[i], pv[i + 1]);
-                dsp[i / 2] = pack_bf16x2(pv[i] * ds[i], pv[i + 1] * ds[i + 1]);
+                    for (int i = 0; i < 16; ++i) if (8 * (i / 4) + (i & 1) < lim + 16 * h + 8 * ((i >> 1) & 1)) pv[h][i] = 0.f;
             }
-            // Into the first half of the very columns this thread has just read: one K step of 16 queries per warpgroup
-            tmem_st_32x32b_x8(tS(it) + lane_off + c0, ptp);
-            tmem_st_32x32b_x8(tdP(it) + lane_off + c0, dsp);
+#pragma unroll
+            for (int h = 0; h < 2; ++h)
+#pragma unroll
+                for (int k = 0; k < 2; ++k) {                   // K steps of 16 queries
+                    const float* v = pv[h] + 8 * k;
+                    tmem_st_16x128b_x2(tS(it) + lane_off + (h << 20) + (2 * half + k) * 16, pack_bf16x2(v[0], v[1]), pack_bf16x2(v[2], v[3]),
+                                       pack_bf16x2(v[4], v[5]), pack_bf16x2(v[6], v[7]));
+                }
             tmem_st_wait();
             tc_fence_before_sync();
-            warp_arrive(p_ready(it));
-            if (++qb == nqb) qb = qb_first;
+            warp_arrive(ready_bar(0, it));
+            if (!mbar_wait(score_bar(1, it), (it >> 1) & 1, abort_flag)) { ok = false; break; }
+            tc_fence_after_sync();
+            uint32_t rp[2][16];
+            __syncwarp();
+#pragma unroll
+            for (int h = 0; h < 2; ++h) tmem_ld_16x256b_x4(tdP(it) + lane_off + (h << 20) + half * 32, rp[h]);
+            tmem_ld_wait();
+#pragma unroll
+            for (int h = 0; h < 2; ++h)
+#pragma unroll
+                for (int k = 0; k < 2; ++k) {
+                    uint32_t d[4];
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) {               // j = 2 (column group) + (row + 8)
+                        const int i = 8 * k + 2 * j;
+                        d[j] = pack_bf16x2(pv[h][i] * fmaf(__uint_as_float(rp[h][i]), p.scale, -st[i / 4].y),
+                                           pv[h][i + 1] * fmaf(__uint_as_float(rp[h][i + 1]), p.scale, -st[i / 4].w));
+                    }
+                    tmem_st_16x128b_x2(tdP(it) + lane_off + (h << 20) + (2 * half + k) * 16, d[0], d[1], d[2], d[3]);
+                }
+            tmem_st_wait();
+            tc_fence_before_sync();
+            warp_arrive(ready_bar(1, it));
+            qb += 2;
+            while (qb >= nqb) qb -= nqb - qb_first;
         }
         if (ok && n_it > 0) ok = mbar_wait(done_bar, 0, abort_flag);
         tc_fence_after_sync();
@@ -391,34 +462,44 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmap_kv128,   // qkv, b
     tc_fence_before_sync();
     __syncthreads();
     tc_fence_after_sync();
-    if (issuer) tmem_dealloc(tmem, TMEM_COLS);
+    if (role == 0) tmem_dealloc(tmem, TMEM_COLS);
 }
 
 // ------------------------------------------------------------------------------------------------
 // dQ.  One CTA owns 128 query rows and walks over `heads_per_cta` query heads of one kv head, and for every head over
 // the key tiles up to the diagonal.  Q and dO of the current head live in tensor memory as the A operands of the score
-// MMAs (they are constant during a key walk), K / V tiles stream through a ring of four shared-memory buffers three
-// tiles ahead of the MMAs, S / dP are double buffered in TMEM, dS takes the place of the dP tile it was computed from
-// (A operand of dQ += dS K), dQ accumulates in TMEM and is drained once per head while the scores of the next head's
-// first tile are computed.
+// MMAs (they are constant during a key walk), K / V tiles stream through a ring of shared-memory buffers, S / dP are double buffered in
+// TMEM, dS takes the place of the dP tile it was computed from (A operand of dQ += dS K), dQ accumulates in TMEM and is drained once
+// per head while the scores of the next head's first tiles are computed.
 template <int HS>
-__global__ void __launch_bounds__(kBwdThreads, 1)
-attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmap_kv64,    // qkv, box 64 rows
+struct DqShape {
+    static constexpr int NBUF = HS == 64 ? 6 : 4;
+    static constexpr int KV_BYTES = 64 * HS * 2, Q_BYTES = 128 * HS * 2;
+    static constexpr int STAT_OFFSET = 2 * NBUF * KV_BYTES + 2 * Q_BYTES;
+    static constexpr int SMEM_BYTES = STAT_OFFSET + 128 * 8 + 256;
+};
+
+template <int HS>
+__global__ void __launch_bounds__(kBwdDqThreads, 1)
+attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmap_qkv64,   // qkv, box 64 rows (K, V and Q tiles)
+                   const __grid_constant__ CUtensorMap tmap_do64,    // dO, box 64 rows
                    const AttnParams p, const int heads_per_cta) {
-    constexpr int BQ = 128, BKV = 64, NCH = HS / 64, NBUF = 4;
-    constexpr int KV_BYTES = BKV * HS * 2;
+    constexpr int BQ = 128, BKV = 64, NCH = HS / 64, NBUF = DqShape<HS>::NBUF;
+    constexpr int KV_BYTES = DqShape<HS>::KV_BYTES, Q_BYTES = DqShape<HS>::Q_BYTES;
     constexpr uint32_t TMEM_COLS = 512;                       // Q | dO (bf16 pairs, A operands) | S0 S1 | dP0 dP1 | dQ
-    constexpr int CW = BKV / kBwdWarpgroups;
-    static_assert(CW == 16, "the column split below is written for 16 columns per thread (one K step of the dQ MMA)");
+    constexpr int CW = 16;                                    // columns of one K step of the dQ MMA
     extern __shared__ __align__(1024) uint8_t smem[];
     uint8_t* sK = smem;                       // NBUF buffers
     uint8_t* sV = sK + NBUF * KV_BYTES;       // NBUF buffers
-    uint64_t* bars = reinterpret_cast<uint64_t*>(sV + NBUF * KV_BYTES);
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 18);
+    uint8_t* sQ = sV + NBUF * KV_BYTES;       // Q and dO of the next head, on their way to tensor memory
+    uint8_t* sdO = sQ + Q_BYTES;
+    float2* sStat = reinterpret_cast<float2*>(smem + DqShape<HS>::STAT_OFFSET);   // (lse * log2(e), delta * softmax scale) of its rows
+    uint64_t* bars = reinterpret_cast<uint64_t*>(sStat + BQ);
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 28);
     volatile uint32_t* abort_flag = tmem_slot + 1;
 
     const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);       // uniform, and known to be
-    const bool issuer = warp == kBwdComputeWarps, producer = warp == kBwdComputeWarps + 1;
+    const int role = warp - kBwdComputeWarps;                 // 0, 1: MMA issuers (one elected lane); 2: TMA loads of K / V, 3: of Q / dO and row statistics
     const int wg = tid >> 7, r = tid & 127;
     if (smem_u32(smem) & 1023u) { if (tid == 0) atomicOr(p.status, kErrOther); return; }
     const int nqb = (p.T + BQ - 1) / BQ;
@@ -435,23 +516,28 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmap_kv64,    // qkv, box
     const int total = n_kv * nh;                                // tiles of the whole walk, t = g * n_kv + j
     const int kcol = (p.Hq + kvh) * HS, vcol = (p.Hq + p.Hkv + kvh) * HS;
 
-    // barriers: 0 head_ready | 1-4 k/v ring | 5-6 S ready | 7-8 dP ready | 9-10 dS in tensor memory | 11 dQ of a head done
-    //           12 dQ of a head drained | 13-16 k/v buffer free.  Two-entry sets alternate with the tile parity.
+    // barriers: 0 Q of a head in place | 1 dO of a head in place | 2-3 S ready | 4-5 dP ready | 6-7 dS in tensor memory | 8-9 S has been
+    //           read | 10 dQ of a head done | 11 dQ of a head drained | 12.. k/v ring | 18.. k/v buffer free | 24 Q / dO of a head staged |
+    //           25 staging free.  Two-entry sets alternate with the tile parity.
     const uint32_t bar0 = smem_u32(bars);
-    const uint32_t head_ready = bar0, dq_bar = bar0 + 88, dq_drained = bar0 + 96;
-    auto kv_bar = [&](int buf) { return bar0 + 8 + 8 * buf; };
-    auto s_bar = [&](int t) { return bar0 + 40 + 8 * (t & 1); };
-    auto dp_bar = [&](int t) { return bar0 + 56 + 8 * (t & 1); };
-    auto p_ready = [&](int t) { return bar0 + 72 + 8 * (t & 1); };
-    auto kv_free = [&](int buf) { return bar0 + 104 + 8 * buf; };
+    const uint32_t q_ready = bar0, do_ready = bar0 + 8, dq_bar = bar0 + 80, dq_drained = bar0 + 88;
+    auto s_bar = [&](int t) { return bar0 + 16 + 8 * (t & 1); };
+    auto dp_bar = [&](int t) { return bar0 + 32 + 8 * (t & 1); };
+    auto p_ready = [&](int t) { return bar0 + 48 + 8 * (t & 1); };
+    auto s_free = [&](int t) { return bar0 + 64 + 8 * (t & 1); };
+    auto kv_bar = [&](int buf) { return bar0 + 96 + 8 * buf; };
+    auto kv_free = [&](int buf) { return bar0 + 144 + 8 * buf; };
+    const uint32_t staged = bar0 + 192, stage_free = bar0 + 200;
     if (tid == 0) {
-        mbar_init(head_ready, kBwdComputeWarps); mbar_init(dq_drained, kBwdComputeWarps); mbar_init(dq_bar, 1);
+        mbar_init(q_ready, kBwdGroupWarps); mbar_init(do_ready, kBwdGroupWarps);
+        mbar_init(dq_drained, kBwdGroupWarps); mbar_init(dq_bar, 1);
+        mbar_init(staged, 2); mbar_init(stage_free, kBwdComputeWarps);
         for (int i = 0; i < NBUF; ++i) { mbar_init(kv_bar(i), 1); mbar_init(kv_free(i), 1); }
-        for (int i = 0; i < 2; ++i) { mbar_init(s_bar(i), 1); mbar_init(dp_bar(i), 1); mbar_init(p_ready(i), kBwdComputeWarps); }
+        for (int i = 0; i < 2; ++i) { mbar_init(s_bar(i), 1); mbar_init(dp_bar(i), 1); mbar_init(p_ready(i), kBwdGroupWarps); mbar_init(s_free(i), kBwdGroupWarps); }
         *abort_flag = 0;
         mbar_init_fence();
     }
-    if (issuer) { tmem_alloc(smem_u32(tmem_slot), TMEM_COLS); tmem_relinquish(); }
+    if (role == 0) { tmem_alloc(smem_u32(tmem_slot), TMEM_COLS); tmem_relinquish(); }
     tc_fence_before_sync();
     __syncthreads();
     tc_fence_after_sync();
@@ -462,10 +548,10 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmap_kv64,    // qkv, box
     const uint32_t lane_off = static_cast<uint32_t>((warp & 3) * 32) << 16;
     bool ok = true;
 
-    if (producer) {
+    if (role == 2) {
         // ============================================================ TMA producer warp
         if ((tid & 31) == 0 && total > 0) {
-            tma_prefetch_desc(&tmap_kv64);
+            tma_prefetch_desc(&tmap_qkv64);
             int j = 0;
             for (int t = 0; t < total; ++t) {
                 const int buf = t % NBUF;
@@ -473,160 +559,227 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmap_kv64,    // qkv, box
                 if (t >= NBUF && !mbar_wait(kv_free(buf), ((t / NBUF) - 1) & 1, abort_flag)) { atomicOr(p.status, kErrOther); break; }
                 mbar_expect_tx(kv_bar(buf), 2 * KV_BYTES);
                 for (int c = 0; c < NCH; ++c) {
-                    tma_load_3d(smem_u32(sK) + buf * KV_BYTES + c * (BKV * 128), &tmap_kv64, kv_bar(buf), kcol + c * 64, j * BKV, b);
-                    tma_load_3d(smem_u32(sV) + buf * KV_BYTES + c * (BKV * 128), &tmap_kv64, kv_bar(buf), vcol + c * 64, j * BKV, b);
+                    tma_load_3d(smem_u32(sK) + buf * KV_BYTES + c * (BKV * 128), &tmap_qkv64, kv_bar(buf), kcol + c * 64, j * BKV, b);
+                    tma_load_3d(smem_u32(sV) + buf * KV_BYTES + c * (BKV * 128), &tmap_qkv64, kv_bar(buf), vcol + c * 64, j * BKV, b);
                 }
                 if (++j == n_kv) j = 0;
             }
         }
-    } else if (issuer) {
-        // ============================================================ MMA issuer warp
-        // As in the dK / dV kernel one thread issues everything: S/dP(t+1) before dQ(t), except that the first tile of a
-        // head (which needs that head's Q / dO in tensor memory) comes after the last dQ MMA of the previous head.
+    } else if (role == 3) {
+        // ============================================================ Q / dO of a head at a time, while the head before is worked on
+        const int lane = tid & 31;
+        if (lane == 0) { tma_prefetch_desc(&tmap_qkv64); tma_prefetch_desc(&tmap_do64); }
+        for (int g = 0; g < nh && total > 0; ++g) {
+            const int hq = h0 + g;
+            float2 st[4];                                       // rows beyond the sequence get probability 0
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const int q = q0 + lane + 32 * i;
+                const long long si = (static_cast<long long>(b) * p.Hq + hq) * p.T + q;
+                st[i] = q < p.T ? make_float2(__ldg(p.lse + si), __ldg(p.delta + si)) : make_float2(INFINITY, 0.f);
+            }
+            if (g > 0 && !mbar_wait_warp(stage_free, (g - 1) & 1, abort_flag)) { if (lane == 0) atomicOr(p.status, kErrOther); break; }
+            if (lane == 0) {
+                mbar_expect_tx(staged, 2 * Q_BYTES);
+                for (int c = 0; c < NCH; ++c)
+                    for (int h = 0; h < 2; ++h) {
+                        const uint32_t off = c * (BQ * 128) + h * (64 * 128);
+                        tma_load_3d(smem_u32(sQ) + off, &tmap_qkv64, staged, hq * HS + c * 64, q0 + h * 64, b);
+                        tma_load_3d(smem_u32(sdO) + off, &tmap_do64, staged, hq * HS + c * 64, q0 + h * 64, b);
+                    }
+            }
+#pragma unroll
+            for (int i = 0; i < 4; ++i) sStat[lane + 32 * i] = make_float2(st[i].x * kLog2e, st[i].y * p.scale);
+            warp_arrive(staged);
+        }
+    } else if (role >= 0) {
+        // ============================================================ MMA issuer warps
+        // Warp 0 issues S two tiles ahead of the sums (its buffer is free once the scores have been read), across the heads: Q of the next
+        // head comes when the last S of the head before is complete.  Warp 1 issues dQ += dS K and then dP two tiles ahead into the buffer
+        // of the dS just read; dO of the next head comes after the last dP of a head, so its first tiles follow the head's last sums.
         if (total > 0) {
             const bool leader = elect_one();
             const uint32_t idesc_s = make_instr_desc(1, 1, false, false, BQ, BKV);
             const uint32_t idesc_dq = make_instr_desc(1, 1, false, true, BQ, HS);
-            auto issue_sp = [&](int t) -> bool {
-                const int buf = t % NBUF;
-                if (!mbar_wait_warp(kv_bar(buf), (t / NBUF) & 1, abort_flag)) return false;
-                tc_fence_after_sync();
-                const uint32_t k_lo = desc_lo(smem_u32(sK) + buf * KV_BYTES, 16), v_lo = desc_lo(smem_u32(sV) + buf * KV_BYTES, 16);
-                const uint32_t s_t = tS(t), dp_t = tdP(t), sb = s_bar(t), db = dp_bar(t);
+            auto scores = [&](uint32_t d, uint32_t a, uint32_t b_lo, uint32_t bar) {
                 if (leader) {
 #pragma unroll
                     for (int k = 0; k < HS / 16; ++k)
-                        mma_issue_f16_tmem_a(s_t, tQ + k * 8, k_lo + (((k / 4) * (BKV * 128) + (k % 4) * 32) >> 4), kDescHi, idesc_s, k > 0);
-                    mma_commit(sb);                              // the exponentials start while dP is still being computed
-#pragma unroll
-                    for (int k = 0; k < HS / 16; ++k)
-                        mma_issue_f16_tmem_a(dp_t, tdO + k * 8, v_lo + (((k / 4) * (BKV * 128) + (k % 4) * 32) >> 4), kDescHi, idesc_s, k > 0);
-                    mma_commit(db);
+                        mma_issue_f16_tmem_a(d, a + k * 8, b_lo + (((k / 4) * (BKV * 128) + (k % 4) * 32) >> 4), kDescHi, idesc_s, k > 0);
+                    mma_commit(bar);
                 }
                 __syncwarp();
-                return true;
             };
-            ok = mbar_wait_warp(head_ready, 0, abort_flag) && issue_sp(0);
-            int t = 0;
-            for (int g = 0; g < nh && ok; ++g) {
-                for (int j = 0; j < n_kv && ok; ++j, ++t) {
-                    if (j + 1 < n_kv && !issue_sp(t + 1)) { ok = false; break; }
-                    if (!mbar_wait_warp(p_ready(t), (t >> 1) & 1, abort_flag)) { ok = false; break; }
-                    // the first dQ MMA of a head overwrites the accumulator: the previous head's must have been read
-                    if (j == 0 && g > 0 && !mbar_wait_warp(dq_drained, (g - 1) & 1, abort_flag)) { ok = false; break; }
+            if (role == 0) {
+                const uint32_t k_lo = desc_lo(smem_u32(sK), 16);
+                int j = 0, head = 0, buf = 0;
+                uint32_t phase = 0;
+                for (int t = 0; t < total; ++t) {
+                    const bool loaded = mbar_test_wait(kv_bar(buf), phase);
+                    if (j == 0) ok = mbar_wait_warp(q_ready, head & 1, abort_flag);
+                    if (ok && t >= 2) ok = mbar_wait_warp(s_free(t), ((t - 2) >> 1) & 1, abort_flag);
+                    if (ok && !__all_sync(0xffffffffu, loaded)) ok = mbar_wait_warp(kv_bar(buf), phase, abort_flag);
+                    if (!ok) break;
                     tc_fence_after_sync();
-                    const int buf = t % NBUF;
-                    const uint32_t k_lo = desc_lo(smem_u32(sK) + buf * KV_BYTES, BKV * 128), dp_t = tdP(t), bar = kv_free(buf);
-                    const uint32_t acc0 = j > 0;
-                    if (leader) {
-#pragma unroll
-                        for (int k = 0; k < BKV / 16; ++k)
-                            mma_issue_f16_tmem_a(tdQ, dp_t + k * CW, k_lo + ((k * (16 * 128)) >> 4), kDescHi, idesc_dq, k > 0 ? 1u : acc0);
-                        mma_commit(bar);
-                    }
-                    __syncwarp();
+                    scores(tS(t), tQ, k_lo + buf * (KV_BYTES >> 4), s_bar(t));
+                    if (++buf == NBUF) { buf = 0; phase ^= 1u; }
+                    if (++j == n_kv) { j = 0; ++head; }
                 }
-                if (!ok) break;
-                if (leader) mma_commit(dq_bar);
-                __syncwarp();
-                if (g + 1 < nh) ok = mbar_wait_warp(head_ready, (g + 1) & 1, abort_flag) && issue_sp(t);
+            } else {
+                const uint32_t k_lo = desc_lo(smem_u32(sK), BKV * 128), v_lo = desc_lo(smem_u32(sV), 16);
+                int dp = 0, dp_buf = 0;                         // next dP tile
+                uint32_t dp_phase = 0;
+                // dP tiles up to tile `upto`, before tile `end`
+                auto issue_dp = [&](int upto, int end, bool loaded) -> bool {
+                    for (; dp <= upto && dp < end; ++dp) {
+                        if (!__all_sync(0xffffffffu, loaded) && !mbar_wait_warp(kv_bar(dp_buf), dp_phase, abort_flag)) return false;
+                        tc_fence_after_sync();
+                        scores(tdP(dp), tdO, v_lo + dp_buf * (KV_BYTES >> 4), dp_bar(dp));
+                        if (++dp_buf == NBUF) { dp_buf = 0; dp_phase ^= 1u; }
+                        loaded = false;
+                    }
+                    return true;
+                };
+                ok = mbar_wait_warp(do_ready, 0, abort_flag) && issue_dp(1, n_kv, false);
+                int t = 0, buf = 0;
+                for (int g = 0; g < nh && ok; ++g) {
+                    const int head_end = (g + 1) * n_kv;
+                    for (int j = 0; j < n_kv; ++j, ++t) {
+                        const bool loaded = t + 2 < head_end && mbar_test_wait(kv_bar(dp_buf), dp_phase);
+                        if (!mbar_wait_warp(p_ready(t), (t >> 1) & 1, abort_flag)) { ok = false; break; }
+                        // the first dQ MMA of a head overwrites the accumulator: the previous head's must have been read
+                        if (j == 0 && g > 0 && !mbar_wait_warp(dq_drained, (g - 1) & 1, abort_flag)) { ok = false; break; }
+                        tc_fence_after_sync();
+                        const uint32_t b_lo = k_lo + buf * (KV_BYTES >> 4), dp_t = tdP(t), bar = kv_free(buf);
+                        const uint32_t acc0 = j > 0;
+                        if (leader) {
+#pragma unroll
+                            for (int k = 0; k < BKV / 16; ++k)
+                                mma_issue_f16_tmem_a(tdQ, dp_t + k * CW, b_lo + ((k * (16 * 128)) >> 4), kDescHi, idesc_dq, k > 0 ? 1u : acc0);
+                            mma_commit(bar);
+                        }
+                        __syncwarp();
+                        if (++buf == NBUF) buf = 0;
+                        if (!issue_dp(t + 2, head_end, loaded)) { ok = false; break; }
+                    }
+                    if (!ok) break;
+                    if (leader) mma_commit(dq_bar);
+                    __syncwarp();
+                    if (g + 1 < nh) ok = mbar_wait_warp(do_ready, (g + 1) & 1, abort_flag) && issue_dp(t + 1, head_end + n_kv, false);
+                }
             }
             if (!ok && leader) { *abort_flag = 1u; atomicOr(p.status, kErrOther); }
             __syncwarp();
         }
     } else {
         // ============================================================ compute warps
+        // Two groups of two warpgroups take turns: group g works on the tiles of parity g, a thread on 32 columns of its row.
         const float sl2 = p.scale * kLog2e;
         const int row = q0 + r;
         const bool row_ok = row < p.T;
-        const int c0 = wg * CW;
+        const int grp = wg >> 1, c0 = (wg & 1) * 2 * CW;
         const int H = p.Hq + 2 * p.Hkv;
-        const bool stores_qdo = wg < HS / 32;                   // uniform per warp: the TMEM stores are warp-collective
-        constexpr int ECW = HS / kBwdWarpgroups;                // dQ columns per thread
-        // this thread's 32-element slices of the Q and dO rows of head hq (16 packed words each) and its row statistics
-        auto load_qdo = [&](int hq, uint32_t (&wq)[16], uint32_t (&wo)[16], float& lse2, float& delta_s) {
-            const long long si = (static_cast<long long>(b) * p.Hq + hq) * p.T + row;
-            lse2 = row_ok ? p.lse[si] * kLog2e : INFINITY;
-            delta_s = row_ok ? p.delta[si] * p.scale : 0.f;
-            if (stores_qdo && row_ok) {
-                const uint4* gq = reinterpret_cast<const uint4*>(p.qkv + ((static_cast<long long>(b) * p.T + row) * H + hq) * HS + wg * 32);
-                const uint4* go = reinterpret_cast<const uint4*>(p.d_out + ((static_cast<long long>(b) * p.T + row) * p.Hq + hq) * HS + wg * 32);
+        constexpr int ECW = HS / 2;                             // dQ columns per thread
+        // Q and dO of head g are moved to tensor memory by one group each: dO by the group of the last tile before the head, Q by the other
+        // one, which is through with its last tile earlier.  A thread moves half a row, and reads the statistics of its row.
+        auto writes_do = [&](int g) { return ((g * n_kv - 1) & 1) == grp; };
+        float lse2 = 0.f, delta_s = 0.f;
+        auto move_half_row = [&](int g) -> bool {
+            if (!mbar_wait(staged, g & 1, abort_flag)) return false;
+            const bool is_do = writes_do(g);
+            const uint8_t* src = (is_do ? sdO : sQ) + r * 128;
 #pragma unroll
-                for (int q4 = 0; q4 < 4; ++q4) {
-                    const uint4 x = __ldg(gq + q4), y = __ldg(go + q4);
-                    wq[4 * q4] = x.x; wq[4 * q4 + 1] = x.y; wq[4 * q4 + 2] = x.z; wq[4 * q4 + 3] = x.w;
-                    wo[4 * q4] = y.x; wo[4 * q4 + 1] = y.y; wo[4 * q4 + 2] = y.z; wo[4 * q4 + 3] = y.w;
+            for (int c = 0; c < HS / 64; ++c) {                 // 32 elements: four 16-byte pieces, swizzled
+                const int e = (wg & 1) * (HS / 2) + c * 32;     // first element
+                uint32_t w[16];
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    const uint4 x = *reinterpret_cast<const uint4*>(src + (e / 64) * (BQ * 128) + ((((e % 64) / 8 + i) ^ (r & 7)) << 4));
+                    w[4 * i] = x.x; w[4 * i + 1] = x.y; w[4 * i + 2] = x.z; w[4 * i + 3] = x.w;
                 }
-            } else {
-#pragma unroll
-                for (int q4 = 0; q4 < 16; ++q4) { wq[q4] = 0u; wo[q4] = 0u; }
+                __syncwarp();
+                tmem_st_32x32b_x16((is_do ? tdO : tQ) + lane_off + e / 2, w);
             }
-        };
-        auto store_qdo = [&](const uint32_t (&wq)[16], const uint32_t (&wo)[16]) {
-            __syncwarp();
-            if (stores_qdo) {
-                tmem_st_32x32b_x16(tQ + lane_off + wg * 16, wq);
-                tmem_st_32x32b_x16(tdO + lane_off + wg * 16, wo);
-                tmem_st_wait();
-            }
+            const float2 st = sStat[r];
+            lse2 = st.x; delta_s = st.y;
+            tmem_st_wait();
             tc_fence_before_sync();
-            warp_arrive(head_ready);
+            warp_arrive(is_do ? do_ready : q_ready);
+            warp_arrive(stage_free);
+            return true;
         };
-        uint32_t wq[16], wo[16];
-        float lse2, delta_s, lse2_next = 0.f, delta_next = 0.f;
-        load_qdo(h0, wq, wo, lse2, delta_s);
-        store_qdo(wq, wo);
-        int t = 0;
+        ok = total > 0 && move_half_row(0);
         for (int g = 0; g < nh && ok; ++g) {
-            if (g + 1 < nh) load_qdo(h0 + g + 1, wq, wo, lse2_next, delta_next);     // prefetch: consumed when this head's walk is over
-            for (int j = 0; j < n_kv; ++j, ++t) {
+            const int t0 = g * n_kv;
+            for (int j = (t0 & 1) ^ grp; j < n_kv; j += 2) {
+                const int t = t0 + j;
                 if (!mbar_wait(s_bar(t), (t >> 1) & 1, abort_flag)) { ok = false; break; }
                 tc_fence_after_sync();
-                uint32_t rv[CW];
-                float pv[CW];
+                float pv[2][CW];
                 __syncwarp();
-                tmem_ld_32x32b_x16(tS(t) + lane_off + c0, rv);
-                tmem_ld_wait();
 #pragma unroll
-                for (int i = 0; i < CW; ++i) pv[i] = fast_exp2(fmaf(__uint_as_float(rv[i]), sl2, -lse2));
+                for (int h = 0; h < 2; ++h) tmem_ld_32x32b_x16(tS(t) + lane_off + c0 + h * CW, *reinterpret_cast<uint32_t(*)[CW]>(pv[h]));
+                tmem_ld_wait();
+                tc_fence_before_sync();
+                warp_arrive(s_free(t));
+#pragma unroll
+                for (int h = 0; h < 2; ++h)
+#pragma unroll
+                    for (int i = 0; i < CW; ++i) pv[h][i] = fast_exp2(fmaf(pv[h][i], sl2, -lse2));
                 if ((j + 1) * BKV > q0) {
                     const int lim = row - j * BKV - c0;         // columns above lim are beyond the diagonal (kv > q)
 #pragma unroll
-                    for (int i = 0; i < CW; ++i) if (i > lim) pv[i] = 0.f;
+                    for (int h = 0; h < 2; ++h)
+#pragma unroll
+                        for (int i = 0; i < CW; ++i) if (h * CW + i > lim) pv[h][i] = 0.f;
                 }
                 if (!mbar_wait(dp_bar(t), (t >> 1) & 1, abort_flag)) { ok = false; break; }
                 tc_fence_after_sync();
                 __syncwarp();
-                tmem_ld_32x32b_x16(tdP(t) + lane_off + c0, rv);
-                tmem_ld_wait();
-                uint32_t dsp[CW / 2];
 #pragma unroll
-                for (int i = 0; i < CW; i += 2)
-                    dsp[i / 2] = pack_bf16x2(pv[i] * fmaf(__uint_as_float(rv[i]), p.scale, -delta_s),
-                                             pv[i + 1] * fmaf(__uint_as_float(rv[i + 1]), p.scale, -delta_s));
-                // into the first half of the columns this thread has just read: one K step of 16 keys per warpgroup
-                tmem_st_32x32b_x8(tdP(t) + lane_off + c0, dsp);
+                for (int h = 0; h < 2; ++h) {
+                    uint32_t rv[CW], dsp[CW / 2];
+                    tmem_ld_32x32b_x16(tdP(t) + lane_off + c0 + h * CW, rv);
+                    tmem_ld_wait();
+#pragma unroll
+                    for (int i = 0; i < CW; i += 2)
+                        dsp[i / 2] = pack_bf16x2(pv[h][i] * fmaf(__uint_as_float(rv[i]), p.scale, -delta_s),
+                                                 pv[h][i + 1] * fmaf(__uint_as_float(rv[i + 1]), p.scale, -delta_s));
+                    // into the first half of the 16 columns this thread has just read: one K step of the dQ MMA
+                    tmem_st_32x32b_x8(tdP(t) + lane_off + c0 + h * CW, dsp);
+                }
                 tmem_st_wait();
                 tc_fence_before_sync();
                 warp_arrive(p_ready(t));
             }
             if (!ok) break;
-            // ---- the head's walk is over.  Its last dP tile is complete, so every MMA that reads Q / dO is: hand over the
-            // next head's, then drain dQ while the tensor core works on the next head's first scores.
-            if (g + 1 < nh) { store_qdo(wq, wo); lse2 = lse2_next; delta_s = delta_next; }
+            // ---- this group's part of the head's walk is over.  Q / dO of the next head may be written once the last MMA that reads this
+            // head's is complete: the last S tile (the other group's, waited for here) for Q, the last dP tile for dO.
+            if (g + 1 < nh) {
+                const int tl = t0 + n_kv - 1;
+                if (!mbar_wait(writes_do(g + 1) ? dp_bar(tl) : s_bar(tl), (tl >> 1) & 1, abort_flag)) { ok = false; break; }
+                tc_fence_after_sync();
+                if (!move_half_row(g + 1)) { ok = false; break; }
+            }
+            // Then the group of the last tile drains dQ; the other one is already at the next head's first tile.
+            if (!writes_do(g + 1)) continue;
             if (!mbar_wait(dq_bar, g & 1, abort_flag)) { ok = false; break; }
             tc_fence_after_sync();
-            uint32_t acc[ECW];
+            bf16* dq = p.dqkv + ((static_cast<long long>(b) * p.T + row) * H + h0 + g) * HS + (wg & 1) * ECW;
             __syncwarp();
 #pragma unroll
-            for (int c = 0; c < ECW; c += 16) tmem_ld_32x32b_x16(tdQ + lane_off + wg * ECW + c, *reinterpret_cast<uint32_t(*)[16]>(acc + c));
-            tmem_ld_wait();
-            tc_fence_before_sync();
-            warp_arrive(dq_drained);
-            if (row_ok) {
-                bf16* dq = p.dqkv + ((static_cast<long long>(b) * p.T + row) * H + h0 + g) * HS + wg * ECW;
-#pragma unroll
-                for (int c = 0; c < ECW; c += 16) store16_bf16(dq + c, *reinterpret_cast<const uint32_t(*)[16]>(acc + c));
+            for (int c = 0; c < ECW; c += 32) {
+                uint32_t acc[32];
+                tmem_ld_32x32b_x32(tdQ + lane_off + (wg & 1) * ECW + c, acc);
+                tmem_ld_wait();
+                if (c + 32 == ECW) {
+                    tc_fence_before_sync();
+                    warp_arrive(dq_drained);
+                }
+                if (row_ok) {
+                    store16_bf16(dq + c, *reinterpret_cast<const uint32_t(*)[16]>(acc));
+                    store16_bf16(dq + c + 16, *reinterpret_cast<const uint32_t(*)[16]>(acc + 16));
+                }
             }
         }
         if (!ok && r == 0) atomicOr(p.status, kErrOther);
@@ -634,7 +787,7 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmap_kv64,    // qkv, box
     tc_fence_before_sync();
     __syncthreads();
     tc_fence_after_sync();
-    if (issuer) tmem_dealloc(tmem, TMEM_COLS);
+    if (role == 0) tmem_dealloc(tmem, TMEM_COLS);
 }
 
 // Tag makes the static flag unique per kernel instantiation (several kernels share one signature).
@@ -697,7 +850,7 @@ int bwd_impl(void* dqkv, float* delta, const void* d_out, const void* out, const
     p.qkv = static_cast<const bf16*>(qkv); p.d_out = static_cast<const bf16*>(d_out);
     const int base = ((T + 127) / 128) * Hkv * B, G = Hq / Hkv;
     {
-        constexpr int smem = 2 * 128 * HS * 2 + 8 * 64 * HS * 2 + 8 * 64 * 4 + 256;
+        constexpr int smem = DkdvShape<HS>::SMEM_BYTES;
         rc = set_smem<1000 + HS>(attn_bwd_dkdv_kernel<HS>, smem);
         if (rc) return rc;
         attn_bwd_dkdv_kernel<HS><<<base, kBwdThreads, smem, s>>>(t128, t64, tdo64, p);
@@ -705,11 +858,11 @@ int bwd_impl(void* dqkv, float* delta, const void* d_out, const void* out, const
         if (rc) return rc;
     }
     {
-        constexpr int smem = 8 * 64 * HS * 2 + 256;
+        constexpr int smem = DqShape<HS>::SMEM_BYTES;
         rc = set_smem<2000 + HS>(attn_bwd_dq_kernel<HS>, smem);
         if (rc) return rc;
         const int heads = heads_per_cta(G, base);
-        attn_bwd_dq_kernel<HS><<<base * ((G + heads - 1) / heads), kBwdThreads, smem, s>>>(t64, p, heads);
+        attn_bwd_dq_kernel<HS><<<base * ((G + heads - 1) / heads), kBwdDqThreads, smem, s>>>(t64, tdo64, p, heads);
         rc = LLMQ_LAUNCH_CHECK();
     }
     return rc;
