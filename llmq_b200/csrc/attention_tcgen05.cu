@@ -15,7 +15,7 @@
 //
 // Backward is split into two deterministic kernels (no atomics):
 //   * dK/dV: one CTA per (batch, kv head, 128 keys) walks over all query heads of the group and all query blocks at or below the
-//     diagonal; dK and dV accumulate in TMEM across the whole walk.
+//     diagonal; dK and dV accumulate in TMEM across the whole walk.  With few items a cluster shares the heads (head_parts).
 //   * dQ   : one CTA per (batch, kv head, 128 queries) and part of the group walks over its query heads and their key blocks; dQ
 //     accumulates in TMEM and is drained once per head.
 // A small pre-pass computes delta = rowsum(dO * O).  Blocks with the longest walks are scheduled first.
@@ -155,6 +155,12 @@ __device__ __forceinline__ uint32_t pack_bf16x2(float lo, float hi) {
     return *reinterpret_cast<uint32_t*>(&h);
 }
 
+__device__ __forceinline__ float4 ld_cluster_f32x4(uint32_t addr) {
+    float4 v;
+    asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr) : "memory");
+    return v;
+}
+
 // ------------------------------------------------------------------------------------------------
 // dK / dV.  Walk over the (query head, query block) tiles.  Q / dO tiles sit in a ring of shared-memory buffers, P^T / dS^T go back to
 // tensor memory.  The thread layout of the score tiles (16 x 256 bit TMEM accesses) gives a thread two of every eight columns of four
@@ -175,7 +181,7 @@ __global__ void __launch_bounds__(kBwdThreads, 1)
 attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmap_kv128,   // qkv, box 128 rows (K and V tiles)
                      const __grid_constant__ CUtensorMap tmap_q64,     // qkv, box 64 rows (Q tiles)
                      const __grid_constant__ CUtensorMap tmap_do64,    // dO, box 64 rows
-                     const AttnParams p) {
+                     const AttnParams p, const int parts) {            // CTAs of a cluster that share the query heads of an item
     using Shape = DkdvShape<HS>;
     constexpr int BKV = 128, BQ = 64, NCH = HS / 64, NBUF = Shape::NBUF;
     constexpr int KV_BYTES = Shape::KV_BYTES, Q_BYTES = Shape::Q_BYTES;
@@ -196,13 +202,15 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmap_kv128,   // qkv, b
     const int wg = tid >> 7, r = tid & 127;                   // compute threads: warpgroup, TMEM lane
     if (smem_u32(smem) & 1023u) { if (tid == 0) atomicOr(p.status, kErrOther); return; }
     // 1-D grid, key block slowest: the blocks with the longest walks (small kb) start first on every SM
-    const int kb = blockIdx.x / (p.Hkv * p.B);
-    const int kvh = (blockIdx.x % (p.Hkv * p.B)) % p.Hkv, b = (blockIdx.x % (p.Hkv * p.B)) / p.Hkv;
+    const int item = blockIdx.x / parts, part = blockIdx.x % parts;
+    const int kb = item / (p.Hkv * p.B);
+    const int kvh = (item % (p.Hkv * p.B)) % p.Hkv, b = (item % (p.Hkv * p.B)) / p.Hkv;
     const int G = p.Hq / p.Hkv;
+    const int h0 = kvh * G + G * part / parts, nh = G * (part + 1) / parts - G * part / parts;      // query heads [h0, h0 + nh)
     const int kv0 = kb * BKV;
     const int nqb = (p.T + BQ - 1) / BQ;
     const int qb_first = kv0 / BQ;
-    const int n_it = (nqb - qb_first) * G;
+    const int n_it = (nqb - qb_first) * nh;
     const int kcol = (p.Hq + kvh) * HS, vcol = (p.Hq + p.Hkv + kvh) * HS;
 
     // barriers: 0 K / V in place | 1-2 S ready | 3-4 dP ready | 5-6 P^T in tensor memory | 7-8 dS^T in tensor memory | 9 all done |
@@ -232,6 +240,7 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmap_kv128,   // qkv, b
     const uint32_t lane_off = static_cast<uint32_t>((warp & 3) * 32) << 16;
     auto tS = [&](int it) { return tmem + (it & 1) * BQ; };
     auto tdP = [&](int it) { return tmem + 2 * BQ + (it & 1) * BQ; };
+    uint4* const sums = reinterpret_cast<uint4*>(smem);       // parts > 1: [dK, dV][128 rows][32] after the walk
     bool ok = true;
 
     if (role == 2) {
@@ -248,7 +257,7 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmap_kv128,   // qkv, b
                 }
             }
         }
-        int hq = kvh * G, qb = qb_first;
+        int hq = h0, qb = qb_first;
         // lse and delta of a tile's 64 queries, two per lane, read one tile ahead; rows beyond the sequence get probability 0
         float2 stat[2], stat_next[2];
         auto load_stats = [&](float2 (&st)[2]) {
@@ -439,10 +448,8 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmap_kv128,   // qkv, b
         if (ok && n_it > 0) {
             // The TMEM loads are warp-collective: every lane executes them, only the stores are predicated.
             const bool row_ok = kv_row < p.T;
-            const int H = p.Hq + 2 * p.Hkv;
-            const long long rbase = (static_cast<long long>(b) * p.T + (row_ok ? kv_row : 0)) * H;
-            bf16* dk = p.dqkv + (rbase + p.Hq + kvh) * HS;
-            bf16* dv = p.dqkv + (rbase + p.Hq + p.Hkv + kvh) * HS;
+            bf16* dk = p.dqkv + ((static_cast<long long>(b) * p.T + (row_ok ? kv_row : 0)) * (p.Hq + 2 * p.Hkv)) * HS + kcol;
+            bf16* dv = dk + (vcol - kcol);
             __syncwarp();
             constexpr int ECW = HS / kBwdWarpgroups;           // output columns per thread
 #pragma unroll
@@ -452,11 +459,47 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmap_kv128,   // qkv, b
                 tmem_ld_32x32b_x16(tdK + lane_off + col, rk);
                 tmem_ld_32x32b_x16(tdV + lane_off + col, rv);
                 tmem_ld_wait();
-                if (row_ok) {
+                if (HS == 128 && parts > 1) {
+                    // every MMA and load of this CTA is complete: the sums of its heads go over K, V and the ring, rows of 32 16-byte
+                    // pieces, swizzled
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) {
+                        const int at = r * 32 + ((col / 4 + i) ^ lane);
+                        sums[at] = make_uint4(rk[4 * i], rk[4 * i + 1], rk[4 * i + 2], rk[4 * i + 3]);
+                        sums[128 * 32 + at] = make_uint4(rv[4 * i], rv[4 * i + 1], rv[4 * i + 2], rv[4 * i + 3]);
+                    }
+                } else if (row_ok) {
                     store16_bf16(dk + col, rk);
                     store16_bf16(dv + col, rv);
                 }
             }
+        }
+    }
+    if constexpr (HS == 128) {
+        if (parts > 1) {
+            // Rows [part * 128 / parts, ...) of dK and dV: the sum over the cluster's CTAs, in the order of their heads
+            __syncwarp();
+            cluster_arrive();
+            cluster_wait();
+            if (role < 0) {
+                const int row0 = 128 * part / parts, rows = 128 * (part + 1) / parts - row0;
+                for (int i = tid; i < rows * 64; i += kBwdComputeThreads) {
+                    const int what = (i >> 5) & 1, row = row0 + (i >> 6), c4 = i & 31;       // dK / dV, row, four columns
+                    const uint32_t local = smem_u32(sums + what * 128 * 32 + row * 32 + (c4 ^ (row & 31)));
+                    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+                    for (int q = 0; q < parts; ++q) {
+                        const float4 x = ld_cluster_f32x4(map_to_cta(local, q));
+                        v.x += x.x; v.y += x.y; v.z += x.z; v.w += x.w;
+                    }
+                    if (ok && kv0 + row < p.T) {
+                        bf16* dst = p.dqkv + ((static_cast<long long>(b) * p.T + kv0 + row) * (p.Hq + 2 * p.Hkv)) * HS + (what == 0 ? kcol : vcol) + 4 * c4;
+                        *reinterpret_cast<uint2*>(dst) = make_uint2(pack_bf16x2(v.x, v.y), pack_bf16x2(v.z, v.w));
+                    }
+                }
+            }
+            __syncwarp();
+            cluster_arrive();                                 // the others may still read this CTA's sums
+            cluster_wait();
         }
     }
     tc_fence_before_sync();
@@ -817,8 +860,7 @@ int device_sms() {
 // where the longest-first order evens the walks out.  Heads do not share sums, so the results do not depend on the cut.  Measured,
 // kernel times in us (parts 1 / 2 / 3 / 4 / 7): 8 x 1024 tokens, 14 / 2 heads of 64 (128 items) 81 / 56 / 57 / 59 / 70;  4 x 1024 (64
 // items) 81 / 48 / 37 / 31 / 38;  4 x 512 (32 items) 50 / 30 / 23 / 17 / 16;  8 x 2048, 28 / 4 heads of 128 (512 items) 398 / 390 / 407 /
-// 415 / 494.  dK / dV sum over the heads: cutting theirs (CTAs of a cluster that add up through distributed shared memory) was 1.3 to
-// 2.4 times as fast below 222 items, but the sums then round in another order, which was not wanted.
+// 415 / 494 (before the rest of the kernel became faster; the order of the cuts is the same).
 int heads_per_cta(int G, int base) {
     int heads = G;
     for (int parts = 1; parts <= G; ++parts) {
@@ -826,6 +868,20 @@ int heads_per_cta(int G, int base) {
         if (2 * base * ((G + heads - 1) / heads) >= 3 * device_sms()) break;
     }
     return heads;
+}
+
+// CTAs of one cluster that share the query heads of a dK / dV item (key block, kv head, batch), head size 128.  An item alone walks all
+// heads of the group, so few items leave SMs idle and the longest walk sets the time: the cluster is as large as two CTAs per SM allow.
+// Its CTAs add their sums up through distributed shared memory, in the order of the heads.  Kernel times in us, one CTA per item (of the kernel
+// before its issue was split, 1.15 times as long) /
+// now:  1 x 333 tokens, 12 / 2 heads (6 items, 6 parts) 37 / 14;  1 x 2048, 12 / 2 (32, 6) 164 / 43;  2 x 2048, 12 / 2 (64, 4) 167 / 79;
+// 2 x 2048, 28 / 4 (128, 2) 200 / 112;  1 x 2048, 32 / 8 (128, 2) 119 / 65;  3 x 2048, 28 / 4 (192, 1) 206 / 178.
+// With head size 64 the sum over the heads stays in one accumulator: its results keep their bits.
+int head_parts(int G, int base) {
+    int parts = 2 * device_sms() / base;
+    if (parts > 8) parts = 8;
+    if (parts > G) parts = G;
+    return parts > 1 ? parts : 1;
 }
 
 template <int HS>
@@ -853,8 +909,14 @@ int bwd_impl(void* dqkv, float* delta, const void* d_out, const void* out, const
         constexpr int smem = DkdvShape<HS>::SMEM_BYTES;
         rc = set_smem<1000 + HS>(attn_bwd_dkdv_kernel<HS>, smem);
         if (rc) return rc;
-        attn_bwd_dkdv_kernel<HS><<<base, kBwdThreads, smem, s>>>(t128, t64, tdo64, p);
-        rc = LLMQ_LAUNCH_CHECK();
+        const int parts = HS == 128 ? head_parts(G, base) : 1;
+        cudaLaunchConfig_t cfg{};
+        cfg.gridDim = dim3(base * parts); cfg.blockDim = dim3(kBwdThreads); cfg.dynamicSmemBytes = smem; cfg.stream = s;
+        cudaLaunchAttribute attr{};
+        attr.id = cudaLaunchAttributeClusterDimension;
+        attr.val.clusterDim.x = parts; attr.val.clusterDim.y = 1; attr.val.clusterDim.z = 1;
+        cfg.attrs = &attr; cfg.numAttrs = parts > 1 ? 1 : 0;
+        rc = static_cast<int>(cudaLaunchKernelEx(&cfg, attn_bwd_dkdv_kernel<HS>, t128, t64, tdo64, p, parts));
         if (rc) return rc;
     }
     {

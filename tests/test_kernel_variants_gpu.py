@@ -50,6 +50,29 @@ def test_attention_head_splits(HS, B, T, Hq, Hkv):
     assert rel(dqkv[:, :, Hq + Hkv:], x.grad[:, :, Hq + Hkv:]) < 1.2e-2
 
 
+# dK / dV of head size 128: CTAs per item on both sides of the steps of the rule (one CTA, clusters of two to eight, odd shares of the heads)
+@pytest.mark.parametrize("T", [70, 200])
+@pytest.mark.parametrize("Hq,Hkv", [(6, 1), (10, 2), (9, 1)])
+def test_attention_backward_shared_heads(T, Hq, Hkv):
+    per = (T + 127) // 128 * Hkv                          # items per sequence
+    counts = [n // per for n in (296, 148, 98, 74, 59, 49, 37, 6)]
+    g = torch.Generator(device=DEV).manual_seed(T)
+    most = counts[0]
+    qkv = torch.randn(most, T, Hq + 2 * Hkv, 128, device=DEV, generator=g).to(BF)
+    dout = torch.randn(most, T, Hq, 128, device=DEV, generator=g).to(BF)
+    want = None
+    for B in counts:
+        out, lse, dqkv = torch.empty(B, T, Hq, 128, device=DEV, dtype=BF), torch.empty(B, Hq, T, device=DEV), torch.full_like(qkv[:B], 9.0)
+        K.attention_forward(out, lse, qkv[:B], Hq, Hkv)
+        K.attention_backward(dqkv, torch.empty(B * Hq * T, device=DEV), dout[:B], out, lse, qkv[:B], Hq, Hkv)
+        if want is None:
+            want = dqkv
+        assert torch.equal(dqkv[:, :, :Hq], want[:B, :, :Hq])            # dQ has one order
+        # the same products summed in another order in fp32, then one rounding to bf16: neighbours at most, where the sum does not cancel
+        d = (dqkv.float() - want[:B].float()).abs()
+        assert (d <= want[:B].float().abs() * 2**-7 + 1e-4 * want.float().abs().max()).all()
+
+
 # sequences of one query tile: a head per CTA and, with more heads than SMs, two heads of a group (the last one of an odd group alone)
 @pytest.mark.parametrize("HS", [64, 128])
 @pytest.mark.parametrize("T", [1, 33, 64, 65, 127, 128])
