@@ -61,6 +61,10 @@ struct GemmParams {
     // MN-major operands whose M / N extent is a multiple of the 128-byte chunk: the tensor map is 3-D (chunk column, K row, chunk)
     // and one load fetches all chunks of a stage
     int a_box3, b_box3;
+    // CTA-pair kernel: columns of a tile (a multiple of 32 up to 256) and the bytes of B that a CTA loads per stage
+    int bn, b_stage_bytes;
+    // 1: C is bf16 with rows of whole aligned 32-byte sectors and the epilogue moves them lane by lane (store_sector)
+    int c_sectors;
 };
 
 // Adds bias[col0 .. col0+31] to the 32 values of one accumulator chunk (every lane needs the same 32 bias values:
@@ -93,6 +97,60 @@ __device__ __forceinline__ void add_bias32(const GemmParams& p, int col0, float 
 // Shared memory one epilogue warp needs for the coalescing store path of epilogue_rows (32 rows x 128 bytes).
 constexpr int EPI_STAGE_BYTES_PER_WARP = 32 * 128;
 
+// 32 bytes (16 bf16) of one row per lane: a whole sector per lane and instruction
+__device__ __forceinline__ void load_sector(const void* p, uint32_t (&r)[8]) {
+    asm volatile("ld.global.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]) : "l"(p) : "memory");
+}
+__device__ __forceinline__ void store_sector(void* p, const uint32_t* r) {
+    asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};"
+                 ::"l"(p), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]) : "memory");
+}
+
+// bf16 C in whole sectors (GemmParams::c_sectors), with or without its previous values: lane = row, 32 columns at a time.  A lane that moves
+// 16 bytes at a time touches every sector twice; adding to C that way 16384 x 3584 x 3584 took 310 us in bf16 and 240 us in e4m3, in whole sectors
+// 287 and 163 (plain: 275 and 145).  Plain outputs of the CTA-pair kernel stay on the staged TMA stores: 4096 x 151936 x 896 824 us, 837 this way.
+__device__ __forceinline__ void epilogue_rows_sectors(const GemmParams& p, uint32_t t_row, int row, int col_base, int ncols, float alpha, float& tmax) {
+    using namespace sm100;
+    const bool row_ok = row < p.M;
+    __nv_bfloat16* crow = static_cast<__nv_bfloat16*>(p.C) + static_cast<long long>(row) * p.ldc;
+#pragma unroll 1
+    for (int c = 0; c < ncols; c += 32) {
+        const int col0 = col_base + c;
+        if (col0 >= p.N) break;                    // uniform across the warp
+        const int halves = col0 + 32 <= p.N ? 2 : 1;                // N is a multiple of 16
+        uint32_t r[32], old[2][8] = {};
+        tmem_ld_32x32b_x32(t_row + c, r);
+        if (p.accumulate && row_ok) {
+#pragma unroll
+            for (int h = 0; h < 2; ++h) if (h < halves) load_sector(crow + col0 + 16 * h, old[h]);
+        }
+        tmem_ld_wait();
+        float v[32];
+#pragma unroll
+        for (int j = 0; j < 32; ++j) v[j] = __uint_as_float(r[j]) * alpha;
+        if (p.bias) add_bias32(p, col0, v);
+        if (p.accumulate) {
+#pragma unroll
+            for (int j = 0; j < 32; ++j) v[j] += __uint_as_float((j & 1) ? old[j / 16][(j % 16) / 2] & 0xffff0000u : old[j / 16][(j % 16) / 2] << 16);
+        }
+        if (p.absmax_out && row_ok) {
+#pragma unroll
+            for (int j = 0; j < 32; ++j) if (j < 16 * halves) tmax = fmaxf(tmax, fabsf(v[j]));
+        }
+        uint32_t packed[16];
+#pragma unroll
+        for (int j = 0; j < 16; ++j) {
+            __nv_bfloat162 b = __floats2bfloat162_rn(v[2 * j], v[2 * j + 1]);
+            packed[j] = *reinterpret_cast<uint32_t*>(&b);
+        }
+        if (row_ok) {
+#pragma unroll
+            for (int h = 0; h < 2; ++h) if (h < halves) store_sector(crow + col0 + 16 * h, packed + 8 * h);
+        }
+    }
+}
+
 // Each lane of the calling warp owns one accumulator row (TMEM lane); `t_row` addresses column 0 of that row
 // block.  Applies alpha and bias, optionally adds the previous C, stores bf16 or fp32, tracks abs-max.
 // The TMEM loads are warp-collective, so all lanes run the loop; only the stores are predicated on the row.
@@ -109,6 +167,7 @@ __device__ __forceinline__ void epilogue_rows(const GemmParams& p, uint32_t t_ro
                                               float alpha, float& tmax, __nv_bfloat16* dst_row = nullptr, uint8_t* stage = nullptr,
                                               const CUtensorMap* tmap_c = nullptr, int* stage_sel = nullptr) {
     using namespace sm100;
+    if (p.c_sectors && dst_row == nullptr) { epilogue_rows_sectors(p, t_row, row, col_base, ncols, alpha, tmax); return; }
     const bool row_ok = row < p.M;
     // (`dst_row` redirection: the rows of one warp are consecutive rows of the same landing slot, N elements apart)
     const int lane_id = threadIdx.x & 31;
@@ -129,7 +188,8 @@ __device__ __forceinline__ void epilogue_rows(const GemmParams& p, uint32_t t_ro
         for (int c = 0; c < ncols; c += 64) {
             const int col0 = col_base + c;
             if (col0 >= p.N) break;                    // uniform across the warp
-            const bool second = col0 + 32 < p.N;       // uniform
+            const bool whole = c + 64 <= ncols;        // uniform; false for the last 32 columns of a tile whose width is not a multiple of 64
+            const bool second = whole && col0 + 32 < p.N;
             uint32_t r[2][32];
             tmem_ld_32x32b_x32(t_row + c, r[0]);
             if (second) tmem_ld_32x32b_x32(t_row + c + 32, r[1]);
@@ -163,7 +223,7 @@ __device__ __forceinline__ void epilogue_rows(const GemmParams& p, uint32_t t_ro
                 asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(a), "r"(packed[4 * i]), "r"(packed[4 * i + 1]),
                              "r"(packed[4 * i + 2]), "r"(packed[4 * i + 3]) : "memory");
             }
-            if (use_tma) {
+            if (use_tma && whole) {
                 fence_proxy_async_smem();
                 __syncwarp();
                 if (lane == 0) { tma_store_2d(tmap_c, stage_addr, col0, row_base); tma_store_commit(); }
@@ -179,7 +239,7 @@ __device__ __forceinline__ void epilogue_rows(const GemmParams& p, uint32_t t_ro
                 const uint32_t a = stage_addr + rr * 128 + ((ch ^ (rr & 7)) << 4);
                 asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(o.x), "=r"(o.y), "=r"(o.z), "=r"(o.w) : "r"(a) : "memory");
                 const int grow = row_base + rr;
-                if (grow < p.M && gcol < p.N) *reinterpret_cast<uint4*>(out_base + rr * out_ld + gcol) = o;
+                if (grow < p.M && gcol < p.N && (whole || ch < 4)) *reinterpret_cast<uint4*>(out_base + rr * out_ld + gcol) = o;
             }
             __syncwarp();
         }

@@ -356,10 +356,35 @@ static int g_gemm_mode = 0;
 static int g_gemm_tma_store = 1;
 extern "C" void llmq_gemm_set_tma_store(int on) { g_gemm_tma_store = on; }
 extern "C" void llmq_gemm_set_mode(int mode) { g_gemm_mode = mode; }
+// Columns of a tile of the CTA-pair kernel: 0 = automatic, 224 or 256 = forced where the operands allow it (tests, measurements).
+static int g_gemm_pair_bn = 0;
+extern "C" void llmq_gemm_set_pair_bn(int bn) { g_gemm_pair_bn = bn; }
+
+static long long waves(long long tiles, int at_once) { return (tiles + at_once - 1) / at_once; }
+static long long tiles_of(int M, int N, int bm, int bn) { return static_cast<long long>((M + bm - 1) / bm) * ((N + bn - 1) / bn); }
 
 // The CTA-pair kernel runs GEMMs of at least 32 tiles of 256 x 256, and those that carry a collective or a fused epilogue (`fused`).
-static bool uses_pair_kernel(int M, int N, int elem_bytes, bool fused) {
-    return elem_bytes != 4 && (fused || g_gemm_mode == 2 || (g_gemm_mode == 0 && M >= 256 && static_cast<long long>(M) * N >= 256LL * 256 * 32));
+// Per round of tiles on all SMs it is 1.1 to 1.2 times as fast as the one-CTA kernel, whose 128 x 256 tiles it loses to where its own leave
+// most of the last round idle: 896 x 4864 x 4096, both operands MN-major, is 76 pair tiles (two rounds of 74, 48.5 us) or 133 of the others
+// (one round of 148, 36.4 us); with equally many rounds 16384 x 4608 x 3584 351 / 388 us, 4096 x 896 x 9728 60.8 / 66.4, 4096 x 4864 x 896
+// 33.7 / 40.6.  With that many tiles the one-CTA kernel does not cut the K loop, so the sums have the same bits.
+static bool uses_pair_kernel(int M, int N, int elem_bytes, bool fused, int num_sms) {
+    if (elem_bytes == 4) return false;
+    if (fused || g_gemm_mode == 2) return true;
+    if (g_gemm_mode != 0 || M < 256 || static_cast<long long>(M) * N < 256LL * 256 * 32) return false;
+    const long long pair = waves(tiles_of(M, N, 256, 256), num_sms / 2);
+    return pair < 2 || 5 * waves(tiles_of(M, N, 128, 256), num_sms) >= 4 * pair;
+}
+
+// Columns of a pair tile: 224 instead of 256 where that saves time, K-major B.  A round of 224-column tiles takes 0.93-0.95 of the time (the
+// loads of A are the same), so it has to need no more rounds; and not many more columns beyond N, which cost loads.  256 / 224 columns, us:
+// 4096 x 896 x 151936 863 / 797 (896 is 4 x 224), 151936 x 896 x 4096 850 / 792, 4096 x 896 x 4864 33.5 / 31.1, 2048 x 3072 x 3072 39.8 / 37.3 (two
+// rounds either way);  left at 256: 16384 x 3584 x 3584 275 / 278 (13 / 14 rounds), 4096 x 1152 x 896 15.5 / 16.1 (1280 / 1344 columns).
+// 192, 160 and 128 columns are slower still per column: a K step takes 0.85, 0.83, 0.79 of the time of one of 256.
+static int pair_tile_columns(int M, int N, int num_sms) {
+    const long long w256 = waves(tiles_of(M, N, 256, 256), num_sms / 2), w224 = waves(tiles_of(M, N, 256, 224), num_sms / 2);
+    const long long c256 = (N + 255) / 256 * 256LL, c224 = (N + 223) / 224 * 224LL;
+    return 100 * w224 <= 103 * w256 && 100 * c224 <= 103 * c256 ? 224 : 256;
 }
 
 // Parts that the one-CTA kernel cuts the K loop into: more than one for outputs with at most half as many 256-column tiles as SMs and a
@@ -380,7 +405,7 @@ static int splitk_parts(int M, int N, int K, int elem_bytes, int num_sms) {
 
 // Floats of the workspace with which a plain GEMM of this shape (A and B of `elem_bytes` an element) cuts its K loop; 0: it does not.
 extern "C" long long llmq_gemm_splitk_floats(int M, int N, int K, int elem_bytes, int num_sms) {
-    if (M <= 0 || N <= 0 || K <= 0 || elem_bytes <= 0 || uses_pair_kernel(M, N, elem_bytes, false)) return 0;
+    if (M <= 0 || N <= 0 || K <= 0 || elem_bytes <= 0 || uses_pair_kernel(M, N, elem_bytes, false, num_sms)) return 0;
     const int parts = splitk_parts(M, N, K, elem_bytes, num_sms);
     return parts > 1 ? static_cast<long long>(parts) * M * N : 0;
 }
@@ -477,7 +502,7 @@ static int gemm_impl(const void* A, const void* B, void* C, const void* bias,
     const int bk = 128 / eb;
     int rc;
     // The CTA-pair kernel stages 128 rows of B per CTA; the one-CTA kernel stages all 256.
-    const bool pair_kernel = uses_pair_kernel(M, N, eb, rs != nullptr || ready_flags != nullptr);
+    const bool pair_kernel = uses_pair_kernel(M, N, eb, rs != nullptr || ready_flags != nullptr, num_sms);
     // An MN-major stage that is several 128-byte chunks wide (16-bit operands; the 256 rows of B of the one-CTA kernel) is fetched with
     // one 3-D load instead of one 2-D load per chunk: the loads of a stage were issued one after the other for longer than its MMAs
     // run.  bf16, CTA pairs, TFLOP/s with 2-D loads / 3-D loads / 3-D loads and a K loop per kind of load (gemm_tcgen05_2cta.cu), K-major
@@ -497,7 +522,9 @@ static int gemm_impl(const void* A, const void* B, void* C, const void* bias,
     if (static_cast<long long>(splits) * M * N > splitk_floats) splits = 1;
     const int tiles128 = ((M + BM - 1) / BM) * ((N + 127) / 128);
     const int bn = (eb != 4 && tiles128 * splits <= num_sms) ? 128 : 256;
-    const int b_rows = pair_kernel ? 128 : bn;
+    int pair_bn = 256;
+    if (pair_kernel && rs == nullptr && ready_flags == nullptr && !b_mn_major) pair_bn = g_gemm_pair_bn ? g_gemm_pair_bn : pair_tile_columns(M, N, num_sms);
+    const int b_rows = pair_kernel ? pair_bn / 2 : bn;
     const bool a_box3 = a_mn_major && eb < 4 && BM > bk && M % bk == 0, b_box3 = b_mn_major && eb < 4 && b_rows > bk && N % bk == 0;
     if (!a_mn_major) rc = llmq_encode_tmap_2d(&ta, A, eb, M, K, lda, BM);
     else if (a_box3) rc = encode_tmap_chunks(&ta, A, eb, K, M, lda, bk, BM / bk);
@@ -515,6 +542,8 @@ static int gemm_impl(const void* A, const void* B, void* C, const void* bias,
     p.b_fmt = b_dtype == 3 ? 2 : (b_dtype == 0 ? 1 : (b_dtype == 1 ? 0 : 1));
     p.C = C; p.ldc = ldc; p.c_dtype = c_dtype; p.accumulate = accumulate;
     p.bias = bias; p.bias_dtype = bias_dtype;
+    p.bn = pair_bn; p.b_stage_bytes = b_rows * 128;
+    p.c_sectors = rs == nullptr && (accumulate || !pair_kernel) && c_dtype == 0 && N % 16 == 0 && ldc % 16 == 0 && (reinterpret_cast<uintptr_t>(C) & 31u) == 0;
     p.scale_a = scale_a; p.scale_b = scale_b; p.alpha = alpha;
     p.absmax_out = absmax_out; p.status = status;
     p.ready_flags = ready_flags; p.ready_gen = ready_gen; p.ready_rows_per_src = ready_rows_per_src > 0 ? ready_rows_per_src : 1;

@@ -1,4 +1,5 @@
-// Two-CTA variant of the tcgen05 GEMM: a cluster of two CTAs on neighbouring SMs computes one 256x256 tile.
+// Two-CTA variant of the tcgen05 GEMM: a cluster of two CTAs on neighbouring SMs computes one 256x256 tile (or a narrower one,
+// GemmParams::bn).
 //
 // Each CTA stages its own 128 rows of A and only half of the 256 rows of B per K step; tcgen05.mma with
 // cta_group::2 reads both halves of B from the two shared memories, so per multiply-accumulate the pair moves
@@ -30,8 +31,8 @@ using namespace sm100;
 namespace {
 
 constexpr int BM = 128;              // rows per CTA (256 per pair)
-constexpr int BN = 256;
-constexpr int BN_HALF = 128;         // rows of B staged by each CTA
+constexpr int BN_MAX = 256;          // columns per tile at most; each CTA stages half of a tile's as rows of B
+constexpr int BN_HALF = 128;
 constexpr int ROW_BYTES = 128;
 constexpr int STAGES = 6;
 constexpr int A_STAGE_BYTES = BM * ROW_BYTES;        // 16 KiB
@@ -81,7 +82,8 @@ gemm_tcgen05_2cta_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gri
     const int k_iters = (p.K + bk - 1) / bk;
     const int tiles_m = (p.M + 2 * BM - 1) / (2 * BM);
     // SwiGLU forward mode: a column tile is 128 features, staged as 128 "up" rows + 128 "gate" rows of B
-    const int tiles_n = p.ep_mode == 1 ? (p.ep_D + BN_HALF - 1) / BN_HALF : (p.N + BN - 1) / BN;
+    const int bn = p.bn, bn_half = bn >> 1;
+    const int tiles_n = p.ep_mode == 1 ? (p.ep_D + BN_HALF - 1) / BN_HALF : (p.N + bn - 1) / bn;
     const int num_tiles = tiles_m * tiles_n;
     const int pair = blockIdx.x >> 1, num_pairs = gridDim.x >> 1;
     // fused reduce-scatter: start with the rows owned by the next rank, finish with our own
@@ -127,7 +129,7 @@ gemm_tcgen05_2cta_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gri
                 int tm, tn; tile_coords(t, tiles_m, tiles_n, rot, tm, tn);
                 const int row0 = (tm * 2 + static_cast<int>(rank)) * BM;               // this CTA's rows of A / C
                 const int brow0 = p.ep_mode == 1 ? tn * BN_HALF + static_cast<int>(rank) * p.ep_D
-                                                 : tn * BN + static_cast<int>(rank) * BN_HALF;   // this CTA's rows of B
+                                                 : tn * bn + static_cast<int>(rank) * bn_half;   // this CTA's rows of B
                 if (p.ready_flags && !p.b_mn_major && brow0 < p.N) {
                     const int last = min(brow0 + BN_HALF, p.N) - 1;
                     for (int src = brow0 / p.ready_rows_per_src; src <= last / p.ready_rows_per_src && ok; ++src) ensure_src(src);
@@ -145,7 +147,7 @@ gemm_tcgen05_2cta_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gri
                         const uint32_t sa = smem_base + stage * STAGE_BYTES;
                         const uint32_t sb = sa + A_STAGE_BYTES;
                         const uint32_t fb = fb0 + 8u * stage;                                // the leader's barrier
-                        if (rank == 0) mbar_expect_tx(full_bar(stage), 2 * STAGE_BYTES);     // bytes of both CTAs
+                        if (rank == 0) mbar_expect_tx(full_bar(stage), 2 * (A_STAGE_BYTES + p.b_stage_bytes));     // bytes of both CTAs
                         if constexpr (a_load == 0)      tma_load_2d_pair(sa, &tmap_a, fb, k * bk, row0);
                         else if constexpr (a_load == 1) tma_load_3d_pair(sa, &tmap_a, fb, 0, k * bk, row0 / mn_chunk);
                         else {
@@ -156,9 +158,9 @@ gemm_tcgen05_2cta_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gri
                         if constexpr (b_load == 0)      tma_load_2d_pair(sb, &tmap_b, fb, k * bk, brow0);
                         else if constexpr (b_load == 1) tma_load_3d_pair(sb, &tmap_b, fb, 0, k * bk, brow0 / mn_chunk);
                         else {
-                            const int nbox = BN_HALF * p.elem_bytes / ROW_BYTES;
+                            const int box_bytes = bk * ROW_BYTES, nbox = p.b_stage_bytes / box_bytes;
                             for (int b = 0; b < nbox; ++b)
-                                tma_load_2d_pair(sb + b * (B_STAGE_BYTES / nbox), &tmap_b, fb, brow0 + b * mn_chunk, k * bk);
+                                tma_load_2d_pair(sb + b * box_bytes, &tmap_b, fb, brow0 + b * mn_chunk, k * bk);
                         }
                         if (++stage == STAGES) { stage = 0; phase ^= 1u; }
                     }
@@ -179,7 +181,7 @@ gemm_tcgen05_2cta_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gri
     } else if (warp == 1) {
         // ------------------------------------------------------------------ MMA issuer (leader only)
         if (lane == 0 && rank == 0) {
-            const uint32_t idesc = make_instr_desc(p.a_fmt, p.b_fmt, p.a_mn_major, p.b_mn_major, 2 * BM, BN);
+            const uint32_t idesc = make_instr_desc(p.a_fmt, p.b_fmt, p.a_mn_major, p.b_mn_major, 2 * BM, bn);
             const int mma_k = 32 / p.elem_bytes;
             const uint32_t box_bytes = static_cast<uint32_t>(bk) * ROW_BYTES;
             const uint32_t a_step = p.a_mn_major ? mma_k * ROW_BYTES : 32;
@@ -195,7 +197,7 @@ gemm_tcgen05_2cta_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gri
             for (int t = pair; t < num_tiles && ok; t += num_pairs) {
                 if (!mbar_wait(tempty_bar(acc), acc_phase ^ 1u, abort_flag)) { atomicOr(p.status, kErrTmemEmpty); ok = false; break; }
                 tc_fence_after_sync();
-                const uint32_t d_tmem = tmem_base + acc * BN;
+                const uint32_t d_tmem = tmem_base + acc * BN_MAX;
                 for (int k = 0; k < k_iters; ++k) {
                     if (!mbar_wait(full_bar(stage), phase, abort_flag)) { atomicOr(p.status, kErrFullWait); ok = false; break; }
                     tc_fence_after_sync();
@@ -240,10 +242,10 @@ gemm_tcgen05_2cta_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gri
                 const long long slot_row = static_cast<long long>(p.rs_rank) * p.rs_shard_rows + (row - owner * p.rs_shard_rows);
                 dst_row = static_cast<__nv_bfloat16*>(p.rs_landing[owner]) + slot_row * p.N;
             }
-            const uint32_t t_row = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + acc * BN;
+            const uint32_t t_row = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + acc * BN_MAX;
             if (p.ep_mode == 1)      epilogue_rows_swiglu_fwd(p, t_row, row, tn * BN_HALF, alpha, tmax);
-            else if (p.ep_mode == 2) epilogue_rows_swiglu_bwd(p, t_row, row, tn * BN, BN, alpha, tmax);
-            else                     epilogue_rows(p, t_row, row, tn * BN, BN, alpha, tmax, dst_row, stage, &tmap_c, &stage_sel);
+            else if (p.ep_mode == 2) epilogue_rows_swiglu_bwd(p, t_row, row, tn * bn, bn, alpha, tmax);
+            else                     epilogue_rows(p, t_row, row, tn * bn, bn, alpha, tmax, dst_row, stage, &tmap_c, &stage_sel);
             tc_fence_before_sync();
             mbar_arrive_cluster(map_to_cta(tempty_bar(acc), 0));            // 2 x 128 arrivals at the leader
             if (++acc == 2) { acc = 0; acc_phase ^= 1u; }
@@ -340,7 +342,7 @@ int llmq_gemm_2cta_launch(const CUtensorMap& ta, const CUtensorMap& tb, const CU
         if (e != cudaSuccess) return static_cast<int>(e);
         attr_set[dev & 63] = true;
     }
-    const int tiles = ((p.M + 2 * BM - 1) / (2 * BM)) * (p.ep_mode == 1 ? (p.ep_D + BN_HALF - 1) / BN_HALF : (p.N + BN - 1) / BN);
+    const int tiles = ((p.M + 2 * BM - 1) / (2 * BM)) * (p.ep_mode == 1 ? (p.ep_D + BN_HALF - 1) / BN_HALF : (p.N + p.bn - 1) / p.bn);
     int pairs = num_sms / 2;
     if (tiles < pairs) pairs = tiles;
     if (p.elem_bytes == 1) gemm_tcgen05_2cta_kernel<true><<<2 * pairs, NUM_THREADS, SMEM_BYTES, stream>>>(ta, tb, tc, p);

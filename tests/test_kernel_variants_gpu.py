@@ -6,6 +6,7 @@ import pytest
 import torch
 
 from llmq_b200.ops import kernels as K
+from llmq_b200.ops import lib as L
 
 pytestmark = pytest.mark.gpu
 DEV = "cuda"
@@ -496,3 +497,69 @@ def test_adamw_and_norm_of_all_tensors_in_one_launch(types, sizes, scalars):
         for k in ("param", "m", "v", "m_scales", "absmax"):
             if x[k] is not None:
                 assert torch.equal(x[k].view(torch.uint8), y[k].view(torch.uint8)), k
+
+
+# CTA-pair tiles of 224 columns (K-major B) against 256: whole and ragged last tiles, a last half block of 32 columns; the same bits
+@pytest.mark.parametrize("f8", [False, True])
+@pytest.mark.parametrize("M,N,depth", [(4096, 896, 64), (2300, 1120, 200), (4096, 680, 136), (8448, 264, 128), (256, 8256, 96)])
+@pytest.mark.parametrize("accumulate,bias", [(False, True), (True, False)])
+def test_gemm_pair_tile_columns(f8, M, N, depth, accumulate, bias):
+    dt = torch.float8_e4m3fn if f8 else BF
+    if f8:
+        depth = (depth + 15) // 16 * 16
+    g = torch.Generator(device=DEV).manual_seed(M + N)
+    a, b = (torch.randn(r, depth, device=DEV, generator=g).to(dt) for r in (M, N))
+    old = torch.randn(M, N, device=DEV, generator=g).to(BF)
+    bi = torch.randn(N, device=DEV, generator=g).to(BF) if bias else None
+    lib, got = L.kernels(), []
+    try:
+        for bn in (256, 224):
+            lib.llmq_gemm_set_pair_bn(bn)
+            wide = torch.full((M, N + 32), 9.0, device=DEV, dtype=BF)
+            c, am = wide[:, :N], torch.zeros(1, device=DEV)
+            c.copy_(old)
+            K.gemm(c, a, b, bias=bi, accumulate=accumulate, absmax=am)
+            assert (wide[:, N:] == 9).all()               # nothing beyond the row
+            got.append((c.clone(), am.item()))
+    finally:
+        lib.llmq_gemm_set_pair_bn(0)
+    assert torch.equal(got[0][0], got[1][0]) and got[0][1] == got[1][1]
+    ref = a.float() @ b.float().t() + (old.float() if accumulate else 0) + (bi.float() if bias else 0)
+    assert rel(got[1][0], ref) < 4e-3                     # bf16 rounding: 2^-9 of a value at most
+
+
+# outputs in whole 32-byte sectors or not: ragged widths, row pitches and addresses on both sides of the rule, in both kernels
+@pytest.mark.parametrize("M,N", [(130, 48), (300, 272), (300, 264), (4096, 560), (2304, 1160)])
+@pytest.mark.parametrize("accumulate", [False, True])
+@pytest.mark.parametrize("pitch,offset", [(0, 0), (16, 0), (8, 0), (16, 8)])
+def test_gemm_output_sectors(M, N, accumulate, pitch, offset):
+    g = torch.Generator(device=DEV).manual_seed(M + N)
+    a, b = (torch.randn(r, 136, device=DEV, generator=g).to(BF) for r in (M, N))
+    old = torch.randn(M, N, device=DEV, generator=g).to(BF)
+    ld = N + pitch
+    flat = torch.full((M * ld + 16,), 9.0, device=DEV, dtype=BF)
+    c = flat[offset:offset + M * ld].view(M, ld)[:, :N]
+    c.copy_(old)
+    K.gemm(c, a, b, accumulate=accumulate)
+    assert rel(c, a.float() @ b.float().t() + (old.float() if accumulate else 0)) < 4e-3
+    rest = torch.ones_like(flat, dtype=torch.bool)
+    rest[offset:offset + M * ld].view(M, ld)[:, :N] = False
+    assert (flat[rest] == 9).all()
+
+
+# as many rounds of pair tiles as of 128-row tiles, and more: the kernel that the rule picks gives the bits of the other one
+@pytest.mark.parametrize("M,N,depth", [(896, 4864, 128), (896, 4608, 128), (1152, 3840, 192)])
+def test_gemm_rounds_of_tiles(M, N, depth):
+    g = torch.Generator(device=DEV).manual_seed(M)
+    a, b = (torch.randn(depth, r, device=DEV, generator=g).to(BF) for r in (M, N))
+    lib, got = L.kernels(), []
+    try:
+        for mode in (0, 1, 2):
+            lib.llmq_gemm_set_mode(mode)
+            c = torch.empty(M, N, device=DEV, dtype=BF)
+            K.gemm(c, a, b, a_mn=True, b_mn=True)
+            got.append(c)
+    finally:
+        lib.llmq_gemm_set_mode(0)
+    assert torch.equal(got[0], got[1]) and torch.equal(got[0], got[2])
+    assert rel(got[0], a.float().t() @ b.float()) < 4e-3
