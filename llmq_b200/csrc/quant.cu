@@ -249,9 +249,11 @@ extern "C" int llmq_abs_max(float* out, const void* x, long long n, int dtype, i
 extern "C" int llmq_quantize(void* out, float* scale_out, const void* x, const float* absmax, long long n, int in_dtype,
                              int out_dtype, int num_sms, cudaStream_t s) {
     if (n <= 0) return 0;
+    // four blocks of 512 threads per SM, as many as reside: us with twice as many / with these, bf16 to e4m3: 4096 x 3584 7.6 / 6.9, 16384 x 3584 28.2 /
+    // 27.8, 16384 x 18944 155 / 151, 1000 x 3584 4.2 / 3.8
 #define Q_CASE(T, TC, Q, QC, VN)                                                                                   \
     if (in_dtype == TC && out_dtype == QC) {                                                                       \
-        quantize_kernel<T, Q><<<grid_for(n / VN + 1, 512, num_sms), 512, 0, s>>>(static_cast<Q*>(out), scale_out,  \
+        quantize_kernel<T, Q><<<grid_for(n / VN + 1, 512, (num_sms + 1) / 2), 512, 0, s>>>(static_cast<Q*>(out), scale_out,  \
                                                                                  static_cast<const T*>(x), absmax, n); \
         return LLMQ_LAUNCH_CHECK();                                                                                \
     }
