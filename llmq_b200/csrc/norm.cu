@@ -252,19 +252,52 @@ rmsnorm_bwd_kernel(T* __restrict__ dinp,               // in: upstream residual 
     block_absmax_commit(absmax_out, tmax, scratch);
 }
 
+// 16 bytes from global to shared memory, asynchronously; a thread waits for its own copies in groups, in order
+__device__ __forceinline__ void copy_async16(void* dst, const void* src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(static_cast<uint32_t>(__cvta_generic_to_shared(dst))), "l"(src) : "memory");
+}
+__device__ __forceinline__ void copy_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void copy_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
+
 // Same contract, for rows of up to 4 column vectors per thread: the row's dout, inp and residual gradient are
 // loaded once and stay in registers across the block-wide dot product (no second pass over L1 / L2), the norm
 // weights are loaded once per CTA, and three CTAs share an SM so that their reductions overlap.  One barrier per row: 16384 x 3584,
 // 470 MB, 94 us; 102 us with the two of a general block reduction; 152 us with the next row loaded ahead (two CTAs per SM, spills).
-template <typename T, int VPT>
+// STAGES > 0: that many rows to come are on their way into shared memory; every thread copies and reads back its own vectors, so the
+// ring needs no barrier.  Rows of one vector a thread are too short to hide the load latency behind one another (16384 x 896 39.4 -> 30.2 us,
+// 4096 x 896 11.4 -> 9.2), with four the residual gradient no longer waits in registers (16384 x 5120 209 -> 184, 2000 x 5120 33 -> 27); with two the
+// registers hold everything, and the detour costs (16384 x 3584 94 -> 103).  fp32 rows have none: half the elements a vector make the registers
+// last (16384 x 3584 160 us either way, 16384 x 896 41 -> 48).
+template <typename T, int VPT, int STAGES>
 __global__ void __launch_bounds__(NORM_THREADS, VPT <= 2 ? 3 : 2)
 rmsnorm_bwd_reg_kernel(T* __restrict__ dinp, float* __restrict__ dw_partial, const T* __restrict__ dout, const T* __restrict__ inp,
                        const T* __restrict__ weight, const float* __restrict__ rstd, int rows, int C, float* __restrict__ absmax_out) {
     __shared__ float scratch[32];
     __shared__ float dots[2][NORM_THREADS / 32];             // alternating, so that one barrier per row is enough
+    extern __shared__ uint4 ring[];                          // [STAGES][3][VPT][NORM_THREADS]
     using V = Vec16<T>;
     float dw[VPT][V::N];
     V vw[VPT];
+    auto slot = [&](int stage, int what, int k) { return ring + ((stage * 3 + what) * VPT + k) * NORM_THREADS + threadIdx.x; };
+    auto fetch = [&](long long row, int stage) {
+        if (row < rows) {
+#pragma unroll
+            for (int k = 0; k < VPT; ++k) {
+                const int c = (k * NORM_THREADS + threadIdx.x) * V::N;
+                if (c < C) {
+                    copy_async16(slot(stage, 0, k), dout + row * C + c);
+                    copy_async16(slot(stage, 1, k), inp + row * C + c);
+                    copy_async16(slot(stage, 2, k), dinp + row * C + c);
+                }
+            }
+        }
+        copy_async_commit();                                 // a group per row, empty beyond the last one
+    };
+    if constexpr (STAGES > 0) {
+#pragma unroll
+        for (int st = 0; st < STAGES; ++st) fetch(blockIdx.x + static_cast<long long>(st) * gridDim.x, st);
+    }
 #pragma unroll
     for (int k = 0; k < VPT; ++k) {
         const int c = (k * NORM_THREADS + threadIdx.x) * V::N;
@@ -274,16 +307,21 @@ rmsnorm_bwd_reg_kernel(T* __restrict__ dinp, float* __restrict__ dw_partial, con
     }
     float tmax = 0.f;
     const float inv_c = 1.f / C;
-    int par = 0;
+    int par = 0, stage = 0;
     for (long long row = blockIdx.x; row < rows; row += gridDim.x, par ^= 1) {
         const T* dy = dout + row * C;
         const T* x = inp + row * C;
         T* dx = dinp + row * C;
-        V vdy[VPT], vx[VPT], vd[VPT];
+        V vdy[VPT], vx[VPT], vd[STAGES > 0 ? 1 : VPT];
+        if constexpr (STAGES > 0) copy_async_wait<STAGES - 1>();
 #pragma unroll
         for (int k = 0; k < VPT; ++k) {
             const int c = (k * NORM_THREADS + threadIdx.x) * V::N;
-            if (c < C) { vdy[k] = V::load_stream(dy + c); vx[k] = V::load_stream(x + c); vd[k] = V::load_stream(dx + c); }
+            if constexpr (STAGES > 0) {
+                if (c < C) { vdy[k] = V::load(reinterpret_cast<const T*>(slot(stage, 0, k))); vx[k] = V::load(reinterpret_cast<const T*>(slot(stage, 1, k))); }
+            } else {
+                if (c < C) { vdy[k] = V::load_stream(dy + c); vx[k] = V::load_stream(x + c); vd[k] = V::load_stream(dx + c); }
+            }
         }
         const float rs = rstd[row];
         float dot = 0.f;
@@ -308,15 +346,21 @@ rmsnorm_bwd_reg_kernel(T* __restrict__ dinp, float* __restrict__ dw_partial, con
         for (int k = 0; k < VPT; ++k) {
             const int c = (k * NORM_THREADS + threadIdx.x) * V::N;
             if (c < C) {
+                V& d = vd[STAGES > 0 ? 0 : k];
+                if constexpr (STAGES > 0) d = V::load(reinterpret_cast<const T*>(slot(stage, 2, k)));
 #pragma unroll
                 for (int i = 0; i < V::N; ++i) {
                     const float xh = to_float(vx[k].v[i]) * rs;
                     const float g = (to_float(vw[k].v[i]) * to_float(vdy[k].v[i]) - xh * dot) * rs;
-                    vd[k].v[i] = from_float<T>(to_float(vd[k].v[i]) + g);
-                    tmax = fmaxf(tmax, fabsf(to_float(vd[k].v[i])));
+                    d.v[i] = from_float<T>(to_float(d.v[i]) + g);
+                    tmax = fmaxf(tmax, fabsf(to_float(d.v[i])));
                 }
-                vd[k].store(dx + c);
+                d.store(dx + c);
             }
+        }
+        if constexpr (STAGES > 0) {
+            fetch(row + static_cast<long long>(STAGES) * gridDim.x, stage);
+            if (++stage == STAGES) stage = 0;
         }
     }
 #pragma unroll
@@ -399,14 +443,29 @@ int launch_bwd(void* dinp, void* dweight, float* scratch, const void* dout, cons
     if (C % V::N) return -1;
     const int vecs = ceil_div_i(C / V::N, NORM_THREADS);
     if (num_blocks > rows) num_blocks = rows;
-#define LAUNCH(KERNEL)                                                                                                       \
-    KERNEL<<<num_blocks, NORM_THREADS, 0, s>>>(static_cast<T*>(dinp), scratch, static_cast<const T*>(dout), static_cast<const T*>(inp), \
+#define LAUNCH(KERNEL, SMEM)                                                                                                 \
+    KERNEL<<<num_blocks, NORM_THREADS, SMEM, s>>>(static_cast<T*>(dinp), scratch, static_cast<const T*>(dout), static_cast<const T*>(inp), \
                                                static_cast<const T*>(w), rstd, rows, C, absmax)
-    if (vecs <= 1) LAUNCH((rmsnorm_bwd_reg_kernel<T, 1>));
-    else if (vecs <= 2) LAUNCH((rmsnorm_bwd_reg_kernel<T, 2>));
-    else if (vecs <= 4) LAUNCH((rmsnorm_bwd_reg_kernel<T, 4>));
-    else if (vecs <= 8) LAUNCH((rmsnorm_bwd_kernel<T, 8>));
+#define LAUNCH_RING(VPT, STAGES)                                                                                             \
+    {                                                                                                                        \
+        constexpr int smem = (STAGES) * 3 * (VPT) * NORM_THREADS * 16;                                                       \
+        static bool attr_set[64] = {};          /* per device */                                                             \
+        int dev = 0;                                                                                                         \
+        cudaGetDevice(&dev);                                                                                                 \
+        if (!attr_set[dev & 63]) {                                                                                           \
+            cudaError_t e = cudaFuncSetAttribute(rmsnorm_bwd_reg_kernel<T, VPT, STAGES>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem); \
+            if (e != cudaSuccess) return static_cast<int>(e);                                                                \
+            attr_set[dev & 63] = true;                                                                                       \
+        }                                                                                                                    \
+        LAUNCH((rmsnorm_bwd_reg_kernel<T, VPT, STAGES>), smem);                                                              \
+    }
+    constexpr bool h = sizeof(T) == 2;
+    if (vecs <= 1) LAUNCH_RING(1, (h ? 4 : 0))
+    else if (vecs <= 2) LAUNCH((rmsnorm_bwd_reg_kernel<T, 2, 0>), 0);
+    else if (vecs <= 4) LAUNCH_RING(4, (h ? 2 : 0))
+    else if (vecs <= 8) LAUNCH((rmsnorm_bwd_kernel<T, 8>), 0);
     else return -2;
+#undef LAUNCH_RING
 #undef LAUNCH
     int rc = LLMQ_LAUNCH_CHECK();
     if (rc) return rc;
