@@ -916,8 +916,11 @@ class LlamaModel:
         shard_of = {}
         norm_fused = getattr(g, "norm_fused", False)       # the reduce-scatter kernels already summed the squares
         items = list(w.master_items())
+        block_shards = {}                                  # all of a block's at once: a view of every tensor each time it is asked for
         for name, master, spec, l in items:
-            shard_of[name] = g.get_block_shard(l)[spec.name] if l is not None else g.get_nb_shard(spec.name)
+            if l is not None and l not in block_shards:
+                block_shards[l] = g.get_block_shard(l)
+            shard_of[name] = block_shards[l][spec.name] if l is not None else g.get_nb_shard(spec.name)
         # Nothing offloaded: every launch of the norm and AdamW loops has the same arguments each step (the step's scalars
         # travel through device memory), so with --use-cuda-graphs the ~400 small launches become two graph replays.
         on_device = self.device.type == "cuda" and all(
@@ -1048,6 +1051,9 @@ class LlamaModel:
     def get_gradients(self) -> Dict[str, torch.Tensor]:
         """Local gradient shards by checkpoint name (for tests and the Python API)."""
         out = {}
+        blocks = {}
         for name, master, spec, l in self.weights.master_items():
-            out[name] = self.grads.get_block_shard(l)[spec.name] if l is not None else self.grads.get_nb_shard(spec.name)
+            if l is not None and l not in blocks:
+                blocks[l] = self.grads.get_block_shard(l)
+            out[name] = blocks[l][spec.name] if l is not None else self.grads.get_nb_shard(spec.name)
         return out

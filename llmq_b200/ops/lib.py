@@ -79,14 +79,13 @@ def ptr(t):
     return ctypes.c_void_p(t.data_ptr())
 
 
-def stream_ptr(stream=None):
-    s = stream if stream is not None else torch.cuda.current_stream()
-    return ctypes.c_void_p(s.cuda_stream)
-
-
 def raw_stream() -> int:
-    """Handle of the current stream of the current device (3 us less than the Stream object of :func:`stream_ptr`)."""
+    """Handle of the current stream of the current device (3 us less host time than a Stream object)."""
     return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
+
+
+def stream_ptr(stream=None):
+    return ctypes.c_void_p(stream.cuda_stream if stream is not None else raw_stream())
 
 
 class KernelError(RuntimeError):
