@@ -376,6 +376,19 @@ static bool uses_pair_kernel(int M, int N, int elem_bytes, bool fused, int num_s
     return pair < 2 || 5 * waves(tiles_of(M, N, 128, 256), num_sms) >= 4 * pair;
 }
 
+// Tile rows of 256 that the pair kernel works through together.  B is read from memory once per group, so a group is as large as its rows of A
+// stay in the L2 beside the B tiles that stream past: up to 40 MB, 4 to 32 tile rows.  Sustained, us with 4 / 8 / 16 / 32 tile rows (in brackets
+// the MB of A in 8):  16384 x 37888 x 3584 e4m3 (7) 1840 / 1790 / 1718 / 1687, 16384 x 18944 x 3584 e4m3 (7) 940 / 896 / 868 / 854,
+// 4096 x 152064 x 3584 bf16 (15) 3444 / 3299 / 3229 / 3207, 4096 x 151936 x 896 bf16 (4) 984 / 946 / 918 / 918, 16384 x 3584 x 18944 e4m3 (39)
+// 919 / 912 / 914 / 985, 17920 x 1536 x 16384 bf16 (67) 689 / 719 / 727 / 767, 16384 x 1536 x 17920 bf16 (73) 744 / 748 / 756 / 799.
+// The order of the tiles is all that changes; kernels whose tiles arrive from or leave for other GPUs keep groups of 8.
+static int pair_group_rows(int K, int elem_bytes, bool fused) {
+    if (fused) return 8;
+    int rows = 32;
+    while (rows > 4 && static_cast<long long>(rows) * 256 * K * elem_bytes > (40ll << 20)) rows /= 2;
+    return rows;
+}
+
 // Columns of a pair tile: 224 instead of 256 where that saves time, K-major B.  A round of 224-column tiles takes 0.93-0.95 of the time (the
 // loads of A are the same), so it has to need no more rounds; and not many more columns beyond N, which cost loads.  256 / 224 columns, us:
 // 4096 x 896 x 151936 863 / 797 (896 is 4 x 224), 151936 x 896 x 4096 850 / 792, 4096 x 896 x 4864 33.5 / 31.1, 2048 x 3072 x 3072 39.8 / 37.3 (two
@@ -542,6 +555,7 @@ static int gemm_impl(const void* A, const void* B, void* C, const void* bias,
     p.b_fmt = b_dtype == 3 ? 2 : (b_dtype == 0 ? 1 : (b_dtype == 1 ? 0 : 1));
     p.C = C; p.ldc = ldc; p.c_dtype = c_dtype; p.accumulate = accumulate;
     p.bias = bias; p.bias_dtype = bias_dtype;
+    p.group_rows = pair_group_rows(K, eb, rs != nullptr || ready_flags != nullptr);
     p.bn = pair_bn; p.b_stage_bytes = b_rows * 128;
     p.c_sectors = rs == nullptr && (accumulate || !pair_kernel) && c_dtype == 0 && N % 16 == 0 && ldc % 16 == 0 && (reinterpret_cast<uintptr_t>(C) & 31u) == 0;
     p.scale_a = scale_a; p.scale_b = scale_b; p.alpha = alpha;

@@ -45,9 +45,8 @@ constexpr int EPI_WARPS = 4;
 constexpr int EPI_STAGE_OFFSET = STAGES * STAGE_BYTES + 1024;
 constexpr int SMEM_BYTES = EPI_STAGE_OFFSET + 2 * EPI_WARPS * EPI_STAGE_BYTES_PER_WARP + 1024;
 
-__device__ __forceinline__ void tile_coords(int t, int tiles_m, int tiles_n, int rot, int& tm, int& tn) {
-    constexpr int G = 8;             // 8 pair-rows (2048 rows of A) share each B tile while it is hot in L2
-    int per_group = G * tiles_n;
+__device__ __forceinline__ void tile_coords(int t, int tiles_m, int tiles_n, int rot, int G, int& tm, int& tn) {
+    int per_group = G * tiles_n;     // G tile rows share each B tile while it is hot in L2
     int group = t / per_group;
     int first_m = group * G;
     int gsz = min(tiles_m - first_m, G);
@@ -126,7 +125,7 @@ gemm_tcgen05_2cta_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gri
                 }
             };
             for (int t = pair; t < num_tiles && ok; t += num_pairs) {
-                int tm, tn; tile_coords(t, tiles_m, tiles_n, rot, tm, tn);
+                int tm, tn; tile_coords(t, tiles_m, tiles_n, rot, p.group_rows, tm, tn);
                 const int row0 = (tm * 2 + static_cast<int>(rank)) * BM;               // this CTA's rows of A / C
                 const int brow0 = p.ep_mode == 1 ? tn * BN_HALF + static_cast<int>(rank) * p.ep_D
                                                  : tn * bn + static_cast<int>(rank) * bn_half;   // this CTA's rows of B
@@ -230,7 +229,7 @@ gemm_tcgen05_2cta_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gri
         int acc = 0; uint32_t acc_phase = 0;
         bool ok = true;
         for (int t = pair; t < num_tiles && ok; t += num_pairs) {
-            int tm, tn; tile_coords(t, tiles_m, tiles_n, rot, tm, tn);
+            int tm, tn; tile_coords(t, tiles_m, tiles_n, rot, p.group_rows, tm, tn);
             if (!mbar_wait(tfull_bar(acc), acc_phase, abort_flag)) { if (lane == 0) atomicOr(p.status, kErrTmemFull); ok = false; break; }
             tc_fence_after_sync();
             __syncwarp();
