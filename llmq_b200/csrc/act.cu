@@ -26,6 +26,7 @@ __global__ void __launch_bounds__(256)
 swiglu_fwd_kernel(T* __restrict__ out, e4m3* __restrict__ q_out, const T* __restrict__ inp, long long rows, int D,
                   float* __restrict__ absmax_out, const float* __restrict__ known_absmax, float* __restrict__ q_scale_out,
                   const FastDiv fd) {
+    grid_release();
     __shared__ float scratch[32];
     using V = Vec16<T>;
     const int vec_per_row = D / V::N;
@@ -113,6 +114,7 @@ template <typename T>
 __global__ void __launch_bounds__(256)
 swiglu_bwd_kernel(T* dinp, const T* __restrict__ dout, const T* inp, long long rows, int D, float* __restrict__ absmax_out,
                   const FastDiv fd) {
+    grid_release();
     __shared__ float scratch[32];
     using V = Vec16<T>;
     const int vec_per_row = D / V::N;
@@ -273,6 +275,8 @@ template <typename T, bool Backward>
 __global__ void __launch_bounds__(256)
 rope_kernel(T* out, const T* inp, const float* __restrict__ freqs, int B, int Tlen, int Hq, int Hkv, int HS,
             float* __restrict__ absmax_out, const FastDiv fd_vec, const FastDiv fd_h, const FastDiv fd_t) {
+    grid_wait();
+    const int bx = after_wait(blockIdx.x), tx = after_wait(threadIdx.x);
     __shared__ float scratch[32];
     using V = Vec16<T>;
     const int half = HS / 2;
@@ -280,7 +284,7 @@ rope_kernel(T* out, const T* inp, const float* __restrict__ freqs, int B, int Tl
     const int H = Hq + 2 * Hkv;
     const long long total = static_cast<long long>(B) * Tlen * H * vec_per_half;
     float tmax = 0.f;
-    for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < total;
+    for (long long i = bx * static_cast<long long>(blockDim.x) + tx; i < total;
          i += static_cast<long long>(gridDim.x) * blockDim.x) {
         int v, h, t;
         long long bt;
@@ -391,15 +395,15 @@ extern "C" int llmq_rope(void* out, const void* inp, const float* freqs, int B, 
         constexpr int VN = 8;
         long long work = static_cast<long long>(B) * T * H * (HS / 2 / 8);
         int g = grid_for(work, num_sms, kRopeRounds);
-        if (backward) rope_kernel<bf16, true><<<g, 256, 0, s>>>(static_cast<bf16*>(out), static_cast<const bf16*>(inp), freqs, B, T, Hq, Hkv, HS, absmax, FastDiv(HS / 2 / VN), FastDiv(H), FastDiv(T));
-        else rope_kernel<bf16, false><<<g, 256, 0, s>>>(static_cast<bf16*>(out), static_cast<const bf16*>(inp), freqs, B, T, Hq, Hkv, HS, absmax, FastDiv(HS / 2 / VN), FastDiv(H), FastDiv(T));
+        if (backward) launch_chained(rope_kernel<bf16, true>, g, 256, 0, s, static_cast<bf16*>(out), static_cast<const bf16*>(inp), freqs, B, T, Hq, Hkv, HS, absmax, FastDiv(HS / 2 / VN), FastDiv(H), FastDiv(T));
+        else launch_chained(rope_kernel<bf16, false>, g, 256, 0, s, static_cast<bf16*>(out), static_cast<const bf16*>(inp), freqs, B, T, Hq, Hkv, HS, absmax, FastDiv(HS / 2 / VN), FastDiv(H), FastDiv(T));
     } else if (dtype == 3) {
         if ((HS / 2) % 4) return -1;
         constexpr int VN = 4;
         long long work = static_cast<long long>(B) * T * H * (HS / 2 / 4);
         int g = grid_for(work, num_sms, kRopeRounds);
-        if (backward) rope_kernel<float, true><<<g, 256, 0, s>>>(static_cast<float*>(out), static_cast<const float*>(inp), freqs, B, T, Hq, Hkv, HS, absmax, FastDiv(HS / 2 / VN), FastDiv(H), FastDiv(T));
-        else rope_kernel<float, false><<<g, 256, 0, s>>>(static_cast<float*>(out), static_cast<const float*>(inp), freqs, B, T, Hq, Hkv, HS, absmax, FastDiv(HS / 2 / VN), FastDiv(H), FastDiv(T));
+        if (backward) launch_chained(rope_kernel<float, true>, g, 256, 0, s, static_cast<float*>(out), static_cast<const float*>(inp), freqs, B, T, Hq, Hkv, HS, absmax, FastDiv(HS / 2 / VN), FastDiv(H), FastDiv(T));
+        else launch_chained(rope_kernel<float, false>, g, 256, 0, s, static_cast<float*>(out), static_cast<const float*>(inp), freqs, B, T, Hq, Hkv, HS, absmax, FastDiv(HS / 2 / VN), FastDiv(H), FastDiv(T));
     } else return -10;
     return LLMQ_LAUNCH_CHECK();
 }

@@ -162,6 +162,7 @@ attn_fwd_pingpong_kernel(const __grid_constant__ CUtensorMap tmap_qkv,     // qk
     __syncthreads();
     tc_fence_after_sync();
     const uint32_t tmem = *tmem_slot;
+    grid_wait();
 
     if (warp == 8) {
         // ============================================================ TMA producer
@@ -477,8 +478,8 @@ int launch(void* out, float* lse, const void* qkv, int B, int T, int Hq, int Hkv
     const bool paired = T <= BQ && Hq / Hkv > 1 && static_cast<long long>(Hq) * B > sms[dev & 63];
     const long long total = paired ? static_cast<long long>(pairs_of_group(p)) * Hkv * B : static_cast<long long>(nqb) * Hq * B;
     const int grid = static_cast<int>(total < sms[dev & 63] ? total : sms[dev & 63]);       // one CTA per SM (tensor memory)
-    if (paired) attn_fwd_pingpong_kernel<HS, true><<<grid, NUM_THREADS, smem, s>>>(tmap, p);
-    else        attn_fwd_pingpong_kernel<HS, false><<<grid, NUM_THREADS, smem, s>>>(tmap, p);
+    if (paired) launch_chained(attn_fwd_pingpong_kernel<HS, true>, grid, NUM_THREADS, smem, s, tmap, p);
+    else        launch_chained(attn_fwd_pingpong_kernel<HS, false>, grid, NUM_THREADS, smem, s, tmap, p);
     return LLMQ_LAUNCH_CHECK();
 }
 

@@ -97,6 +97,10 @@ int encode_btw(CUtensorMap* out, const void* base, int B, int T, long long W, in
     return r == CUDA_SUCCESS ? 0 : 1000 + static_cast<int>(r);
 }
 
+// not __ldg: the compiler may move such a load in front of grid_wait()
+template <typename V>
+__device__ __forceinline__ V load_plain(const V* p) { return *p; }
+
 struct AttnParams {
     int B, T, Hq, Hkv;
     float scale;                 // 1/sqrt(HS)
@@ -114,9 +118,11 @@ struct AttnParams {
 template <int HS>
 __global__ void __launch_bounds__(256)
 attn_delta_kernel(float* __restrict__ delta, const bf16* __restrict__ o, const bf16* __restrict__ d_o, int B, int T, int Hq) {
+    grid_wait();
+    const int bx = after_wait(blockIdx.x), tx = after_wait(threadIdx.x);
     constexpr int LANES = HS / 8;                       // lanes per row
     static_assert(LANES == 8 || LANES == 16, "head sizes 64 and 128");
-    const long long gid = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x;
+    const long long gid = bx * static_cast<long long>(blockDim.x) + tx;
     const long long w = gid / LANES;                    // row index over (b, t, h)
     const int sub = static_cast<int>(gid % LANES);
     const long long total = static_cast<long long>(B) * T * Hq;
@@ -235,6 +241,7 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmap_kv128,   // qkv, b
     __syncthreads();
     tc_fence_after_sync();
     const uint32_t tmem = *tmem_slot;
+    grid_wait();
     const uint32_t tdV = tmem + 4 * BQ, tdK = tdV + HS;
     const uint32_t tK = tdK + HS, tV = tK + HS / 2;           // HS = 64
     const uint32_t lane_off = static_cast<uint32_t>((warp & 3) * 32) << 16;
@@ -265,7 +272,7 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmap_kv128,   // qkv, b
             for (int i = 0; i < 2; ++i) {
                 const int q = qb * BQ + lane + 32 * i;
                 const long long si = (static_cast<long long>(b) * p.Hq + hq) * p.T + q;
-                st[i] = q < p.T ? make_float2(__ldg(p.lse + si), __ldg(p.delta + si)) : make_float2(INFINITY, 0.f);
+                st[i] = q < p.T ? make_float2(load_plain(p.lse + si), load_plain(p.delta + si)) : make_float2(INFINITY, 0.f);
             }
         };
         if (n_it > 0) load_stats(stat);
@@ -367,7 +374,7 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmap_kv128,   // qkv, b
                                                                       (grp == 0 ? kcol : vcol) + half * 32);
 #pragma unroll
                     for (int q4 = 0; q4 < 4; ++q4) {
-                        const uint4 x = __ldg(src + q4);
+                        const uint4 x = load_plain(src + q4);
                         w[4 * q4] = x.x; w[4 * q4 + 1] = x.y; w[4 * q4 + 2] = x.z; w[4 * q4 + 3] = x.w;
                     }
                 }
@@ -585,6 +592,7 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmap_qkv64,   // qkv, box
     __syncthreads();
     tc_fence_after_sync();
     const uint32_t tmem = *tmem_slot;
+    grid_wait();
     const uint32_t tQ = tmem, tdO = tmem + HS / 2, tdQ = tmem + HS + 4 * BKV;
     auto tS = [&](int t) { return tmem + HS + (t & 1) * BKV; };
     auto tdP = [&](int t) { return tmem + HS + 2 * BKV + (t & 1) * BKV; };
@@ -619,7 +627,7 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmap_qkv64,   // qkv, box
             for (int i = 0; i < 4; ++i) {
                 const int q = q0 + lane + 32 * i;
                 const long long si = (static_cast<long long>(b) * p.Hq + hq) * p.T + q;
-                st[i] = q < p.T ? make_float2(__ldg(p.lse + si), __ldg(p.delta + si)) : make_float2(INFINITY, 0.f);
+                st[i] = q < p.T ? make_float2(load_plain(p.lse + si), load_plain(p.delta + si)) : make_float2(INFINITY, 0.f);
             }
             if (g > 0 && !mbar_wait_warp(stage_free, (g - 1) & 1, abort_flag)) { if (lane == 0) atomicOr(p.status, kErrOther); break; }
             if (lane == 0) {
@@ -891,7 +899,7 @@ int bwd_impl(void* dqkv, float* delta, const void* d_out, const void* out, const
     {
         long long rows = static_cast<long long>(B) * T * Hq;
         long long blocks = (rows * (HS / 8) + 255) / 256;
-        attn_delta_kernel<HS><<<static_cast<unsigned int>(blocks), 256, 0, s>>>(delta, static_cast<const bf16*>(out), static_cast<const bf16*>(d_out), B, T, Hq);
+        launch_chained(attn_delta_kernel<HS>, static_cast<unsigned int>(blocks), 256, 0, s, delta, static_cast<const bf16*>(out), static_cast<const bf16*>(d_out), B, T, Hq);
         int rc = LLMQ_LAUNCH_CHECK();
         if (rc) return rc;
     }
@@ -910,13 +918,7 @@ int bwd_impl(void* dqkv, float* delta, const void* d_out, const void* out, const
         rc = set_smem<1000 + HS>(attn_bwd_dkdv_kernel<HS>, smem);
         if (rc) return rc;
         const int parts = HS == 128 ? head_parts(G, base) : 1;
-        cudaLaunchConfig_t cfg{};
-        cfg.gridDim = dim3(base * parts); cfg.blockDim = dim3(kBwdThreads); cfg.dynamicSmemBytes = smem; cfg.stream = s;
-        cudaLaunchAttribute attr{};
-        attr.id = cudaLaunchAttributeClusterDimension;
-        attr.val.clusterDim.x = parts; attr.val.clusterDim.y = 1; attr.val.clusterDim.z = 1;
-        cfg.attrs = &attr; cfg.numAttrs = parts > 1 ? 1 : 0;
-        rc = static_cast<int>(cudaLaunchKernelEx(&cfg, attn_bwd_dkdv_kernel<HS>, t128, t64, tdo64, p, parts));
+        rc = static_cast<int>(launch_chained_cluster(attn_bwd_dkdv_kernel<HS>, base * parts, kBwdThreads, smem, s, parts, t128, t64, tdo64, p, parts));
         if (rc) return rc;
     }
     {
@@ -924,7 +926,7 @@ int bwd_impl(void* dqkv, float* delta, const void* d_out, const void* out, const
         rc = set_smem<2000 + HS>(attn_bwd_dq_kernel<HS>, smem);
         if (rc) return rc;
         const int heads = heads_per_cta(G, base);
-        attn_bwd_dq_kernel<HS><<<base * ((G + heads - 1) / heads), kBwdDqThreads, smem, s>>>(t64, tdo64, p, heads);
+        launch_chained(attn_bwd_dq_kernel<HS>, base * ((G + heads - 1) / heads), kBwdDqThreads, smem, s, t64, tdo64, p, heads);
         rc = LLMQ_LAUNCH_CHECK();
     }
     return rc;

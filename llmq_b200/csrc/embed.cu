@@ -13,10 +13,12 @@ namespace {
 template <typename T>
 __global__ void __launch_bounds__(256)
 encoder_fwd_kernel(T* __restrict__ out, const int* __restrict__ tokens, const T* __restrict__ wte, long long BT, int C, int V) {
+    grid_wait();
+    const int bx = after_wait(blockIdx.x), tx = after_wait(threadIdx.x);
     using Vt = Vec16<T>;
     const int vec_per_row = C / Vt::N;
     const long long total = BT * vec_per_row;
-    for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < total;
+    for (long long i = bx * static_cast<long long>(blockDim.x) + tx; i < total;
          i += static_cast<long long>(gridDim.x) * blockDim.x) {
         long long r = i / vec_per_row;
         int c = static_cast<int>(i - r * vec_per_row) * Vt::N;
@@ -32,8 +34,10 @@ encoder_fwd_kernel(T* __restrict__ out, const int* __restrict__ tokens, const T*
 // 2.7e8 for 16384 tokens, a few microseconds.
 __global__ void __launch_bounds__(256)
 token_rank_kernel(int* __restrict__ rank, int* __restrict__ count, const int* __restrict__ tokens, int BT) {
+    grid_wait();
+    const int bx = after_wait(blockIdx.x), tx = after_wait(threadIdx.x);
     __shared__ int chunk[2048];
-    const int p = blockIdx.x * 256 + threadIdx.x;
+    const int p = bx * 256 + tx;
     const int tok = p < BT ? tokens[p] : -1;
     const int per_split = (BT + gridDim.y - 1) / gridDim.y;
     const int q_begin = blockIdx.y * per_split, q_end = min(BT, q_begin + per_split);
@@ -41,7 +45,7 @@ token_rank_kernel(int* __restrict__ rank, int* __restrict__ count, const int* __
     for (int q0 = q_begin; q0 < q_end; q0 += 2048) {
         const int n = min(2048, q_end - q0);
         __syncthreads();
-        for (int i = threadIdx.x; i < n; i += 256) chunk[i] = tokens[q0 + i];
+        for (int i = tx; i < n; i += 256) chunk[i] = tokens[q0 + i];
         __syncthreads();
         const int before = min(n, max(0, p - q0));            // entries of this chunk with q < p
         int i = 0;
@@ -61,15 +65,17 @@ template <typename T>
 __global__ void __launch_bounds__(256)
 encoder_bwd_kernel(T* __restrict__ dwte, const T* __restrict__ dout, const int* __restrict__ tokens, const int* __restrict__ rank,
                    const int* __restrict__ count, int BT, int C, int V) {
+    grid_wait();
+    const int bx = after_wait(blockIdx.x), tx = after_wait(threadIdx.x);
     using Vt = Vec16<T>;
     constexpr int LIST = 1024;
     __shared__ int list[LIST];
     __shared__ int warp_cnt[8];
-    const int p = blockIdx.x;
+    const int p = bx;
     if (rank[p] != 0) return;
     const long long tok = tokens[p];
     if (tok < 0 || tok >= V) return;                           // ids outside the vocabulary never index memory
-    const int c = (blockIdx.y * 256 + threadIdx.x) * Vt::N;
+    const int c = (blockIdx.y * 256 + tx) * Vt::N;
     const bool active = c < C;
     float acc[Vt::N];
     Vt cur;
@@ -80,13 +86,13 @@ encoder_bwd_kernel(T* __restrict__ dwte, const T* __restrict__ dout, const int* 
         for (int k = 0; k < Vt::N; ++k) acc[k] = to_float(cur.v[k]) + to_float(g.v[k]);
     }
     int remaining = count[p] - 1;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int lane = tx & 31, warp = tx >> 5;
     int q0 = p + 1;
     while (remaining > 0 && q0 < BT) {                          // uniform across the CTA
         // fill the list with up to LIST later positions of this token, in ascending order
         int filled = 0;
         while (filled + 256 <= LIST && q0 < BT && filled < remaining) {
-            const int q = q0 + threadIdx.x;
+            const int q = q0 + tx;
             const bool m = q < BT && tokens[q] == static_cast<int>(tok);
             const unsigned ballot = __ballot_sync(0xffffffffu, m);
             if (lane == 0) warp_cnt[warp] = __popc(ballot);
@@ -121,9 +127,11 @@ encoder_bwd_kernel(T* __restrict__ dwte, const T* __restrict__ dout, const int* 
 template <typename T>
 __global__ void __launch_bounds__(256)
 bias_bwd_partial_kernel(float* __restrict__ partial, const T* __restrict__ dout, long long rows, int C) {
+    grid_wait();
+    const int bx = after_wait(blockIdx.x), tx = after_wait(threadIdx.x);
     __shared__ float tile[8][33];
-    const int cx = threadIdx.x & 31, ry = threadIdx.x >> 5;      // 32 columns x 8 row lanes
-    const int c = blockIdx.x * 32 + cx;
+    const int cx = tx & 31, ry = tx >> 5;      // 32 columns x 8 row lanes
+    const int c = bx * 32 + cx;
     float s = 0.f;
     if (c < C) {
         for (long long r = blockIdx.y * 8 + ry; r < rows; r += static_cast<long long>(gridDim.y) * 8) s += to_float(dout[r * C + c]);
@@ -144,9 +152,11 @@ bias_bwd_partial_kernel(float* __restrict__ partial, const T* __restrict__ dout,
 template <typename T>
 __global__ void __launch_bounds__(256)
 bias_bwd_partial_vec4_kernel(float* __restrict__ partial, const T* __restrict__ dout, long long rows, int C) {
+    grid_wait();
+    const int bx = after_wait(blockIdx.x), tx = after_wait(threadIdx.x);
     __shared__ float tile[8][32][5];
-    const int cx = threadIdx.x & 31, ry = threadIdx.x >> 5;
-    const int c = blockIdx.x * 128 + cx * 4;
+    const int cx = tx & 31, ry = tx >> 5;
+    const int c = bx * 128 + cx * 4;
     float s[4] = {0.f, 0.f, 0.f, 0.f};
     if (c < C) {
         struct alignas(sizeof(T) * 4) Quad { T v[4]; };
@@ -173,7 +183,9 @@ bias_bwd_partial_vec4_kernel(float* __restrict__ partial, const T* __restrict__ 
 template <typename T>
 __global__ void bias_bwd_final_kernel(T* __restrict__ dbias, const float* __restrict__ partial, int slices, int C,
                                       const float* __restrict__ scale_a, const float* __restrict__ scale_b, int accumulate) {
-    int c = blockIdx.x * blockDim.x + threadIdx.x;
+    grid_wait(scale_a, scale_b);
+    const int bx = after_wait(blockIdx.x), tx = after_wait(threadIdx.x);
+    int c = bx * blockDim.x + tx;
     if (c >= C) return;
     float s = 0.f;
     for (int k = 0; k < slices; ++k) s += partial[static_cast<long long>(k) * C + c];
@@ -191,12 +203,12 @@ extern "C" int llmq_encoder_forward(void* out, const int* tokens, const void* wt
     if (dtype == 0) {
         if (C % 8) return -1;
         long long blocks = ceil_div_ll(BT * (C / 8), 256);
-        encoder_fwd_kernel<bf16><<<static_cast<int>(blocks < num_sms * 8LL ? blocks : num_sms * 8LL), 256, 0, s>>>(
+        launch_chained(encoder_fwd_kernel<bf16>, static_cast<int>(blocks < num_sms * 8LL ? blocks : num_sms * 8LL), 256, 0, s,
             static_cast<bf16*>(out), tokens, static_cast<const bf16*>(wte), BT, C, V);
     } else if (dtype == 3) {
         if (C % 4) return -1;
         long long blocks = ceil_div_ll(BT * (C / 4), 256);
-        encoder_fwd_kernel<float><<<static_cast<int>(blocks < num_sms * 8LL ? blocks : num_sms * 8LL), 256, 0, s>>>(
+        launch_chained(encoder_fwd_kernel<float>, static_cast<int>(blocks < num_sms * 8LL ? blocks : num_sms * 8LL), 256, 0, s,
             static_cast<float*>(out), tokens, static_cast<const float*>(wte), BT, C, V);
     } else return -10;
     return LLMQ_LAUNCH_CHECK();
@@ -216,11 +228,11 @@ extern "C" int llmq_encoder_backward(void* dwte, const void* dout, const int* to
     const int pblocks = ceil_div_i(BT, 256);
     int splits = 1;
     while (splits < 8 && pblocks * splits < 256 && BT / (splits * 2) >= 2048) splits *= 2;
-    token_rank_kernel<<<dim3(pblocks, splits), 256, 0, s>>>(rank, count, tokens, BT);
+    launch_chained(token_rank_kernel, dim3(pblocks, splits), 256, 0, s, rank, count, tokens, BT);
     if (dtype == 0) {
-        encoder_bwd_kernel<bf16><<<dim3(BT, ceil_div_i(C, 256 * 8)), 256, 0, s>>>(static_cast<bf16*>(dwte), static_cast<const bf16*>(dout), tokens, rank, count, BT, C, V);
+        launch_chained(encoder_bwd_kernel<bf16>, dim3(BT, ceil_div_i(C, 256 * 8)), 256, 0, s, static_cast<bf16*>(dwte), static_cast<const bf16*>(dout), tokens, rank, count, BT, C, V);
     } else {
-        encoder_bwd_kernel<float><<<dim3(BT, ceil_div_i(C, 256 * 4)), 256, 0, s>>>(static_cast<float*>(dwte), static_cast<const float*>(dout), tokens, rank, count, BT, C, V);
+        launch_chained(encoder_bwd_kernel<float>, dim3(BT, ceil_div_i(C, 256 * 4)), 256, 0, s, static_cast<float*>(dwte), static_cast<const float*>(dout), tokens, rank, count, BT, C, V);
     }
     return LLMQ_LAUNCH_CHECK();
 }
@@ -234,8 +246,8 @@ extern "C" int llmq_bias_backward(void* dbias, float* partial, const void* dout,
     dim3 grid(ceil_div_i(C, vec4 ? 128 : 32), slices);
 #define BIAS_PARTIAL(T)                                                                                             \
     do {                                                                                                            \
-        if (vec4) bias_bwd_partial_vec4_kernel<T><<<grid, 256, 0, s>>>(partial, static_cast<const T*>(dout), rows, C); \
-        else bias_bwd_partial_kernel<T><<<grid, 256, 0, s>>>(partial, static_cast<const T*>(dout), rows, C);       \
+        if (vec4) launch_chained(bias_bwd_partial_vec4_kernel<T>, grid, 256, 0, s, partial, static_cast<const T*>(dout), rows, C); \
+        else launch_chained(bias_bwd_partial_kernel<T>, grid, 256, 0, s, partial, static_cast<const T*>(dout), rows, C);       \
     } while (0)
     if (dout_dtype == 0) BIAS_PARTIAL(bf16);
     else if (dout_dtype == 3) BIAS_PARTIAL(float);
@@ -245,8 +257,8 @@ extern "C" int llmq_bias_backward(void* dbias, float* partial, const void* dout,
     else return -10;
     int rc = LLMQ_LAUNCH_CHECK();
     if (rc) return rc;
-    if (dbias_dtype == 0) bias_bwd_final_kernel<bf16><<<ceil_div_i(C, 256), 256, 0, s>>>(static_cast<bf16*>(dbias), partial, slices, C, scale_a, scale_b, accumulate);
-    else if (dbias_dtype == 3) bias_bwd_final_kernel<float><<<ceil_div_i(C, 256), 256, 0, s>>>(static_cast<float*>(dbias), partial, slices, C, scale_a, scale_b, accumulate);
+    if (dbias_dtype == 0) launch_chained(bias_bwd_final_kernel<bf16>, ceil_div_i(C, 256), 256, 0, s, static_cast<bf16*>(dbias), partial, slices, C, scale_a, scale_b, accumulate);
+    else if (dbias_dtype == 3) launch_chained(bias_bwd_final_kernel<float>, ceil_div_i(C, 256), 256, 0, s, static_cast<float*>(dbias), partial, slices, C, scale_a, scale_b, accumulate);
     else return -10;
     return LLMQ_LAUNCH_CHECK();
 }

@@ -76,7 +76,7 @@ __device__ __forceinline__ void add_bias32(const GemmParams& p, int col0, float 
         const uint4* bp = reinterpret_cast<const uint4*>(static_cast<const __nv_bfloat16*>(p.bias) + col0);
 #pragma unroll
         for (int g = 0; g < 4; ++g) {
-            uint4 bv = __ldg(bp + g);
+            const uint4 bv = bp[g];        // not __ldg: the compiler may move such a load in front of grid_wait()
             const __nv_bfloat162* bh = reinterpret_cast<const __nv_bfloat162*>(&bv);
 #pragma unroll
             for (int j = 0; j < 4; ++j) {

@@ -100,6 +100,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
     __syncthreads();
     tc_fence_after_sync();
     const uint32_t tmem_base = *tmem_slot;
+    grid_wait();
 
     if (warp == 0) {
         // ------------------------------------------------------------------ TMA producer
@@ -224,6 +225,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
 
 // Sum of the split-K parts + the normal epilogue (alpha, bias, accumulate, bf16 / fp32 store, abs-max).
 __global__ void __launch_bounds__(256) splitk_reduce_kernel(const GemmParams p, float alpha_host) {
+    grid_wait();
     __shared__ float scratch[32];
     float alpha = alpha_host;
     if (p.scale_a) alpha *= *p.scale_a;
@@ -255,6 +257,7 @@ __global__ void __launch_bounds__(256) splitk_reduce_kernel(const GemmParams p, 
 // 4, aligned C): 16-byte loads of the parts, and a multiply instead of a 64-bit division per element.  1152 x 896 from two parts:
 // 3.8 us against 14.
 __global__ void __launch_bounds__(256) splitk_reduce_vec_kernel(const GemmParams p, float alpha_host, const FastDiv fd) {
+    grid_wait();
     __shared__ float scratch[32];
     float alpha = alpha_host;
     if (p.scale_a) alpha *= *p.scale_a;
@@ -599,12 +602,12 @@ static int gemm_impl(const void* A, const void* B, void* C, const void* bias,
     const int items = tiles * splits;
     int grid = items < num_sms ? items : num_sms;
     if (bn == 128) {
-        if (eb == 1) gemm_tcgen05_kernel<1, 128><<<grid, NUM_THREADS, Tile<128>::SMEM_BYTES, stream>>>(ta, tb, p);
-        else         gemm_tcgen05_kernel<0, 128><<<grid, NUM_THREADS, Tile<128>::SMEM_BYTES, stream>>>(ta, tb, p);
+        if (eb == 1) launch_chained(gemm_tcgen05_kernel<1, 128>, grid, NUM_THREADS, Tile<128>::SMEM_BYTES, stream, ta, tb, p);
+        else         launch_chained(gemm_tcgen05_kernel<0, 128>, grid, NUM_THREADS, Tile<128>::SMEM_BYTES, stream, ta, tb, p);
     } else {
-        if (eb == 1)      gemm_tcgen05_kernel<1, 256><<<grid, NUM_THREADS, Tile<256>::SMEM_BYTES, stream>>>(ta, tb, p);
-        else if (eb == 2) gemm_tcgen05_kernel<0, 256><<<grid, NUM_THREADS, Tile<256>::SMEM_BYTES, stream>>>(ta, tb, p);
-        else              gemm_tcgen05_kernel<2, 256><<<grid, NUM_THREADS, Tile<256>::SMEM_BYTES, stream>>>(ta, tb, p);
+        if (eb == 1)      launch_chained(gemm_tcgen05_kernel<1, 256>, grid, NUM_THREADS, Tile<256>::SMEM_BYTES, stream, ta, tb, p);
+        else if (eb == 2) launch_chained(gemm_tcgen05_kernel<0, 256>, grid, NUM_THREADS, Tile<256>::SMEM_BYTES, stream, ta, tb, p);
+        else              launch_chained(gemm_tcgen05_kernel<2, 256>, grid, NUM_THREADS, Tile<256>::SMEM_BYTES, stream, ta, tb, p);
     }
     if (splits > 1) {
         const long long total = static_cast<long long>(M) * N;             // at most kSplitFloats / 2
@@ -612,12 +615,12 @@ static int gemm_impl(const void* A, const void* B, void* C, const void* bias,
         if (N % 4 == 0 && ldc % 4 == 0 && reinterpret_cast<uintptr_t>(C) % out_bytes == 0) {
             long long blocks = (total / 4 + 255) / 256;
             if (blocks > 8LL * num_sms) blocks = 8LL * num_sms;
-            splitk_reduce_vec_kernel<<<static_cast<unsigned int>(blocks), 256, 0, stream>>>(p, p.alpha, FastDiv(static_cast<uint32_t>(N / 4)));
+            launch_chained(splitk_reduce_vec_kernel, static_cast<unsigned int>(blocks), 256, 0, stream, p, p.alpha, FastDiv(static_cast<uint32_t>(N / 4)));
             return static_cast<int>(cudaGetLastError());
         }
         long long blocks = (total + 255) / 256;
         if (blocks > 4LL * num_sms) blocks = 4LL * num_sms;
-        splitk_reduce_kernel<<<static_cast<unsigned int>(blocks), 256, 0, stream>>>(p, p.alpha);
+        launch_chained(splitk_reduce_kernel, static_cast<unsigned int>(blocks), 256, 0, stream, p, p.alpha);
     }
     return static_cast<int>(cudaGetLastError());
 }

@@ -104,6 +104,9 @@ gemm_tcgen05_2cta_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gri
     cluster_wait();
     tc_fence_after_sync();
     const uint32_t tmem_base = *tmem_slot;
+    // a kernel that waits for other GPUs keeps its successor off the SMs
+    if (!p.ready_flags && p.rs_world == 0) grid_release();
+    grid_wait_only();
 
     if (warp == 0) {
         // ------------------------------------------------------------------ TMA producer (both CTAs)
@@ -344,7 +347,7 @@ int llmq_gemm_2cta_launch(const CUtensorMap& ta, const CUtensorMap& tb, const CU
     const int tiles = ((p.M + 2 * BM - 1) / (2 * BM)) * (p.ep_mode == 1 ? (p.ep_D + BN_HALF - 1) / BN_HALF : (p.N + p.bn - 1) / p.bn);
     int pairs = num_sms / 2;
     if (tiles < pairs) pairs = tiles;
-    if (p.elem_bytes == 1) gemm_tcgen05_2cta_kernel<true><<<2 * pairs, NUM_THREADS, SMEM_BYTES, stream>>>(ta, tb, tc, p);
-    else                   gemm_tcgen05_2cta_kernel<false><<<2 * pairs, NUM_THREADS, SMEM_BYTES, stream>>>(ta, tb, tc, p);
+    if (p.elem_bytes == 1) launch_chained(gemm_tcgen05_2cta_kernel<true>, 2 * pairs, NUM_THREADS, SMEM_BYTES, stream, ta, tb, tc, p);
+    else                   launch_chained(gemm_tcgen05_2cta_kernel<false>, 2 * pairs, NUM_THREADS, SMEM_BYTES, stream, ta, tb, tc, p);
     return static_cast<int>(cudaGetLastError());
 }

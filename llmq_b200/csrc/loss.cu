@@ -268,6 +268,7 @@ fused_ce_row_kernel(bf16* logits, float* __restrict__ losses, float* __restrict_
 
 // max and sum of the per-token LSE values (z-loss monitoring); out = {max, sum}
 __global__ void __launch_bounds__(1024) lse_stats_kernel(float* __restrict__ out, const float* __restrict__ lse, long long n, int accumulate) {
+    grid_wait(out, lse);
     __shared__ float scratch[32];
     float m = -INFINITY, s = 0.f;
     for (long long i = threadIdx.x; i < n; i += blockDim.x) { float v = lse[i]; m = fmaxf(m, v); s += v; }
@@ -281,14 +282,16 @@ __global__ void __launch_bounds__(1024) lse_stats_kernel(float* __restrict__ out
 
 // out[g] = sum over batch and over positions [g*group, (g+1)*group) of losses(B, T)
 __global__ void __launch_bounds__(256) grouped_loss_kernel(float* __restrict__ out, const float* __restrict__ losses, int B, int T, int group) {
+    grid_wait();
+    const int bx = after_wait(blockIdx.x), tx = after_wait(threadIdx.x);
     __shared__ float scratch[32];
-    const int g = blockIdx.x;
+    const int g = bx;
     const int t0 = g * group, t1 = min(T, t0 + group);
     float s = 0.f;
     for (int b = 0; b < B; ++b)
-        for (int t = t0 + threadIdx.x; t < t1; t += blockDim.x) s += losses[static_cast<long long>(b) * T + t];
+        for (int t = t0 + tx; t < t1; t += blockDim.x) s += losses[static_cast<long long>(b) * T + t];
     s = block_reduce_sum(s, scratch);
-    if (threadIdx.x == 0) out[g] = s;
+    if (tx == 0) out[g] = s;
 }
 
 }  // namespace
@@ -320,13 +323,13 @@ extern "C" int llmq_fused_classifier(void* logits, float* losses, float* lse_out
 }
 
 extern "C" int llmq_lse_stats(float* out, const float* lse, long long n, int accumulate, cudaStream_t s) {
-    lse_stats_kernel<<<1, 1024, 0, s>>>(out, lse, n, accumulate);
+    launch_chained(lse_stats_kernel, 1, 1024, 0, s, out, lse, n, accumulate);
     return LLMQ_LAUNCH_CHECK();
 }
 
 extern "C" int llmq_grouped_loss_sum(float* out, const float* losses, int B, int T, int group, cudaStream_t s) {
     int groups = ceil_div_i(T, group);
     if (groups <= 0) return 0;
-    grouped_loss_kernel<<<groups, 256, 0, s>>>(out, losses, B, T, group);
+    launch_chained(grouped_loss_kernel, groups, 256, 0, s, out, losses, B, T, group);
     return LLMQ_LAUNCH_CHECK();
 }

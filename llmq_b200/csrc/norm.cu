@@ -21,6 +21,7 @@ rmsnorm_fwd_kernel(T* __restrict__ residual_out,      // may be null when not fu
                    const T* __restrict__ weight, float eps, int C,
                    float* __restrict__ absmax_out, const float* __restrict__ known_absmax,
                    float* __restrict__ q_scale_out) {
+    grid_release();
     __shared__ float scratch[32];
     using V = Vec16<T>;
     const long long row = blockIdx.x;
@@ -88,6 +89,7 @@ __global__ void __launch_bounds__(THREADS)
 rmsnorm_fwd_reg_kernel(T* __restrict__ residual_out, T* __restrict__ y_out, e4m3* __restrict__ q_out, float* __restrict__ rstd_out,
                        const T* __restrict__ in_a, const T* __restrict__ in_b, const T* __restrict__ weight, float eps, int C,
                        float* __restrict__ absmax_out, const float* __restrict__ known_absmax, float* __restrict__ q_scale_out) {
+    grid_release();
     __shared__ float scratch[8], scratch_max[THREADS / 32];
     using V = Vec16<T>;
     const long long row = blockIdx.x;
@@ -192,6 +194,7 @@ rmsnorm_bwd_kernel(T* __restrict__ dinp,               // in: upstream residual 
                    float* __restrict__ dw_partial,     // [gridDim.x, C]
                    const T* __restrict__ dout, const T* __restrict__ inp, const T* __restrict__ weight,
                    const float* __restrict__ rstd, int rows, int C, float* __restrict__ absmax_out) {
+    grid_release();
     __shared__ float scratch[32];
     using V = Vec16<T>;
     float dw[VPT][V::N];
@@ -273,6 +276,7 @@ template <typename T, int VPT, int STAGES>
 __global__ void __launch_bounds__(NORM_THREADS, VPT <= 2 ? 3 : 2)
 rmsnorm_bwd_reg_kernel(T* __restrict__ dinp, float* __restrict__ dw_partial, const T* __restrict__ dout, const T* __restrict__ inp,
                        const T* __restrict__ weight, const float* __restrict__ rstd, int rows, int C, float* __restrict__ absmax_out) {
+    grid_release();
     __shared__ float scratch[32];
     __shared__ float dots[2][NORM_THREADS / 32];             // alternating, so that one barrier per row is enough
     extern __shared__ uint4 ring[];                          // [STAGES][3][VPT][NORM_THREADS]
@@ -381,9 +385,11 @@ constexpr int RED_COLS = 64, RED_GROUPS = 16;
 template <typename T>
 __global__ void __launch_bounds__(RED_COLS * RED_GROUPS)
 rmsnorm_bwd_reduce_kernel(T* __restrict__ dweight, const float* __restrict__ dw_partial, int nparts, int C, int accumulate) {
+    grid_wait();
+    const int bx = after_wait(blockIdx.x), tx = after_wait(threadIdx.x);
     __shared__ float part[RED_GROUPS][RED_COLS];
-    const int x = threadIdx.x % RED_COLS, y = threadIdx.x / RED_COLS;
-    const int c = blockIdx.x * RED_COLS + x;
+    const int x = tx % RED_COLS, y = tx / RED_COLS;
+    const int c = bx * RED_COLS + x;
     float s = 0.f;
     if (c < C) {
 #pragma unroll 4
@@ -469,7 +475,7 @@ int launch_bwd(void* dinp, void* dweight, float* scratch, const void* dout, cons
 #undef LAUNCH
     int rc = LLMQ_LAUNCH_CHECK();
     if (rc) return rc;
-    rmsnorm_bwd_reduce_kernel<T><<<ceil_div_i(C, RED_COLS), RED_COLS * RED_GROUPS, 0, s>>>(static_cast<T*>(dweight), scratch, num_blocks, C, accumulate_dw);
+    launch_chained(rmsnorm_bwd_reduce_kernel<T>, ceil_div_i(C, RED_COLS), RED_COLS * RED_GROUPS, 0, s, static_cast<T*>(dweight), scratch, num_blocks, C, accumulate_dw);
     return LLMQ_LAUNCH_CHECK();
 }
 

@@ -154,6 +154,8 @@ adamw_kernel(P* __restrict__ param, const G* __restrict__ grad, M* __restrict__ 
              float* __restrict__ m_scales, long long n, float lr, float beta1, float beta2, float bc1, float bc2, float eps,
              float wd, const float* __restrict__ grad_scale, float* __restrict__ absmax_out, uint32_t seed, long long elem_offset,
              const float* __restrict__ hyper) {
+    grid_wait(grad_scale, hyper);
+    const int bx = after_wait(blockIdx.x), tx = after_wait(threadIdx.x);
     __shared__ float scratch[32];
     if (hyper) {
         // Step-dependent scalars from device memory: {lr, beta1, beta2, 1/(1-beta1^t), 1/(1-beta2^t), eps, weight decay,
@@ -169,7 +171,7 @@ adamw_kernel(P* __restrict__ param, const G* __restrict__ grad, M* __restrict__ 
     const long long stride = static_cast<long long>(gridDim.x) * blockDim.x;
     // all threads of a 16-lane group must iterate together for the e4m3 path: round the loop bound up
     const long long nvec_pad = (nvec + 31) / 32 * 32;       // whole warps take part in the shuffles
-    for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < nvec_pad; i += stride)
+    for (long long i = bx * static_cast<long long>(blockDim.x) + tx; i < nvec_pad; i += stride)
         adamw_vec(i, i < nvec, param, grad, m_state, v_state, m_scales, lr, beta1, beta2, bc1, bc2, eps, wd, gs, seed, elem_offset, tmax);
     block_absmax_commit(absmax_out, tmax, scratch);
 }
@@ -190,13 +192,15 @@ template <typename P, typename G, typename M, typename Vv>
 __global__ void __launch_bounds__(256)
 adamw_multi_kernel(const AdamTensor* __restrict__ tensors, int n_tensors, long long n_chunks, float lr, float beta1, float beta2, float bc1,
                    float bc2, float eps, float wd, const float* __restrict__ grad_scale, uint32_t seed, const float* __restrict__ hyper) {
+    grid_wait(tensors, grad_scale, hyper);
+    const int bx = after_wait(blockIdx.x), tx = after_wait(threadIdx.x);
     __shared__ float scratch[32];
     if (hyper) {
         lr = hyper[0]; beta1 = hyper[1]; beta2 = hyper[2]; bc1 = hyper[3]; bc2 = hyper[4]; eps = hyper[5]; wd = hyper[6];
         seed += __float_as_uint(hyper[7]);
     }
     const float gs = grad_scale ? *grad_scale : 1.f;
-    for (long long chunk = blockIdx.x; chunk < n_chunks; chunk += gridDim.x) {
+    for (long long chunk = bx; chunk < n_chunks; chunk += gridDim.x) {
         int lo = 0, hi = n_tensors - 1;          // last tensor whose first chunk is not behind this one
         while (lo < hi) {
             const int mid = (lo + hi + 1) / 2;
@@ -206,7 +210,7 @@ adamw_multi_kernel(const AdamTensor* __restrict__ tensors, int n_tensors, long l
         const long long nvec = t.n / 8, v0 = (chunk - t.first_chunk) * (kAdamChunk / 8);
         const long long v1 = min((nvec + 31) / 32 * 32, v0 + kAdamChunk / 8);
         float tmax = 0.f;
-        for (long long i = v0 + threadIdx.x; i < v1; i += blockDim.x)
+        for (long long i = v0 + tx; i < v1; i += blockDim.x)
             adamw_vec(i, i < nvec, static_cast<P*>(t.param), static_cast<const G*>(t.grad), static_cast<M*>(t.m), static_cast<Vv*>(t.v), t.m_scales,
                       lr, beta1, beta2, bc1, bc2, eps, t.decay ? wd : 0.f, gs, seed + static_cast<uint32_t>(t.seed), t.elem_offset, tmax);
         block_absmax_commit(t.absmax, tmax, scratch);
@@ -251,9 +255,11 @@ __device__ __forceinline__ float thread_sum_squares(const T* __restrict__ x, lon
 // loads with the registers they want (BLOCKS 0: no bound): 67.9 M 49.6, 50.5, 50.9 / 60.0, 49.4, 57.8.
 template <typename T, int FLIGHT, bool STREAM, int BLOCKS>
 __global__ void __launch_bounds__(512, BLOCKS) norm_squared_kernel(float* __restrict__ out, const T* __restrict__ x, long long n) {
+    grid_wait();
+    const int bx = after_wait(blockIdx.x), tx = after_wait(threadIdx.x);
     __shared__ float scratch[32];
     const float s = block_reduce_sum(thread_sum_squares<T, FLIGHT, STREAM>(x, n), scratch);
-    if (threadIdx.x == 0) out[blockIdx.x] += s;
+    if (tx == 0) out[bx] += s;
 }
 
 // The gradients of all tensors in one launch.  Bit for bit what norm_squared_kernel adds up launch by launch: the same sums per thread
@@ -261,9 +267,11 @@ __global__ void __launch_bounds__(512, BLOCKS) norm_squared_kernel(float* __rest
 // that a block waits at one pair of barriers per 16 tensors instead of two barriers per tensor.
 template <typename T>
 __global__ void __launch_bounds__(512) norm_squared_multi_kernel(float* __restrict__ out, const AdamTensor* __restrict__ tensors, int n_tensors) {
+    grid_wait(tensors);
+    const int bx = after_wait(blockIdx.x), tx = after_wait(threadIdx.x);
     __shared__ float warp_sums[16][16], sums[16];
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    float total = threadIdx.x == 0 ? out[blockIdx.x] : 0.f;
+    const int warp = tx >> 5, lane = tx & 31;
+    float total = tx == 0 ? out[bx] : 0.f;
     for (int t0 = 0; t0 < n_tensors; t0 += 16) {
         const int n = min(16, n_tensors - t0);
         for (int t = 0; t < n; ++t) {
@@ -276,12 +284,13 @@ __global__ void __launch_bounds__(512) norm_squared_multi_kernel(float* __restri
             if (lane == 0) sums[warp] = s;
         }
         __syncthreads();
-        if (threadIdx.x == 0) for (int t = 0; t < n; ++t) total += sums[t];
+        if (tx == 0) for (int t = 0; t < n; ++t) total += sums[t];
     }
-    if (threadIdx.x == 0) out[blockIdx.x] = total;
+    if (tx == 0) out[bx] = total;
 }
 
 __global__ void __launch_bounds__(512) deterministic_sum_kernel(float* __restrict__ out, const float* __restrict__ in, int n) {
+    grid_wait(out, in);
     __shared__ float scratch[32];
     float s = 0.f;
     for (int i = threadIdx.x; i < n; i += blockDim.x) s += in[i];
@@ -291,6 +300,7 @@ __global__ void __launch_bounds__(512) deterministic_sum_kernel(float* __restric
 
 // io[0]: squared norm in -> norm out;  io[1]: multiplier that clips the gradient to `clip` (1 if no clipping)
 __global__ void norm_finish_kernel(float* io, float clip, float* host_norm) {
+    grid_wait(io, host_norm);
     float nsq = io[0];
     float norm = sqrtf(nsq);
     float scale = 1.f;
@@ -382,7 +392,7 @@ extern "C" int llmq_adamw_hyper(void* param, const void* grad, void* m, void* v,
     const int g = m_dtype == 3 && v_dtype == 3 && rounds < (1ll << 30) ? static_cast<int>(rounds) : grid_for(n / 8, 256, num_sms);
 #define A_CASE(P, PC, G, GC, M, MC, V, VC)                                                                          \
     if (p_dtype == PC && g_dtype == GC && m_dtype == MC && v_dtype == VC) {                                         \
-        adamw_kernel<P, G, M, V><<<g, 256, 0, s>>>(static_cast<P*>(param), static_cast<const G*>(grad), static_cast<M*>(m), \
+        launch_chained(adamw_kernel<P, G, M, V>, g, 256, 0, s, static_cast<P*>(param), static_cast<const G*>(grad), static_cast<M*>(m), \
                                                    static_cast<V*>(v), m_scales, n, lr, beta1, beta2, bc1, bc2, eps, wd,   \
                                                    grad_scale, absmax_out, seed, elem_offset, hyper);               \
         return LLMQ_LAUNCH_CHECK();                                                                                 \
@@ -414,7 +424,7 @@ extern "C" int llmq_adamw_multi(const void* tensors, int n_tensors, long long n_
     const AdamTensor* t = static_cast<const AdamTensor*>(tensors);
 #define A_CASE(P, PC, G, GC, M, MC, V, VC)                                                                          \
     if (p_dtype == PC && g_dtype == GC && m_dtype == MC && v_dtype == VC) {                                         \
-        adamw_multi_kernel<P, G, M, V><<<g, 256, 0, s>>>(t, n_tensors, n_chunks, lr, beta1, beta2, bc1, bc2, eps, wd, grad_scale, seed, hyper); \
+        launch_chained(adamw_multi_kernel<P, G, M, V>, g, 256, 0, s, t, n_tensors, n_chunks, lr, beta1, beta2, bc1, bc2, eps, wd, grad_scale, seed, hyper); \
         return LLMQ_LAUNCH_CHECK();                                                                                 \
     }
     A_CASE(bf16, 0, bf16, 0, bf16, 0, bf16, 0)
@@ -434,8 +444,8 @@ extern "C" int llmq_adamw_multi(const void* tensors, int n_tensors, long long n_
 extern "C" int llmq_norm_squared_multi(float* partials, const void* tensors, int n_tensors, int dtype, int num_partials, cudaStream_t s) {
     if (n_tensors <= 0) return 0;
     const AdamTensor* t = static_cast<const AdamTensor*>(tensors);
-    if (dtype == 0) norm_squared_multi_kernel<bf16><<<num_partials, 512, 0, s>>>(partials, t, n_tensors);
-    else if (dtype == 3) norm_squared_multi_kernel<float><<<num_partials, 512, 0, s>>>(partials, t, n_tensors);
+    if (dtype == 0) launch_chained(norm_squared_multi_kernel<bf16>, num_partials, 512, 0, s, partials, t, n_tensors);
+    else if (dtype == 3) launch_chained(norm_squared_multi_kernel<float>, num_partials, 512, 0, s, partials, t, n_tensors);
     else return -10;
     return LLMQ_LAUNCH_CHECK();
 }
@@ -446,7 +456,7 @@ extern "C" int llmq_norm_squared(float* partials, const void* x, long long n, in
     const bool many = n / (dtype == 0 ? 8 : 4) >= 4LL * 512 * num_partials;
     const bf16* h = static_cast<const bf16*>(x);
     const float* f = static_cast<const float*>(x);
-#define GO(P, ...) norm_squared_kernel<__VA_ARGS__><<<num_partials, 512, 0, s>>>(partials, P, n)
+#define GO(P, ...) launch_chained(norm_squared_kernel<__VA_ARGS__>, num_partials, 512, 0, s, partials, P, n)
     if (dtype == 0)               { if (many) GO(h, bf16, 4, true, 4); else GO(h, bf16, 1, false, 4); }
     else if (!many)               GO(f, float, 1, false, 4);
     else if (n * 4 <= 126LL << 20) GO(f, float, 4, false, 4);
@@ -456,12 +466,12 @@ extern "C" int llmq_norm_squared(float* partials, const void* x, long long n, in
 }
 
 extern "C" int llmq_deterministic_sum(float* out, const float* in, int n, cudaStream_t s) {
-    deterministic_sum_kernel<<<1, 512, 0, s>>>(out, in, n);
+    launch_chained(deterministic_sum_kernel, 1, 512, 0, s, out, in, n);
     return LLMQ_LAUNCH_CHECK();
 }
 
 extern "C" int llmq_norm_finish(float* io, float clip, float* host_norm, cudaStream_t s) {
-    norm_finish_kernel<<<1, 1, 0, s>>>(io, clip, host_norm);
+    launch_chained(norm_finish_kernel, 1, 1, 0, s, io, clip, host_norm);
     return LLMQ_LAUNCH_CHECK();
 }
 

@@ -563,3 +563,58 @@ def test_gemm_rounds_of_tiles(M, N, depth):
         lib.llmq_gemm_set_mode(0)
     assert torch.equal(got[0], got[1]) and torch.equal(got[0], got[2])
     assert rel(got[0], a.float().t() @ b.float()) < 4e-3
+
+
+def test_chained_launches_see_what_the_kernel_before_wrote():
+    """Kernels that start while their predecessor runs, each reading scalars or rows that the one before it writes: the results of back-to-back
+    launches and of a captured graph are those of launches with a synchronisation in between."""
+    g = torch.Generator(device=DEV).manual_seed(3)
+    n, B, T, Hq, Hkv, HS = 1 << 20, 2, 200, 6, 2, 64
+    C = (Hq + 2 * Hkv) * HS
+    x0, w = torch.randn(B * T, 256, device=DEV, generator=g).to(BF), (torch.randn(C, 256, device=DEV, generator=g) * 0.06).to(BF)
+    p0, fr = torch.randn(n, device=DEV, generator=g).to(BF), torch.randn(T, HS // 2, 2, device=DEV, generator=g)
+    dout, grad = torch.randn(B, T, Hq, HS, device=DEV, generator=g).to(BF), torch.randn(n, device=DEV, generator=g).to(BF)
+
+    def chain(between):
+        x, p = x0.clone(), p0.clone()
+        m, v, parts, io = torch.zeros_like(p), torch.zeros_like(p), torch.zeros(512, device=DEV), torch.zeros(2, device=DEV)
+        qkv, rot = torch.empty(B * T, C, device=DEV, dtype=BF), torch.empty(B, T, Hq + 2 * Hkv, HS, device=DEV, dtype=BF)
+        out, lse = torch.empty(B, T, Hq, HS, device=DEV, dtype=BF), torch.empty(B, Hq, T, device=DEV)
+        dqkv, scratch, dw, dx = torch.empty_like(rot), torch.empty(B * Hq * T, device=DEV), torch.empty(C, 256, device=DEV, dtype=BF), torch.empty_like(x)
+
+        def body():
+            for step in range(4):
+                for f in (lambda: K.gemm(qkv, x, w), lambda: K.rope(rot, qkv.view_as(rot), fr, Hq, Hkv),
+                          lambda: K.attention_forward(out, lse, rot, Hq, Hkv), lambda: K.attention_backward(dqkv, scratch, dout, out, lse, rot, Hq, Hkv),
+                          lambda: K.gemm(dw, dqkv.view(B * T, C), x, a_mn=True, b_mn=True), lambda: K.gemm(dx, dqkv.view(B * T, C), w, b_mn=True),
+                          lambda: parts.zero_(), lambda: K.norm_squared(parts, p), lambda: K.deterministic_sum(io[0:1], parts), lambda: K.norm_finish(io, 1.0),
+                          lambda: K.adamw(p, grad, m, v, lr=1e-2, beta1=0.9, beta2=0.95, step=step + 1, eps=1e-8, weight_decay=0.1, grad_scale=io[1:2], seed=step),
+                          lambda: x.add_(dx, alpha=0.1)):
+                    f()
+                    if between:
+                        torch.cuda.synchronize()
+        return body, (qkv, out, lse, dqkv, dw, dx, p, m, v, io, x)
+
+    body, want = chain(True)
+    body()
+    for _ in range(5):
+        body, got = chain(False)
+        torch.cuda.synchronize()
+        body()
+        assert all(torch.equal(a, b) for a, b in zip(got, want))
+    body, got = chain(False)
+    start = [t.clone() for t in got]
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.stream(side):
+        body()                                                 # workspaces and attributes exist before the capture
+        with torch.cuda.graph(graph, stream=side):
+            body()
+    torch.cuda.current_stream().wait_stream(side)
+    for _ in range(3):
+        for t, s in zip(got, start):
+            t.copy_(s)
+        graph.replay()
+        torch.cuda.synchronize()
+        assert all(torch.equal(a, b) for a, b in zip(got, want))
