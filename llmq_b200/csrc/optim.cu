@@ -255,7 +255,7 @@ __device__ __forceinline__ float thread_sum_squares(const T* __restrict__ x, lon
 // loads with the registers they want (BLOCKS 0: no bound): 67.9 M 49.6, 50.5, 50.9 / 60.0, 49.4, 57.8.
 template <typename T, int FLIGHT, bool STREAM, int BLOCKS>
 __global__ void __launch_bounds__(512, BLOCKS) norm_squared_kernel(float* __restrict__ out, const T* __restrict__ x, long long n) {
-    grid_wait();
+    grid_wait(x);                        // thread_sum_squares() finds its loads through plain indices
     const int bx = after_wait(blockIdx.x), tx = after_wait(threadIdx.x);
     __shared__ float scratch[32];
     const float s = block_reduce_sum(thread_sum_squares<T, FLIGHT, STREAM>(x, n), scratch);

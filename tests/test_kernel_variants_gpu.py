@@ -618,3 +618,50 @@ def test_chained_launches_see_what_the_kernel_before_wrote():
         graph.replay()
         torch.cuda.synchronize()
         assert all(torch.equal(a, b) for a, b in zip(got, want))
+
+
+def _same_with_and_without_waits(chain):
+    """``chain()`` gives (launches, tensors they write).  Launched back to back and replayed from a graph, they leave the bits that they leave with
+    a synchronisation after every launch."""
+    launches, want = chain()
+    start = [t.clone() for t in want]
+    for f in launches:
+        f()
+        torch.cuda.synchronize()
+    for _ in range(4):
+        launches, got = chain()
+        torch.cuda.synchronize()
+        for f in launches:
+            f()
+        assert all(torch.equal(a, b) for a, b in zip(got, want))
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.stream(side):
+        with torch.cuda.graph(graph, stream=side):
+            for f in launches:
+                f()
+    torch.cuda.current_stream().wait_stream(side)
+    for _ in range(3):
+        for t, s in zip(got, start):
+            t.copy_(s)
+        graph.replay()
+        torch.cuda.synchronize()
+        assert all(torch.equal(a, b) for a, b in zip(got, want))
+
+
+# the norm starts while the GEMM or the update that writes its tensor runs: one and four loads in flight, fp32 beyond the L2
+@pytest.mark.parametrize("dtype,M,N", [(BF, 1001, 896), (BF, 2048, 2048), (torch.float32, 520, 1000), (torch.float32, 2048, 1024), (torch.float32, 8192, 4104)])
+def test_norm_right_behind_the_kernel_that_writes_its_tensor(dtype, M, N):
+    g = torch.Generator(device=DEV).manual_seed(N)
+    a, b = torch.randn(M, 192, device=DEV, generator=g).to(BF), torch.randn(N, 192, device=DEV, generator=g).to(BF)
+    p0, grad = torch.randn(M * N, device=DEV, generator=g).to(dtype), torch.randn(M * N, device=DEV, generator=g).to(dtype)
+
+    def chain():
+        dw, p = torch.full((M, N), 100.0, device=DEV, dtype=dtype), p0.clone()
+        m, v, parts, parts2, io = torch.zeros_like(p), torch.zeros_like(p), torch.zeros(512, device=DEV), torch.zeros(512, device=DEV), torch.zeros(4, device=DEV)
+        return [lambda: K.gemm(dw, a, b), lambda: K.norm_squared(parts, dw), lambda: K.deterministic_sum(io[0:1], parts),
+                lambda: K.adamw(p, grad, m, v, lr=0.1, beta1=0.9, beta2=0.95, step=1, eps=1e-8, weight_decay=0.1, seed=5),
+                lambda: K.norm_squared(parts2, p), lambda: K.deterministic_sum(io[2:3], parts2)], (dw, p, m, v, parts, parts2, io)
+
+    _same_with_and_without_waits(chain)
