@@ -107,8 +107,7 @@ struct AttnParams {
     float* lse;                  // (B,Hq,T), natural log
     const float* delta;          // (B,Hq,T)
     bf16* dqkv;                  // packed gradient
-    const bf16* qkv;             // packed inputs and the output gradient as plain pointers
-    const bf16* d_out;
+    const bf16* qkv;             // packed inputs as a plain pointer
     unsigned int* status;
 };
 
@@ -911,14 +910,15 @@ int bwd_impl(void* dqkv, float* delta, const void* d_out, const void* out, const
     AttnParams p{};
     p.B = B; p.T = T; p.Hq = Hq; p.Hkv = Hkv; p.scale = 1.f / sqrtf(static_cast<float>(HS));
     p.lse = const_cast<float*>(lse); p.delta = delta; p.dqkv = static_cast<bf16*>(dqkv); p.status = status;
-    p.qkv = static_cast<const bf16*>(qkv); p.d_out = static_cast<const bf16*>(d_out);
+    p.qkv = static_cast<const bf16*>(qkv);
     const int base = ((T + 127) / 128) * Hkv * B, G = Hq / Hkv;
     {
         constexpr int smem = DkdvShape<HS>::SMEM_BYTES;
         rc = set_smem<1000 + HS>(attn_bwd_dkdv_kernel<HS>, smem);
         if (rc) return rc;
         const int parts = HS == 128 ? head_parts(G, base) : 1;
-        rc = static_cast<int>(launch_chained_cluster(attn_bwd_dkdv_kernel<HS>, base * parts, kBwdThreads, smem, s, parts, t128, t64, tdo64, p, parts));
+        launch_chained_cluster(attn_bwd_dkdv_kernel<HS>, base * parts, kBwdThreads, smem, s, parts, t128, t64, tdo64, p, parts);
+        rc = LLMQ_LAUNCH_CHECK();
         if (rc) return rc;
     }
     {

@@ -42,9 +42,10 @@ __device__ __forceinline__ int after_wait(unsigned int index) {
     asm volatile("" : "+r"(index));
     return static_cast<int>(index);
 }
-// `cluster` > 1: blocks per cluster along x
+// `cluster` > 1: blocks per cluster along x.  As with <<<>>>, the caller takes the status with LLMQ_LAUNCH_CHECK(), which also clears it: one
+// that stayed behind would be reported again by the launch check of a later, unrelated kernel.
 template <typename... P, typename... A>
-cudaError_t launch_chained_cluster(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, int cluster, A&&... args) {
+void launch_chained_cluster(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, int cluster, A&&... args) {
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = grid; cfg.blockDim = block; cfg.dynamicSmemBytes = smem; cfg.stream = stream;
     cudaLaunchAttribute attr[2]{};
@@ -53,11 +54,11 @@ cudaError_t launch_chained_cluster(void (*kernel)(P...), dim3 grid, dim3 block, 
     attr[1].id = cudaLaunchAttributeClusterDimension;
     attr[1].val.clusterDim.x = cluster; attr[1].val.clusterDim.y = 1; attr[1].val.clusterDim.z = 1;
     cfg.attrs = attr; cfg.numAttrs = cluster > 1 ? 2 : 1;
-    return cudaLaunchKernelEx(&cfg, kernel, std::forward<A>(args)...);
+    static_cast<void>(cudaLaunchKernelEx(&cfg, kernel, std::forward<A>(args)...));
 }
 template <typename... P, typename... A>
-cudaError_t launch_chained(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, A&&... args) {
-    return launch_chained_cluster(kernel, grid, block, smem, stream, 1, std::forward<A>(args)...);
+void launch_chained(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, A&&... args) {
+    launch_chained_cluster(kernel, grid, block, smem, stream, 1, std::forward<A>(args)...);
 }
 
 __host__ __device__ constexpr long long ceil_div_ll(long long a, long long b) { return (a + b - 1) / b; }

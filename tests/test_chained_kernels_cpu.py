@@ -79,6 +79,16 @@ def test_loads_of_chained_kernels_come_after_the_wait():
     assert early_loads(sources) == []
 
 
+def test_every_chained_launch_clears_its_status():
+    """The status of a launch is taken with LLMQ_LAUNCH_CHECK() or cudaGetLastError(): the launch's own result would leave it recorded, and the next
+    kernel's check would report it once more."""
+    for f in FILES:
+        s = _source(f)
+        assert not re.findall(r"(?:=|\breturn\b|\()\s*launch_chained(?:_cluster)?\(.*", s), f.name
+        for m in re.finditer(r"\blaunch_chained(?:_cluster)?\(\s*\w+_kernel\b", s):
+            assert re.search(r"LLMQ_LAUNCH_CHECK\(\)|cudaGetLastError\(\)", s[m.end():s.index("\n}", m.end())]), (f.name, m.group())
+
+
 @pytest.mark.parametrize("wait,load,found", [
     ("grid_wait();", "x[after_wait(threadIdx.x)]", False), ("grid_wait(x);", "x[threadIdx.x]", False), ("grid_wait(x);", "sum(x)", False),
     ("grid_wait();", "x[threadIdx.x]", True), ("grid_wait();", "sum(x)", True), ("", "x[after_wait(threadIdx.x)]", True)])
