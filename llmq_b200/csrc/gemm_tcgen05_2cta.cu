@@ -160,9 +160,9 @@ gemm_tcgen05_2cta_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gri
                         if constexpr (b_load == 0)      tma_load_2d_pair(sb, &tmap_b, fb, k * bk, brow0);
                         else if constexpr (b_load == 1) tma_load_3d_pair(sb, &tmap_b, fb, 0, k * bk, brow0 / mn_chunk);
                         else {
-                            const int box_bytes = bk * ROW_BYTES, nbox = p.b_stage_bytes / box_bytes;
+                            const int nbox = BN_HALF * p.elem_bytes / ROW_BYTES;
                             for (int b = 0; b < nbox; ++b)
-                                tma_load_2d_pair(sb + b * box_bytes, &tmap_b, fb, brow0 + b * mn_chunk, k * bk);
+                                tma_load_2d_pair(sb + b * (B_STAGE_BYTES / nbox), &tmap_b, fb, brow0 + b * mn_chunk, k * bk);
                         }
                         if (++stage == STAGES) { stage = 0; phase ^= 1u; }
                     }
