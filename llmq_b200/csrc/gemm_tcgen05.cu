@@ -200,7 +200,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
         float tmax = 0.f;
         int acc = 0; uint32_t acc_phase = 0;
         bool ok = true;
-        for (int t = blockIdx.x; t < num_tiles && ok; t += gridDim.x) {
+        for (int t = after_wait(blockIdx.x); t < num_tiles && ok; t += gridDim.x) {
             int tm, tn; tile_coords(t / splits, tiles_m, tiles_n, tm, tn);
             if (!mbar_wait(tfull_bar(acc), acc_phase, abort_flag)) { if (lane == 0) atomicOr(p.status, kErrTmemFull); ok = false; break; }
             tc_fence_after_sync();

@@ -231,7 +231,7 @@ gemm_tcgen05_2cta_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gri
         float tmax = 0.f;
         int acc = 0; uint32_t acc_phase = 0;
         bool ok = true;
-        for (int t = pair; t < num_tiles && ok; t += num_pairs) {
+        for (int t = after_wait(pair); t < num_tiles && ok; t += num_pairs) {
             int tm, tn; tile_coords(t, tiles_m, tiles_n, rot, p.group_rows, tm, tn);
             if (!mbar_wait(tfull_bar(acc), acc_phase, abort_flag)) { if (lane == 0) atomicOr(p.status, kErrTmemFull); ok = false; break; }
             tc_fence_after_sync();
