@@ -179,6 +179,11 @@ adamw_kernel(P* __restrict__ param, const G* __restrict__ grad, M* __restrict__ 
 // All tensors of an optimizer step in one launch.  A model has a handful of large tensors and hundreds of small ones; one launch per
 // tensor left the GPU waiting for the host (about 10 us a call) and for the last CTAs of every launch.  A CTA takes chunks of
 // kAdamChunk elements and finds the tensor of a chunk by bisection.  Same arithmetic and random words as adamw_kernel.
+// The table and the step's scalars are found through a zero that comes out of the wait, so that they can be loaded again instead of kept in registers
+// (64, four blocks per SM; 80 and three with their pointers out of the wait: 24 layers of 0.5B shapes, bf16, 960 us, 770 now).  One chunk per block: as
+// many blocks as reside stride through the same few megabytes of every stream in step (as in llmq_adamw_hyper); 8 blocks per SM / this, us:
+// 24 layers of 0.5B shapes, bf16 801 / 773, bf16 and fp32 moments, 6 of 1.5B shapes 935 / 811, all fp32 1178 / 1026, e4m3 and bf16 moments, 12 layers 1701 /
+// 1596, 24 layers of 256 channels, bf16 73.7 / 74.7.
 struct AdamTensor {                              // 11 x 8 bytes, filled by the host
     void* param; const void* grad; void* m; void* v;
     float* m_scales; float* absmax;              // optional
@@ -192,16 +197,17 @@ template <typename P, typename G, typename M, typename Vv>
 __global__ void __launch_bounds__(256)
 adamw_multi_kernel(const AdamTensor* __restrict__ tensors, int n_tensors, long long n_chunks, float lr, float beta1, float beta2, float bc1,
                    float bc2, float eps, float wd, const float* __restrict__ grad_scale, uint32_t seed, const float* __restrict__ hyper) {
-    grid_wait(tensors, grad_scale, hyper);
-    const int bx = after_wait(blockIdx.x), tx = after_wait(threadIdx.x);
+    grid_wait(grad_scale);
+    const int bx = after_wait(blockIdx.x), tx = after_wait(threadIdx.x), zero = after_wait(0u);
     __shared__ float scratch[32];
     if (hyper) {
-        lr = hyper[0]; beta1 = hyper[1]; beta2 = hyper[2]; bc1 = hyper[3]; bc2 = hyper[4]; eps = hyper[5]; wd = hyper[6];
-        seed += __float_as_uint(hyper[7]);
+        const float* h = hyper + zero;
+        lr = h[0]; beta1 = h[1]; beta2 = h[2]; bc1 = h[3]; bc2 = h[4]; eps = h[5]; wd = h[6];
+        seed += __float_as_uint(h[7]);
     }
     const float gs = grad_scale ? *grad_scale : 1.f;
     for (long long chunk = bx; chunk < n_chunks; chunk += gridDim.x) {
-        int lo = 0, hi = n_tensors - 1;          // last tensor whose first chunk is not behind this one
+        int lo = zero, hi = n_tensors - 1;          // last tensor whose first chunk is not behind this one
         while (lo < hi) {
             const int mid = (lo + hi + 1) / 2;
             if (tensors[mid].first_chunk <= chunk) lo = mid; else hi = mid - 1;
@@ -267,12 +273,12 @@ __global__ void __launch_bounds__(512, BLOCKS) norm_squared_kernel(float* __rest
 // that a block waits at one pair of barriers per 16 tensors instead of two barriers per tensor.
 template <typename T>
 __global__ void __launch_bounds__(512) norm_squared_multi_kernel(float* __restrict__ out, const AdamTensor* __restrict__ tensors, int n_tensors) {
-    grid_wait(tensors);
-    const int bx = after_wait(blockIdx.x), tx = after_wait(threadIdx.x);
+    grid_wait();
+    const int bx = after_wait(blockIdx.x), tx = after_wait(threadIdx.x), zero = after_wait(0u);
     __shared__ float warp_sums[16][16], sums[16];
     const int warp = tx >> 5, lane = tx & 31;
     float total = tx == 0 ? out[bx] : 0.f;
-    for (int t0 = 0; t0 < n_tensors; t0 += 16) {
+    for (int t0 = zero; t0 < n_tensors; t0 += 16) {
         const int n = min(16, n_tensors - t0);
         for (int t = 0; t < n; ++t) {
             const float s = warp_reduce_sum(thread_sum_squares<T, 4, true>(static_cast<const T*>(tensors[t0 + t].grad), tensors[t0 + t].n));
@@ -420,7 +426,7 @@ extern "C" int llmq_adamw_multi(const void* tensors, int n_tensors, long long n_
     if (n_tensors <= 0 || n_chunks <= 0) return 0;
     const float bc1 = 1.f / (1.f - powf(beta1, static_cast<float>(step)));
     const float bc2 = 1.f / (1.f - powf(beta2, static_cast<float>(step)));
-    const int g = static_cast<int>(n_chunks < 8LL * num_sms ? n_chunks : 8LL * num_sms);
+    const int g = static_cast<int>(n_chunks < (1ll << 30) ? n_chunks : (1ll << 30));
     const AdamTensor* t = static_cast<const AdamTensor*>(tensors);
 #define A_CASE(P, PC, G, GC, M, MC, V, VC)                                                                          \
     if (p_dtype == PC && g_dtype == GC && m_dtype == MC && v_dtype == VC) {                                         \

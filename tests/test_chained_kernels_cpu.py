@@ -61,6 +61,9 @@ def early_loads(sources):
         after = re.sub(r"after_wait\([^()]*\)", "", body[wait.end():])
         if "__ldg(" in after:
             problems.append(f"{kernel}: __ldg")
+        for p in read_only:                                   # p[0], *p: an address that is known before the wait
+            if re.search(rf"\b{p}\[\d+\]|[?=(,]\s*\*{p}\b", after):
+                problems.append(f"{kernel}: {p} is read at a constant address")
         if not read_only:
             continue
         if re.search(RAW_INDEX, after):
@@ -68,7 +71,7 @@ def early_loads(sources):
         for call in re.finditer(r"\b(\w+)(?:<[\w\s,]*>)?\(", after):
             if call.group(1) in functions and re.search(RAW_INDEX, functions[call.group(1)][1]):
                 args = after[call.end():_closing(after, call.end() - 1) - 1]
-                for p in read_only & set(re.findall(r"\w+", args)):
+                for p in read_only & set(re.findall(r"(\w+)\s*(?:,|$)", args)):              # handed over as it is
                     problems.append(f"{kernel}: {p} goes to {call.group(1)}(), which has plain indices")
     return problems
 
@@ -91,7 +94,8 @@ def test_every_chained_launch_clears_its_status():
 
 @pytest.mark.parametrize("wait,load,found", [
     ("grid_wait();", "x[after_wait(threadIdx.x)]", False), ("grid_wait(x);", "x[threadIdx.x]", False), ("grid_wait(x);", "sum(x)", False),
-    ("grid_wait();", "x[threadIdx.x]", True), ("grid_wait();", "sum(x)", True), ("", "x[after_wait(threadIdx.x)]", True)])
+    ("grid_wait();", "x[threadIdx.x]", True), ("grid_wait();", "x[0]", True), ("grid_wait(x);", "x[0]", False),
+    ("grid_wait();", "sum(x)", True), ("", "x[after_wait(threadIdx.x)]", True)])
 def test_early_loads_are_found(wait, load, found):
     s = ("__device__ __forceinline__ float sum(const float* __restrict__ x) { return x[threadIdx.x]; }\n"
          "__global__ void __launch_bounds__(512, 4) a_kernel(float* __restrict__ out, const float* __restrict__ x) { %s out[0] = %s; }\n"
