@@ -26,7 +26,6 @@ __global__ void __launch_bounds__(256)
 swiglu_fwd_kernel(T* __restrict__ out, e4m3* __restrict__ q_out, const T* __restrict__ inp, long long rows, int D,
                   float* __restrict__ absmax_out, const float* __restrict__ known_absmax, float* __restrict__ q_scale_out,
                   const FastDiv fd) {
-    grid_release();
     __shared__ float scratch[32];
     using V = Vec16<T>;
     const int vec_per_row = D / V::N;
@@ -114,7 +113,6 @@ template <typename T>
 __global__ void __launch_bounds__(256)
 swiglu_bwd_kernel(T* dinp, const T* __restrict__ dout, const T* inp, long long rows, int D, float* __restrict__ absmax_out,
                   const FastDiv fd) {
-    grid_release();
     __shared__ float scratch[32];
     using V = Vec16<T>;
     const int vec_per_row = D / V::N;

@@ -162,6 +162,7 @@ attn_fwd_pingpong_kernel(const __grid_constant__ CUtensorMap tmap_qkv,     // qk
     __syncthreads();
     tc_fence_after_sync();
     const uint32_t tmem = *tmem_slot;
+    grid_release();
     grid_wait();
 
     if (warp == 8) {

@@ -117,6 +117,7 @@ struct AttnParams {
 template <int HS>
 __global__ void __launch_bounds__(256)
 attn_delta_kernel(float* __restrict__ delta, const bf16* __restrict__ o, const bf16* __restrict__ d_o, int B, int T, int Hq) {
+    grid_release();
     grid_wait();
     const int bx = after_wait(blockIdx.x), tx = after_wait(threadIdx.x);
     constexpr int LANES = HS / 8;                       // lanes per row
@@ -240,6 +241,7 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmap_kv128,   // qkv, b
     __syncthreads();
     tc_fence_after_sync();
     const uint32_t tmem = *tmem_slot;
+    grid_release();
     grid_wait();
     const uint32_t tdV = tmem + 4 * BQ, tdK = tdV + HS;
     const uint32_t tK = tdK + HS, tV = tK + HS / 2;           // HS = 64
@@ -591,6 +593,7 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmap_qkv64,   // qkv, box
     __syncthreads();
     tc_fence_after_sync();
     const uint32_t tmem = *tmem_slot;
+    grid_release();
     grid_wait();
     const uint32_t tQ = tmem, tdO = tmem + HS / 2, tdQ = tmem + HS + 4 * BKV;
     auto tS = [&](int t) { return tmem + HS + (t & 1) * BKV; };

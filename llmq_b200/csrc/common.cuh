@@ -15,27 +15,29 @@ typedef __nv_fp8_e5m2 e5m2;
 #define LLMQ_LAUNCH_CHECK() static_cast<int>(cudaGetLastError())
 
 // ------------------------------------------------------------------------------------------------
-// Programmatic dependent launch.  A kernel launched with launch_chained() may start while the kernel before it on the stream still
-// runs: launch overhead, block scheduling and whatever it does before grid_wait() (barriers, tensor memory) then overlap with that
-// kernel's tail.  It must not touch global memory before grid_wait(), which returns when the kernel before it is complete and its
-// writes are visible; as that one has waited for its own predecessor, the order of the whole stream holds.  grid_release() lets the next
-// kernel start once every block of this one has called it (or has left); a kernel that waits for other GPUs must not call it.  Both
-// are no-ops in a kernel that was launched the ordinary way or has no such successor.
+// Programmatic dependent launch.  A kernel launched with launch_chained() is set up while the kernel before it on the stream still runs, and may
+// start then: launch overhead, block scheduling and whatever it does before grid_wait() (barriers, tensor memory) overlap with that
+// kernel.  It must not touch global memory before grid_wait(), which returns when the kernel before it is complete and its
+// writes are visible; as that one has waited for its own predecessor, the order of the whole stream holds.  In a kernel that was launched the
+// ordinary way the wait is a no-op.
+// Without more the next kernel starts when every block of this one has left.  grid_release() lets it start once every block has called it, which
+// pays for kernels that keep an SM to themselves and have a long way to their first load: GEMM and attention (GEMMs that leave many SMs idle for
+// long do not, see gemm_tcgen05.cu).  Elsewhere blocks of the next kernel, put beside running ones, end up several on one SM with another
+// SM idle, and for grids of many small blocks the call itself costs time.  us with / without the release, launched behind themselves in a graph:
+// AdamW tables of 2.4 M elements 21.5 / 9.6, gradient norm, clipping and that AdamW 36.4 / 21.4, bias gradient 7308 x 1000 8.2 / 6.4, RoPE of 60 tokens 2.1 / 1.7,
+// RMSNorm forward 8165 x 512 9.2 / 6.1.  A kernel that waits for other GPUs must not call it.
 // Launched this way: attention, RoPE, GEMM, their small second passes, the embedding, the norm and the AdamW launches of an update.  A pass over
-// rope, attention forward, backward (three kernels) and rope: 333 tokens, 12 / 2 heads of 128 53 -> 43 us, 8 x 1024 tokens, 14 / 2 heads of 64 187 -> 172;
-// gradient norm and AdamW of 67.9 M elements 203 -> 196.  The long streaming kernels (SwiGLU, RMSNorm, quantise, transposes, classifier) are not:
-// what the compiler loses by the two functions below costs them more than a launch (RMSNorm pass 186 -> 195 us, SwiGLU 793 -> 811); SwiGLU
-// and RMSNorm still release their successor.
+// rope, attention forward, backward (three kernels) and rope, launched plainly / this way: 333 tokens, 12 / 2 heads of 128 in a graph 66 / 39, 8 x 1024
+// tokens, 14 / 2 heads of 64 221 / 175.  The long streaming kernels (SwiGLU, RMSNorm, quantise, transposes, classifier) are not:
+// what the compiler loses by the two functions below costs them more than a launch (RMSNorm pass 186 -> 195 us, SwiGLU 793 -> 811).
 __device__ __forceinline__ void grid_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-__device__ __forceinline__ void grid_wait_only() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 // Loads through const __restrict__ pointers (and __ldg, __ldcs) count as loads of memory that nothing writes while the kernel runs: the compiler
 // may move them in front of the wait.  It cannot when their address comes out of it, so everything that is loaded is either found through a
-// block or thread index that went through after_wait(), or through one of `pointers`.  (All pointers that way would also lose their
-// __restrict__, and the kernels the freedom to load ahead of their stores: AdamW 204 -> 218 us.)
+// block or thread index (or a zero) that went through after_wait(), or through one of `pointers`.  (All pointers that way would also lose their
+// __restrict__, and the kernels the freedom to load ahead of their stores or to load again instead of keeping a register: AdamW 204 -> 218 us.)
 template <typename... P>
 __device__ __forceinline__ void grid_wait(P&... pointers) {
-    grid_release();
-    grid_wait_only();
+    asm volatile("griddepcontrol.wait;" ::: "memory");
     ((void)([&] { asm volatile("" : "+l"(pointers)); }()), ...);
 }
 __device__ __forceinline__ int after_wait(unsigned int index) {

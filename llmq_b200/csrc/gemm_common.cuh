@@ -63,6 +63,8 @@ struct GemmParams {
     int a_box3, b_box3;
     // CTA-pair kernel: columns of a tile (a multiple of 32 up to 256) and the bytes of B that a CTA loads per stage
     int bn, b_stage_bytes;
+    // CTA-pair kernel: the next kernel may start while this one runs
+    int early_release;
     // CTA-pair kernel: tile rows (256 rows of A each) that are worked through together, column tile by column tile
     int group_rows;
     // 1: C is bf16 with rows of whole aligned 32-byte sectors and the epilogue moves them lane by lane (store_sector)

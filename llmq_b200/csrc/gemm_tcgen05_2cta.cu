@@ -104,9 +104,8 @@ gemm_tcgen05_2cta_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gri
     cluster_wait();
     tc_fence_after_sync();
     const uint32_t tmem_base = *tmem_slot;
-    // a kernel that waits for other GPUs keeps its successor off the SMs
-    if (!p.ready_flags && p.rs_world == 0) grid_release();
-    grid_wait_only();
+    if (p.early_release) grid_release();
+    grid_wait();
 
     if (warp == 0) {
         // ------------------------------------------------------------------ TMA producer (both CTAs)

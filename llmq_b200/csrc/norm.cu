@@ -21,7 +21,6 @@ rmsnorm_fwd_kernel(T* __restrict__ residual_out,      // may be null when not fu
                    const T* __restrict__ weight, float eps, int C,
                    float* __restrict__ absmax_out, const float* __restrict__ known_absmax,
                    float* __restrict__ q_scale_out) {
-    grid_release();
     __shared__ float scratch[32];
     using V = Vec16<T>;
     const long long row = blockIdx.x;
@@ -89,7 +88,6 @@ __global__ void __launch_bounds__(THREADS)
 rmsnorm_fwd_reg_kernel(T* __restrict__ residual_out, T* __restrict__ y_out, e4m3* __restrict__ q_out, float* __restrict__ rstd_out,
                        const T* __restrict__ in_a, const T* __restrict__ in_b, const T* __restrict__ weight, float eps, int C,
                        float* __restrict__ absmax_out, const float* __restrict__ known_absmax, float* __restrict__ q_scale_out) {
-    grid_release();
     __shared__ float scratch[8], scratch_max[THREADS / 32];
     using V = Vec16<T>;
     const long long row = blockIdx.x;
@@ -194,7 +192,6 @@ rmsnorm_bwd_kernel(T* __restrict__ dinp,               // in: upstream residual 
                    float* __restrict__ dw_partial,     // [gridDim.x, C]
                    const T* __restrict__ dout, const T* __restrict__ inp, const T* __restrict__ weight,
                    const float* __restrict__ rstd, int rows, int C, float* __restrict__ absmax_out) {
-    grid_release();
     __shared__ float scratch[32];
     using V = Vec16<T>;
     float dw[VPT][V::N];
@@ -276,7 +273,6 @@ template <typename T, int VPT, int STAGES>
 __global__ void __launch_bounds__(NORM_THREADS, VPT <= 2 ? 3 : 2)
 rmsnorm_bwd_reg_kernel(T* __restrict__ dinp, float* __restrict__ dw_partial, const T* __restrict__ dout, const T* __restrict__ inp,
                        const T* __restrict__ weight, const float* __restrict__ rstd, int rows, int C, float* __restrict__ absmax_out) {
-    grid_release();
     __shared__ float scratch[32];
     __shared__ float dots[2][NORM_THREADS / 32];             // alternating, so that one barrier per row is enough
     extern __shared__ uint4 ring[];                          // [STAGES][3][VPT][NORM_THREADS]
