@@ -454,7 +454,7 @@ int launch(void* out, float* lse, const void* qkv, int B, int T, int Hq, int Hkv
                         CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                         CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS) return 1000 + static_cast<int>(r);
-    constexpr int smem = (2 + 2 * KV_STAGES) * (HS / 64) * CHUNK_BYTES + 256;
+    constexpr int smem = one_block_per_sm((2 + 2 * KV_STAGES) * (HS / 64) * CHUNK_BYTES + 256);
     static bool attr_done[64] = {};
     int dev = 0;
     cudaGetDevice(&dev);

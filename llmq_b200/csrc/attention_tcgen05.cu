@@ -916,7 +916,7 @@ int bwd_impl(void* dqkv, float* delta, const void* d_out, const void* out, const
     p.qkv = static_cast<const bf16*>(qkv);
     const int base = ((T + 127) / 128) * Hkv * B, G = Hq / Hkv;
     {
-        constexpr int smem = DkdvShape<HS>::SMEM_BYTES;
+        constexpr int smem = one_block_per_sm(DkdvShape<HS>::SMEM_BYTES);
         rc = set_smem<1000 + HS>(attn_bwd_dkdv_kernel<HS>, smem);
         if (rc) return rc;
         const int parts = HS == 128 ? head_parts(G, base) : 1;
@@ -925,7 +925,7 @@ int bwd_impl(void* dqkv, float* delta, const void* d_out, const void* out, const
         if (rc) return rc;
     }
     {
-        constexpr int smem = DqShape<HS>::SMEM_BYTES;
+        constexpr int smem = one_block_per_sm(DqShape<HS>::SMEM_BYTES);
         rc = set_smem<2000 + HS>(attn_bwd_dq_kernel<HS>, smem);
         if (rc) return rc;
         const int heads = heads_per_cta(G, base);

@@ -108,6 +108,10 @@ __device__ __forceinline__ bool mbar_test_wait(uint32_t bar, uint32_t parity) {
     return ok != 0;
 }
 
+// Dynamic shared memory of a kernel that allocates all of tensor memory: at least so much that no second block fits on an SM.  A block that is
+// launched while the kernel before it runs is put where there is room; two on one SM would run one after the other, with another SM idle.
+constexpr int one_block_per_sm(int bytes) { return bytes > 116 * 1024 ? bytes : 116 * 1024; }
+
 // Limit for every device-side wait, in nanoseconds of the global timer.
 constexpr uint64_t kWaitLimitNs = 2000ull * 1000ull * 1000ull;
 
