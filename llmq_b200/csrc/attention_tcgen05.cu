@@ -32,7 +32,7 @@
 //   1 x 8192, 32 / 8 heads of 128          880 -> 752   708 -> 620
 //   8 x 1024, 14 / 2 heads of 64            87 -> 68     56 -> 42
 //   2 x 4096, 32 / 8 heads of 64           368 -> 285   300 -> 221
-//   1 x 333, 12 / 2 heads of 128            37 -> 30     10 -> 9
+//   1 x 333, 12 / 2 heads of 128            37 -> 30     10 -> 9      (one CTA per item; with the cluster of head_parts dK / dV takes 14)
 // Not better: score tiles of 128 columns without a second buffer; with head size 64 P^T in columns of its own and S issued before the sums
 // of the tile two before (dK / dV 68 -> 77: the groups then meet at the exponentials).
 #include <cstdlib>
@@ -879,19 +879,53 @@ int heads_per_cta(int G, int base) {
     }
     return heads;
 }
+// Clusters of `parts` CTAs (plain CTAs for one) of the dK / dV kernel that reside at once
+template <int HS>
+int resident_clusters(int parts, int smem) {
+    static int known[64][9] = {};
+    int dev = 0;
+    cudaGetDevice(&dev);
+    int& n = known[dev & 63][parts];
+    if (n > 0) return n;
+    int found = device_sms();
+    if (parts > 1) {
+        cudaLaunchConfig_t cfg{};
+        cfg.gridDim = device_sms() * parts; cfg.blockDim = kBwdThreads; cfg.dynamicSmemBytes = smem;
+        cudaLaunchAttribute attr[1]{};
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = parts; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+        cfg.attrs = attr; cfg.numAttrs = 1;
+        if (cudaOccupancyMaxActiveClusters(&found, attn_bwd_dkdv_kernel<HS>, &cfg) != cudaSuccess) { cudaGetLastError(); return 0; }
+    }
+    return n = found;
+}
+
 
 // CTAs of one cluster that share the query heads of a dK / dV item (key block, kv head, batch), head size 128.  An item alone walks all
-// heads of the group, so few items leave SMs idle and the longest walk sets the time: the cluster is as large as two CTAs per SM allow.
-// Its CTAs add their sums up through distributed shared memory, in the order of the heads.  Kernel times in us, one CTA per item (of the kernel
-// before its issue was split, 1.15 times as long) /
-// now:  1 x 333 tokens, 12 / 2 heads (6 items, 6 parts) 37 / 14;  1 x 2048, 12 / 2 (32, 6) 164 / 43;  2 x 2048, 12 / 2 (64, 4) 167 / 79;
-// 2 x 2048, 28 / 4 (128, 2) 200 / 112;  1 x 2048, 32 / 8 (128, 2) 119 / 65;  3 x 2048, 28 / 4 (192, 1) 206 / 178.
+// heads of the group, so few items leave SMs idle and the longest walk sets the time.  A cluster's CTAs add their sums up through
+// distributed shared memory, in the order of the heads, which costs a short walk more than it saves; and clusters do not fill the SMs (of
+// 7 CTAs 15 reside, of 2 74), so one more round of them costs more than the shorter walks bring.  The part count is the one with the smallest
+// estimate, in us: 5 for every round of resident CTAs, 2 + 0.6 per part for its sums, and 0.9 for every tile of the longest walk or, if that is
+// longer, of the average walk of all rounds.  Over 12 lengths of 16 to 4096 tokens, groups of 2 to 12 heads and 4 to 144 items the picked count takes 1.005
+// of the time of the best one on average; as many parts as give two CTAs per SM took 1.18 and one CTA 1.22.  attention_backward, us, one CTA /
+// two CTAs per SM / this rule:  9 x 16 tokens, 28 / 4 heads (36 items) 23 / 42 / 23;  16 x 128, 28 / 4 (64) 43 / 50 / 40;  3 x 512, 64 / 8 (96) 154 / 128 /
+// 111 at 1024 tokens;  1 x 2048, 12 / 2 (32) 172 / 70 / 70;  2 x 2048, 28 / 4 (128) 262 / 201 / 201.
 // With head size 64 the sum over the heads stays in one accumulator: its results keep their bits.
-int head_parts(int G, int base) {
-    int parts = 2 * device_sms() / base;
-    if (parts > 8) parts = 8;
-    if (parts > G) parts = G;
-    return parts > 1 ? parts : 1;
+template <int HS>
+int head_parts(int G, int base, int T, int smem) {
+    const int nqb = (T + 63) / 64, nkb = (T + 127) / 128;
+    const double mean_tiles = nqb - (nkb - 1);               // query blocks at or below the diagonal, mean over the key blocks
+    int best = 1;
+    double best_us = 0.;
+    for (int parts = 1; parts <= 8 && parts <= G; ++parts) {
+        const int resident = resident_clusters<HS>(parts, smem), heads = (G + parts - 1) / parts;
+        if (resident <= 0) continue;
+        const double rounds = (base + resident - 1) / resident, longest = static_cast<double>(nqb) * heads;
+        const double average = mean_tiles * heads * base / resident;
+        const double us = rounds * (5. + (parts > 1 ? 2. + 0.6 * parts : 0.)) + 0.9 * (longest > average ? longest : average);
+        if (parts == 1 || us < best_us) { best = parts; best_us = us; }
+    }
+    return best;
 }
 
 template <int HS>
@@ -919,7 +953,7 @@ int bwd_impl(void* dqkv, float* delta, const void* d_out, const void* out, const
         constexpr int smem = one_block_per_sm(DkdvShape<HS>::SMEM_BYTES);
         rc = set_smem<1000 + HS>(attn_bwd_dkdv_kernel<HS>, smem);
         if (rc) return rc;
-        const int parts = HS == 128 ? head_parts(G, base) : 1;
+        const int parts = HS == 128 ? head_parts<HS>(G, base, T, smem) : 1;
         launch_chained_cluster(attn_bwd_dkdv_kernel<HS>, base * parts, kBwdThreads, smem, s, parts, t128, t64, tdo64, p, parts);
         rc = LLMQ_LAUNCH_CHECK();
         if (rc) return rc;
@@ -948,6 +982,14 @@ extern "C" int llmq_attention_forward(void* out, float* lse, const void* qkv, in
     if (Hq % Hkv) return -1;
     if (HS == 64 || HS == 128) return llmq_attention_forward_pingpong(out, lse, qkv, B, T, Hq, Hkv, HS, absmax, status, s);
     return -2;
+}
+
+// CTAs that share the query heads of a dK / dV item in llmq_attention_backward of this shape; negative: an error of the runtime
+extern "C" int llmq_attention_dkdv_parts(int B, int T, int Hq, int Hkv, int HS) {
+    if (HS != 128) return 1;
+    constexpr int smem = one_block_per_sm(DkdvShape<128>::SMEM_BYTES);
+    const int rc = set_smem<1000 + 128>(attn_bwd_dkdv_kernel<128>, smem);
+    return rc ? -rc : head_parts<128>(Hq / Hkv, ((T + 127) / 128) * Hkv * B, T, smem);
 }
 
 // dqkv (B,T,Hq+2Hkv,HS) is fully overwritten.  delta is scratch of B*Hq*T floats.

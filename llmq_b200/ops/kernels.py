@@ -956,7 +956,10 @@ def _attention_ref(qkv: torch.Tensor, Hq: int, Hkv: int):
 
 def attention_backward(dqkv: torch.Tensor, scratch: Optional[torch.Tensor], dout: torch.Tensor, out: torch.Tensor, lse: torch.Tensor,
                        qkv: torch.Tensor, Hq: int, Hkv: int) -> None:
-    """Packed gradient of :func:`attention_forward`; ``scratch`` holds B*Hq*T floats."""
+    """Packed gradient of :func:`attention_forward`; ``scratch`` holds B*Hq*T floats.
+
+    Deterministic: the same call gives the same bits.  With head size 128 several thread blocks share the query heads of a key block when there are
+    few of them, so the order in which dK and dV sum over the heads, and with it their last bits, depends on batch, length, head counts and GPU."""
     B, T, H, HS = qkv.shape
     if qkv.is_cuda and qkv.dtype == torch.float32:
         qh, oh, dh, gh = _attn_half(qkv), _attn_half(out), _attn_half(dout), _attn_half(dqkv)

@@ -74,6 +74,28 @@ def test_attention_backward_shared_heads(T, Hq, Hkv):
         assert (d <= want[:B].float().abs() * 2**-7 + 1e-4 * want.float().abs().max()).all()
 
 
+# the CTAs that share the heads of an item: short walks and many items alone, every size of a cluster; each against the same sequences in a batch
+# whose items are walked by one CTA
+@pytest.mark.parametrize("T,B,Hq,Hkv,parts", [(16, 9, 28, 4, 1), (64, 2, 40, 8, 1), (128, 16, 28, 4, 2), (70, 1, 6, 1, 3), (70, 1, 7, 1, 4), (70, 1, 9, 1, 5),
+                                              (200, 1, 6, 1, 6), (130, 1, 7, 1, 7), (130, 1, 8, 1, 8), (1000, 12, 8, 1, 2)])
+def test_attention_backward_parts_of_an_item(T, B, Hq, Hkv, parts):
+    lib, most = L.kernels(), 300 // ((T + 127) // 128 * Hkv)
+    assert torch.cuda.get_device_properties(0).multi_processor_count != 148 or lib.llmq_attention_dkdv_parts(B, T, Hq, Hkv, 128) == parts
+    assert lib.llmq_attention_dkdv_parts(most, T, Hq, Hkv, 128) == 1 and lib.llmq_attention_dkdv_parts(B, T, Hq, Hkv, 64) == 1
+    g = torch.Generator(device=DEV).manual_seed(T)
+    qkv = torch.randn(most, T, Hq + 2 * Hkv, 128, device=DEV, generator=g).to(BF)
+    dout = torch.randn(most, T, Hq, 128, device=DEV, generator=g).to(BF)
+    got = []
+    for n in (B, most):
+        out, lse, dqkv = torch.empty(n, T, Hq, 128, device=DEV, dtype=BF), torch.empty(n, Hq, T, device=DEV), torch.full_like(qkv[:n], 9.0)
+        K.attention_forward(out, lse, qkv[:n], Hq, Hkv)
+        K.attention_backward(dqkv, torch.empty(n * Hq * T, device=DEV), dout[:n], out, lse, qkv[:n], Hq, Hkv)
+        got.append(dqkv[:B].float())
+    # one CTA: the same bits; a cluster: fp32 sums in another order, then one rounding to bf16
+    d = (got[0] - got[1]).abs()
+    assert torch.equal(got[0], got[1]) if parts == 1 else (d <= got[1].abs() * 2**-7 + 1e-4 * got[1].abs().max()).all()
+
+
 # sequences of one query tile: a head per CTA and, with more heads than SMs, two heads of a group (the last one of an odd group alone)
 @pytest.mark.parametrize("HS", [64, 128])
 @pytest.mark.parametrize("T", [1, 33, 64, 65, 127, 128])
