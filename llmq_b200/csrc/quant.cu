@@ -250,10 +250,11 @@ extern "C" int llmq_quantize(void* out, float* scale_out, const void* x, const f
                              int out_dtype, int num_sms, cudaStream_t s) {
     if (n <= 0) return 0;
     // four blocks of 512 threads per SM, as many as reside: us with twice as many / with these, bf16 to e4m3: 4096 x 3584 7.6 / 6.9, 16384 x 3584 28.2 /
-    // 27.8, 16384 x 18944 155 / 151, 1000 x 3584 4.2 / 3.8
+    // 27.8, 16384 x 18944 155 / 151, 1000 x 3584 4.2 / 3.8.  fp32 to bf16 takes 40 registers, with which three reside: 27.8 M values 29.2 / 33.6 (40.0 with three
+    // per SM), 1.3 M 2.8 / 3.0.
 #define Q_CASE(T, TC, Q, QC, VN)                                                                                   \
     if (in_dtype == TC && out_dtype == QC) {                                                                       \
-        quantize_kernel<T, Q><<<grid_for(n / VN + 1, 512, (num_sms + 1) / 2), 512, 0, s>>>(static_cast<Q*>(out), scale_out,  \
+        quantize_kernel<T, Q><<<grid_for(n / VN + 1, 512, sizeof(T) == 4 && sizeof(Q) == 2 ? num_sms : (num_sms + 1) / 2), 512, 0, s>>>(static_cast<Q*>(out), scale_out,  \
                                                                                  static_cast<const T*>(x), absmax, n); \
         return LLMQ_LAUNCH_CHECK();                                                                                \
     }
