@@ -576,6 +576,12 @@ static int gemm_impl(const void* A, const void* B, void* C, const void* bias,
     }
 
     if (pair_kernel) {
+        // A kernel that waits for other GPUs keeps its successor off the SMs.  So does one that leaves a third of them idle for long: the CTA pairs of
+        // the next GEMM would be put onto just these, which is a worse choice of SMs than one among all.  Behind itself, us, with / without the release:
+        // 640 x 3584 x 18944 96.5 / 91.6, 773 x 3072 x 16384 90.1 / 86.4, 2048 x 1536 x 10752 61.0 / 58.3;  with fewer than 64 K steps, or more tiles, it is 2 to 5 %
+        // faster with it.
+        const bool idle_sms = 10 * tiles_of(M, N, 256, pair_bn) < 7 * (num_sms / 2) && K >= 64 * bk;
+        p.early_release = ready_flags == nullptr && p.rs_world == 0 && !idle_sms;
         // plain bf16 outputs leave the epilogue through TMA stores: a tensor map of C with 64-column x 32-row boxes
         CUtensorMap tc = ta;
         if (c_dtype == 0 && !accumulate && p.rs_world == 0 && p.ep_mode == 0 && (N % 8) == 0 && (ldc % 8) == 0 &&
@@ -583,12 +589,6 @@ static int gemm_impl(const void* A, const void* B, void* C, const void* bias,
             if (llmq_encode_tmap_2d(&tc, C, 2, M, N, ldc, 32) == 0) p.c_tma = 1;
         }
         return llmq_gemm_2cta_launch(ta, tb, tc, p, num_sms, stream);
-        // A kernel that waits for other GPUs keeps its successor off the SMs.  So does one that leaves a third of them idle for long: the CTA pairs of
-        // the next GEMM would be put onto just these, which is a worse choice of SMs than one among all.  Behind itself, us, with / without the release:
-        // 640 x 3584 x 18944 96.5 / 91.6, 773 x 3072 x 16384 90.1 / 86.4, 2048 x 1536 x 10752 61.0 / 58.3;  with fewer than 64 K steps, or more tiles, it is 2 to 5 %
-        // faster with it.
-        const bool idle_sms = 10 * tiles_of(M, N, 256, pair_bn) < 7 * (num_sms / 2) && K >= 64 * bk;
-        p.early_release = ready_flags == nullptr && p.rs_world == 0 && !idle_sms;
     }
 
     static bool attr_set[64] = {};          // the attribute is per device
