@@ -360,9 +360,14 @@ static int g_gemm_mode = 0;
 static int g_gemm_tma_store = 1;
 extern "C" void llmq_gemm_set_tma_store(int on) { g_gemm_tma_store = on; }
 extern "C" void llmq_gemm_set_mode(int mode) { g_gemm_mode = mode; }
-// Columns of a tile of the CTA-pair kernel: 0 = automatic, 224 or 256 = forced where the operands allow it (tests, measurements).
+// Columns of a tile of the CTA-pair kernel: 0 = automatic, 224 or 256 = forced where the operands allow it (tests, measurements).  Other widths are
+// refused (-1): the number goes into the MMA's descriptor and the byte counts of its barriers.
 static int g_gemm_pair_bn = 0;
-extern "C" void llmq_gemm_set_pair_bn(int bn) { g_gemm_pair_bn = bn; }
+extern "C" int llmq_gemm_set_pair_bn(int bn) {
+    if (bn != 0 && bn != 224 && bn != 256) return -1;
+    g_gemm_pair_bn = bn;
+    return 0;
+}
 
 static long long waves(long long tiles, int at_once) { return (tiles + at_once - 1) / at_once; }
 static long long tiles_of(int M, int N, int bm, int bn) { return static_cast<long long>((M + bm - 1) / bm) * ((N + bn - 1) / bn); }

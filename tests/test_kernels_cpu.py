@@ -97,3 +97,12 @@ def test_optimizer_table_refuses_rows_that_its_kernel_cannot_take(change, messag
            "m_scales": torch.ones(2), "absmax": torch.zeros(1), "elem_offset": 0, "seed": 0, "decay": True}
     with pytest.raises(ValueError, match=message):
         K.AdamTable([{**row, **change}], "cpu")
+
+
+def test_tile_width_of_the_pair_gemm_is_checked():
+    lib = L.kernels()
+    try:
+        assert [lib.llmq_gemm_set_pair_bn(n) for n in (224, 256, 0)] == [0, 0, 0]
+        assert [lib.llmq_gemm_set_pair_bn(n) for n in (-1, 1, 128, 225, 512)] == [-1] * 5
+    finally:
+        lib.llmq_gemm_set_pair_bn(0)
