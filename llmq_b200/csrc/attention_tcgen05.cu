@@ -867,10 +867,9 @@ int device_sms() {
 
 // Query heads of a group that one CTA of the dQ kernel walks over; `base` = (query block, kv head, batch) items.  A CTA that walks a
 // whole group pays its start-up once, but few items leave SMs idle: the group is cut into the fewest parts that give 1.5 CTAs per SM,
-// where the longest-first order evens the walks out.  Heads do not share sums, so the results do not depend on the cut.  Measured,
-// kernel times in us (parts 1 / 2 / 3 / 4 / 7): 8 x 1024 tokens, 14 / 2 heads of 64 (128 items) 81 / 56 / 57 / 59 / 70;  4 x 1024 (64
-// items) 81 / 48 / 37 / 31 / 38;  4 x 512 (32 items) 50 / 30 / 23 / 17 / 16;  8 x 2048, 28 / 4 heads of 128 (512 items) 398 / 390 / 407 /
-// 415 / 494 (before the rest of the kernel became faster; the order of the cuts is the same).
+// where the longest-first order evens the walks out.  Heads do not share sums, so the results do not depend on the cut.  attention_backward as a
+// whole, us (parts 1 / 2 / 3 / 4 / 7): 8 x 1024 tokens, 14 / 2 heads of 64 (128 items) 131 / 112 / 114 / 117 / 127;  4 x 1024 (64 items) 126 / 104 / 98 / 94 / 100;
+// 4 x 512 (32 items) 71 / 58 / 54 / 50 / 51;  2 x 2048, 28 / 4 heads of 128 (128 items) 264 / 204 / 203 / 212 / 216.
 int heads_per_cta(int G, int base) {
     int heads = G;
     for (int parts = 1; parts <= G; ++parts) {
@@ -879,6 +878,7 @@ int heads_per_cta(int G, int base) {
     }
     return heads;
 }
+
 // Clusters of `parts` CTAs (plain CTAs for one) of the dK / dV kernel that reside at once
 template <int HS>
 int resident_clusters(int parts, int smem) {
@@ -899,7 +899,6 @@ int resident_clusters(int parts, int smem) {
     }
     return n = found;
 }
-
 
 // CTAs of one cluster that share the query heads of a dK / dV item (key block, kv head, batch), head size 128.  An item alone walks all
 // heads of the group, so few items leave SMs idle and the longest walk sets the time.  A cluster's CTAs add their sums up through

@@ -386,11 +386,13 @@ static bool uses_pair_kernel(int M, int N, int elem_bytes, bool fused, int num_s
 }
 
 // Tile rows of 256 that the pair kernel works through together.  B is read from memory once per group, so a group is as large as its rows of A
-// stay in the L2 beside the B tiles that stream past: up to 40 MB, 4 to 32 tile rows.  Sustained, us with 4 / 8 / 16 / 32 tile rows (in brackets
-// the MB of A in 8):  16384 x 37888 x 3584 e4m3 (7) 1840 / 1790 / 1718 / 1687, 16384 x 18944 x 3584 e4m3 (7) 940 / 896 / 868 / 854,
+// stay in the L2 beside the B tiles that stream past: up to 40 MB, but at least 4 and at most 32 tile rows.  Sustained, us with 4 / 8 / 16 / 32 tile
+// rows (in brackets the MB of A in 8):  16384 x 37888 x 3584 e4m3 (7) 1840 / 1790 / 1718 / 1687, 16384 x 18944 x 3584 e4m3 (7) 940 / 896 / 868 / 854,
 // 4096 x 152064 x 3584 bf16 (15) 3444 / 3299 / 3229 / 3207, 4096 x 151936 x 896 bf16 (4) 984 / 946 / 918 / 918, 16384 x 3584 x 18944 e4m3 (39)
-// 919 / 912 / 914 / 985, 17920 x 1536 x 16384 bf16 (67) 689 / 719 / 727 / 767, 16384 x 1536 x 17920 bf16 (73) 744 / 748 / 756 / 799.
-// The order of the tiles is all that changes; kernels whose tiles arrive from or leave for other GPUs keep groups of 8.
+// 919 / 912 / 914 / 985.  With a longer K no group's rows of A stay, and 4, 8 and 16 take the same time within the spread of 2 % (9 interleaved runs each, medians):
+// 17920 x 1536 x 16384 bf16 (67) 719 / 719 / 719, 16384 x 3584 x 18944 bf16 (74) 1740 / 1748 / 1757, 4096 x 2048 x 128256 bf16 (501) 1818 / 1806 / 1779,
+// 4096 x 3584 x 152064 bf16 (594) 4109 / 4098 / 4081, 16384 x 8192 x 32768 e4m3 (64) 3679 / 3681 / 3687.
+// The order of the tiles is all that changes; kernels with a collective or a SwiGLU epilogue (`fused`) keep groups of 8.
 static int pair_group_rows(int K, int elem_bytes, bool fused) {
     if (fused) return 8;
     int rows = 32;
@@ -399,7 +401,7 @@ static int pair_group_rows(int K, int elem_bytes, bool fused) {
 }
 
 // Columns of a pair tile: 224 instead of 256 where that saves time, K-major B.  A round of 224-column tiles takes 0.93-0.95 of the time (the
-// loads of A are the same), so it has to need no more rounds; and not many more columns beyond N, which cost loads.  256 / 224 columns, us:
+// loads of A are the same), so it may need at most 3 % more rounds (none below 34), and 3 % more columns beyond N, which cost loads.  256 / 224 columns, us:
 // 4096 x 896 x 151936 863 / 797 (896 is 4 x 224), 151936 x 896 x 4096 850 / 792, 4096 x 896 x 4864 33.5 / 31.1, 2048 x 3072 x 3072 39.8 / 37.3 (two
 // rounds either way);  left at 256: 16384 x 3584 x 3584 275 / 278 (13 / 14 rounds), 4096 x 1152 x 896 15.5 / 16.1 (1280 / 1344 columns).
 // 192, 160 and 128 columns are slower still per column: a K step takes 0.85, 0.83, 0.79 of the time of one of 256.
