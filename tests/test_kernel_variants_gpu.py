@@ -687,3 +687,59 @@ def test_norm_right_behind_the_kernel_that_writes_its_tensor(dtype, M, N):
                 lambda: K.norm_squared(parts2, p), lambda: K.deterministic_sum(io[2:3], parts2)], (dw, p, m, v, parts, parts2, io)
 
     _same_with_and_without_waits(chain)
+
+
+def test_second_passes_and_tables_see_what_the_kernel_before_wrote():
+    """The other kernels that start while their predecessor runs, each right behind the one that writes its rows or its scale: split-K and its sum, the
+    bias and norm weight sums, the embedding and its gradient, the loss statistics, the update of a table."""
+    g = torch.Generator(device=DEV).manual_seed(11)
+    r = lambda *s, std=1.0: (torch.randn(*s, device=DEV, generator=g) * std).to(BF)
+    B, T, C, V = 4, 512, 256, 300
+    tok = torch.randint(0, V, (B * T,), device=DEV, generator=g, dtype=torch.int32)
+    wte0, w0, wn0, b0 = r(V, C), r(C, C, std=0.06), r(C), r(C, std=0.1)
+
+    def chain():
+        p = [t.clone() for t in (wte0, w0, wn0)]
+        d = [torch.zeros_like(t) for t in p]
+        m, v = [torch.zeros_like(t) for t in p], [torch.zeros_like(t) for t in p]
+        wte, w, wn = p
+        x, h, dx = (torch.zeros(B * T, C, device=DEV, dtype=BF) for _ in range(3))
+        f32, rstd, db = torch.zeros(B, T, device=DEV), torch.zeros(B * T, device=DEV), b0.clone()
+        st, gl, parts, io = torch.zeros(2, device=DEV), torch.zeros(T // 64, device=DEV), torch.zeros(512, device=DEV), torch.ones(2, device=DEV)
+        s1, s2 = torch.zeros(64 * C, device=DEV), torch.zeros(K.rmsnorm_backward_scratch_elems(C, torch.device(DEV, 0)), device=DEV)
+        table = K.AdamTable([dict(param=a.view(-1), grad=b.view(-1), m=c.view(-1), v=e.view(-1), elem_offset=0, seed=i, decay=True)
+                             for i, (a, b, c, e) in enumerate(zip(p, d, m, v))], DEV)
+        hyper = dict(lr=1e-2, beta1=0.9, beta2=0.95, eps=1e-8, weight_decay=0.1, seed=7)
+        launches = []
+        for step in range(3):
+            launches += [lambda: parts.zero_(), lambda: K.encoder_forward(x, tok, wte), lambda: K.gemm(h, x, w, bias=db),
+                         lambda: K.bias_backward(db, h, s1, scale_a=io[1:2], accumulate=False),
+                         lambda: K.gemm(d[1], h, x, a_mn=True, b_mn=True),                  # cut into parts of K = 2048 tokens
+                         lambda: K.gemm(f32, x[:B], x[:T]), lambda: K.lse_stats(st, f32), lambda: K.gemm(f32, h[:B], x[:T]),
+                         lambda: K.grouped_loss_sum(gl, f32, 64),
+                         lambda: K.rmsnorm_forward(dx, rstd, h, wn, 1e-6), lambda: K.gemm(dx, h, w, b_mn=True, alpha=0.01),
+                         lambda: K.rmsnorm_backward(dx, d[2], s2, x, h, wn, rstd, accumulate_dweight=False), lambda: K.gemm(dx, h, w, b_mn=True, alpha=0.02),
+                         lambda: K.encoder_backward(d[0], dx, tok), lambda: K.norm_squared_multi(parts, table),
+                         lambda: K.deterministic_sum(io[0:1], parts), lambda: K.norm_finish(io, 1.0),
+                         lambda step=step: K.adamw_multi(table, grad_scale=io[1:2], step=step + 1, **hyper)]
+        return launches, (*p, *d, *m, *v, x, h, dx, f32, rstd, db, st, gl, parts, io)
+
+    assert L.kernels().llmq_gemm_splitk_floats(C, C, B * T, 2, K.num_sms(torch.device(DEV, 0))) > 0
+    _same_with_and_without_waits(chain)
+
+
+# the ring of the backward kernel turns: more rows per block than it has stages, one vector a thread (four stages) and three or four (two)
+@pytest.mark.parametrize("C", [896, 2048, 4104, 5120, 8192])
+@pytest.mark.parametrize("rows", [1001, 1777, 3000])
+def test_rmsnorm_backward_ring_turns(C, rows):
+    g = torch.Generator(device=DEV).manual_seed(C + rows)
+    x, w, dy, dres, dw0 = (torch.randn(*s, device=DEV, generator=g).to(BF) for s in ((rows, C), (C,), (rows, C), (rows, C), (C,)))
+    rs = torch.rsqrt(x.double().square().mean(-1, keepdim=True) + 1e-6)
+    dinp, dw, am = dres.clone(), dw0.clone(), torch.zeros(1, device=DEV)
+    scratch = torch.full((K.rmsnorm_backward_scratch_elems(C, torch.device(DEV, 0)),), math.nan, device=DEV)
+    K.rmsnorm_backward(dinp, dw, scratch, dy, x, w, rs[:, 0].float().contiguous(), absmax=am)
+    xh, wdy = x.double() * rs, w.double() * dy.double()
+    gx = dres.double() + (wdy - xh * (wdy * xh).mean(-1, keepdim=True)) * rs
+    # every element: one rounding to bf16 (2^-9 of it) and fp32 arithmetic on terms of a few units
+    assert ((dinp.double() - gx).abs() <= gx.abs() * 2**-8 + 1e-5 * (1 + wdy.abs() * rs)).all()
+    assert rel(dw, dw0.double() + (dy.double() * xh).sum(0)) < 2**-8 and am.item() == dinp.float().abs().max().item()
