@@ -5,20 +5,23 @@
 // packed gradient dqkv with the same layout.  It takes the place of the cuDNN SDPA graphs and the
 // scalar fallback kernel of the reference (src/kernels/cudnn_att.cpp:46-263, src/kernels/attention.cu).
 //
-// The forward kernel is in attention_fwd_pingpong.cu.  The two gradient kernels share one organisation.  A CTA owns a 128-row tile
+// The forward kernel is in attention_fwd_pingpong.cu.  The two kinds of gradient CTAs share one organisation.  A CTA owns a 128-row tile
 // (keys for dK / dV, queries for dQ) and walks over 64-column score tiles.  16 compute warps form two groups that take the tiles in
 // turn, two warps issue MMAs, the others load by TMA.  Everything is handed over through mbarriers (one arrival per warp); score tiles
 // are double buffered in tensor memory, the streamed operand (Q / dO for dK / dV, K / V for dQ) sits in a ring of shared-memory buffers.
 // P^T, dS^T and dS never leave tensor memory: the bf16 values take the place of the scores they were computed from and are the A
-// operands of the accumulating MMAs.  Q and dO of the dQ kernel, and with head size 64 K and V of the other one, are A operands in tensor
+// operands of the accumulating MMAs.  Q and dO of the dQ CTAs, and with head size 64 K and V of the others, are A operands in tensor
 // memory too.  The shared-memory tile of V / K / Q / dO doubles as an MN-major B operand, so no transposed copy is ever made.
 //
-// Backward is split into two deterministic kernels (no atomics):
+// Backward is made of two kinds of CTAs, both deterministic (no atomics):
 //   * dK/dV: one CTA per (batch, kv head, 128 keys) walks over all query heads of the group and all query blocks at or below the
-//     diagonal; dK and dV accumulate in TMEM across the whole walk.  With few items a cluster shares the heads (head_parts).
+//     diagonal; dK and dV accumulate in TMEM across the whole walk.  With few items a cluster shares the heads (split_heads).
 //   * dQ   : one CTA per (batch, kv head, 128 queries) and part of the group walks over its query heads and their key blocks; dQ
 //     accumulates in TMEM and is drained once per head.
-// A small pre-pass computes delta = rowsum(dO * O).  Blocks with the longest walks are scheduled first.
+// A small pre-pass computes delta = rowsum(dO * O).  Both kinds are launched as one grid: neither needs what the other writes, so the dQ CTAs
+// start on the SMs that the dK / dV CTAs leave idle, at the end of their longest walks or, with few items, from the start.  The CTAs with the longest walks
+// of each kind come first.  attention_backward in us, a launch for each kind / one:  8 x 1024 tokens, 14 / 2 heads of 64 112 / 80;  4 x 1024 94 / 73;  1 x 333, 12 / 2
+// heads of 128 21.9 / 15.1;  2 x 700, 24 / 8 of 128 54 / 38;  where each kind alone fills the SMs for many rounds, 8 x 2048, 28 / 4 of 128, 761 / 758.
 //
 // What bounds it: no unit is saturated except the tensor pipe of dK / dV with head size 128 (1300 cycles of MMAs in about 1400 per tile;
 // 48 cycles per N = 64 MMA with both operands in shared memory, 33 with A in tensor memory, 64 per N = 128), the rest is the chain of
@@ -26,13 +29,13 @@
 // while MMAs with both operands in shared memory run: those take nearly all of its bandwidth.  Hence two groups of compute warps, two
 // issuing warps, row statistics in few wide loads, and everything that comes from global memory (Q / dO and the statistics of the next
 // head or tile) fetched a tile or a head ahead by a warp of its own; the statistics that the producer used to wait for tile by tile alone
-// cost 10 to 20 % of dK / dV.  Kernel times in us, one group and one issuing warp -> now:
+// cost 10 to 20 % of dK / dV.  Times of the two kinds launched one after the other, us, one group and one issuing warp -> now:
 //                                          dK / dV         dQ
 //   8 x 2048 tokens, 28 / 4 heads of 128   425 -> 364   403 -> 331
 //   1 x 8192, 32 / 8 heads of 128          880 -> 752   708 -> 620
 //   8 x 1024, 14 / 2 heads of 64            87 -> 68     56 -> 42
 //   2 x 4096, 32 / 8 heads of 64           368 -> 285   300 -> 221
-//   1 x 333, 12 / 2 heads of 128            37 -> 30     10 -> 9      (one CTA per item; with the cluster of head_parts dK / dV takes 14)
+//   1 x 333, 12 / 2 heads of 128            37 -> 30     10 -> 9      (one CTA per item; with a cluster dK / dV takes 14)
 // Not better: score tiles of 128 columns without a second buffer; with head size 64 P^T in columns of its own and S issued before the sums
 // of the tile two before (dK / dV 68 -> 77: the groups then meet at the exponentials).
 #include <cstdlib>
@@ -50,9 +53,10 @@ constexpr int kBwdWarpgroups = 4;
 constexpr int kBwdComputeThreads = 128 * kBwdWarpgroups;
 constexpr int kBwdComputeWarps = kBwdComputeThreads / 32;
 constexpr int kBwdGroupWarps = kBwdComputeWarps / 2;              // two groups, alternating score tiles
-// + three helper warps: two MMA issuers and the TMA producer
-constexpr int kBwdThreads = kBwdComputeThreads + 96;
-constexpr int kBwdDqThreads = kBwdComputeThreads + 128;           // the dQ kernel has a second producer
+// + four helper warps: two MMA issuers and one (dK / dV) or two (dQ) TMA producers
+constexpr int kBwdThreads = kBwdComputeThreads + 128;
+// A block's code is used twice: barriers and tensor memory before the wait for the kernel before (nothing of global memory is touched), the walk after it
+enum { kBwdSetup, kBwdRun };
 // One arrival per warp (512 single arrivals on one shared-memory word would serialise): the lanes' earlier
 // writes and fences are ordered before lane 0's releasing arrive by the warp barrier.
 __device__ __forceinline__ void warp_arrive(uint32_t bar) {
@@ -182,12 +186,13 @@ struct DkdvShape {
     static constexpr int SMEM_BYTES = STAT_OFFSET + NBUF * 64 * 8 + 256;
 };
 
-template <int HS>
-__global__ void __launch_bounds__(kBwdThreads, 1)
-attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmap_kv128,   // qkv, box 128 rows (K and V tiles)
-                     const __grid_constant__ CUtensorMap tmap_q64,     // qkv, box 64 rows (Q tiles)
-                     const __grid_constant__ CUtensorMap tmap_do64,    // dO, box 64 rows
-                     const AttnParams p, const int parts) {            // CTAs of a cluster that share the query heads of an item
+template <int HS, int Phase>
+__device__ __forceinline__ void
+bwd_dkdv_block(const CUtensorMap& tmap_kv128,                          // qkv, box 128 rows (K and V tiles)
+               const CUtensorMap& tmap_q64,                            // qkv, box 64 rows (Q tiles)
+               const CUtensorMap& tmap_do64,                           // dO, box 64 rows
+               const AttnParams& p, const int parts,                   // CTAs of a cluster that share the query heads of an item
+               const int block) {
     using Shape = DkdvShape<HS>;
     constexpr int BKV = 128, BQ = 64, NCH = HS / 64, NBUF = Shape::NBUF;
     constexpr int KV_BYTES = Shape::KV_BYTES, Q_BYTES = Shape::Q_BYTES;
@@ -204,11 +209,10 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmap_kv128,   // qkv, b
     volatile uint32_t* abort_flag = tmem_slot + 1;
 
     const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);       // uniform, and known to be
-    const int role = warp - kBwdComputeWarps;                 // 0, 1: MMA issuers (one elected lane); 2: TMA loads and row statistics
+    const int role = warp - kBwdComputeWarps;                 // 0, 1: MMA issuers (one elected lane); 2: TMA loads and row statistics; 3: none
     const int wg = tid >> 7, r = tid & 127;                   // compute threads: warpgroup, TMEM lane
-    if (smem_u32(smem) & 1023u) { if (tid == 0) atomicOr(p.status, kErrOther); return; }
     // 1-D grid, key block slowest: the blocks with the longest walks (small kb) start first on every SM
-    const int item = blockIdx.x / parts, part = blockIdx.x % parts;
+    const int item = block / parts, part = block % parts;
     const int kb = item / (p.Hkv * p.B);
     const int kvh = (item % (p.Hkv * p.B)) % p.Hkv, b = (item % (p.Hkv * p.B)) / p.Hkv;
     const int G = p.Hq / p.Hkv;
@@ -228,21 +232,22 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmap_kv128,   // qkv, b
     auto ready_bar = [&](int which, int it) { return bar0 + 40 + 16 * which + 8 * (it & 1); };     // 0: P^T, 1: dS^T
     auto qdo_bar = [&](int buf) { return bar0 + 80 + 8 * buf; };
     auto qdo_free = [&](int buf) { return bar0 + 128 + 8 * buf; };
-    if (tid == 0) {
-        mbar_init(kv_bar, kTmemKV ? kBwdComputeWarps : 1); mbar_init(done_bar, 2);
-        for (int i = 0; i < NBUF; ++i) { mbar_init(qdo_bar(i), 2); mbar_init(qdo_free(i), 2); }
-        for (int w = 0; w < 2; ++w)
-            for (int i = 0; i < 2; ++i) { mbar_init(score_bar(w, i), 1); mbar_init(ready_bar(w, i), kBwdGroupWarps); }
-        *abort_flag = 0;
-        mbar_init_fence();
+    if constexpr (Phase == kBwdSetup) {
+        if (tid == 0) {
+            mbar_init(kv_bar, kTmemKV ? kBwdComputeWarps : 1); mbar_init(done_bar, 2);
+            for (int i = 0; i < NBUF; ++i) { mbar_init(qdo_bar(i), 2); mbar_init(qdo_free(i), 2); }
+            for (int w = 0; w < 2; ++w)
+                for (int i = 0; i < 2; ++i) { mbar_init(score_bar(w, i), 1); mbar_init(ready_bar(w, i), kBwdGroupWarps); }
+            *abort_flag = 0;
+            mbar_init_fence();
+        }
+        if (role == 0) { tmem_alloc(smem_u32(tmem_slot), TMEM_COLS); tmem_relinquish(); }
+        tc_fence_before_sync();
+        __syncthreads();
+        tc_fence_after_sync();
+        return;
     }
-    if (role == 0) { tmem_alloc(smem_u32(tmem_slot), TMEM_COLS); tmem_relinquish(); }
-    tc_fence_before_sync();
-    __syncthreads();
-    tc_fence_after_sync();
     const uint32_t tmem = *tmem_slot;
-    grid_release();
-    grid_wait();
     const uint32_t tdV = tmem + 4 * BQ, tdK = tdV + HS;
     const uint32_t tK = tdK + HS, tV = tK + HS / 2;           // HS = 64
     const uint32_t lane_off = static_cast<uint32_t>((warp & 3) * 32) << 16;
@@ -301,7 +306,7 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmap_kv128,   // qkv, b
             }
             warp_arrive(qdo_bar(buf));
         }
-    } else if (role >= 0) {
+    } else if (role == 0 || role == 1) {
         // ============================================================ MMA issuer warps
         // Warp 0 issues S^T = K Q^T and dV += P^T dO, warp 1 dP^T = V dO^T and dK += dS^T Q: the same sequence, on other operands.  P^T (dS^T)
         // of tile it lies in the buffer of S (dP) of tile it + 2; MMAs of one thread execute in issue order, so a buffer that a later MMA
@@ -358,7 +363,7 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmap_kv128,   // qkv, b
             }
             __syncwarp();
         }
-    } else {
+    } else if (role < 0) {
         // ============================================================ compute warps
         // Two groups of two warpgroups take turns: group g works on the tiles of parity g, warpgroup `half` of it on 32 of their columns.
         const float sl2 = p.scale * kLog2e;
@@ -530,11 +535,11 @@ struct DqShape {
     static constexpr int SMEM_BYTES = STAT_OFFSET + 128 * 8 + 256;
 };
 
-template <int HS>
-__global__ void __launch_bounds__(kBwdDqThreads, 1)
-attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmap_qkv64,   // qkv, box 64 rows (K, V and Q tiles)
-                   const __grid_constant__ CUtensorMap tmap_do64,    // dO, box 64 rows
-                   const AttnParams p, const int heads_per_cta) {
+template <int HS, int Phase>
+__device__ __forceinline__ void
+bwd_dq_block(const CUtensorMap& tmap_qkv64,                          // qkv, box 64 rows (K, V and Q tiles)
+             const CUtensorMap& tmap_do64,                           // dO, box 64 rows
+             const AttnParams& p, const int heads_per_cta, const int block) {
     constexpr int BQ = 128, BKV = 64, NCH = HS / 64, NBUF = DqShape<HS>::NBUF;
     constexpr int KV_BYTES = DqShape<HS>::KV_BYTES, Q_BYTES = DqShape<HS>::Q_BYTES;
     constexpr uint32_t TMEM_COLS = 512;                       // Q | dO (bf16 pairs, A operands) | S0 S1 | dP0 dP1 | dQ
@@ -552,13 +557,12 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmap_qkv64,   // qkv, box
     const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);       // uniform, and known to be
     const int role = warp - kBwdComputeWarps;                 // 0, 1: MMA issuers (one elected lane); 2: TMA loads of K / V, 3: of Q / dO and row statistics
     const int wg = tid >> 7, r = tid & 127;
-    if (smem_u32(smem) & 1023u) { if (tid == 0) atomicOr(p.status, kErrOther); return; }
     const int nqb = (p.T + BQ - 1) / BQ;
     const int G = p.Hq / p.Hkv;
     const int parts = (G + heads_per_cta - 1) / heads_per_cta;
     const int per_qb = p.Hkv * p.B * parts;
-    const int qb = nqb - 1 - blockIdx.x / per_qb;               // 1-D grid, longest key walks first
-    const int rest = blockIdx.x % per_qb;
+    const int qb = nqb - 1 - block / per_qb;                    // longest key walks first
+    const int rest = block % per_qb;
     const int kvh = rest % p.Hkv, b = (rest / p.Hkv) % p.B, part = rest / (p.Hkv * p.B);
     const int h0 = kvh * G + part * heads_per_cta;              // query heads [h0, h0 + nh)
     const int nh = min(heads_per_cta, G - part * heads_per_cta);
@@ -579,22 +583,23 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmap_qkv64,   // qkv, box
     auto kv_bar = [&](int buf) { return bar0 + 96 + 8 * buf; };
     auto kv_free = [&](int buf) { return bar0 + 144 + 8 * buf; };
     const uint32_t staged = bar0 + 192, stage_free = bar0 + 200;
-    if (tid == 0) {
-        mbar_init(q_ready, kBwdGroupWarps); mbar_init(do_ready, kBwdGroupWarps);
-        mbar_init(dq_drained, kBwdGroupWarps); mbar_init(dq_bar, 1);
-        mbar_init(staged, 2); mbar_init(stage_free, kBwdComputeWarps);
-        for (int i = 0; i < NBUF; ++i) { mbar_init(kv_bar(i), 1); mbar_init(kv_free(i), 1); }
-        for (int i = 0; i < 2; ++i) { mbar_init(s_bar(i), 1); mbar_init(dp_bar(i), 1); mbar_init(p_ready(i), kBwdGroupWarps); mbar_init(s_free(i), kBwdGroupWarps); }
-        *abort_flag = 0;
-        mbar_init_fence();
+    if constexpr (Phase == kBwdSetup) {
+        if (tid == 0) {
+            mbar_init(q_ready, kBwdGroupWarps); mbar_init(do_ready, kBwdGroupWarps);
+            mbar_init(dq_drained, kBwdGroupWarps); mbar_init(dq_bar, 1);
+            mbar_init(staged, 2); mbar_init(stage_free, kBwdComputeWarps);
+            for (int i = 0; i < NBUF; ++i) { mbar_init(kv_bar(i), 1); mbar_init(kv_free(i), 1); }
+            for (int i = 0; i < 2; ++i) { mbar_init(s_bar(i), 1); mbar_init(dp_bar(i), 1); mbar_init(p_ready(i), kBwdGroupWarps); mbar_init(s_free(i), kBwdGroupWarps); }
+            *abort_flag = 0;
+            mbar_init_fence();
+        }
+        if (role == 0) { tmem_alloc(smem_u32(tmem_slot), TMEM_COLS); tmem_relinquish(); }
+        tc_fence_before_sync();
+        __syncthreads();
+        tc_fence_after_sync();
+        return;
     }
-    if (role == 0) { tmem_alloc(smem_u32(tmem_slot), TMEM_COLS); tmem_relinquish(); }
-    tc_fence_before_sync();
-    __syncthreads();
-    tc_fence_after_sync();
     const uint32_t tmem = *tmem_slot;
-    grid_release();
-    grid_wait();
     const uint32_t tQ = tmem, tdO = tmem + HS / 2, tdQ = tmem + HS + 4 * BKV;
     auto tS = [&](int t) { return tmem + HS + (t & 1) * BKV; };
     auto tdP = [&](int t) { return tmem + HS + 2 * BKV + (t & 1) * BKV; };
@@ -843,6 +848,25 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmap_qkv64,   // qkv, box
     if (role == 0) tmem_dealloc(tmem, TMEM_COLS);
 }
 
+// Blocks [0, n_dkdv) are the dK / dV CTAs, clusters of `parts`; the n_dq blocks behind them are the dQ CTAs, the last cluster filled up with idle ones.
+template <int HS>
+__global__ void __launch_bounds__(kBwdThreads, 1)
+attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_kv128, const __grid_constant__ CUtensorMap tmap_qkv64,
+                const __grid_constant__ CUtensorMap tmap_do64, const AttnParams p, const int parts, const int n_dkdv, const int heads_per_cta,
+                const int n_dq) {
+    extern __shared__ __align__(1024) uint8_t smem[];
+    if (smem_u32(smem) & 1023u) { if (threadIdx.x == 0) atomicOr(p.status, kErrOther); return; }
+    const int block = static_cast<int>(blockIdx.x);
+    if (block >= n_dkdv + n_dq) return;
+    const bool dkdv = block < n_dkdv;
+    if (dkdv) bwd_dkdv_block<HS, kBwdSetup>(tmap_kv128, tmap_qkv64, tmap_do64, p, parts, block);
+    else      bwd_dq_block<HS, kBwdSetup>(tmap_qkv64, tmap_do64, p, heads_per_cta, block - n_dkdv);
+    grid_release();
+    grid_wait();
+    if (dkdv) bwd_dkdv_block<HS, kBwdRun>(tmap_kv128, tmap_qkv64, tmap_do64, p, parts, block);
+    else      bwd_dq_block<HS, kBwdRun>(tmap_qkv64, tmap_do64, p, heads_per_cta, block - n_dkdv);
+}
+
 // Tag makes the static flag unique per kernel instantiation (several kernels share one signature).
 template <int Tag, typename K>
 int set_smem(K kernel, int bytes) {
@@ -857,6 +881,11 @@ int set_smem(K kernel, int bytes) {
     return 0;
 }
 
+template <int HS>
+constexpr int bwd_smem() {
+    return one_block_per_sm(DkdvShape<HS>::SMEM_BYTES > DqShape<HS>::SMEM_BYTES ? DkdvShape<HS>::SMEM_BYTES : DqShape<HS>::SMEM_BYTES);
+}
+
 int device_sms() {
     static int sms[64] = {};
     int dev = 0;
@@ -865,12 +894,10 @@ int device_sms() {
     return sms[dev & 63] > 0 ? sms[dev & 63] : 148;
 }
 
-// Query heads of a group that one CTA of the dQ kernel walks over; `base` = (query block, kv head, batch) items.  A CTA that walks a
-// whole group pays its start-up once, but few items leave SMs idle: the group is cut into the fewest parts that give 1.5 CTAs per SM,
-// where the longest-first order evens the walks out.  Heads do not share sums, so the results do not depend on the cut.  attention_backward as a
-// whole, us (parts 1 / 2 / 3 / 4 / 7): 8 x 1024 tokens, 14 / 2 heads of 64 (128 items) 131 / 112 / 114 / 117 / 127;  4 x 1024 (64 items) 126 / 104 / 98 / 94 / 100;
-// 4 x 512 (32 items) 71 / 58 / 54 / 50 / 51;  2 x 2048, 28 / 4 heads of 128 (128 items) 264 / 204 / 203 / 212 / 216.
-int heads_per_cta(int G, int base) {
+// Query heads of a group that a dQ CTA walks over; `base` = (query block, kv head, batch) items.  A CTA that walks a whole group pays its
+// start-up once, but few items leave SMs idle: the group is cut into the fewest parts that give 1.5 CTAs per SM.  Heads do not share
+// sums, so the results do not depend on the cut.
+int dq_heads(int G, int base) {
     int heads = G;
     for (int parts = 1; parts <= G; ++parts) {
         heads = (G + parts - 1) / parts;
@@ -879,7 +906,7 @@ int heads_per_cta(int G, int base) {
     return heads;
 }
 
-// Clusters of `parts` CTAs (plain CTAs for one) of the dK / dV kernel that reside at once
+// Clusters of `parts` CTAs (plain CTAs for one) that reside at once
 template <int HS>
 int resident_clusters(int parts, int smem) {
     static int known[64][9] = {};
@@ -895,35 +922,61 @@ int resident_clusters(int parts, int smem) {
         attr[0].id = cudaLaunchAttributeClusterDimension;
         attr[0].val.clusterDim.x = parts; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
         cfg.attrs = attr; cfg.numAttrs = 1;
-        if (cudaOccupancyMaxActiveClusters(&found, attn_bwd_dkdv_kernel<HS>, &cfg) != cudaSuccess) { cudaGetLastError(); return 0; }
+        if (cudaOccupancyMaxActiveClusters(&found, attn_bwd_kernel<HS>, &cfg) != cudaSuccess) { cudaGetLastError(); return 0; }
     }
     return n = found;
 }
 
-// CTAs of one cluster that share the query heads of a dK / dV item (key block, kv head, batch), head size 128.  An item alone walks all
-// heads of the group, so few items leave SMs idle and the longest walk sets the time.  A cluster's CTAs add their sums up through
-// distributed shared memory, in the order of the heads, which costs a short walk more than it saves; and clusters do not fill the SMs (of
-// 7 CTAs 15 reside, of 2 74), so one more round of them costs more than the shorter walks bring.  The part count is the one with the smallest
-// estimate, in us: 5 for every round of resident CTAs, 2 + 0.6 per part for its sums, and 0.9 for every tile of the longest walk or, if that is
-// longer, of the average walk of all rounds.  Over 12 lengths of 16 to 4096 tokens, groups of 2 to 12 heads and 4 to 144 items the picked count takes 1.005
-// of the time of the best one on average; as many parts as give two CTAs per SM took 1.18 and one CTA 1.22.  attention_backward, us, one CTA /
-// two CTAs per SM / this rule:  9 x 16 tokens, 28 / 4 heads (36 items) 23 / 42 / 23;  16 x 128, 28 / 4 (64) 43 / 50 / 40;  3 x 512, 64 / 8 (96) 154 / 128 /
-// 111 at 1024 tokens;  1 x 2048, 12 / 2 (32) 172 / 70 / 70;  2 x 2048, 28 / 4 (128) 262 / 201 / 201.
-// With head size 64 the sum over the heads stays in one accumulator: its results keep their bits.
+// How the query heads of a group are shared out.  dkdv: CTAs of one cluster that share the heads of a dK / dV item (key block, kv head, batch); they
+// add their sums up through distributed shared memory, in the order of the heads.  dq: heads that a dQ CTA walks over.
+struct HeadSplit {
+    int dkdv, dq;
+};
+
+// With head size 64 the sum over the heads stays in one accumulator, so that its results keep their bits, and the dQ CTAs follow dq_heads (within 0.3 % of the best
+// cut over 20 shapes).  With head size 128 the pair is the one with the smallest estimate, in us: a dK / dV CTA costs 5, with a cluster 2 + 0.5
+// per part more for its sums, 0.25 a head and 0.85 a tile; a dQ CTA 4.2, 1.7 a head (Q and dO in, dQ out) and 0.6 a tile; all of them together take the longest CTA
+// or, if that is longer and they do not all reside at once, the average of the resident CTAs and half a CTA behind it (clusters do not fill the SMs:
+// of 7 CTAs 15 reside, of 2 74).  Over 55 shapes (20 to 6731 tokens, 1 to 8 sequences, groups of 1 to 12 heads) the picked pair
+// takes 1.03 of the time of the best one on average, the rules for two launches one after the other took 1.10.  attention_backward, us, with those / picked:
+// 1 x 1024 tokens, 32 / 8 heads 58 / 42;  6 x 405, 12 / 2 35 / 31;  2 x 683, 28 / 4 58 / 44;  3 x 2048, 28 / 4 312 / 284;  4 x 1024, 16 / 2 86 / 70.
+// For sequences of one key block, whose few tiles the estimate of a tile says little about, the older rule stays unless the estimate is 1.35 times better:
+// 8 x 100, 32 / 8 30 / 21, but 24 x 128, 28 / 4 49 by the older rule and 56 by the estimate.
 template <int HS>
-int head_parts(int G, int base, int T, int smem) {
+HeadSplit split_heads(int G, int base, int T, int smem) {
+    const int heads_rule = dq_heads(G, base);
+    if constexpr (HS == 64) return {1, heads_rule};
     const int nqb = (T + 63) / 64, nkb = (T + 127) / 128;
     const double mean_tiles = nqb - (nkb - 1);               // query blocks at or below the diagonal, mean over the key blocks
-    int best = 1;
-    double best_us = 0.;
+    HeadSplit best{1, heads_rule};
+    double best_us = 0., rule_us = 0., rule_best = 0.;       // rule_us: estimate of the older rule, which looks at dK / dV alone; rule_best: the pair estimate of its parts
+    int rule_parts = 1;
     for (int parts = 1; parts <= 8 && parts <= G; ++parts) {
         const int resident = resident_clusters<HS>(parts, smem), heads = (G + parts - 1) / parts;
         if (resident <= 0) continue;
-        const double rounds = (base + resident - 1) / resident, longest = static_cast<double>(nqb) * heads;
-        const double average = mean_tiles * heads * base / resident;
+        const double sums = parts > 1 ? 2. + 0.5 * parts : 0.;
+        double parts_us = 0.;
+        for (int dq = G, last = 0; dq >= 1; --dq) {
+            const int cut = (G + dq - 1) / dq;               // dQ CTAs of an item; the smallest `dq` of every cut is looked at
+            if (dq > 1 && (G + dq - 2) / (dq - 1) == cut) continue;
+            if (cut == last) continue;
+            last = cut;
+            const double longest_dkdv = 5. + sums + heads * (0.25 + 0.85 * nqb), longest_dq = 4.2 + dq * (1.7 + 0.6 * nqb);
+            double us = longest_dkdv > longest_dq ? longest_dkdv : longest_dq;
+            const double ctas = static_cast<double>(base) * (parts + cut), at_once = static_cast<double>(resident) * parts;
+            if (ctas > at_once) {
+                const double work = base * (parts * (5. + sums) + G * (0.25 + 0.85 * mean_tiles) + cut * 4.2 + G * (1.7 + 0.6 * (nkb + 1)));
+                const double mean = work / ctas, shared = work / at_once + 0.5 * (us < mean ? us : mean);
+                if (shared > us) us = shared;
+            }
+            if (best_us == 0. || us < best_us) { best = {parts, dq}; best_us = us; }
+            if (parts_us == 0. || us < parts_us) parts_us = us;
+        }
+        const double rounds = (base + resident - 1) / resident, longest = static_cast<double>(nqb) * heads, average = mean_tiles * heads * base / resident;
         const double us = rounds * (5. + (parts > 1 ? 2. + 0.6 * parts : 0.)) + 0.9 * (longest > average ? longest : average);
-        if (parts == 1 || us < best_us) { best = parts; best_us = us; }
+        if (rule_us == 0. || us < rule_us) { rule_us = us; rule_parts = parts; rule_best = parts_us; }
     }
+    if (nkb == 1 && rule_best <= 1.35 * best_us) return {rule_parts, heads_rule};
     return best;
 }
 
@@ -948,23 +1001,14 @@ int bwd_impl(void* dqkv, float* delta, const void* d_out, const void* out, const
     p.lse = const_cast<float*>(lse); p.delta = delta; p.dqkv = static_cast<bf16*>(dqkv); p.status = status;
     p.qkv = static_cast<const bf16*>(qkv);
     const int base = ((T + 127) / 128) * Hkv * B, G = Hq / Hkv;
-    {
-        constexpr int smem = one_block_per_sm(DkdvShape<HS>::SMEM_BYTES);
-        rc = set_smem<1000 + HS>(attn_bwd_dkdv_kernel<HS>, smem);
-        if (rc) return rc;
-        const int parts = HS == 128 ? head_parts<HS>(G, base, T, smem) : 1;
-        launch_chained_cluster(attn_bwd_dkdv_kernel<HS>, base * parts, kBwdThreads, smem, s, parts, t128, t64, tdo64, p, parts);
-        rc = LLMQ_LAUNCH_CHECK();
-        if (rc) return rc;
-    }
-    {
-        constexpr int smem = one_block_per_sm(DqShape<HS>::SMEM_BYTES);
-        rc = set_smem<2000 + HS>(attn_bwd_dq_kernel<HS>, smem);
-        if (rc) return rc;
-        const int heads = heads_per_cta(G, base);
-        launch_chained(attn_bwd_dq_kernel<HS>, base * ((G + heads - 1) / heads), kBwdDqThreads, smem, s, t64, tdo64, p, heads);
-        rc = LLMQ_LAUNCH_CHECK();
-    }
+    constexpr int smem = bwd_smem<HS>();
+    rc = set_smem<1000 + HS>(attn_bwd_kernel<HS>, smem);
+    if (rc) return rc;
+    const HeadSplit split = split_heads<HS>(G, base, T, smem);
+    const int parts = split.dkdv, n_dkdv = base * parts, n_dq = base * ((G + split.dq - 1) / split.dq);
+    launch_chained_cluster(attn_bwd_kernel<HS>, n_dkdv + (n_dq + parts - 1) / parts * parts, kBwdThreads, smem, s, parts, t128, t64, tdo64, p, parts,
+                           n_dkdv, split.dq, n_dq);
+    rc = LLMQ_LAUNCH_CHECK();
     return rc;
 }
 
@@ -986,9 +1030,9 @@ extern "C" int llmq_attention_forward(void* out, float* lse, const void* qkv, in
 // CTAs that share the query heads of a dK / dV item in llmq_attention_backward of this shape; negative: an error of the runtime
 extern "C" int llmq_attention_dkdv_parts(int B, int T, int Hq, int Hkv, int HS) {
     if (HS != 128) return 1;
-    constexpr int smem = one_block_per_sm(DkdvShape<128>::SMEM_BYTES);
-    const int rc = set_smem<1000 + 128>(attn_bwd_dkdv_kernel<128>, smem);
-    return rc ? -rc : head_parts<128>(Hq / Hkv, ((T + 127) / 128) * Hkv * B, T, smem);
+    constexpr int smem = bwd_smem<128>();
+    const int rc = set_smem<1000 + 128>(attn_bwd_kernel<128>, smem);
+    return rc ? -rc : split_heads<128>(Hq / Hkv, ((T + 127) / 128) * Hkv * B, T, smem).dkdv;
 }
 
 // dqkv (B,T,Hq+2Hkv,HS) is fully overwritten.  delta is scratch of B*Hq*T floats.

@@ -96,6 +96,31 @@ def test_attention_backward_parts_of_an_item(T, B, Hq, Hkv, parts):
     assert torch.equal(got[0], got[1]) if parts == 1 else (d <= got[1].abs() * 2**-7 + 1e-4 * got[1].abs().max()).all()
 
 
+# dK / dV and dQ CTAs in one grid: the last cluster filled up with blocks that have nothing to do (dQ CTAs that are no multiple of the cluster size),
+# one and two key blocks on both sides of the rule, groups that the dQ CTAs cut unevenly; each against the walk of a batch that has no clusters
+@pytest.mark.parametrize("HS", [64, 128])
+@pytest.mark.parametrize("B,T,Hq,Hkv", [(1, 70, 9, 1), (1, 128, 28, 4), (1, 129, 28, 4), (1, 333, 12, 2), (3, 257, 5, 1), (2, 683, 28, 4), (1, 1024, 32, 8), (9, 100, 32, 8)])
+def test_attention_backward_one_grid(HS, B, T, Hq, Hkv):
+    most = max(B, 300 // ((T + 127) // 128 * Hkv) + 1)
+    g = torch.Generator(device=DEV).manual_seed(T)
+    qkv = torch.randn(most, T, Hq + 2 * Hkv, HS, device=DEV, generator=g).to(BF)
+    dout = torch.randn(most, T, Hq, HS, device=DEV, generator=g).to(BF)
+    got = []
+    for n in (B, most):
+        out, lse, dqkv = torch.empty(n, T, Hq, HS, device=DEV, dtype=BF), torch.empty(n, Hq, T, device=DEV), torch.full_like(qkv[:n], 9.0)
+        K.attention_forward(out, lse, qkv[:n], Hq, Hkv)
+        K.attention_backward(dqkv, torch.empty(n * Hq * T, device=DEV), dout[:n], out, lse, qkv[:n], Hq, Hkv)
+        got.append(dqkv[:B].float())
+    assert torch.equal(got[0][:, :, :Hq], got[1][:, :, :Hq])             # dQ has one order
+    # head size 64: one order; 128: fp32 sums of a cluster in another order, then one rounding to bf16
+    d = (got[0] - got[1]).abs()
+    assert torch.equal(got[0], got[1]) if HS == 64 else (d <= got[1].abs() * 2**-7 + 1e-4 * got[1].abs().max()).all()
+    x = qkv[:B].float().requires_grad_(True)
+    o, _ = K._attention_ref(x, Hq, Hkv)
+    o.backward(dout[:B].float())
+    assert rel(got[0], x.grad) < 1.2e-2                                  # 16-bit probabilities and score gradients, 16-bit outputs
+
+
 # sequences of one query tile: a head per CTA and, with more heads than SMs, two heads of a group (the last one of an odd group alone)
 @pytest.mark.parametrize("HS", [64, 128])
 @pytest.mark.parametrize("T", [1, 33, 64, 65, 127, 128])
