@@ -51,8 +51,8 @@ struct GemmParams {
     void* ep_ptr;
     int ep_D;
     // Optional split-K (one-CTA kernel only): the K loop of every tile is cut into k_splits parts handled by different
-    // CTAs; each writes its raw fp32 accumulator to partial[split][M][N] and a second kernel sums the parts and applies
-    // the normal epilogue.  For outputs with fewer tiles than SMs and a long K (weight gradients of small models).
+    // CTAs.  They sum their raw fp32 accumulators through distributed shared memory, or each writes its own to
+    // partial[split][M][N] and a second kernel sums the parts; both apply the normal epilogue.  For outputs with fewer tiles than SMs and a long K (weight gradients of small models).
     int k_splits;
     float* partial;
     // CTA-pair kernel: 1 when the kernel's third tensor map describes C (bf16, plain store) and the epilogue may write

@@ -19,6 +19,7 @@
 //              128x256 (or 128x128) fp32 accumulators in TMEM, tcgen05.commit to free the stage
 //   warps 2-5  epilogue: tcgen05.ld the finished accumulator (while the other one is being
 //              computed), scale, add bias, optionally add the previous C, track abs-max, store
+// Outputs with few tiles and a long K cut the K loop; the parts of a tile are summed by the CTAs of a cluster or by a second kernel.
 #include "ptx_sm100.cuh"
 #include "api.h"
 #include "common.cuh"
@@ -54,8 +55,76 @@ __device__ __forceinline__ void tile_coords(int t, int tiles_m, int tiles_n, int
     tn = r / gsz;
 }
 
+__device__ __forceinline__ float4 ld_cluster_f32x4(uint32_t addr) {
+    float4 v;
+    asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr) : "memory");
+    return v;
+}
+
+// Split K, the parts of a tile in one cluster: every CTA has put its fp32 accumulator [128][BN] at the start of its shared memory (16-byte pieces, piece index ^
+// (row % 8)).  CTA `part` adds up rows [128 part / parts, ...) of all of them, in the order of the parts like the two-kernel form (same bits), and writes the
+// result.  What it saves is the latency of a second kernel and of parts x M x N floats through the L2; see the rule in gemm_impl.
+template <int BN>
+__device__ __forceinline__ void cluster_reduce(const GemmParams& p, uint32_t smem_base, int tm, int tn, int part, int parts, float alpha, float& tmax) {
+    constexpr int PIECES = BN / 4;
+    const int row0 = BM * part / parts, rows = BM * (part + 1) / parts - row0;
+    uint32_t base[8];
+#pragma unroll
+    for (int q = 0; q < 8; ++q) base[q] = map_to_cta(smem_base, q < parts ? q : 0);
+    // four pieces per thread at a time: all their loads, from the other CTAs and of the old values, are under way together
+    constexpr int U = 4;
+    for (int i0 = after_wait(threadIdx.x); i0 < rows * PIECES; i0 += U * NUM_THREADS) {
+        uint4 old[U];
+        float4 x[U][8];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const int i = i0 + u * NUM_THREADS, r = row0 + i / PIECES, piece = i % PIECES, row = tm * BM + r, col = tn * BN + piece * 4;
+            const bool inside = i < rows * PIECES && row < p.M && col < p.N;
+            if (p.accumulate && inside) {
+                if (p.c_dtype == 0) {
+                    const uint2 o = *reinterpret_cast<const uint2*>(static_cast<bf16*>(p.C) + row * p.ldc + col);
+                    old[u].x = o.x; old[u].y = o.y;            // as they are: what is computed from a load here would wait for it
+                } else {
+                    old[u] = *reinterpret_cast<const uint4*>(static_cast<float*>(p.C) + row * p.ldc + col);
+                }
+            }
+            const uint32_t at = r * (BN * 4) + ((piece ^ (r & 7)) << 4);
+#pragma unroll
+            for (int q = 0; q < 8; ++q) if (q < parts && inside) x[u][q] = ld_cluster_f32x4(base[q] + at);
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const int i = i0 + u * NUM_THREADS, r = row0 + i / PIECES, piece = i % PIECES, row = tm * BM + r, col = tn * BN + piece * 4;
+            if (i >= rows * PIECES || row >= p.M || col >= p.N) continue;
+            float v[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+            for (int q = 0; q < 8; ++q) if (q < parts) { v[0] += x[u][q].x; v[1] += x[u][q].y; v[2] += x[u][q].z; v[3] += x[u][q].w; }
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                v[k] *= alpha;
+                if (p.bias) v[k] += p.bias_dtype == 0 ? __bfloat162float(static_cast<const bf16*>(p.bias)[col + k]) : static_cast<const float*>(p.bias)[col + k];
+            }
+            if (p.accumulate && p.c_dtype == 0) {
+                v[0] += __uint_as_float(old[u].x << 16); v[1] += __uint_as_float(old[u].x & 0xffff0000u);
+                v[2] += __uint_as_float(old[u].y << 16); v[3] += __uint_as_float(old[u].y & 0xffff0000u);
+            } else if (p.accumulate) {
+                v[0] += __uint_as_float(old[u].x); v[1] += __uint_as_float(old[u].y); v[2] += __uint_as_float(old[u].z); v[3] += __uint_as_float(old[u].w);
+            }
+            if (p.c_dtype == 0) {
+                const __nv_bfloat162 lo = __floats2bfloat162_rn(v[0], v[1]), hi = __floats2bfloat162_rn(v[2], v[3]);
+                *reinterpret_cast<uint2*>(static_cast<bf16*>(p.C) + row * p.ldc + col) = make_uint2(*reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi));
+            } else {
+                *reinterpret_cast<float4*>(static_cast<float*>(p.C) + row * p.ldc + col) = make_float4(v[0], v[1], v[2], v[3]);
+            }
+#pragma unroll
+            for (int k = 0; k < 4; ++k) tmax = fmaxf(tmax, fabsf(v[k]));
+        }
+    }
+}
+
 // Kind: MMA kind of ptx_sm100.cuh's mma_issue (0 bf16, 1 8-bit floats, 2 tf32 on fp32 operands).
-template <int Kind, int BN>
+// Cluster: the CTAs of a cluster are the K parts of one tile (grid = tiles x parts, one work item per CTA).
+template <int Kind, int BN, bool Cluster>
 __global__ void __launch_bounds__(NUM_THREADS, 1)
 gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
                     const GemmParams p) {
@@ -206,16 +275,46 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
             if (!mbar_wait(tfull_bar(acc), acc_phase, abort_flag)) { if (lane == 0) atomicOr(p.status, kErrTmemFull); ok = false; break; }
             tc_fence_after_sync();
             const uint32_t t_row = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + acc * BN;
-            if (splits > 1) epilogue_rows_partial(p, t_row, tm * BM + q * 32 + lane, tn * BN, BN, t % splits);
+            if constexpr (Cluster) {
+                uint8_t* const mine = smem + (q * 32 + lane) * (BN * 4);
+#pragma unroll 1
+                for (int c = 0; c < BN; c += 32) {
+                    uint32_t r[32];
+                    tmem_ld_32x32b_x32(t_row + c, r);
+                    tmem_ld_wait();
+#pragma unroll
+                    for (int i = 0; i < 8; ++i)
+                        *reinterpret_cast<uint4*>(mine + (((c / 4 + i) ^ (lane & 7)) << 4)) = make_uint4(r[4 * i], r[4 * i + 1], r[4 * i + 2], r[4 * i + 3]);
+                }
+            }
+            else if (splits > 1) epilogue_rows_partial(p, t_row, tm * BM + q * 32 + lane, tn * BN, BN, t % splits);
             else            epilogue_rows(p, t_row, tm * BM + q * 32 + lane, tn * BN, BN, alpha, tmax);
             tc_fence_before_sync();
             mbar_arrive(tempty_bar(acc));                  // 128 arrivals release the accumulator
             if (++acc == 2) { acc = 0; acc_phase ^= 1u; }
         }
+        if (!Cluster && p.absmax_out) {
+            tmax = warp_reduce_max(tmax);
+            if (lane == 0 && tmax > 0.f) atomic_max_float(p.absmax_out, tmax);
+        }
+    }
+    if constexpr (Cluster) {
+        // Every CTA of a cluster gets here, also one that gave up on a wait (the status word says so and the output is void)
+        __syncwarp();
+        cluster_arrive();
+        cluster_wait();
+        float alpha = p.alpha, tmax = 0.f;
+        if (p.scale_a) alpha *= *p.scale_a;
+        if (p.scale_b) alpha *= *p.scale_b;
+        int tm, tn; tile_coords(after_wait(blockIdx.x) / splits, tiles_m, tiles_n, tm, tn);
+        cluster_reduce<BN>(p, smem_base, tm, tn, blockIdx.x % splits, splits, alpha, tmax);
         if (p.absmax_out) {
             tmax = warp_reduce_max(tmax);
             if (lane == 0 && tmax > 0.f) atomic_max_float(p.absmax_out, tmax);
         }
+        __syncwarp();
+        cluster_arrive();                                      // the others may still read this CTA's accumulator
+        cluster_wait();
     }
 
     tc_fence_before_sync();
@@ -298,6 +397,44 @@ __global__ void __launch_bounds__(256) splitk_reduce_vec_kernel(const GemmParams
         for (int k = 0; k < 4; ++k) tmax = fmaxf(tmax, fabsf(v[k]));
     }
     if (p.absmax_out) block_absmax_commit(p.absmax_out, tmax, scratch);
+}
+
+// Launches the one-CTA kernel for `items` (tile, K part) pairs: `cluster` = the parts of a tile in one cluster
+template <int Kind, int BN>
+int launch_one_cta(const CUtensorMap& ta, const CUtensorMap& tb, const GemmParams& p, int items, bool cluster, int num_sms, cudaStream_t stream) {
+    static bool attr_set[64] = {};          // the attribute is per device
+    constexpr int smem = Tile<BN>::SMEM_BYTES;
+    int dev = 0;
+    cudaGetDevice(&dev);
+    if (!attr_set[dev & 63]) {
+        cudaError_t e = cudaFuncSetAttribute(gemm_tcgen05_kernel<Kind, BN, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(gemm_tcgen05_kernel<Kind, BN, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+        if (e != cudaSuccess) return static_cast<int>(e);
+        attr_set[dev & 63] = true;
+    }
+    if (cluster) launch_chained_cluster(gemm_tcgen05_kernel<Kind, BN, true>, items, NUM_THREADS, smem, stream, p.k_splits, ta, tb, p);
+    else         launch_chained(gemm_tcgen05_kernel<Kind, BN, false>, items < num_sms ? items : num_sms, NUM_THREADS, smem, stream, ta, tb, p);
+    return LLMQ_LAUNCH_CHECK();
+}
+
+// Clusters of `parts` CTAs of the one-CTA kernel that reside at once (the same for all operand types: one CTA per SM)
+int resident_clusters(int parts) {
+    static int known[64][9] = {};
+    int dev = 0;
+    cudaGetDevice(&dev);
+    int& n = known[dev & 63][parts];
+    if (n > 0) return n;
+    constexpr int smem = Tile<256>::SMEM_BYTES;
+    if (cudaFuncSetAttribute(gemm_tcgen05_kernel<0, 256, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) { cudaGetLastError(); return 0; }
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = 64 * parts; cfg.blockDim = NUM_THREADS; cfg.dynamicSmemBytes = smem;
+    cudaLaunchAttribute attr[1]{};
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = parts; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr; cfg.numAttrs = 1;
+    int found = 0;
+    if (cudaOccupancyMaxActiveClusters(&found, gemm_tcgen05_kernel<0, 256, true>, &cfg) != cudaSuccess) { cudaGetLastError(); return 0; }
+    return n = found;
 }
 
 // ------------------------------------------------------------------------------------------------
@@ -598,31 +735,22 @@ static int gemm_impl(const void* A, const void* B, void* C, const void* bias,
         return llmq_gemm_2cta_launch(ta, tb, tc, p, num_sms, stream);
     }
 
-    static bool attr_set[64] = {};          // the attribute is per device
-    int dev = 0;
-    cudaGetDevice(&dev);
-    if (!attr_set[dev & 63]) {
-        const cudaFuncAttribute at = cudaFuncAttributeMaxDynamicSharedMemorySize;
-        cudaError_t e = cudaFuncSetAttribute(gemm_tcgen05_kernel<1, 256>, at, Tile<256>::SMEM_BYTES);
-        if (e == cudaSuccess) e = cudaFuncSetAttribute(gemm_tcgen05_kernel<0, 256>, at, Tile<256>::SMEM_BYTES);
-        if (e == cudaSuccess) e = cudaFuncSetAttribute(gemm_tcgen05_kernel<2, 256>, at, Tile<256>::SMEM_BYTES);
-        if (e == cudaSuccess) e = cudaFuncSetAttribute(gemm_tcgen05_kernel<1, 128>, at, Tile<128>::SMEM_BYTES);
-        if (e == cudaSuccess) e = cudaFuncSetAttribute(gemm_tcgen05_kernel<0, 128>, at, Tile<128>::SMEM_BYTES);
-        if (e != cudaSuccess) return static_cast<int>(e);
-        attr_set[dev & 63] = true;
-    }
+    // The parts of a tile form a cluster, which adds them up in distributed shared memory, where all clusters reside at once (148 SMs hold 74 / 45 / 33 / 26 /
+    // 22 / 15 / 15 of 2 .. 8 CTAs) and rows are whole 16-byte vectors of sums.  Otherwise the parts go through the workspace to a second kernel:
+    // a second round of clusters costs more than that.  us in a graph, two kernels / clusters: 1001 x 896 x 1152 12.9 / 9.9, 1152 x 896 x 1001 added to C
+    // 14.6 / 11.2, 896 x 896 x 1024 13.8 / 10.1, 339 x 3584 x 3584 added 22.4 / 16.4, 117 x 17920 x 1536 19.5 / 14.2, 576 x 1536 x 8960 30.4 / 24.4, 256 x 256 x 8192
+    // 11.1 / 9.2, 1966 x 896 x 9728 42 / 35 (50 shapes whose clusters reside: 0.68 to 1.02, 0.85 on average);  with more tiles 1152 x 896 x 4096 (36 of 4 parts) 22.6 / 28.4,
+    // 287 x 3072 x 8192 (36 of 4) 25.8 / 36.2, 256 x 2048 x 8192 e4m3 (16 of 8) 15.2 / 23.5.
     const int tiles = bn == 128 ? tiles128 : tiles256;
+    const int out_bytes = c_dtype == 0 ? 8 : 16;                           // four columns
+    const bool vec = N % 4 == 0 && ldc % 4 == 0 && reinterpret_cast<uintptr_t>(C) % out_bytes == 0;
     if (splits > 1) { p.k_splits = splits; p.partial = splitk_ws; }
-    const int items = tiles * splits;
-    int grid = items < num_sms ? items : num_sms;
-    if (bn == 128) {
-        if (eb == 1) launch_chained(gemm_tcgen05_kernel<1, 128>, grid, NUM_THREADS, Tile<128>::SMEM_BYTES, stream, ta, tb, p);
-        else         launch_chained(gemm_tcgen05_kernel<0, 128>, grid, NUM_THREADS, Tile<128>::SMEM_BYTES, stream, ta, tb, p);
-    } else {
-        if (eb == 1)      launch_chained(gemm_tcgen05_kernel<1, 256>, grid, NUM_THREADS, Tile<256>::SMEM_BYTES, stream, ta, tb, p);
-        else if (eb == 2) launch_chained(gemm_tcgen05_kernel<0, 256>, grid, NUM_THREADS, Tile<256>::SMEM_BYTES, stream, ta, tb, p);
-        else              launch_chained(gemm_tcgen05_kernel<2, 256>, grid, NUM_THREADS, Tile<256>::SMEM_BYTES, stream, ta, tb, p);
-    }
+    const bool cluster = splits > 1 && vec && tiles <= resident_clusters(splits);
+    if (bn == 128) rc = eb == 1 ? launch_one_cta<1, 128>(ta, tb, p, tiles * splits, cluster, num_sms, stream) : launch_one_cta<0, 128>(ta, tb, p, tiles * splits, cluster, num_sms, stream);
+    else if (eb == 1) rc = launch_one_cta<1, 256>(ta, tb, p, tiles * splits, cluster, num_sms, stream);
+    else if (eb == 2) rc = launch_one_cta<0, 256>(ta, tb, p, tiles * splits, cluster, num_sms, stream);
+    else              rc = launch_one_cta<2, 256>(ta, tb, p, tiles * splits, cluster, num_sms, stream);
+    if (rc || cluster) return rc;
     if (splits > 1) {
         const long long total = static_cast<long long>(M) * N;             // at most kSplitFloats / 2
         const int out_bytes = c_dtype == 0 ? 8 : 16;                       // four columns

@@ -11,6 +11,7 @@ from llmq_b200.ops import lib as L
 pytestmark = pytest.mark.gpu
 DEV = "cuda"
 BF = torch.bfloat16
+F8 = torch.float8_e4m3fn
 
 
 @pytest.fixture(autouse=True)
@@ -321,6 +322,34 @@ def test_split_k_reduce(N, out_dt):
     want = 0.5 * (a.double() @ b.double().t()) + bias.double() + prev.double()
     assert rel(out, want) < (2 ** -8 if out_dt == BF else 1e-5)
     assert abs(am.item() - want.abs().max().item()) < 1e-3 * want.abs().max().item()
+
+
+# K cut into 2 to 8 parts that a cluster adds up, uneven shares of its rows (3, 5, 6, 7 parts), ragged last tiles, both tile widths; one tile more than clusters
+# reside (36 of 4 parts, 28 of 5, 16 of 8) and N = 301 go through the second kernel
+@pytest.mark.parametrize("M,N,Kd,parts", [(1001, 896, 1152, 2), (130, 8196, 2048, 2), (339, 3584, 3584, 3), (64, 2048, 1536, 3), (200, 2052, 2048, 4), (1152, 896, 2048, 4),
+                                          (385, 1280, 3584, 7), (848, 896, 2560, 5), (385, 1024, 3072, 6), (97, 304, 4096, 8), (256, 2048, 4096, 8), (97, 301, 4096, 8)])
+@pytest.mark.parametrize("dt,out_dt", [(BF, BF), (F8, BF), (BF, torch.float32), (torch.float32, torch.float32)])
+def test_split_k_parts(M, N, Kd, parts, dt, out_dt):
+    Kd *= {1: 2, 2: 1, 4: 1}[dt.itemsize]                    # as many K steps of 128 bytes (fp32: twice as many, so the same parts or more)
+    floats = L.kernels().llmq_gemm_splitk_floats(M, N, Kd, dt.itemsize, 148)
+    assert floats == parts * M * N or dt == torch.float32 and floats >= parts * M * N
+    g = torch.Generator(device=DEV).manual_seed(M)
+    a, b = torch.randn(M, Kd, device=DEV, generator=g).to(dt), torch.randn(N, Kd, device=DEV, generator=g).to(dt)
+    bias, prev, scale = torch.randn(N, device=DEV, generator=g).to(BF), torch.randn(M, N, device=DEV, generator=g).to(out_dt), torch.full((1,), 0.5, device=DEV)
+    rows = torch.full((M + 1, N), 9.0, device=DEV, dtype=out_dt)
+    am = torch.zeros(1, device=DEV)
+    plain, added = rows[:M], prev.clone()
+    K.gemm(plain, a, b)
+    K.gemm(added, a, b, bias=bias, accumulate=True, scale_a=scale, absmax=am)
+    K.check_status(torch.device(DEV, 0))
+    prod = a.double() @ b.double().t()
+    want = 0.5 * prod + bias.double() + prev.double()
+    # fp32 sums; products of fp32 operands have 10-bit mantissas (tf32 truncates: 2^-10 an operand); one rounding to bf16 of the outputs
+    eps = 2e-3 if dt == torch.float32 else 1e-5
+    eps += 2 ** -8 if out_dt == BF else 0
+    assert rel(plain, prod) < eps and rel(added, want) < eps
+    assert (rows[M] == 9).all()
+    assert abs(am.item() - want.abs().max().item()) < 4e-3 * want.abs().max().item()
 
 
 def _split_k_operands(n, seed):
