@@ -4,6 +4,7 @@
 // the intermediate rounded to the storage type (matches the HF modelling code), abs-max of y fused.
 #include "api.h"
 #include "common.cuh"
+#include "ptx_sm100.cuh"
 
 namespace {
 
@@ -252,52 +253,23 @@ rmsnorm_bwd_kernel(T* __restrict__ dinp,               // in: upstream residual 
     block_absmax_commit(absmax_out, tmax, scratch);
 }
 
-// 16 bytes from global to shared memory, asynchronously; a thread waits for its own copies in groups, in order
-__device__ __forceinline__ void copy_async16(void* dst, const void* src) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(static_cast<uint32_t>(__cvta_generic_to_shared(dst))), "l"(src) : "memory");
+// `bytes` (a multiple of 16, both addresses aligned to 16) from global to shared memory by the copy engine; counted by the barrier
+__device__ __forceinline__ void copy_row_async(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+                 ::"r"(dst), "l"(src), "r"(bytes), "r"(bar) : "memory");
 }
-__device__ __forceinline__ void copy_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void copy_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 
-// Same contract, for rows of up to 4 column vectors per thread: the row's dout, inp and residual gradient are
-// loaded once and stay in registers across the block-wide dot product (no second pass over L1 / L2), the norm
-// weights are loaded once per CTA, and three CTAs share an SM so that their reductions overlap.  One barrier per row: 16384 x 3584,
-// 470 MB, 94 us; 102 us with the two of a general block reduction; 152 us with the next row loaded ahead (two CTAs per SM, spills).
-// STAGES > 0: that many rows to come are on their way into shared memory; every thread copies and reads back its own vectors, so the
-// ring needs no barrier.  Rows of one vector a thread are too short to hide the load latency behind one another (16384 x 896 39.4 -> 30.2 us,
-// 4096 x 896 11.4 -> 9.2), with four the residual gradient no longer waits in registers (16384 x 5120 209 -> 184, 2000 x 5120 33 -> 27); with two the
-// registers hold everything, and the detour costs (16384 x 3584 94 -> 103).  fp32 rows have none: half the elements a vector make the registers
-// last (16384 x 3584 160 us either way, 16384 x 896 41 -> 48).
-template <typename T, int VPT, int STAGES>
+// Same contract, for fp32 rows of two to four column vectors per thread: the row's dout, inp and residual gradient are loaded once and stay in
+// registers across the block-wide dot product.  4000 x 4096 51.6 us, 53.2 with the rows in shared memory (below), 1000 x 2048 12.2 / 13.2.
+template <typename T, int VPT>
 __global__ void __launch_bounds__(NORM_THREADS, VPT <= 2 ? 3 : 2)
 rmsnorm_bwd_reg_kernel(T* __restrict__ dinp, float* __restrict__ dw_partial, const T* __restrict__ dout, const T* __restrict__ inp,
                        const T* __restrict__ weight, const float* __restrict__ rstd, int rows, int C, float* __restrict__ absmax_out) {
     __shared__ float scratch[32];
     __shared__ float dots[2][NORM_THREADS / 32];             // alternating, so that one barrier per row is enough
-    extern __shared__ uint4 ring[];                          // [STAGES][3][VPT][NORM_THREADS]
     using V = Vec16<T>;
     float dw[VPT][V::N];
     V vw[VPT];
-    auto slot = [&](int stage, int what, int k) { return ring + ((stage * 3 + what) * VPT + k) * NORM_THREADS + threadIdx.x; };
-    auto fetch = [&](long long row, int stage) {
-        if (row < rows) {
-#pragma unroll
-            for (int k = 0; k < VPT; ++k) {
-                const int c = (k * NORM_THREADS + threadIdx.x) * V::N;
-                if (c < C) {
-                    copy_async16(slot(stage, 0, k), dout + row * C + c);
-                    copy_async16(slot(stage, 1, k), inp + row * C + c);
-                    copy_async16(slot(stage, 2, k), dinp + row * C + c);
-                }
-            }
-        }
-        copy_async_commit();                                 // a group per row, empty beyond the last one
-    };
-    if constexpr (STAGES > 0) {
-#pragma unroll
-        for (int st = 0; st < STAGES; ++st) fetch(blockIdx.x + static_cast<long long>(st) * gridDim.x, st);
-    }
 #pragma unroll
     for (int k = 0; k < VPT; ++k) {
         const int c = (k * NORM_THREADS + threadIdx.x) * V::N;
@@ -307,21 +279,16 @@ rmsnorm_bwd_reg_kernel(T* __restrict__ dinp, float* __restrict__ dw_partial, con
     }
     float tmax = 0.f;
     const float inv_c = 1.f / C;
-    int par = 0, stage = 0;
+    int par = 0;
     for (long long row = blockIdx.x; row < rows; row += gridDim.x, par ^= 1) {
         const T* dy = dout + row * C;
         const T* x = inp + row * C;
         T* dx = dinp + row * C;
-        V vdy[VPT], vx[VPT], vd[STAGES > 0 ? 1 : VPT];
-        if constexpr (STAGES > 0) copy_async_wait<STAGES - 1>();
+        V vdy[VPT], vx[VPT], vd[VPT];
 #pragma unroll
         for (int k = 0; k < VPT; ++k) {
             const int c = (k * NORM_THREADS + threadIdx.x) * V::N;
-            if constexpr (STAGES > 0) {
-                if (c < C) { vdy[k] = V::load(reinterpret_cast<const T*>(slot(stage, 0, k))); vx[k] = V::load(reinterpret_cast<const T*>(slot(stage, 1, k))); }
-            } else {
-                if (c < C) { vdy[k] = V::load_stream(dy + c); vx[k] = V::load_stream(x + c); vd[k] = V::load_stream(dx + c); }
-            }
+            if (c < C) { vdy[k] = V::load_stream(dy + c); vx[k] = V::load_stream(x + c); vd[k] = V::load_stream(dx + c); }
         }
         const float rs = rstd[row];
         float dot = 0.f;
@@ -346,8 +313,7 @@ rmsnorm_bwd_reg_kernel(T* __restrict__ dinp, float* __restrict__ dw_partial, con
         for (int k = 0; k < VPT; ++k) {
             const int c = (k * NORM_THREADS + threadIdx.x) * V::N;
             if (c < C) {
-                V& d = vd[STAGES > 0 ? 0 : k];
-                if constexpr (STAGES > 0) d = V::load(reinterpret_cast<const T*>(slot(stage, 2, k)));
+                V& d = vd[k];
 #pragma unroll
                 for (int i = 0; i < V::N; ++i) {
                     const float xh = to_float(vx[k].v[i]) * rs;
@@ -357,10 +323,6 @@ rmsnorm_bwd_reg_kernel(T* __restrict__ dinp, float* __restrict__ dw_partial, con
                 }
                 d.store(dx + c);
             }
-        }
-        if constexpr (STAGES > 0) {
-            fetch(row + static_cast<long long>(STAGES) * gridDim.x, stage);
-            if (++stage == STAGES) stage = 0;
         }
     }
 #pragma unroll
@@ -374,10 +336,114 @@ rmsnorm_bwd_reg_kernel(T* __restrict__ dinp, float* __restrict__ dw_partial, con
     block_absmax_commit(absmax_out, tmax, scratch);
 }
 
-// Column sums of the per-CTA partial rows.  A CTA owns 64 columns; its 16 thread rows walk the partial rows with a stride
+// Same contract, for rows of up to 4 column vectors per thread.  Rows to come are on their way into shared memory: three bulk copies per row, issued by one
+// thread, so that neither registers nor load instructions are spent on what is in flight, and the registers hold the weight gradient and little
+// else (both passes over a row read it from shared memory).  One barrier per row; it also says that the row before has been read, whose place the next
+// copies take.  Memory is the limit for long rows.  us, rows in registers (two vectors a thread) or copied thread by thread (one, four) / now:
+// 16384 x 3584, 470 MB, 98.7 / 77.9;  16384 x 3072 91 / 71;  4096 x 3584 31.6 / 30.3;  16384 x 5120 191 / 146;  4000 x 8192 91 / 66;  16384 x 2048 66 / 54;  16384 x 896 42.5 / 37.5;
+// 4096 x 896 16.3 / 14.7;  fp32 4096 x 896 18.7 / 17.3.  Two rows per turn and barrier, with two CTAs per SM: 16384 x 3584 84.
+template <typename T, int VPT, int STAGES, int CTAS>
+__global__ void __launch_bounds__(NORM_THREADS, CTAS)
+rmsnorm_bwd_ring_kernel(T* __restrict__ dinp, float* __restrict__ dw_partial, const T* __restrict__ dout, const T* __restrict__ inp,
+                        const T* __restrict__ weight, const float* __restrict__ rstd, int rows, int C, float* __restrict__ absmax_out) {
+    __shared__ float scratch[32];
+    static_assert(STAGES >= 2, "the row in use and the ones on their way");
+    __shared__ float dots[2][NORM_THREADS / 32];             // alternating, so that one barrier per row is enough
+    extern __shared__ __align__(16) uint8_t ring[];          // [STAGES][dout, inp, dinp][C]
+    __shared__ uint64_t full[STAGES];
+    __shared__ uint32_t gave_up;
+    using V = Vec16<T>;
+    float dw[VPT][V::N];
+    V vw[VPT];
+    const uint32_t row_bytes = C * sizeof(T);
+    auto slot = [&](int stage, int what) { return ring + (stage * 3 + what) * row_bytes; };
+    auto fetch = [&](long long row, int stage) {             // one thread
+        if (row < rows) {
+            const uint32_t bar = sm100::smem_u32(full + stage);
+            sm100::mbar_expect_tx(bar, 3 * row_bytes);
+            copy_row_async(sm100::smem_u32(slot(stage, 0)), dout + row * C, row_bytes, bar);
+            copy_row_async(sm100::smem_u32(slot(stage, 1)), inp + row * C, row_bytes, bar);
+            copy_row_async(sm100::smem_u32(slot(stage, 2)), dinp + row * C, row_bytes, bar);
+        }
+    };
+    const long long step = gridDim.x;
+    if (threadIdx.x == 0) {
+        for (int st = 0; st < STAGES; ++st) sm100::mbar_init(sm100::smem_u32(full + st), 1);
+        gave_up = 0;
+        sm100::mbar_init_fence();
+        for (int st = 0; st < STAGES; ++st) fetch(blockIdx.x + st * step, st);
+    }
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < VPT; ++k) {
+        const int c = (k * NORM_THREADS + threadIdx.x) * V::N;
+        if (c < C) vw[k] = V::load(weight + c);
+#pragma unroll
+        for (int i = 0; i < V::N; ++i) dw[k][i] = 0.f;
+    }
+    float tmax = 0.f;
+    const float inv_c = 1.f / C;
+    int par = 0, stage = 0;
+    uint32_t phase = 0;
+    bool ok = true;
+    for (long long row = blockIdx.x; row < rows; row += step, par ^= 1) {
+        const float rs = rstd[row];
+        float dot = 0.f;
+        ok = sm100::mbar_wait(sm100::smem_u32(full + stage), phase, &gave_up) && ok;
+#pragma unroll
+        for (int k = 0; k < VPT; ++k) {
+            const int c = (k * NORM_THREADS + threadIdx.x) * V::N;
+            if (c < C) {
+                const V vdy = V::load(reinterpret_cast<const T*>(slot(stage, 0)) + c), vx = V::load(reinterpret_cast<const T*>(slot(stage, 1)) + c);
+#pragma unroll
+                for (int i = 0; i < V::N; ++i) {
+                    const float xh = to_float(vx.v[i]) * rs;
+                    const float g = to_float(vdy.v[i]);
+                    dot += to_float(vw[k].v[i]) * g * xh;
+                    dw[k][i] += g * xh;
+                }
+            }
+        }
+        dot = warp_reduce_sum(dot);
+        if ((threadIdx.x & 31) == 0) dots[par][threadIdx.x >> 5] = dot;
+        __syncthreads();
+        // every thread is through with the row before: the row STAGES behind that one takes its place
+        if (threadIdx.x == 0 && row != blockIdx.x) fetch(row + (STAGES - 1) * step, stage == 0 ? STAGES - 1 : stage - 1);
+        dot = tree8(dots[par]) * inv_c;
+        T* dx = dinp + row * C;
+#pragma unroll
+        for (int k = 0; k < VPT; ++k) {
+            const int c = (k * NORM_THREADS + threadIdx.x) * V::N;
+            if (c < C) {
+                const V vdy = V::load(reinterpret_cast<const T*>(slot(stage, 0)) + c), vx = V::load(reinterpret_cast<const T*>(slot(stage, 1)) + c);
+                V vd = V::load(reinterpret_cast<const T*>(slot(stage, 2)) + c);
+#pragma unroll
+                for (int i = 0; i < V::N; ++i) {
+                    const float xh = to_float(vx.v[i]) * rs;
+                    const float g = (to_float(vw[k].v[i]) * to_float(vdy.v[i]) - xh * dot) * rs;
+                    vd.v[i] = from_float<T>(to_float(vd.v[i]) + g);
+                    tmax = fmaxf(tmax, fabsf(to_float(vd.v[i])));
+                }
+                vd.store(dx + c);
+            }
+        }
+        if (++stage == STAGES) { stage = 0; phase ^= 1u; }
+    }
+#pragma unroll
+    for (int k = 0; k < VPT; ++k) {
+        const int c = (k * NORM_THREADS + threadIdx.x) * V::N;
+        if (c < C) {
+#pragma unroll
+            for (int i = 0; i < V::N; ++i) dw_partial[static_cast<long long>(blockIdx.x) * C + c + i] = ok ? dw[k][i] : NAN;      // a copy that never came shows
+        }
+    }
+    block_absmax_commit(absmax_out, tmax, scratch);
+}
+
+// Column sums of the per-CTA partial rows.  A CTA owns 32 columns; its 16 thread rows walk the partial rows with a stride
 // of 16 (28 loads per thread for 444 partial rows instead of 444 dependent loads in one thread) and are summed through
 // shared memory in a fixed order, so the result does not depend on the schedule.
-constexpr int RED_COLS = 64, RED_GROUPS = 16;
+constexpr int RED_COLS = 32, RED_GROUPS = 16;
 template <typename T>
 __global__ void __launch_bounds__(RED_COLS * RED_GROUPS)
 rmsnorm_bwd_reduce_kernel(T* __restrict__ dweight, const float* __restrict__ dw_partial, int nparts, int C, int accumulate) {
@@ -438,38 +504,65 @@ int launch_fwd(void* residual_out, void* y_out, void* q_out, float* rstd, const 
     return LLMQ_LAUNCH_CHECK();
 }
 
+int device_sms() {
+    static int sms[64] = {};
+    int dev = 0;
+    cudaGetDevice(&dev);
+    int& n = sms[dev & 63];
+    if (n <= 0 && (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0)) n = 148;
+    return n;
+}
+
+template <typename T, int VPT, int STAGES, int CTAS>
+int launch_bwd_ring(T* dinp, float* scratch, const T* dout, const T* inp, const T* w, const float* rstd, int rows, int C, float* absmax, int blocks, cudaStream_t s) {
+    static bool attr_set[64] = {};          // per device
+    int dev = 0;
+    cudaGetDevice(&dev);
+    if (!attr_set[dev & 63]) {
+        cudaError_t e = cudaFuncSetAttribute(rmsnorm_bwd_ring_kernel<T, VPT, STAGES, CTAS>, cudaFuncAttributeMaxDynamicSharedMemorySize, STAGES * 3 * VPT * NORM_THREADS * 16);
+        if (e != cudaSuccess) return static_cast<int>(e);
+        attr_set[dev & 63] = true;
+    }
+    rmsnorm_bwd_ring_kernel<T, VPT, STAGES, CTAS><<<blocks, NORM_THREADS, STAGES * 3 * C * sizeof(T), s>>>(dinp, scratch, dout, inp, w, rstd, rows, C, absmax);
+    return LLMQ_LAUNCH_CHECK();
+}
+
 template <typename T>
-int launch_bwd(void* dinp, void* dweight, float* scratch, const void* dout, const void* inp, const void* w,
+int launch_bwd(void* dinp_, void* dweight, float* scratch, const void* dout_, const void* inp_, const void* w_,
                const float* rstd, int rows, int C, float* absmax, int accumulate_dw, int num_blocks, cudaStream_t s) {
     using V = Vec16<T>;
     if (C % V::N) return -1;
     const int vecs = ceil_div_i(C / V::N, NORM_THREADS);
-    if (num_blocks > rows) num_blocks = rows;
-#define LAUNCH(KERNEL, SMEM)                                                                                                 \
-    KERNEL<<<num_blocks, NORM_THREADS, SMEM, s>>>(static_cast<T*>(dinp), scratch, static_cast<const T*>(dout), static_cast<const T*>(inp), \
-                                               static_cast<const T*>(w), rstd, rows, C, absmax)
-#define LAUNCH_RING(VPT, STAGES)                                                                                             \
-    {                                                                                                                        \
-        constexpr int smem = (STAGES) * 3 * (VPT) * NORM_THREADS * 16;                                                       \
-        static bool attr_set[64] = {};          /* per device */                                                             \
-        int dev = 0;                                                                                                         \
-        cudaGetDevice(&dev);                                                                                                 \
-        if (!attr_set[dev & 63]) {                                                                                           \
-            cudaError_t e = cudaFuncSetAttribute(rmsnorm_bwd_reg_kernel<T, VPT, STAGES>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem); \
-            if (e != cudaSuccess) return static_cast<int>(e);                                                                \
-            attr_set[dev & 63] = true;                                                                                       \
-        }                                                                                                                    \
-        LAUNCH((rmsnorm_bwd_reg_kernel<T, VPT, STAGES>), smem);                                                              \
+    // Blocks: few rows go to few blocks, whose rows follow one another through the ring; every block costs a partial row that the second kernel has to read.
+    // us with one / two / three blocks per SM:  444 x 3072 8.6 / 9.8 / 11.9,  444 x 4096 9.8 / 11.4 / 13.9,  888 x 4096
+    // 14.4 / 16.0 / 18.2,  888 x 1536 8.3 / 8.6 / 9.3,  1200 x 3072 15.0 / 14.9 / 16.4,  2500 x 4096 25.9 / 24.0 / 26.3,  4000 x 3072 31.8 / 26.5 / 25.8,
+    // 8000 x 2048 49 / 35 / 33;  three or four vectors a thread, of which two blocks reside: 888 x 5120 17.6 / 18.1 / 22.7,  8000 x 5120 90 / 66 / 79.
+    // Rows of up to 1024 columns keep three: their sums over the rows, and with them the weight gradients, keep their order.
+    if (sizeof(T) == 2 && C > 1024 && C <= 4 * NORM_THREADS * V::N) {
+        const int sms = device_sms();
+        const int most = (rows <= 7 * sms ? 1 : vecs > 2 || rows <= 24 * sms ? 2 : 3) * sms;
+        if (num_blocks > most) num_blocks = most;
     }
-    constexpr bool h = sizeof(T) == 2;
-    if (vecs <= 1) LAUNCH_RING(1, (h ? 4 : 0))
-    else if (vecs <= 2) LAUNCH((rmsnorm_bwd_reg_kernel<T, 2, 0>), 0);
-    else if (vecs <= 4) LAUNCH_RING(4, (h ? 2 : 0))
-    else if (vecs <= 8) LAUNCH((rmsnorm_bwd_kernel<T, 8>), 0);
-    else return -2;
-#undef LAUNCH_RING
-#undef LAUNCH
-    int rc = LLMQ_LAUNCH_CHECK();
+    if (num_blocks > rows) num_blocks = rows;
+    T* dinp = static_cast<T*>(dinp_);
+    const T *dout = static_cast<const T*>(dout_), *inp = static_cast<const T*>(inp_), *w = static_cast<const T*>(w_);
+    int rc;
+    // stages and CTAs per SM: as much shared memory as fits
+    if (vecs <= 1) rc = launch_bwd_ring<T, 1, 4, 3>(dinp, scratch, dout, inp, w, rstd, rows, C, absmax, num_blocks, s);
+    else if (vecs <= 4) {
+        if constexpr (sizeof(T) == 2) {
+            if (vecs <= 2) rc = launch_bwd_ring<T, 2, 3, 3>(dinp, scratch, dout, inp, w, rstd, rows, C, absmax, num_blocks, s);
+            else           rc = launch_bwd_ring<T, 4, 2, 2>(dinp, scratch, dout, inp, w, rstd, rows, C, absmax, num_blocks, s);
+        } else {
+            if (vecs <= 2) rmsnorm_bwd_reg_kernel<T, 2><<<num_blocks, NORM_THREADS, 0, s>>>(dinp, scratch, dout, inp, w, rstd, rows, C, absmax);
+            else           rmsnorm_bwd_reg_kernel<T, 4><<<num_blocks, NORM_THREADS, 0, s>>>(dinp, scratch, dout, inp, w, rstd, rows, C, absmax);
+            rc = LLMQ_LAUNCH_CHECK();
+        }
+    }
+    else if (vecs <= 8) {
+        rmsnorm_bwd_kernel<T, 8><<<num_blocks, NORM_THREADS, 0, s>>>(dinp, scratch, dout, inp, w, rstd, rows, C, absmax);
+        rc = LLMQ_LAUNCH_CHECK();
+    } else return -2;
     if (rc) return rc;
     launch_chained(rmsnorm_bwd_reduce_kernel<T>, ceil_div_i(C, RED_COLS), RED_COLS * RED_GROUPS, 0, s, static_cast<T*>(dweight), scratch, num_blocks, C, accumulate_dw);
     return LLMQ_LAUNCH_CHECK();

@@ -782,6 +782,23 @@ def test_second_passes_and_tables_see_what_the_kernel_before_wrote():
     _same_with_and_without_waits(chain)
 
 
+# blocks per SM of the backward kernel on both sides of the rule (7 and 24 rows per SM, three or four vectors a thread), as many rows as blocks and one more
+@pytest.mark.parametrize("C", [1024, 1032, 3584, 4096, 4104])
+@pytest.mark.parametrize("rows", [1, 2, 148, 149, 1036, 1037, 3552, 3553])
+def test_rmsnorm_backward_blocks(C, rows):
+    g = torch.Generator(device=DEV).manual_seed(C + rows)
+    x, w, dy, dres, dw0 = (torch.randn(*s, device=DEV, generator=g).to(BF) for s in ((rows, C), (C,), (rows, C), (rows, C), (C,)))
+    rs = torch.rsqrt(x.double().square().mean(-1, keepdim=True) + 1e-6)
+    dinp, dw, am = dres.clone(), dw0.clone(), torch.zeros(1, device=DEV)
+    scratch = torch.full((K.rmsnorm_backward_scratch_elems(C, torch.device(DEV, 0)),), math.nan, device=DEV)
+    K.rmsnorm_backward(dinp, dw, scratch, dy, x, w, rs[:, 0].float().contiguous(), absmax=am)
+    xh, wdy = x.double() * rs, w.double() * dy.double()
+    gx = dres.double() + (wdy - xh * (wdy * xh).mean(-1, keepdim=True)) * rs
+    # every element: one rounding to bf16 (2^-9 of it) and fp32 arithmetic on terms of a few units
+    assert ((dinp.double() - gx).abs() <= gx.abs() * 2**-8 + 1e-5 * (1 + wdy.abs() * rs)).all()
+    assert rel(dw, dw0.double() + (dy.double() * xh).sum(0)) < 2**-8 and am.item() == dinp.float().abs().max().item()
+
+
 # the ring of the backward kernel turns: more rows per block than it has stages, one vector a thread (four stages) and three or four (two)
 @pytest.mark.parametrize("C", [896, 2048, 4104, 5120, 8192])
 @pytest.mark.parametrize("rows", [1001, 1777, 3000])
