@@ -1,10 +1,13 @@
 """In-tree native build: compiles every CUDA source for sm_100a and the host runtime with g++.
 
-Two shared libraries are produced under ``llmq_b200/lib``:
+Shared libraries are produced under ``llmq_b200/lib``:
 
 * ``libllmq_b200_kernels.so`` - all device kernels and their C launchers (``csrc/*.cu``)
 * ``libllmq_b200_rt.so``      - host-side runtime: token-file data loader, safetensors writer,
   bump/stack arena bookkeeping, pinned staging helpers (``csrc/rt/*.cpp``)
+
+and, where torch and the headers of Python are at hand, ``llmq_b200_binding.so``, an extension module for the interpreter that runs the
+build (``csrc/py/binding.cpp``); without it the same kernels are called through ctypes, with more host time per call.
 
 The build is incremental (object files are rebuilt only when a source or header is newer) and
 needs no GPU: nvcc cross-compiles.  Run ``python -m llmq_b200.build`` or call :func:`build`.
@@ -82,6 +85,29 @@ def build(verbose: bool = False, force: bool = False) -> None:
         cmd = ["g++", "-shared", "-pthread", "-o", str(rlib), *map(str, cpp_objs),
                "-L/usr/local/cuda/lib64", "-lcudart_static", "-ldl", "-lrt"]
         _compile(cmd, "link runtime", rlib, verbose)
+    _build_binding(verbose, force)
+
+
+def _build_binding(verbose: bool, force: bool) -> None:
+    """The extension module, for this interpreter and its torch."""
+    import importlib.util
+    import sysconfig
+
+    src, out = CSRC / "py" / "binding.cpp", LIBDIR / "llmq_b200_binding.so"
+    torch_spec = importlib.util.find_spec("torch")
+    python_inc = sysconfig.get_paths()["include"]
+    if torch_spec is None or not os.path.exists(os.path.join(python_inc, "Python.h")):
+        return
+    torch_dir = Path(torch_spec.origin).parent
+    if not (torch_dir / "include" / "torch" / "csrc" / "autograd" / "python_variable.h").exists():
+        return
+    version = torch_dir / "version.py"
+    if not force and out.exists() and out.stat().st_mtime > max(src.stat().st_mtime, version.stat().st_mtime if version.exists() else 0.0):
+        return
+    cmd = ["g++", "-O2", "-std=c++20", "-fPIC", "-shared", "-Wall", "-I", str(torch_dir / "include"), "-I", str(torch_dir / "include/torch/csrc/api/include"),
+           "-I", python_inc, "-I", "/usr/local/cuda/include", str(src), "-o", str(out), f"-L{torch_dir / 'lib'}", "-ltorch_python", "-ltorch_cpu", "-lc10",
+           "-lc10_cuda", f"-Wl,-rpath,{torch_dir / 'lib'}"]
+    _compile(cmd, src, out, verbose)
 
 
 def build_tests(verbose: bool = False) -> Path:

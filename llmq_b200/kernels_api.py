@@ -8,21 +8,21 @@ cuBLAS handle or workspace: it is the in-tree tcgen05 GEMM.
 from __future__ import annotations
 
 import inspect
-from operator import itemgetter
+from functools import partial
 from typing import Optional
 
 import torch
 from torch.autograd import forward_ad
-from torch.autograd.graph import increment_version
 
 from .ops import kernels as K
+from .ops import lib as L
 
 T = torch.Tensor
 _C = torch._C
 
 
 # bound once: the checks below run on every call
-_strided, _impls, _is_compiling = torch.strided, torch.library._impls, torch.compiler.is_compiling
+_impls, _is_compiling = torch.library._impls, torch.compiler.is_compiling
 _dispatch_modes, _function_modes, _transform_level = _C._len_torch_dispatch_stack, _C._len_torch_function_stack, _C._functorch.maybe_current_level
 _tracing_state, _profiling = _C._get_tracing_state, _C._autograd._profiler_enabled
 
@@ -37,11 +37,14 @@ def _op(name: str, mutates_args):
     """``torch.library.custom_op`` whose plain eager calls go straight to the function.
 
     Four Python layers of the custom-op machinery (autograd, in-place tracking, back-end wrapper, aliasing check) take longer than
-    most of these kernels run (27 us a call, against 5 us for the checks below, on one x86 core); they matter only to a caller that
+    most of these kernels run (27 us a call, against 1 us for the checks below, on one x86 core); they matter only to a caller that
     differentiates, traces, transforms or profiles the op.  So a call with positional arguments of exactly the schema's types,
     tensors that are plain and an undisturbed dispatcher runs the body and bumps the version of what it mutates, which is what the
     dispatcher would have done; every other call, and every call once a kernel, formula or rule was registered on the op, takes
-    the op as it is registered in ``torch.ops.llmq_b200``."""
+    the op as it is registered in ``torch.ops.llmq_b200``.  The arguments are looked over by the extension module of csrc/py/binding.cpp, or, where
+    it was not built, by the same checks in Python (3 us a call)."""
+
+    native = L.binding()
 
     def wrap(fn):
         op = torch.library.custom_op(name, fn, mutates_args=mutates_args)
@@ -50,34 +53,31 @@ def _op(name: str, mutates_args):
         optional = tuple(q.annotation == Optional[T] for q in params)
         required = sum(q.default is q.empty for q in params)
         mutated = tuple(i for i, q in enumerate(params) if q.name in mutates_args)
-        always = itemgetter(*mutated) if not any(optional[i] or i >= required for i in mutated) else None
+        if native:
+            spec = native.spec(kinds, optional, required, mutated)
+            plain, bump = partial(native.plain, spec), partial(native.bump, spec)
+        else:
+            def plain(args) -> bool:
+                return required <= len(args) <= len(kinds) and all(
+                    type(v) is kind if kind is not None else v is None and opt or
+                    # a strided CPU or CUDA tensor that nothing but its own kernel has to see: no subclass, gradient, inference or lazy
+                    # bit, and not a zero tensor, which has no memory until the dispatcher gives it some
+                    (type(v) is T and not v.requires_grad and v.layout is torch.strided and not v.is_inference() and not v.is_neg() and not v._is_zerotensor()
+                     and (v.is_cuda or v.device.type == "cpu")) for v, kind, opt in zip(args, kinds, optional))
+
+            def bump(args) -> None:
+                torch.autograd.graph.increment_version([args[i] for i in mutated if i < len(args) and args[i] is not None])
         # what torch.library.impl / Library.impl note when somebody adds a kernel to the op behind this object's back
         added = frozenset(name.replace("::", "/") + "/" + key for key in
                           ("CPU", "CUDA", "AutogradCPU", "AutogradCUDA", "AutocastCPU", "AutocastCUDA", "BackendSelect"))
-
-        def is_plain(args) -> bool:
-            if not required <= len(args) <= len(kinds) or not _plain_context():
-                return False
-            for v, kind, opt in zip(args, kinds, optional):
-                if kind is None:
-                    if v is None and opt:
-                        continue
-                    # a strided CPU or CUDA tensor that nothing but its own kernel has to see: no subclass, gradient, inference or lazy
-                    # bit, and not a zero tensor, which has no memory until the dispatcher gives it some
-                    if (type(v) is not T or v.requires_grad or v.layout is not _strided or v.is_inference() or v.is_neg() or v._is_zerotensor()
-                            or not (v.is_cuda or v.device.type == "cpu")):
-                        return False
-                elif type(v) is not kind:
-                    return False
-            return True
 
         class EagerOp(type(op)):
             direct = True
 
             def __call__(self, *args, **kwargs):
-                if self.direct and not kwargs and _impls.isdisjoint(added) and is_plain(args):
+                if self.direct and not kwargs and _impls.isdisjoint(added) and _plain_context() and plain(args):
                     fn(*args)
-                    increment_version(always(args) if always else [args[i] for i in mutated if i < len(args) and args[i] is not None])
+                    bump(args)
                     return None
                 return super().__call__(*args, **kwargs)
 

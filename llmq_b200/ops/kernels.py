@@ -28,6 +28,9 @@ _state = {}
 
 
 def _dev_state(device):
+    st = _state.get(device)                  # a tensor's device has an index
+    if st is not None:
+        return st
     device = torch.device(device)
     idx = device.index if device.index is not None else torch.cuda.current_device()
     st = _state.get(idx)
@@ -39,7 +42,7 @@ def _dev_state(device):
                 "status": torch.zeros(1, dtype=torch.int32, device=f"cuda:{idx}"),
                 "splitk": os.environ.get("LLMQ_GEMM_SPLITK", "1") != "0",
             }
-        _state[idx] = st
+        _state[idx] = _state[torch.device("cuda", idx)] = st
     return st
 
 
@@ -114,8 +117,8 @@ def gemm(out: torch.Tensor, a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = Fa
     likewise ``b`` holds logical [N,K] as [N,K] or, with ``b_mn``, as [K,N].  2-D, last dim contiguous.
     """
     M, N = out.shape
-    K = a.shape[0] if a_mn else a.shape[1]
-    assert (a.shape[1] if a_mn else a.shape[0]) == M, (a.shape, out.shape, a_mn)
+    K, m = a.shape if a_mn else (a.shape[1], a.shape[0])
+    assert m == M, (a.shape, out.shape, a_mn)
     assert (b.shape == (K, N)) if b_mn else (b.shape == (N, K)), (b.shape, (N, K), b_mn)
     if out.is_cuda and a.dtype == torch.float32 and (a_mn or b_mn):
         # fp32 operands (tf32 MMA kind) are only fed K-major: transpose the other forms first.  The copies, like the other scratch of
@@ -136,13 +139,12 @@ def gemm(out: torch.Tensor, a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = Fa
         rflags, rgen, rrows, rlimit = ready if ready is not None else (0, 0, 0, 0.0)
         stream = L.raw_stream()
         ws = _splitk_workspace(M, N, K, a.element_size(), st, out.device, stream) if ready is None else None
-        rc = L.kernels().llmq_gemm_ready(
-            L.ptr(a), L.ptr(b), L.ptr(out), L.ptr(bias), M, N, K, L.dtype_code(a.dtype), L.dtype_code(b.dtype),
-            int(a_mn), int(b_mn), _ll(a.stride(0)), _ll(b.stride(0)), _ll(out.stride(0)),
+        rc = L.calls().llmq_gemm_ready(
+            a, b, out, bias, M, N, K, L.dtype_code(a.dtype), L.dtype_code(b.dtype),
+            int(a_mn), int(b_mn), a.stride(0), b.stride(0), out.stride(0),
             0 if out.dtype == torch.bfloat16 else 1, 0 if (bias is None or bias.dtype == torch.bfloat16) else 1,
-            int(accumulate), L.ptr(scale_a), L.ptr(scale_b), _f(alpha), L.ptr(absmax), L.ptr(st["status"]), st["sms"],
-            ctypes.c_void_p(rflags), ctypes.c_uint(rgen), int(rrows), ctypes.c_double(rlimit), L.ptr(ws), _ll(0 if ws is None else ws.numel()),
-            ctypes.c_void_p(stream))
+            int(accumulate), scale_a, scale_b, alpha, absmax, st["status"], st["sms"],
+            rflags, rgen, int(rrows), rlimit, ws, 0 if ws is None else ws.numel())
         L.check(rc, "gemm")
         return
     af = a.float().t() if a_mn else a.float()
@@ -311,9 +313,9 @@ def rmsnorm_forward(y: Optional[torch.Tensor], rstd: Optional[torch.Tensor], inp
     C = inp.shape[-1]
     rows = inp.numel() // C
     if inp.is_cuda:
-        rc = L.kernels().llmq_rmsnorm_forward(
-            L.ptr(residual_out), L.ptr(y), L.ptr(q_out), L.ptr(rstd), L.ptr(inp), L.ptr(inp2), L.ptr(weight), _f(eps), rows, C,
-            L.dtype_code(inp.dtype), L.ptr(absmax), L.ptr(known_absmax), L.ptr(q_scale), L.stream_ptr())
+        rc = L.calls().llmq_rmsnorm_forward(
+            residual_out, y, q_out, rstd, inp, inp2, weight, eps, rows, C,
+            L.dtype_code(inp.dtype), absmax, known_absmax, q_scale)
         L.check(rc, "rmsnorm_forward")
         return
     x = inp.float()
@@ -355,9 +357,9 @@ def rmsnorm_backward(dinp: torch.Tensor, dweight: torch.Tensor, scratch: Optiona
     if inp.is_cuda:
         blocks = NORM_BWD_BLOCKS_PER_SM * num_sms(inp.device)
         assert scratch is not None and scratch.numel() >= blocks * C and scratch.dtype == torch.float32
-        rc = L.kernels().llmq_rmsnorm_backward(
-            L.ptr(dinp), L.ptr(dweight), L.ptr(scratch), L.ptr(dout), L.ptr(inp), L.ptr(weight), L.ptr(rstd), rows, C,
-            L.dtype_code(inp.dtype), L.ptr(absmax), int(accumulate_dweight), blocks, L.stream_ptr())
+        rc = L.calls().llmq_rmsnorm_backward(
+            dinp, dweight, scratch, dout, inp, weight, rstd, rows, C,
+            L.dtype_code(inp.dtype), absmax, int(accumulate_dweight), blocks)
         L.check(rc, "rmsnorm_backward")
         return
     x = inp.float().reshape(rows, C)
@@ -386,8 +388,8 @@ def swiglu_forward(out: Optional[torch.Tensor], inp: torch.Tensor, *, absmax: Op
     D = inp.shape[-1] // 2
     rows = inp.numel() // (2 * D)
     if inp.is_cuda:
-        rc = L.kernels().llmq_swiglu_forward(L.ptr(out), L.ptr(q_out), L.ptr(inp), _ll(rows), D, L.dtype_code(inp.dtype),
-                                             L.ptr(absmax), L.ptr(known_absmax), L.ptr(q_scale), num_sms(inp.device), L.stream_ptr())
+        rc = L.calls().llmq_swiglu_forward(out, q_out, inp, rows, D, L.dtype_code(inp.dtype),
+                                           absmax, known_absmax, q_scale, num_sms(inp.device))
         L.check(rc, "swiglu_forward")
         return
     x = inp.float().reshape(rows, 2 * D)
@@ -424,8 +426,8 @@ def swiglu_backward(dinp: torch.Tensor, dout: torch.Tensor, inp: torch.Tensor, *
     D = inp.shape[-1] // 2
     rows = inp.numel() // (2 * D)
     if inp.is_cuda:
-        rc = L.kernels().llmq_swiglu_backward(L.ptr(dinp), L.ptr(dout), L.ptr(inp), _ll(rows), D, L.dtype_code(inp.dtype),
-                                              L.ptr(absmax), num_sms(inp.device), L.stream_ptr())
+        rc = L.calls().llmq_swiglu_backward(dinp, dout, inp, rows, D, L.dtype_code(inp.dtype),
+                                            absmax, num_sms(inp.device))
         L.check(rc, "swiglu_backward")
         return
     x = inp.float().reshape(rows, 2 * D)
@@ -495,8 +497,8 @@ def rope(out: torch.Tensor, inp: torch.Tensor, freqs: torch.Tensor, Hq: int, Hkv
     B, T, H, HS = inp.shape
     assert H == Hq + 2 * Hkv
     if inp.is_cuda:
-        rc = L.kernels().llmq_rope(L.ptr(out), L.ptr(inp), L.ptr(freqs), B, T, Hq, Hkv, HS, L.dtype_code(inp.dtype), int(backward),
-                                   L.ptr(absmax), num_sms(inp.device), L.stream_ptr())
+        rc = L.calls().llmq_rope(out, inp, freqs, B, T, Hq, Hkv, HS, L.dtype_code(inp.dtype), int(backward),
+                                 absmax, num_sms(inp.device))
         L.check(rc, "rope")
         return
     x = inp.float()
@@ -522,8 +524,7 @@ def rope(out: torch.Tensor, inp: torch.Tensor, freqs: torch.Tensor, Hq: int, Hkv
 def abs_max(out: torch.Tensor, x: torch.Tensor) -> None:
     """out = max(out, max|x|)  (``out`` is normally zeroed first)."""
     if x.is_cuda:
-        L.check(L.kernels().llmq_abs_max(L.ptr(out), L.ptr(x), _ll(x.numel()), L.dtype_code(x.dtype), num_sms(x.device),
-                                         L.stream_ptr()), "abs_max")
+        L.check(L.calls().llmq_abs_max(out, x, x.numel(), L.dtype_code(x.dtype), num_sms(x.device)), "abs_max")
         return
     out.copy_(torch.maximum(out, x.float().abs().max().reshape_as(out)))
 
@@ -531,8 +532,8 @@ def abs_max(out: torch.Tensor, x: torch.Tensor) -> None:
 def quantize(out: torch.Tensor, scale_out: Optional[torch.Tensor], x: torch.Tensor, absmax: Optional[torch.Tensor]) -> None:
     """out = sat(x * QMAX / max(absmax, 1e-10)); scale_out = absmax / QMAX (1 when out is not an fp8 type)."""
     if x.is_cuda:
-        L.check(L.kernels().llmq_quantize(L.ptr(out), L.ptr(scale_out), L.ptr(x), L.ptr(absmax), _ll(x.numel()), L.dtype_code(x.dtype),
-                                          L.dtype_code(out.dtype), num_sms(x.device), L.stream_ptr()), "quantize")
+        L.check(L.calls().llmq_quantize(out, scale_out, x, absmax, x.numel(), L.dtype_code(x.dtype),
+                                        L.dtype_code(out.dtype), num_sms(x.device)), "quantize")
         return
     if _is_f8(out.dtype):
         qm = _FP8_MAX[out.dtype]
@@ -554,8 +555,8 @@ def quantize_transpose(out_rows: Optional[torch.Tensor], out_t: torch.Tensor, sc
     x2 = x.reshape(-1, x.shape[-1])
     rows, cols = x2.shape
     if x.is_cuda and rows % 16 == 0 and cols % 16 == 0:
-        L.check(L.kernels().llmq_quantize_transpose(L.ptr(out_rows), L.ptr(out_t), L.ptr(scale_out), L.ptr(x2), L.ptr(absmax), rows, cols,
-                                                    L.dtype_code(x.dtype), L.dtype_code(out_t.dtype), L.stream_ptr()), "quantize_transpose")
+        L.check(L.calls().llmq_quantize_transpose(out_rows, out_t, scale_out, x2, absmax, rows, cols,
+                                                  L.dtype_code(x.dtype), L.dtype_code(out_t.dtype)), "quantize_transpose")
         return
     if x2.element_size() == 1:
         if out_rows is not None:
@@ -572,12 +573,12 @@ def transpose(out: torch.Tensor, x: torch.Tensor, *, absmax: Optional[torch.Tens
     """out[c, r] = x[r, c]; with ``absmax`` the values are quantised to ``out.dtype`` on the way."""
     rows, cols = x.shape
     if x.is_cuda and out.element_size() == 1 and rows % 16 == 0 and cols % 16 == 0 and (absmax is not None or x.element_size() == 1):
-        L.check(L.kernels().llmq_quantize_transpose(None, L.ptr(out), L.ptr(scale_out), L.ptr(x), L.ptr(absmax), rows, cols,
-                                                    L.dtype_code(x.dtype), L.dtype_code(out.dtype), L.stream_ptr()), "transpose")
+        L.check(L.calls().llmq_quantize_transpose(None, out, scale_out, x, absmax, rows, cols,
+                                                  L.dtype_code(x.dtype), L.dtype_code(out.dtype)), "transpose")
         return
     if x.is_cuda:
-        L.check(L.kernels().llmq_transpose(L.ptr(out), L.ptr(scale_out), L.ptr(x), L.ptr(absmax), rows, cols, L.dtype_code(x.dtype),
-                                           L.dtype_code(out.dtype), L.stream_ptr()), "transpose")
+        L.check(L.calls().llmq_transpose(out, scale_out, x, absmax, rows, cols, L.dtype_code(x.dtype),
+                                         L.dtype_code(out.dtype)), "transpose")
         return
     if absmax is not None:
         tmp = torch.empty(rows, cols, dtype=out.dtype)
@@ -623,9 +624,8 @@ def fused_classifier(logits: torch.Tensor, losses: torch.Tensor, lse: Optional[t
     """Cross-entropy over rows of ``logits`` (rows, V): losses += lse - logit[target]; logits <- gradient in place."""
     rows, V = logits.shape
     if logits.is_cuda:
-        L.check(L.kernels().llmq_fused_classifier(L.ptr(logits), L.ptr(losses), L.ptr(lse), L.ptr(targets), _f(dloss), _f(z_reg), rows, V,
-                                                  _ll(logits.stride(0)), L.dtype_code(logits.dtype), int(write_dlogits),
-                                                  L.stream_ptr()), "fused_classifier")
+        L.check(L.calls().llmq_fused_classifier(logits, losses, lse, targets, dloss, z_reg, rows, V,
+                                                logits.stride(0), L.dtype_code(logits.dtype), int(write_dlogits)), "fused_classifier")
         return
     x = logits.float()
     tg = targets.reshape(rows).long()
@@ -688,11 +688,11 @@ def adamw(param: torch.Tensor, grad: torch.Tensor, m: torch.Tensor, v: torch.Ten
     and ``seed`` is an offset to the step's seed."""
     n = param.numel()
     if param.is_cuda:
-        L.check(L.kernels().llmq_adamw_hyper(L.ptr(param), L.ptr(grad), L.ptr(m), L.ptr(v), L.ptr(m_scales), _ll(n), _f(lr), _f(beta1),
-                                             _f(beta2), int(step), _f(eps), _f(weight_decay), L.ptr(grad_scale), L.ptr(absmax),
-                                             ctypes.c_uint(seed & 0xFFFFFFFF), _ll(elem_offset), L.dtype_code(param.dtype),
-                                             L.dtype_code(grad.dtype), L.dtype_code(m.dtype), L.dtype_code(v.dtype), num_sms(param.device),
-                                             L.ptr(hyper), L.stream_ptr()), "adamw")
+        L.check(L.calls().llmq_adamw_hyper(param, grad, m, v, m_scales, n, lr, beta1,
+                                           beta2, int(step), eps, weight_decay, grad_scale, absmax,
+                                           seed & 0xFFFFFFFF, elem_offset, L.dtype_code(param.dtype),
+                                           L.dtype_code(grad.dtype), L.dtype_code(m.dtype), L.dtype_code(v.dtype), num_sms(param.device),
+                                           hyper), "adamw")
         return
     gen = torch.Generator().manual_seed((seed * 2654435761 + elem_offset) % (2 ** 63))
     g = grad.float().reshape(-1)
@@ -797,15 +797,14 @@ NORM_PARTIALS = 512
 def norm_squared(partials: torch.Tensor, x: torch.Tensor) -> None:
     """partials[b] += partial sum of squares of x (deterministic per-block slots)."""
     if x.is_cuda:
-        L.check(L.kernels().llmq_norm_squared(L.ptr(partials), L.ptr(x), _ll(x.numel()), L.dtype_code(x.dtype), partials.numel(),
-                                              L.stream_ptr()), "norm_squared")
+        L.check(L.calls().llmq_norm_squared(partials, x, x.numel(), L.dtype_code(x.dtype), partials.numel()), "norm_squared")
         return
     partials[0] += x.float().pow(2).sum()
 
 
 def deterministic_sum(out: torch.Tensor, x: torch.Tensor) -> None:
     if x.is_cuda:
-        L.check(L.kernels().llmq_deterministic_sum(L.ptr(out), L.ptr(x), x.numel(), L.stream_ptr()), "deterministic_sum")
+        L.check(L.calls().llmq_deterministic_sum(out, x, x.numel()), "deterministic_sum")
         return
     out.copy_(x.float().sum().reshape_as(out))
 
@@ -813,7 +812,7 @@ def deterministic_sum(out: torch.Tensor, x: torch.Tensor) -> None:
 def norm_finish(io: torch.Tensor, clip: float, host_norm: Optional[torch.Tensor] = None) -> None:
     """io[0]: squared norm -> norm; io[1] <- clip multiplier (min(1, clip / norm); 0 for a non-finite norm)."""
     if io.is_cuda:
-        L.check(L.kernels().llmq_norm_finish(L.ptr(io), _f(clip), L.ptr(host_norm), L.stream_ptr()), "norm_finish")
+        L.check(L.calls().llmq_norm_finish(io, clip, host_norm), "norm_finish")
         return
     norm = io[0].sqrt()
     scale = torch.ones(())
@@ -893,9 +892,9 @@ def bias_backward(dbias: torch.Tensor, dout: torch.Tensor, scratch: Optional[tor
     if dout.is_cuda:
         slices = 64
         assert scratch is not None and scratch.numel() >= slices * C
-        L.check(L.kernels().llmq_bias_backward(L.ptr(dbias), L.ptr(scratch), L.ptr(dout), _ll(rows), C, slices, L.ptr(scale_a), L.ptr(scale_b),
-                                               int(accumulate), L.dtype_code(dout.dtype), L.dtype_code(dbias.dtype), L.stream_ptr()),
-                "bias_backward")
+        L.check(L.calls().llmq_bias_backward(dbias, scratch, dout, rows, C, slices, scale_a, scale_b,
+                                             int(accumulate), L.dtype_code(dout.dtype), L.dtype_code(dbias.dtype)),
+                                             "bias_backward")
         return
     s = dout.float().reshape(rows, C).sum(0)
     if scale_a is not None:
@@ -925,8 +924,8 @@ def attention_forward(out: torch.Tensor, lse: torch.Tensor, qkv: torch.Tensor, H
         return
     if qkv.is_cuda:
         assert qkv.dtype == torch.bfloat16 and out.dtype == torch.bfloat16
-        L.check(L.kernels().llmq_attention_forward(L.ptr(out), L.ptr(lse), L.ptr(qkv), B, T, Hq, Hkv, HS, L.ptr(absmax),
-                                                   L.ptr(status_word(qkv.device)), L.stream_ptr()), "attention_forward")
+        L.check(L.calls().llmq_attention_forward(out, lse, qkv, B, T, Hq, Hkv, HS, absmax,
+                                                 status_word(qkv.device)), "attention_forward")
         return
     o, l = _attention_ref(qkv.float(), Hq, Hkv)
     out.copy_(o.to(out.dtype))
@@ -972,8 +971,8 @@ def attention_backward(dqkv: torch.Tensor, scratch: Optional[torch.Tensor], dout
     if qkv.is_cuda:
         assert qkv.dtype == torch.bfloat16 and dqkv.dtype == torch.bfloat16
         assert scratch is not None and scratch.numel() >= B * Hq * T
-        L.check(L.kernels().llmq_attention_backward(L.ptr(dqkv), L.ptr(scratch), L.ptr(dout), L.ptr(out), L.ptr(lse), L.ptr(qkv), B, T, Hq, Hkv,
-                                                    HS, L.ptr(status_word(qkv.device)), L.stream_ptr()), "attention_backward")
+        L.check(L.calls().llmq_attention_backward(dqkv, scratch, dout, out, lse, qkv, B, T, Hq, Hkv,
+                                                  HS, status_word(qkv.device)), "attention_backward")
         return
     # written out (no autograd): this also runs below the autograd dispatch key, inside a torch custom op
     x, G = qkv.float(), Hq // Hkv

@@ -7,16 +7,21 @@ can never pass on a PyTorch fallback by accident.
 from __future__ import annotations
 
 import ctypes
+import importlib.util
 import os
 import threading
 from pathlib import Path
+from types import SimpleNamespace
 
 import torch
 
-_LIBDIR = Path(os.environ.get("LLMQ_LIB_DIR") or (Path(__file__).resolve().parent.parent / "lib"))      # LLMQ_LIB_DIR: another build of the libraries
+_PKG_LIBDIR = Path(__file__).resolve().parent.parent / "lib"
+_LIBDIR = Path(os.environ.get("LLMQ_LIB_DIR") or _PKG_LIBDIR)      # LLMQ_LIB_DIR: another build of the libraries
 _lock = threading.Lock()
 _kernels = None
 _rt = None
+_binding = None            # the extension module, False when it was not built
+_calls = None
 
 DT_BF16, DT_E4M3, DT_E5M2, DT_FP32, DT_FP16, DT_INT32, DT_INT8 = range(7)
 
@@ -56,6 +61,58 @@ def kernels():
                 lib.llmq_gemm_splitk_floats.restype = ctypes.c_longlong
                 _kernels = lib
     return _kernels
+
+
+# Arguments of the entry points in calls(), without the stream: p pointer (tensor, address or None), i int, u unsigned, l long long, f float, d double
+SIGNATURES = {
+    "llmq_gemm_ready": "ppppiiiiiiillliiippfppipuidpl", "llmq_rmsnorm_forward": "pppppppfiiippp", "llmq_rmsnorm_backward": "pppppppiiipii",
+    "llmq_swiglu_forward": "pppliipppi", "llmq_swiglu_backward": "pppliipi", "llmq_rope": "pppiiiiiiipi",
+    "llmq_attention_forward": "pppiiiiipp", "llmq_attention_backward": "ppppppiiiiip", "llmq_bias_backward": "pppliippiii", "llmq_abs_max": "pplii",
+    "llmq_quantize": "ppppliii", "llmq_quantize_transpose": "pppppiiii", "llmq_transpose": "ppppiiii", "llmq_fused_classifier": "ppppffiilii",
+    "llmq_norm_squared": "pplii", "llmq_deterministic_sum": "ppi", "llmq_norm_finish": "pfp", "llmq_adamw_hyper": "ppppplfffiffppuliiiiip",
+}
+_CTYPES = {"p": ctypes.c_void_p, "i": ctypes.c_int, "u": ctypes.c_uint, "l": ctypes.c_longlong, "f": ctypes.c_float, "d": ctypes.c_double}
+
+
+def binding():
+    """The extension module of ``csrc/py/binding.cpp``, or None where it was not built (it needs the headers of torch and Python)."""
+    global _binding
+    if _binding is None:
+        with _lock:
+            if _binding is None:
+                found = False
+                for path in (_LIBDIR / "llmq_b200_binding.so", _PKG_LIBDIR / "llmq_b200_binding.so"):
+                    if path.exists():
+                        spec = importlib.util.spec_from_file_location("llmq_b200_binding", path)
+                        found = importlib.util.module_from_spec(spec)
+                        spec.loader.exec_module(found)
+                        break
+                _binding = found
+    return _binding or None
+
+
+def _through_ctypes(fn, codes):
+    fn.argtypes = [_CTYPES[c] for c in codes] + [ctypes.c_void_p]
+    take = [{"p": lambda a: a.data_ptr() if isinstance(a, torch.Tensor) else a, "f": float, "d": float}.get(c, int) for c in codes]
+
+    def call(*args):
+        return fn(*[t(a) for t, a in zip(take, args, strict=True)], raw_stream())
+    return call
+
+
+def calls():
+    """The entry points of SIGNATURES as functions of tensors and numbers that launch on the current stream and return the C function's code:
+    those of :func:`binding`, or slower ones of the same kernels through ctypes."""
+    global _calls
+    if _calls is None:
+        lib, b = kernels(), binding()
+        if b is not None:
+            for name in SIGNATURES:
+                b.bind(name, ctypes.cast(getattr(lib, name), ctypes.c_void_p).value)
+            _calls = b
+        else:
+            _calls = SimpleNamespace(**{name: _through_ctypes(getattr(lib, name), codes) for name, codes in SIGNATURES.items()})
+    return _calls
 
 
 def runtime():
