@@ -19,44 +19,62 @@ namespace {
 typedef void* P;               // tensor, address or None
 typedef long long LL;
 
+// get(): the C value; with an exception set, ok becomes false
 template <typename T> struct Arg;
 template <> struct Arg<P> {
     static constexpr char code = 'p';
-    static P get(PyObject* o) {
+    static P get(PyObject* o, bool& ok) {
         if (o == Py_None) return nullptr;
         if (THPVariable_Check(o)) return THPVariable_Unpack(o).data_ptr();
-        if (PyLong_Check(o)) return PyLong_AsVoidPtr(o);
+        if (PyLong_Check(o)) {
+            P v = PyLong_AsVoidPtr(o);
+            ok = v || !PyErr_Occurred();
+            return v;
+        }
+        ok = false;
         PyErr_Format(PyExc_TypeError, "expected a tensor, an address or None, got %s", Py_TYPE(o)->tp_name);
         return nullptr;
     }
 };
 template <> struct Arg<int> {
     static constexpr char code = 'i';
-    static int get(PyObject* o) {
+    static int get(PyObject* o, bool& ok) {
         const long v = PyLong_AsLong(o);
-        if (v < INT_MIN || v > INT_MAX) PyErr_SetString(PyExc_OverflowError, "size does not fit a C int");
+        if (v == -1) ok = !PyErr_Occurred();
+        if (v < INT_MIN || v > INT_MAX) { ok = false; PyErr_SetString(PyExc_OverflowError, "size does not fit a C int"); }
         return static_cast<int>(v);
     }
 };
 template <> struct Arg<unsigned int> {
     static constexpr char code = 'u';
-    static unsigned int get(PyObject* o) {
+    static unsigned int get(PyObject* o, bool& ok) {
         const unsigned long v = PyLong_AsUnsignedLong(o);
-        if (v > UINT_MAX && !PyErr_Occurred()) PyErr_SetString(PyExc_OverflowError, "value does not fit an unsigned C int");
+        if (v > UINT_MAX) {                                  // also where the conversion failed
+            ok = false;
+            if (!PyErr_Occurred()) PyErr_SetString(PyExc_OverflowError, "value does not fit an unsigned C int");
+        }
         return static_cast<unsigned int>(v);
     }
 };
 template <> struct Arg<LL> {
     static constexpr char code = 'l';
-    static LL get(PyObject* o) { return PyLong_AsLongLong(o); }
-};
-template <> struct Arg<float> {
-    static constexpr char code = 'f';
-    static float get(PyObject* o) { return static_cast<float>(PyFloat_AsDouble(o)); }
+    static LL get(PyObject* o, bool& ok) {
+        const LL v = PyLong_AsLongLong(o);
+        if (v == -1) ok = !PyErr_Occurred();
+        return v;
+    }
 };
 template <> struct Arg<double> {
     static constexpr char code = 'd';
-    static double get(PyObject* o) { return PyFloat_AsDouble(o); }
+    static double get(PyObject* o, bool& ok) {
+        const double v = PyFloat_AsDouble(o);
+        if (v == -1.) ok = !PyErr_Occurred();
+        return v;
+    }
+};
+template <> struct Arg<float> {
+    static constexpr char code = 'f';
+    static float get(PyObject* o, bool& ok) { return static_cast<float>(Arg<double>::get(o, ok)); }
 };
 
 template <int Id, typename... A>
@@ -74,8 +92,9 @@ struct Entry {
     template <size_t... I>
     static PyObject* invoke(PyObject* const* args, std::index_sequence<I...>) {
         try {
-            std::tuple<A...> v{Arg<A>::get(args[I])...};
-            if (PyErr_Occurred()) return nullptr;
+            bool ok = true;
+            std::tuple<A...> v{(ok ? Arg<A>::get(args[I], ok) : A())...};      // in order, up to the first that fails
+            if (!ok) return nullptr;
             const cudaStream_t stream = c10::cuda::getCurrentCUDAStream().stream();
             int rc;
             Py_BEGIN_ALLOW_THREADS
