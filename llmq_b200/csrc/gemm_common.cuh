@@ -67,7 +67,7 @@ struct GemmParams {
     int early_release;
     // CTA-pair kernel: tile rows (256 rows of A each) that are worked through together, column tile by column tile
     int group_rows;
-    // 1: C is bf16 with rows of whole aligned 32-byte sectors and the epilogue moves them lane by lane (store_sector)
+    // 1: C is bf16 with rows of whole aligned 32-byte sectors and the epilogue writes them lane by lane (store_sector)
     int c_sectors;
 };
 
@@ -104,18 +104,13 @@ __device__ __forceinline__ void add_bias32(const GemmParams& p, int col0, float 
 constexpr int EPI_STAGE_BYTES_PER_WARP = 32 * 128;
 
 // 32 bytes (16 bf16) of one row per lane: a whole sector per lane and instruction
-__device__ __forceinline__ void load_sector(const void* p, uint32_t (&r)[8]) {
-    asm volatile("ld.global.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]) : "l"(p) : "memory");
-}
 __device__ __forceinline__ void store_sector(void* p, const uint32_t* r) {
     asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};"
                  ::"l"(p), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]) : "memory");
 }
 
-// bf16 C in whole sectors (GemmParams::c_sectors), with or without its previous values: lane = row, 32 columns at a time.  A lane that moves
-// 16 bytes at a time touches every sector twice; adding to C that way 16384 x 3584 x 3584 took 310 us in bf16 and 240 us in e4m3, in whole sectors
-// 287 and 163 (plain: 275 and 145).  Plain outputs of the CTA-pair kernel stay on the staged TMA stores: 4096 x 151936 x 896 824 us, 837 this way.
+// bf16 C in whole sectors (GemmParams::c_sectors), not added to: lane = row, 32 columns at a time.  A lane that moves 16 bytes at a time touches every sector
+// twice.  Plain outputs of the CTA-pair kernel stay on the staged TMA stores: 4096 x 151936 x 896 824 us, 837 this way.
 __device__ __forceinline__ void epilogue_rows_sectors(const GemmParams& p, uint32_t t_row, int row, int col_base, int ncols, float alpha, float& tmax) {
     using namespace sm100;
     const bool row_ok = row < p.M;
@@ -125,21 +120,13 @@ __device__ __forceinline__ void epilogue_rows_sectors(const GemmParams& p, uint3
         const int col0 = col_base + c;
         if (col0 >= p.N) break;                    // uniform across the warp
         const int halves = col0 + 32 <= p.N ? 2 : 1;                // N is a multiple of 16
-        uint32_t r[32], old[2][8] = {};
+        uint32_t r[32];
         tmem_ld_32x32b_x32(t_row + c, r);
-        if (p.accumulate && row_ok) {
-#pragma unroll
-            for (int h = 0; h < 2; ++h) if (h < halves) load_sector(crow + col0 + 16 * h, old[h]);
-        }
         tmem_ld_wait();
         float v[32];
 #pragma unroll
         for (int j = 0; j < 32; ++j) v[j] = __uint_as_float(r[j]) * alpha;
         if (p.bias) add_bias32(p, col0, v);
-        if (p.accumulate) {
-#pragma unroll
-            for (int j = 0; j < 32; ++j) v[j] += __uint_as_float((j & 1) ? old[j / 16][(j % 16) / 2] & 0xffff0000u : old[j / 16][(j % 16) / 2] << 16);
-        }
         if (p.absmax_out && row_ok) {
 #pragma unroll
             for (int j = 0; j < 32; ++j) if (j < 16 * halves) tmax = fmaxf(tmax, fabsf(v[j]));
@@ -153,6 +140,118 @@ __device__ __forceinline__ void epilogue_rows_sectors(const GemmParams& p, uint3
         if (row_ok) {
 #pragma unroll
             for (int h = 0; h < 2; ++h) if (h < halves) store_sector(crow + col0 + 16 * h, packed + 8 * h);
+        }
+    }
+}
+
+// The previous values of a bf16 C that is added to, for one epilogue warp: blocks of 32 rows x 64 columns, in the order in which the warp works on them, are copied into
+// its two staging buffers (128 bytes a row, 16-byte pieces at piece ^ (row % 8)) two blocks ahead, across the tiles.  Eight lanes copy a row's 128
+// bytes.  Sectors read by the lane whose row they are, 32 rows at once, hold the memory to a third of its rate: 37888 x 3584 added to with K = 64 to 1024
+// 210-270 us, 125-190 this way (add_ in place 83);  27648 x 5120 x 576 e4m3 253 / 142 (of which 177 / 142 by the one-CTA kernel), 7168 x 5120 x 832 70 / 42, 17920 x 1536 x 1024
+// 51 / 34, 5120 x 5120 x 759 bf16 51 / 39.
+constexpr int OLD_BLOCK_BYTES = 32 * 128;
+template <typename Origin>
+struct OldBlocks {
+    const GemmParams& p;
+    const Origin origin;           // tile number -> first row of the warp's 32, first column
+    uint8_t* const stage;          // 2 x OLD_BLOCK_BYTES
+    const int stride, num_tiles, ncols;
+    int t, c = 0, row_base = 0, col_base = 0;
+    uint32_t fetched = 0, used = 0;
+
+    __device__ __forceinline__ OldBlocks(const GemmParams& p, const Origin& origin, uint8_t* stage, int first, int stride, int num_tiles, int ncols)
+        : p(p), origin(origin), stage(stage), stride(stride), num_tiles(num_tiles), ncols(ncols), t(first) {
+        if (t < num_tiles) origin(t, row_base, col_base);
+        fetch();
+        fetch();
+    }
+    // starts the copy of the next block; a group per block, empty behind the last one
+    __device__ __forceinline__ void fetch() {
+        if (t < num_tiles) {
+            const int lane = threadIdx.x & 31, sub = lane >> 3, ch = lane & 7, col = col_base + c + ch * 8;
+            const uint32_t buf = smem_addr(fetched & 1);
+            if (col < p.N && c + ch * 8 < ncols) {
+#pragma unroll
+                for (int j = 0; j < 8; ++j) {
+                    const int r = 4 * j + sub;
+                    if (row_base + r < p.M)
+                        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(buf + r * 128 + ((ch ^ (r & 7)) << 4)),
+                                     "l"(static_cast<const __nv_bfloat16*>(p.C) + static_cast<long long>(row_base + r) * p.ldc + col) : "memory");
+                }
+            }
+            c += 64;
+            if (c >= ncols || col_base + c >= p.N) {
+                c = 0;
+                t += stride;
+                if (t < num_tiles) origin(t, row_base, col_base);
+            }
+        }
+        ++fetched;
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    }
+    // this lane's row of the next block in order; the block after the next one is on its way then
+    __device__ __forceinline__ void take(uint32_t (&old)[32]) {
+        asm volatile("cp.async.wait_group 1;" ::: "memory");
+        __syncwarp();
+        const int lane = threadIdx.x & 31;
+        const uint32_t buf = smem_addr(used & 1);
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+            asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(old[4 * i]), "=r"(old[4 * i + 1]), "=r"(old[4 * i + 2]), "=r"(old[4 * i + 3])
+                         : "r"(buf + lane * 128 + ((i ^ (lane & 7)) << 4)) : "memory");
+        __syncwarp();
+        ++used;
+        fetch();
+    }
+    // copies that nobody took, where a wait ran out
+    __device__ __forceinline__ void drain() const { asm volatile("cp.async.wait_all;" ::: "memory"); }
+    __device__ __forceinline__ uint32_t smem_addr(uint32_t i) const { return sm100::smem_u32(stage) + i * OLD_BLOCK_BYTES; }
+};
+
+struct NoOldBlocks {
+    template <typename... A>
+    __device__ __forceinline__ NoOldBlocks(const A&...) {}
+};
+
+// bf16 C that is added to (GemmParams::c_sectors and accumulate): lane = row, 64 columns at a time
+template <typename Old>
+__device__ __forceinline__ void epilogue_rows_added(const GemmParams& p, uint32_t t_row, int row, int col_base, int ncols, float alpha, float& tmax, Old& blocks) {
+    using namespace sm100;
+    const bool row_ok = row < p.M;
+    __nv_bfloat16* crow = static_cast<__nv_bfloat16*>(p.C) + static_cast<long long>(row) * p.ldc;
+#pragma unroll 1
+    for (int c = 0; c < ncols; c += 64) {
+        const int col0 = col_base + c;
+        if (col0 >= p.N) break;                    // uniform across the warp
+        const int cols = min(min(64, ncols - c), p.N - col0);       // a multiple of 16
+        uint32_t r[2][32], old[32];
+        tmem_ld_32x32b_x32(t_row + c, r[0]);
+        if (cols > 32) tmem_ld_32x32b_x32(t_row + c + 32, r[1]);
+        blocks.take(old);
+        tmem_ld_wait();
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            if (32 * h >= cols) break;             // uniform
+            float v[32];
+#pragma unroll
+            for (int j = 0; j < 32; ++j) v[j] = __uint_as_float(r[h][j]) * alpha;
+            if (p.bias) add_bias32(p, col0 + 32 * h, v);
+#pragma unroll
+            for (int j = 0; j < 32; ++j) v[j] += __uint_as_float((j & 1) ? old[16 * h + j / 2] & 0xffff0000u : old[16 * h + j / 2] << 16);
+            if (p.absmax_out && row_ok) {
+#pragma unroll
+                for (int j = 0; j < 32; ++j) if (32 * h + j < cols) tmax = fmaxf(tmax, fabsf(v[j]));
+            }
+            uint32_t packed[16];
+#pragma unroll
+            for (int j = 0; j < 16; ++j) {
+                __nv_bfloat162 b = __floats2bfloat162_rn(v[2 * j], v[2 * j + 1]);
+                packed[j] = *reinterpret_cast<uint32_t*>(&b);
+            }
+            if (row_ok) {
+#pragma unroll
+                for (int k = 0; k < 2; ++k) if (32 * h + 16 * k < cols) store_sector(crow + col0 + 32 * h + 16 * k, packed + 8 * k);
+            }
         }
     }
 }
@@ -173,7 +272,7 @@ __device__ __forceinline__ void epilogue_rows(const GemmParams& p, uint32_t t_ro
                                               float alpha, float& tmax, __nv_bfloat16* dst_row = nullptr, uint8_t* stage = nullptr,
                                               const CUtensorMap* tmap_c = nullptr, int* stage_sel = nullptr) {
     using namespace sm100;
-    if (p.c_sectors && dst_row == nullptr) { epilogue_rows_sectors(p, t_row, row, col_base, ncols, alpha, tmax); return; }
+    if (p.c_sectors && !p.accumulate && dst_row == nullptr) { epilogue_rows_sectors(p, t_row, row, col_base, ncols, alpha, tmax); return; }
     const bool row_ok = row < p.M;
     // (`dst_row` redirection: the rows of one warp are consecutive rows of the same landing slot, N elements apart)
     const int lane_id = threadIdx.x & 31;

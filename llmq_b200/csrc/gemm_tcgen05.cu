@@ -20,6 +20,7 @@
 //   warps 2-5  epilogue: tcgen05.ld the finished accumulator (while the other one is being
 //              computed), scale, add bias, optionally add the previous C, track abs-max, store
 // Outputs with few tiles and a long K cut the K loop; the parts of a tile are summed by the CTAs of a cluster or by a second kernel.
+#include <type_traits>
 #include "ptx_sm100.cuh"
 #include "api.h"
 #include "common.cuh"
@@ -40,6 +41,10 @@ template <int BN> struct Tile {
     static constexpr int STAGE_BYTES = A_STAGE_BYTES + B_STAGE_BYTES;
     static constexpr int TMEM_COLS = 2 * BN;
     static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 1024 /*alignment slack*/ + 256 /*barriers*/;
+    // outputs that are added to: two blocks of previous values of C per epilogue warp behind the barriers.  Only then, since a kernel that is launched
+    // early starts sooner the less shared memory is taken (the second kernel of a cut K loop: 1152 x 896 x 4096 23.4 us, 22.5 without).
+    static constexpr int OLD_OFFSET = STAGES * STAGE_BYTES + 256;
+    static constexpr int SMEM_BYTES_ADDED = SMEM_BYTES + 4 * 2 * OLD_BLOCK_BYTES;
 };
 
 
@@ -123,13 +128,16 @@ __device__ __forceinline__ void cluster_reduce(const GemmParams& p, uint32_t sme
 }
 
 // Kind: MMA kind of ptx_sm100.cuh's mma_issue (0 bf16, 1 8-bit floats, 2 tf32 on fp32 operands).
-// Cluster: the CTAs of a cluster are the K parts of one tile (grid = tiles x parts, one work item per CTA).
-template <int Kind, int BN, bool Cluster>
+// Mode: kCluster, the CTAs of a cluster are the K parts of one tile (grid = tiles x parts, one work item per CTA); kAdded, a bf16 C that is added to, in
+// whole sectors (GemmParams::c_sectors).
+enum { kPlain, kCluster, kAdded };
+template <int Kind, int BN, int Mode>
 __global__ void __launch_bounds__(NUM_THREADS, 1)
 gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
                     const GemmParams p) {
     constexpr int STAGES = Tile<BN>::STAGES, B_STAGE_BYTES = Tile<BN>::B_STAGE_BYTES, STAGE_BYTES = Tile<BN>::STAGE_BYTES;
     constexpr int TMEM_COLS = Tile<BN>::TMEM_COLS;
+    constexpr bool Cluster = Mode == kCluster, Added = Mode == kAdded;
     extern __shared__ uint8_t smem_raw[];
     // 128B-swizzled tiles must start on a 1024-byte boundary
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -270,12 +278,20 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
         float tmax = 0.f;
         int acc = 0; uint32_t acc_phase = 0;
         bool ok = true;
+        auto origin = [&](int t, int& row, int& col) {
+            int tm, tn; tile_coords(t, tiles_m, tiles_n, tm, tn);
+            row = tm * BM + q * 32;
+            col = tn * BN;
+        };
+        std::conditional_t<Added, OldBlocks<decltype(origin)>, NoOldBlocks> old(p, origin, smem + Tile<BN>::OLD_OFFSET + q * 2 * OLD_BLOCK_BYTES, after_wait(blockIdx.x),
+                                                                                gridDim.x, num_tiles, BN);
         for (int t = after_wait(blockIdx.x); t < num_tiles && ok; t += gridDim.x) {
             int tm, tn; tile_coords(t / splits, tiles_m, tiles_n, tm, tn);
             if (!mbar_wait(tfull_bar(acc), acc_phase, abort_flag)) { if (lane == 0) atomicOr(p.status, kErrTmemFull); ok = false; break; }
             tc_fence_after_sync();
             const uint32_t t_row = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + acc * BN;
-            if constexpr (Cluster) {
+            if constexpr (Added) epilogue_rows_added(p, t_row, tm * BM + q * 32 + lane, tn * BN, BN, alpha, tmax, old);
+            else if constexpr (Cluster) {
                 uint8_t* const mine = smem + (q * 32 + lane) * (BN * 4);
 #pragma unroll 1
                 for (int c = 0; c < BN; c += 32) {
@@ -288,11 +304,12 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
                 }
             }
             else if (splits > 1) epilogue_rows_partial(p, t_row, tm * BM + q * 32 + lane, tn * BN, BN, t % splits);
-            else            epilogue_rows(p, t_row, tm * BM + q * 32 + lane, tn * BN, BN, alpha, tmax);
+            else             epilogue_rows(p, t_row, tm * BM + q * 32 + lane, tn * BN, BN, alpha, tmax);
             tc_fence_before_sync();
             mbar_arrive(tempty_bar(acc));                  // 128 arrivals release the accumulator
             if (++acc == 2) { acc = 0; acc_phase ^= 1u; }
         }
+        if constexpr (Added) old.drain();
         if (!Cluster && p.absmax_out) {
             tmax = warp_reduce_max(tmax);
             if (lane == 0 && tmax > 0.f) atomic_max_float(p.absmax_out, tmax);
@@ -403,17 +420,21 @@ __global__ void __launch_bounds__(256) splitk_reduce_vec_kernel(const GemmParams
 template <int Kind, int BN>
 int launch_one_cta(const CUtensorMap& ta, const CUtensorMap& tb, const GemmParams& p, int items, bool cluster, int num_sms, cudaStream_t stream) {
     static bool attr_set[64] = {};          // the attribute is per device
-    constexpr int smem = Tile<BN>::SMEM_BYTES;
+    constexpr int smem = Tile<BN>::SMEM_BYTES, smem_added = Tile<BN>::SMEM_BYTES_ADDED;
     int dev = 0;
     cudaGetDevice(&dev);
     if (!attr_set[dev & 63]) {
-        cudaError_t e = cudaFuncSetAttribute(gemm_tcgen05_kernel<Kind, BN, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-        if (e == cudaSuccess) e = cudaFuncSetAttribute(gemm_tcgen05_kernel<Kind, BN, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+        const cudaFuncAttribute at = cudaFuncAttributeMaxDynamicSharedMemorySize;
+        cudaError_t e = cudaFuncSetAttribute(gemm_tcgen05_kernel<Kind, BN, kPlain>, at, smem);
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(gemm_tcgen05_kernel<Kind, BN, kCluster>, at, smem);
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(gemm_tcgen05_kernel<Kind, BN, kAdded>, at, smem_added);
         if (e != cudaSuccess) return static_cast<int>(e);
         attr_set[dev & 63] = true;
     }
-    if (cluster) launch_chained_cluster(gemm_tcgen05_kernel<Kind, BN, true>, items, NUM_THREADS, smem, stream, p.k_splits, ta, tb, p);
-    else         launch_chained(gemm_tcgen05_kernel<Kind, BN, false>, items < num_sms ? items : num_sms, NUM_THREADS, smem, stream, ta, tb, p);
+    const int grid = items < num_sms ? items : num_sms;
+    if (cluster) launch_chained_cluster(gemm_tcgen05_kernel<Kind, BN, kCluster>, items, NUM_THREADS, smem, stream, p.k_splits, ta, tb, p);
+    else if (p.accumulate && p.c_sectors && p.k_splits <= 1) launch_chained(gemm_tcgen05_kernel<Kind, BN, kAdded>, grid, NUM_THREADS, smem_added, stream, ta, tb, p);
+    else         launch_chained(gemm_tcgen05_kernel<Kind, BN, kPlain>, grid, NUM_THREADS, smem, stream, ta, tb, p);
     return LLMQ_LAUNCH_CHECK();
 }
 
@@ -425,7 +446,7 @@ int resident_clusters(int parts) {
     int& n = known[dev & 63][parts];
     if (n > 0) return n;
     constexpr int smem = Tile<256>::SMEM_BYTES;
-    if (cudaFuncSetAttribute(gemm_tcgen05_kernel<0, 256, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) { cudaGetLastError(); return 0; }
+    if (cudaFuncSetAttribute(gemm_tcgen05_kernel<0, 256, kCluster>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) { cudaGetLastError(); return 0; }
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = 64 * parts; cfg.blockDim = NUM_THREADS; cfg.dynamicSmemBytes = smem;
     cudaLaunchAttribute attr[1]{};
@@ -433,7 +454,7 @@ int resident_clusters(int parts) {
     attr[0].val.clusterDim.x = parts; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
     cfg.attrs = attr; cfg.numAttrs = 1;
     int found = 0;
-    if (cudaOccupancyMaxActiveClusters(&found, gemm_tcgen05_kernel<0, 256, true>, &cfg) != cudaSuccess) { cudaGetLastError(); return 0; }
+    if (cudaOccupancyMaxActiveClusters(&found, gemm_tcgen05_kernel<0, 256, kCluster>, &cfg) != cudaSuccess) { cudaGetLastError(); return 0; }
     return n = found;
 }
 
@@ -514,12 +535,28 @@ static long long tiles_of(int M, int N, int bm, int bn) { return static_cast<lon
 // most of the last round idle: 896 x 4864 x 4096, both operands MN-major, is 76 pair tiles (two rounds of 74, 48.5 us) or 133 of the others
 // (one round of 148, 36.4 us); with equally many rounds 16384 x 4608 x 3584 351 / 388 us, 4096 x 896 x 9728 60.8 / 66.4, 4096 x 4864 x 896
 // 33.7 / 40.6.  With that many tiles the one-CTA kernel does not cut the K loop, so the sums have the same bits.
-static bool uses_pair_kernel(int M, int N, int elem_bytes, bool fused, int num_sms) {
+// Where they leave half of the GPU idle, with 48 or more K steps of 128 bytes, the one-CTA kernel in two K parts wins, pairs / parts in us: 1062 x 2048 x 3072 bf16 22 / 20,
+// x 8192 46 / 33;  614 x 3584 x 12288 both MN-major 85 / 55;  1536 x 1536 x 8192 e4m3 26 / 23;  with 32 steps 17.4 / 17.5, with 16 12.7 / 14.8.
+static bool uses_pair_kernel(int M, int N, int K, int elem_bytes, bool fused, int num_sms) {
     if (elem_bytes == 4) return false;
     if (fused || g_gemm_mode == 2) return true;
     if (g_gemm_mode != 0 || M < 256 || static_cast<long long>(M) * N < 256LL * 256 * 32) return false;
+    if (2 * tiles_of(M, N, 128, 256) <= num_sms && K > 47 * (128 / elem_bytes)) return false;
     const long long pair = waves(tiles_of(M, N, 256, 256), num_sms / 2);
     return pair < 2 || 5 * waves(tiles_of(M, N, 128, 256), num_sms) >= 4 * pair;
+}
+
+// GEMMs of that many tiles that the one-CTA kernel is better at all the same.  Short K: what bounds them is the output, which its epilogue writes (and, where it is
+// added to, reads) straight from the accumulators while a tile of a pair has twice the rows to drain before its successor.  Up to 8 K steps of 128 bytes it takes 0.75 to 0.98 of the
+// pairs' time, one / pair tiles in us: 37888 x 3584 x 256 bf16 88 / 103, added to 130 / 165;  9728 x 896 x 512 0.88;  37888 x 3584 x 512 both MN-major 1.01;  with 10 steps 0.96
+// (both MN-major 1.05), with 12 1.02 (1.10).  And one round of tiles on all SMs with up to 64 K steps, 16 with both operands MN-major: a pair starts later than
+// a CTA, 2976 x 1536 x 1536 13.6 / 16.1, 1232 x 2048 x 2048 e4m3 10.4 / 11.9, 1960 x 2048 x 2048 15.5 / 17.1;  longer walks are bound by the loads, of which a pair has fewer:
+// 743 x 5120 x 13824 92 / 80, 2048 x 2048 x 4746 both MN-major 37 / 31.  Neither cuts K, so the sums have the same bits.
+static bool better_with_one_cta(int M, int N, int K, int elem_bytes, bool both_mn, int num_sms) {
+    if (g_gemm_mode != 0) return false;
+    const int bk = 128 / elem_bytes, k_iters = (K + bk - 1) / bk;
+    const long long tiles = tiles_of(M, N, 128, 256);
+    return k_iters <= 8 || (tiles <= num_sms && 2 * tiles > num_sms && k_iters <= (both_mn ? 16 : 64));
 }
 
 // Tile rows of 256 that the pair kernel works through together.  B is read from memory once per group, so a group is as large as its rows of A
@@ -566,7 +603,7 @@ static int splitk_parts(int M, int N, int K, int elem_bytes, int num_sms) {
 
 // Floats of the workspace with which a plain GEMM of this shape (A and B of `elem_bytes` an element) cuts its K loop; 0: it does not.
 extern "C" long long llmq_gemm_splitk_floats(int M, int N, int K, int elem_bytes, int num_sms) {
-    if (M <= 0 || N <= 0 || K <= 0 || elem_bytes <= 0 || uses_pair_kernel(M, N, elem_bytes, false, num_sms)) return 0;
+    if (M <= 0 || N <= 0 || K <= 0 || elem_bytes <= 0 || uses_pair_kernel(M, N, K, elem_bytes, false, num_sms)) return 0;
     const int parts = splitk_parts(M, N, K, elem_bytes, num_sms);
     return parts > 1 ? static_cast<long long>(parts) * M * N : 0;
 }
@@ -663,7 +700,8 @@ static int gemm_impl(const void* A, const void* B, void* C, const void* bias,
     const int bk = 128 / eb;
     int rc;
     // The CTA-pair kernel stages 128 rows of B per CTA; the one-CTA kernel stages all 256.
-    const bool pair_kernel = uses_pair_kernel(M, N, eb, rs != nullptr || ready_flags != nullptr, num_sms);
+    const bool fused = rs != nullptr || ready_flags != nullptr;
+    const bool pair_kernel = uses_pair_kernel(M, N, K, eb, fused, num_sms) && (fused || !better_with_one_cta(M, N, K, eb, a_mn_major && b_mn_major, num_sms));
     // An MN-major stage that is several 128-byte chunks wide (16-bit operands; the 256 rows of B of the one-CTA kernel) is fetched with
     // one 3-D load instead of one 2-D load per chunk: the loads of a stage were issued one after the other for longer than its MMAs
     // run.  bf16, CTA pairs, TFLOP/s with 2-D loads / 3-D loads / 3-D loads and a K loop per kind of load (gemm_tcgen05_2cta.cu), K-major

@@ -56,7 +56,9 @@ __device__ __forceinline__ void tile_coords(int t, int tiles_m, int tiles_n, int
     tn = r / gsz;
 }
 
-template <bool F8>
+// Added: a bf16 C that is added to, in whole sectors (GemmParams::c_sectors).  An instance of its own: in one kernel the other outputs took 1 to 2 % longer
+// (16384 x 37888 x 3584 e4m3 1441 / 1460 us).
+template <bool F8, bool Added>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(NUM_THREADS, 1)
 gemm_tcgen05_2cta_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
                          const __grid_constant__ CUtensorMap tmap_c, const GemmParams p) {
@@ -230,6 +232,12 @@ gemm_tcgen05_2cta_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gri
         float tmax = 0.f;
         int acc = 0; uint32_t acc_phase = 0;
         bool ok = true;
+        auto origin = [&](int t, int& row, int& col) {
+            int tm, tn; tile_coords(t, tiles_m, tiles_n, rot, p.group_rows, tm, tn);
+            row = (tm * 2 + static_cast<int>(rank)) * BM + q * 32;
+            col = tn * bn;
+        };
+        std::conditional_t<Added, OldBlocks<decltype(origin)>, NoOldBlocks> old(p, origin, stage, after_wait(pair), num_pairs, num_tiles, bn);
         for (int t = after_wait(pair); t < num_tiles && ok; t += num_pairs) {
             int tm, tn; tile_coords(t, tiles_m, tiles_n, rot, p.group_rows, tm, tn);
             if (!mbar_wait(tfull_bar(acc), acc_phase, abort_flag)) { if (lane == 0) atomicOr(p.status, kErrTmemFull); ok = false; break; }
@@ -244,7 +252,8 @@ gemm_tcgen05_2cta_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gri
                 dst_row = static_cast<__nv_bfloat16*>(p.rs_landing[owner]) + slot_row * p.N;
             }
             const uint32_t t_row = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + acc * BN_MAX;
-            if (p.ep_mode == 1)      epilogue_rows_swiglu_fwd(p, t_row, row, tn * BN_HALF, alpha, tmax);
+            if constexpr (Added) epilogue_rows_added(p, t_row, row, tn * bn, bn, alpha, tmax, old);
+            else if (p.ep_mode == 1) epilogue_rows_swiglu_fwd(p, t_row, row, tn * BN_HALF, alpha, tmax);
             else if (p.ep_mode == 2) epilogue_rows_swiglu_bwd(p, t_row, row, tn * bn, bn, alpha, tmax);
             else                     epilogue_rows(p, t_row, row, tn * bn, bn, alpha, tmax, dst_row, stage, &tmap_c, &stage_sel);
             tc_fence_before_sync();
@@ -317,6 +326,7 @@ gemm_tcgen05_2cta_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gri
             tmax = warp_reduce_max(tmax);
             if (lane == 0 && tmax > 0.f) atomic_max_float(p.absmax_out, tmax);
         }
+        if constexpr (Added) old.drain();
         if (p.c_tma && lane == 0) tma_store_wait<0>();          // the staged blocks have left shared memory and are written
     }
 
@@ -338,15 +348,24 @@ int llmq_gemm_2cta_launch(const CUtensorMap& ta, const CUtensorMap& tb, const CU
     int dev = 0;
     cudaGetDevice(&dev);
     if (!attr_set[dev & 63]) {
-        cudaError_t e = cudaFuncSetAttribute(gemm_tcgen05_2cta_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
-        if (e == cudaSuccess) e = cudaFuncSetAttribute(gemm_tcgen05_2cta_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
+        const cudaFuncAttribute at = cudaFuncAttributeMaxDynamicSharedMemorySize;
+        cudaError_t e = cudaFuncSetAttribute(gemm_tcgen05_2cta_kernel<true, false>, at, SMEM_BYTES);
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(gemm_tcgen05_2cta_kernel<false, false>, at, SMEM_BYTES);
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(gemm_tcgen05_2cta_kernel<true, true>, at, SMEM_BYTES);
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(gemm_tcgen05_2cta_kernel<false, true>, at, SMEM_BYTES);
         if (e != cudaSuccess) return static_cast<int>(e);
         attr_set[dev & 63] = true;
     }
     const int tiles = ((p.M + 2 * BM - 1) / (2 * BM)) * (p.ep_mode == 1 ? (p.ep_D + BN_HALF - 1) / BN_HALF : (p.N + p.bn - 1) / p.bn);
     int pairs = num_sms / 2;
     if (tiles < pairs) pairs = tiles;
-    if (p.elem_bytes == 1) launch_chained(gemm_tcgen05_2cta_kernel<true>, 2 * pairs, NUM_THREADS, SMEM_BYTES, stream, ta, tb, tc, p);
-    else                   launch_chained(gemm_tcgen05_2cta_kernel<false>, 2 * pairs, NUM_THREADS, SMEM_BYTES, stream, ta, tb, tc, p);
+    const bool added = p.c_sectors && p.accumulate;
+    if (p.elem_bytes == 1) {
+        if (added) launch_chained(gemm_tcgen05_2cta_kernel<true, true>, 2 * pairs, NUM_THREADS, SMEM_BYTES, stream, ta, tb, tc, p);
+        else       launch_chained(gemm_tcgen05_2cta_kernel<true, false>, 2 * pairs, NUM_THREADS, SMEM_BYTES, stream, ta, tb, tc, p);
+    } else {
+        if (added) launch_chained(gemm_tcgen05_2cta_kernel<false, true>, 2 * pairs, NUM_THREADS, SMEM_BYTES, stream, ta, tb, tc, p);
+        else       launch_chained(gemm_tcgen05_2cta_kernel<false, false>, 2 * pairs, NUM_THREADS, SMEM_BYTES, stream, ta, tb, tc, p);
+    }
     return static_cast<int>(cudaGetLastError());
 }

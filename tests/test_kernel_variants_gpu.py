@@ -352,6 +352,56 @@ def test_split_k_parts(M, N, Kd, parts, dt, out_dt):
     assert abs(am.item() - want.abs().max().item()) < 4e-3 * want.abs().max().item()
 
 
+# the kernel for a plain GEMM on both sides of each line of the rule: short K (8 and 9 steps of 128 bytes), one round of tiles (64 / 65 steps, both operands MN-major
+# 16 / 17), more than half of the SMs idle (47 / 48 steps, from where K is cut in two); odd edges of the last tiles
+@pytest.mark.parametrize("M,N,steps,mn,parts", [(9728, 904, 8, 0, 1), (9728, 904, 9, 0, 1), (2320, 1160, 64, 0, 1), (2320, 1160, 65, 0, 1), (2056, 2064, 16, 1, 1),
+                                                (2056, 2064, 17, 1, 1), (1064, 2040, 47, 0, 1), (1064, 2040, 48, 0, 2)])
+@pytest.mark.parametrize("dt", [BF, F8])
+def test_gemm_kernel_choice(M, N, steps, mn, parts, dt):
+    lib, step = L.kernels(), 128 // dt.itemsize
+    Kd = steps * step - 8 * (2 // dt.itemsize)                # the last step is not whole
+    if mn and dt == F8:
+        M, N = M // 16 * 16, N // 16 * 16
+    assert lib.llmq_gemm_splitk_floats(M, N, Kd, dt.itemsize, 148) == (parts * M * N if parts > 1 else 0)
+    g = torch.Generator(device=DEV).manual_seed(M + steps)
+    a, b = (torch.randn(*((Kd, r) if mn else (r, Kd)), device=DEV, generator=g).to(dt) for r in (M, N))
+    got = []
+    try:
+        for mode in (0, 1, 2):
+            lib.llmq_gemm_set_mode(mode)
+            out = torch.full((M, N), 9.0, device=DEV, dtype=BF)
+            K.gemm(out, a, b, a_mn=bool(mn), b_mn=bool(mn))
+            got.append(out)
+    finally:
+        lib.llmq_gemm_set_mode(0)
+    ad, bd = (x.double().t() if mn else x.double() for x in (a, b))
+    assert rel(got[0], ad @ bd.t()) < 2**-8                   # fp32 sums, one rounding to bf16
+    assert parts > 1 or torch.equal(got[0], got[2])           # one order of the sum over K
+
+
+# bf16 outputs that are added to: blocks of 64 columns and remainders of 16, 32 and 48, ragged rows, tiles of 224 and 256 columns, several tiles per CTA in both kernels
+@pytest.mark.parametrize("M,N,Kd", [(130, 336, 64), (1000, 1008, 128), (300, 65, 64), (4100, 912, 640), (4096, 896, 1280), (9000, 2096, 192), (9000, 2096, 1216)])
+@pytest.mark.parametrize("dt", [BF, F8])
+@pytest.mark.parametrize("mode", [0, 1, 2])
+def test_gemm_added_to(M, N, Kd, dt, mode):
+    g = torch.Generator(device=DEV).manual_seed(N)
+    a, b = torch.randn(M, Kd, device=DEV, generator=g).to(dt), torch.randn(N, Kd, device=DEV, generator=g).to(dt)
+    bias, scale = torch.randn(N, device=DEV, generator=g).to(BF), torch.full((1,), 0.5, device=DEV)
+    whole = torch.randn(M + 1, N, device=DEV, generator=g).to(BF)
+    before = whole.clone()
+    out, am = whole[:M], torch.zeros(1, device=DEV)
+    try:
+        L.kernels().llmq_gemm_set_mode(mode)
+        K.gemm(out, a, b, bias=bias, accumulate=True, scale_a=scale, absmax=am)
+    finally:
+        L.kernels().llmq_gemm_set_mode(0)
+    want = 0.5 * (a.double() @ b.double().t()) + bias.double() + before[:M].double()
+    # one rounding to bf16 and fp32 sums of Kd products of a few units
+    assert ((out.double() - want).abs() <= want.abs() * 2**-8 + 1e-4 * Kd**0.5).all()
+    assert torch.equal(whole[M], before[M])
+    assert abs(am.item() - want.abs().max().item()) < 1e-4 * want.abs().max().item()
+
+
 def _split_k_operands(n, seed):
     """n GEMMs of one shape (8 parts, 2 MB of partial sums each) and what each gives by itself."""
     g = torch.Generator(device=DEV).manual_seed(seed)
