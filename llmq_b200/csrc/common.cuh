@@ -223,6 +223,15 @@ __device__ __forceinline__ e4m3 sr_e4m3(float x, uint32_t rnd) {
     bits &= 0xFFF00000u;
     return e4m3(__uint_as_float(bits));
 }
+// Two values at once, packed (lo in the low byte): the same bits as two calls of sr_e4m3, with one conversion and one branch where both are normal and
+// finite, as nearly all are.
+__device__ __forceinline__ uint32_t sr_e4m3x2(float lo, float hi, uint32_t r_lo, uint32_t r_hi) {
+    const float a = fabsf(lo), b = fabsf(hi);
+    if (fminf(a, b) >= 0.015625f && a < 448.f && b < 448.f)
+        return pack_e4m3x2(__uint_as_float((__float_as_uint(lo) + (r_lo & 0xFFFFFu)) & 0xFFF00000u), __uint_as_float((__float_as_uint(hi) + (r_hi & 0xFFFFFu)) & 0xFFF00000u));
+    const e4m3 x = sr_e4m3(lo, r_lo), y = sr_e4m3(hi, r_hi);
+    return static_cast<uint32_t>(x.__x) | static_cast<uint32_t>(y.__x) << 8;
+}
 template <typename T> __device__ __forceinline__ T sr_round(float x, uint32_t rnd);
 template <> __device__ __forceinline__ float sr_round<float>(float x, uint32_t) { return x; }
 template <> __device__ __forceinline__ bf16 sr_round<bf16>(float x, uint32_t rnd) { return sr_bf16(x, rnd); }

@@ -849,6 +849,26 @@ def test_rmsnorm_backward_blocks(C, rows):
     assert rel(dw, dw0.double() + (dy.double() * xh).sum(0)) < 2**-8 and am.item() == dinp.float().abs().max().item()
 
 
+# e4m3 first moments rounded in pairs: blocks of zeros, of values far below the largest (subnormal quotients beside normal ones), of subnormal and of huge gradients
+@pytest.mark.parametrize("n", [128, 1152, 128 * 1001])
+def test_adamw_e4m3_scales_and_rounding(n):
+    g = torch.Generator(device=DEV).manual_seed(n)
+    grad = torch.randn(n // 128, 128, device=DEV, generator=g) * torch.logspace(-30, 30, n // 128, device=DEV)[:, None]
+    grad *= 10 ** -(6 * torch.rand(n // 128, 128, device=DEV, generator=g))
+    grad[0] = 0
+    grad = grad.to(BF).view(-1)
+    p, v = torch.zeros(n, device=DEV, dtype=BF), torch.ones(n, device=DEV, dtype=BF)
+    m, ms = torch.zeros(n, device=DEV, dtype=F8), torch.ones(n // 128, device=DEV)
+    K.adamw(p, grad, m, v, lr=0.0, beta1=0.0, beta2=0.5, step=1, eps=1e-8, weight_decay=0.0, m_scales=ms, seed=11)      # beta1 = 0: the moment is the gradient
+    want = grad.float().view(-1, 128)
+    top = want.abs().amax(-1)
+    assert torch.equal(ms, (top.clamp_min(1e-30).double() / 448).float())        # the rounded quotient
+    q, x = m.float().view(-1, 128), want.double() / ms.double()[:, None]
+    quantum = torch.exp2(torch.floor(torch.log2(x.abs().clamp_min(2.0**-6))) - 3)
+    assert ((q.double() - x).abs() < quantum * (1 + 1e-5)).all()                              # stochastic rounding: one of the two neighbours
+    assert abs((q.double() - x).div(quantum).mean().item()) < 4 / n**0.5                      # and unbiased
+
+
 # the ring of the backward kernel turns: more rows per block than it has stages, one vector a thread (four stages) and three or four (two)
 @pytest.mark.parametrize("C", [896, 2048, 4104, 5120, 8192])
 @pytest.mark.parametrize("rows", [1001, 1777, 3000])
