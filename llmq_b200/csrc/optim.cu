@@ -323,9 +323,7 @@ __global__ void __launch_bounds__(512) deterministic_sum_kernel(float* __restric
 }
 
 // io[0]: squared norm in -> norm out;  io[1]: multiplier that clips the gradient to `clip` (1 if no clipping)
-__global__ void norm_finish_kernel(float* io, float clip, float* host_norm) {
-    grid_wait(io, host_norm);
-    float nsq = io[0];
+__device__ __forceinline__ void finish_norm(float* io, float nsq, float clip, float* host_norm) {
     float norm = sqrtf(nsq);
     float scale = 1.f;
     if (clip > 0.f && norm > clip) scale = clip / norm;
@@ -333,6 +331,19 @@ __global__ void norm_finish_kernel(float* io, float clip, float* host_norm) {
     io[0] = norm;
     io[1] = scale;
     if (host_norm) *host_norm = norm;
+}
+__global__ void norm_finish_kernel(float* io, float clip, float* host_norm) {
+    grid_wait(io, host_norm);
+    finish_norm(io, io[0], clip, host_norm);
+}
+// deterministic_sum_kernel and norm_finish_kernel in one launch, for callers that have nothing to do in between (2 us a launch)
+__global__ void __launch_bounds__(512) norm_sum_finish_kernel(float* __restrict__ io, const float* __restrict__ in, int n, float clip, float* __restrict__ host_norm) {
+    grid_wait(io, in, host_norm);
+    __shared__ float scratch[32];
+    float s = 0.f;
+    for (int i = threadIdx.x; i < n; i += blockDim.x) s += in[i];
+    s = block_reduce_sum(s, scratch);
+    if (threadIdx.x == 0) finish_norm(io, s, clip, host_norm);
 }
 
 // dst = SR(scale * (a + b))
@@ -496,6 +507,12 @@ extern "C" int llmq_deterministic_sum(float* out, const float* in, int n, cudaSt
 
 extern "C" int llmq_norm_finish(float* io, float clip, float* host_norm, cudaStream_t s) {
     launch_chained(norm_finish_kernel, 1, 1, 0, s, io, clip, host_norm);
+    return LLMQ_LAUNCH_CHECK();
+}
+
+// io[0] <- norm of which `in` holds the partial squares, io[1] <- the multiplier of llmq_norm_finish
+extern "C" int llmq_norm_sum_finish(float* io, const float* in, int n, float clip, float* host_norm, cudaStream_t s) {
+    launch_chained(norm_sum_finish_kernel, 1, 512, 0, s, io, in, n, clip, host_norm);
     return LLMQ_LAUNCH_CHECK();
 }
 

@@ -127,6 +127,7 @@ struct Entry {
     X(llmq_fused_classifier, P, P, P, P, float, float, int, int, LL, int, int)                                                       \
     X(llmq_norm_squared, P, P, LL, int, int)                                                                                         \
     X(llmq_deterministic_sum, P, P, int)                                                                                             \
+    X(llmq_norm_sum_finish, P, P, int, float, P)                                                                                     \
     X(llmq_norm_finish, P, float, P)                                                                                                 \
     X(llmq_adamw_hyper, P, P, P, P, P, LL, float, float, float, int, float, float, P, P, unsigned int, LL, int, int, int, int, int, P)
 

@@ -272,8 +272,7 @@ def global_norm_squared(out: T, values: T) -> None:
 
 @_op("llmq_b200::global_norm_finish", mutates_args=("io", "partials"))
 def global_norm_finish(io: T, partials: T, grad_clip: float) -> None:
-    K.deterministic_sum(io[0:1], partials)
-    K.norm_finish(io, grad_clip)
+    K.norm_sum_finish(io, partials, grad_clip)
 
 
 @_op("llmq_b200::adamw_update", mutates_args=("params", "m", "v", "m_scales", "abs_max"))

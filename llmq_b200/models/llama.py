@@ -941,10 +941,13 @@ class LlamaModel:
                 self.graphs.run(("opt-norm",), norms)
             else:
                 norms()
-        K.deterministic_sum(self.norm_io[0:1], g.norm_partials if norm_fused else self.norm_partials)
+        partials = g.norm_partials if norm_fused else self.norm_partials
         if self.comm.world > 1:
+            K.deterministic_sum(self.norm_io[0:1], partials)
             self._all_reduce_small(self.norm_io[0:1], "sum")
-        K.norm_finish(self.norm_io, grad_clip)
+            K.norm_finish(self.norm_io, grad_clip)
+        else:
+            K.norm_sum_finish(self.norm_io, partials, grad_clip)
         scale = self.norm_io[1:2]
         # ---- AdamW on every shard
         w.zero_absmax()

@@ -809,6 +809,15 @@ def deterministic_sum(out: torch.Tensor, x: torch.Tensor) -> None:
     out.copy_(x.float().sum().reshape_as(out))
 
 
+def norm_sum_finish(io: torch.Tensor, partials: torch.Tensor, clip: float, host_norm: Optional[torch.Tensor] = None) -> None:
+    """``deterministic_sum(io[0:1], partials)`` and ``norm_finish(io, clip, host_norm)`` in one launch."""
+    if io.is_cuda:
+        L.check(L.calls().llmq_norm_sum_finish(io, partials, partials.numel(), clip, host_norm), "norm_sum_finish")
+        return
+    deterministic_sum(io[0:1], partials)
+    norm_finish(io, clip, host_norm)
+
+
 def norm_finish(io: torch.Tensor, clip: float, host_norm: Optional[torch.Tensor] = None) -> None:
     """io[0]: squared norm -> norm; io[1] <- clip multiplier (min(1, clip / norm); 0 for a non-finite norm)."""
     if io.is_cuda:

@@ -69,7 +69,7 @@ SIGNATURES = {
     "llmq_swiglu_forward": "pppliipppi", "llmq_swiglu_backward": "pppliipi", "llmq_rope": "pppiiiiiiipi",
     "llmq_attention_forward": "pppiiiiipp", "llmq_attention_backward": "ppppppiiiiip", "llmq_bias_backward": "pppliippiii", "llmq_abs_max": "pplii",
     "llmq_quantize": "ppppliii", "llmq_quantize_transpose": "pppppiiii", "llmq_transpose": "ppppiiii", "llmq_fused_classifier": "ppppffiilii",
-    "llmq_norm_squared": "pplii", "llmq_deterministic_sum": "ppi", "llmq_norm_finish": "pfp", "llmq_adamw_hyper": "ppppplfffiffppuliiiiip",
+    "llmq_norm_squared": "pplii", "llmq_deterministic_sum": "ppi", "llmq_norm_sum_finish": "ppifp", "llmq_norm_finish": "pfp", "llmq_adamw_hyper": "ppppplfffiffppuliiiiip",
 }
 _CTYPES = {"p": ctypes.c_void_p, "i": ctypes.c_int, "u": ctypes.c_uint, "l": ctypes.c_longlong, "f": ctypes.c_float, "d": ctypes.c_double}
 
@@ -149,7 +149,7 @@ class KernelError(RuntimeError):
     pass
 
 
-# Number of device kernels launched through this module (each entry point knows how many it launches).
+# Number of device kernels launched through this module (each entry point knows how many it launches; small bias gradients take one instead of two).
 _EXTRA_LAUNCHES = {"rmsnorm_backward": 1, "bias_backward": 1, "attention_backward": 1, "encoder_backward": 1}
 launch_count = 0
 

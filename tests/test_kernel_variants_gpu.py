@@ -849,6 +849,45 @@ def test_rmsnorm_backward_blocks(C, rows):
     assert rel(dw, dw0.double() + (dy.double() * xh).sum(0)) < 2**-8 and am.item() == dinp.float().abs().max().item()
 
 
+# the bias gradient in one launch (columns in fours) against the two kernels that take unaligned gradients: the same sums in the same order; rows around
+# multiples of 8 and 512, columns around multiples of 16 and 128
+@pytest.mark.parametrize("rows", [1, 7, 65, 511, 513, 1001, 3000])
+@pytest.mark.parametrize("C", [4, 124, 128, 148, 1152])
+@pytest.mark.parametrize("dt,out_dt", [(BF, BF), (torch.float32, torch.float32), (F8, BF), (torch.float8_e5m2, torch.float32)])
+def test_bias_backward_one_launch(rows, C, dt, out_dt):
+    g = torch.Generator(device=DEV).manual_seed(rows + C)
+    dout = torch.randn(rows, C, device=DEV, generator=g).to(dt)
+    shifted = torch.empty(rows * C + 8, device=DEV, dtype=dt)[4 // dt.itemsize or 1:][:rows * C].view(rows, C)
+    shifted.copy_(dout)
+    assert dout.data_ptr() % 16 == 0 and shifted.data_ptr() % 16 != 0
+    sa, sb, d0 = torch.full((1,), 0.5, device=DEV), torch.full((1,), 3.0, device=DEV), torch.randn(C, device=DEV, generator=g).to(out_dt)
+    for acc in (False, True):
+        got = []
+        for d in (dout, shifted):
+            db, scratch = d0.clone(), torch.full((64 * C,), math.nan, device=DEV)
+            K.bias_backward(db, d, scratch, scale_a=sa, scale_b=sb, accumulate=acc)
+            got.append(db)
+        assert torch.equal(*got)
+        want = 1.5 * dout.double().sum(0) + (d0.double() if acc else 0)
+        assert ((got[0].double() - want).abs() <= want.abs() * (2**-8 if out_dt == BF else 1e-6) + 1e-5 * rows**0.5 * (448 if dt.itemsize == 1 else 1)).all()
+
+
+# the sum of the partial squares and the clipping factor in one launch: fewer and more partials than threads, no clipping, a norm that is not finite
+@pytest.mark.parametrize("n", [1, 31, 512, 513, 2000])
+@pytest.mark.parametrize("clip,bad", [(0.0, None), (1.0, None), (1e6, None), (1.0, math.inf), (1.0, math.nan)])
+def test_norm_sum_finish(n, clip, bad):
+    x = torch.rand(n, device=DEV, generator=torch.Generator(device=DEV).manual_seed(n))
+    if bad is not None:
+        x[n // 2] = bad
+    io, two = torch.full((3,), 9.0, device=DEV), torch.full((3,), 9.0, device=DEV)
+    K.norm_sum_finish(io, x, clip, io[2:3])
+    K.deterministic_sum(two[0:1], x)
+    K.norm_finish(two, clip, two[2:3])
+    assert torch.equal(io.view(torch.int32), two.view(torch.int32))
+    if bad is None:
+        assert abs(io[0].item() - x.double().sum().sqrt().item()) < 1e-5 * io[0].item()
+
+
 # e4m3 first moments rounded in pairs: blocks of zeros, of values far below the largest (subnormal quotients beside normal ones), of subnormal and of huge gradients
 @pytest.mark.parametrize("n", [128, 1152, 128 * 1001])
 def test_adamw_e4m3_scales_and_rounding(n):
