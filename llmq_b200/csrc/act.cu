@@ -341,8 +341,8 @@ __global__ void rope_table_kernel(float* freqs, int Tlen, int half, float theta)
 // is more.  With just the resident blocks all of them stride through the same few megabytes of every stream in step, which costs memory
 // throughput; many more mix rounds, and start-up comes into it.  us with 8 blocks per SM / with this rule, bf16: SwiGLU forward and backward (4
 // rounds) 16384 x 18944 309 / 285 and 585 / 456, 4096 x 4864 22.8 / 21.9 and 38.7 / 33.0, 2000 x 13824 29.6 / 27.2 and 51.0 / 43.7, 512 x 8192 the same
-// grid;  SwiGLU to e4m3 (8 rounds) 303 / 276, 22.1 / 22.1, 29.1 / 28.3;  RoPE (8 rounds) 8 x 2048 x 36 x 128 55.7 / 49.0, in place 54.8 / 48.1, with
-// abs-max 56.4 / 50.7.  One round per block: 336 and 501, 360, 50.7.
+// grid;  RoPE (8 rounds) 8 x 2048 x 36 x 128 55.7 / 49.0, in place 54.8 / 48.1, with abs-max 56.4 / 50.7.  One round per block: 336 and 501, 50.7.
+// SwiGLU to e4m3, 4 / 8 rounds: 4096 x 4864 21.1 / 23.2, 3000 x 8192 24.3 / 26.0, 2048 x 18944 36.2 / 36.8, 16384 x 18944 255 / 249.
 int grid_for(long long work_items, int num_sms, int per_block) {
     const long long blocks = ceil_div_ll(work_items, 256), resident = static_cast<long long>(num_sms) * 8;
     long long g = ceil_div_ll(blocks, per_block);
@@ -350,7 +350,9 @@ int grid_for(long long work_items, int num_sms, int per_block) {
     if (g > (1ll << 30)) g = 1ll << 30;
     return static_cast<int>(g > 0 ? g : 1);
 }
-constexpr int kSwigluRounds = 4, kSwigluQuantRounds = 8, kRopeRounds = 8;
+constexpr int kSwigluRounds = 4, kRopeRounds = 8;
+// SwiGLU forward; `vecs` vectors of the output
+int swiglu_fwd_rounds(bool quantised, long long vecs) { return quantised && vecs > (16ll << 20) ? 8 : kSwigluRounds; }
 
 }  // namespace
 
@@ -359,11 +361,11 @@ extern "C" int llmq_swiglu_forward(void* out, void* q_out, const void* inp, long
     if (rows <= 0) return 0;
     if (dtype == 0) {
         if (D % 8) return -1;
-        swiglu_fwd_kernel<bf16><<<grid_for(rows * (D / 8), num_sms, q_out ? kSwigluQuantRounds : kSwigluRounds), 256, 0, s>>>(
+        swiglu_fwd_kernel<bf16><<<grid_for(rows * (D / 8), num_sms, swiglu_fwd_rounds(q_out, rows * (D / 8))), 256, 0, s>>>(
             static_cast<bf16*>(out), static_cast<e4m3*>(q_out), static_cast<const bf16*>(inp), rows, D, absmax, known_absmax, q_scale, FastDiv(D / 8));
     } else if (dtype == 3) {
         if (D % 4) return -1;
-        swiglu_fwd_kernel<float><<<grid_for(rows * (D / 4), num_sms, q_out ? kSwigluQuantRounds : kSwigluRounds), 256, 0, s>>>(
+        swiglu_fwd_kernel<float><<<grid_for(rows * (D / 4), num_sms, swiglu_fwd_rounds(q_out, rows * (D / 4))), 256, 0, s>>>(
             static_cast<float*>(out), static_cast<e4m3*>(q_out), static_cast<const float*>(inp), rows, D, absmax, known_absmax, q_scale, FastDiv(D / 4));
     } else return -10;
     return LLMQ_LAUNCH_CHECK();

@@ -236,4 +236,11 @@ template <typename T> __device__ __forceinline__ T sr_round(float x, uint32_t rn
 template <> __device__ __forceinline__ float sr_round<float>(float x, uint32_t) { return x; }
 template <> __device__ __forceinline__ bf16 sr_round<bf16>(float x, uint32_t rnd) { return sr_bf16(x, rnd); }
 
-__device__ __forceinline__ float fast_sigmoid(float x) { return __fdividef(1.f, 1.f + __expf(-x)); }
+// 1 / (1 + e^-x), the same bits as __fdividef(1.f, 1.f + __expf(-x)): subnormal values, for which those two take extra instructions, vanish in the sum or
+// are results that both give as 0 (a denominator above 2^126)
+__device__ __forceinline__ float fast_sigmoid(float x) {
+    float e, r;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(-x * 1.4426950408889634f));
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(1.f + e));
+    return r;
+}

@@ -888,6 +888,21 @@ def test_norm_sum_finish(n, clip, bad):
         assert abs(io[0].item() - x.double().sum().sqrt().item()) < 1e-5 * io[0].item()
 
 
+# SwiGLU where the sigmoid of the gate goes under or over: large gates of both signs, zeros, infinities.  bf16 rounds the product of an fp32 sigmoid (a few units of 2^-24, and for gates
+# below -88, whose sigmoid is less than 2^-126, either of 0 and the value)
+@pytest.mark.parametrize("dt", [BF, torch.float32])
+def test_swiglu_gate_extremes(dt):
+    gates = torch.tensor([0.0, -0.0, 1e-30, -1e-30, 1.0, -1.0, 17.0, -17.0, 60.0, -60.0, 87.0, -87.0, 89.0, -89.0, 104.0, -104.0, 1e4, -1e4, 3e38, -3e38, math.inf, -20.0, 20.0, 5.5])
+    gate = gates.to(DEV).to(dt).repeat(3, 8)
+    inp = torch.cat([torch.full_like(gate, 1.5), gate], 1)
+    out = torch.empty_like(gate)
+    K.swiglu_forward(out, inp)
+    want = 1.5 * gate.double() * torch.sigmoid(gate.double())
+    finite = want.isfinite() & (want.abs() < torch.finfo(dt).max)
+    assert ((out.double() - want).abs()[finite] <= (2**-8 if dt == BF else 2**-20) * want.abs()[finite] + 1e-34).all()
+    assert (out[~finite] == math.inf).all()
+
+
 # e4m3 first moments rounded in pairs: blocks of zeros, of values far below the largest (subnormal quotients beside normal ones), of subnormal and of huge gradients
 @pytest.mark.parametrize("n", [128, 1152, 128 * 1001])
 def test_adamw_e4m3_scales_and_rounding(n):
