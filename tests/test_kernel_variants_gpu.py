@@ -889,10 +889,10 @@ def test_norm_sum_finish(n, clip, bad):
 
 
 # SwiGLU where the sigmoid of the gate goes under or over: large gates of both signs, zeros, infinities.  bf16 rounds the product of an fp32 sigmoid (a few units of 2^-24, and for gates
-# below -88, whose sigmoid is less than 2^-126, either of 0 and the value)
+# below -88, whose sigmoid is less than 2^-126, either of 0 and the value);  up x gate, which is taken first, is finite for the negative gates
 @pytest.mark.parametrize("dt", [BF, torch.float32])
 def test_swiglu_gate_extremes(dt):
-    gates = torch.tensor([0.0, -0.0, 1e-30, -1e-30, 1.0, -1.0, 17.0, -17.0, 60.0, -60.0, 87.0, -87.0, 89.0, -89.0, 104.0, -104.0, 1e4, -1e4, 3e38, -3e38, math.inf, -20.0, 20.0, 5.5])
+    gates = torch.tensor([0.0, -0.0, 1e-30, -1e-30, 1.0, -1.0, 17.0, -17.0, 60.0, -60.0, 87.0, -87.0, 89.0, -89.0, 104.0, -104.0, 1e4, -1e4, 3e38, -1e38, math.inf, -20.0, 20.0, 5.5])
     gate = gates.to(DEV).to(dt).repeat(3, 8)
     inp = torch.cat([torch.full_like(gate, 1.5), gate], 1)
     out = torch.empty_like(gate)
