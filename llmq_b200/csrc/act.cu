@@ -269,58 +269,88 @@ swiglu_bwd_quant_kernel(e4m3* __restrict__ q_rows, e4m3* __restrict__ q_t, float
 // RoPE on the packed (B, T, Hq + 2*Hkv, HS) tensor; query and key heads are rotated with the half-split
 // pairing (d, d + HS/2), value heads are copied (or left alone when in place).  freqs is (T, HS/2, 2)
 // fp32 {cos, sin}.  Backward is the conjugate rotation.
+//
+// A thread has one pair of vectors of two heads of a token, half of its heads apart (neighbouring threads have neighbouring vectors): it reads the angles,
+// 64 bytes, once for both and has four loads under way.  us, a head per thread / two:  8 x 2048 tokens, 28 / 4 heads of 128 53.9 / 46.6 (floor 46.2), with
+// abs-max 55.1 / 49.2;  1 x 8192, 32 / 8 of 128 40.1 / 32.4;  8 x 1024, 14 / 2 of 64 9.4 / 8.3 and 10.6 / 9.1;  1 x 333, 12 / 2 of 128 2.00 / 1.96.  Three
+// and four heads: 51.0 and 48.6, 9.4 and 9.5.  Calls that give no SM more than a block take a thread per head (lanes = H), only latency counts there:
+// 1 x 60, 12 / 2 of 128 1.66 / 1.86, 1 x 512, 14 / 2 of 64 1.67 / 1.93.
+constexpr int kRopeHeads = 2;
+struct RopeShape {
+    int H, rotated, half, lanes;              // heads, of them rotated, half a head size, heads / kRopeHeads rounded up (or heads, each thread with one)
+    FastDiv vec, lane, tokens;                // by vectors per half head, lanes, sequence length
+    long long total;                          // threads
+    int wide;                                 // the angles may be read 16 bytes at a time
+};
 template <typename T, bool Backward>
 __global__ void __launch_bounds__(256)
-rope_kernel(T* out, const T* inp, const float* __restrict__ freqs, int B, int Tlen, int Hq, int Hkv, int HS,
-            float* __restrict__ absmax_out, const FastDiv fd_vec, const FastDiv fd_h, const FastDiv fd_t) {
+rope_kernel(T* out, const T* inp, const float* __restrict__ freqs, const RopeShape p, float* __restrict__ absmax_out) {
     grid_wait();
     const int bx = after_wait(blockIdx.x), tx = after_wait(threadIdx.x);
     __shared__ float scratch[32];
     using V = Vec16<T>;
-    const int half = HS / 2;
-    const int vec_per_half = half / V::N;
-    const int H = Hq + 2 * Hkv;
-    const long long total = static_cast<long long>(B) * Tlen * H * vec_per_half;
     float tmax = 0.f;
-    for (long long i = bx * static_cast<long long>(blockDim.x) + tx; i < total;
-         i += static_cast<long long>(gridDim.x) * blockDim.x) {
-        int v, h, t;
+    const bool in_place = out == inp;
+    for (long long i = bx * static_cast<long long>(blockDim.x) + tx; i < p.total; i += static_cast<long long>(gridDim.x) * blockDim.x) {
+        int v, h0, t;
         long long bt;
-        if (total < (1ll << 31)) {
+        if (p.total < (1ll << 31)) {
             uint32_t rest, vv, hh, btt, bb, tt;
-            fd_vec.divmod(static_cast<uint32_t>(i), rest, vv);
-            fd_h.divmod(rest, btt, hh);
-            fd_t.divmod(btt, bb, tt);
-            v = static_cast<int>(vv); h = static_cast<int>(hh); t = static_cast<int>(tt); bt = btt;
+            p.vec.divmod(static_cast<uint32_t>(i), rest, vv);
+            p.lane.divmod(rest, btt, hh);
+            p.tokens.divmod(btt, bb, tt);
+            v = static_cast<int>(vv); h0 = static_cast<int>(hh); t = static_cast<int>(tt); bt = btt;
         } else {
-            v = static_cast<int>(i % vec_per_half);
-            long long rest = i / vec_per_half;
-            h = static_cast<int>(rest % H);
-            bt = rest / H;
-            t = static_cast<int>(bt % Tlen);
+            v = static_cast<int>(i % p.vec.d);
+            const long long rest = i / p.vec.d;
+            h0 = static_cast<int>(rest % p.lanes);
+            bt = rest / p.lanes;
+            t = static_cast<int>(bt % p.tokens.d);
         }
-        long long base = (bt * H + h) * HS + v * V::N;
-        V x1 = V::load(inp + base), x2 = V::load(inp + base + half);
-        if (h < Hq + Hkv) {
-            const float* f = freqs + (static_cast<long long>(t) * half + v * V::N) * 2;
+        const long long base = (bt * p.H + h0) * (2 * p.half) + v * V::N;
+        const int step = p.lanes * 2 * p.half;
+        // value heads of an in-place call are only read for the abs-max
+        const int heads = in_place && !absmax_out ? p.rotated : p.H;
+        V x1[kRopeHeads], x2[kRopeHeads];
 #pragma unroll
-            for (int k = 0; k < V::N; ++k) {
-                float c = f[2 * k], s = f[2 * k + 1];
-                if (Backward) s = -s;
-                float a = to_float(x1.v[k]), b = to_float(x2.v[k]);
-                x1.v[k] = from_float<T>(a * c - b * s);
-                x2.v[k] = from_float<T>(b * c + a * s);
+        for (int k = 0; k < kRopeHeads; ++k) {
+            if (h0 + k * p.lanes < heads) { x1[k] = V::load(inp + base + k * step); x2[k] = V::load(inp + base + k * step + p.half); }
+        }
+        float f[2 * V::N];
+        if (h0 < p.rotated) {
+            const float* fp = freqs + (static_cast<long long>(t) * p.half + v * V::N) * 2;
+            if (p.wide) {
+#pragma unroll
+                for (int k = 0; k < V::N / 2; ++k) {
+                    const float4 w = reinterpret_cast<const float4*>(fp)[k];
+                    f[4 * k] = w.x; f[4 * k + 1] = w.y; f[4 * k + 2] = w.z; f[4 * k + 3] = w.w;
+                }
+            } else {
+#pragma unroll
+                for (int k = 0; k < 2 * V::N; ++k) f[k] = fp[k];
             }
-        } else if (out == inp && !absmax_out) {
-            continue;
         }
-        if (absmax_out) {
 #pragma unroll
-            for (int k = 0; k < V::N; ++k) tmax = fmaxf(tmax, fmaxf(fabsf(to_float(x1.v[k])), fabsf(to_float(x2.v[k]))));
-        }
-        if (!(out == inp && h >= Hq + Hkv)) {
-            x1.store(out + base);
-            x2.store(out + base + half);
+        for (int k = 0; k < kRopeHeads; ++k) {
+            const int h = h0 + k * p.lanes;
+            if (h >= heads) continue;
+            if (h < p.rotated) {
+#pragma unroll
+                for (int j = 0; j < V::N; ++j) {
+                    const float c = f[2 * j], s = Backward ? -f[2 * j + 1] : f[2 * j + 1];
+                    const float a = to_float(x1[k].v[j]), b = to_float(x2[k].v[j]);
+                    x1[k].v[j] = from_float<T>(a * c - b * s);
+                    x2[k].v[j] = from_float<T>(b * c + a * s);
+                }
+            }
+            if (absmax_out) {
+#pragma unroll
+                for (int j = 0; j < V::N; ++j) tmax = fmaxf(tmax, fmaxf(fabsf(to_float(x1[k].v[j])), fabsf(to_float(x2[k].v[j]))));
+            }
+            if (!(in_place && h >= p.rotated)) {
+                x1[k].store(out + base + k * step);
+                x2[k].store(out + base + k * step + p.half);
+            }
         }
     }
     block_absmax_commit(absmax_out, tmax, scratch);
@@ -341,8 +371,8 @@ __global__ void rope_table_kernel(float* freqs, int Tlen, int half, float theta)
 // is more.  With just the resident blocks all of them stride through the same few megabytes of every stream in step, which costs memory
 // throughput; many more mix rounds, and start-up comes into it.  us with 8 blocks per SM / with this rule, bf16: SwiGLU forward and backward (4
 // rounds) 16384 x 18944 309 / 285 and 585 / 456, 4096 x 4864 22.8 / 21.9 and 38.7 / 33.0, 2000 x 13824 29.6 / 27.2 and 51.0 / 43.7, 512 x 8192 the same
-// grid;  RoPE (8 rounds) 8 x 2048 x 36 x 128 55.7 / 49.0, in place 54.8 / 48.1, with abs-max 56.4 / 50.7.  One round per block: 336 and 501, 50.7.
-// SwiGLU to e4m3, 4 / 8 rounds: 4096 x 4864 21.1 / 23.2, 3000 x 8192 24.3 / 26.0, 2048 x 18944 36.2 / 36.8, 16384 x 18944 255 / 249.
+// grid.  One round per block: 336 and 501.  SwiGLU to e4m3, 4 / 8 rounds: 4096 x 4864 21.1 / 23.2, 3000 x 8192 24.3 / 26.0, 2048 x 18944 36.2 / 36.8,
+// 16384 x 18944 255 / 249.  RoPE, 2 / 4 rounds: 8 x 2048 x 36 x 128 46.6 / 47.6, 1 x 8192 x 48 x 128 32.4 / 33.5, smaller ones the same.
 int grid_for(long long work_items, int num_sms, int per_block) {
     const long long blocks = ceil_div_ll(work_items, 256), resident = static_cast<long long>(num_sms) * 8;
     long long g = ceil_div_ll(blocks, per_block);
@@ -350,7 +380,7 @@ int grid_for(long long work_items, int num_sms, int per_block) {
     if (g > (1ll << 30)) g = 1ll << 30;
     return static_cast<int>(g > 0 ? g : 1);
 }
-constexpr int kSwigluRounds = 4, kRopeRounds = 8;
+constexpr int kSwigluRounds = 4, kRopeRounds = 2;
 // SwiGLU forward; `vecs` vectors of the output
 int swiglu_fwd_rounds(bool quantised, long long vecs) { return quantised && vecs > (16ll << 20) ? 8 : kSwigluRounds; }
 
@@ -386,26 +416,33 @@ extern "C" int llmq_swiglu_backward(void* dinp, const void* dout, const void* in
     return LLMQ_LAUNCH_CHECK();
 }
 
+template <typename T>
+static int launch_rope(void* out, const void* inp, const float* freqs, int B, int T_, int Hq, int Hkv, int HS, int backward, float* absmax, int num_sms, cudaStream_t s) {
+    const int vecs = HS / 2 / Vec16<T>::N;
+    RopeShape p;
+    p.H = Hq + 2 * Hkv; p.rotated = Hq + Hkv; p.half = HS / 2;
+    p.lanes = static_cast<long long>(B) * T_ * p.H * vecs <= 256ll * num_sms ? p.H : ceil_div_i(p.H, kRopeHeads);
+    p.vec = FastDiv(vecs); p.lane = FastDiv(p.lanes); p.tokens = FastDiv(T_);
+    p.total = static_cast<long long>(B) * T_ * p.lanes * vecs;
+    p.wide = reinterpret_cast<uintptr_t>(freqs) % 16 == 0;
+    const int g = grid_for(p.total, num_sms, kRopeRounds);
+    if (backward) launch_chained(rope_kernel<T, true>, g, 256, 0, s, static_cast<T*>(out), static_cast<const T*>(inp), freqs, p, absmax);
+    else          launch_chained(rope_kernel<T, false>, g, 256, 0, s, static_cast<T*>(out), static_cast<const T*>(inp), freqs, p, absmax);
+    return LLMQ_LAUNCH_CHECK();
+}
+
 extern "C" int llmq_rope(void* out, const void* inp, const float* freqs, int B, int T, int Hq, int Hkv, int HS, int dtype,
                          int backward, float* absmax, int num_sms, cudaStream_t s) {
     if (B <= 0 || T <= 0) return 0;
-    const int H = Hq + 2 * Hkv;
     if (dtype == 0) {
         if ((HS / 2) % 8) return -1;
-        constexpr int VN = 8;
-        long long work = static_cast<long long>(B) * T * H * (HS / 2 / 8);
-        int g = grid_for(work, num_sms, kRopeRounds);
-        if (backward) launch_chained(rope_kernel<bf16, true>, g, 256, 0, s, static_cast<bf16*>(out), static_cast<const bf16*>(inp), freqs, B, T, Hq, Hkv, HS, absmax, FastDiv(HS / 2 / VN), FastDiv(H), FastDiv(T));
-        else launch_chained(rope_kernel<bf16, false>, g, 256, 0, s, static_cast<bf16*>(out), static_cast<const bf16*>(inp), freqs, B, T, Hq, Hkv, HS, absmax, FastDiv(HS / 2 / VN), FastDiv(H), FastDiv(T));
-    } else if (dtype == 3) {
+        return launch_rope<bf16>(out, inp, freqs, B, T, Hq, Hkv, HS, backward, absmax, num_sms, s);
+    }
+    if (dtype == 3) {
         if ((HS / 2) % 4) return -1;
-        constexpr int VN = 4;
-        long long work = static_cast<long long>(B) * T * H * (HS / 2 / 4);
-        int g = grid_for(work, num_sms, kRopeRounds);
-        if (backward) launch_chained(rope_kernel<float, true>, g, 256, 0, s, static_cast<float*>(out), static_cast<const float*>(inp), freqs, B, T, Hq, Hkv, HS, absmax, FastDiv(HS / 2 / VN), FastDiv(H), FastDiv(T));
-        else launch_chained(rope_kernel<float, false>, g, 256, 0, s, static_cast<float*>(out), static_cast<const float*>(inp), freqs, B, T, Hq, Hkv, HS, absmax, FastDiv(HS / 2 / VN), FastDiv(H), FastDiv(T));
-    } else return -10;
-    return LLMQ_LAUNCH_CHECK();
+        return launch_rope<float>(out, inp, freqs, B, T, Hq, Hkv, HS, backward, absmax, num_sms, s);
+    }
+    return -10;
 }
 
 extern "C" int llmq_rope_table(float* freqs, int T, int HS, float theta, cudaStream_t s) {

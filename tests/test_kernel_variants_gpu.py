@@ -905,6 +905,34 @@ def test_swiglu_gate_extremes(dt):
     assert (out[~finite] == math.inf).all()
 
 
+# RoPE, a head of a token per thread (small calls) and two: odd and even numbers of heads (the last thread of a token has one), head sizes whose halves are 1, 2, 3, 4 and 8 vectors, one token, in
+# place with and without the abs-max (value heads are then only read), angles that are not aligned to 16 bytes
+@pytest.mark.parametrize("B,T,Hq,Hkv,HS", [(1, 1, 1, 1, 16), (2, 7, 2, 1, 32), (3, 33, 3, 2, 48), (1, 100, 14, 2, 64), (2, 65, 5, 2, 128), (1, 257, 1, 3, 128),
+                                           (2, 701, 11, 2, 64), (3, 999, 3, 1, 48), (1, 1301, 2, 3, 128)])
+@pytest.mark.parametrize("dt", [BF, torch.float32])
+@pytest.mark.parametrize("backward", [False, True])
+def test_rope_heads(B, T, Hq, Hkv, HS, dt, backward):
+    g = torch.Generator(device=DEV).manual_seed(T)
+    x = torch.randn(B, T, Hq + 2 * Hkv, HS, device=DEV, generator=g).to(dt)
+    table = K.rope_table(T, HS, 1e4, torch.device(DEV, 0))
+    shifted = torch.empty(table.numel() + 1, device=DEV)[1:].view_as(table).copy_(table)
+    assert shifted.data_ptr() % 16 == 4
+    cos, sin = table[:, :, 0].double()[None, :, None], table[:, :, 1].double()[None, :, None] * (-1 if backward else 1)
+    a, b = x.double()[..., :HS // 2], x.double()[..., HS // 2:]
+    want = torch.cat([torch.cat([a * cos - b * sin, b * cos + a * sin], -1)[:, :, :Hq + Hkv], x.double()[:, :, Hq + Hkv:]], 2)
+    eps = 2**-8 if dt == BF else 1e-6
+    for freqs in (table, shifted):
+        for absmax in (None, torch.zeros(1, device=DEV)):
+            for in_place in (False, True):
+                src = x.clone()
+                out = src if in_place else torch.full_like(x, 9.0)
+                if absmax is not None:
+                    absmax.zero_()
+                K.rope(out, src, freqs, Hq, Hkv, backward=backward, absmax=absmax)
+                assert ((out.double() - want).abs() <= eps * want.abs() + 1e-6 * (1 + x.double().abs().max())).all()
+                assert absmax is None or absmax.item() == out.float().abs().max().item()
+
+
 # e4m3 first moments rounded in pairs: blocks of zeros, of values far below the largest (subnormal quotients beside normal ones), of subnormal and of huge gradients
 @pytest.mark.parametrize("n", [128, 1152, 128 * 1001])
 def test_adamw_e4m3_scales_and_rounding(n):
