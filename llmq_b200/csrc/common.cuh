@@ -236,6 +236,12 @@ template <typename T> __device__ __forceinline__ T sr_round(float x, uint32_t rn
 template <> __device__ __forceinline__ float sr_round<float>(float x, uint32_t) { return x; }
 template <> __device__ __forceinline__ bf16 sr_round<bf16>(float x, uint32_t rnd) { return sr_bf16(x, rnd); }
 
+// 32 bytes (16 bf16), aligned to as much: a whole sector per lane and instruction
+__device__ __forceinline__ void store_sector(void* p, const uint32_t* r) {
+    asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};"
+                 ::"l"(p), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]) : "memory");
+}
+
 // 1 / (1 + e^-x), the same bits as __fdividef(1.f, 1.f + __expf(-x)): subnormal values, for which those two take extra instructions, vanish in the sum or
 // are results that both give as 0 (a denominator above 2^126)
 __device__ __forceinline__ float fast_sigmoid(float x) {

@@ -103,12 +103,6 @@ __device__ __forceinline__ void add_bias32(const GemmParams& p, int col0, float 
 // Shared memory one epilogue warp needs for the coalescing store path of epilogue_rows (32 rows x 128 bytes).
 constexpr int EPI_STAGE_BYTES_PER_WARP = 32 * 128;
 
-// 32 bytes (16 bf16) of one row per lane: a whole sector per lane and instruction
-__device__ __forceinline__ void store_sector(void* p, const uint32_t* r) {
-    asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};"
-                 ::"l"(p), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]) : "memory");
-}
-
 // bf16 C in whole sectors (GemmParams::c_sectors), not added to: lane = row, 32 columns at a time.  A lane that moves 16 bytes at a time touches every sector
 // twice.  Plain outputs of the CTA-pair kernel stay on the staged TMA stores: 4096 x 151936 x 896 824 us, 837 this way.
 __device__ __forceinline__ void epilogue_rows_sectors(const GemmParams& p, uint32_t t_row, int row, int col_base, int ncols, float alpha, float& tmax) {

@@ -52,6 +52,25 @@ def test_attention_head_splits(HS, B, T, Hq, Hkv):
     assert rel(dqkv[:, :, Hq + Hkv:], x.grad[:, :, Hq + Hkv:]) < 1.2e-2
 
 
+# Forward, many items per CTA: even and odd numbers of items with both query tiles (their extra key tile alternates between the pipelines), items without a second tile before them, an
+# output that is aligned to 16 bytes only
+@pytest.mark.parametrize("HS", [64, 128])
+@pytest.mark.parametrize("B,T,Hq,Hkv", [(3, 256, 50, 10), (12, 256, 50, 10), (3, 300, 60, 30), (5, 513, 32, 8), (6, 640, 40, 8)])
+def test_attention_forward_items(HS, B, T, Hq, Hkv):
+    g = torch.Generator(device=DEV).manual_seed(T)
+    qkv = torch.randn(B, T, Hq + 2 * Hkv, HS, device=DEV, generator=g).to(BF)
+    out, lse, absmax = torch.full((B, T, Hq, HS), 9.0, device=DEV, dtype=BF), torch.empty(B, Hq, T, device=DEV), torch.zeros(1, device=DEV)
+    K.attention_forward(out, lse, qkv, Hq, Hkv, absmax=absmax)
+    shifted, lse2 = torch.full((out.numel() + 8,), 9.0, device=DEV, dtype=BF)[8:].view_as(out), torch.empty_like(lse)
+    assert shifted.data_ptr() % 32 == 16
+    K.attention_forward(shifted, lse2, qkv, Hq, Hkv)
+    assert torch.equal(out, shifted) and torch.equal(lse, lse2) and absmax.item() == out.float().abs().max().item()
+    for b in range(B):
+        o, l = K._attention_ref(qkv[b:b + 1].float(), Hq, Hkv)
+        # 16-bit probabilities (2^-9 each, random signs) and the 16-bit output
+        assert rel(out[b:b + 1], o) < 1e-2 and (lse[b:b + 1] - l).abs().max() < 2e-3
+
+
 # dK / dV of head size 128: CTAs per item on both sides of the steps of the rule (one CTA, clusters of two to eight, odd shares of the heads)
 @pytest.mark.parametrize("T", [70, 200])
 @pytest.mark.parametrize("Hq,Hkv", [(6, 1), (10, 2), (9, 1)])
