@@ -71,6 +71,22 @@ def test_attention_forward_items(HS, B, T, Hq, Hkv):
         assert rel(out[b:b + 1], o) < 1e-2 and (lse[b:b + 1] - l).abs().max() < 2e-3
 
 
+# A gradient that is aligned to 16 bytes only, without and with dK / dV parts
+@pytest.mark.parametrize("HS", [64, 128])
+@pytest.mark.parametrize("B,T,Hq,Hkv", [(2, 100, 6, 2), (1, 300, 8, 1)])
+def test_attention_backward_alignment(HS, B, T, Hq, Hkv):
+    g = torch.Generator(device=DEV).manual_seed(T)
+    qkv = torch.randn(B, T, Hq + 2 * Hkv, HS, device=DEV, generator=g).to(BF)
+    dout, out = torch.randn(B, T, Hq, HS, device=DEV, generator=g).to(BF), torch.empty(B, T, Hq, HS, device=DEV, dtype=BF)
+    lse, scratch = torch.empty(B, Hq, T, device=DEV), torch.empty(B * Hq * T, device=DEV)
+    K.attention_forward(out, lse, qkv, Hq, Hkv)
+    dqkv, shifted = torch.full_like(qkv, 9.0), torch.full((qkv.numel() + 8,), 9.0, device=DEV, dtype=BF)[8:].view_as(qkv)
+    assert dqkv.data_ptr() % 32 == 0 and shifted.data_ptr() % 32 == 16
+    for d in (dqkv, shifted):
+        K.attention_backward(d, scratch, dout, out, lse, qkv, Hq, Hkv)
+    assert torch.equal(dqkv, shifted)
+
+
 # dK / dV of head size 128: CTAs per item on both sides of the steps of the rule (one CTA, clusters of two to eight, odd shares of the heads)
 @pytest.mark.parametrize("T", [70, 200])
 @pytest.mark.parametrize("Hq,Hkv", [(6, 1), (10, 2), (9, 1)])
