@@ -14,7 +14,7 @@
 // so while one tile's warpgroup computes exponentials the tensor core runs the other tile's MMAs.  us, where the 168 registers of an even split made the
 // score rows spill (which waits for the L1) and the output left in 16-byte stores, each an access of its own / now:  8 x 2048 tokens, 28 / 4 heads of
 // 128 274 / 238 (clock counters: 6000 cycles from the end of a walk to the next item, 2500 now),  1 x 8192, 32 / 8 of 128 471 / 454,  8 x 1024, 14 / 2
-// of 64 39.1 / 33.6,  1 x 8192, 32 / 8 of 64 412 / 388,  1 x 333, 12 / 2 of 128 12.4 / 8.8.  A tile takes 3800 cycles at head size 128 (1600 of them
+// of 64 39.1 / 33.2,  1 x 8192, 32 / 8 of 64 412 / 385,  1 x 333, 12 / 2 of 128 12.4 / 8.8.  A tile takes 3800 cycles at head size 128 (1600 of them
 // exponentials, 1100 from P to the next scores, 500 the maximum) and two tiles are under way; 3200 at head size 64, bound by the exponentials of both.
 // K and V tiles stream through two (head size 128) or three shared-memory stages each (TMA, 128-byte swizzle); Q_A and Q_B stay in shared memory
 // for the whole walk.  O is rescaled only when a row maximum moved by more than 2^8 since the last rescale (the stale
@@ -130,7 +130,7 @@ __global__ void __launch_bounds__(NUM_THREADS, 1)
 attn_fwd_pingpong_kernel(const __grid_constant__ CUtensorMap tmap_qkv,     // qkv as (B, T, W), box 128 rows x 64 columns
                          const FwdParams p) {
     constexpr int NCH = HS / 64, TILE_BYTES = NCH * CHUNK_BYTES, ST = KV_STAGES<HS>;
-    constexpr bool ALTERNATE = HS == 64 && !PAIRED;
+    constexpr bool ALTERNATE = HS == 64 && !PAIRED, SPLIT = HS == 64 && !PAIRED;
     extern __shared__ __align__(1024) uint8_t smem[];
     uint8_t* sQ = smem;                                   // [2 tiles][TILE_BYTES]
     uint8_t* sK = sQ + 2 * TILE_BYTES;                    // [ST][TILE_BYTES]
@@ -235,6 +235,14 @@ attn_fwd_pingpong_kernel(const __grid_constant__ CUtensorMap tmap_qkv,     // qk
             const uint32_t hi = desc_hi(1024);
             const uint32_t tS = tmem + x * BKV, tO = tmem + 2 * BKV + x * HS;
             const uint32_t q_lo = desc_lo(smem_u32(sQ) + x * TILE_BYTES, 16);
+            const uint32_t idesc_half = make_instr_desc(1, 1, false, false, BQ, BKV / 2);
+            // scores of the keys from `key` on, as many as idesc says
+            auto scores = [&](int st, int key, uint32_t idesc) {
+                const uint32_t k_lo = desc_lo(smem_u32(sK) + st * TILE_BYTES + key * 128, 16);
+#pragma unroll
+                for (int k = 0; k < HS / 16; ++k)
+                    mma_issue<0, false>(tS + key, q_lo + (((k / 4) * CHUNK_BYTES + (k % 4) * 32) >> 4), hi, k_lo + (((k / 4) * CHUNK_BYTES + (k % 4) * 32) >> 4), hi, idesc, k > 0);
+            };
             uint32_t kv = 0, tiles = 0, walks = 0;           // stage uses, key tiles of this query tile, items in which it had any
             Order order;
             bool ok = true;
@@ -247,15 +255,15 @@ attn_fwd_pingpong_kernel(const __grid_constant__ CUtensorMap tmap_qkv,     // qk
                 for (int j = 0; j < n && ok; ++j, ++kv, ++tiles) {
                     const int st = kv % ST;
                     const uint32_t par = (kv / ST) & 1;
-                    if (!mbar_wait_warp(k_full(st), par, abort_flag)) { ok = false; break; }
-                    tc_fence_after_sync();
-                    const uint32_t k_lo = desc_lo(smem_u32(sK) + st * TILE_BYTES, 16), ke = k_empty(st);
+                    if (j == 0 || !SPLIT) {
+                        if (!mbar_wait_warp(k_full(st), par, abort_flag)) { ok = false; break; }
+                        tc_fence_after_sync();
+                    }
+                    const uint32_t ke = k_empty(st);
                     const bool last = j == n - 1;
                     if (leader) {
-#pragma unroll
-                        for (int k = 0; k < HS / 16; ++k)
-                            mma_issue<0, false>(tS, q_lo + (((k / 4) * CHUNK_BYTES + (k % 4) * 32) >> 4), hi,
-                                                k_lo + (((k / 4) * CHUNK_BYTES + (k % 4) * 32) >> 4), hi, idesc_s, k > 0);
+                        if (j == 0 || !SPLIT) scores(st, 0, idesc_s);
+                        else                  scores(st, 0, idesc_half);         // the other keys were issued during the previous tile
                         mma_commit(s_full(x));
                         mma_commit(ke);
                         if (last) mma_commit(q_empty(x));        // the item's last read of this Q tile
@@ -279,6 +287,16 @@ attn_fwd_pingpong_kernel(const __grid_constant__ CUtensorMap tmap_qkv,     // qk
                             if (half == 1) { mma_commit(o_done(x)); mma_commit(ve); }
                         }
                         __syncwarp();
+                        // The first half of P is there, so the score row has been read: the scores of the next tile's last 64 keys, whose columns P does not
+                        // use, need not wait for this tile's products.  Head size 64: 1 x 8192, 32 / 8 heads 392 -> 385 us.  Head size 128, where products
+                        // of 64 columns take more than half the time of 128: 239 -> 241 us for 8 x 2048, 28 / 4.
+                        if (SPLIT && half == 0 && j + 1 < n) {
+                            const int next = (kv + 1) % ST;
+                            if (!mbar_wait_warp(k_full(next), ((kv + 1) / ST) & 1, abort_flag)) { ok = false; break; }
+                            tc_fence_after_sync();
+                            if (leader) scores(next, BKV / 2, idesc_half);
+                            __syncwarp();
+                        }
                     }
                     if (!ok) break;
                 }
