@@ -273,9 +273,10 @@ swiglu_bwd_quant_kernel(e4m3* __restrict__ q_rows, e4m3* __restrict__ q_t, float
 // A thread has one pair of vectors of two heads of a token, half of its heads apart (neighbouring threads have neighbouring vectors): it reads the angles,
 // 64 bytes, once for both and has four loads under way.  us, a head per thread / two:  8 x 2048 tokens, 28 / 4 heads of 128 53.9 / 46.6 (floor 46.2), with
 // abs-max 55.1 / 49.2;  1 x 8192, 32 / 8 of 128 40.1 / 32.4;  8 x 1024, 14 / 2 of 64 9.4 / 8.3 and 10.6 / 9.1;  1 x 333, 12 / 2 of 128 2.00 / 1.96.  Three
-// and four heads: 51.0 and 48.6, 9.4 and 9.5.  Calls that give no SM more than a block take a thread per head (lanes = H), only latency counts there:
-// 1 x 60, 12 / 2 of 128 1.66 / 1.86, 1 x 512, 14 / 2 of 64 1.67 / 1.93.
-constexpr int kRopeHeads = 2;
+// and four heads: 51.0 and 48.6, 9.4 and 9.5.  Blocks of 128 threads, because half as many threads in blocks of 256 divide badly among the SMs: 4 x 797, 4 / 4
+// heads of 64 2.97 / 3.30 / 2.95 (128), 1 x 256, 32 / 8 of 128 2.52 / 2.72 / 2.32.  Calls that give no SM more than two such blocks take a thread per head
+// (lanes = H), only latency counts there: 1 x 60, 12 / 2 of 128 1.66 / 1.86, 1 x 512, 14 / 2 of 64 1.67 / 1.93.
+constexpr int kRopeHeads = 2, kRopeThreads = 128;
 struct RopeShape {
     int H, rotated, half, lanes;              // heads, of them rotated, half a head size, heads / kRopeHeads rounded up (or heads, each thread with one)
     FastDiv vec, lane, tokens;                // by vectors per half head, lanes, sequence length
@@ -283,7 +284,7 @@ struct RopeShape {
     int wide;                                 // the angles may be read 16 bytes at a time
 };
 template <typename T, bool Backward>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(kRopeThreads)
 rope_kernel(T* out, const T* inp, const float* __restrict__ freqs, const RopeShape p, float* __restrict__ absmax_out) {
     grid_wait();
     const int bx = after_wait(blockIdx.x), tx = after_wait(threadIdx.x);
@@ -373,8 +374,8 @@ __global__ void rope_table_kernel(float* freqs, int Tlen, int half, float theta)
 // rounds) 16384 x 18944 309 / 285 and 585 / 456, 4096 x 4864 22.8 / 21.9 and 38.7 / 33.0, 2000 x 13824 29.6 / 27.2 and 51.0 / 43.7, 512 x 8192 the same
 // grid.  One round per block: 336 and 501.  SwiGLU to e4m3, 4 / 8 rounds: 4096 x 4864 21.1 / 23.2, 3000 x 8192 24.3 / 26.0, 2048 x 18944 36.2 / 36.8,
 // 16384 x 18944 255 / 249.  RoPE, 2 / 4 rounds: 8 x 2048 x 36 x 128 46.6 / 47.6, 1 x 8192 x 48 x 128 32.4 / 33.5, smaller ones the same.
-int grid_for(long long work_items, int num_sms, int per_block) {
-    const long long blocks = ceil_div_ll(work_items, 256), resident = static_cast<long long>(num_sms) * 8;
+int grid_for(long long work_items, int num_sms, int per_block, int threads = 256) {
+    const long long blocks = ceil_div_ll(work_items, threads), resident = static_cast<long long>(num_sms) * (2048 / threads);
     long long g = ceil_div_ll(blocks, per_block);
     if (g < resident) g = blocks < resident ? blocks : resident;
     if (g > (1ll << 30)) g = 1ll << 30;
@@ -425,9 +426,9 @@ static int launch_rope(void* out, const void* inp, const float* freqs, int B, in
     p.vec = FastDiv(vecs); p.lane = FastDiv(p.lanes); p.tokens = FastDiv(T_);
     p.total = static_cast<long long>(B) * T_ * p.lanes * vecs;
     p.wide = reinterpret_cast<uintptr_t>(freqs) % 16 == 0;
-    const int g = grid_for(p.total, num_sms, kRopeRounds);
-    if (backward) launch_chained(rope_kernel<T, true>, g, 256, 0, s, static_cast<T*>(out), static_cast<const T*>(inp), freqs, p, absmax);
-    else          launch_chained(rope_kernel<T, false>, g, 256, 0, s, static_cast<T*>(out), static_cast<const T*>(inp), freqs, p, absmax);
+    const int g = grid_for(p.total, num_sms, kRopeRounds, kRopeThreads);
+    if (backward) launch_chained(rope_kernel<T, true>, g, kRopeThreads, 0, s, static_cast<T*>(out), static_cast<const T*>(inp), freqs, p, absmax);
+    else          launch_chained(rope_kernel<T, false>, g, kRopeThreads, 0, s, static_cast<T*>(out), static_cast<const T*>(inp), freqs, p, absmax);
     return LLMQ_LAUNCH_CHECK();
 }
 

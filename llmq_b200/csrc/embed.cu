@@ -185,7 +185,8 @@ bias_bwd_partial_vec4_kernel(float* __restrict__ partial, const T* __restrict__ 
 // (four per thread); a CTA takes eight slices of the rows, of which every thread walks through all at once, so that eight loads of it are under way.  The
 // sums of the 64 slices of a column meet in distributed shared memory; each CTA ends 16 columns.  For small gradients, where the second launch and its
 // latency are what counts: 1001 x 1152 bf16 5.5 / 3.8 us, 256 x 1152 5.2 / 3.3;  4096 x 1152 6.4 / 6.7, and with more than one round of clusters or more
-// rows per CTA the two kernels have four times the warps: 16384 x 4608 29 / 82, 300 x 37888 21 / 38.
+// rows per CTA the two kernels have four times the warps: 16384 x 4608 29 / 82, 300 x 37888 21 / 38.  8-bit elements, whose conversions count, 1024 x 896
+// 5.2 / 4.9, 1536 x 896 5.2 / 6.0.
 constexpr int kBiasSlices = 64, kBiasCtas = 8, kBiasOwn = kBiasSlices / kBiasCtas;
 template <typename T, typename D>
 __global__ void __launch_bounds__(256)
@@ -311,7 +312,7 @@ extern "C" int llmq_bias_backward(void* dbias, float* partial, const void* dout,
     if (dbias_dtype != 0 && dbias_dtype != 3) return -10;
     const bool vec4 = C % 4 == 0 && reinterpret_cast<uintptr_t>(dout) % 16 == 0;
     const int blocks = ceil_div_i(C, 128) * kBiasCtas;
-    if (vec4 && slices == kBiasSlices && rows <= 2048 && blocks <= 148) {
+    if (vec4 && slices == kBiasSlices && rows <= (dout_dtype == 1 || dout_dtype == 2 ? 1024 : 2048) && blocks <= 148) {
 #define BIAS_CLUSTER(T)                                                                                                \
     do {                                                                                                               \
         if (dbias_dtype == 0) launch_chained_cluster(bias_bwd_cluster_kernel<T, bf16>, blocks, 256, 0, s, kBiasCtas, static_cast<bf16*>(dbias), static_cast<const T*>(dout), rows, C, scale_a, scale_b, accumulate);   \

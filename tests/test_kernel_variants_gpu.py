@@ -387,6 +387,26 @@ def test_split_k_parts(M, N, Kd, parts, dt, out_dt):
     assert abs(am.item() - want.abs().max().item()) < 4e-3 * want.abs().max().item()
 
 
+# split K of outputs that fill their tiles partly: fewer rows than parts, rows and columns around the shares of a cluster's CTAs, 8 to 64 pieces of four columns
+@pytest.mark.parametrize("M,N", [(1, 16), (5, 264), (16, 32), (31, 40), (130, 72), (208, 136), (257, 304)])
+@pytest.mark.parametrize("Kd", [1216, 4096])
+@pytest.mark.parametrize("out_dt", [BF, torch.float32])
+def test_split_k_narrow(M, N, Kd, out_dt):
+    assert L.kernels().llmq_gemm_splitk_floats(M, N, Kd, 2, 148) > 0
+    g = torch.Generator(device=DEV).manual_seed(M)
+    a, b = torch.randn(M, Kd, device=DEV, generator=g).to(BF), torch.randn(N, Kd, device=DEV, generator=g).to(BF)
+    rows = torch.full((M + 1, N), 9.0, device=DEV, dtype=out_dt)
+    prev = torch.randn(M, N, device=DEV, generator=g).to(out_dt)
+    added = prev.clone()
+    K.gemm(rows[:M], a, b)
+    K.gemm(added, a, b, accumulate=True)
+    K.check_status(torch.device(DEV, 0))
+    prod = a.double() @ b.double().t()
+    eps = 1e-5 + (2 ** -8 if out_dt == BF else 0)             # fp32 sums, one rounding of the outputs
+    assert rel(rows[:M], prod) < eps and rel(added, prod + prev.double()) < eps
+    assert (rows[M] == 9).all()
+
+
 # the kernel for a plain GEMM on both sides of each line of the rule: short K (8 and 9 steps of 128 bytes), one round of tiles (64 / 65 steps, both operands MN-major
 # 16 / 17), more than half of the SMs idle (47 / 48 steps, from where K is cut in two); odd edges of the last tiles
 @pytest.mark.parametrize("M,N,steps,mn,parts", [(9728, 904, 8, 0, 1), (9728, 904, 9, 0, 1), (2320, 1160, 64, 0, 1), (2320, 1160, 65, 0, 1), (2056, 2064, 16, 1, 1),
