@@ -27,7 +27,7 @@ typedef __nv_fp8_e5m2 e5m2;
 // AdamW tables of 2.4 M elements 21.5 / 9.6, gradient norm, clipping and that AdamW 36.4 / 21.4, bias gradient 7308 x 1000 8.2 / 6.4, RoPE of 60 tokens 2.1 / 1.7,
 // RMSNorm forward 8165 x 512 9.2 / 6.1.  A kernel that waits for other GPUs must not call it.
 // Launched this way: attention, RoPE, GEMM, their small second passes, the embedding, the norm and the AdamW launches of an update.  A pass over
-// rope, attention forward, backward (three kernels) and rope, launched plainly / this way: 333 tokens, 12 / 2 heads of 128 in a graph 66 / 39, 8 x 1024
+// rope, attention forward, backward (then three kernels) and rope, launched plainly / this way: 333 tokens, 12 / 2 heads of 128 in a graph 66 / 39, 8 x 1024
 // tokens, 14 / 2 heads of 64 221 / 175.  The long streaming kernels (SwiGLU, RMSNorm, quantise, transposes, classifier) are not:
 // what the compiler loses by the two functions below costs them more than a launch (RMSNorm pass 186 -> 195 us, SwiGLU 793 -> 811).
 __device__ __forceinline__ void grid_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
