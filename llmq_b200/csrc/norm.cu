@@ -259,7 +259,7 @@ __device__ __forceinline__ void copy_row_async(uint32_t dst, const void* src, ui
                  ::"r"(dst), "l"(src), "r"(bytes), "r"(bar) : "memory");
 }
 
-// Same contract, for fp32 rows of two to four column vectors per thread: the row's dout, inp and residual gradient are loaded once and stay in
+// Same contract, for fp32 rows of two to four column vectors per thread, and for blocks with one or two rows of one: the row's dout, inp and residual gradient are loaded once and stay in
 // registers across the block-wide dot product.  4000 x 4096 51.6 us, 53.2 with the rows in shared memory (below), 1000 x 2048 12.2 / 13.2.
 template <typename T, int VPT>
 __global__ void __launch_bounds__(NORM_THREADS, VPT <= 2 ? 3 : 2)
@@ -548,7 +548,13 @@ int launch_bwd(void* dinp_, void* dweight, float* scratch, const void* dout_, co
     const T *dout = static_cast<const T*>(dout_), *inp = static_cast<const T*>(inp_), *w = static_cast<const T*>(w_);
     int rc;
     // stages and CTAs per SM: as much shared memory as fits
-    if (vecs <= 1) rc = launch_bwd_ring<T, 1, 4, 3>(dinp, scratch, dout, inp, w, rstd, rows, C, absmax, num_blocks, s);
+    // Blocks with one or two short rows have nothing to fetch ahead, and setting up the ring costs 0.3 us: us with / without it, bf16: 20 x 896 4.2 / 3.9, 113 x 1536 5.7 / 5.2,
+    // 888 x 256 7.3 / 7.0, 888 x 1024 9.1 / 9.1;  fp32 888 x 896 8.3 / 7.8.  More rows: 4096 x 896 bf16 13.8 / 16.3 (from HBM 15.2 / 18.4), fp32 13.2 / 15.7.
+    if (vecs <= 1 && rows <= 2 * num_blocks) {
+        rmsnorm_bwd_reg_kernel<T, 1><<<num_blocks, NORM_THREADS, 0, s>>>(dinp, scratch, dout, inp, w, rstd, rows, C, absmax);
+        rc = LLMQ_LAUNCH_CHECK();
+    }
+    else if (vecs <= 1) rc = launch_bwd_ring<T, 1, 4, 3>(dinp, scratch, dout, inp, w, rstd, rows, C, absmax, num_blocks, s);
     else if (vecs <= 4) {
         if constexpr (sizeof(T) == 2) {
             if (vecs <= 2) rc = launch_bwd_ring<T, 2, 3, 3>(dinp, scratch, dout, inp, w, rstd, rows, C, absmax, num_blocks, s);

@@ -904,6 +904,25 @@ def test_rmsnorm_backward_blocks(C, rows):
     assert rel(dw, dw0.double() + (dy.double() * xh).sum(0)) < 2**-8 and am.item() == dinp.float().abs().max().item()
 
 
+# short rows on both sides of two rows per block: one vector per thread, blocks of the whole GPU (three per SM) and of C > 1024 (one per SM)
+@pytest.mark.parametrize("C", [8, 256, 1000, 1024, 2048])
+@pytest.mark.parametrize("rows", [1, 296, 297, 444, 445, 888, 889])
+@pytest.mark.parametrize("dt", [BF, torch.float32])
+def test_rmsnorm_backward_few_rows(C, rows, dt):
+    g = torch.Generator(device=DEV).manual_seed(C + rows)
+    x, w, dy, dres, dw0 = (torch.randn(*s, device=DEV, generator=g).to(dt) for s in ((rows, C), (C,), (rows, C), (rows, C), (C,)))
+    rs = torch.rsqrt(x.double().square().mean(-1, keepdim=True) + 1e-6)
+    dinp, dw, am = dres.clone(), dw0.clone(), torch.zeros(1, device=DEV)
+    scratch = torch.full((K.rmsnorm_backward_scratch_elems(C, torch.device(DEV, 0)),), math.nan, device=DEV)
+    K.rmsnorm_backward(dinp, dw, scratch, dy, x, w, rs[:, 0].float().contiguous(), absmax=am)
+    xh, wdy = x.double() * rs, w.double() * dy.double()
+    gx = dres.double() + (wdy - xh * (wdy * xh).mean(-1, keepdim=True)) * rs
+    # as above: one rounding of the output, fp32 arithmetic on terms of a few units
+    eps = 2**-8 if dt == BF else 2**-20
+    assert ((dinp.double() - gx).abs() <= gx.abs() * eps + 1e-5 * (1 + wdy.abs() * rs)).all()
+    assert rel(dw, dw0.double() + (dy.double() * xh).sum(0)) < (2**-8 if dt == BF else 1e-5) and am.item() == dinp.float().abs().max().item()
+
+
 # the bias gradient in one launch (columns in fours) against the two kernels that take unaligned gradients: the same sums in the same order; rows around
 # multiples of 8 and 512, columns around multiples of 16 and 128
 @pytest.mark.parametrize("rows", [1, 7, 65, 511, 513, 1001, 3000])
