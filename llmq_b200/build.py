@@ -6,8 +6,8 @@ Shared libraries are produced under ``llmq_b200/lib``:
 * ``libllmq_b200_rt.so``      - host-side runtime: token-file data loader, safetensors writer,
   bump/stack arena bookkeeping, pinned staging helpers (``csrc/rt/*.cpp``)
 
-and, where torch and the headers of Python are at hand, ``llmq_b200_binding.so``, an extension module for the interpreter that runs the
-build (``csrc/py/binding.cpp``); without it the same kernels are called through ctypes, with more host time per call.
+and, where torch and the headers of Python are at hand, ``llmq_b200_binding.<interpreter tag>.so``, an extension module for the interpreter that
+runs the build and for its torch (``csrc/py/binding.cpp``); without it the same kernels are called through ctypes, with more host time per call.
 
 The build is incremental (object files are rebuilt only when a source or header is newer) and
 needs no GPU: nvcc cross-compiles.  Run ``python -m llmq_b200.build`` or call :func:`build`.
@@ -15,6 +15,7 @@ needs no GPU: nvcc cross-compiles.  Run ``python -m llmq_b200.build`` or call :f
 from __future__ import annotations
 
 import os
+import re
 import subprocess
 import sys
 from concurrent.futures import ThreadPoolExecutor
@@ -93,7 +94,8 @@ def _build_binding(verbose: bool, force: bool) -> None:
     import importlib.util
     import sysconfig
 
-    src, out = CSRC / "py" / "binding.cpp", LIBDIR / "llmq_b200_binding.so"
+    # the interpreter's tag is in the name: another one builds a file of its own
+    src, out = CSRC / "py" / "binding.cpp", LIBDIR / ("llmq_b200_binding" + (sysconfig.get_config_var("EXT_SUFFIX") or ".so"))
     torch_spec = importlib.util.find_spec("torch")
     python_inc = sysconfig.get_paths()["include"]
     if torch_spec is None or not os.path.exists(os.path.join(python_inc, "Python.h")):
@@ -102,9 +104,10 @@ def _build_binding(verbose: bool, force: bool) -> None:
     if not (torch_dir / "include" / "torch" / "csrc" / "autograd" / "python_variable.h").exists():
         return
     version = torch_dir / "version.py"
-    if not force and out.exists() and out.stat().st_mtime > max(src.stat().st_mtime, version.stat().st_mtime if version.exists() else 0.0):
+    found = re.search(r"""^__version__\s*=\s*['"]([^'"]+)['"]""", version.read_text(), re.M) if version.exists() else None
+    if found is None or not force and out.exists() and out.stat().st_mtime > max(src.stat().st_mtime, version.stat().st_mtime):
         return
-    cmd = ["g++", "-O2", "-std=c++20", "-fPIC", "-shared", "-Wall", "-I", str(torch_dir / "include"), "-I", str(torch_dir / "include/torch/csrc/api/include"),
+    cmd = ["g++", "-O2", "-std=c++20", "-fPIC", "-shared", "-Wall", f'-DLLMQ_TORCH_VERSION="{found.group(1)}"', "-I", str(torch_dir / "include"), "-I", str(torch_dir / "include/torch/csrc/api/include"),
            "-I", python_inc, "-I", "/usr/local/cuda/include", str(src), "-o", str(out), f"-L{torch_dir / 'lib'}", "-ltorch_python", "-ltorch_cpu", "-lc10",
            "-lc10_cuda", f"-Wl,-rpath,{torch_dir / 'lib'}"]
     _compile(cmd, src, out, verbose)

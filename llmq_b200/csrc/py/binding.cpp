@@ -257,4 +257,9 @@ PyModuleDef module = {PyModuleDef_HEAD_INIT, "llmq_b200_binding", nullptr, -1, m
 
 }  // namespace
 
-PyMODINIT_FUNC PyInit_llmq_b200_binding() { return PyModule_Create(&module); }
+// torch_version: the one that this file was compiled against, which the loader compares with the one at hand
+PyMODINIT_FUNC PyInit_llmq_b200_binding() {
+    PyObject* m = PyModule_Create(&module);
+    if (m && PyModule_AddStringConstant(m, "torch_version", LLMQ_TORCH_VERSION) < 0) Py_CLEAR(m);
+    return m;
+}

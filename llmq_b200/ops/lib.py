@@ -9,7 +9,9 @@ from __future__ import annotations
 import ctypes
 import importlib.util
 import os
+import sysconfig
 import threading
+import warnings
 from pathlib import Path
 from types import SimpleNamespace
 
@@ -74,19 +76,41 @@ SIGNATURES = {
 _CTYPES = {"p": ctypes.c_void_p, "i": ctypes.c_int, "u": ctypes.c_uint, "l": ctypes.c_longlong, "f": ctypes.c_float, "d": ctypes.c_double}
 
 
+# Name of the extension module for this interpreter
+BINDING_FILE = "llmq_b200_binding" + (sysconfig.get_config_var("EXT_SUFFIX") or ".so")
+
+
+def _load_binding(path: Path):
+    """The extension module at ``path``; ImportError where it is not one for this torch and these entry points.
+
+    It reads tensors through torch's inline accessors and calls the C functions with the argument types it was compiled with, so it is
+    used with the very torch that it was compiled against and with the entry points of SIGNATURES, or not at all."""
+    spec = importlib.util.spec_from_file_location("llmq_b200_binding", path)
+    module = importlib.util.module_from_spec(spec)
+    spec.loader.exec_module(module)
+    if module.torch_version != str(torch.__version__):
+        raise ImportError(f"compiled against torch {module.torch_version}, this is {torch.__version__}")
+    if module.signatures() != SIGNATURES:
+        raise ImportError("its entry points are not those of this package")
+    return module
+
+
 def binding():
-    """The extension module of ``csrc/py/binding.cpp``, or None where it was not built (it needs the headers of torch and Python)."""
+    """The extension module of ``csrc/py/binding.cpp``, or None where there is none that loads (it needs the headers of torch and Python, and fits one
+    interpreter and one torch); the same kernels are then called through ctypes."""
     global _binding
     if _binding is None:
         with _lock:
             if _binding is None:
                 found = False
-                for path in (_LIBDIR / "llmq_b200_binding.so", _PKG_LIBDIR / "llmq_b200_binding.so"):
-                    if path.exists():
-                        spec = importlib.util.spec_from_file_location("llmq_b200_binding", path)
-                        found = importlib.util.module_from_spec(spec)
-                        spec.loader.exec_module(found)
+                for path in dict.fromkeys((_LIBDIR / BINDING_FILE, _PKG_LIBDIR / BINDING_FILE)):
+                    if not path.exists():
+                        continue
+                    try:
+                        found = _load_binding(path)
                         break
+                    except (ImportError, OSError, AttributeError) as e:
+                        warnings.warn(f"{path} is not used, calls go through ctypes: {e}; run `python -m llmq_b200.build`", RuntimeWarning, stacklevel=2)
                 _binding = found
     return _binding or None
 

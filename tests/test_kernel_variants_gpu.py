@@ -1042,3 +1042,22 @@ def test_rmsnorm_backward_ring_turns(C, rows):
     # every element: one rounding to bf16 (2^-9 of it) and fp32 arithmetic on terms of a few units
     assert ((dinp.double() - gx).abs() <= gx.abs() * 2**-8 + 1e-5 * (1 + wdy.abs() * rs)).all()
     assert rel(dw, dw0.double() + (dy.double() * xh).sum(0)) < 2**-8 and am.item() == dinp.float().abs().max().item()
+
+
+# the entry points through ctypes, for installations whose extension module does not load: the same kernels and results
+def test_calls_through_ctypes(monkeypatch):
+    g = torch.Generator(device=DEV).manual_seed(3)
+    a, b = torch.randn(130, 512, device=DEV, generator=g).to(BF), torch.randn(96, 512, device=DEV, generator=g).to(BF)
+    qkv, table = torch.randn(1, 70, 8, 64, device=DEV, generator=g).to(BF), K.rope_table(70, 64, 1e4, torch.device(DEV, 0))
+    got = []
+    for native in (True, False):
+        if not native:
+            monkeypatch.setattr(L, "_calls", None)
+            monkeypatch.setattr(L, "binding", lambda: None)
+        out, rot, am = torch.zeros(130, 96, device=DEV, dtype=BF), torch.empty_like(qkv), torch.zeros(1, device=DEV)
+        att, lse = torch.empty(1, 70, 4, 64, device=DEV, dtype=BF), torch.empty(1, 4, 70, device=DEV)
+        K.gemm(out, a, b, alpha=0.5, absmax=am)
+        K.rope(rot, qkv, table, 4, 2)
+        K.attention_forward(att, lse, rot, 4, 2)
+        got.append((out, rot, am, att, lse))
+    assert all(torch.equal(x, y) for x, y in zip(*got)) and got[0][2].item() > 0
