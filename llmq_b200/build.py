@@ -6,7 +6,7 @@ Shared libraries are produced under ``llmq_b200/lib``:
 * ``libllmq_b200_rt.so``      - host-side runtime: token-file data loader, safetensors writer,
   bump/stack arena bookkeeping, pinned staging helpers (``csrc/rt/*.cpp``)
 
-and, where torch and the headers of Python are at hand, ``llmq_b200_binding.<interpreter tag>.so``, an extension module for the interpreter that
+and, where a torch with CUDA and the headers of Python are at hand, ``llmq_b200_binding.<interpreter tag>.so``, an extension module for the interpreter that
 runs the build and for its torch (``csrc/py/binding.cpp``); without it the same kernels are called through ctypes, with more host time per call.
 
 The build is incremental (object files are rebuilt only when a source or header is newer) and
@@ -90,7 +90,7 @@ def build(verbose: bool = False, force: bool = False) -> None:
 
 
 def _build_binding(verbose: bool, force: bool) -> None:
-    """The extension module, for this interpreter and its torch."""
+    """The extension module, for this interpreter and its torch; optional, so that nothing here makes the build fail."""
     import importlib.util
     import sysconfig
 
@@ -101,7 +101,8 @@ def _build_binding(verbose: bool, force: bool) -> None:
     if torch_spec is None or not os.path.exists(os.path.join(python_inc, "Python.h")):
         return
     torch_dir = Path(torch_spec.origin).parent
-    if not (torch_dir / "include" / "torch" / "csrc" / "autograd" / "python_variable.h").exists():
+    needed = ("include/torch/csrc/autograd/python_variable.h", "include/c10/cuda/CUDAStream.h", "lib/libc10_cuda.so")      # a torch without CUDA lacks the last two
+    if not all((torch_dir / f).exists() for f in needed):
         return
     version = torch_dir / "version.py"
     found = re.search(r"""^__version__\s*=\s*['"]([^'"]+)['"]""", version.read_text(), re.M) if version.exists() else None
@@ -110,7 +111,11 @@ def _build_binding(verbose: bool, force: bool) -> None:
     cmd = ["g++", "-O2", "-std=c++20", "-fPIC", "-shared", "-Wall", f'-DLLMQ_TORCH_VERSION="{found.group(1)}"', "-I", str(torch_dir / "include"), "-I", str(torch_dir / "include/torch/csrc/api/include"),
            "-I", python_inc, "-I", "/usr/local/cuda/include", str(src), "-o", str(out), f"-L{torch_dir / 'lib'}", "-ltorch_python", "-ltorch_cpu", "-lc10",
            "-lc10_cuda", f"-Wl,-rpath,{torch_dir / 'lib'}"]
-    _compile(cmd, src, out, verbose)
+    try:
+        _compile(cmd, src, out, verbose)
+    except (RuntimeError, OSError) as e:
+        out.unlink(missing_ok=True)
+        print(f"{out.name} was not built, kernels are called through ctypes: {e}", file=sys.stderr)
 
 
 def build_tests(verbose: bool = False) -> Path:
