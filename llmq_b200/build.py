@@ -118,8 +118,19 @@ def _build_binding(verbose: bool, force: bool) -> None:
         print(f"{out.name} was not built, kernels are called through ctypes: {e}", file=sys.stderr)
 
 
+def build_lost_row(row: int = 300, verbose: bool = False) -> Path:
+    """``build/norm_lost_row.so``: the norm kernels with a wait limit of 20 ms, of which the RMSNorm backward never gets the row ``row`` into shared memory."""
+    src, out = CSRC / "norm.cu", PKG.parent / "build" / "norm_lost_row.so"
+    if not out.exists() or out.stat().st_mtime < max(src.stat().st_mtime, _newest_header_mtime([CSRC])):
+        out.parent.mkdir(parents=True, exist_ok=True)
+        cmd = [_nvcc(), *NVCC_FLAGS, "-shared", f"-DLLMQ_TEST_LOST_ROW={row}", "-DLLMQ_WAIT_LIMIT_NS=20000000ull", "-I", str(CSRC), str(src), "-o", str(out)]
+        _compile(cmd, src, out, verbose)
+    return out
+
+
 def build_tests(verbose: bool = False) -> Path:
-    """Native unit-test executable ``build/test_kernels`` (``csrc/tests/test_kernels.cu``), linked against the kernels library."""
+    """Native unit-test executable ``build/test_kernels`` (``csrc/tests/test_kernels.cu``), linked against the kernels library,
+    and the library of :func:`build_lost_row`."""
     build(verbose=verbose)
     exe = PKG.parent / "build" / "test_kernels"
     src = CSRC / "tests" / "test_kernels.cu"
@@ -128,6 +139,7 @@ def build_tests(verbose: bool = False) -> Path:
         cmd = [_nvcc(), "-gencode", "arch=compute_100a,code=sm_100a", "-O2", "-std=c++17", str(src), "-o", str(exe),
                "-L", str(LIBDIR), "-lllmq_b200_kernels", "-Xlinker", "-rpath", "-Xlinker", "$ORIGIN/../llmq_b200/lib"]
         _compile(cmd, src, exe, verbose)
+    build_lost_row(verbose=verbose)
     return exe
 
 

@@ -336,29 +336,58 @@ rmsnorm_bwd_reg_kernel(T* __restrict__ dinp, float* __restrict__ dw_partial, con
     block_absmax_commit(absmax_out, tmax, scratch);
 }
 
+// Waits for a row's copies; false when the limit ran out, in this thread or (in later rows) in another one
+__device__ __forceinline__ bool row_wait(uint32_t bar, uint32_t parity, volatile uint32_t* gave_up) {
+    return sm100::mbar_try_wait(bar, parity) || (!*gave_up && sm100::mbar_wait(bar, parity, gave_up));
+}
+
+// The end of a block whose copies did not come: what may still be under way, the copies of the STAGES rows from `first_lost` on, has to land before the block
+// gives its shared memory back, and its rows become NaN
+template <int STAGES, typename T>
+__device__ __noinline__ void give_up_rows(T* dinp, int rows, int C, uint32_t full, long long first_lost) {
+    const long long step = gridDim.x;
+    if (threadIdx.x == 0) {
+        const uint64_t t0 = sm100::globaltimer_ns();
+        long long n = (first_lost - blockIdx.x) / step;
+        for (int i = 0; i < STAGES; ++i, ++n)
+            while (blockIdx.x + n * step < rows && !sm100::mbar_try_wait(full + 8 * static_cast<uint32_t>(n % STAGES), (n / STAGES) & 1) &&
+                   sm100::globaltimer_ns() - t0 < sm100::kWaitLimitNs) {}
+    }
+    for (long long row = blockIdx.x; row < rows; row += step)
+        for (int c = threadIdx.x; c < C; c += NORM_THREADS) dinp[row * C + c] = from_float<T>(NAN);
+}
+
 // Same contract, for rows of up to 4 column vectors per thread.  Rows to come are on their way into shared memory: three bulk copies per row, issued by one
 // thread, so that neither registers nor load instructions are spent on what is in flight, and the registers hold the weight gradient and little
 // else (both passes over a row read it from shared memory).  One barrier per row; it also says that the row before has been read, whose place the next
 // copies take.  Memory is the limit for long rows.  us, rows in registers (two vectors a thread) or copied thread by thread (one, four) / now:
 // 16384 x 3584, 470 MB, 98.7 / 77.9;  16384 x 3072 91 / 71;  4096 x 3584 31.6 / 30.3;  16384 x 5120 191 / 146;  4000 x 8192 91 / 66;  16384 x 2048 66 / 54;  16384 x 896 42.5 / 37.5;
 // 4096 x 896 16.3 / 14.7;  fp32 4096 x 896 18.7 / 17.3.  Two rows per turn and barrier, with two CTAs per SM: 16384 x 3584 84.
+// A copy that does not come within the limit of the waits: the status word says so, and the weight gradient and all rows of its block become NaN, so that
+// callers without a status word see it too.  (Leaving the loop there costs 1 to 10 % where nothing is wrong.)
 template <typename T, int VPT, int STAGES, int CTAS>
 __global__ void __launch_bounds__(NORM_THREADS, CTAS)
 rmsnorm_bwd_ring_kernel(T* __restrict__ dinp, float* __restrict__ dw_partial, const T* __restrict__ dout, const T* __restrict__ inp,
-                        const T* __restrict__ weight, const float* __restrict__ rstd, int rows, int C, float* __restrict__ absmax_out) {
+                        const T* __restrict__ weight, const float* __restrict__ rstd, int rows, int C, float* __restrict__ absmax_out,
+                        unsigned int* __restrict__ status) {
     __shared__ float scratch[32];
     static_assert(STAGES >= 2, "the row in use and the ones on their way");
     __shared__ float dots[2][NORM_THREADS / 32];             // alternating, so that one barrier per row is enough
     extern __shared__ __align__(16) uint8_t ring[];          // [STAGES][dout, inp, dinp][C]
     __shared__ uint64_t full[STAGES];
     __shared__ uint32_t gave_up;
+    __shared__ long long first_lost;                         // where thread 0's wait ran out
     using V = Vec16<T>;
     float dw[VPT][V::N];
     V vw[VPT];
     const uint32_t row_bytes = C * sizeof(T);
+    int fetch_end = rows;
     auto slot = [&](int stage, int what) { return ring + (stage * 3 + what) * row_bytes; };
     auto fetch = [&](long long row, int stage) {             // one thread
-        if (row < rows) {
+#ifdef LLMQ_TEST_LOST_ROW
+        if (row == LLMQ_TEST_LOST_ROW) return;               // builds for tests: a row whose copies never come
+#endif
+        if (row < fetch_end) {
             const uint32_t bar = sm100::smem_u32(full + stage);
             sm100::mbar_expect_tx(bar, 3 * row_bytes);
             copy_row_async(sm100::smem_u32(slot(stage, 0)), dout + row * C, row_bytes, bar);
@@ -370,6 +399,7 @@ rmsnorm_bwd_ring_kernel(T* __restrict__ dinp, float* __restrict__ dw_partial, co
     if (threadIdx.x == 0) {
         for (int st = 0; st < STAGES; ++st) sm100::mbar_init(sm100::smem_u32(full + st), 1);
         gave_up = 0;
+        first_lost = rows;
         sm100::mbar_init_fence();
         for (int st = 0; st < STAGES; ++st) fetch(blockIdx.x + st * step, st);
     }
@@ -385,11 +415,13 @@ rmsnorm_bwd_ring_kernel(T* __restrict__ dinp, float* __restrict__ dw_partial, co
     const float inv_c = 1.f / C;
     int par = 0, stage = 0;
     uint32_t phase = 0;
-    bool ok = true;
     for (long long row = blockIdx.x; row < rows; row += step, par ^= 1) {
         const float rs = rstd[row];
         float dot = 0.f;
-        ok = sm100::mbar_wait(sm100::smem_u32(full + stage), phase, &gave_up) && ok;
+        if (!row_wait(sm100::smem_u32(full + stage), phase, &gave_up)) {
+            if (threadIdx.x == 0 && fetch_end) first_lost = row;
+            fetch_end = 0;                                   // nothing is fetched any more
+        }
 #pragma unroll
         for (int k = 0; k < VPT; ++k) {
             const int c = (k * NORM_THREADS + threadIdx.x) * V::N;
@@ -429,12 +461,19 @@ rmsnorm_bwd_ring_kernel(T* __restrict__ dinp, float* __restrict__ dw_partial, co
         }
         if (++stage == STAGES) { stage = 0; phase ^= 1u; }
     }
+    // Set before the barrier of a row, so the same for all threads here
+    const bool lost = *static_cast<volatile uint32_t*>(&gave_up) != 0;
+    if (lost) {
+        tmax = 0.f;
+        if (threadIdx.x == 0 && status) atomicOr(status, static_cast<unsigned int>(sm100::kErrOther));
+        give_up_rows<STAGES>(dinp, rows, C, sm100::smem_u32(full), first_lost);
+    }
 #pragma unroll
     for (int k = 0; k < VPT; ++k) {
         const int c = (k * NORM_THREADS + threadIdx.x) * V::N;
         if (c < C) {
 #pragma unroll
-            for (int i = 0; i < V::N; ++i) dw_partial[static_cast<long long>(blockIdx.x) * C + c + i] = ok ? dw[k][i] : NAN;      // a copy that never came shows
+            for (int i = 0; i < V::N; ++i) dw_partial[static_cast<long long>(blockIdx.x) * C + c + i] = lost ? NAN : dw[k][i];
         }
     }
     block_absmax_commit(absmax_out, tmax, scratch);
@@ -514,7 +553,7 @@ int device_sms() {
 }
 
 template <typename T, int VPT, int STAGES, int CTAS>
-int launch_bwd_ring(T* dinp, float* scratch, const T* dout, const T* inp, const T* w, const float* rstd, int rows, int C, float* absmax, int blocks, cudaStream_t s) {
+int launch_bwd_ring(T* dinp, float* scratch, const T* dout, const T* inp, const T* w, const float* rstd, int rows, int C, float* absmax, int blocks, unsigned int* status, cudaStream_t s) {
     static bool attr_set[64] = {};          // per device
     int dev = 0;
     cudaGetDevice(&dev);
@@ -523,13 +562,13 @@ int launch_bwd_ring(T* dinp, float* scratch, const T* dout, const T* inp, const 
         if (e != cudaSuccess) return static_cast<int>(e);
         attr_set[dev & 63] = true;
     }
-    rmsnorm_bwd_ring_kernel<T, VPT, STAGES, CTAS><<<blocks, NORM_THREADS, STAGES * 3 * C * sizeof(T), s>>>(dinp, scratch, dout, inp, w, rstd, rows, C, absmax);
+    rmsnorm_bwd_ring_kernel<T, VPT, STAGES, CTAS><<<blocks, NORM_THREADS, STAGES * 3 * C * sizeof(T), s>>>(dinp, scratch, dout, inp, w, rstd, rows, C, absmax, status);
     return LLMQ_LAUNCH_CHECK();
 }
 
 template <typename T>
 int launch_bwd(void* dinp_, void* dweight, float* scratch, const void* dout_, const void* inp_, const void* w_,
-               const float* rstd, int rows, int C, float* absmax, int accumulate_dw, int num_blocks, cudaStream_t s) {
+               const float* rstd, int rows, int C, float* absmax, int accumulate_dw, int num_blocks, unsigned int* status, cudaStream_t s) {
     using V = Vec16<T>;
     if (C % V::N) return -1;
     const int vecs = ceil_div_i(C / V::N, NORM_THREADS);
@@ -554,11 +593,11 @@ int launch_bwd(void* dinp_, void* dweight, float* scratch, const void* dout_, co
         rmsnorm_bwd_reg_kernel<T, 1><<<num_blocks, NORM_THREADS, 0, s>>>(dinp, scratch, dout, inp, w, rstd, rows, C, absmax);
         rc = LLMQ_LAUNCH_CHECK();
     }
-    else if (vecs <= 1) rc = launch_bwd_ring<T, 1, 4, 3>(dinp, scratch, dout, inp, w, rstd, rows, C, absmax, num_blocks, s);
+    else if (vecs <= 1) rc = launch_bwd_ring<T, 1, 4, 3>(dinp, scratch, dout, inp, w, rstd, rows, C, absmax, num_blocks, status, s);
     else if (vecs <= 4) {
         if constexpr (sizeof(T) == 2) {
-            if (vecs <= 2) rc = launch_bwd_ring<T, 2, 3, 3>(dinp, scratch, dout, inp, w, rstd, rows, C, absmax, num_blocks, s);
-            else           rc = launch_bwd_ring<T, 4, 2, 2>(dinp, scratch, dout, inp, w, rstd, rows, C, absmax, num_blocks, s);
+            if (vecs <= 2) rc = launch_bwd_ring<T, 2, 3, 3>(dinp, scratch, dout, inp, w, rstd, rows, C, absmax, num_blocks, status, s);
+            else           rc = launch_bwd_ring<T, 4, 2, 2>(dinp, scratch, dout, inp, w, rstd, rows, C, absmax, num_blocks, status, s);
         } else {
             if (vecs <= 2) rmsnorm_bwd_reg_kernel<T, 2><<<num_blocks, NORM_THREADS, 0, s>>>(dinp, scratch, dout, inp, w, rstd, rows, C, absmax);
             else           rmsnorm_bwd_reg_kernel<T, 4><<<num_blocks, NORM_THREADS, 0, s>>>(dinp, scratch, dout, inp, w, rstd, rows, C, absmax);
@@ -585,13 +624,13 @@ extern "C" int llmq_rmsnorm_forward(void* residual_out, void* y_out, void* q_out
     return -10;
 }
 
-// scratch must hold num_blocks * C floats.
+// scratch must hold num_blocks * C floats.  status: optional device word that takes a bit when a wait of the kernel runs out.
 extern "C" int llmq_rmsnorm_backward(void* dinp, void* dweight, float* scratch, const void* dout, const void* inp,
                                      const void* weight, const float* rstd, int rows, int C, int dtype, float* absmax,
-                                     int accumulate_dweight, int num_blocks, cudaStream_t stream) {
+                                     int accumulate_dweight, int num_blocks, unsigned int* status, cudaStream_t stream) {
     if (rows <= 0) return 0;
-    if (dtype == 0) return launch_bwd<bf16>(dinp, dweight, scratch, dout, inp, weight, rstd, rows, C, absmax, accumulate_dweight, num_blocks, stream);
-    if (dtype == 3) return launch_bwd<float>(dinp, dweight, scratch, dout, inp, weight, rstd, rows, C, absmax, accumulate_dweight, num_blocks, stream);
+    if (dtype == 0) return launch_bwd<bf16>(dinp, dweight, scratch, dout, inp, weight, rstd, rows, C, absmax, accumulate_dweight, num_blocks, status, stream);
+    if (dtype == 3) return launch_bwd<float>(dinp, dweight, scratch, dout, inp, weight, rstd, rows, C, absmax, accumulate_dweight, num_blocks, status, stream);
     return -10;
 }
 
@@ -640,7 +679,7 @@ extern "C" int llmq_rmsnorm_backward_noalloc(void* dinp, void* dweight, const vo
     const long long fit = LLMQ_NOALLOC_SCRATCH_FLOATS / C;
     if (blocks > fit) blocks = fit;
     if (blocks < 1) return LLMQ_NOALLOC_ERR_TOO_LARGE;
-    if (dtype == 0) return launch_bwd<bf16>(dinp, dweight, scratch, dout, inp, weight, rstd, rows, C, absmax, accumulate_dweight, static_cast<int>(blocks), stream);
-    if (dtype == 3) return launch_bwd<float>(dinp, dweight, scratch, dout, inp, weight, rstd, rows, C, absmax, accumulate_dweight, static_cast<int>(blocks), stream);
+    if (dtype == 0) return launch_bwd<bf16>(dinp, dweight, scratch, dout, inp, weight, rstd, rows, C, absmax, accumulate_dweight, static_cast<int>(blocks), nullptr, stream);
+    if (dtype == 3) return launch_bwd<float>(dinp, dweight, scratch, dout, inp, weight, rstd, rows, C, absmax, accumulate_dweight, static_cast<int>(blocks), nullptr, stream);
     return -10;
 }

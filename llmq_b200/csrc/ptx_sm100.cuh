@@ -112,8 +112,11 @@ __device__ __forceinline__ bool mbar_test_wait(uint32_t bar, uint32_t parity) {
 // launched while the kernel before it runs is put where there is room; two on one SM would run one after the other, with another SM idle.
 constexpr int one_block_per_sm(int bytes) { return bytes > 116 * 1024 ? bytes : 116 * 1024; }
 
-// Limit for every device-side wait, in nanoseconds of the global timer.
-constexpr uint64_t kWaitLimitNs = 2000ull * 1000ull * 1000ull;
+// Limit for every device-side wait, in nanoseconds of the global timer (builds for tests of waits that run out have a shorter one).
+#ifndef LLMQ_WAIT_LIMIT_NS
+#define LLMQ_WAIT_LIMIT_NS (2000ull * 1000ull * 1000ull)
+#endif
+constexpr uint64_t kWaitLimitNs = LLMQ_WAIT_LIMIT_NS;
 
 // Waits for the phase with the given parity to complete.  Returns false when the limit ran out
 // or when another thread of the CTA already flagged an abort (abort_flag lives in shared memory).

@@ -113,7 +113,7 @@ struct Entry {
 #define LLMQ_ENTRIES(X)                                                                                                              \
     X(llmq_gemm_ready, P, P, P, P, int, int, int, int, int, int, int, LL, LL, LL, int, int, int, P, P, float, P, P, int, P, unsigned int, int, double, P, LL) \
     X(llmq_rmsnorm_forward, P, P, P, P, P, P, P, float, int, int, int, P, P, P)                                                      \
-    X(llmq_rmsnorm_backward, P, P, P, P, P, P, P, int, int, int, P, int, int)                                                        \
+    X(llmq_rmsnorm_backward, P, P, P, P, P, P, P, int, int, int, P, int, int, P)                                                     \
     X(llmq_swiglu_forward, P, P, P, LL, int, int, P, P, P, int)                                                                      \
     X(llmq_swiglu_backward, P, P, P, LL, int, int, P, int)                                                                           \
     X(llmq_rope, P, P, P, int, int, int, int, int, int, int, P, int)                                                                 \

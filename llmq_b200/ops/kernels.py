@@ -359,7 +359,7 @@ def rmsnorm_backward(dinp: torch.Tensor, dweight: torch.Tensor, scratch: Optiona
         assert scratch is not None and scratch.numel() >= blocks * C and scratch.dtype == torch.float32
         rc = L.calls().llmq_rmsnorm_backward(
             dinp, dweight, scratch, dout, inp, weight, rstd, rows, C,
-            L.dtype_code(inp.dtype), absmax, int(accumulate_dweight), blocks)
+            L.dtype_code(inp.dtype), absmax, int(accumulate_dweight), blocks, status_word(inp.device))
         L.check(rc, "rmsnorm_backward")
         return
     x = inp.float().reshape(rows, C)

@@ -1061,3 +1061,32 @@ def test_calls_through_ctypes(monkeypatch):
         K.attention_forward(att, lse, rot, 4, 2)
         got.append((out, rot, am, att, lse))
     assert all(torch.equal(x, y) for x, y in zip(*got)) and got[0][2].item() > 0
+
+
+# a row whose copies never come (a build of the kernel that does not issue those of row 300, with a limit of 20 ms): the block that waits for it ends, the status word and NaNs in the weight
+# gradient and in all rows of that block say so, and no other row differs
+@pytest.mark.parametrize("C,rows", [(896, 2000), (3584, 1001), (5120, 700)])
+def test_rmsnorm_backward_lost_copy(C, rows):
+    import ctypes
+    from llmq_b200.build import build_lost_row
+    g = torch.Generator(device=DEV).manual_seed(C)
+    x, w, dy, dres = (torch.randn(*s, device=DEV, generator=g).to(BF) for s in ((rows, C), (C,), (rows, C), (rows, C)))
+    rs = torch.rsqrt(x.float().square().mean(-1) + 1e-6)
+    want, scratch = dres.clone(), torch.zeros(K.rmsnorm_backward_scratch_elems(C, torch.device(DEV, 0)), device=DEV)
+    K.rmsnorm_backward(want, torch.zeros_like(w), scratch, dy, x, w, rs)
+    lossy = L._through_ctypes(ctypes.CDLL(str(build_lost_row(300))).llmq_rmsnorm_backward, L.SIGNATURES["llmq_rmsnorm_backward"])
+    sms = K.num_sms(torch.device(DEV, 0))
+    blocks = sms if C > 1024 else 3 * sms                    # rows per block: see the kernel's launch
+    for status in (torch.zeros(1, dtype=torch.int32, device=DEV), None):
+        dinp, dw, am = dres.clone(), torch.zeros_like(w), torch.zeros(1, device=DEV)
+        assert lossy(dinp, dw, scratch, dy, x, w, rs, rows, C, 0, am, 0, 3 * sms, status) == 0
+        torch.cuda.synchronize()
+        lost = torch.zeros(rows, dtype=torch.bool, device=DEV)
+        lost[300 % blocks::blocks] = True
+        assert dinp[lost].isnan().all() and torch.equal(dinp[~lost], want[~lost]) and dw.isnan().all()
+        assert status is None or status.item() == 32
+        assert am.item() <= want.float().abs().max().item()
+    again = dres.clone()
+    K.rmsnorm_backward(again, torch.zeros_like(w), scratch, dy, x, w, rs)
+    assert torch.equal(again, want)
+    K.check_status(torch.device(DEV, 0))
