@@ -73,12 +73,13 @@ __device__ __forceinline__ float div_approx(float a, float b) {
     return r;
 }
 // The scale of a block whose largest value is `am` (at least 1e-30), am / 448, and its reciprocal: approximations and one correction each with the remainder in an
-// fma (Markstein's method), which gives the rounded quotients without the range checks of a general division.
+// fma (Markstein's method), which gives the rounded quotients without the range checks of a general division.  An infinity is its own scale, of reciprocal 0.
 __device__ __forceinline__ float e4m3_scale(float am, float& inv) {
     constexpr float kR = 1.f / 448.f;
     const float q = am * kR, sc = fmaf(fmaf(-448.f, q, am), kR, q);
     const float y = div_approx(1.f, sc);
     inv = fmaf(y, fmaf(-sc, y, 1.f), y);
+    if (isinf(am)) { inv = 0.f; return am; }                // the remainders are NaN
     return sc;
 }
 template <typename T> __device__ __forceinline__ void store8_srw(T* p, const float (&f)[8], const SrWords& w, uint32_t j0);

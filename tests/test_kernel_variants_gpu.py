@@ -1090,3 +1090,25 @@ def test_rmsnorm_backward_lost_copy(C, rows):
     K.rmsnorm_backward(again, torch.zeros_like(w), scratch, dy, x, w, rs)
     assert torch.equal(again, want)
     K.check_status(torch.device(DEV, 0))
+
+
+# e4m3 first moments of gradients that are not finite: the scale of a block with an infinity is infinite, its finite moments are 0 and the infinity and a NaN are NaN; a NaN alone leaves its
+# neighbours and their scale as they are; the largest finite gradients have a finite scale
+def test_adamw_e4m3_not_finite():
+    n, big = 128 * 6, torch.finfo(BF).max
+    grad = torch.randn(6, 128, device=DEV, generator=torch.Generator(device=DEV).manual_seed(7))
+    grad[0, 5], grad[1, 127], grad[2, 64], grad[3, 0] = math.inf, -math.inf, math.nan, big
+    grad[4, 1], grad[4, 2] = math.inf, math.nan
+    p, v = torch.zeros(n, device=DEV, dtype=BF), torch.ones(n, device=DEV, dtype=BF)
+    m, ms = torch.zeros(n, device=DEV, dtype=F8), torch.ones(6, device=DEV)
+    K.adamw(p, grad.to(BF).view(-1), m, v, lr=0.0, beta1=0.0, beta2=0.5, step=1, eps=1e-8, weight_decay=0.0, m_scales=ms, seed=11)
+    want, q = grad.to(BF).float(), m.float().view(6, 128)
+    top = want.abs().nan_to_num(0.0, math.inf).amax(-1)
+    assert torch.equal(ms, (top.double() / 448).float())
+    for b in (0, 1, 4):
+        assert torch.equal(q[b].isnan(), ~want[b].isfinite()) and (q[b][want[b].isfinite()] == 0).all()
+    for b in (2, 3, 5):
+        ok = ~want[b].isnan()
+        x = want[b].double() / ms[b].double()
+        assert torch.equal(q[b].isnan(), ~ok)
+        assert ((q[b].double() - x).abs()[ok] < (torch.exp2(torch.floor(torch.log2(x.abs().clamp_min(2.0**-6))) - 3) * (1 + 1e-5))[ok]).all()
