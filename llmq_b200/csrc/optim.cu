@@ -97,8 +97,8 @@ template <> __device__ __forceinline__ void store8_srw<float>(float* p, const fl
 // One thread updates 8 consecutive parameters.  Bound by memory and by instruction issue at once: the 12 random words, 24 roundings
 // and conversions of a thread took longer than its loads and stores.  Roundings in pairs (sr_bf16x2) bring 67.9 M parameters with
 // bf16 state (950 MB) from 193 to 166-182 us.  For e4m3 first moments 16 consecutive threads share one
-// fp32 scale (128 elements); the scale is recomputed from the new values every step.  They are converted and rounded in pairs too (sr_e4m3x2), and no
-// division checks its range: 67.9 M parameters with e4m3 and bf16 state 193.7 / 175.8 us, with bf16 state 156.4 / 154.5 (one box), same bits.
+// fp32 scale (128 elements); the scale is recomputed from the new values every step.  They are converted and rounded in pairs too (sr_e4m3x2), and the
+// division by the scale checks no range: 67.9 M parameters with e4m3 and bf16 state 193.2 / 179.9 us, same bits.
 template <typename P, typename G, typename M, typename Vv>
 __device__ __forceinline__ void adamw_vec(long long i, bool active, P* __restrict__ param, const G* __restrict__ grad, M* __restrict__ m_state,
                                           Vv* __restrict__ v_state, float* __restrict__ m_scales, float lr, float beta1, float beta2, float bc1,
@@ -125,9 +125,8 @@ __device__ __forceinline__ void adamw_vec(long long i, bool active, P* __restric
         m[k] = beta1 * m[k] + (1.f - beta1) * gk;
         v[k] = beta2 * v[k] + (1.f - beta2) * gk * gk;
         float mh = m[k] * bc1, vh = v[k] * bc2;
-        // fp32 first moments, which memory bounds, keep the form that the compiler schedules better: 67.9 M parameters 219 us, 222 with the other one
-        const float d = sqrt_approx(vh) + eps, u = sizeof(M) == 4 ? __fdividef(mh, d) : div_approx(mh, d);
-        p[k] -= lr * (u + wd * p[k]);
+        // not div.approx.ftz (1 to 2 % faster): it takes a subnormal moment for 0, and this quotient is 1 / eps times as large
+        p[k] -= lr * (__fdividef(mh, sqrt_approx(vh) + eps) + wd * p[k]);
     }
     const uint64_t ctr = static_cast<uint64_t>(e + elem_offset);
     const SrWords words(ctr, seed);

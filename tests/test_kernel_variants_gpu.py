@@ -1112,3 +1112,18 @@ def test_adamw_e4m3_not_finite():
         x = want[b].double() / ms[b].double()
         assert torch.equal(q[b].isnan(), ~ok)
         assert ((q[b].double() - x).abs()[ok] < (torch.exp2(torch.floor(torch.log2(x.abs().clamp_min(2.0**-6))) - 3) * (1 + 1e-5))[ok]).all()
+
+
+# gradients below the smallest normal number still move a parameter that is 0: they are divided by eps
+@pytest.mark.parametrize("params,moments", [(BF, BF), (BF, F8), (BF, torch.float32), (torch.float32, BF), (torch.float32, torch.float32)])
+@pytest.mark.parametrize("eps", [1e-8, 1e-39])
+def test_adamw_subnormal_gradients(params, moments, eps):
+    n = 256
+    grad = (2.0 ** -torch.arange(120, 133, device=DEV, dtype=torch.float64)).repeat(20)[:n].to(BF)
+    assert (grad > 0).all() and (grad.float() < torch.finfo(torch.float32).tiny).any()
+    p, v = torch.zeros(n, device=DEV, dtype=params), torch.zeros(n, device=DEV, dtype=torch.float32 if moments == torch.float32 else BF)
+    ms = torch.ones(n // 128, device=DEV) if moments == F8 else None
+    K.adamw(p, grad, torch.zeros(n, device=DEV).to(moments), v, lr=1.0, beta1=0.0, beta2=0.0, step=1, eps=eps, weight_decay=0.0, m_scales=ms, seed=3)
+    want = grad.double() / torch.tensor(eps, dtype=torch.float32).double().item()
+    # the fp32 quotient, a few units in the last place; bf16 parameters are rounded up or down
+    assert ((p.double() + want).abs() <= (2**-7 if params == BF else 1e-6) * want).all()
