@@ -539,12 +539,15 @@ static long long tiles_of(int M, int N, int bm, int bn) { return static_cast<lon
 // (one round of 148, 36.4 us); with equally many rounds 16384 x 4608 x 3584 351 / 388 us, 4096 x 896 x 9728 60.8 / 66.4, 4096 x 4864 x 896
 // 33.7 / 40.6.  With that many tiles the one-CTA kernel does not cut the K loop, so the sums have the same bits.
 // Where they leave half of the GPU idle, with 48 or more K steps of 128 bytes, the one-CTA kernel in two K parts wins, pairs / parts in us: 1062 x 2048 x 3072 bf16 22 / 20,
-// x 8192 46 / 33;  614 x 3584 x 12288 both MN-major 85 / 55;  1536 x 1536 x 8192 e4m3 26 / 23;  with 32 steps 17.4 / 17.5, with 16 12.7 / 14.8.
-static bool uses_pair_kernel(int M, int N, int K, int elem_bytes, bool fused, int num_sms) {
+// x 8192 46 / 33;  614 x 3584 x 12288 both MN-major 85 / 55;  1536 x 1536 x 8192 e4m3 26 / 23;  with 32 steps 17.4 / 17.5, with 16 12.7 / 14.8.  Where K may
+// not be cut (no workspace) it walks the whole of K on tiles of 128 columns, in 0.73 to 1.02 of the pairs' time over 30 shapes (two took 1.08): 880 x 2448 x 5088 21.0 / 27.4, 1112 x 2048 x 6784
+// B MN-major 35.7 / 37.6, 1000 x 2256 x 6368 A MN-major 41.4 / 42.6.  With both MN-major it takes 1.02 to 1.34 of it (14 shapes: 1512 x 1520 x 5904 49.5 / 44.5, 2208 x 1024 x 28224 e4m3
+// 107 / 80), and the pairs keep them (`few_tiles` false).
+static bool uses_pair_kernel(int M, int N, int K, int elem_bytes, bool fused, bool few_tiles, int num_sms) {
     if (elem_bytes == 4) return false;
     if (fused || g_gemm_mode == 2) return true;
     if (g_gemm_mode != 0 || M < 256 || static_cast<long long>(M) * N < 256LL * 256 * 32) return false;
-    if (2 * tiles_of(M, N, 128, 256) <= num_sms && K > 47 * (128 / elem_bytes)) return false;
+    if (few_tiles && 2 * tiles_of(M, N, 128, 256) <= num_sms && K > 47 * (128 / elem_bytes)) return false;
     const long long pair = waves(tiles_of(M, N, 256, 256), num_sms / 2);
     return pair < 2 || 5 * waves(tiles_of(M, N, 128, 256), num_sms) >= 4 * pair;
 }
@@ -560,6 +563,14 @@ static bool better_with_one_cta(int M, int N, int K, int elem_bytes, bool both_m
     const int bk = 128 / elem_bytes, k_iters = (K + bk - 1) / bk;
     const long long tiles = tiles_of(M, N, 128, 256);
     return k_iters <= 8 || (tiles <= num_sms && 2 * tiles > num_sms && k_iters <= (both_mn ? 16 : 64));
+}
+
+static bool takes_pair_kernel(int M, int N, int K, int elem_bytes, bool both_mn, bool fused, bool may_cut, int num_sms) {
+    return uses_pair_kernel(M, N, K, elem_bytes, fused, may_cut || !both_mn, num_sms) && (fused || !better_with_one_cta(M, N, K, elem_bytes, both_mn, num_sms));
+}
+// CTAs that work on a tile of a plain GEMM of this shape: 2 or 1 (for tests; nothing is launched)
+extern "C" int llmq_gemm_tile_ctas(int M, int N, int K, int elem_bytes, int both_mn_major, int may_cut, int num_sms) {
+    return takes_pair_kernel(M, N, K, elem_bytes, both_mn_major != 0, false, may_cut != 0, num_sms) ? 2 : 1;
 }
 
 // Tile rows of 256 that the pair kernel works through together.  B is read from memory once per group, so a group is as large as its rows of A
@@ -606,7 +617,7 @@ static int splitk_parts(int M, int N, int K, int elem_bytes, int num_sms) {
 
 // Floats of the workspace with which a plain GEMM of this shape (A and B of `elem_bytes` an element) cuts its K loop; 0: it does not.
 extern "C" long long llmq_gemm_splitk_floats(int M, int N, int K, int elem_bytes, int num_sms) {
-    if (M <= 0 || N <= 0 || K <= 0 || elem_bytes <= 0 || uses_pair_kernel(M, N, K, elem_bytes, false, num_sms)) return 0;
+    if (M <= 0 || N <= 0 || K <= 0 || elem_bytes <= 0 || uses_pair_kernel(M, N, K, elem_bytes, false, true, num_sms)) return 0;
     const int parts = splitk_parts(M, N, K, elem_bytes, num_sms);
     return parts > 1 ? static_cast<long long>(parts) * M * N : 0;
 }
@@ -704,7 +715,9 @@ static int gemm_impl(const void* A, const void* B, void* C, const void* bias,
     int rc;
     // The CTA-pair kernel stages 128 rows of B per CTA; the one-CTA kernel stages all 256.
     const bool fused = rs != nullptr || ready_flags != nullptr;
-    const bool pair_kernel = uses_pair_kernel(M, N, K, eb, fused, num_sms) && (fused || !better_with_one_cta(M, N, K, eb, a_mn_major && b_mn_major, num_sms));
+    const long long part_floats = static_cast<long long>(splitk_parts(M, N, K, eb, num_sms)) * M * N;
+    const bool may_cut = splitk_ws && part_floats <= splitk_floats;
+    const bool pair_kernel = takes_pair_kernel(M, N, K, eb, a_mn_major && b_mn_major, fused, may_cut, num_sms);
     // An MN-major stage that is several 128-byte chunks wide (16-bit operands; the 256 rows of B of the one-CTA kernel) is fetched with
     // one 3-D load instead of one 2-D load per chunk: the loads of a stage were issued one after the other for longer than its MMAs
     // run.  bf16, CTA pairs, TFLOP/s with 2-D loads / 3-D loads / 3-D loads and a K loop per kind of load (gemm_tcgen05_2cta.cu), K-major
@@ -720,8 +733,7 @@ static int gemm_impl(const void* A, const void* B, void* C, const void* bias,
     // 12.8 / 17.6;  with more 1024 x 1536 x 1536 (288) 19.2 / 19.2, 2048 x 896 x 4864 (224) 30.2 / 28.1, 256 x 7168 x 3584 (224) 25.3 /
     // 23.6;  both MN-major 512 x 1536 x 1536 14.3 / 18.5, 2048 x 896 x 4864 45.4 / 33.1, 512 x 3584 x 3584 (224) 36.2 / 28.7.
     const int tiles256 = ((M + BM - 1) / BM) * ((N + 255) / 256);
-    int splits = splitk_ws ? splitk_parts(M, N, K, eb, num_sms) : 1;
-    if (static_cast<long long>(splits) * M * N > splitk_floats) splits = 1;
+    const int splits = may_cut ? static_cast<int>(part_floats / (static_cast<long long>(M) * N)) : 1;
     const int tiles128 = ((M + BM - 1) / BM) * ((N + 127) / 128);
     const int bn = (eb != 4 && tiles128 * splits <= num_sms) ? 128 : 256;
     int pair_bn = 256;

@@ -86,6 +86,21 @@ def test_split_k_workspace_rule(elem_bytes):
     assert lib.llmq_gemm_splitk_floats(0, 8, 8, elem_bytes, sms) == 0
 
 
+# one or two CTAs per tile on both sides of each line of the rule: few output elements, short K, one round of tiles, half of the SMs idle with and without a workspace to cut K with
+@pytest.mark.skipif(not L.have_kernels(), reason="native library not built")
+@pytest.mark.parametrize("M,N,steps,both_mn,may_cut,ctas", [(255, 16384, 40, 0, 1, 1), (1024, 2047, 40, 0, 1, 1), (9728, 904, 8, 0, 1, 1), (9728, 904, 9, 0, 1, 2),
+                                                            (2320, 1160, 64, 0, 1, 1), (2320, 1160, 65, 0, 1, 2), (2040, 2064, 16, 1, 1, 1), (2040, 2064, 17, 1, 1, 2),
+                                                            (1064, 2040, 47, 0, 1, 2), (1064, 2040, 48, 0, 1, 1), (1064, 2040, 48, 0, 0, 1), (1064, 2040, 47, 1, 0, 2),
+                                                            (1064, 2040, 48, 1, 1, 1), (1064, 2040, 48, 1, 0, 2)])
+@pytest.mark.parametrize("elem_bytes", [1, 2])
+def test_gemm_tile_rule(M, N, steps, both_mn, may_cut, ctas, elem_bytes):
+    lib, K = L.kernels(), steps * (128 // elem_bytes)
+    assert lib.llmq_gemm_tile_ctas(M, N, K, elem_bytes, both_mn, may_cut, 148) == ctas
+    if may_cut and steps >= 47:
+        assert (lib.llmq_gemm_splitk_floats(M, N, K, elem_bytes, 148) > 0) == (ctas == 1 and steps == 48)
+    assert lib.llmq_gemm_tile_ctas(M, N, K * elem_bytes // 4, 4, both_mn, may_cut, 148) == 1      # fp32 operands
+
+
 @pytest.mark.skipif(not L.have_kernels(), reason="native library not built")
 @pytest.mark.parametrize("change,message", [
     (dict(m_scales=None), "need m_scales"), (dict(m_scales=torch.ones(1)), "m_scales holds 2"), (dict(m_scales=torch.ones(2).bfloat16()), "m_scales holds"),
