@@ -615,11 +615,41 @@ static int splitk_parts(int M, int N, int K, int elem_bytes, int num_sms) {
     return parts;
 }
 
+// The parts of a tile form a cluster, which adds them up in distributed shared memory, where all clusters reside at once (148 SMs hold 74 / 45 / 33 / 26 /
+// 22 / 15 / 15 of 2 .. 8 CTAs) and rows are whole 16-byte vectors of sums.  Otherwise the parts go through the workspace to a second kernel:
+// a second round of clusters costs more than that.  us in a graph, two kernels / clusters: 1001 x 896 x 1152 12.9 / 9.9, 1152 x 896 x 1001 added to C
+// 14.6 / 11.2, 896 x 896 x 1024 13.8 / 10.1, 339 x 3584 x 3584 added 22.4 / 16.4, 117 x 17920 x 1536 19.5 / 14.2, 576 x 1536 x 8960 30.4 / 24.4, 256 x 256 x 8192
+// 11.1 / 9.2, 1966 x 896 x 9728 42 / 35 (50 shapes whose clusters reside: 0.68 to 1.02, 0.85 on average);  with more tiles 1152 x 896 x 4096 (36 of 4 parts) 22.6 / 28.4,
+// 287 x 3072 x 8192 (36 of 4) 25.8 / 36.2, 256 x 2048 x 8192 e4m3 (16 of 8) 15.2 / 23.5.
+struct SplitPlan {
+    int parts, bn;                            // parts of K, columns of a tile
+    bool cluster;                             // the parts of a tile are added up by a cluster
+    int tiles;
+};
+static SplitPlan split_plan(const void* C, int M, int N, int K, int elem_bytes, long long ldc, int c_dtype, bool may_cut, int num_sms) {
+    SplitPlan s;
+    s.parts = may_cut ? splitk_parts(M, N, K, elem_bytes, num_sms) : 1;
+    const int tiles128 = static_cast<int>(tiles_of(M, N, BM, 128));
+    s.bn = elem_bytes != 4 && static_cast<long long>(tiles128) * s.parts <= num_sms ? 128 : 256;
+    s.tiles = s.bn == 128 ? tiles128 : static_cast<int>(tiles_of(M, N, BM, 256));
+    const int out_bytes = c_dtype == 0 ? 8 : 16;                           // four columns
+    const bool vec = N % 4 == 0 && ldc % 4 == 0 && reinterpret_cast<uintptr_t>(C) % out_bytes == 0;
+    s.cluster = s.parts > 1 && vec && s.tiles <= resident_clusters(s.parts);
+    return s;
+}
+
 // Floats of the workspace with which a plain GEMM of this shape (A and B of `elem_bytes` an element) cuts its K loop; 0: it does not.
 extern "C" long long llmq_gemm_splitk_floats(int M, int N, int K, int elem_bytes, int num_sms) {
     if (M <= 0 || N <= 0 || K <= 0 || elem_bytes <= 0 || uses_pair_kernel(M, N, K, elem_bytes, false, true, num_sms)) return 0;
     const int parts = splitk_parts(M, N, K, elem_bytes, num_sms);
     return parts > 1 ? static_cast<long long>(parts) * M * N : 0;
+}
+
+// How a plain GEMM with this output cuts its K loop if it may: 0 not at all, 1 in parts that clusters add up, 2 in parts that go through a workspace of
+// llmq_gemm_splitk_floats.  Launches nothing; the stream is not used.
+extern "C" int llmq_gemm_split_mode(const void* C, int M, int N, int K, int elem_bytes, long long ldc, int c_dtype, int num_sms, cudaStream_t) {
+    if (llmq_gemm_splitk_floats(M, N, K, elem_bytes, num_sms) == 0) return 0;
+    return split_plan(C, M, N, K, elem_bytes, ldc, c_dtype, true, num_sms).cluster ? 1 : 2;
 }
 
 extern "C" int llmq_gemm_ready(const void*, const void*, void*, const void*, int, int, int, int, int, int, int, long long, long long, long long, int, int, int,
@@ -645,7 +675,7 @@ extern "C" int llmq_gemm(const void* A, const void* B, void* C, const void* bias
 // Same, with the fused all-gather hook: rows of the stored B matrix are written by peer GPUs; ready_flags[src]
 // reaching ready_gen marks source src's rows complete.  The producer warps poll the flags tile by tile.
 // splitk_ws (optional): `splitk_floats` fp32 elements that no other work in flight uses; with fewer than llmq_gemm_splitk_floats
-// of them the K loop stays whole.
+// of them the K loop stays whole.  splitk_floats = -1: it is cut where that needs no workspace (llmq_gemm_split_mode 1).
 extern "C" int llmq_gemm_ready(const void* A, const void* B, void* C, const void* bias,
                                int M, int N, int K, int ab_dtype, int b_dtype, int a_mn_major, int b_mn_major,
                                long long lda, long long ldb, long long ldc, int c_dtype, int bias_dtype, int accumulate,
@@ -715,8 +745,8 @@ static int gemm_impl(const void* A, const void* B, void* C, const void* bias,
     int rc;
     // The CTA-pair kernel stages 128 rows of B per CTA; the one-CTA kernel stages all 256.
     const bool fused = rs != nullptr || ready_flags != nullptr;
-    const long long part_floats = static_cast<long long>(splitk_parts(M, N, K, eb, num_sms)) * M * N;
-    const bool may_cut = splitk_ws && part_floats <= splitk_floats;
+    const bool may_cut = splitk_floats < 0 ? split_plan(C, M, N, K, eb, ldc, c_dtype, true, num_sms).cluster
+                                           : splitk_ws && static_cast<long long>(splitk_parts(M, N, K, eb, num_sms)) * M * N <= splitk_floats;
     const bool pair_kernel = takes_pair_kernel(M, N, K, eb, a_mn_major && b_mn_major, fused, may_cut, num_sms);
     // An MN-major stage that is several 128-byte chunks wide (16-bit operands; the 256 rows of B of the one-CTA kernel) is fetched with
     // one 3-D load instead of one 2-D load per chunk: the loads of a stage were issued one after the other for longer than its MMAs
@@ -732,10 +762,8 @@ static int gemm_impl(const void* A, const void* B, void* C, const void* bias,
     // 256 x 896 x 896 8.4 / 11.9 us, 2304 x 896 x 896 9.6 / 12.5, 1001 x 896 x 1152 (112 items) 13.1 / 17.8, 512 x 1536 x 1536 (144 items)
     // 12.8 / 17.6;  with more 1024 x 1536 x 1536 (288) 19.2 / 19.2, 2048 x 896 x 4864 (224) 30.2 / 28.1, 256 x 7168 x 3584 (224) 25.3 /
     // 23.6;  both MN-major 512 x 1536 x 1536 14.3 / 18.5, 2048 x 896 x 4864 45.4 / 33.1, 512 x 3584 x 3584 (224) 36.2 / 28.7.
-    const int tiles256 = ((M + BM - 1) / BM) * ((N + 255) / 256);
-    const int splits = may_cut ? static_cast<int>(part_floats / (static_cast<long long>(M) * N)) : 1;
-    const int tiles128 = ((M + BM - 1) / BM) * ((N + 127) / 128);
-    const int bn = (eb != 4 && tiles128 * splits <= num_sms) ? 128 : 256;
+    const SplitPlan plan = split_plan(C, M, N, K, eb, ldc, c_dtype, may_cut, num_sms);
+    const int splits = plan.parts, bn = plan.bn;
     int pair_bn = 256;
     if (pair_kernel && rs == nullptr && ready_flags == nullptr && !b_mn_major) pair_bn = g_gemm_pair_bn ? g_gemm_pair_bn : pair_tile_columns(M, N, num_sms);
     const int b_rows = pair_kernel ? pair_bn / 2 : bn;
@@ -788,17 +816,9 @@ static int gemm_impl(const void* A, const void* B, void* C, const void* bias,
         return llmq_gemm_2cta_launch(ta, tb, tc, p, num_sms, stream);
     }
 
-    // The parts of a tile form a cluster, which adds them up in distributed shared memory, where all clusters reside at once (148 SMs hold 74 / 45 / 33 / 26 /
-    // 22 / 15 / 15 of 2 .. 8 CTAs) and rows are whole 16-byte vectors of sums.  Otherwise the parts go through the workspace to a second kernel:
-    // a second round of clusters costs more than that.  us in a graph, two kernels / clusters: 1001 x 896 x 1152 12.9 / 9.9, 1152 x 896 x 1001 added to C
-    // 14.6 / 11.2, 896 x 896 x 1024 13.8 / 10.1, 339 x 3584 x 3584 added 22.4 / 16.4, 117 x 17920 x 1536 19.5 / 14.2, 576 x 1536 x 8960 30.4 / 24.4, 256 x 256 x 8192
-    // 11.1 / 9.2, 1966 x 896 x 9728 42 / 35 (50 shapes whose clusters reside: 0.68 to 1.02, 0.85 on average);  with more tiles 1152 x 896 x 4096 (36 of 4 parts) 22.6 / 28.4,
-    // 287 x 3072 x 8192 (36 of 4) 25.8 / 36.2, 256 x 2048 x 8192 e4m3 (16 of 8) 15.2 / 23.5.
-    const int tiles = bn == 128 ? tiles128 : tiles256;
-    const int out_bytes = c_dtype == 0 ? 8 : 16;                           // four columns
-    const bool vec = N % 4 == 0 && ldc % 4 == 0 && reinterpret_cast<uintptr_t>(C) % out_bytes == 0;
+    const int tiles = plan.tiles;
+    const bool cluster = plan.cluster;
     if (splits > 1) { p.k_splits = splits; p.partial = splitk_ws; }
-    const bool cluster = splits > 1 && vec && tiles <= resident_clusters(splits);
     if (bn == 128) rc = eb == 1 ? launch_one_cta<1, 128>(ta, tb, p, tiles * splits, cluster, num_sms, stream) : launch_one_cta<0, 128>(ta, tb, p, tiles * splits, cluster, num_sms, stream);
     else if (eb == 1) rc = launch_one_cta<1, 256>(ta, tb, p, tiles * splits, cluster, num_sms, stream);
     else if (eb == 2) rc = launch_one_cta<0, 256>(ta, tb, p, tiles * splits, cluster, num_sms, stream);

@@ -112,6 +112,7 @@ struct Entry {
 // name, types of the arguments without the stream, which is the last one of every function
 #define LLMQ_ENTRIES(X)                                                                                                              \
     X(llmq_gemm_ready, P, P, P, P, int, int, int, int, int, int, int, LL, LL, LL, int, int, int, P, P, float, P, P, int, P, unsigned int, int, double, P, LL) \
+    X(llmq_gemm_split_mode, P, int, int, int, int, LL, int, int)                                                                    \
     X(llmq_rmsnorm_forward, P, P, P, P, P, P, P, float, int, int, int, P, P, P)                                                      \
     X(llmq_rmsnorm_backward, P, P, P, P, P, P, P, int, int, int, P, int, int, P)                                                     \
     X(llmq_swiglu_forward, P, P, P, LL, int, int, P, P, P, int)                                                                      \

@@ -50,16 +50,14 @@ _thread = threading.local()
 SPLITK_KEPT = 8
 
 
-def _splitk_workspace(M: int, N: int, K: int, elem_bytes: int, st, device, stream: int) -> Optional[torch.Tensor]:
-    """fp32 scratch of a GEMM that cuts its K loop (small outputs with a long K: weight gradients of small models), or None.
+def _splitk_workspace(M: int, N: int, K: int, elem_bytes: int, st, device, stream: int) -> torch.Tensor:
+    """fp32 scratch of a GEMM that cuts its K loop (small outputs with a long K: weight gradients of small models) into parts that a second kernel adds up.
 
     Nothing else in flight may use it, so each thread keeps one per device and stream: GEMMs of one thread on one stream follow one
     another.  A captured GEMM gets one of its own, in the memory pool of its graph, since graphs captured on one stream can be replayed
     on several.  At most SPLITK_KEPT of up to 64 MB stay with a thread; the others go back to the caching allocator, which hands them
     out again in the order of the stream that they were made for.  One per call from the allocator took 4 us more of host time."""
     floats = L.kernels().llmq_gemm_splitk_floats(M, N, K, elem_bytes, st["sms"])
-    if floats == 0 or not st["splitk"]:
-        return None
     if torch.cuda.is_current_stream_capturing():
         return torch.empty(floats, dtype=torch.float32, device=device)
     kept = _thread.__dict__.setdefault("splitk", {})
@@ -137,14 +135,15 @@ def gemm(out: torch.Tensor, a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = Fa
         assert a.stride(-1) == 1 and b.stride(-1) == 1 and out.stride(-1) == 1
         assert a.dtype == b.dtype or (_is_f8(a.dtype) and _is_f8(b.dtype)), (a.dtype, b.dtype)
         rflags, rgen, rrows, rlimit = ready if ready is not None else (0, 0, 0, 0.0)
-        stream = L.raw_stream()
-        ws = _splitk_workspace(M, N, K, a.element_size(), st, out.device, stream) if ready is None else None
-        rc = L.calls().llmq_gemm_ready(
+        calls, ldc, c_dtype = L.calls(), out.stride(0), 0 if out.dtype == torch.bfloat16 else 1
+        # 0: K stays whole, 1: it is cut and clusters add the parts up, 2: the parts need a workspace
+        split = calls.llmq_gemm_split_mode(out, M, N, K, a.element_size(), ldc, c_dtype, st["sms"]) if ready is None and st["splitk"] else 0
+        ws = _splitk_workspace(M, N, K, a.element_size(), st, out.device, L.raw_stream()) if split == 2 else None
+        rc = calls.llmq_gemm_ready(
             a, b, out, bias, M, N, K, L.dtype_code(a.dtype), L.dtype_code(b.dtype),
-            int(a_mn), int(b_mn), a.stride(0), b.stride(0), out.stride(0),
-            0 if out.dtype == torch.bfloat16 else 1, 0 if (bias is None or bias.dtype == torch.bfloat16) else 1,
+            int(a_mn), int(b_mn), a.stride(0), b.stride(0), ldc, c_dtype, 0 if (bias is None or bias.dtype == torch.bfloat16) else 1,
             int(accumulate), scale_a, scale_b, alpha, absmax, st["status"], st["sms"],
-            rflags, rgen, int(rrows), rlimit, ws, 0 if ws is None else ws.numel())
+            rflags, rgen, int(rrows), rlimit, ws, -(split == 1) if ws is None else ws.numel())
         L.check(rc, "gemm")
         return
     af = a.float().t() if a_mn else a.float()

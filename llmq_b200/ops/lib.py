@@ -67,7 +67,7 @@ def kernels():
 
 # Arguments of the entry points in calls(), without the stream: p pointer (tensor, address or None), i int, u unsigned, l long long, f float, d double
 SIGNATURES = {
-    "llmq_gemm_ready": "ppppiiiiiiillliiippfppipuidpl", "llmq_rmsnorm_forward": "pppppppfiiippp", "llmq_rmsnorm_backward": "pppppppiiipiip",
+    "llmq_gemm_ready": "ppppiiiiiiillliiippfppipuidpl", "llmq_gemm_split_mode": "piiiilii", "llmq_rmsnorm_forward": "pppppppfiiippp", "llmq_rmsnorm_backward": "pppppppiiipiip",
     "llmq_swiglu_forward": "pppliipppi", "llmq_swiglu_backward": "pppliipi", "llmq_rope": "pppiiiiiiipi",
     "llmq_attention_forward": "pppiiiiipp", "llmq_attention_backward": "ppppppiiiiip", "llmq_bias_backward": "pppliippiii", "llmq_abs_max": "pplii",
     "llmq_quantize": "ppppliii", "llmq_quantize_transpose": "pppppiiii", "llmq_transpose": "ppppiiii", "llmq_fused_classifier": "ppppffiilii",

@@ -457,11 +457,12 @@ def test_gemm_added_to(M, N, Kd, dt, mode):
     assert abs(am.item() - want.abs().max().item()) < 1e-4 * want.abs().max().item()
 
 
-def _split_k_operands(n, seed):
-    """n GEMMs of one shape (8 parts, 2 MB of partial sums each) and what each gives by itself."""
+def _split_k_operands(n, seed, N):
+    """n GEMMs of one shape (8 parts; 2 MB of partial sums each where N is no multiple of 4, clusters add them up where it is) and what each gives by itself."""
     g = torch.Generator(device=DEV).manual_seed(seed)
-    a, b = torch.randn(n, 200, 8192, device=DEV, generator=g).to(BF), torch.randn(n, 304, 8192, device=DEV, generator=g).to(BF)
-    want = torch.empty(n, 200, 304, device=DEV)
+    a, b = torch.randn(n, 200, 8192, device=DEV, generator=g).to(BF), torch.randn(n, N, 8192, device=DEV, generator=g).to(BF)
+    want = torch.empty(n, 200, N, device=DEV)
+    assert L.calls().llmq_gemm_split_mode(want[0], 200, N, 8192, 2, N, 1, 148) == (2 if N % 4 else 1)
     for i in range(n):
         K.gemm(want[i], a[i], b[i])
         torch.cuda.synchronize()
@@ -470,11 +471,12 @@ def _split_k_operands(n, seed):
 
 
 @pytest.mark.parametrize("how", ["streams", "threads", "graphs"])
-def test_split_k_on_several_streams(how):
+@pytest.mark.parametrize("N", [301, 304])
+def test_split_k_on_several_streams(how, N):
     """GEMMs that cut K, side by side on four streams (of one thread, of four threads, of four captured graphs): the partial sums of
     one are never those of another."""
     n, lanes = 16, 4
-    a, b, want = _split_k_operands(n, 3)
+    a, b, want = _split_k_operands(n, 3, N)
     out, streams = torch.zeros_like(want), [torch.cuda.Stream() for _ in range(lanes)]
     torch.cuda.synchronize()
 
@@ -508,7 +510,7 @@ def test_split_k_on_several_streams(how):
 
 
 def test_split_k_workspaces_kept_by_a_thread_are_bounded():
-    a, b, want = _split_k_operands(2, 4)
+    a, b, want = _split_k_operands(2, 4, 301)
     out = torch.zeros_like(want)
     with ThreadPoolExecutor(1) as pool:
         def many():
@@ -521,7 +523,28 @@ def test_split_k_workspaces_kept_by_a_thread_are_bounded():
                 assert torch.equal(out[0], want[0]) and torch.equal(out[1, :100], want[1, :100])
             return {k: v.numel() for k, v in K._thread.splitk.items()}
         kept = pool.submit(many).result()
-    assert 1 <= len(kept) <= K.SPLITK_KEPT and set(kept.values()) == {8 * 200 * 304}
+    assert 1 <= len(kept) <= K.SPLITK_KEPT and set(kept.values()) == {8 * 200 * 301}
+
+
+def test_split_k_added_up_by_clusters_takes_no_workspace():
+    a, b, want = _split_k_operands(1, 5, 304)
+    out, graph = torch.zeros_like(want), torch.cuda.CUDAGraph()
+    with ThreadPoolExecutor(1) as pool:
+        def one():
+            torch.zeros(1, device=DEV)
+            K.gemm(out[0], a[0], b[0])
+            torch.cuda.synchronize()
+            return dict(K._thread.__dict__.get("splitk", {}))
+        assert pool.submit(one).result() == {} and torch.equal(out, want)
+    with torch.cuda.graph(graph):
+        K.gemm(out[0], a[0], b[0])
+        used = torch.cuda.memory_allocated()
+        K.gemm(out[0], a[0], b[0])
+        assert torch.cuda.memory_allocated() == used
+    out.zero_()
+    graph.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(out, want)
 
 
 @pytest.mark.parametrize("op", ["gemm_fp32", "attention_fp32", "encoder_backward"])
