@@ -892,14 +892,6 @@ constexpr int bwd_smem() {
     return one_block_per_sm(DkdvShape<HS>::SMEM_BYTES > DqShape<HS>::SMEM_BYTES ? DkdvShape<HS>::SMEM_BYTES : DqShape<HS>::SMEM_BYTES);
 }
 
-int device_sms() {
-    static int sms[64] = {};
-    int dev = 0;
-    cudaGetDevice(&dev);
-    if (!sms[dev & 63]) cudaDeviceGetAttribute(&sms[dev & 63], cudaDevAttrMultiProcessorCount, dev);
-    return sms[dev & 63] > 0 ? sms[dev & 63] : 148;
-}
-
 // Query heads of a group that a dQ CTA walks over; `base` = (query block, kv head, batch) items.  A CTA that walks a whole group pays its
 // start-up once, but few items leave SMs idle: the group is cut into the fewest parts that give 1.5 CTAs per SM.  Heads do not share
 // sums, so the results do not depend on the cut.

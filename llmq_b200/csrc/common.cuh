@@ -64,6 +64,15 @@ void launch_chained(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cu
 }
 
 __host__ __device__ constexpr long long ceil_div_ll(long long a, long long b) { return (a + b - 1) / b; }
+// SMs of the current device
+inline int device_sms() {
+    static int sms[64] = {};
+    int dev = 0;
+    cudaGetDevice(&dev);
+    int& n = sms[dev & 63];
+    if (n <= 0 && (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0)) n = 148;
+    return n;
+}
 __host__ __device__ constexpr int ceil_div_i(int a, int b) { return (a + b - 1) / b; }
 
 // ------------------------------------------------------------------------------------------------

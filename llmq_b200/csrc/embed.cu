@@ -192,7 +192,7 @@ template <typename T, typename D>
 __global__ void __launch_bounds__(256)
 bias_bwd_cluster_kernel(D* __restrict__ dbias, const T* __restrict__ dout, long long rows, int C, const float* __restrict__ scale_a, const float* __restrict__ scale_b, int accumulate) {
     grid_wait(dbias, dout, scale_a, scale_b);
-    __shared__ float tile[8][8][128];                          // [slice][row lane][column], then [64 slices][16 columns]
+    __shared__ __align__(16) float tile[8][8][128];                          // [slice][row lane][column], then [64 slices][16 columns]
     __shared__ __align__(16) float part[kBiasOwn][128];
     const int cta = blockIdx.x % kBiasCtas, col0 = blockIdx.x / kBiasCtas * 128;
     const int cx = threadIdx.x & 31, ry = threadIdx.x >> 5;
@@ -312,7 +312,7 @@ extern "C" int llmq_bias_backward(void* dbias, float* partial, const void* dout,
     if (dbias_dtype != 0 && dbias_dtype != 3) return -10;
     const bool vec4 = C % 4 == 0 && reinterpret_cast<uintptr_t>(dout) % 16 == 0;
     const int blocks = ceil_div_i(C, 128) * kBiasCtas;
-    if (vec4 && slices == kBiasSlices && rows <= (dout_dtype == 1 || dout_dtype == 2 ? 1024 : 2048) && blocks <= 148) {
+    if (vec4 && slices == kBiasSlices && rows <= (dout_dtype == 1 || dout_dtype == 2 ? 1024 : 2048) && blocks <= device_sms()) {
 #define BIAS_CLUSTER(T)                                                                                                \
     do {                                                                                                               \
         if (dbias_dtype == 0) launch_chained_cluster(bias_bwd_cluster_kernel<T, bf16>, blocks, 256, 0, s, kBiasCtas, static_cast<bf16*>(dbias), static_cast<const T*>(dout), rows, C, scale_a, scale_b, accumulate);   \

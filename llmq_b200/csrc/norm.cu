@@ -543,15 +543,6 @@ int launch_fwd(void* residual_out, void* y_out, void* q_out, float* rstd, const 
     return LLMQ_LAUNCH_CHECK();
 }
 
-int device_sms() {
-    static int sms[64] = {};
-    int dev = 0;
-    cudaGetDevice(&dev);
-    int& n = sms[dev & 63];
-    if (n <= 0 && (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0)) n = 148;
-    return n;
-}
-
 template <typename T, int VPT, int STAGES, int CTAS>
 int launch_bwd_ring(T* dinp, float* scratch, const T* dout, const T* inp, const T* w, const float* rstd, int rows, int C, float* absmax, int blocks, unsigned int* status, cudaStream_t s) {
     static bool attr_set[64] = {};          // per device
