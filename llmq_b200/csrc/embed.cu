@@ -254,8 +254,15 @@ __global__ void bias_bwd_final_kernel(T* __restrict__ dbias, const float* __rest
     int c = bx * blockDim.x + tx;
     if (c >= C) return;
     float s = 0.f;
-#pragma unroll 16                                              // loads under way, added up in order
-    for (int k = 0; k < slices; ++k) s += partial[static_cast<long long>(k) * C + c];
+    // 16 loads under way, added up in order; the last ones too, which are 15 loads one after the other in an unrolled loop's remainder: 500 x 4608 bf16, 63
+    // slices, 10.3 / 7.3 us
+    for (int k0 = 0; k0 < slices; k0 += 16) {
+        float v[16];
+#pragma unroll
+        for (int j = 0; j < 16; ++j) v[j] = partial[static_cast<long long>(min(k0 + j, slices - 1)) * C + c];
+#pragma unroll
+        for (int j = 0; j < 16; ++j) s = k0 + j < slices ? s + v[j] : s;
+    }
     if (scale_a) s *= *scale_a;
     if (scale_b) s *= *scale_b;
     if (accumulate) s += to_float(dbias[c]);
