@@ -186,7 +186,7 @@ bias_bwd_partial_vec4_kernel(float* __restrict__ partial, const T* __restrict__ 
 // sums of the 64 slices of a column meet in distributed shared memory; each CTA ends 16 columns.  For small gradients, where the second launch and its
 // latency are what counts: 1001 x 1152 bf16 5.5 / 3.8 us, 256 x 1152 5.2 / 3.3;  4096 x 1152 6.4 / 6.7, and with more than one round of clusters or more
 // rows per CTA the two kernels have four times the warps: 16384 x 4608 29 / 82, 300 x 37888 21 / 38.  8-bit elements, whose conversions count, 1024 x 896
-// 5.2 / 4.9, 1536 x 896 5.2 / 6.0.
+// 5.2 / 4.9, 1536 x 896 5.2 / 6.0 (see llmq_bias_backward for the lines).
 constexpr int kBiasSlices = 64, kBiasCtas = 8, kBiasOwn = kBiasSlices / kBiasCtas;
 template <typename T, typename D>
 __global__ void __launch_bounds__(256)
@@ -256,12 +256,15 @@ __global__ void bias_bwd_final_kernel(T* __restrict__ dbias, const float* __rest
     float s = 0.f;
     // 16 loads under way, added up in order; the last ones too, which are 15 loads one after the other in an unrolled loop's remainder: 500 x 4608 bf16, 63
     // slices, 10.3 / 7.3 us
-    for (int k0 = 0; k0 < slices; k0 += 16) {
-        float v[16];
+    int k = 0;
+#pragma unroll 16
+    for (; k < slices / 16 * 16; ++k) s += partial[static_cast<long long>(k) * C + c];
+    if (k < slices) {
+        float v[15];
 #pragma unroll
-        for (int j = 0; j < 16; ++j) v[j] = partial[static_cast<long long>(min(k0 + j, slices - 1)) * C + c];
+        for (int j = 0; j < 15; ++j) v[j] = partial[static_cast<long long>(min(k + j, slices - 1)) * C + c];
 #pragma unroll
-        for (int j = 0; j < 16; ++j) s = k0 + j < slices ? s + v[j] : s;
+        for (int j = 0; j < 15; ++j) s = k + j < slices ? s + v[j] : s;
     }
     if (scale_a) s *= *scale_a;
     if (scale_b) s *= *scale_b;
@@ -319,7 +322,12 @@ extern "C" int llmq_bias_backward(void* dbias, float* partial, const void* dout,
     if (dbias_dtype != 0 && dbias_dtype != 3) return -10;
     const bool vec4 = C % 4 == 0 && reinterpret_cast<uintptr_t>(dout) % 16 == 0;
     const int blocks = ceil_div_i(C, 128) * kBiasCtas;
-    if (vec4 && slices == kBiasSlices && rows <= (dout_dtype == 1 || dout_dtype == 2 ? 1024 : 2048) && blocks <= device_sms()) {
+    // Rows up to which one launch is not slower.  Few columns are few clusters, whose CTAs then have the longer way through the rows: us, one / two launches, bf16 2048 rows of 64
+    // columns 4.7 / 4.1, 128 4.6 / 4.1, 256 4.7 / 4.3, 512 4.7 / 4.5, 896 4.8 / 5.2, 1700 of 128 4.6 / 4.2, 256 4.5 / 4.5, 384 4.5 / 5.0;  8-bit 1024 rows of 64 4.8 / 4.2, 256 4.7 / 4.5,
+    // 512 4.8 / 4.5, 896 5.0 / 5.4, 500 of 128 3.8 / 4.3.
+    const bool byte = dout_dtype == 1 || dout_dtype == 2;
+    const int most = byte ? (C <= 640 ? 512 : 1024) : C < 256 ? 1536 : C <= 640 ? 1792 : 2048;
+    if (vec4 && slices == kBiasSlices && rows <= most && blocks <= device_sms()) {
 #define BIAS_CLUSTER(T)                                                                                                \
     do {                                                                                                               \
         if (dbias_dtype == 0) launch_chained_cluster(bias_bwd_cluster_kernel<T, bf16>, blocks, 256, 0, s, kBiasCtas, static_cast<bf16*>(dbias), static_cast<const T*>(dout), rows, C, scale_a, scale_b, accumulate);   \

@@ -969,6 +969,17 @@ def test_bias_backward_one_launch(rows, C, dt, out_dt):
         assert ((got[0].double() - want).abs() <= want.abs() * (2**-8 if out_dt == BF else 1e-6) + 1e-5 * rows**0.5 * (448 if dt.itemsize == 1 else 1)).all()
 
 
+# on both sides of the rows up to which one launch is taken, and numbers of partial sums (one per 8 rows) that are no multiples of 16, in the two-launch form
+@pytest.mark.parametrize("rows,C", [(1536, 128), (1537, 128), (1792, 256), (1793, 256), (2048, 1152), (2049, 1152), (8, 2432), (100, 2432), (129, 2432), (500, 2432)])
+@pytest.mark.parametrize("dt", [BF, F8])
+def test_bias_backward_lines(rows, C, dt):
+    g = torch.Generator(device=DEV).manual_seed(rows + C)
+    dout, db = torch.randn(rows, C, device=DEV, generator=g).to(dt), torch.full((C,), 9.0, device=DEV)
+    K.bias_backward(db, dout, torch.full((64 * C,), math.nan, device=DEV))
+    # fp32 sums of numbers of a few units
+    assert ((db.double() - dout.double().sum(0)).abs() <= 1e-5 * rows**0.5).all()
+
+
 # the sum of the partial squares and the clipping factor in one launch: fewer and more partials than threads, no clipping, a norm that is not finite
 @pytest.mark.parametrize("n", [1, 31, 512, 513, 2000])
 @pytest.mark.parametrize("clip,bad", [(0.0, None), (1.0, None), (1e6, None), (1.0, math.inf), (1.0, math.nan)])
