@@ -253,23 +253,53 @@ rmsnorm_bwd_kernel(T* __restrict__ dinp,               // in: upstream residual 
     block_absmax_commit(absmax_out, tmax, scratch);
 }
 
+// 16 bytes from global to shared memory, asynchronously; a thread waits for its own copies in groups, in order
+__device__ __forceinline__ void copy_async16(void* dst, const void* src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(static_cast<uint32_t>(__cvta_generic_to_shared(dst))), "l"(src) : "memory");
+}
+__device__ __forceinline__ void copy_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void copy_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
+
 // `bytes` (a multiple of 16, both addresses aligned to 16) from global to shared memory by the copy engine; counted by the barrier
 __device__ __forceinline__ void copy_row_async(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
     asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
                  ::"r"(dst), "l"(src), "r"(bytes), "r"(bar) : "memory");
 }
 
-// Same contract, for fp32 rows of two to four column vectors per thread, and for blocks with one or two rows of one: the row's dout, inp and residual gradient are loaded once and stay in
-// registers across the block-wide dot product.  4000 x 4096 51.6 us, 53.2 with the rows in shared memory (below), 1000 x 2048 12.2 / 13.2.
-template <typename T, int VPT>
+// Same contract, for fp32 rows of two to four column vectors per thread, for short rows and for blocks with one or two (launch_bwd has the lines): the row's dout,
+// inp and residual gradient are loaded once and stay in registers across the block-wide dot product.  fp32 4000 x 4096 51.6 us, 53.2 with the rows in shared memory (below), 1000 x 2048 12.2 / 13.2.
+// STAGES > 0: that many rows to come are on their way into shared memory; every thread copies and reads back its own vectors, so that no row waits for a barrier
+// or for the thread that issues.
+template <typename T, int VPT, int STAGES>
 __global__ void __launch_bounds__(NORM_THREADS, VPT <= 2 ? 3 : 2)
 rmsnorm_bwd_reg_kernel(T* __restrict__ dinp, float* __restrict__ dw_partial, const T* __restrict__ dout, const T* __restrict__ inp,
                        const T* __restrict__ weight, const float* __restrict__ rstd, int rows, int C, float* __restrict__ absmax_out) {
     __shared__ float scratch[32];
     __shared__ float dots[2][NORM_THREADS / 32];             // alternating, so that one barrier per row is enough
+    extern __shared__ __align__(16) uint8_t ring[];          // [STAGES][dout, inp, dinp][C]
     using V = Vec16<T>;
     float dw[VPT][V::N];
     V vw[VPT];
+    auto slot = [&](int stage, int what, int c) { return reinterpret_cast<T*>(ring) + (stage * 3 + what) * C + c; };
+    auto fetch = [&](long long row, int stage) {
+        if (row < rows) {
+#pragma unroll
+            for (int k = 0; k < VPT; ++k) {
+                const int c = (k * NORM_THREADS + threadIdx.x) * V::N;
+                if (c < C) {
+                    copy_async16(slot(stage, 0, c), dout + row * C + c);
+                    copy_async16(slot(stage, 1, c), inp + row * C + c);
+                    copy_async16(slot(stage, 2, c), dinp + row * C + c);
+                }
+            }
+        }
+        copy_async_commit();                                 // a group per row, empty beyond the last one
+    };
+    if constexpr (STAGES > 0) {
+#pragma unroll
+        for (int st = 0; st < STAGES; ++st) fetch(blockIdx.x + static_cast<long long>(st) * gridDim.x, st);
+    }
 #pragma unroll
     for (int k = 0; k < VPT; ++k) {
         const int c = (k * NORM_THREADS + threadIdx.x) * V::N;
@@ -279,16 +309,21 @@ rmsnorm_bwd_reg_kernel(T* __restrict__ dinp, float* __restrict__ dw_partial, con
     }
     float tmax = 0.f;
     const float inv_c = 1.f / C;
-    int par = 0;
+    int par = 0, stage = 0;
     for (long long row = blockIdx.x; row < rows; row += gridDim.x, par ^= 1) {
         const T* dy = dout + row * C;
         const T* x = inp + row * C;
         T* dx = dinp + row * C;
-        V vdy[VPT], vx[VPT], vd[VPT];
+        V vdy[VPT], vx[VPT], vd[STAGES > 0 ? 1 : VPT];
+        if constexpr (STAGES > 0) copy_async_wait<STAGES - 1>();
 #pragma unroll
         for (int k = 0; k < VPT; ++k) {
             const int c = (k * NORM_THREADS + threadIdx.x) * V::N;
-            if (c < C) { vdy[k] = V::load_stream(dy + c); vx[k] = V::load_stream(x + c); vd[k] = V::load_stream(dx + c); }
+            if constexpr (STAGES > 0) {
+                if (c < C) { vdy[k] = V::load(slot(stage, 0, c)); vx[k] = V::load(slot(stage, 1, c)); }
+            } else {
+                if (c < C) { vdy[k] = V::load_stream(dy + c); vx[k] = V::load_stream(x + c); vd[k] = V::load_stream(dx + c); }
+            }
         }
         const float rs = rstd[row];
         float dot = 0.f;
@@ -313,7 +348,8 @@ rmsnorm_bwd_reg_kernel(T* __restrict__ dinp, float* __restrict__ dw_partial, con
         for (int k = 0; k < VPT; ++k) {
             const int c = (k * NORM_THREADS + threadIdx.x) * V::N;
             if (c < C) {
-                V& d = vd[k];
+                V& d = vd[STAGES > 0 ? 0 : k];
+                if constexpr (STAGES > 0) d = V::load(slot(stage, 2, c));
 #pragma unroll
                 for (int i = 0; i < V::N; ++i) {
                     const float xh = to_float(vx[k].v[i]) * rs;
@@ -323,6 +359,10 @@ rmsnorm_bwd_reg_kernel(T* __restrict__ dinp, float* __restrict__ dw_partial, con
                 }
                 d.store(dx + c);
             }
+        }
+        if constexpr (STAGES > 0) {
+            fetch(row + static_cast<long long>(STAGES) * gridDim.x, stage);
+            if (++stage == STAGES) stage = 0;
         }
     }
 #pragma unroll
@@ -578,10 +618,22 @@ int launch_bwd(void* dinp_, void* dweight, float* scratch, const void* dout_, co
     const T *dout = static_cast<const T*>(dout_), *inp = static_cast<const T*>(inp_), *w = static_cast<const T*>(w_);
     int rc;
     // stages and CTAs per SM: as much shared memory as fits
-    // Blocks with one or two short rows have nothing to fetch ahead, and setting up the ring costs 0.3 us: us with / without it, bf16: 20 x 896 4.2 / 3.9, 113 x 1536 5.7 / 5.2,
-    // 888 x 256 7.3 / 7.0, 888 x 1024 9.1 / 9.1;  fp32 888 x 896 8.3 / 7.8.  More rows: 4096 x 896 bf16 13.8 / 16.3 (from HBM 15.2 / 18.4), fp32 13.2 / 15.7.
-    if (vecs <= 1 && rows <= 2 * num_blocks) {
-        rmsnorm_bwd_reg_kernel<T, 1><<<num_blocks, NORM_THREADS, 0, s>>>(dinp, scratch, dout, inp, w, rstd, rows, C, absmax);
+    // Rows of one vector a thread.  Blocks with one or two of them have nothing to fetch ahead, and setting up the ring costs 0.3 us: us with / without it, bf16: 20 x 896 4.2 / 3.9,
+    // 113 x 1536 5.7 / 5.2, 888 x 256 7.3 / 7.0.  Short rows spend a turn of the ring on its barriers and its one issuing thread, which shows where the operands lie in the L2 already.  bf16
+    // rows of up to 768 channels are copied by their threads, which is as fast from HBM until the operands are larger than the L2; us, rows by bulk copies / by their threads, from L2
+    // and from HBM: 4096 x 256 12.1 / 10.9, 16384 x 256 28.6 / 24.5 and 29.4 / 29.9, 8192 x 512 19.0 / 16.9 and 19.8 / 20.2, 8192 x 768 20.8 / 19.1 and 21.8 / 21.8;  65536 x 256 (101 MB)
+    // 99.2 / 99.9 and 99.2 / 101.8;  8192 x 896 20.8 / 19.6 and 22.2 / 23.0, 4096 x 896 14.0 / 13.6 and 15.3 / 16.1.  fp32 rows, from L2 and from HBM, by bulk copies / in
+    // registers: 2000 x 1024 10.8 / 9.9 and 13.5 / 13.8, 3000 x 768 (28 MB) 11.5 / 10.5 and 14.2 / 15.4, 4096 x 256 11.3 / 10.4 and 12.0 / 14.5;  beyond 32 MB, where they
+    // rarely lie in the L2 as a whole, 8192 x 512 (50 MB) 16.9 / 15.1 and 18.8 / 24.6, 8192 x 768 (75 MB) 18.3 / 20.5 and 23.6 / 27.6.
+    const long long bytes = 3ll * rows * C * static_cast<long long>(sizeof(T));
+    const bool in_registers = rows <= 2 * num_blocks || (sizeof(T) == 4 && bytes <= (32ll << 20)), by_threads = sizeof(T) == 2 && C <= 768 && bytes <= (96ll << 20);
+    if (vecs <= 1 && in_registers) {
+        rmsnorm_bwd_reg_kernel<T, 1, 0><<<num_blocks, NORM_THREADS, 0, s>>>(dinp, scratch, dout, inp, w, rstd, rows, C, absmax);
+        rc = LLMQ_LAUNCH_CHECK();
+    }
+    else if (vecs <= 1 && by_threads) {
+        constexpr int stages = 4;                            // 18 KB at most
+        rmsnorm_bwd_reg_kernel<T, 1, stages><<<num_blocks, NORM_THREADS, stages * 3 * C * sizeof(T), s>>>(dinp, scratch, dout, inp, w, rstd, rows, C, absmax);
         rc = LLMQ_LAUNCH_CHECK();
     }
     else if (vecs <= 1) rc = launch_bwd_ring<T, 1, 4, 3>(dinp, scratch, dout, inp, w, rstd, rows, C, absmax, num_blocks, status, s);
@@ -590,8 +642,8 @@ int launch_bwd(void* dinp_, void* dweight, float* scratch, const void* dout_, co
             if (vecs <= 2) rc = launch_bwd_ring<T, 2, 3, 3>(dinp, scratch, dout, inp, w, rstd, rows, C, absmax, num_blocks, status, s);
             else           rc = launch_bwd_ring<T, 4, 2, 2>(dinp, scratch, dout, inp, w, rstd, rows, C, absmax, num_blocks, status, s);
         } else {
-            if (vecs <= 2) rmsnorm_bwd_reg_kernel<T, 2><<<num_blocks, NORM_THREADS, 0, s>>>(dinp, scratch, dout, inp, w, rstd, rows, C, absmax);
-            else           rmsnorm_bwd_reg_kernel<T, 4><<<num_blocks, NORM_THREADS, 0, s>>>(dinp, scratch, dout, inp, w, rstd, rows, C, absmax);
+            if (vecs <= 2) rmsnorm_bwd_reg_kernel<T, 2, 0><<<num_blocks, NORM_THREADS, 0, s>>>(dinp, scratch, dout, inp, w, rstd, rows, C, absmax);
+            else           rmsnorm_bwd_reg_kernel<T, 4, 0><<<num_blocks, NORM_THREADS, 0, s>>>(dinp, scratch, dout, inp, w, rstd, rows, C, absmax);
             rc = LLMQ_LAUNCH_CHECK();
         }
     }

@@ -1097,6 +1097,13 @@ def test_calls_through_ctypes(monkeypatch):
     assert all(torch.equal(x, y) for x, y in zip(*got)) and got[0][2].item() > 0
 
 
+# on both sides of the lines between the kernels of short rows: bf16 768 channels (more than two rows a block), fp32 32 MB, 96 MB; the ring of per-thread copies turns
+@pytest.mark.parametrize("C,rows,dt", [(8, 5001, BF), (264, 4099, BF), (768, 1333, BF), (776, 1333, BF), (512, 32768, BF), (512, 32769, BF), (1024, 2730, torch.float32),
+                                       (1024, 2731, torch.float32), (200, 1001, torch.float32)])
+def test_rmsnorm_backward_short_rows(C, rows, dt):
+    test_rmsnorm_backward_few_rows(C, rows, dt)
+
+
 # a row whose copies never come (a build of the kernel that does not issue those of row 300, with a limit of 20 ms): the block that waits for it ends, the status word and NaNs in the weight
 # gradient and in all rows of that block say so, and no other row differs
 @pytest.mark.parametrize("C,rows", [(896, 2000), (3584, 1001), (5120, 700)])
