@@ -86,19 +86,26 @@ def test_split_k_workspace_rule(elem_bytes):
     assert lib.llmq_gemm_splitk_floats(0, 8, 8, elem_bytes, sms) == 0
 
 
-# one or two CTAs per tile on both sides of each line of the rule: few output elements, short K, one round of tiles, half of the SMs idle with and without a workspace to cut K with
+# one or two CTAs per tile on both sides of each line of the rule: few output elements, short K, one round of tiles (both by the bytes that rows start at multiples of), half of the SMs idle with
+# and without a workspace to cut K with
 @pytest.mark.skipif(not L.have_kernels(), reason="native library not built")
-@pytest.mark.parametrize("M,N,steps,both_mn,may_cut,ctas", [(255, 16384, 40, 0, 1, 1), (1024, 2047, 40, 0, 1, 1), (9728, 904, 8, 0, 1, 1), (9728, 904, 9, 0, 1, 2),
-                                                            (2320, 1160, 64, 0, 1, 1), (2320, 1160, 65, 0, 1, 2), (2040, 2064, 16, 1, 1, 1), (2040, 2064, 17, 1, 1, 2),
+@pytest.mark.parametrize("M,N,steps,both_mn,may_cut,ctas", [(255, 16384, 40, 0, 1, 1), (1024, 2047, 40, 0, 1, 1), (9728, 904, 6, 0, 1, 1), (9728, 904, 7, 0, 1, 1), (9728, 904, 8, 0, 1, 1), (9728, 904, 9, 0, 1, 2),
+                                                            (2320, 1160, 12, 0, 1, 1), (2320, 1160, 13, 0, 1, 1), (2320, 1160, 24, 0, 1, 1), (2320, 1160, 25, 0, 1, 1), (2320, 1160, 32, 0, 1, 1),
+                                                            (2320, 1160, 33, 0, 1, 1), (2320, 1160, 64, 0, 1, 1), (2320, 1160, 65, 0, 1, 2), (2040, 2064, 16, 1, 1, 1), (2040, 2064, 17, 1, 1, 2),
                                                             (1064, 2040, 47, 0, 1, 2), (1064, 2040, 48, 0, 1, 1), (1064, 2040, 48, 0, 0, 1), (1064, 2040, 47, 1, 0, 2),
                                                             (1064, 2040, 48, 1, 1, 1), (1064, 2040, 48, 1, 0, 2)])
 @pytest.mark.parametrize("elem_bytes", [1, 2])
 def test_gemm_tile_rule(M, N, steps, both_mn, may_cut, ctas, elem_bytes):
     lib, K = L.kernels(), steps * (128 // elem_bytes)
-    assert lib.llmq_gemm_tile_ctas(M, N, K, elem_bytes, both_mn, may_cut, 148) == ctas
+    assert lib.llmq_gemm_tile_ctas(M, N, K, elem_bytes, both_mn, 128, may_cut, 148) == ctas
     if may_cut and steps >= 47:
         assert (lib.llmq_gemm_splitk_floats(M, N, K, elem_bytes, 148) > 0) == (ctas == 1 and steps == 48)
-    assert lib.llmq_gemm_tile_ctas(M, N, K * elem_bytes // 4, 4, both_mn, may_cut, 148) == 1      # fp32 operands
+    assert lib.llmq_gemm_tile_ctas(M, N, K * elem_bytes // 4, 4, both_mn, 128, may_cut, 148) == 1      # fp32 operands
+    for line, walk, short in ((64, 32, 8), (32, 24, 8), (16, 12, 6)):
+        if (M, N) in ((2320, 1160), (2040, 2064)):           # one round
+            assert lib.llmq_gemm_tile_ctas(M, N, K, elem_bytes, both_mn, line, may_cut, 148) == (1 if steps <= (min(walk, 16) if both_mn else walk) else 2)
+        if (M, N) == (9728, 904):
+            assert lib.llmq_gemm_tile_ctas(M, N, K, elem_bytes, both_mn, line, may_cut, 148) == (1 if steps <= short else 2)
 
 
 @pytest.mark.skipif(not L.have_kernels(), reason="native library not built")
