@@ -103,8 +103,16 @@ __device__ __forceinline__ void add_bias32(const GemmParams& p, int col0, float 
 // Shared memory one epilogue warp needs for the coalescing store path of epilogue_rows (32 rows x 128 bytes).
 constexpr int EPI_STAGE_BYTES_PER_WARP = 32 * 128;
 
-// bf16 C in whole sectors (GemmParams::c_sectors), not added to: lane = row, 32 columns at a time.  A lane that moves 16 bytes at a time touches every sector
-// twice.  Plain outputs of the CTA-pair kernel stay on the staged TMA stores: 4096 x 151936 x 896 824 us, 837 this way.
+// 32 bytes (16 bf16) of one row per lane: a whole sector per lane and instruction
+__device__ __forceinline__ void load_sector(const void* p, uint32_t (&r)[8]) {
+    asm volatile("ld.global.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]) : "l"(p) : "memory");
+}
+
+// bf16 C in whole sectors (GemmParams::c_sectors): lane = row, 32 columns at a time.  A lane that moves 16 bytes at a time touches every sector
+// twice.  Plain outputs of the CTA-pair kernel stay on the staged TMA stores: 4096 x 151936 x 896 824 us, 837 this way.  Old: the output is added to, for the few
+// columns of which a block of OldBlocks would be mostly empty.
+template <bool Old = false>
 __device__ __forceinline__ void epilogue_rows_sectors(const GemmParams& p, uint32_t t_row, int row, int col_base, int ncols, float alpha, float& tmax) {
     using namespace sm100;
     const bool row_ok = row < p.M;
@@ -114,13 +122,21 @@ __device__ __forceinline__ void epilogue_rows_sectors(const GemmParams& p, uint3
         const int col0 = col_base + c;
         if (col0 >= p.N) break;                    // uniform across the warp
         const int halves = col0 + 32 <= p.N ? 2 : 1;                // N is a multiple of 16
-        uint32_t r[32];
+        uint32_t r[32], old[2][8] = {};
         tmem_ld_32x32b_x32(t_row + c, r);
+        if constexpr (Old) {
+#pragma unroll
+            for (int h = 0; h < 2; ++h) if (h < halves && row_ok) load_sector(crow + col0 + 16 * h, old[h]);
+        }
         tmem_ld_wait();
         float v[32];
 #pragma unroll
         for (int j = 0; j < 32; ++j) v[j] = __uint_as_float(r[j]) * alpha;
         if (p.bias) add_bias32(p, col0, v);
+        if constexpr (Old) {
+#pragma unroll
+            for (int j = 0; j < 32; ++j) v[j] += __uint_as_float((j & 1) ? old[j / 16][(j % 16) / 2] & 0xffff0000u : old[j / 16][(j % 16) / 2] << 16);
+        }
         if (p.absmax_out && row_ok) {
 #pragma unroll
             for (int j = 0; j < 32; ++j) if (j < 16 * halves) tmax = fmaxf(tmax, fabsf(v[j]));

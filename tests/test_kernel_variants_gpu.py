@@ -434,8 +434,8 @@ def test_gemm_kernel_choice(M, N, steps, mn, parts, dt):
     assert parts > 1 or torch.equal(got[0], got[2])           # one order of the sum over K
 
 
-# bf16 outputs that are added to: blocks of 64 columns and remainders of 16, 32 and 48, ragged rows, tiles of 224 and 256 columns, several tiles per CTA in both kernels
-@pytest.mark.parametrize("M,N,Kd", [(130, 336, 64), (1000, 1008, 128), (300, 65, 64), (4100, 912, 640), (4096, 896, 1280), (9000, 2096, 192), (9000, 2096, 1216)])
+# bf16 outputs that are added to: up to 32 columns, blocks of 64 columns and remainders of 16, 32 and 48, ragged rows, tiles of 224 and 256 columns, several tiles per CTA in both kernels
+@pytest.mark.parametrize("M,N,Kd", [(130, 16, 64), (300, 32, 192), (20000, 32, 64), (300, 48, 64), (130, 336, 64), (1000, 1008, 128), (300, 65, 64), (4100, 912, 640), (4096, 896, 1280), (9000, 2096, 192), (9000, 2096, 1216)])
 @pytest.mark.parametrize("dt", [BF, F8])
 @pytest.mark.parametrize("mode", [0, 1, 2])
 def test_gemm_added_to(M, N, Kd, dt, mode):
