@@ -938,44 +938,42 @@ struct HeadSplit {
 // of 7 CTAs 15 reside, of 2 74).  Over 55 shapes (20 to 6731 tokens, 1 to 8 sequences, groups of 1 to 12 heads) the picked pair
 // takes 1.03 of the time of the best one on average, the rules for two launches one after the other took 1.10.  attention_backward, us, with those / picked:
 // 1 x 1024 tokens, 32 / 8 heads 58 / 42;  6 x 405, 12 / 2 35 / 31;  2 x 683, 28 / 4 58 / 44;  3 x 2048, 28 / 4 312 / 284;  4 x 1024, 16 / 2 86 / 70.
-// For sequences of one key block, whose few tiles the estimate of a tile says little about, the older rule stays unless the estimate is 1.35 times better:
-// 8 x 100, 32 / 8 30 / 21, but 24 x 128, 28 / 4 49 by the older rule and 56 by the estimate.
+// For sequences of one key block, whose few tiles the estimate of a tile says little about (7 x 33 tokens, 12 / 2 heads 10.7 by the rules for two launches, 12.0 by the estimate), those rules
+// stay unless the estimate of what they give is 1.45 times that of the best pair; over 19 such shapes that takes 1.04 of the best one. Both:  8 x 100, 32 / 8 30 / 21, 12 x 128, 28 / 4 34.5 / 24.3,
+// 9 x 16, 28 / 4 16.1 / 12.3.
 template <int HS>
 HeadSplit split_heads(int G, int base, int T, int smem) {
     const int heads_rule = dq_heads(G, base);
     if constexpr (HS == 64) return {1, heads_rule};
     const int nqb = (T + 63) / 64, nkb = (T + 127) / 128;
     const double mean_tiles = nqb - (nkb - 1);               // query blocks at or below the diagonal, mean over the key blocks
-    HeadSplit best{1, heads_rule};
-    double best_us = 0., rule_us = 0., rule_best = 0.;       // rule_us: estimate of the older rule, which looks at dK / dV alone; rule_best: the pair estimate of its parts
-    int rule_parts = 1;
-    for (int parts = 1; parts <= 8 && parts <= G; ++parts) {
-        const int resident = resident_clusters<HS>(parts, smem), heads = (G + parts - 1) / parts;
-        if (resident <= 0) continue;
+    const auto estimate = [&](int parts, int dq, int resident) {
+        const int heads = (G + parts - 1) / parts, cut = (G + dq - 1) / dq;              // dQ CTAs of an item
         const double sums = parts > 1 ? 2. + 0.5 * parts : 0.;
-        double parts_us = 0.;
-        for (int dq = G, last = 0; dq >= 1; --dq) {
-            const int cut = (G + dq - 1) / dq;               // dQ CTAs of an item; the smallest `dq` of every cut is looked at
-            if (dq > 1 && (G + dq - 2) / (dq - 1) == cut) continue;
-            if (cut == last) continue;
-            last = cut;
-            const double longest_dkdv = 5. + sums + heads * (0.25 + 0.85 * nqb), longest_dq = 4.2 + dq * (1.7 + 0.6 * nqb);
-            double us = longest_dkdv > longest_dq ? longest_dkdv : longest_dq;
-            const double ctas = static_cast<double>(base) * (parts + cut), at_once = static_cast<double>(resident) * parts;
-            if (ctas > at_once) {
-                const double work = base * (parts * (5. + sums) + G * (0.25 + 0.85 * mean_tiles) + cut * 4.2 + G * (1.7 + 0.6 * (nkb + 1)));
-                const double mean = work / ctas, shared = work / at_once + 0.5 * (us < mean ? us : mean);
-                if (shared > us) us = shared;
-            }
+        const double longest_dkdv = 5. + sums + heads * (0.25 + 0.85 * nqb), longest_dq = 4.2 + dq * (1.7 + 0.6 * nqb);
+        const double us = longest_dkdv > longest_dq ? longest_dkdv : longest_dq;
+        const double ctas = static_cast<double>(base) * (parts + cut), at_once = static_cast<double>(resident) * parts;
+        if (ctas <= at_once) return us;
+        const double work = base * (parts * (5. + sums) + G * (0.25 + 0.85 * mean_tiles) + cut * 4.2 + G * (1.7 + 0.6 * (nkb + 1)));
+        const double mean = work / ctas, shared = work / at_once + 0.5 * (us < mean ? us : mean);
+        return shared > us ? shared : us;
+    };
+    HeadSplit best{1, heads_rule}, rule{1, heads_rule};      // rule: that of two launches, which looks at dK / dV alone
+    double best_us = 0., rule_us = 0., rule_estimate = 0.;
+    for (int parts = 1; parts <= 8 && parts <= G; ++parts) {
+        const int resident = resident_clusters<HS>(parts, smem);
+        if (resident <= 0) continue;
+        for (int dq = G; dq >= 1; --dq) {
+            if (dq > 1 && (G + dq - 2) / (dq - 1) == (G + dq - 1) / dq) continue;        // the smallest `dq` of every cut is looked at
+            const double us = estimate(parts, dq, resident);
             if (best_us == 0. || us < best_us) { best = {parts, dq}; best_us = us; }
-            if (parts_us == 0. || us < parts_us) parts_us = us;
         }
+        const int heads = (G + parts - 1) / parts;
         const double rounds = (base + resident - 1) / resident, longest = static_cast<double>(nqb) * heads, average = mean_tiles * heads * base / resident;
         const double us = rounds * (5. + (parts > 1 ? 2. + 0.6 * parts : 0.)) + 0.9 * (longest > average ? longest : average);
-        if (rule_us == 0. || us < rule_us) { rule_us = us; rule_parts = parts; rule_best = parts_us; }
+        if (rule_us == 0. || us < rule_us) { rule_us = us; rule.dkdv = parts; rule_estimate = estimate(parts, heads_rule, resident); }
     }
-    if (nkb == 1 && rule_best <= 1.35 * best_us) return {rule_parts, heads_rule};
-    return best;
+    return nkb == 1 && rule_estimate <= 1.45 * best_us ? rule : best;
 }
 
 template <int HS>

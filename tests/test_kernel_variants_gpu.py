@@ -1168,3 +1168,10 @@ def test_adamw_subnormal_gradients(params, moments, eps):
     want = grad.double() / torch.tensor(eps, dtype=torch.float32).double().item()
     # the fp32 quotient, a few units in the last place; bf16 parameters are rounded up or down
     assert ((p.double() + want).abs() <= (2**-7 if params == BF else 1e-6) * want).all()
+
+
+# short sequences: the older rule's pair is kept or left by the estimate of that pair (12 sequences of 128 tokens leave it, 16 keep it)
+@pytest.mark.parametrize("B,T,Hq,Hkv,parts", [(12, 128, 28, 4, 1), (16, 128, 28, 4, 2), (7, 33, 12, 2, 1), (8, 20, 16, 2, 4)])
+def test_attention_backward_parts_of_short_sequences(B, T, Hq, Hkv, parts):
+    assert torch.cuda.get_device_properties(0).multi_processor_count != 148 or L.kernels().llmq_attention_dkdv_parts(B, T, Hq, Hkv, 128) == parts
+    test_attention_head_splits(128, B, T, Hq, Hkv)
