@@ -251,8 +251,8 @@ __device__ __forceinline__ void store_sector(void* p, const uint32_t* r) {
                  ::"l"(p), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]) : "memory");
 }
 
-// 1 / (1 + e^-x), the same bits as __fdividef(1.f, 1.f + __expf(-x)): subnormal values, for which those two take extra instructions, vanish in the sum or
-// are results that both give as 0 (a denominator above 2^126)
+// 1 / (1 + e^-x) = 1 / (1 + 2^(-x log2 e)).  The exponent in fp32 (its rounding and that of log2 e) makes the result of a negative x wrong by up to 1.23 |x| 2^-24 of itself, the approximations by
+// a few times 2^-23; subnormal numbers are flushed: of the power, which vanishes in the sum, and of the result, which is 0 below 2^-126.
 __device__ __forceinline__ float fast_sigmoid(float x) {
     float e, r;
     asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(-x * 1.4426950408889634f));

@@ -138,6 +138,7 @@ def test_attention_backward_parts_of_an_item(T, B, Hq, Hkv, parts):
 @pytest.mark.parametrize("B,T,Hq,Hkv", [(1, 70, 9, 1), (1, 128, 28, 4), (1, 129, 28, 4), (1, 333, 12, 2), (3, 257, 5, 1), (2, 683, 28, 4), (1, 1024, 32, 8), (9, 100, 32, 8)])
 def test_attention_backward_one_grid(HS, B, T, Hq, Hkv):
     most = max(B, 300 // ((T + 127) // 128 * Hkv) + 1)
+    assert L.kernels().llmq_attention_dkdv_parts(most, T, Hq, Hkv, HS) == 1
     g = torch.Generator(device=DEV).manual_seed(T)
     qkv = torch.randn(most, T, Hq + 2 * Hkv, HS, device=DEV, generator=g).to(BF)
     dout = torch.randn(most, T, Hq, HS, device=DEV, generator=g).to(BF)
@@ -359,6 +360,15 @@ def test_split_k_reduce(N, out_dt):
     assert abs(am.item() - want.abs().max().item()) < 1e-3 * want.abs().max().item()
 
 
+def _through_the_second_kernel(M, N, Kd, out, a, b, **kw):
+    """The same GEMM into a view that is not aligned to four columns, whose parts therefore go through the workspace."""
+    view = torch.full((M + 1, N + 4), 9.0, device=DEV, dtype=out.dtype)[:M, 1:N + 1]
+    view.copy_(out)
+    assert L.calls().llmq_gemm_split_mode(view, M, N, Kd, a.element_size(), view.stride(0), int(out.dtype != BF), 148) == 2
+    K.gemm(view, a, b, **kw)
+    return view
+
+
 # K cut into 2 to 8 parts that a cluster adds up, uneven shares of its rows (3, 5, 6, 7 parts), ragged last tiles, both tile widths; one tile more than clusters
 # reside (36 of 4 parts, 28 of 5, 16 of 8) and N = 301 go through the second kernel
 @pytest.mark.parametrize("M,N,Kd,parts", [(1001, 896, 1152, 2), (130, 8196, 2048, 2), (339, 3584, 3584, 3), (64, 2048, 1536, 3), (200, 2052, 2048, 4), (1152, 896, 2048, 4),
@@ -374,9 +384,11 @@ def test_split_k_parts(M, N, Kd, parts, dt, out_dt):
     rows = torch.full((M + 1, N), 9.0, device=DEV, dtype=out_dt)
     am = torch.zeros(1, device=DEV)
     plain, added = rows[:M], prev.clone()
+    two = _through_the_second_kernel(M, N, Kd, plain, a, b), _through_the_second_kernel(M, N, Kd, prev, a, b, bias=bias, accumulate=True, scale_a=scale)
     K.gemm(plain, a, b)
     K.gemm(added, a, b, bias=bias, accumulate=True, scale_a=scale, absmax=am)
     K.check_status(torch.device(DEV, 0))
+    assert torch.equal(plain, two[0]) and torch.equal(added, two[1])             # the parts are added up in one order
     prod = a.double() @ b.double().t()
     want = 0.5 * prod + bias.double() + prev.double()
     # fp32 sums; products of fp32 operands have 10-bit mantissas (tf32 truncates: 2^-10 an operand); one rounding to bf16 of the outputs
@@ -398,40 +410,45 @@ def test_split_k_narrow(M, N, Kd, out_dt):
     rows = torch.full((M + 1, N), 9.0, device=DEV, dtype=out_dt)
     prev = torch.randn(M, N, device=DEV, generator=g).to(out_dt)
     added = prev.clone()
+    two = _through_the_second_kernel(M, N, Kd, prev, a, b), _through_the_second_kernel(M, N, Kd, prev, a, b, accumulate=True)
     K.gemm(rows[:M], a, b)
     K.gemm(added, a, b, accumulate=True)
     K.check_status(torch.device(DEV, 0))
+    assert torch.equal(rows[:M], two[0]) and torch.equal(added, two[1])
     prod = a.double() @ b.double().t()
     eps = 1e-5 + (2 ** -8 if out_dt == BF else 0)             # fp32 sums, one rounding of the outputs
     assert rel(rows[:M], prod) < eps and rel(added, prod + prev.double()) < eps
     assert (rows[M] == 9).all()
 
 
-# the kernel for a plain GEMM on both sides of each line of the rule: short K (8 and 9 steps of 128 bytes), one round of tiles (64 / 65 steps, both operands MN-major
-# 16 / 17), more than half of the SMs idle (47 / 48 steps, from where K is cut in two); odd edges of the last tiles
-@pytest.mark.parametrize("M,N,steps,mn,parts", [(9728, 904, 8, 0, 1), (9728, 904, 9, 0, 1), (2320, 1160, 64, 0, 1), (2320, 1160, 65, 0, 1), (2056, 2064, 16, 1, 1),
-                                                (2056, 2064, 17, 1, 1), (1064, 2040, 47, 0, 1), (1064, 2040, 48, 0, 2)])
+# the kernel for a plain GEMM on both sides of each line of the rule for rows that start with a 128-byte line: short K (8 and 9 steps of 128 bytes), one round of tiles (64 / 65 steps, both
+# operands MN-major 16 / 17), more than half of the SMs idle (47 / 48 steps, from where K is cut in two); odd edges of the last tiles
+@pytest.mark.parametrize("M,N,steps,mn,ctas,parts", [(9728, 904, 8, 0, 1, 1), (9728, 904, 9, 0, 2, 1), (2320, 1160, 64, 0, 1, 1), (2320, 1160, 65, 0, 2, 1), (2040, 2064, 16, 1, 1, 1),
+                                                     (2040, 2064, 17, 1, 2, 1), (1064, 2040, 47, 0, 2, 1), (1064, 2040, 48, 0, 1, 2)])
 @pytest.mark.parametrize("dt", [BF, F8])
-def test_gemm_kernel_choice(M, N, steps, mn, parts, dt):
+def test_gemm_kernel_choice(M, N, steps, mn, ctas, parts, dt):
     lib, step = L.kernels(), 128 // dt.itemsize
     Kd = steps * step - 8 * (2 // dt.itemsize)                # the last step is not whole
     if mn and dt == F8:
         M, N = M // 16 * 16, N // 16 * 16
     assert lib.llmq_gemm_splitk_floats(M, N, Kd, dt.itemsize, 148) == (parts * M * N if parts > 1 else 0)
+    assert lib.llmq_gemm_tile_ctas(M, N, Kd, dt.itemsize, mn, 128, 1, 148) == ctas
     g = torch.Generator(device=DEV).manual_seed(M + steps)
-    a, b = (torch.randn(*((Kd, r) if mn else (r, Kd)), device=DEV, generator=g).to(dt) for r in (M, N))
+    shapes = [(Kd, r) if mn else (r, Kd) for r in (M, N)]
+    a, b = (torch.randn(rows, -(-cols // 128) * 128, device=DEV, generator=g).to(dt)[:, :cols] for rows, cols in shapes)
     got = []
     try:
         for mode in (0, 1, 2):
             lib.llmq_gemm_set_mode(mode)
             out = torch.full((M, N), 9.0, device=DEV, dtype=BF)
+            cut = lib.llmq_gemm_splitk_floats(M, N, Kd, dt.itemsize, 148) > 0
             K.gemm(out, a, b, a_mn=bool(mn), b_mn=bool(mn))
-            got.append(out)
+            got.append((out, cut))
     finally:
         lib.llmq_gemm_set_mode(0)
     ad, bd = (x.double().t() if mn else x.double() for x in (a, b))
-    assert rel(got[0], ad @ bd.t()) < 2**-8                   # fp32 sums, one rounding to bf16
-    assert parts > 1 or torch.equal(got[0], got[2])           # one order of the sum over K
+    assert rel(got[0][0], ad @ bd.t()) < 2**-8                # fp32 sums, one rounding to bf16
+    assert all(torch.equal(got[0][0], out) for out, cut in got if cut == (parts > 1))            # one order of the sum over K, cut or not
 
 
 # bf16 outputs that are added to: up to 32 columns, blocks of 64 columns and remainders of 16, 32 and 48, ragged rows, tiles of 224 and 256 columns, several tiles per CTA in both kernels
@@ -1011,6 +1028,24 @@ def test_swiglu_gate_extremes(dt):
     tol = (2**-8 if dt == BF else 0) + (8 + gate.double().abs().clamp(max=104)) * 2**-24
     assert ((out.double() - want).abs()[finite] <= (tol * want.abs() + 1e-34)[finite]).all()
     assert (out[~finite] == math.inf).all()
+
+
+# the sigmoid 1 / (1 + 2^(-g log2 e)) at every bf16 gate, and at fp32 gates of random bits, with the bound above and the error of log2 e as an fp32 number (1.3e-8 of it, 0.23 x 2^-24), by which the
+# sigmoid is wrong by another 0.23 |g| 2^-24
+@pytest.mark.parametrize("dt", [BF, torch.float32])
+def test_swiglu_every_gate(dt):
+    if dt == BF:
+        gate = torch.arange(-32768, 32768, device=DEV).to(torch.int16).view(BF)
+    else:
+        gate = torch.randint(-2**31, 2**31, (1 << 21,), device=DEV, generator=torch.Generator(device=DEV).manual_seed(1)).to(torch.int32).view(torch.float32)
+    gate = gate.view(-1, 512)
+    out = torch.empty_like(gate)
+    K.swiglu_forward(out, torch.cat([torch.ones_like(gate), gate], 1))
+    want = gate.double() * torch.sigmoid(gate.double())
+    assert torch.equal(out.isnan(), want.isnan())
+    finite = want.isfinite() & (want.abs() < torch.finfo(dt).max)
+    tol = (2**-8 if dt == BF else 0) + (8 + 1.25 * gate.double().abs().clamp(max=104)) * 2**-24
+    assert ((out.double() - want).abs()[finite] <= (tol * want.abs() + 1e-34)[finite]).all()
 
 
 # RoPE, a head of a token per thread (small calls) and two: odd and even numbers of heads (the last thread of a token has one), head sizes whose halves are 1, 2, 3, 4 and 8 vectors, one token, in
