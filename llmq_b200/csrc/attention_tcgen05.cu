@@ -23,19 +23,20 @@
 // of each kind come first.  attention_backward in us, a launch for each kind / one:  8 x 1024 tokens, 14 / 2 heads of 64 112 / 80;  4 x 1024 94 / 73;  1 x 333, 12 / 2
 // heads of 128 21.9 / 15.1;  2 x 700, 24 / 8 of 128 54 / 38;  where each kind alone fills the SMs for many rounds, 8 x 2048, 28 / 4 of 128, 761 / 758.
 //
-// What bounds it: no unit is saturated except the tensor pipe of dK / dV with head size 128 (1300 cycles of MMAs in about 1400 per tile;
-// 48 cycles per N = 64 MMA with both operands in shared memory, 33 with A in tensor memory, 64 per N = 128), the rest is the chain of
+// What bounds it, head size 128: a tile of dK / dV takes 1190 cycles (clock stamps, 8 x 2048 tokens, 28 / 4 heads).  Its MMAs need 1024 of the tensor pipe and 1024 of shared memory: 16 of N = 64
+// with both operands in shared memory, 32 cycles of the pipe and 48 of reading them, 8 of N = 128 with A in tensor memory, 64 and 32; one after the other they take 1300.  A tile of dQ
+// takes 880, its MMAs 768.  At head size 64 no unit is saturated.  The rest is the chain of
 // hand-overs of a tile.  A wait on an mbarrier costs a warp about 150 cycles even when the phase is complete, and several times that
 // while MMAs with both operands in shared memory run: those take nearly all of its bandwidth.  Hence two groups of compute warps, two
 // issuing warps, row statistics in few wide loads, and everything that comes from global memory (Q / dO and the statistics of the next
 // head or tile) fetched a tile or a head ahead by a warp of its own; the statistics that the producer used to wait for tile by tile alone
-// cost 10 to 20 % of dK / dV.  Times of the two kinds launched one after the other, us, one group and one issuing warp -> now:
-//                                          dK / dV         dQ
-//   8 x 2048 tokens, 28 / 4 heads of 128   425 -> 364   403 -> 331
-//   1 x 8192, 32 / 8 heads of 128          880 -> 752   708 -> 620
-//   8 x 1024, 14 / 2 heads of 64            87 -> 68     56 -> 42
-//   2 x 4096, 32 / 8 heads of 64           368 -> 285   300 -> 221
-//   1 x 333, 12 / 2 heads of 128            37 -> 30     10 -> 9      (one CTA per item; with a cluster dK / dV takes 14)
+// cost 10 to 20 % of dK / dV.  Times of the two kinds as two launches, one after the other, before they shared a grid, us, one group and one issuing warp / two:
+//                                          dK / dV      dQ
+//   8 x 2048 tokens, 28 / 4 heads of 128   425 / 364   403 / 331
+//   1 x 8192, 32 / 8 heads of 128          880 / 752   708 / 620
+//   8 x 1024, 14 / 2 heads of 64            87 / 68     56 / 42
+//   2 x 4096, 32 / 8 heads of 64           368 / 285   300 / 221
+//   1 x 333, 12 / 2 heads of 128            37 / 30     10 / 9      (one CTA per item; with a cluster dK / dV took 14)
 // Not better: score tiles of 128 columns without a second buffer; with head size 64 P^T in columns of its own and S issued before the sums
 // of the tile two before (dK / dV 68 -> 77: the groups then meet at the exponentials).
 #include <cstdlib>

@@ -566,20 +566,24 @@ static bool uses_pair_kernel(int M, int N, int K, int elem_bytes, bool fused, bo
 // shorter.  One / pair tiles over 890 shapes: one round, rows of whole lines 0.63-1.05 up to 64 steps;  of 64 bytes 0.76-1.04 up to 34 steps, then up to 1.14;  of 32 0.76-1.01 up to 24, 1.10
 // with 28, 1.20 with 46;  of 16 (8-bit elements) 0.92-1.06 up to 14, 1.13 with 28, 1.30 with 60 (1728 x 2080 x 7632 e4m3 38.8 / 29.8).  Short K with rows of 16 0.67-0.99 up to 6 steps, up to 1.13 with
 // 7 and 8 (2784 x 7632 x 1008 e4m3 30.0 / 26.4).
-static bool better_with_one_cta(int M, int N, int K, int elem_bytes, bool both_mn, int line, int num_sms) {
-    if (g_gemm_mode != 0) return false;
+// `output`: bf16 that is not added to and not made of whole sectors leaves the epilogue of this kernel 16 bytes a lane or less, that of the pairs through TMA or coalesced stores, and the pairs keep
+// it (73 shapes with N a multiple of 4 or 8, 0.67-1.27 of the pairs' time, 1.04 on average: 7744 x 312 x 736 10.4 / 9.2, 6704 x 4280 x 104 31.7 / 28.7).  fp32: 0.54-1.03 up to 32 steps, up to 1.06 behind.
+enum GemmOutput { kOutSectors, kOutPieces, kOutFp32 };          // bf16 in whole sectors or added to, other bf16, fp32
+static bool better_with_one_cta(int M, int N, int K, int elem_bytes, bool both_mn, int line, int output, int num_sms) {
+    if (g_gemm_mode != 0 || output == kOutPieces) return false;
     const int bk = 128 / elem_bytes, k_iters = (K + bk - 1) / bk;
     const long long tiles = tiles_of(M, N, 128, 256);
-    const int walk = line >= 128 ? 64 : line >= 64 ? 32 : line >= 32 ? 24 : 12;
+    int walk = line >= 128 ? 64 : line >= 64 ? 32 : line >= 32 ? 24 : 12;
+    if (output == kOutFp32 && walk > 32) walk = 32;
     return k_iters <= (line >= 32 ? 8 : 6) || (tiles <= num_sms && 2 * tiles > num_sms && k_iters <= (both_mn && walk > 16 ? 16 : walk));
 }
 
-static bool takes_pair_kernel(int M, int N, int K, int elem_bytes, bool both_mn, int line, bool fused, bool may_cut, int num_sms) {
-    return uses_pair_kernel(M, N, K, elem_bytes, fused, may_cut || !both_mn, num_sms) && (fused || !better_with_one_cta(M, N, K, elem_bytes, both_mn, line, num_sms));
+static bool takes_pair_kernel(int M, int N, int K, int elem_bytes, bool both_mn, int line, int output, bool fused, bool may_cut, int num_sms) {
+    return uses_pair_kernel(M, N, K, elem_bytes, fused, may_cut || !both_mn, num_sms) && (fused || !better_with_one_cta(M, N, K, elem_bytes, both_mn, line, output, num_sms));
 }
-// CTAs that work on a tile of a plain GEMM of this shape: 2 or 1 (for tests; nothing is launched)
-extern "C" int llmq_gemm_tile_ctas(int M, int N, int K, int elem_bytes, int both_mn_major, int line, int may_cut, int num_sms) {
-    return takes_pair_kernel(M, N, K, elem_bytes, both_mn_major != 0, line, false, may_cut != 0, num_sms) ? 2 : 1;
+// CTAs that work on a tile of a plain GEMM of this shape (output: a GemmOutput): 2 or 1 (for tests; nothing is launched)
+extern "C" int llmq_gemm_tile_ctas(int M, int N, int K, int elem_bytes, int both_mn_major, int line, int output, int may_cut, int num_sms) {
+    return takes_pair_kernel(M, N, K, elem_bytes, both_mn_major != 0, line, output, false, may_cut != 0, num_sms) ? 2 : 1;
 }
 
 // Tile rows of 256 that the pair kernel works through together.  B is read from memory once per group, so a group is as large as its rows of A
@@ -757,7 +761,9 @@ static int gemm_impl(const void* A, const void* B, void* C, const void* bias,
     const bool may_cut = splitk_floats < 0 ? split_plan(C, M, N, K, eb, ldc, c_dtype, true, num_sms).cluster
                                            : splitk_ws && static_cast<long long>(splitk_parts(M, N, K, eb, num_sms)) * M * N <= splitk_floats;
     const uintptr_t starts = reinterpret_cast<uintptr_t>(A) | reinterpret_cast<uintptr_t>(B) | static_cast<uintptr_t>(lda * eb) | static_cast<uintptr_t>(ldb * eb) | 128u;
-    const bool pair_kernel = takes_pair_kernel(M, N, K, eb, a_mn_major && b_mn_major, static_cast<int>(starts & (~starts + 1)), fused, may_cut, num_sms);
+    const bool sectors = c_dtype == 0 && N % 16 == 0 && ldc % 16 == 0 && (reinterpret_cast<uintptr_t>(C) & 31u) == 0;
+    const int output = c_dtype != 0 ? kOutFp32 : sectors || accumulate ? kOutSectors : kOutPieces;
+    const bool pair_kernel = takes_pair_kernel(M, N, K, eb, a_mn_major && b_mn_major, static_cast<int>(starts & (~starts + 1)), output, fused, may_cut, num_sms);
     // An MN-major stage that is several 128-byte chunks wide (16-bit operands; the 256 rows of B of the one-CTA kernel) is fetched with
     // one 3-D load instead of one 2-D load per chunk: the loads of a stage were issued one after the other for longer than its MMAs
     // run.  bf16, CTA pairs, TFLOP/s with 2-D loads / 3-D loads / 3-D loads and a K loop per kind of load (gemm_tcgen05_2cta.cu), K-major
@@ -796,7 +802,7 @@ static int gemm_impl(const void* A, const void* B, void* C, const void* bias,
     p.bias = bias; p.bias_dtype = bias_dtype;
     p.group_rows = pair_group_rows(K, eb, rs != nullptr || ready_flags != nullptr);
     p.bn = pair_bn; p.b_stage_bytes = b_rows * 128;
-    p.c_sectors = rs == nullptr && (accumulate || !pair_kernel) && c_dtype == 0 && N % 16 == 0 && ldc % 16 == 0 && (reinterpret_cast<uintptr_t>(C) & 31u) == 0;
+    p.c_sectors = rs == nullptr && (accumulate || !pair_kernel) && sectors;
     p.scale_a = scale_a; p.scale_b = scale_b; p.alpha = alpha;
     p.absmax_out = absmax_out; p.status = status;
     p.ready_flags = ready_flags; p.ready_gen = ready_gen; p.ready_rows_per_src = ready_rows_per_src > 0 ? ready_rows_per_src : 1;

@@ -626,14 +626,11 @@ int launch_bwd(void* dinp_, void* dweight, float* scratch, const void* dout_, co
     // registers: 2000 x 1024 10.8 / 9.9 and 13.5 / 13.8, 3000 x 768 (28 MB) 11.5 / 10.5 and 14.2 / 15.4, 4096 x 256 11.3 / 10.4 and 12.0 / 14.5;  beyond 32 MB, where they
     // rarely lie in the L2 as a whole, 8192 x 512 (50 MB) 16.9 / 15.1 and 18.8 / 24.6, 8192 x 768 (75 MB) 18.3 / 20.5 and 23.6 / 27.6.
     const long long bytes = 3ll * rows * C * static_cast<long long>(sizeof(T));
-    const bool in_registers = rows <= 2 * num_blocks || (sizeof(T) == 4 && bytes <= (32ll << 20)), by_threads = sizeof(T) == 2 && C <= 768 && bytes <= (96ll << 20);
-    if (vecs <= 1 && in_registers) {
-        rmsnorm_bwd_reg_kernel<T, 1, 0><<<num_blocks, NORM_THREADS, 0, s>>>(dinp, scratch, dout, inp, w, rstd, rows, C, absmax);
-        rc = LLMQ_LAUNCH_CHECK();
-    }
-    else if (vecs <= 1 && by_threads) {
-        constexpr int stages = 4;                            // 18 KB at most
-        rmsnorm_bwd_reg_kernel<T, 1, stages><<<num_blocks, NORM_THREADS, stages * 3 * C * sizeof(T), s>>>(dinp, scratch, dout, inp, w, rstd, rows, C, absmax);
+    const bool in_registers = rows <= 2 * num_blocks || (sizeof(T) == 4 && bytes <= (32ll << 20)), by_threads = C <= 768 && bytes <= (96ll << 20);
+    if (vecs <= 1 && (in_registers || (sizeof(T) == 2 && by_threads))) {
+        constexpr int stages = sizeof(T) == 2 ? 4 : 0;       // 18 KB at most
+        if (in_registers) rmsnorm_bwd_reg_kernel<T, 1, 0><<<num_blocks, NORM_THREADS, 0, s>>>(dinp, scratch, dout, inp, w, rstd, rows, C, absmax);
+        else rmsnorm_bwd_reg_kernel<T, 1, stages><<<num_blocks, NORM_THREADS, stages * 3 * C * sizeof(T), s>>>(dinp, scratch, dout, inp, w, rstd, rows, C, absmax);
         rc = LLMQ_LAUNCH_CHECK();
     }
     else if (vecs <= 1) rc = launch_bwd_ring<T, 1, 4, 3>(dinp, scratch, dout, inp, w, rstd, rows, C, absmax, num_blocks, status, s);

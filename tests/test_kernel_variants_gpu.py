@@ -423,8 +423,8 @@ def test_split_k_narrow(M, N, Kd, out_dt):
 
 # the kernel for a plain GEMM on both sides of each line of the rule for rows that start with a 128-byte line: short K (8 and 9 steps of 128 bytes), one round of tiles (64 / 65 steps, both
 # operands MN-major 16 / 17), more than half of the SMs idle (47 / 48 steps, from where K is cut in two); odd edges of the last tiles
-@pytest.mark.parametrize("M,N,steps,mn,ctas,parts", [(9728, 904, 8, 0, 1, 1), (9728, 904, 9, 0, 2, 1), (2320, 1160, 64, 0, 1, 1), (2320, 1160, 65, 0, 2, 1), (2040, 2064, 16, 1, 1, 1),
-                                                     (2040, 2064, 17, 1, 2, 1), (1064, 2040, 47, 0, 2, 1), (1064, 2040, 48, 0, 1, 2)])
+@pytest.mark.parametrize("M,N,steps,mn,ctas,parts", [(9728, 912, 8, 0, 1, 1), (9728, 912, 9, 0, 2, 1), (2320, 1168, 64, 0, 1, 1), (2320, 1168, 65, 0, 2, 1), (2040, 2064, 16, 1, 1, 1),
+                                                     (2040, 2064, 17, 1, 2, 1), (1064, 2032, 47, 0, 2, 1), (1064, 2032, 48, 0, 1, 2)])
 @pytest.mark.parametrize("dt", [BF, F8])
 def test_gemm_kernel_choice(M, N, steps, mn, ctas, parts, dt):
     lib, step = L.kernels(), 128 // dt.itemsize
@@ -432,7 +432,7 @@ def test_gemm_kernel_choice(M, N, steps, mn, ctas, parts, dt):
     if mn and dt == F8:
         M, N = M // 16 * 16, N // 16 * 16
     assert lib.llmq_gemm_splitk_floats(M, N, Kd, dt.itemsize, 148) == (parts * M * N if parts > 1 else 0)
-    assert lib.llmq_gemm_tile_ctas(M, N, Kd, dt.itemsize, mn, 128, 1, 148) == ctas
+    assert lib.llmq_gemm_tile_ctas(M, N, Kd, dt.itemsize, mn, 128, 0, 1, 148) == ctas
     g = torch.Generator(device=DEV).manual_seed(M + steps)
     shapes = [(Kd, r) if mn else (r, Kd) for r in (M, N)]
     a, b = (torch.randn(rows, -(-cols // 128) * 128, device=DEV, generator=g).to(dt)[:, :cols] for rows, cols in shapes)

@@ -97,15 +97,18 @@ def test_split_k_workspace_rule(elem_bytes):
 @pytest.mark.parametrize("elem_bytes", [1, 2])
 def test_gemm_tile_rule(M, N, steps, both_mn, may_cut, ctas, elem_bytes):
     lib, K = L.kernels(), steps * (128 // elem_bytes)
-    assert lib.llmq_gemm_tile_ctas(M, N, K, elem_bytes, both_mn, 128, may_cut, 148) == ctas
+    assert lib.llmq_gemm_tile_ctas(M, N, K, elem_bytes, both_mn, 128, 0, may_cut, 148) == ctas
     if may_cut and steps >= 47:
         assert (lib.llmq_gemm_splitk_floats(M, N, K, elem_bytes, 148) > 0) == (ctas == 1 and steps == 48)
-    assert lib.llmq_gemm_tile_ctas(M, N, K * elem_bytes // 4, 4, both_mn, 128, may_cut, 148) == 1      # fp32 operands
+    assert lib.llmq_gemm_tile_ctas(M, N, K * elem_bytes // 4, 4, both_mn, 128, 0, may_cut, 148) == 1      # fp32 operands
+    if (M, N) in ((2320, 1160), (2040, 2064), (9728, 904)):
+        assert lib.llmq_gemm_tile_ctas(M, N, K, elem_bytes, both_mn, 128, 1, may_cut, 148) == 2              # bf16 that is not made of whole sectors
+        assert lib.llmq_gemm_tile_ctas(M, N, K, elem_bytes, both_mn, 128, 2, may_cut, 148) == (2 if steps > 32 else ctas)        # fp32
     for line, walk, short in ((64, 32, 8), (32, 24, 8), (16, 12, 6)):
         if (M, N) in ((2320, 1160), (2040, 2064)):           # one round
-            assert lib.llmq_gemm_tile_ctas(M, N, K, elem_bytes, both_mn, line, may_cut, 148) == (1 if steps <= (min(walk, 16) if both_mn else walk) else 2)
+            assert lib.llmq_gemm_tile_ctas(M, N, K, elem_bytes, both_mn, line, 0, may_cut, 148) == (1 if steps <= (min(walk, 16) if both_mn else walk) else 2)
         if (M, N) == (9728, 904):
-            assert lib.llmq_gemm_tile_ctas(M, N, K, elem_bytes, both_mn, line, may_cut, 148) == (1 if steps <= short else 2)
+            assert lib.llmq_gemm_tile_ctas(M, N, K, elem_bytes, both_mn, line, 0, may_cut, 148) == (1 if steps <= short else 2)
 
 
 @pytest.mark.skipif(not L.have_kernels(), reason="native library not built")
